@@ -16,6 +16,8 @@
 //        * and on the way back PULLS its k expert outputs per token from the owners' output buffers with 16-byte P2P
 //          loads, doing the weighted combine on the fly.
 //      No host synchronisation, no NCCL call, no re-sort.  Flags are epoch-valued words in a symmetric flag page.
+//  (4) the same for experts that are all local: counting sort of the choices, row gather, weighted row sum and their
+//      gradients.
 #include <stdio.h>
 
 #include "common.cuh"
@@ -454,6 +456,171 @@ __global__ void __launch_bounds__(256) moe_gather_combine_kernel(const T* __rest
   }
 }
 
+// ------------------------------------------------------------------------------------------------ (4) local experts
+// Dropless dispatch / combine without expert parallelism.  A choice i = t * k + j sends token t to expert topk_idx[i]; its
+// row sits at slot[i] of a buffer in which every expert's rows keep the order of their choices and start on a multiple of
+// `align` rows (what the grouped weight-gradient GEMM wants).  A counting sort by two kernels replaces a radix sort of the
+// choices, a host read of the counts and a dozen index operations; the row kernels below replace index_select / index_add
+// (bf16 atomics: 1049 us of a 3350 us layer of 64 experts, 24576 rows of 2048) by one read and one write of every row.
+constexpr int SORT_THREADS = 512;
+constexpr int SORT_ITEMS = 8;
+
+__global__ void __launch_bounds__(256) moe_count_kernel(const int64_t* __restrict__ topk_idx, int64_t n, int E,
+                                                        int* __restrict__ counts) {
+  extern __shared__ int hist[];
+  for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = 0;
+  __syncthreads();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t e = topk_idx[i];
+    if (e >= 0 && e < E) atomicAdd(&hist[e], 1);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x)
+    if (hist[e]) atomicAdd(&counts[e], hist[e]);
+}
+
+// block e < E: places expert e's choices in order and marks the padding rows behind them (src = -1); block E marks the rows
+// behind the last expert, choices of no expert (slot = -1) and writes the padded counts.
+__global__ void __launch_bounds__(SORT_THREADS) moe_place_kernel(const int64_t* __restrict__ topk_idx, int64_t n, int E, int align,
+                                                                 int bound, const int* __restrict__ counts, int* __restrict__ slot,
+                                                                 int* __restrict__ src, int64_t* __restrict__ padded_counts) {
+  __shared__ int warp_sum_s[SORT_THREADS / 32];
+  __shared__ int start_s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, e = blockIdx.x;
+  int part = 0;
+  for (int o = tid; o < e; o += SORT_THREADS) part += (counts[o] + align - 1) / align * align;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+  if (lane == 0) warp_sum_s[warp] = part;
+  __syncthreads();
+  if (tid == 0) {
+    int acc = 0;
+    for (int w = 0; w < SORT_THREADS / 32; ++w) acc += warp_sum_s[w];
+    start_s = acc;
+  }
+  __syncthreads();
+  int at = start_s;
+  if (e == E) {
+    for (int r = at + tid; r < bound; r += SORT_THREADS) src[r] = -1;
+    for (int o = tid; o < E; o += SORT_THREADS) padded_counts[o] = (counts[o] + align - 1) / align * align;
+    for (int64_t i = tid; i < n; i += SORT_THREADS)
+      if (topk_idx[i] < 0 || topk_idx[i] >= E) slot[i] = -1;
+    return;
+  }
+  const int end = at + (counts[e] + align - 1) / align * align;
+  // a thread looks at SORT_ITEMS neighbouring choices per round, so that a round's two barriers cover 4096 of them (one
+  // choice per thread: 26 us for 24576 choices of 64 experts, all of it barrier latency)
+  for (int64_t base = 0; base < n; base += SORT_THREADS * SORT_ITEMS) {
+    const int64_t i0 = base + (int64_t)tid * SORT_ITEMS;
+    unsigned hit = 0;
+#pragma unroll
+    for (int j = 0; j < SORT_ITEMS; ++j) hit |= (unsigned)(i0 + j < n && topk_idx[i0 + j] == e) << j;
+    const int own = __popc(hit);
+    int upto = own;                                        // inclusive sum over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    __syncthreads();                                       // the sums of the last round have been read
+    if (lane == 31) warp_sum_s[warp] = upto;
+    __syncthreads();
+    int before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < SORT_THREADS / 32; ++w) {
+      const int c = warp_sum_s[w];
+      before += w < warp ? c : 0;
+      total += c;
+    }
+    int r = at + before + upto - own;
+#pragma unroll
+    for (int j = 0; j < SORT_ITEMS; ++j)
+      if (hit >> j & 1) {
+        slot[i0 + j] = r;
+        src[r++] = (int)(i0 + j);
+      }
+    at += total;
+  }
+  for (int r = at + tid; r < end; r += SORT_THREADS) src[r] = -1;
+}
+
+// rows[r] = x[src[r] / k], zeros where src[r] < 0.  One warp per row, 16-byte vectors, four in flight per lane.
+__global__ void __launch_bounds__(256) moe_take_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ src,
+                                                            uint4* __restrict__ rows, int bound, int k, int row_vecs) {
+  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= bound) return;
+  const int i = src[r];
+  const uint4* s = x + (int64_t)(i < 0 ? 0 : i / k) * row_vecs;
+  uint4* d = rows + (int64_t)r * row_vecs;
+#pragma unroll 4
+  for (int c = lane; c < row_vecs; c += 32) d[c] = i < 0 ? make_uint4(0u, 0u, 0u, 0u) : __ldg(s + c);
+}
+
+// out[t] = sum_j w[t, j] rows[slot[t, j]] (w = null: plain sum), fp32, j ascending, one rounding
+template <typename T>
+__global__ void __launch_bounds__(256) moe_sum_rows_kernel(const T* __restrict__ rows, const int* __restrict__ slot,
+                                                           const float* __restrict__ w, T* __restrict__ out, int k, int H) {
+  constexpr int VEC = Vec16<T>::N;
+  const int64_t t = blockIdx.x;
+  for (int c = threadIdx.x * VEC; c < H; c += blockDim.x * VEC) {
+    float acc[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
+#pragma unroll 4
+    for (int j = 0; j < k; ++j) {
+      const int r = __ldg(slot + t * k + j);
+      if (r < 0) continue;
+      const float f = w != nullptr ? __ldg(w + t * k + j) : 1.f;
+      Vec16<T> v;
+      v.load_nc(rows + (int64_t)r * H + c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) acc[e] = fmaf(f, v.get(e), acc[e]);
+    }
+    Vec16<T> o;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) o.set(e, acc[e]);
+    o.store_na(out + t * H + c);
+  }
+}
+
+// drows[r] = w[src[r]] g[src[r] / k] (zeros where src[r] < 0), dw[src[r]] = <g[src[r] / k], rows[r]>.  One warp per row.
+template <typename T>
+__global__ void __launch_bounds__(256) moe_sum_rows_bwd_kernel(const T* __restrict__ g, const T* __restrict__ rows,
+                                                               const int* __restrict__ src, const float* __restrict__ w,
+                                                               T* __restrict__ drows, float* __restrict__ dw, int bound, int k,
+                                                               int H) {
+  constexpr int VEC = Vec16<T>::N;
+  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= bound) return;
+  const int i = src[r];
+  T* d = drows + (int64_t)r * H;
+  Vec16<T> o;
+  if (i < 0) {
+    o.raw = make_uint4(0u, 0u, 0u, 0u);
+    for (int c = lane * VEC; c < H; c += 32 * VEC) o.store(d + c);
+    return;
+  }
+  const T* gr = g + (int64_t)(i / k) * H;
+  const T* yr = rows + (int64_t)r * H;
+  const float f = w[i];
+  float dot = 0.f;
+#pragma unroll 4
+  for (int c = lane * VEC; c < H; c += 32 * VEC) {
+    Vec16<T> a, b;
+    a.load(gr + c);
+    b.load_nc(yr + c);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      const float x = a.get(e);
+      dot = fmaf(x, b.get(e), dot);
+      o.set(e, f * x);
+    }
+    o.store(d + c);
+  }
+  dot = warp_sum(dot);
+  if (lane == 0) dw[i] = dot;
+}
+
 }  // namespace
 
 // Copy the live part of a receive buffer into an autograd-owned tensor: rows of the padded local layout that hold a
@@ -487,6 +654,47 @@ __global__ void __launch_bounds__(256) ep_take_rows_kernel(uint4* __restrict__ d
 extern "C" {
 
 int cb_moe_flag_words() { return FLAG_WORDS; }
+
+// ---- local experts.  counts int32 [E] (zeroed here), slot int32 [n], src int32 [bound], padded_counts int64 [E];
+// bound >= n + E * (align - 1) rounded up to align
+int cb_moe_sort(const int64_t* topk_idx, int64_t n, int E, int align, int bound, int* counts, int* slot, int* src,
+                int64_t* padded_counts, cudaStream_t st) {
+  if (E <= 0 || E > 8192) return (int)cudaErrorInvalidValue;
+  cudaError_t err = cudaMemsetAsync(counts, 0, (size_t)E * sizeof(int), st);
+  if (err != cudaSuccess) return (int)err;
+  const int64_t blocks = (n + 1023) / 1024;
+  if (n > 0)
+    moe_count_kernel<<<(unsigned)(blocks < cb_num_sms() ? blocks : cb_num_sms()), 256, E * sizeof(int), st>>>(topk_idx, n, E, counts);
+  moe_place_kernel<<<E + 1, SORT_THREADS, 0, st>>>(topk_idx, n, E, align, bound, counts, slot, src, padded_counts);
+  return CB_LAUNCH_CHECK();
+}
+
+// rows of row_bytes (a multiple of 16) bytes, 16-byte aligned
+int cb_moe_take_rows(const void* x, const int* src, void* rows, int bound, int k, int row_bytes, cudaStream_t st) {
+  if (bound == 0) return 0;
+  moe_take_rows_kernel<<<(bound + 7) / 8, 256, 0, st>>>((const uint4*)x, src, (uint4*)rows, bound, k, row_bytes / 16);
+  return CB_LAUNCH_CHECK();
+}
+
+int cb_moe_sum_rows(const void* rows, const int* slot, const float* w, void* out, int tokens, int k, int H, int dtype,
+                    cudaStream_t st) {
+  if (tokens == 0) return 0;
+  CB_DISPATCH_FLOAT(dtype, T, {
+    const int vecs = H / Vec16<T>::N;
+    const int block = vecs >= 256 ? 256 : (vecs + 31) / 32 * 32;
+    moe_sum_rows_kernel<T><<<tokens, block, 0, st>>>((const T*)rows, slot, w, (T*)out, k, H);
+  });
+  return CB_LAUNCH_CHECK();
+}
+
+int cb_moe_sum_rows_bwd(const void* g, const void* rows, const int* src, const float* w, void* drows, float* dw, int bound,
+                        int k, int H, int dtype, cudaStream_t st) {
+  if (bound == 0) return 0;
+  CB_DISPATCH_FLOAT(dtype, T, {
+    moe_sum_rows_bwd_kernel<T><<<(bound + 7) / 8, 256, 0, st>>>((const T*)g, (const T*)rows, src, w, (T*)drows, dw, bound, k, H);
+  });
+  return CB_LAUNCH_CHECK();
+}
 
 // ---- legacy
 int cb_moe_dispatch_fwd(const void* tokens, void* expert_in, const int* mask, const int* dest_idx, int s, int e, int c,

@@ -13,8 +13,11 @@ from typing import Optional
 import torch
 import torch.distributed as dist
 
+from ..ops._dispatch import use_native
+from ..ops.moe import CombineRows, TakeRows, rows_ok, sort_choices
 from ..parallel import comm
 from ._operation import AllToAllUneven
+from .grouped_gemm import ALIGN
 
 __all__ = ["moe_forward", "set_moe_backend", "get_moe_backend"]
 
@@ -92,6 +95,16 @@ def moe_forward(x: torch.Tensor, topk_w: torch.Tensor, topk_idx: torch.Tensor, e
     T, H = x.shape
     k = topk_idx.shape[1]
     ep = comm.group_size(ep_group) if ep_group is not None else 1     # None = no expert parallelism (NOT the world)
+    if ep == 1 and T > 0 and use_native(x) and _aligned_rows(x) and rows_ok(x):
+        # all experts here: the rows are sorted, gathered, combined and differentiated by kernels of their own, without a
+        # host synchronisation (`ops/moe.py`); the index operations below remain for CPU tensors and 32-bit rows
+        slot, src, counts = sort_choices(topk_idx, num_experts, ALIGN)
+        counts.cb200_aligned = True
+        ys = experts(TakeRows.apply(x, slot, src, k), counts)
+        if rows_ok(ys):
+            return CombineRows.apply(ys, topk_w, slot, src)
+        picked = ys.index_select(0, slot.long()).view(T, k, -1)        # experts of another width or type
+        return (picked * topk_w.unsqueeze(-1).to(ys.dtype)).sum(1)
     n_local = num_experts // ep
     flat_idx = topk_idx.reshape(-1)                                    # [T*k]
     order = torch.argsort(flat_idx, stable=True)                       # rows grouped by global expert id

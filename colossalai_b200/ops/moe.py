@@ -214,3 +214,83 @@ def gather_combine(rows: torch.Tensor, row_of: torch.Tensor, weights: torch.Tens
         g = 1.0 if extra_gate is None else torch.sigmoid(extra_gate.float().reshape(T, 1))
         out = out + g * extra.float()
     return out
+
+
+# ------------------------------------------------------------------------------------------------ local experts
+def sort_choices(topk_idx: torch.Tensor, num_experts: int, align: int):
+    """topk_idx [T, k] on the GPU -> (slot int32 [T * k], src int32 [bound], counts int64 [E]): choice i's row sits at
+    slot[i] of a buffer grouped by expert in which every expert's rows, in the order of their choices, are padded to a
+    multiple of `align`; src[r] is the choice of row r (-1: padding); counts are the padded ones.  A choice outside
+    [0, E) gets slot -1.  No host synchronisation."""
+    idx = topk_idx.reshape(-1).to(torch.int64).contiguous()
+    n, dev = idx.numel(), idx.device
+    bound = (n + num_experts * (align - 1) + align - 1) // align * align
+    work = torch.empty(num_experts + n + bound, dtype=torch.int32, device=dev)
+    counts, slot, src = work[:num_experts], work[num_experts: num_experts + n], work[num_experts + n:]
+    padded = torch.empty(num_experts, dtype=torch.int64, device=dev)
+    loader.check(_get_lib().cb_moe_sort(loader.ptr(idx), ctypes.c_int64(n), num_experts, align, bound, loader.ptr(counts),
+                                        loader.ptr(slot), loader.ptr(src), loader.ptr(padded), loader.stream_ptr()), "moe_sort")
+    loader.launch_counter.add("moe_sort", 2)
+    return slot, src, padded
+
+
+def rows_ok(x: torch.Tensor) -> bool:
+    """Rows that the local-expert kernels move in 16-byte vectors."""
+    return x.is_cuda and x.dim() == 2 and x.dtype in (torch.float32, torch.float16, torch.bfloat16) \
+        and x.shape[1] * x.element_size() % 16 == 0
+
+
+def _aligned(x: torch.Tensor) -> torch.Tensor:
+    x = x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
+def _sum_rows(rows: torch.Tensor, slot: torch.Tensor, w: Optional[torch.Tensor], tokens: int, k: int) -> torch.Tensor:
+    out = torch.empty(tokens, rows.shape[1], dtype=rows.dtype, device=rows.device)
+    loader.check(_get_lib().cb_moe_sum_rows(loader.ptr(rows), loader.ptr(slot), loader.ptr(w), loader.ptr(out), tokens, k,
+                                            rows.shape[1], code(rows.dtype), loader.stream_ptr()), "moe_sum_rows")
+    loader.launch_counter.add("moe_sum_rows")
+    return out
+
+
+class TakeRows(torch.autograd.Function):
+    """x [T, H] -> rows [bound, H] grouped by expert (padding rows zero); the gradient sums a token's rows in fp32."""
+
+    @staticmethod
+    def forward(ctx, x, slot, src, k):
+        x = _aligned(x)
+        rows = torch.empty(src.numel(), x.shape[1], dtype=x.dtype, device=x.device)
+        loader.check(_get_lib().cb_moe_take_rows(loader.ptr(x), loader.ptr(src), loader.ptr(rows), src.numel(), k,
+                                                 x.shape[1] * x.element_size(), loader.stream_ptr()), "moe_take_rows")
+        loader.launch_counter.add("moe_take_rows")
+        ctx.save_for_backward(slot)
+        ctx.shape = (x.shape[0], k)
+        return rows
+
+    @staticmethod
+    def backward(ctx, drows):
+        slot, = ctx.saved_tensors
+        return _sum_rows(_aligned(drows), slot, None, *ctx.shape), None, None, None
+
+
+class CombineRows(torch.autograd.Function):
+    """rows [bound, H] grouped by expert, weights [T, k] -> out [T, H] = sum_j weights[t, j] rows[slot[t, j]], in fp32 with
+    one rounding."""
+
+    @staticmethod
+    def forward(ctx, rows, weights, slot, src):
+        rows, w = _aligned(rows), weights.float().contiguous()
+        ctx.save_for_backward(rows, w, slot, src)
+        ctx.w_dtype = weights.dtype
+        return _sum_rows(rows, slot, w, *weights.shape)
+
+    @staticmethod
+    def backward(ctx, dout):
+        rows, w, slot, src = ctx.saved_tensors
+        g = _aligned(dout)
+        drows, dw = torch.empty_like(rows), torch.zeros_like(w)
+        loader.check(_get_lib().cb_moe_sum_rows_bwd(loader.ptr(g), loader.ptr(rows), loader.ptr(src), loader.ptr(w),
+                                                    loader.ptr(drows), loader.ptr(dw), src.numel(), w.shape[1], rows.shape[1],
+                                                    code(rows.dtype), loader.stream_ptr()), "moe_sum_rows_bwd")
+        loader.launch_counter.add("moe_sum_rows_bwd")
+        return drows, dw.to(ctx.w_dtype), None, None

@@ -244,3 +244,47 @@ if __name__ == "__main__":
     import os
 
     spawn(_fused_ep_worker, int(os.environ.get("NGPU", "2")))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,k,E,H", [(1, 1, 1, 8), (3, 2, 5, 24), (129, 8, 64, 264), (700, 3, 300, 2056), (4097, 2, 3, 64)])
+def test_local_expert_rows(T, k, E, H, dtype):
+    """Sort, gather, combine and their gradients at the edges: one token, experts without tokens, more choices than one
+    round of the sort covers, rows that are no multiple of a warp's or a block's vectors."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, H, device="cuda", generator=g).to(dtype).requires_grad_()
+    idx = torch.stack([torch.randperm(E, device="cuda", generator=g)[:k] for _ in range(T)])
+    idx[idx == 0] = E - 1                                                   # nobody asks for expert 0 (unless E = 1)
+    w = torch.rand(T, k, device="cuda", generator=g).requires_grad_()
+    slot, src, counts = mops.sort_choices(idx, E, 128)
+    flat = idx.reshape(-1)
+    real = torch.bincount(flat, minlength=E)
+    assert torch.equal(counts, (real + 127) // 128 * 128)
+    starts = torch.cumsum(counts, 0) - counts
+    order = torch.argsort(flat, stable=True)
+    want = torch.empty_like(flat)
+    want[order] = torch.arange(T * k, device="cuda") - (torch.cumsum(real, 0) - real)[flat[order]] + starts[flat[order]]
+    assert torch.equal(slot.long(), want)
+    back = torch.full((src.numel(),), -1, device="cuda")
+    back[want] = torch.arange(T * k, device="cuda")
+    assert torch.equal(src.long(), back)
+    rows = mops.TakeRows.apply(x, slot, src, k)
+    assert torch.equal(rows[want], x.detach()[torch.arange(T * k, device="cuda") // k]) and not rows[back < 0].any()
+    scale = torch.rand(src.numel(), 1, device="cuda", generator=g).to(dtype)
+    mid = rows * scale                                                      # each row an "expert" of its own
+    out = mops.CombineRows.apply(mid, w, slot, src)
+    dout = torch.randn(T, H, device="cuda", generator=g).to(dtype)
+    dx, dw = torch.autograd.grad(out, (x, w), dout)
+    m64 = mid.detach().double()[want].view(T, k, H)
+    ref = (m64 * w.detach().double()[..., None]).sum(1)
+    eps = torch.finfo(dtype).eps
+    # one rounding of an fp32 sum: half a step of the result (below the smallest normal number the steps stay eps times
+    # that number wide), plus fp32 rounding of the terms
+    sub = 0.5 * eps * torch.finfo(dtype).smallest_normal
+    assert (out.double() - ref).abs().le(0.51 * eps * ref.abs() + sub + 1e-6 * m64.abs().sum(1)).all()
+    dref = (m64 * dout.double()[:, None]).sum(-1)
+    assert (dw.double() - dref).abs().le(1e-5 * (m64 * dout.double()[:, None]).abs().sum(-1) + 1e-7).all()
+    # w g rounded, times scale rounded, summed and rounded: three half steps of each term's size
+    terms = w.detach().double()[..., None] * dout.double()[:, None] * scale.double()[want].view(T, k, 1)
+    assert (dx.double() - terms.sum(1)).abs().le(1.6 * eps * terms.abs().sum(1) + 1e-6).all()
