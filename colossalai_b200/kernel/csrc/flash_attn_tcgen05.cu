@@ -2,19 +2,25 @@
 //
 //   O = softmax(scale * Q K^T + causal mask) V,   LSE = log sum exp     (GQA: Hq = g * Hkv, head_dim 64 or 128)
 //
-// One CTA = one 128-row query tile of one (batch, head).  Six warps:
-//   warp 0      TMA producer: Q once, then (K_j, V_j) tiles of 128 keys through a 2-stage ring (SWIZZLE_128B boxes)
-//   warp 1      MMA issuer (one elected thread): S_j = Q K_j^T and O_j = P_j V_j with tcgen05.mma, accumulators in TMEM
-//   warps 2..5  softmax: thread r owns query row r — tcgen05.ld of its S row, running max / sum in the exp2 domain,
-//               P_j written as bf16 into shared memory in the K-major 128B-swizzled layout the tensor core reads,
-//               O_j pulled back from TMEM and folded into the register accumulator with the rescale factor
-// S is double-buffered in TMEM so Q K_{j+1}^T runs on the tensor pipe while the softmax warps work on tile j.
-// TMEM map (512 columns allocated): [0,128) S buffer 0, [128,256) S buffer 1, [256,256+D) O_j.
-// Shared memory: Q 128 x D, 2 x (K 128 x D + V 128 x D), P 128 x 128 (all bf16/fp16) + mbarriers = 193 KB at D = 128.
-//
-// STATUS: written against the validated primitives of sm100.cuh / gemm_tcgen05.cu (descriptors, TMA boxes, TMEM
-// loads) but NOT yet executed on hardware — `ops/flash_attn_native.py` keeps it behind CB200_FLASH_NATIVE=1 and the
-// numerics test (tests/test_kernels/test_flash_attn_native.py) must pass on a B200 before it becomes a default.
+// Persistent CTAs, one per SM, walk a list of work units, the longest first.  A unit = TWO 128-row query tiles over the same
+// key tiles: two query heads of one kv head where the group is even (the same keys are visible to both), else two
+// neighbouring query tiles of one head.  Twelve warps:
+//   warp 0       TMA producer: both Q tiles of a unit, then K_0, V_0, K_1, V_1, ... (128 keys each) through one ring
+//   warp 1       MMA issuer (one elected thread): S_t = Q_t K_j^T and O_t += P_t V_j with tcgen05.mma, accumulators in TMEM
+//   warp 3       finds the units of a packed batch from its device-resident boundaries, two units ahead
+//   warps 4..7   softmax of tile 0, warps 8..11 of tile 1: thread r owns query row r - tcgen05.ld of its S row, running max /
+//                sum in the exp2 domain, P_t written back to TMEM as the 16-bit A operand of the second product
+// Bound: the softmax - 128 exponentials per row and key tile at 16 a clock and SM take as long as the products of D = 128.
+// Two tiles, so that one tile's softmax runs under the other's products (one tile per CTA and the mask as predicated code:
+// 4096 tokens, 32 / 8 heads of 128, causal 239 us = 575 TFLOP/s; now 160 us = 859).  P through TMEM, because a product with
+// both operands in shared memory reads 8 KB per 64-clock MMA, all that shared memory delivers.  Persistent, because a unit
+// of a short sequence walks a handful of key tiles and a CTA of its own spent a third of its life on launch, allocation and
+// its first loads (16 x 1024 tokens, heads of 64: one tile per CTA 290 us, two 198 us, persistent 178 us; packed uneven
+// prompts of that size 360 -> 216 us).  Two threads per row (16 softmax warps) were 5 - 10 % slower than one.
+// TMEM map (512 columns), D = 128: [0,128) S_0, [128,256) S_1, then O_0, O_1; P_t overwrites the first half of S_t once its
+// rows are in registers, so S_t of the next key tile is issued behind the P V that reads P_t.  D = 64: O_t are 64 wide
+// and P_t have columns of their own, [384,448) and [448,512): the next S_t is issued as soon as this one has been read.
+// Shared memory at D = 128: 2 x Q 32 KB + 5 ring slots of 32 KB (at D = 64 2 x 16 KB + 8 x 16 KB) + mbarriers.
 //
 // Reference being replaced: flash-attn 2 `flash_attn_func` / `_flash_attn_varlen_forward` (mma.sync kernels) used by
 // `colossalai/shardformer/layer/attn.py:356-372,720-755`.
@@ -22,6 +28,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "sm100.cuh"
@@ -32,18 +40,36 @@ using namespace sm100;
 constexpr int BLOCK_Q = 128;
 constexpr int BLOCK_KV = 128;
 constexpr int UMMA_K = 16;
-constexpr int NUM_THREADS = 192;
-constexpr int KV_STAGES = 2;
+constexpr int SOFTMAX_WARP0 = 4;
+constexpr int NUM_THREADS = (SOFTMAX_WARP0 + 8) * 32;
+constexpr int UNIT_RING = 2;
+
+// Waits give up after a bounded number of polls (each of which the hardware may suspend), far beyond any wait of a kernel
+// that works; the CTA then drains its copies, frees its tensor memory and leaves, and the flag below is raised.
+constexpr int WAIT_LIMIT = 1 << 22;
+__device__ int g_flash_error;
+
+SM100_DEVICE bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try_wait(bar, parity)) return true;
+  for (int i = 0; i < WAIT_LIMIT; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 63) == 63 && *abort_flag) return false;
+  }
+  *abort_flag = 1;
+  g_flash_error = 1;
+  return false;
+}
 
 template <int D> struct FaCfg {
+  static constexpr bool SPLIT_P = D == 64;                 // P has tensor memory of its own
   static constexpr int Q_BYTES = BLOCK_Q * D * 2;
-  static constexpr int K_BYTES = BLOCK_KV * D * 2;
-  static constexpr int V_BYTES = BLOCK_KV * D * 2;
-  static constexpr int P_BYTES = BLOCK_Q * BLOCK_KV * 2;
-  static constexpr int KV_STAGE_BYTES = K_BYTES + V_BYTES;
-  static constexpr int SMEM_BYTES = Q_BYTES + KV_STAGES * KV_STAGE_BYTES + 2 * P_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int SLOT_BYTES = BLOCK_KV * D * 2;      // one K or V tile
+  static constexpr int SLOTS = D == 128 ? 5 : 8;
+  static constexpr int BAR_BYTES = 512;
+  static constexpr int SMEM_BYTES = 2 * Q_BYTES + SLOTS * SLOT_BYTES + 1024 /*align*/ + BAR_BYTES;
   static constexpr int TMEM_COLS = 512;
   static constexpr int O_COL = 256;
+  static constexpr int P_COL = SPLIT_P ? 384 : 0, P_STEP = SPLIT_P ? 64 : 128;
 };
 
 struct FaParams {
@@ -53,6 +79,9 @@ struct FaParams {
   int batch, seqlen_q, seqlen_k;     // equal-length sequences, token-major tensors [batch * seqlen, heads * D]
   int hq, hkv;
   int causal;
+  int pair_heads;                    // a unit's tiles: 1 = one query tile of two heads, 0 = two query tiles of one head
+  int head_units;                    // hq / 2 or hq
+  int seq_units;                     // equal lengths: units of one sequence and head
   float scale_log2;                  // softmax scale * log2(e)
   void* out;                         // [batch * seqlen_q, hq * D]
   float* lse;                        // [batch * seqlen_q, hq] natural-log LSE
@@ -73,62 +102,98 @@ SM100_DEVICE float fast_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// two fp32 operations in one instruction
+SM100_DEVICE uint64_t pack_f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+SM100_DEVICE void unpack_f32x2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+SM100_DEVICE uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+SM100_DEVICE uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+template <bool BF16> SM100_DEVICE uint32_t pack_16(float a, float b) {
+  if (BF16) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+  }
+  __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
 
-template <int D, bool EXTRA>
+// Packed batches: units of `per` rows in descending order of their index inside the sequence (the unit with index i walks the
+// key tiles of i + 1 units), over all sequences: count(i) = units with an index >= i.  One warp, every lane gets the result.
+SM100_DEVICE int packed_count(const int* cu, int batch, int per, int i) {
+  const int lane = threadIdx.x & 31;
+  int c = 0;
+  for (int b = lane; b < batch; b += 32) c += max(0, (__ldg(cu + b + 1) - __ldg(cu + b) + per - 1) / per - i);
+  return __reduce_add_sync(0xffffffffu, c);
+}
+SM100_DEVICE void packed_unit(const int* cu, int batch, int per, int r, int& unit, int& start, int& len) {
+  const int lane = threadIdx.x & 31;
+  int longest = 0;
+  for (int b = lane; b < batch; b += 32) longest = max(longest, (__ldg(cu + b + 1) - __ldg(cu + b) + per - 1) / per);
+  int lo = 0, hi = __reduce_max_sync(0xffffffffu, longest);       // largest index lo with count(lo) > r
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (packed_count(cu, batch, per, mid) > r) lo = mid; else hi = mid;
+  }
+  int nth = r - packed_count(cu, batch, per, lo + 1);             // the nth sequence that has a unit `lo`
+  unit = lo; start = 0; len = 0;
+  for (int b0 = 0; b0 < batch; b0 += 32) {
+    const int b = b0 + lane;
+    const int s0 = b < batch ? __ldg(cu + b) : 0, n = b < batch ? __ldg(cu + b + 1) - s0 : 0;
+    const unsigned m = __ballot_sync(0xffffffffu, (n + per - 1) / per > lo);
+    if (nth < __popc(m)) {
+      const int pick = (int)__fns(m, 0, nth + 1);
+      start = __shfl_sync(0xffffffffu, s0, pick);
+      len = __shfl_sync(0xffffffffu, n, pick);
+      return;
+    }
+    nth -= __popc(m);
+  }
+}
+
+struct FaUnit {
+  int live, index, q_start, k_start, len_q, len_k, head0;
+};
+
+template <int D, bool EXTRA, bool BF16>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const FaParams p) {
   using C = FaCfg<D>;
+  constexpr int SLOTS = C::SLOTS;
+  constexpr bool SPLIT_P = C::SPLIT_P;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_q = smem;
-  uint8_t* smem_kv = smem + C::Q_BYTES;
-  uint8_t* smem_p = smem_kv + KV_STAGES * C::KV_STAGE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_p + 2 * C::P_BYTES);
+  uint8_t* smem_q = smem;                                    // two tiles
+  uint8_t* smem_kv = smem + 2 * C::Q_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_kv + SLOTS * C::SLOT_BYTES);
   uint64_t* q_full = bars;                 // [1]
-  uint64_t* kv_full = bars + 1;            // [2]
-  uint64_t* kv_empty = bars + 3;           // [2]
-  uint64_t* s_full = bars + 5;             // [2]
-  uint64_t* s_empty = bars + 7;            // [2]  4 softmax warps
-  uint64_t* p_full = bars + 9;             // [1]  4 softmax warps
-  uint64_t* o_full = bars + 10;            // [1]
-  uint64_t* o_empty = bars + 11;           // [1]  4 softmax warps
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 12);
+  uint64_t* q_empty = bars + 1;            // [1]  the unit's last Q K^T retired
+  uint64_t* full = bars + 2;               // [SLOTS]
+  uint64_t* empty = full + SLOTS;          // [SLOTS]
+  uint64_t* s_full = empty + SLOTS;        // [2]  S_t is in tensor memory
+  uint64_t* s_empty = s_full + 2;          // [2]  4 softmax warps have read it (SPLIT_P)
+  uint64_t* p_full = s_empty + 2;          // [2]  4 softmax warps have written P_t
+  uint64_t* o_full = p_full + 2;           // [2]  P_t V_j retired: every j (SPLIT_P), else a unit's last one
+  uint64_t* o_empty = o_full + 2;          // [2]  4 softmax warps have read O_t
+  uint64_t* u_full = o_empty + 2;          // [UNIT_RING]
+  uint64_t* u_empty = u_full + UNIT_RING;  // [UNIT_RING]  10 warps have read the unit
+  FaUnit* units = reinterpret_cast<FaUnit*>(u_empty + UNIT_RING);
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(units + UNIT_RING);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int head = blockIdx.y;
-  const int kv_head = head / (p.hq / p.hkv);
-  int q_tile, seq_row0, len_q, len_k;
-  if (p.cu_seqlens != nullptr) {
-    // packed batch: blockIdx.x enumerates (sequence, query tile) pairs in order; surplus CTAs (the grid is sized for
-    // the worst case without knowing the lengths on the host) leave at once
-    int t = (int)blockIdx.x, bsel = -1, start = 0, len = 0;
-    for (int bb = 0; bb < p.batch; ++bb) {
-      start = p.cu_seqlens[bb];
-      len = p.cu_seqlens[bb + 1] - start;
-      const int nt = (len + BLOCK_Q - 1) / BLOCK_Q;
-      if (t < nt) { bsel = bb; break; }
-      t -= nt;
-    }
-    if (bsel < 0) return;                      // uniform across the CTA: nothing has been allocated yet
-    q_tile = t; seq_row0 = start; len_q = len; len_k = len;
-  } else {
-    // heaviest (longest causal) query tiles first
-    const int q_tiles = (p.seqlen_q + BLOCK_Q - 1) / BLOCK_Q;
-    q_tile = p.causal ? (q_tiles - 1 - (int)blockIdx.x) : (int)blockIdx.x;
-    seq_row0 = -1; len_q = p.seqlen_q; len_k = p.seqlen_k;
-  }
-  const int b = blockIdx.z;
-  const int q_row0 = (seq_row0 >= 0 ? seq_row0 : b * p.seqlen_q) + q_tile * BLOCK_Q;   // row in the token-major Q / O
-  const int kv_row0 = seq_row0 >= 0 ? seq_row0 : b * p.seqlen_k;
-  const int kv_tiles_all = (len_k + BLOCK_KV - 1) / BLOCK_KV;
-  // causal with seqlen_q == seqlen_k: key tiles 0..q_tile; otherwise all of them
-  const int kv_last = p.causal ? min(q_tile + 1, kv_tiles_all) : kv_tiles_all;   // one past the last visible key tile
-  // sliding window: the lowest key any row of this query tile can see is (q_tile * BLOCK_Q - window + 1)
-  const int kv_first = (EXTRA && p.window > 0) ? max(0, q_tile * BLOCK_Q - p.window + 1) / BLOCK_KV : 0;
-  const int kv_tiles = kv_last - kv_first;         // tiles walked; loop index j <-> key tile kv_first + j
-  const bool ragged_k = (len_k % BLOCK_KV) != 0;   // the last key tile runs past the end of the sequence
   const bool resume = p.o_state != nullptr && p.has_prev != 0;   // block mode: continue from the stored state
 
   if (warp == 0 && lane == 0) {
@@ -138,15 +203,23 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   }
   if (warp == 1 && lane == 0) {
     mbar_init(q_full, 1);
+    mbar_init(q_empty, 1);
+    for (int i = 0; i < SLOTS; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
       mbar_init(&s_full[i], 1);
       mbar_init(&s_empty[i], 4);
+      mbar_init(&p_full[i], 4);
+      mbar_init(&o_full[i], 1);
+      mbar_init(&o_empty[i], 4);
     }
-    mbar_init(p_full, 4);
-    mbar_init(o_full, 1);
-    mbar_init(o_empty, 4);
+    for (int i = 0; i < UNIT_RING; ++i) {
+      mbar_init(&u_full[i], 1);
+      mbar_init(&u_empty[i], 10);
+    }
+    *abort_flag = 0;
     fence_barrier_init();
   }
   if (warp == 2) tmem_alloc<C::TMEM_COLS>(tmem_ptr_smem);
@@ -155,274 +228,410 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  if (warp == 0) {
-    // ================================================================ TMA producer
-    if (lane == 0) {
-      mbar_arrive_expect_tx(q_full, C::Q_BYTES);
-#pragma unroll
-      for (int h = 0; h < D / 64; ++h)                     // boxes [128 rows, 64 d] -> K-major swizzled sub-tiles
-        tma_load_2d(&tmap_q, q_full, smem_q + h * (BLOCK_Q * 128), head * D + h * 64, q_row0);
-    }
-    int stage = 0;
-    uint32_t phase = 0;
-    for (int j = 0; j < kv_tiles; ++j) {
-      mbar_wait(&kv_empty[stage], phase ^ 1);
-      if (lane == 0) {
-        uint8_t* sk = smem_kv + stage * C::KV_STAGE_BYTES;
-        uint8_t* sv = sk + C::K_BYTES;
-        mbar_arrive_expect_tx(&kv_full[stage], C::KV_STAGE_BYTES);
-        const int row = kv_row0 + (kv_first + j) * BLOCK_KV;
-#pragma unroll
-        for (int h = 0; h < D / 64; ++h) {
-          tma_load_2d(&tmap_k, &kv_full[stage], sk + h * (BLOCK_KV * 128), kv_head * D + h * 64, row);   // K-major B
-          tma_load_2d(&tmap_v, &kv_full[stage], sv + h * (BLOCK_KV * 128), kv_head * D + h * 64, row);   // MN-major B
+  // ---- a unit as every role sees it
+  FaUnit un;
+  int ui = 0;                               // units taken so far
+  auto next_unit = [&]() -> bool {          // whole warps
+    const int e = ui % UNIT_RING;
+    if (!__all_sync(0xffffffffu, wait_or_abort(&u_full[e], (uint32_t)((ui / UNIT_RING) & 1), abort_flag))) return false;
+    un = units[e];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&u_empty[e]);
+    ++ui;
+    return un.live != 0;
+  };
+  auto tile_of = [&](int t) { return p.pair_heads ? un.index : 2 * un.index + t; };
+  auto head_of = [&](int t) { return p.pair_heads ? un.head0 + t : un.head0; };
+  // causal with seqlen_q == seqlen_k: key tiles 0..q_tile; otherwise all of them.  Sliding window: the lowest key any row of
+  // the first tile can see is (tile_of(0) * BLOCK_Q - window + 1)
+  auto first_key_tile = [&]() { return (EXTRA && p.window > 0) ? max(0, tile_of(0) * BLOCK_Q - p.window + 1) / BLOCK_KV : 0; };
+  auto steps_of = [&](int t) {              // key tiles that tile t walks (0: the tile lies behind the sequence's end)
+    if (tile_of(t) * BLOCK_Q >= un.len_q) return 0;
+    const int all = (un.len_k + BLOCK_KV - 1) / BLOCK_KV;
+    return (p.causal ? min(tile_of(t) + 1, all) : all) - first_key_tile();
+  };
+
+  if (warp == 3) {
+    // ================================================================ unit list
+    const int per = p.pair_heads ? BLOCK_Q : 2 * BLOCK_Q;      // query rows of a unit
+    const int ranks = p.cu_seqlens != nullptr ? packed_count(p.cu_seqlens, p.batch, per, 0) : p.seq_units * p.batch;
+    const int total = ranks * p.head_units;
+    bool ok = true;
+    for (int i = 0; ok; ++i) {
+      // CTA c takes the list's entries c, 2 G - 1 - c, 2 G + c, ...: the longest first, and no CTA always the longer of a round
+      const int u = i * (int)gridDim.x + ((i & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
+      FaUnit x;
+      x.live = i * (int)gridDim.x < total;
+      x.index = 0; x.q_start = x.k_start = x.len_q = x.len_k = x.head0 = 0;      // (a unit without rows: not this CTA's turn)
+      if (u < total) {
+        const int rank = u / p.head_units;
+        x.head0 = (u - rank * p.head_units) * (p.pair_heads ? 2 : 1);
+        if (p.cu_seqlens != nullptr) {
+          packed_unit(p.cu_seqlens, p.batch, per, rank, x.index, x.q_start, x.len_q);
+          x.k_start = x.q_start; x.len_k = x.len_q;
+        } else {
+          const int b = rank % p.batch;
+          x.index = p.causal ? p.seq_units - 1 - rank / p.batch : rank / p.batch;
+          x.q_start = b * p.seqlen_q; x.k_start = b * p.seqlen_k; x.len_q = p.seqlen_q; x.len_k = p.seqlen_k;
         }
       }
+      const int e = i % UNIT_RING;
+      ok = __all_sync(0xffffffffu, wait_or_abort(&u_empty[e], (uint32_t)(((i / UNIT_RING) & 1) ^ 1), abort_flag));
+      if (lane == 0 && ok) {
+        units[e] = x;
+        mbar_arrive(&u_full[e]);
+      }
       __syncwarp();
-      if (++stage == KV_STAGES) { stage = 0; phase ^= 1; }
+      if (!x.live) break;
     }
+  } else if (warp == 0) {
+    // ================================================================ TMA producer
+    int issued = 0, nq = 0;
+    while (next_unit()) {
+      const int n0 = steps_of(0), n1 = steps_of(1), steps = max(n0, n1);
+      if (steps == 0) continue;
+      bool ok = true;
+      if (lane == 0) {
+        ok = wait_or_abort(q_empty, (uint32_t)((nq & 1) ^ 1), abort_flag);
+        if (ok) {
+          mbar_arrive_expect_tx(q_full, (n1 > 0 ? 2 : 1) * C::Q_BYTES);
+          for (int t = 0; t < (n1 > 0 ? 2 : 1); ++t)
+#pragma unroll
+            for (int h = 0; h < D / 64; ++h)                   // boxes [128 rows, 64 d] -> K-major swizzled sub-tiles
+              tma_load_2d(&tmap_q, q_full, smem_q + t * C::Q_BYTES + h * (BLOCK_Q * 128), head_of(t) * D + h * 64,
+                          un.q_start + tile_of(t) * BLOCK_Q);
+          ++nq;
+          const int kv_head = un.head0 / (p.hq / p.hkv), k_tile0 = first_key_tile();
+          for (int i = 0; i < 2 * steps && ok; ++i) {          // K_j (K-major B of Q K^T), V_j (MN-major B of P V)
+            const int slot = issued % SLOTS;
+            ok = wait_or_abort(&empty[slot], (uint32_t)(((issued / SLOTS) & 1) ^ 1), abort_flag);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&full[slot], C::SLOT_BYTES);
+            const int row = un.k_start + (k_tile0 + (i >> 1)) * BLOCK_KV;
+#pragma unroll
+            for (int h = 0; h < D / 64; ++h)
+              tma_load_2d((i & 1) ? &tmap_v : &tmap_k, &full[slot], smem_kv + slot * C::SLOT_BYTES + h * (BLOCK_KV * 128),
+                          kv_head * D + h * 64, row);
+            ++issued;
+          }
+        }
+      }
+      if (!__all_sync(0xffffffffu, ok)) break;
+    }
+    if (lane == 0 && *abort_flag) {                            // leave no copy in flight behind
+      int none = 0;
+      if (nq > 0) wait_or_abort(q_full, (uint32_t)((nq - 1) & 1), &none);
+      for (int i = max(0, issued - SLOTS); i < issued; ++i) {
+        none = 0;
+        wait_or_abort(&full[i % SLOTS], (uint32_t)((i / SLOTS) & 1), &none);
+      }
+    }
+    __syncwarp();
   } else if (warp == 1) {
     // ================================================================ MMA issuer
-    const uint32_t sq = smem_u32(smem_q);
-    const uint32_t sp = smem_u32(smem_p);
-    const uint64_t dq = make_smem_desc_sw128(sq, 16, 1024);                       // K-major, K = D
-    const uint64_t dp = make_smem_desc_sw128(sp, 16, 1024);                       // K-major, K = keys
-    auto issue_qk = [&](int j) {
-      const int stage = j % KV_STAGES;
-      const int sb = j & 1;
-      mbar_wait(&kv_full[stage], (uint32_t)((j / KV_STAGES) & 1));
-      mbar_wait(&s_empty[sb], (uint32_t)(((j >> 1) & 1) ^ 1));
-      tc_fence_after();
+    const uint64_t dq = make_smem_desc_sw128(smem_u32(smem_q), 16, 1024);                 // K-major, K = D
+    const uint64_t dk0 = make_smem_desc_sw128(smem_u32(smem_kv), 16, 1024);               // K-major
+    const uint64_t dv0 = make_smem_desc_sw128(smem_u32(smem_kv), BLOCK_KV * 128, 1024);   // MN-major: [keys, D] row-major
+    int base = 0, nq = 0;                    // ring index of the unit's K_0; units with work so far
+    int done[2] = {0, 0}, uses[2] = {0, 0};  // per tile: key tiles of earlier units, units it had work in
+    while (next_unit()) {
+      const int n0 = steps_of(0), n1 = steps_of(1), steps = max(n0, n1);
+      if (steps == 0) continue;
+      bool ok = true;
       if (lane == 0) {
-        const uint32_t sk = smem_u32(smem_kv + stage * C::KV_STAGE_BYTES);
-        const uint64_t dk = make_smem_desc_sw128(sk, 16, 1024);
+        auto wait_slot = [&](int i) {
+          i += base;
+          return wait_or_abort(&full[i % SLOTS], (uint32_t)((i / SLOTS) & 1), abort_flag);
+        };
+        auto qk = [&](int t, int j) -> bool {
+          if (SPLIT_P && !wait_or_abort(&s_empty[t], (uint32_t)(((done[t] + j) & 1) ^ 1), abort_flag)) return false;
+          tc_fence_after();
+          const uint32_t ko = ((base + 2 * j) % SLOTS) * C::SLOT_BYTES;
 #pragma unroll
-        for (int k = 0; k < D / UMMA_K; ++k) {
-          const uint32_t off = (k >> 2) * (128 * 128) + (k & 3) * (UMMA_K * 2);
-          umma_f16_ss(tmem_base + sb * BLOCK_KV, advance_desc(dq, off), advance_desc(dk, off), p.idesc_qk,
-                      k > 0 ? 1u : 0u);
-        }
-        umma_commit(&s_full[sb]);
-      }
-      __syncwarp();
-    };
-    mbar_wait(q_full, 0);
-    tc_fence_after();
-    issue_qk(0);
-    for (int j = 0; j < kv_tiles; ++j) {
-      if (j + 1 < kv_tiles) issue_qk(j + 1);            // tensor pipe works on the next scores during softmax(j)
-      const int stage = j % KV_STAGES;
-      mbar_wait(p_full, (uint32_t)(j & 1));             // P_j is in shared memory (and O was rescaled if it had to be)
-      tc_fence_after();
-      if (lane == 0) {
-        const uint32_t sv = smem_u32(smem_kv + stage * C::KV_STAGE_BYTES + C::K_BYTES);
-        const uint64_t dv = make_smem_desc_sw128(sv, BLOCK_KV * 128, 1024);        // MN-major: [keys, D] row-major
-        const uint64_t dpj = advance_desc(dp, (uint32_t)(j & 1) * C::P_BYTES);
-        // O accumulates in TMEM over all key tiles (the first MMA of the first tile overwrites, unless the
-        // accumulator was pre-loaded with the state of earlier launches)
-        const bool fresh = (j == 0) && !resume;
+          for (int k = 0; k < D / UMMA_K; ++k) {
+            const uint32_t off = (k >> 2) * (128 * 128) + (k & 3) * (UMMA_K * 2);
+            umma_f16_ss(tmem_base + t * BLOCK_KV, advance_desc(dq, t * C::Q_BYTES + off), advance_desc(dk0, ko + off),
+                        p.idesc_qk, k > 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[t]);
+          return true;
+        };
+        auto pv = [&](int t, int j) -> bool {
+          if (!wait_or_abort(&p_full[t], (uint32_t)((done[t] + j) & 1), abort_flag)) return false;   // O_t rescaled if it had to be
+          // O accumulates in TMEM over all key tiles (the first MMA of a unit overwrites, unless the accumulator was
+          // pre-loaded with the state of earlier launches); P: 16 keys = 8 columns
+          const bool fresh = j == 0 && !resume;
+          if (fresh && !wait_or_abort(&o_empty[t], (uint32_t)((uses[t] & 1) ^ 1), abort_flag)) return false;
+          tc_fence_after();
+          const uint32_t vo = ((base + 2 * j + 1) % SLOTS) * C::SLOT_BYTES;
 #pragma unroll
-        for (int k = 0; k < BLOCK_KV / UMMA_K; ++k) {
-          const uint32_t ao = (k >> 2) * (128 * 128) + (k & 3) * (UMMA_K * 2);
-          const uint32_t bo = k * (UMMA_K * 128);
-          umma_f16_ss(tmem_base + C::O_COL, advance_desc(dpj, ao), advance_desc(dv, bo), p.idesc_pv,
-                      (fresh && k == 0) ? 0u : 1u);
+          for (int k = 0; k < BLOCK_KV / UMMA_K; ++k)
+            umma_f16_ts(tmem_base + C::O_COL + t * D, tmem_base + C::P_COL + t * C::P_STEP + k * 8,
+                        advance_desc(dv0, vo + k * (UMMA_K * 128)), p.idesc_pv, (fresh && k == 0) ? 0u : 1u);
+          if (SPLIT_P || j == (t ? n1 : n0) - 1) umma_commit(&o_full[t]);
+          return true;
+        };
+        auto release = [&](int i) { umma_commit(&empty[(base + i) % SLOTS]); };
+        ok = wait_or_abort(q_full, (uint32_t)(nq & 1), abort_flag) && wait_slot(0);
+        if (n0 > 0) ok = ok && qk(0, 0);
+        if (n1 > 0) ok = ok && qk(1, 0);
+        if (ok) {
+          release(0);
+          if (steps == 1) umma_commit(q_empty);
         }
-        umma_commit(o_full);
-        umma_commit(&kv_empty[stage]);                  // K_j and V_j are consumed once P_j V_j has retired
+        for (int j = 0; j < steps && ok; ++j) {
+          const bool next = j + 1 < steps;
+          if (SPLIT_P) {
+            if (next) {                                        // both S of the next key tile, as soon as these were read
+              ok = wait_slot(2 * j + 2);
+              if (j + 1 < n0) ok = ok && qk(0, j + 1);
+              if (j + 1 < n1) ok = ok && qk(1, j + 1);
+              if (ok) release(2 * j + 2);
+              if (ok && j + 2 == steps) umma_commit(q_empty);  // the unit's last Q K^T has been issued
+            }
+            ok = ok && wait_slot(2 * j + 1);
+            if (j < n0) ok = ok && pv(0, j);
+            if (j < n1) ok = ok && pv(1, j);
+            if (ok) release(2 * j + 1);
+          } else {
+            // P_t lies in S_t: the next S_t follows the product that reads P_t (MMAs of one thread run in order)
+            ok = wait_slot(2 * j + 1);
+            if (j < n0) ok = ok && pv(0, j);
+            if (j + 1 < n0) ok = ok && wait_slot(2 * j + 2) && qk(0, j + 1);
+            if (j < n1) ok = ok && pv(1, j);
+            if (ok) release(2 * j + 1);
+            if (j + 1 < n1) ok = ok && wait_slot(2 * j + 2) && qk(1, j + 1);
+            if (next && ok) release(2 * j + 2);
+            if (ok && j + 2 == steps) umma_commit(q_empty);
+          }
+        }
+        base += 2 * steps;
+        ++nq;
+        done[0] += n0; done[1] += n1;
+        uses[0] += n0 > 0; uses[1] += n1 > 0;
       }
-      __syncwarp();
+      if (!__all_sync(0xffffffffu, ok)) break;
     }
-  } else {
-    // ================================================================ softmax + output (warps 2..5)
+    __syncwarp();
+  } else if (warp >= SOFTMAX_WARP0) {
+    // ================================================================ softmax + output
     // Thread = query row.  The output accumulator lives in TMEM for the whole walk (P_j V_j accumulates onto it in the
     // tensor core); the exponentials are taken against a LAGGING row max: the accumulator is only rescaled when the
     // true max has grown by more than 2^TAU since the last rescale (exact: numerator and denominator use the same
-    // reference, which is what the log-sum-exp is reported against).  Per key tile a thread therefore reads its 128
-    // scores ONCE (four tcgen05.ld in flight, one wait), releases the score buffer at once, and touches the
-    // accumulator only on the rare rescale.
+    // reference, which is what the log-sum-exp is reported against).
     constexpr float TAU = 8.f;
+    const int t = (warp - SOFTMAX_WARP0) >> 2;           // this warp's query tile
     const int quarter = warp & 3;                        // TMEM lane quarter this warp may access
     const int r = quarter * 32 + lane;                   // query row inside the tile
-    const int q_pos = q_tile * BLOCK_Q + r;              // position inside the sequence
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    const uint32_t o_addr = tmem_base + lane_addr + C::O_COL;
-    float m_run = -INFINITY;                             // reference max of the exponentials (exp2 domain)
-    float l_run = 0.f;
-    if (resume) {
-      // resume from the merged result of the key blocks processed by earlier launches (normalised output + LSE):
-      // every row stores its previous output (or zeros) into the TMEM accumulator, P_0 V_0 accumulates onto it
-      const size_t row_ = (size_t)q_row0 + r;
-      float lse_prev = -INFINITY;
-      if (q_pos < len_q) lse_prev = p.lse[row_ * p.hq + head];
-      const bool live = lse_prev > -INFINITY;
-      if (live) { m_run = lse_prev * 1.4426950408889634f; l_run = 1.f; }
-      const float4* src = reinterpret_cast<const float4*>(p.o_state + row_ * ((size_t)p.hq * D) + (size_t)head * D);
+    const uint32_t o_addr = tmem_base + lane_addr + C::O_COL + t * D;
+    const uint32_t s_addr = tmem_base + lane_addr + t * BLOCK_KV;
+    const uint32_t p_addr = tmem_base + lane_addr + C::P_COL + t * C::P_STEP;
+    int done = 0, uses = 0;                              // key tiles / units of this tile so far
+    bool ok = true;
+    while (ok && next_unit()) {
+      const int n_steps = steps_of(t);
+      if (n_steps == 0) continue;
+      const int q_tile = tile_of(t), head = head_of(t), len_q = un.len_q, len_k = un.len_k;
+      const int kv_first = first_key_tile();
+      const int q_pos = q_tile * BLOCK_Q + r;              // position inside the sequence
+      const size_t row = (size_t)un.q_start + q_pos;       // row in the token-major Q / O
+      const int last_tile = (len_k + BLOCK_KV - 1) / BLOCK_KV - 1;
+      const bool ragged_k = (len_k % BLOCK_KV) != 0;       // the last key tile runs past the end of the sequence
+      float m_run = -INFINITY;                             // reference max of the exponentials (exp2 domain)
+      float l_run = 0.f;
+      if (resume) {
+        // resume from the merged result of the key blocks processed by earlier launches (normalised output + LSE):
+        // every row stores its previous output (or zeros) into the TMEM accumulator, P_0 V_0 accumulates onto it
+        float lse_prev = -INFINITY;
+        if (q_pos < len_q) lse_prev = p.lse[row * p.hq + head];
+        const bool live = lse_prev > -INFINITY;
+        if (live) { m_run = lse_prev * 1.4426950408889634f; l_run = 1.f; }
+        const float4* src = reinterpret_cast<const float4*>(p.o_state + row * ((size_t)p.hq * D) + (size_t)head * D);
 #pragma unroll
-      for (int c = 0; c < D; c += 16) {
-        uint32_t w[16];
+        for (int c = 0; c < D; c += 16) {
+          uint32_t w[16];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 t4 = live ? src[(c >> 2) + i] : make_float4(0.f, 0.f, 0.f, 0.f);
-          w[4 * i] = __float_as_uint(t4.x); w[4 * i + 1] = __float_as_uint(t4.y);
-          w[4 * i + 2] = __float_as_uint(t4.z); w[4 * i + 3] = __float_as_uint(t4.w);
+          for (int i = 0; i < 4; ++i) {
+            const float4 t4 = live ? src[(c >> 2) + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            w[4 * i] = __float_as_uint(t4.x); w[4 * i + 1] = __float_as_uint(t4.y);
+            w[4 * i + 2] = __float_as_uint(t4.z); w[4 * i + 3] = __float_as_uint(t4.w);
+          }
+          tmem_st_32x32b_x16(o_addr + c, w);
         }
-        tmem_st_32x32b_x16(o_addr + c, w);
+        tmem_st_wait();
       }
-      tmem_st_wait();
-    }
-    const float slope2 = (EXTRA && p.alibi != nullptr) ? p.alibi[head] * 1.4426950408889634f : 0.f;
-    (void)slope2;
-    for (int j = 0; j < kv_tiles; ++j) {
-      const int sb = j & 1;
-      mbar_wait(&s_full[sb], (uint32_t)((j >> 1) & 1));
+      const float slope2 = (EXTRA && p.alibi != nullptr) ? p.alibi[head] * 1.4426950408889634f : 0.f;
+      (void)slope2;
+      // one key tile; two copies of the code, because a branch around the mask alone is turned into 128 predicated
+      // comparisons and selections that every tile executes
+      auto step = [&](int j, auto masked_tag) -> bool {
+        constexpr bool MASKED = decltype(masked_tag)::value;
+        const int kt = kv_first + j;                         // key tile of this step
+        // ---- the whole score row into registers
+        uint32_t v[BLOCK_KV];
+#pragma unroll
+        for (int c = 0; c < BLOCK_KV; c += 32) tmem_ld_32x32b_x32(s_addr + c, *reinterpret_cast<uint32_t(*)[32]>(&v[c]));
+        tmem_ld_wait();
+        if (SPLIT_P) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&s_empty[t]);           // S_t may be overwritten by Q K_{j+1}^T
+        }
+        // plain variant: the softmax scale (> 0) is folded into the exponent's FMA, the max is taken on the raw scores;
+        // EXTRA variant: scale and ALiBi bias are applied here and the exponent uses a unit multiplier
+        if (EXTRA || MASKED) {
+          const int k_base = kt * BLOCK_KV;
+          const int k_lim = (p.causal && kt == q_tile) ? min(q_pos, len_k - 1) : (len_k - 1);   // last visible key of this row
+          const int k_low = (EXTRA && p.window > 0) ? q_pos - p.window + 1 : 0;                  // first visible key
+#pragma unroll
+          for (int i = 0; i < BLOCK_KV; ++i) {
+            float sc = __uint_as_float(v[i]);
+            if (EXTRA) sc = fmaf(slope2, (float)(k_base + i - q_pos), sc * p.scale_log2);
+            if (MASKED && ((k_base + i) > k_lim || (EXTRA && (k_base + i) < k_low))) sc = -INFINITY;
+            v[i] = __float_as_uint(sc);
+          }
+        }
+        // (four independent partial maxima / sums: a single running value would be a 128-long dependent chain)
+        float mt[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int i = 0; i < BLOCK_KV; i += 8)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            mt[e] = fmaxf(fmaxf(mt[e], __uint_as_float(v[i + e])), __uint_as_float(v[i + e + 4]));
+        const float ex_mul = EXTRA ? 1.f : p.scale_log2;
+        const float m_tile = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3])) * ex_mul;
+        // ---- lagging max / rare rescale of the TMEM accumulator
+        const float m_new = fmaxf(m_run, m_tile);
+        bool waited = !SPLIT_P || j == 0;                      // P V of the last key tile is known to have retired
+        if (j == 0 && !resume) {
+          m_run = m_new;                                       // nothing accumulated yet
+        } else {
+          const bool need = (m_new - m_run) > TAU;             // (-inf) - (-inf) = NaN -> false
+          if (__any_sync(0xffffffffu, need)) {
+            if (!waited) {
+              if (!__all_sync(0xffffffffu, wait_or_abort(&o_full[t], (uint32_t)((done - 1) & 1), abort_flag))) return false;
+              waited = true;
+              tc_fence_after();
+            }
+            const float alpha = need ? fast_exp2(m_run - m_new) : 1.f;
+#pragma unroll 1
+            for (int c = 0; c < D; c += 16) {
+              uint32_t w[16];
+              tmem_ld_32x32b_x16(o_addr + c, w);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) * alpha);
+              tmem_st_32x32b_x16(o_addr + c, w);
+            }
+            tmem_st_wait();
+            l_run *= alpha;
+            if (need) m_run = m_new;
+          }
+        }
+        if (!waited) {                                          // P_{j-1} has been read: its columns are free
+          if (!__all_sync(0xffffffffu, wait_or_abort(&o_full[t], (uint32_t)((done - 1) & 1), abort_flag))) return false;
+          tc_fence_after();
+        }
+        const float m_use = (m_run == -INFINITY) ? 0.f : m_run;     // keeps the exponent finite on a fully masked row
+        // ---- p = exp2(s - m), row sum, 16-bit P to tensor memory
+        const uint64_t mul2 = pack_f32x2(ex_mul, ex_mul), sub2 = pack_f32x2(-m_use, -m_use);
+        uint64_t lt[2] = {0ull, 0ull};
+#pragma unroll
+        for (int c = 0; c < BLOCK_KV; c += 32) {
+          uint32_t packed[16];
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            float p0, p1;
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c + i]), __uint_as_float(v[c + i + 1])), mul2, sub2), p0, p1);
+            p0 = fast_exp2(p0);
+            p1 = fast_exp2(p1);
+            lt[(i >> 1) & 1] = add_f32x2(lt[(i >> 1) & 1], pack_f32x2(p0, p1));
+            packed[i >> 1] = pack_16<BF16>(p0, p1);
+          }
+          tmem_st_32x32b_x16(p_addr + (c >> 1), packed);
+        }
+        float l0, l1, l2, l3;
+        unpack_f32x2(lt[0], l0, l1);
+        unpack_f32x2(lt[1], l2, l3);
+        l_run += (l0 + l1) + (l2 + l3);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[t]);            // P_j is in tensor memory, the accumulator is consistent
+        return true;
+      };
+      for (int j = 0; j < n_steps && ok; ++j) {
+        ok = __all_sync(0xffffffffu, wait_or_abort(&s_full[t], (uint32_t)(done & 1), abort_flag));
+        if (!ok) break;
+        tc_fence_after();
+        const int kt = kv_first + j;
+        const bool masked = (p.causal && kt == q_tile) || (ragged_k && kt == last_tile) || (EXTRA && p.window > 0);
+        ok = masked ? step(j, std::true_type{}) : step(j, std::false_type{});
+        ++done;
+      }
+      if (!ok) break;
+      // ---- epilogue: the last P V has retired; normalise and store this thread's row
+      ok = __all_sync(0xffffffffu, wait_or_abort(&o_full[t], (uint32_t)((SPLIT_P ? done - 1 : uses) & 1), abort_flag));
+      if (!ok) break;
       tc_fence_after();
-      const uint32_t s_addr = tmem_base + lane_addr + sb * BLOCK_KV;
-      const int kt = kv_first + j;                                       // key tile of this step
-      const bool diag = p.causal && (kt == q_tile);
-      const bool tail_k = ragged_k && (kt == kv_tiles_all - 1);
-      const bool masked = diag || tail_k || (EXTRA && p.window > 0);
-      const int k_lim = diag ? min(q_pos, len_k - 1) : (len_k - 1);      // last visible key position of this row
-      const int k_low = (EXTRA && p.window > 0) ? q_pos - p.window + 1 : 0;   // first visible key position
-      const int k_base = kt * BLOCK_KV;
-      // ---- the whole score row into registers
-      uint32_t v[BLOCK_KV];
-#pragma unroll
-      for (int c = 0; c < BLOCK_KV; c += 32) tmem_ld_32x32b_x32(s_addr + c, *reinterpret_cast<uint32_t(*)[32]>(&v[c]));
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s_empty[sb]);          // S buffer may be overwritten by Q K_{j+2}^T
-      // plain variant: the softmax scale (> 0) is folded into the exponent's FMA, the max is taken on the raw scores;
-      // EXTRA variant: scale and ALiBi bias are applied here and the exponent uses a unit multiplier
-      // (four independent partial maxima / sums: a single running value would be a 128-long dependent chain)
-      float mt[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int i = 0; i < BLOCK_KV; ++i) {
-        float sc = __uint_as_float(v[i]);
-        if (EXTRA) sc = fmaf(slope2, (float)(k_base + i - q_pos), sc * p.scale_log2);
-        if (masked && ((k_base + i) > k_lim || (EXTRA && (k_base + i) < k_low))) sc = -INFINITY;
-        v[i] = __float_as_uint(sc);
-        mt[i & 3] = fmaxf(mt[i & 3], sc);
-      }
-      float m_tile = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3]));
-      const float ex_mul = EXTRA ? 1.f : p.scale_log2;
-      m_tile *= ex_mul;
-      // ---- lagging max / rare rescale of the TMEM accumulator
-      const float m_new = fmaxf(m_run, m_tile);
-      if (j == 0 && !resume) {
-        m_run = m_new;                                   // nothing accumulated yet
-      } else {
-        const bool need = (m_new - m_run) > TAU;         // (-inf) - (-inf) = NaN -> false
-        if (__any_sync(0xffffffffu, need)) {
-          if (j > 0) {                                   // P_{j-1} V_{j-1} has retired: the accumulator is stable
-            mbar_wait(o_full, (uint32_t)((j - 1) & 1));
-            tc_fence_after();
-          }
-          const float alpha = need ? fast_exp2(m_run - m_new) : 1.f;
+      const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
+      const bool row_ok = q_pos < len_q;                   // rows past the end of a (packed) sequence are never stored
 #pragma unroll 1
-          for (int c = 0; c < D; c += 32) {
-            uint32_t t[32];
-            tmem_ld_32x32b_x32(o_addr + c, t);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
-            tmem_st_32x32b_x16(o_addr + c, *reinterpret_cast<uint32_t(*)[16]>(&t[0]));
-            tmem_st_32x32b_x16(o_addr + c + 16, *reinterpret_cast<uint32_t(*)[16]>(&t[16]));
-          }
-          tmem_st_wait();
-          l_run *= alpha;
-          if (need) m_run = m_new;
+      for (int c = 0; c < D; c += 32) {
+        uint32_t w[32];
+        __syncwarp();
+        tmem_ld_32x32b_x32(o_addr + c, w);                 // executed by every lane (warp-collective), stores predicated
+        tmem_ld_wait();
+        if (c + 32 == D) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&o_empty[t]);         // O_t may be overwritten by the next unit
         }
-      }
-      const float m_use = (m_run == -INFINITY) ? 0.f : m_run;     // keeps the exponent finite on a fully masked row
-      // ---- p = exp2(s - m), row sum, 16-bit P into the swizzled K-major tile of buffer j & 1
-      // (that buffer was last read by P_{j-2} V_{j-2}, which retired before Q K_j^T - issued after it - completed)
-      uint8_t* p_row = smem_p + (j & 1) * C::P_BYTES + r * 128;
-      float lt[4] = {0.f, 0.f, 0.f, 0.f};
+        if (!row_ok) {
+          // a row past the end of its (packed) sequence: computed on garbage, never stored
+        } else if (p.o_state != nullptr) {
+          float4* dst = reinterpret_cast<float4*>(p.o_state + row * ((size_t)p.hq * D) + (size_t)head * D + c);
 #pragma unroll
-      for (int c = 0; c < BLOCK_KV; c += 32) {
-        uint32_t packed[16];
+          for (int i = 0; i < 8; ++i)
+            dst[i] = make_float4(__uint_as_float(w[4 * i]) * inv_l, __uint_as_float(w[4 * i + 1]) * inv_l,
+                                 __uint_as_float(w[4 * i + 2]) * inv_l, __uint_as_float(w[4 * i + 3]) * inv_l);
+        } else {
+          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) +
+                                                (row * ((size_t)p.hq * D) + (size_t)head * D + c) * 2);
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float p0 = fast_exp2(fmaf(__uint_as_float(v[c + i]), ex_mul, -m_use));
-          const float p1 = fast_exp2(fmaf(__uint_as_float(v[c + i + 1]), ex_mul, -m_use));
-          lt[(i >> 1) & 3] += p0 + p1;
-          if (p.out_dtype == CB_BF16) {
-            __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-            packed[i >> 1] = *reinterpret_cast<uint32_t*>(&h);
-          } else {
-            __half2 h = __floats2half2_rn(p0, p1);
-            packed[i >> 1] = *reinterpret_cast<uint32_t*>(&h);
+          for (int i = 0; i < 4; ++i) {
+            uint32_t h[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              h[e] = pack_16<BF16>(__uint_as_float(w[8 * i + 2 * e]) * inv_l, __uint_as_float(w[8 * i + 2 * e + 1]) * inv_l);
+            dst[i] = make_uint4(h[0], h[1], h[2], h[3]);
           }
         }
-        // 32 keys = 64 bytes = four 16-byte chunks of this row inside sub-tile (c / 64)
-        uint8_t* sub = p_row + (c >> 6) * (BLOCK_Q * 128);
-        const int chunk0 = (c & 32) ? 4 : 0;
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const int chunk = (chunk0 + q4) ^ (r & 7);     // SWIZZLE_128B: 16-byte chunk index XOR (row mod 8)
-          *reinterpret_cast<uint4*>(sub + chunk * 16) =
-              make_uint4(packed[q4 * 4], packed[q4 * 4 + 1], packed[q4 * 4 + 2], packed[q4 * 4 + 3]);
-        }
       }
-      const float l_tile = (lt[0] + lt[1]) + (lt[2] + lt[3]);
-      l_run += l_tile;
-      // keep in step with the accumulator barrier: observe "P_{j-1} V_{j-1} retired" once per tile.  It completed long
-      // ago in the common case (no stall), but a parity wait is only unambiguous while the waiter is at most ONE phase
-      // behind - the epilogue's wait for the last tile would otherwise pass on the phase before the previous one
-      // (seen on hardware with two-tile launches: output read before the last two P V had landed).
-      if (j > 0) mbar_wait(o_full, (uint32_t)((j - 1) & 1));
-      tc_fence_before();
-      fence_proxy_async();                               // generic-proxy smem writes -> visible to the tensor core
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);                // P_j is in shared memory, the accumulator is consistent
+      if (p.lse && row_ok)
+        p.lse[row * p.hq + head] = l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
+      ++uses;
     }
-    // ---- epilogue: the last P V has retired; normalise and store this thread's row
-    mbar_wait(o_full, (uint32_t)((kv_tiles - 1) & 1));
-    tc_fence_after();
-    const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
-    const size_t row = (size_t)q_row0 + r;
-    const bool row_ok = q_pos < len_q;                   // rows past the end of a (packed) sequence are never stored
-#pragma unroll 1
-    for (int c = 0; c < D; c += 32) {
-      uint32_t t[32];
-      __syncwarp();
-      tmem_ld_32x32b_x32(o_addr + c, t);                 // executed by every lane (warp-collective), stores predicated
-      tmem_ld_wait();
-      if (!row_ok) {
-        // a row past the end of its (packed) sequence: computed on garbage, never stored
-      } else if (p.o_state != nullptr) {
-        float4* dst = reinterpret_cast<float4*>(p.o_state + row * ((size_t)p.hq * D) + (size_t)head * D + c);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          dst[i] = make_float4(__uint_as_float(t[4 * i]) * inv_l, __uint_as_float(t[4 * i + 1]) * inv_l,
-                               __uint_as_float(t[4 * i + 2]) * inv_l, __uint_as_float(t[4 * i + 3]) * inv_l);
-      } else {
-        uint32_t w[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float a0 = __uint_as_float(t[2 * i]) * inv_l, a1 = __uint_as_float(t[2 * i + 1]) * inv_l;
-          if (p.out_dtype == CB_BF16) {
-            __nv_bfloat162 h = __floats2bfloat162_rn(a0, a1);
-            w[i] = *reinterpret_cast<uint32_t*>(&h);
-          } else {
-            __half2 h = __floats2half2_rn(a0, a1);
-            w[i] = *reinterpret_cast<uint32_t*>(&h);
-          }
-        }
-        uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) +
-                                              (row * ((size_t)p.hq * D) + (size_t)head * D + c) * 2);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-      }
-    }
-    if (p.lse && q_pos < len_q)
-      p.lse[row * p.hq + head] = l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 2) tmem_dealloc<C::TMEM_COLS>(tmem_base);
+}
+
+template <int D, bool EXTRA, bool BF16>
+int launch_flash_fwd_kernel(dim3 grid, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p,
+                            cudaStream_t stream) {
+  using C = FaCfg<D>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<D, EXTRA, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         C::SMEM_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
+  flash_fwd_kernel<D, EXTRA, BF16><<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  return (int)cudaGetLastError();
 }
 
 template <int D>
@@ -430,7 +639,6 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* out, flo
                      int seqlen_k, int hq, int hkv, int causal, float scale, int dtype, cudaStream_t stream,
                      const int* cu_seqlens = nullptr, long long total_tokens = 0, float* o_state = nullptr,
                      int has_prev = 0, int window = 0, const float* alibi = nullptr) {
-  using C = FaCfg<D>;
   const bool bf16 = dtype == CB_BF16;
   CUtensorMap tq, tk, tv;
   const uint64_t rows_q = cu_seqlens ? (uint64_t)total_tokens : (uint64_t)batch * seqlen_q;
@@ -445,28 +653,24 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* out, flo
   p.cu_seqlens = cu_seqlens;
   p.o_state = o_state; p.has_prev = has_prev;
   p.batch = batch; p.seqlen_q = seqlen_q; p.seqlen_k = seqlen_k; p.hq = hq; p.hkv = hkv; p.causal = causal;
+  p.pair_heads = (hq / hkv) % 2 == 0;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.out = out; p.lse = lse; p.out_dtype = dtype;
   p.window = window; p.alibi = alibi;
   p.idesc_qk = make_idesc_f16(BLOCK_Q, BLOCK_KV, bf16 ? 1 : 0, 0, 0);      // S[128 x 128] = Q (K-major) x K (K-major)
   p.idesc_pv = make_idesc_f16(BLOCK_Q, D, bf16 ? 1 : 0, 0, 1);              // O[128 x D]  = P (K-major) x V (MN-major)
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(flash_fwd_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
-  // packed: at most total/128 + batch query tiles exist; uniform: ceil(seqlen / 128) per sequence
-  dim3 grid(cu_seqlens ? (unsigned)(total_tokens / BLOCK_Q + batch) : (unsigned)((seqlen_q + BLOCK_Q - 1) / BLOCK_Q), hq,
-            cu_seqlens ? 1 : batch);
+  // units of `per` query rows; packed: at most total / per + batch of them exist per head
+  const int per = p.pair_heads ? BLOCK_Q : 2 * BLOCK_Q;
+  p.head_units = p.pair_heads ? hq / 2 : hq;
+  p.seq_units = cu_seqlens ? 0 : (seqlen_q + per - 1) / per;
+  const long long most = (cu_seqlens ? total_tokens / per + batch : (long long)p.seq_units * batch) * p.head_units;
+  if (most > (1ll << 30)) return (int)cudaErrorInvalidValue;
+  const dim3 grid((unsigned)(most < cb_num_sms() ? most : cb_num_sms()));
   if (window > 0 || alibi != nullptr)
-    flash_fwd_kernel<D, true><<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, p);
-  else
-    flash_fwd_kernel<D, false><<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, p);
-  return (int)cudaGetLastError();
+    return bf16 ? launch_flash_fwd_kernel<D, true, true>(grid, tq, tk, tv, p, stream)
+                : launch_flash_fwd_kernel<D, true, false>(grid, tq, tk, tv, p, stream);
+  return bf16 ? launch_flash_fwd_kernel<D, false, true>(grid, tq, tk, tv, p, stream)
+              : launch_flash_fwd_kernel<D, false, false>(grid, tq, tk, tv, p, stream);
 }
 
 

@@ -243,3 +243,32 @@ def test_flash_block_mode_state_carry(rows, Hq, Hkv, big_second):
     ref_lse = torch.logsumexp(sc, -1).transpose(0, 1)
     torch.testing.assert_close(lse, ref_lse, atol=3e-3, rtol=3e-3)
     torch.testing.assert_close(o_state, ref, atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("lens", [[0, 1, 0, 255, 256, 257, 0], [3] * 70 + [129], list(range(1, 300, 7)), [513, 0, 384, 385]])
+@pytest.mark.parametrize("Hq,Hkv,D", [(3, 3, 64), (10, 2, 128), (12, 2, 64), (160, 160, 128)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_flash_unit_list_of_packed_batches(lens, Hq, Hkv, D, causal):
+    """The device-side list of work units: empty sequences, more sequences than a warp has lanes, ends on and beside the
+    edges of one and of two query tiles, odd and even groups (two tiles of a head / two heads of a tile), far more and
+    far fewer units than SMs.  Every row is written exactly once with the right neighbours."""
+    from colossalai_b200.ops import flash_attn_native as fa
+
+    if Hq == 160 and len(lens) > 50:
+        lens = lens[-40:]
+    torch.manual_seed(len(lens))
+    T = sum(lens)
+    q, k, v = (torch.randn(T, h, D, device="cuda", dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    cu = torch.tensor([0] + lens, device="cuda").cumsum(0).to(torch.int32)
+    out, lse = fa.flash_fwd(q, k, v, 1, causal, None, cu_seqlens=cu)
+    a = 0
+    for n in lens:
+        if n:
+            kk, vv = (x[a:a + n].float().repeat_interleave(Hq // Hkv, 1) for x in (k, v))
+            s = torch.einsum("qhd,khd->hqk", q[a:a + n].float(), kk) * D ** -0.5
+            if causal:
+                s = s.masked_fill(~torch.ones(n, n, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+            # P is rounded to bf16 (2^-9 of each weight), the result once more
+            torch.testing.assert_close(out[a:a + n].float(), torch.einsum("hqk,khd->qhd", s.softmax(-1), vv), atol=2e-2, rtol=2e-2)
+            torch.testing.assert_close(lse[a:a + n], s.logsumexp(-1).t(), atol=2e-3, rtol=2e-3)
+        a += n
