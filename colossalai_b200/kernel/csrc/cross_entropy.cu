@@ -1,52 +1,80 @@
 // Fused (vocab-parallel) cross-entropy building blocks for sm_100a.
-// One CTA per token row; the [T, V_local] logits are streamed with 16-byte loads.  Forward reads the logits twice
-// (row max, then sum-exp relative to the GLOBAL max that python all-reduces in between); backward reads once and
-// writes the gradient once.  Replaces the eager torch composition in the reference's DistCrossEntropy
+// One CTA per token row.  Forward reads the logits once: running max and sum of exponentials against it, and the target's
+// logit (vocab-parallel callers rescale the sums to the all-reduced max); a one-block kernel turns the rows into the loss.
+// Backward reads once and writes the gradient once.  Replaces the eager torch composition in the reference's DistCrossEntropy
 // (colossalai/shardformer/layer/loss.py:25-127) which materialises exp(logits) and a one-hot mask.
+// Bound: HBM.  4096 rows of 128256 bf16: max and sum in passes of their own took 174 + 180 us, the one pass 172 us; the
+// gradient (read + write) runs at 6.3 TB/s.
+#include <type_traits>
+
 #include "common.cuh"
 
-template <typename T>
-__global__ void __launch_bounds__(512) ce_row_max_kernel(const T* __restrict__ x, float* __restrict__ out, int V, int Vv) {
-  constexpr int VEC = Vec16<T>::N;
-  __shared__ float red[32];
-  const T* row = x + (size_t)blockIdx.x * V;
-  float m = -INFINITY;
-  for (int c = threadIdx.x * VEC; c < Vv; c += blockDim.x * VEC) {
-    Vec16<T> v;
-    v.load_nc(row + c);
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) if (c + i < Vv) m = fmaxf(m, v.get(i));
-  }
-  m = block_max(m, red);
-  if (threadIdx.x == 0) out[blockIdx.x] = m;
-}
+constexpr int CE_THREADS = 512;
+constexpr int CE_UNROLL = 4;           // 16-byte vectors a thread has in flight
 
+// stats: [3, rows] fp32 = max over the row, sum of exp(x - max), the target's logit (0 if it is not in this shard)
 template <typename T>
-__global__ void __launch_bounds__(512) ce_sumexp_target_kernel(const T* __restrict__ x,
-                                                               const int64_t* __restrict__ target,
-                                                               const float* __restrict__ gmax, float* __restrict__ out,
-                                                               int Trows, int V, int Vv, int64_t vocab_start,
-                                                               int64_t ignore_index) {
+__global__ void __launch_bounds__(CE_THREADS) ce_row_stats_kernel(const T* __restrict__ x, const int64_t* __restrict__ target,
+                                                                  float* __restrict__ stats, int rows, int V, int Vv,
+                                                                  int64_t vocab_start, int64_t ignore_index) {
   constexpr int VEC = Vec16<T>::N;
   __shared__ float red[64];
   const int r = blockIdx.x;
   const T* row = x + (size_t)r * V;
-  const float m = gmax[r];
-  float s[1] = {0.f};
-  for (int c = threadIdx.x * VEC; c < Vv; c += blockDim.x * VEC) {
-    Vec16<T> v;
-    v.load_nc(row + c);
+  float m = -INFINITY, s = 0.f;
+  constexpr int STEP = CE_THREADS * VEC;
+  auto take = [&](int c0, auto whole_tag) {      // (a row's end is a copy of the code: no comparison per element elsewhere)
+    constexpr bool WHOLE = decltype(whole_tag)::value;
+    Vec16<T> v[CE_UNROLL];
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) if (c + i < Vv) s[0] += __expf(v.get(i) - m);
-  }
-  block_sum<1>(s, red);
+    for (int u = 0; u < CE_UNROLL; ++u)
+      if (WHOLE || c0 + u * STEP < Vv) v[u].load_nc(row + c0 + u * STEP);
+    float mc = -INFINITY;
+#pragma unroll
+    for (int u = 0; u < CE_UNROLL; ++u)
+#pragma unroll
+      for (int i = 0; i < VEC; ++i)
+        if (WHOLE || c0 + u * STEP + i < Vv) mc = fmaxf(mc, v[u].get(i));
+    if (mc > m) {                                // (a row of -inf so far keeps s = 0: exp(-inf - -inf) is not taken)
+      s *= __expf(m - mc);
+      m = mc;
+    }
+    const float ref = m == -INFINITY ? 0.f : m;
+#pragma unroll
+    for (int u = 0; u < CE_UNROLL; ++u)
+#pragma unroll
+      for (int i = 0; i < VEC; ++i)
+        if (WHOLE || c0 + u * STEP + i < Vv) s += __expf(v[u].get(i) - ref);
+  };
+  int c0 = threadIdx.x * VEC;
+  for (; c0 + (CE_UNROLL - 1) * STEP + VEC <= Vv; c0 += CE_UNROLL * STEP) take(c0, std::true_type{});
+  for (; c0 < Vv; c0 += CE_UNROLL * STEP) take(c0, std::false_type{});
+  const float mr = block_max(m, red);
+  float t[1] = {s * (m == -INFINITY ? 1.f : __expf(m - mr))};          // m = -inf: s is 0, or NaN from a NaN logit
+  block_sum<1>(t, red + 32);
   if (threadIdx.x == 0) {
-    out[r] = s[0];
-    const int64_t t = target[r];
-    const int64_t local = t - vocab_start;
-    float tl = 0.f;
-    if (t != ignore_index && local >= 0 && local < Vv) tl = to_f32<T>(row[local]);
-    out[Trows + r] = tl;
+    stats[r] = mr;
+    stats[rows + r] = t[0];
+    const int64_t tg = target[r], local = tg - vocab_start;
+    stats[2 * rows + r] = (tg != ignore_index && local >= 0 && local < Vv) ? to_f32<T>(row[local]) : 0.f;
+  }
+}
+
+// loss = sum over rows with a label of log(sumexp) + max - target logit, divided by their number (at least 1) when `mean`
+__global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__ stats, const int64_t* __restrict__ target,
+                                                       float* __restrict__ loss, int64_t* __restrict__ n_valid, int rows,
+                                                       int64_t ignore_index, int mean) {
+  __shared__ float red[64];
+  float acc[2] = {0.f, 0.f};           // (up to 2^24 rows per thread are counted exactly)
+  for (int r = threadIdx.x; r < rows; r += blockDim.x)
+    if (target[r] != ignore_index) {
+      acc[0] += (float)log((double)stats[rows + r]) + stats[r] - stats[2 * rows + r];   // (logf is approximate here)
+      acc[1] += 1.f;
+    }
+  block_sum<2>(acc, red);
+  if (threadIdx.x == 0) {
+    *n_valid = (int64_t)acc[1];
+    *loss = mean ? acc[0] / fmaxf(acc[1], 1.f) : acc[0];
   }
 }
 
@@ -55,7 +83,9 @@ __global__ void __launch_bounds__(512) ce_softmax_grad_kernel(const T* __restric
                                                               const int64_t* __restrict__ target,
                                                               const float* __restrict__ gmax,
                                                               const float* __restrict__ sumexp,
-                                                              const float* __restrict__ row_scale, T* __restrict__ g,
+                                                              const float* __restrict__ row_scale,
+                                                              const float* __restrict__ scale,
+                                                              const int64_t* __restrict__ n_valid, T* __restrict__ g,
                                                               int V, int Vv, int64_t vocab_start,
                                                               int64_t ignore_index) {
   constexpr int VEC = Vec16<T>::N;
@@ -64,8 +94,10 @@ __global__ void __launch_bounds__(512) ce_softmax_grad_kernel(const T* __restric
   T* grow = g + (size_t)r * V;
   const int64_t t = target[r];
   const bool ignored = (t == ignore_index);
-  const float m = gmax[r], inv = ignored ? 0.f : row_scale[r] / sumexp[r];
-  const float sc = ignored ? 0.f : row_scale[r];
+  // a factor per row, or one for all divided by the number of labels
+  const float f = row_scale != nullptr ? row_scale[r] : (n_valid != nullptr ? *scale / (float)max(*n_valid, (int64_t)1) : *scale);
+  const float m = gmax[r], inv = ignored ? 0.f : f / sumexp[r];
+  const float sc = ignored ? 0.f : f;
   const int64_t local = t - vocab_start;
   for (int c = threadIdx.x * VEC; c < V; c += blockDim.x * VEC) {
     Vec16<T> v, o;
@@ -82,27 +114,28 @@ __global__ void __launch_bounds__(512) ce_softmax_grad_kernel(const T* __restric
 
 extern "C" {
 
-int cb_ce_row_max(const void* x, float* out, int T_, int V, int Vv, int dtype, cudaStream_t s) {
-  if (T_ == 0) return 0;
-  CB_DISPATCH_FLOAT(dtype, T, { ce_row_max_kernel<T><<<T_, 512, 0, s>>>((const T*)x, out, V, Vv); });
-  return CB_LAUNCH_CHECK();
-}
-
-int cb_ce_sumexp_target(const void* x, const int64_t* target, const float* gmax, float* out, int T_, int V, int Vv,
-                        int64_t vocab_start, int64_t ignore_index, int dtype, cudaStream_t s) {
-  if (T_ == 0) return 0;
+int cb_ce_row_stats(const void* x, const int64_t* target, float* stats, int rows, int V, int Vv, int64_t vocab_start,
+                    int64_t ignore_index, int dtype, cudaStream_t s) {
+  if (rows == 0) return 0;
   CB_DISPATCH_FLOAT(dtype, T, {
-    ce_sumexp_target_kernel<T><<<T_, 512, 0, s>>>((const T*)x, target, gmax, out, T_, V, Vv, vocab_start, ignore_index);
+    ce_row_stats_kernel<T><<<rows, CE_THREADS, 0, s>>>((const T*)x, target, stats, rows, V, Vv, vocab_start, ignore_index);
   });
   return CB_LAUNCH_CHECK();
 }
 
+int cb_ce_loss(const float* stats, const int64_t* target, float* loss, int64_t* n_valid, int rows, int64_t ignore_index, int mean,
+               cudaStream_t s) {
+  ce_loss_kernel<<<1, 1024, 0, s>>>(stats, target, loss, n_valid, rows, ignore_index, mean);
+  return CB_LAUNCH_CHECK();
+}
+
+// row_scale: fp32 [T], or null and then scale fp32 [1] and n_valid int64 [1] (null: 1)
 int cb_ce_softmax_grad(const void* x, const int64_t* target, const float* gmax, const float* sumexp,
-                       const float* row_scale, void* g, int T_, int V, int Vv, int64_t vocab_start,
-                       int64_t ignore_index, int dtype, cudaStream_t s) {
+                       const float* row_scale, const float* scale, const int64_t* n_valid, void* g, int T_, int V, int Vv,
+                       int64_t vocab_start, int64_t ignore_index, int dtype, cudaStream_t s) {
   if (T_ == 0) return 0;
   CB_DISPATCH_FLOAT(dtype, T, {
-    ce_softmax_grad_kernel<T><<<T_, 512, 0, s>>>((const T*)x, target, gmax, sumexp, row_scale, (T*)g, V, Vv,
+    ce_softmax_grad_kernel<T><<<T_, 512, 0, s>>>((const T*)x, target, gmax, sumexp, row_scale, scale, n_valid, (T*)g, V, Vv,
                                                 vocab_start, ignore_index);
   });
   return CB_LAUNCH_CHECK();

@@ -44,36 +44,26 @@ class DistCrossEntropy(torch.autograd.Function):
         start = rank * V_local
         # columns beyond the true vocab (padding added so the vocab divides tp * 64) must not enter the softmax
         vcols = V_local if vocab_size is None else max(min(V_local, vocab_size - start), 0)
-        # local statistics: max, sumexp (relative to the GLOBAL max after all-reduce), target logit
-        local_max = ce_ops.row_max(vocab_logits, vcols) if vcols > 0 else \
-            torch.full((T,), float("-inf"), device=vocab_logits.device)           # [T] fp32
-        if ws > 1:
-            dist.all_reduce(local_max, op=dist.ReduceOp.MAX, group=process_group)
-        stats = ce_ops.sumexp_and_target(vocab_logits, target, local_max, start, ignore_index, vcols)  # [2, T] fp32
-        if ws > 1:
-            dist.all_reduce(stats, group=process_group)
-        sumexp, tgt_logit = stats[0], stats[1]
-        valid = target != ignore_index
-        n_valid = valid.sum()
-        loss_tok = torch.where(valid, torch.log(sumexp) + local_max - tgt_logit, torch.zeros_like(sumexp))
-        if mode == "mean":
-            loss = loss_tok.sum() / n_valid.clamp(min=1)
-        elif mode == "sum":
-            loss = loss_tok.sum()
-        else:
+        if mode not in ("mean", "sum"):
             raise ValueError(mode)
-        ctx.save_for_backward(vocab_logits, target, local_max, sumexp, n_valid)
+        # local statistics: max, sumexp (against it), target logit, from one pass over the logits            fp32 [3, T]
+        stats = ce_ops.row_stats(vocab_logits, target, start, ignore_index, vcols)
+        if ws > 1:
+            gmax = stats[0].clone()
+            dist.all_reduce(gmax, op=dist.ReduceOp.MAX, group=process_group)
+            sums = ce_ops.rescale(stats, gmax)
+            dist.all_reduce(sums, group=process_group)
+            stats = torch.cat([gmax.unsqueeze(0), sums])
+        loss, n_valid = ce_ops.loss_from_stats(stats, target, ignore_index, mode == "mean")
+        ctx.save_for_backward(vocab_logits, target, stats, n_valid)
         ctx.start, ctx.ignore_index, ctx.mode, ctx.valid = start, ignore_index, mode, vcols
         return loss.to(dtype)
 
     @staticmethod
     def backward(ctx, grad_output):
-        logits, target, gmax, sumexp, n_valid = ctx.saved_tensors
-        scale = grad_output.float()
-        if ctx.mode == "mean":
-            scale = scale / n_valid.clamp(min=1)
-        grad = ce_ops.softmax_grad(logits, target, gmax, sumexp, scale, ctx.start, ctx.ignore_index,
-                                   valid_cols=ctx.valid)
+        logits, target, stats, n_valid = ctx.saved_tensors
+        grad = ce_ops.softmax_grad(logits, target, stats[0], stats[1], grad_output.float(), ctx.start, ctx.ignore_index,
+                                   valid_cols=ctx.valid, n_valid=n_valid if ctx.mode == "mean" else None)
         return grad, None, None, None, None, None, None
 
 
@@ -89,14 +79,15 @@ class DistLogProb(torch.autograd.Function):
         V_local = logits.shape[-1]
         start = rank * V_local
         valid = V_local if vocab_size is None else max(min(V_local, vocab_size - start), 0)
-        gmax = ce_ops.row_max(logits, valid)
+        stats = ce_ops.row_stats(logits, tgt, start, -(10**9), valid)
+        gmax, sums = stats[0], stats[1:]
         if ws > 1:
+            gmax = gmax.clone()
             dist.all_reduce(gmax, op=dist.ReduceOp.MAX, group=process_group)
-        stats = ce_ops.sumexp_and_target(logits, tgt, gmax, start, -(10**9), valid)
-        if ws > 1:
-            dist.all_reduce(stats, group=process_group)
-        logp = stats[1] - gmax - torch.log(stats[0])
-        ctx.save_for_backward(logits, tgt, gmax, stats[0])
+            sums = ce_ops.rescale(stats, gmax)
+            dist.all_reduce(sums, group=process_group)
+        logp = sums[1] - gmax - torch.log(sums[0])
+        ctx.save_for_backward(logits, tgt, gmax, sums[0])
         ctx.start, ctx.shape, ctx.valid = start, shape, valid
         return logp.view(shape).to(dtype)
 

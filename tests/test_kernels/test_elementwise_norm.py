@@ -137,6 +137,37 @@ def test_cross_entropy_blocks(dtype, V, valid, start):
     torch.testing.assert_close(g.float(), g_ref.float(), atol=2e-3 if dtype != torch.float32 else 1e-6, rtol=2e-2)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("V,valid", [(8, 8), (16384, 16384), (16392, 16385), (50304, 50257), (4096, 1), (4096, 0)])
+def test_cross_entropy_one_pass_stats(dtype, V, valid):
+    """Row maximum and sum in one pass at the ends of a thread's share, with rows of the type's lowest value, of -inf in
+    front, of one finite entry, and sorted rows whose running maximum moves at every vector."""
+    torch.manual_seed(V)
+    x = 3 * torch.randn(9, V, device="cuda")
+    x[1] = torch.finfo(dtype).min
+    x[2] = float("-inf")
+    x[2, -1] = x[2, max(valid - 1, 0)] = 1.0
+    x[3] = torch.linspace(-40, 40, V, device="cuda")
+    x[4] = torch.linspace(40, -40, V, device="cuda")
+    x[5] = float("-inf")
+    x[6, V // 2] = float("nan")
+    x = x.to(dtype)
+    t = torch.full((9,), 5, device="cuda")
+    t[7], t[8] = -100, 5 + V
+    m, s, tl = ce.row_stats(x, t, 5, -100, valid)
+    x64 = x[:, :valid].double()
+    if valid == 0:
+        assert torch.isneginf(m).all() and not s.any() and not tl.any()
+        return
+    rows = [r for r in range(9) if r not in (5, 6)]
+    assert torch.equal(m[rows].double(), x64.max(-1).values[rows])
+    # approximate exponentials of 2^-21 each and fp32 sums of at most V / 512 + 40 terms in a row
+    ref = (x64 - x64.max(-1, keepdim=True).values).exp().sum(-1)
+    assert ((s.double() - ref).abs() <= 2e-5 * ref)[rows].all()
+    assert torch.isneginf(m[5]) and s[5] == 0 and (valid <= V // 2 or torch.isnan(s[6]))
+    assert torch.equal(tl[rows[:5]], x[rows[:5], 0].float()) and tl[7] == 0 and tl[8] == 0
+
+
 def test_dist_cross_entropy_matches_torch():
     from colossalai_b200.shardformer.layer.loss import cross_entropy_1d
 
