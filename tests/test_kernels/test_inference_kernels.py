@@ -171,3 +171,21 @@ def test_engine_gpu_cuda_graph_matches_eager():
         outs.append(ids)
     assert outs[0] == outs[1]
     assert loader.launch_counter.by_name.get("paged_decode_attention", 0) > 0
+
+
+@pytest.mark.parametrize("lens", [[0, 0, 0], [1], [0, 1, 0, 33, 0], [16] * 33, [4097] + [1] * 40, [5000, 3, 0, 2048], list(range(1, 130))])
+@pytest.mark.parametrize("Hq,Hkv,D,window", [(4, 4, 64, 0), (10, 2, 128, 0), (48, 6, 64, 40), (3, 1, 128, 1)])
+def test_paged_decode_pieces(lens, Hq, Hkv, D, window):
+    """The balanced split of all visible tokens over the CTAs: empty sequences (zeros), sequences in one piece and in many,
+    shares that span many sequences, more than one round of 32 sequences, head counts that leave a CTA partly filled."""
+    dev = torch.device("cuda")
+    torch.manual_seed(len(lens))
+    kc, vc, tables = _mk_cache(len(lens), max(max(lens), 1) + 5, 16, Hkv, D, torch.bfloat16, dev)
+    q = torch.randn(len(lens), Hq, D, device=dev, dtype=torch.bfloat16)
+    seq = torch.tensor(lens, device=dev, dtype=torch.int32)
+    out = iops.paged_decode_attention(q, kc, vc, tables, seq, window=window or None)
+    live = [i for i, n in enumerate(lens) if n]
+    assert not out[[i for i, n in enumerate(lens) if not n]].any()
+    if live:
+        ref = iops.paged_decode_attention_ref(q.float()[live], kc.float(), vc.float(), tables[live], seq[live], window=window or None)
+        torch.testing.assert_close(out[live].float(), ref, atol=2e-2, rtol=2e-2)      # weights rounded to bf16
