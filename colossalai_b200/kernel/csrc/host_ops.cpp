@@ -1,0 +1,297 @@
+// Host side of the small hot operators in native code: allocation, autograd and launch without the interpreter.
+//
+// A python autograd function costs 30 us for a forward and 155 us for a forward + backward of a norm whose kernels take 2 and
+// 5 us (measured on the host of a B200: stream lookup 3.3 us, argument conversion and launch 9.6 us, three allocations, the
+// hand-over of the interpreter to the autograd thread 47 us); every serving call and every training call on a few hundred
+// rows was bound by that.  The same functions as C++ autograd functions: norm of 16 rows 35.8 -> 13.7 us a call
+// (with the python checks in front), forward + backward of a few rows 143 -> 86 us, most of which is autograd itself.
+// The kernels stay behind their C launchers (`bind` takes their addresses); tensors that something watches - tracing,
+// functorch, forward-mode, dispatch modes, subclasses - never come here (`ops/_dispatch.py:plain_call`).
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include <atomic>
+#include <cmath>
+#include <map>
+#include <string>
+
+using torch::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+using OptTensor = c10::optional<Tensor>;
+
+namespace {
+
+int code_of(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return 0;
+    case at::kHalf: return 1;
+    case at::kBFloat16: return 2;
+    default: TORCH_CHECK(false, "unsupported dtype ", t.scalar_type());
+  }
+}
+const void* ptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
+void* mut(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+template <typename T> T* mut_as(const Tensor& t) { return reinterpret_cast<T*>(mut(t)); }
+template <typename T> const T* as(const Tensor& t) { return reinterpret_cast<const T*>(ptr(t)); }
+cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+// 16-byte loads: a contiguous tensor at an odd offset of its storage is copied
+Tensor packed(const Tensor& t) {
+  Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.const_data_ptr()) % 16 == 0 ? c : c.clone(at::MemoryFormat::Contiguous);
+}
+
+// ---- launchers
+struct Launchers {
+  int (*rmsnorm_fwd)(const void*, const void*, const void*, void*, void*, float*, int, int, float, int, cudaStream_t);
+  int (*rmsnorm_bwd)(const void*, const void*, const void*, const float*, const void*, void*, float*, void*, int, int, int, int,
+                     cudaStream_t);
+  int (*norm_bwd_grid)(int);
+  int (*glu_fwd)(const void*, void*, int64_t, int, int, int, const int64_t*, cudaStream_t);
+  int (*glu_bwd)(const void*, const void*, void*, int64_t, int, int, int, const int64_t*, cudaStream_t);
+  int (*row_stats)(const void*, const int64_t*, float*, int, int, int, int64_t, int64_t, int, cudaStream_t);
+  int (*ce_loss)(const float*, const int64_t*, float*, int64_t*, int, int64_t, int, cudaStream_t);
+  int (*softmax_grad)(const void*, const int64_t*, const float*, const float*, const float*, const float*, const int64_t*, void*,
+                      int, int, int, int64_t, int64_t, int, cudaStream_t);
+  int (*flash_varlen_fwd)(const void*, const void*, const void*, void*, float*, const int*, int, long long, int, int, int, int,
+                          float, int, cudaStream_t);
+  int (*flash_bwd)(const void*, const void*, const void*, const void*, const void*, const float*, void*, void*, void*, float*,
+                   float*, int, int, int, int, int, int, float, int, const int*, long long, cudaStream_t);
+  int (*decode_splits)(int, int, int, int, int, int*);
+  int (*decode)(const void*, const void*, const void*, const int*, const int*, void*, float*, float*, int, int, int, int, int, int,
+                int, int, float, const float*, int64_t, int64_t, int, int, cudaStream_t);
+} L;
+
+// launches by name since the last `counts`
+struct Count {
+  const char* name;
+  std::atomic<long long> n{0};
+};
+Count n_norm_fwd{"rmsnorm_fwd"}, n_norm_bwd{"rmsnorm_bwd"}, n_glu_fwd{"glu_fwd"}, n_glu_bwd{"glu_bwd"},
+    n_stats{"ce_row_stats"}, n_loss{"ce_loss"}, n_grad{"ce_softmax_grad"}, n_flash_fwd{"flash_attn_varlen_fwd"},
+    n_flash_bwd{"flash_attn_bwd"}, n_decode{"paged_decode_attention"};
+Count* const COUNTS[] = {&n_norm_fwd, &n_norm_bwd, &n_glu_fwd, &n_glu_bwd, &n_stats, &n_loss, &n_grad, &n_flash_fwd, &n_flash_bwd,
+                         &n_decode};
+
+void launched(int rc, Count& c, int n = 1) {
+  TORCH_CHECK(rc == 0, c.name, ": native launcher returned CUDA error ", rc);
+  c.n.fetch_add(n, std::memory_order_relaxed);
+}
+
+// ------------------------------------------------------------------------------------------------ RMS norm
+struct RmsNorm : torch::autograd::Function<RmsNorm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, double eps, const OptTensor& residual) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const bool has_res = residual.has_value() && residual->defined();
+    const Tensor x2 = x.contiguous(), r2 = has_res ? residual->contiguous() : Tensor();
+    const int H = (int)x2.size(-1), rows = H ? (int)(x2.numel() / H) : 0;
+    Tensor y = at::empty_like(x2), h = has_res ? at::empty_like(x2) : x2;
+    Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
+    launched(L.rmsnorm_fwd(ptr(x2), ptr(r2), ptr(weight), mut(y), has_res ? mut(h) : nullptr, mut_as<float>(rstd), rows, H, (float)eps,
+                           code_of(x), stream_of(x)),
+             n_norm_fwd);
+    ctx->save_for_backward({h, weight, rstd});
+    ctx->saved_data["has_res"] = has_res;
+    ctx->set_materialize_grads(false);
+    return has_res ? variable_list{y, h} : variable_list{y};
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &h = saved[0], &weight = saved[1], &rstd = saved[2];
+    const bool has_res = ctx->saved_data["has_res"].toBool();
+    if (!grads[0].defined() && (!has_res || !grads[1].defined())) return {Tensor(), Tensor(), Tensor(), Tensor()};
+    const c10::cuda::CUDAGuard guard(h.device());
+    const int H = (int)h.size(-1), rows = H ? (int)(h.numel() / H) : 0;
+    const Tensor dy = grads[0].defined() ? grads[0].contiguous() : at::zeros_like(h);
+    const Tensor dres = has_res && grads[1].defined() ? grads[1].contiguous() : Tensor();
+    Tensor dx = at::empty_like(h), dw = at::empty_like(weight);
+    Tensor partial = at::empty({(int64_t)L.norm_bwd_grid(rows) * H}, rstd.options());
+    launched(L.rmsnorm_bwd(ptr(dy), ptr(h), ptr(weight), as<float>(rstd), ptr(dres), mut(dx), mut_as<float>(partial), mut(dw), 0, rows, H,
+                           code_of(h), stream_of(h)),
+             n_norm_bwd, 2);
+    return {dx, dw, Tensor(), has_res ? dx : Tensor()};
+  }
+};
+
+// ------------------------------------------------------------------------------------------------ gated unit
+struct Glu : torch::autograd::Function<Glu> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& gate_up, int64_t act) {
+    const c10::cuda::CUDAGuard guard(gate_up.device());
+    const Tensor gu = gate_up.contiguous();
+    const int64_t I = gu.size(-1) / 2, rows = I ? gu.numel() / (2 * I) : 0;
+    std::vector<int64_t> shape = gu.sizes().vec();
+    shape.back() = I;
+    Tensor out = at::empty(shape, gu.options());
+    launched(L.glu_fwd(ptr(gu), mut(out), rows, (int)I, (int)act, code_of(gu), nullptr, stream_of(gu)), n_glu_fwd);
+    ctx->save_for_backward({gu});
+    ctx->saved_data["act"] = act;
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor gu = ctx->get_saved_variables()[0];
+    const c10::cuda::CUDAGuard guard(gu.device());
+    const int64_t I = gu.size(-1) / 2, rows = I ? gu.numel() / (2 * I) : 0;
+    const Tensor d = grads[0].contiguous();
+    Tensor dgu = at::empty_like(gu);
+    launched(L.glu_bwd(ptr(d), ptr(gu), mut(dgu), rows, (int)I, (int)ctx->saved_data["act"].toInt(), code_of(gu), nullptr,
+                       stream_of(gu)),
+             n_glu_bwd);
+    return {dgu, Tensor()};
+  }
+};
+
+// ------------------------------------------------------------------------------------------------ cross entropy
+// one vocabulary shard: logits [T, V] contiguous, target int64 [T] contiguous
+struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& logits, const Tensor& target, int64_t ignore, int64_t start, int64_t valid,
+                        bool mean) {
+    const c10::cuda::CUDAGuard guard(logits.device());
+    const int rows = (int)logits.size(0), V = (int)logits.size(1);
+    Tensor stats = at::empty({3, rows}, logits.options().dtype(at::kFloat));
+    Tensor loss = at::empty({}, stats.options()), n_valid = at::empty({}, target.options());
+    const cudaStream_t s = stream_of(logits);
+    launched(L.row_stats(ptr(logits), as<int64_t>(target), mut_as<float>(stats), rows, V, (int)valid, start, ignore, code_of(logits), s),
+             n_stats);
+    launched(L.ce_loss(as<float>(stats), as<int64_t>(target), mut_as<float>(loss), mut_as<int64_t>(n_valid), rows, ignore, mean, s),
+             n_loss);
+    ctx->save_for_backward({logits, target, stats, n_valid});
+    ctx->saved_data["args"] = std::vector<int64_t>{ignore, start, valid, (int64_t)mean};
+    return loss;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &logits = saved[0], &target = saved[1], &stats = saved[2], &n_valid = saved[3];
+    const std::vector<int64_t> a = ctx->saved_data["args"].toIntVector();
+    const c10::cuda::CUDAGuard guard(logits.device());
+    const int rows = (int)logits.size(0), V = (int)logits.size(1);
+    const Tensor scale = grads[0].to(at::kFloat).contiguous();
+    Tensor g = at::empty_like(logits);
+    launched(L.softmax_grad(ptr(logits), as<int64_t>(target), as<float>(stats), as<float>(stats) + rows, nullptr, as<float>(scale),
+                            a[3] ? as<int64_t>(n_valid) : nullptr, mut(g), rows, V, (int)a[2], a[1], a[0], code_of(logits),
+                            stream_of(logits)),
+             n_grad);
+    return {g, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// ------------------------------------------------------------------------------------------------ packed attention
+// q [T, Hq, D], k / v [T, Hkv, D] contiguous and 16-byte aligned, cu int32 [B + 1] contiguous on the device
+struct PackedAttention : torch::autograd::Function<PackedAttention> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu, bool causal,
+                        double scale) {
+    const c10::cuda::CUDAGuard guard(q.device());
+    const int64_t T = q.size(0), Hq = q.size(1), D = q.size(2);
+    Tensor out = at::empty_like(q), lse = at::empty({T, Hq}, q.options().dtype(at::kFloat));
+    launched(L.flash_varlen_fwd(ptr(q), ptr(k), ptr(v), mut(out), mut_as<float>(lse), as<int>(cu), (int)cu.numel() - 1, T, (int)Hq,
+                                (int)k.size(1), (int)D, causal, (float)scale, code_of(q), stream_of(q)),
+             n_flash_fwd);
+    ctx->save_for_backward({q, k, v, out, lse, cu});
+    ctx->saved_data["causal"] = causal;
+    ctx->saved_data["scale"] = scale;
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const Tensor &q = s[0], &k = s[1], &v = s[2], &out = s[3], &lse = s[4], &cu = s[5];
+    const c10::cuda::CUDAGuard guard(q.device());
+    const int64_t T = q.size(0), Hq = q.size(1), D = q.size(2);
+    const Tensor dout = packed(grads[0]);
+    Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
+    Tensor delta = at::empty({T, Hq}, lse.options()), acc = at::empty({T, Hq, D}, lse.options());
+    launched(L.flash_bwd(ptr(q), ptr(k), ptr(v), ptr(out), ptr(dout), as<float>(lse), mut(dq), mut(dk), mut(dv), mut_as<float>(delta),
+                         mut_as<float>(acc), (int)cu.numel() - 1, 0, (int)Hq, (int)k.size(1), (int)D,
+                         ctx->saved_data["causal"].toBool(), (float)ctx->saved_data["scale"].toDouble(), code_of(q), as<int>(cu), T,
+                         stream_of(q)),
+             n_flash_bwd);
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// ------------------------------------------------------------------------------------------------ paged decode
+// q [n, Hq, D]; caches [pages, page, Hkv, D]; tables int32 [n, width], lens int32 [n]; workspaces: fp32 buffers the caller
+// keeps (used when they are large enough), else allocated here
+Tensor paged_decode(const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& tables, const Tensor& lens, double scale,
+                    const OptTensor& slopes, int64_t window, const OptTensor& ws_out, const OptTensor& ws_ml) {
+  const c10::cuda::CUDAGuard guard(q.device());
+  const int64_t n = q.size(0), Hq = q.size(1), D = q.size(2), page = kc.size(1), Hkv = kc.size(2), width = tables.size(1);
+  int part = 0;
+  const int64_t splits = L.decode_splits((int)n, (int)Hq, (int)Hkv, (int)D, (int)(width * page), &part);
+  const int64_t rows = n * splits * Hq;
+  Tensor o = ws_out.has_value() && ws_out->numel() >= rows * D ? *ws_out : Tensor();
+  Tensor ml = ws_ml.has_value() && ws_ml->numel() >= rows * 2 ? *ws_ml : Tensor();
+  if (!o.defined() || !ml.defined()) {
+    o = at::empty({rows * D}, q.options().dtype(at::kFloat));
+    ml = at::empty({rows * 2}, q.options().dtype(at::kFloat));
+  }
+  const Tensor qc = q.stride(2) == 1 && q.stride(1) == D ? q : q.contiguous();
+  Tensor out = at::empty(q.sizes(), q.options());
+  const float* sl = slopes.has_value() ? as<float>(*slopes) : nullptr;
+  launched(L.decode(ptr(qc), ptr(kc), ptr(vc), as<int>(tables), as<int>(lens), mut(out), mut_as<float>(o), mut_as<float>(ml), (int)n,
+                    (int)Hq, (int)Hkv, (int)D, (int)page, (int)width, (int)splits, part, (float)scale, sl, qc.stride(0), out.stride(0),
+                    code_of(q), (int)window, stream_of(q)),
+           n_decode, 2);
+  return out;
+}
+
+template <typename F> void take(const std::map<std::string, uint64_t>& table, const char* name, F& slot) {
+  const auto it = table.find(name);
+  TORCH_CHECK(it != table.end() && it->second != 0, "launcher ", name, " is missing");
+  slot = reinterpret_cast<F>(it->second);
+}
+
+void bind(const std::map<std::string, uint64_t>& t) {
+  take(t, "cb_rmsnorm_fwd", L.rmsnorm_fwd);
+  take(t, "cb_rmsnorm_bwd", L.rmsnorm_bwd);
+  take(t, "cb_norm_bwd_grid", L.norm_bwd_grid);
+  take(t, "cb_glu_fwd_bounded", L.glu_fwd);
+  take(t, "cb_glu_bwd_bounded", L.glu_bwd);
+  take(t, "cb_ce_row_stats", L.row_stats);
+  take(t, "cb_ce_loss", L.ce_loss);
+  take(t, "cb_ce_softmax_grad", L.softmax_grad);
+  take(t, "cb_flash_attn_varlen_fwd", L.flash_varlen_fwd);
+  take(t, "cb_flash_attn_bwd", L.flash_bwd);
+  take(t, "cb_decode_num_splits", L.decode_splits);
+  take(t, "cb_paged_decode_attention", L.decode);
+}
+
+std::map<std::string, long long> counts(bool clear) {
+  std::map<std::string, long long> r;
+  for (Count* c : COUNTS) {
+    const long long n = clear ? c->n.exchange(0) : c->n.load();
+    if (n) r[c->name] = n;
+  }
+  return r;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(cb200_host, m) {
+  using release = py::call_guard<py::gil_scoped_release>;
+  m.def("bind", &bind);
+  m.def("counts", &counts);
+  m.def("rms_norm", [](const Tensor& x, const Tensor& w, double eps) { return RmsNorm::apply(x, w, eps, OptTensor())[0]; }, release());
+  m.def("rms_norm_residual",
+        [](const Tensor& x, const Tensor& w, double eps, const Tensor& r) {
+          const variable_list o = RmsNorm::apply(x, w, eps, OptTensor(r));
+          return std::make_tuple(o[0], o[1]);
+        },
+        release());
+  m.def("glu", [](const Tensor& gu, int64_t act) { return Glu::apply(gu, act); }, release());
+  m.def("cross_entropy",
+        [](const Tensor& x, const Tensor& t, int64_t ignore, int64_t start, int64_t valid, bool mean) {
+          return CrossEntropy::apply(x, t, ignore, start, valid, mean);
+        },
+        release());
+  m.def("packed_attention",
+        [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu, bool causal, double scale) {
+          return PackedAttention::apply(q, k, v, cu, causal, scale);
+        },
+        release());
+  m.def("paged_decode", &paged_decode, release());
+}

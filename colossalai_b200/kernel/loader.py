@@ -3,8 +3,8 @@
 Parity: reference `colossalai/kernel/kernel_loader.py:31-131` + `extensions/{base,cpp,cuda}_extension.py`
 (AOT/JIT build of op families, `KernelLoader.load()`).  B200-first differences:
   * ONE arch: every `.cu` is compiled with `-gencode arch=compute_100a,code=sm_100a -lineinfo`;
-  * kernels export plain C launchers (`extern "C"`, raw pointers + cudaStream_t) and are loaded with ctypes —
-    no torch headers in the CUDA translation units, so a full rebuild takes seconds and the `.so` files live
+  * kernels export plain C launchers (`extern "C"`, raw pointers + cudaStream_t) and are loaded with ctypes, or called
+    from one small torch module for the operators whose host time counts — no torch headers in the CUDA translation units, so a full rebuild takes seconds and the `.so` files live
     IN-TREE (`colossalai_b200/kernel/_build/`) so they travel to the GPU box with the repo snapshot;
   * on a GPU box a missing/unloadable library is a hard error (no silent eager fallback); on a CPU-only box the
     python ops use their torch reference path (the plumbing tier of the test-suite).
@@ -13,9 +13,11 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.util
 import os
 import shutil
 import subprocess
+import sysconfig
 import threading
 from pathlib import Path
 from typing import Dict, List, Optional
@@ -54,6 +56,8 @@ LIBS: Dict[str, dict] = {
     "cb200_mixers": {"sources": ["mixers.cu"], "kind": "cuda", "drop_flags": ["--use_fast_math"]},
     "cb200_cpu_adam": {"sources": ["cpu_adam.cpp"], "kind": "cpp"},
     "cb200_aio": {"sources": ["async_file_io.cpp"], "kind": "cpp", "extra": ["-lpthread"]},
+    # the one library that sees torch: allocation, autograd and launches of the small hot operators (a python module)
+    "cb200_host": {"sources": ["host_ops.cpp"], "kind": "torch"},
 }
 
 
@@ -61,17 +65,26 @@ class _LaunchCounter:
     """Counts launches of OUR kernels (reported by bench.py as `gpu_launches`)."""
 
     def __init__(self) -> None:
-        self.count = 0
-        self.by_name: Dict[str, int] = {}
+        self._by_name: Dict[str, int] = {}
         self.enabled = True
+        self.native = None              # counts of the launches that native code made since the last call
 
     def add(self, name: str, n: int = 1) -> None:
         if self.enabled:
-            self.count += n
-            self.by_name[name] = self.by_name.get(name, 0) + n
+            self._by_name[name] = self._by_name.get(name, 0) + n
+
+    @property
+    def by_name(self) -> Dict[str, int]:
+        if self.native is not None:
+            for name, n in self.native(True).items():
+                self.add(name, n)
+        return self._by_name
+
+    @property
+    def count(self) -> int:
+        return sum(self.by_name.values())
 
     def reset(self) -> None:
-        self.count = 0
         self.by_name.clear()
 
 
@@ -93,10 +106,14 @@ def _src_hash(name: str) -> str:
     for hdr in sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")):
         h.update(hdr.read_bytes())
     h.update(" ".join(_flags(spec)).encode())
+    if spec["kind"] == "torch":
+        h.update(torch.__version__.encode())
     return h.hexdigest()[:16]
 
 
 def _flags(spec: dict) -> List[str]:
+    if spec["kind"] == "torch":
+        return ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
     base = NVCC_FLAGS if spec["kind"] == "cuda" else CXX_FLAGS
     return [f for f in base if f not in spec.get("drop_flags", ())]
 
@@ -130,6 +147,13 @@ def build(name: str, verbose: bool = False, force: bool = False) -> Path:
               ["-o", str(out), "-lcuda"] + spec.get("extra", [])
         # libcuda may be absent on the build box: resolve driver entry points at run time instead
         cmd = [c for c in cmd if c != "-lcuda"]
+    elif spec["kind"] == "torch":
+        root = Path(torch.__file__).resolve().parent
+        cuda = Path(_nvcc() or "/usr/local/cuda/bin/nvcc").resolve().parent.parent
+        inc = [root / "include", root / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
+        cmd = ["g++"] + _flags(spec) + [f"-I{d}" for d in inc] + [f"-DTORCH_EXTENSION_NAME={name}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + srcs + ["-o", str(out), f"-L{root / 'lib'}",
+               "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda", "-ltorch_cuda"]
     else:
         cmd = ["g++"] + _flags(spec) + ["-I", str(CSRC)] + srcs + ["-o", str(out)] + spec.get("extra", [])
     tmp = str(out) + f".tmp{os.getpid()}"
@@ -154,7 +178,7 @@ def build_all(verbose: bool = False, force: bool = False, parallel: int = 8) -> 
 
 def native_available(name: str) -> bool:
     """True when the library can be used for CUDA tensors (GPU present and .so present/buildable)."""
-    if LIBS[name]["kind"] == "cuda" and not torch.cuda.is_available():
+    if LIBS[name]["kind"] != "cpp" and not torch.cuda.is_available():
         return False
     return lib_path(name).exists() or all((CSRC / s).exists() for s in LIBS[name]["sources"])
 
@@ -173,6 +197,40 @@ def load(name: str) -> ctypes.CDLL:
         lib = ctypes.CDLL(str(p), mode=ctypes.RTLD_GLOBAL)
         _loaded[name] = lib
         return lib
+
+
+# launchers that the host module calls, by library
+_HOST_CALLS = {
+    "cb200_norm": ["cb_rmsnorm_fwd", "cb_rmsnorm_bwd", "cb_norm_bwd_grid"],
+    "cb200_elementwise": ["cb_glu_fwd_bounded", "cb_glu_bwd_bounded"],
+    "cb200_loss": ["cb_ce_row_stats", "cb_ce_loss", "cb_ce_softmax_grad"],
+    "cb200_attn": ["cb_flash_attn_varlen_fwd", "cb_flash_attn_bwd"],
+    "cb200_infer": ["cb_decode_num_splits", "cb_paged_decode_attention"],
+}
+_host = None
+
+
+def host():
+    """The native host module (`csrc/host_ops.cpp`), with the kernels' launchers bound."""
+    global _host
+    if _host is None:
+        libs = {lib: load(lib) for lib in _HOST_CALLS}
+        with _lock:
+            if _host is None:
+                p = lib_path("cb200_host")
+                if not p.exists() or (is_stale("cb200_host") and os.environ.get("CB200_NO_REBUILD") != "1"):
+                    try:
+                        build("cb200_host")
+                    except Exception:
+                        if not p.exists():
+                            raise
+                spec = importlib.util.spec_from_file_location("cb200_host", p)
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+                mod.bind({f: ctypes.cast(getattr(libs[lib], f), ctypes.c_void_p).value for lib, fs in _HOST_CALLS.items() for f in fs})
+                launch_counter.native = mod.counts
+                _host = mod
+    return _host
 
 
 class KernelLoader:
@@ -196,7 +254,7 @@ def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def check(err: int, what: str) -> None:

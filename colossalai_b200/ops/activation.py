@@ -12,7 +12,7 @@ import torch
 import torch.nn.functional as F
 
 from ..kernel import loader
-from ._dispatch import use_native
+from ._dispatch import plain_call, use_native
 from ._dtypes import code
 
 _ACT = {"silu": 0, "swiglu": 0, "gelu_tanh": 1, "gelu_new": 1, "gelu_pytorch_tanh": 1, "gelu": 2, "geglu": 2,
@@ -81,6 +81,8 @@ def glu(gate_up: torch.Tensor, act: str = "silu", valid_rows: Optional[torch.Ten
     if use_native(gate_up) and gate_up.dtype in (torch.float32, torch.float16, torch.bfloat16) and I % vec == 0:
         if valid_rows is not None:
             valid_rows = valid_rows.to(device=gate_up.device, dtype=torch.int64).reshape(1).contiguous()
+        elif plain_call(gate_up):
+            return loader.host().glu(gate_up, _ACT[act])
         return _GLUFn.apply(gate_up, _ACT[act], valid_rows)
     return glu_ref(gate_up, act)
 

@@ -13,7 +13,8 @@ from typing import Optional, Tuple
 import torch
 import torch.nn.functional as F
 
-from ._dispatch import use_native
+from ..kernel import loader
+from ._dispatch import plain_call, use_native
 
 __all__ = ["attention", "attention_ref", "attention_with_lse_ref", "AttnMaskType"]
 
@@ -112,5 +113,9 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, batch: int = 1,
         needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
         packed = cu_seqlens_q is not None and (q.shape[-1] == 128 or (q.shape[-1] == 64 and not needs_grad))
         if fa.supported(q, k, v, cu_seqlens_q, cu_seqlens_k, force=packed):
+            if packed and plain_call(q, k, v, cu_seqlens_q) and fa.shapes_ok(q, k, batch, causal, cu_seqlens_q) \
+                    and (not needs_grad or fa.bwd_supported(q, k, batch)):
+                return loader.host().packed_attention(q, k, v, fa._cu32(cu_seqlens_q, q.device), bool(causal),
+                                                      scale if scale is not None else 1.0 / math.sqrt(q.shape[-1]))
             return fa.flash_attention(q, k, v, batch=batch, causal=causal, scale=scale, cu_seqlens_q=cu_seqlens_q)
     return attention_ref(q, k, v, batch, causal, scale, cu_seqlens_q, cu_seqlens_k, attn_mask)

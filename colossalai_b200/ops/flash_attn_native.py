@@ -10,6 +10,7 @@ keeps the native forward but uses the library backward (which only needs q, k, v
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from typing import Optional, Tuple
@@ -35,6 +36,11 @@ def enable(flag: bool = True) -> None:
     _ENABLED = flag
 
 
+@functools.lru_cache(maxsize=None)
+def _major(device: int) -> int:
+    return torch.cuda.get_device_capability(device)[0]
+
+
 def _tensor_ok(t: torch.Tensor) -> bool:
     return t.is_cuda and t.dim() == 3 and t.dtype in (torch.bfloat16, torch.float16) and t.is_contiguous() \
         and t.data_ptr() % 16 == 0
@@ -44,11 +50,11 @@ def supported(q, k, v, cu_seqlens_q=None, cu_seqlens_k=None, force: bool = False
     """Can the native kernels take this call?  Packed batches (`cu_seqlens`) are supported for self attention (the same
     boundaries for queries and keys).  `force` ignores the CB200_FLASH_NATIVE switch (packed batches use the native
     kernels by default: the library path there is a python loop over sequences with a host sync)."""
-    if not (_ENABLED or force) or not torch.cuda.is_available():
+    if not (_ENABLED or force) or not q.is_cuda:
         return False
     if cu_seqlens_q is not None and cu_seqlens_k is not None and cu_seqlens_k is not cu_seqlens_q:
         return False
-    if not (_tensor_ok(q) and _tensor_ok(k) and _tensor_ok(v)) or torch.cuda.get_device_capability()[0] != 10:
+    if not (_tensor_ok(q) and _tensor_ok(k) and _tensor_ok(v)) or _major(torch.cuda.current_device()) != 10:
         return False
     D = q.shape[-1]
     return D in (64, 128) and k.shape[-1] == D and v.shape[-1] == D and q.shape[1] % k.shape[1] == 0 \

@@ -9,7 +9,7 @@ from typing import Optional, Tuple
 import torch
 
 from ..kernel import loader
-from ._dispatch import use_native
+from ._dispatch import plain_call, use_native
 from ._dtypes import code
 
 _lib = None
@@ -42,6 +42,15 @@ def kv_cache_write(k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_ca
     v_cache[blk, slot] = v.to(v_cache.dtype)
 
 
+def _workspace_buffers(q: torch.Tensor):
+    from ..inference.flash_decoding_utils import FDIntermTensors
+
+    fd = FDIntermTensors()
+    if not fd.is_initialized or fd.mid_output.device != q.device or fd.mid_output.dtype != torch.float32:
+        return None, None
+    return fd.mid_output, fd.mid_output_lse
+
+
 def _decode_workspace(q: torch.Tensor, n: int, heads: int, splits: int, head_dim: int):
     """Persistent split-KV buffers (`inference.flash_decoding_utils.FDIntermTensors`) when the engine set them up."""
     from ..inference.flash_decoding_utils import FDIntermTensors
@@ -62,6 +71,9 @@ def paged_decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     if (use_native(q) and q.dtype in (torch.float16, torch.bfloat16) and k_cache.dtype == q.dtype
             and D in (64, 128, 256) and Hq // Hkv <= 8):
+        if plain_call(q, k_cache, v_cache, block_tables, seq_lens, alibi_slopes):
+            ws = _workspace_buffers(q)
+            return loader.host().paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale, alibi_slopes, int(window or 0), *ws)
         lib = _get_lib()
         max_len = block_tables.shape[1] * bs
         part = ctypes.c_int(0)

@@ -12,7 +12,7 @@ from typing import Optional, Tuple
 import torch
 
 from ..kernel import loader
-from ._dispatch import use_native
+from ._dispatch import plain_call, use_native
 from ._dtypes import code
 
 _lib = None
@@ -103,6 +103,11 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
              residual: Optional[torch.Tensor] = None):
     """RMSNorm over the last dim.  With `residual`, returns `(norm(x + residual) * w, x + residual)`."""
     if _native_ok(x, weight):
+        if plain_call(x, weight, residual):
+            if residual is None:
+                return loader.host().rms_norm(x, weight, eps)
+            if residual.dtype == x.dtype and residual.shape == x.shape and residual.device == x.device:
+                return loader.host().rms_norm_residual(x, weight, eps, residual)
         return _RMSNormFn.apply(x, weight, eps, residual)
     return rms_norm_ref(x, weight, eps, residual)
 

@@ -1,0 +1,156 @@
+"""The native host module against the python autograd functions that calls under tracing, modes and subclasses keep: the same
+kernels on the same values, so every result is the same bit for bit - except where atomics order a sum (dQ of attention)."""
+import importlib
+
+import pytest
+import torch
+
+from colossalai_b200 import ops
+from colossalai_b200.kernel import loader
+from colossalai_b200.ops import inference
+from colossalai_b200.shardformer.layer import loss as loss_mod
+
+MODULES = [importlib.import_module("colossalai_b200.ops." + m) for m in ("norm", "activation", "attention", "inference")] + [loss_mod]
+
+
+def test_plain_call_sees_what_watches():
+    from torch.autograd import forward_ad
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from colossalai_b200.ops._dispatch import plain_call
+    from colossalai_b200.tensor import ColoParameter
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, f, types, args=(), kwargs=None):
+            return f(*args, **(kwargs or {}))
+
+    x, seen = torch.randn(3), []
+    assert plain_call(x, None, torch.nn.Parameter(x))
+    assert not plain_call(x, ColoParameter(x.clone()))
+    look = lambda t: (seen.append(plain_call(t)), t + 1)[1]      # noqa: E731
+    torch.func.vmap(look)(x)
+    torch.func.grad(lambda t: look(t).sum())(x)
+    with forward_ad.dual_level():
+        look(x)
+    with Mode():
+        look(x)
+    torch.jit.trace(look, x, check_trace=False)
+    assert seen == [False] * 5 and plain_call(x)
+
+
+def _both(monkeypatch, fn):
+    """fn() on the host module and on the python functions; how many launches each made."""
+    out = []
+    for plain in (None, lambda *a: False):
+        with monkeypatch.context() as m:
+            if plain is not None:
+                for mod in MODULES:
+                    m.setattr(mod, "plain_call", plain)
+            else:
+                loader.host()
+            loader.launch_counter.reset()
+            out.append(fn())
+            torch.cuda.synchronize()
+            out.append(loader.launch_counter.count)
+    assert out[1] == out[3] > 0, "the same kernels on both ways"
+    return out[0], out[2]
+
+
+def _same(a, b):
+    assert len(a) == len(b)
+    for x, y in zip(a, b):
+        assert (x is None) == (y is None)
+        if x is not None:
+            assert x.dtype == y.dtype and x.shape == y.shape and torch.equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 8), (3, 5, 64), (300, 4096)])
+@pytest.mark.parametrize("use", ["both", "norm", "sum", "no_residual"])
+def test_rms_norm(monkeypatch, dtype, shape, use):
+    def fn():
+        torch.manual_seed(0)
+        x = torch.randn(shape[-1:] + shape[:-1], device="cuda", dtype=dtype).movedim(0, -1).requires_grad_()     # strided rows
+        r = torch.randn(shape, device="cuda", dtype=dtype, requires_grad=True)
+        w = torch.nn.Parameter(torch.rand(shape[-1], device="cuda", dtype=dtype))
+        if use == "no_residual":
+            y = ops.rms_norm(x, w, 1e-5)
+            y.backward(torch.randn_like(y))
+            return y.detach(), x.grad, w.grad
+        y, h = ops.rms_norm(x, w, 1e-5, r)
+        outs = {"both": (y, h), "norm": (y,), "sum": (h,)}[use]
+        torch.autograd.backward(outs, [torch.randn(shape, device="cuda").to(dtype) for _ in outs])
+        return y.detach(), h.detach(), x.grad, r.grad, w.grad
+
+    _same(*_both(monkeypatch, fn))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "gelu"])
+def test_glu_saved_tensor_hooks_and_checkpoint(monkeypatch, act):
+    from torch.autograd.graph import saved_tensors_hooks
+    from torch.utils.checkpoint import checkpoint
+
+    def fn():
+        torch.manual_seed(0)
+        gu = torch.randn(2, 7, 48, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+        packed = []
+        with saved_tensors_hooks(lambda t: (packed.append(t.shape), t.cpu())[1], lambda t: t.cuda()):
+            y = ops.glu(gu, act)
+        assert packed
+        (g1,) = torch.autograd.grad(y, gu, torch.ones_like(y))
+        z = checkpoint(lambda t: ops.glu(t, act), gu, use_reentrant=False)
+        (g2,) = torch.autograd.grad(z, gu, torch.ones_like(z))
+        return y.detach(), g1, z.detach(), g2
+
+    _same(*_both(monkeypatch, fn))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["mean", "sum"])
+@pytest.mark.parametrize("vocab", [1000, 1024])
+@pytest.mark.parametrize("labels", [torch.int64, torch.int32])
+def test_cross_entropy(monkeypatch, mode, vocab, labels):
+    def fn():
+        torch.manual_seed(0)
+        x = torch.randn(33, 1024, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+        t = torch.randint(0, vocab, (33,), device="cuda")
+        t[::5] = -100
+        out = loss_mod.cross_entropy_1d(x, t.to(labels), process_group="local", vocab_size=vocab, mode=mode)
+        (g,) = torch.autograd.grad(out * 3, x)
+        return out.detach(), g
+
+    _same(*_both(monkeypatch, fn))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,grad", [(128, True), (128, False), (64, False)])
+def test_packed_attention(monkeypatch, D, grad):
+    def fn():
+        torch.manual_seed(0)
+        q, k, v = (torch.randn(300, h, D, device="cuda", dtype=torch.bfloat16, requires_grad=grad) for h in (8, 2, 2))
+        cu = torch.tensor([0, 7, 7, 200, 300], device="cuda")
+        o = ops.attention(q, k, v, causal=True, cu_seqlens_q=cu, cu_seqlens_k=cu)
+        return (o.detach(),) + (torch.autograd.grad(o, (q, k, v), torch.ones(300, 8, 1, device="cuda").bfloat16().expand(300, 8, D))
+                                if grad else ())
+
+    a, b = _both(monkeypatch, fn)
+    _same(a[:1] + a[2:], b[:1] + b[2:])
+    if grad:
+        torch.testing.assert_close(a[1], b[1], rtol=2 ** -7, atol=2e-3)      # fp32 sums in the order of the reductions
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [64, 256])
+def test_paged_decode(monkeypatch, D):
+    def fn():
+        torch.manual_seed(0)
+        qkv = torch.randn(5, (8 + 4) * D, device="cuda", dtype=torch.float16)
+        kc, vc = (torch.randn(40, 16, 2, D, device="cuda", dtype=torch.float16) for _ in range(2))
+        tables = torch.randperm(40, device="cuda")[:40].view(5, 8).int()
+        lens = torch.tensor([1, 16, 100, 128, 77], device="cuda", dtype=torch.int32)
+        q = qkv[:, : 8 * D].view(5, 8, D)                                         # rows of a wider projection
+        return inference.paged_decode_attention(q, kc, vc, tables, lens, window=50),
+
+    _same(*_both(monkeypatch, fn))
