@@ -48,7 +48,7 @@ struct Launchers {
   int (*rmsnorm_fwd)(const void*, const void*, const void*, void*, void*, float*, int, int, float, int, cudaStream_t);
   int (*rmsnorm_bwd)(const void*, const void*, const void*, const float*, const void*, void*, float*, void*, int, int, int, int,
                      cudaStream_t);
-  int (*norm_bwd_grid)(int);
+  int (*norm_bwd_grid)(int, int, int);
   int (*glu_fwd)(const void*, void*, int64_t, int, int, int, const int64_t*, cudaStream_t);
   int (*glu_bwd)(const void*, const void*, void*, int64_t, int, int, int, const int64_t*, cudaStream_t);
   int (*row_stats)(const void*, const int64_t*, float*, int, int, int, int64_t, int64_t, int, cudaStream_t);
@@ -107,8 +107,8 @@ struct RmsNorm : torch::autograd::Function<RmsNorm> {
     const int H = (int)h.size(-1), rows = H ? (int)(h.numel() / H) : 0;
     const Tensor dy = grads[0].defined() ? grads[0].contiguous() : at::zeros_like(h);
     const Tensor dres = has_res && grads[1].defined() ? grads[1].contiguous() : Tensor();
-    Tensor dx = at::empty_like(h), dw = at::empty_like(weight);
-    Tensor partial = at::empty({(int64_t)L.norm_bwd_grid(rows) * H}, rstd.options());
+    Tensor dx = at::empty_like(h), dw = rows ? at::empty_like(weight) : at::zeros_like(weight);
+    Tensor partial = at::empty({(int64_t)L.norm_bwd_grid(rows, H, code_of(h)) * H}, rstd.options());
     launched(L.rmsnorm_bwd(ptr(dy), ptr(h), ptr(weight), as<float>(rstd), ptr(dres), mut(dx), mut_as<float>(partial), mut(dw), 0, rows, H,
                            code_of(h), stream_of(h)),
              n_norm_bwd, 2);

@@ -88,9 +88,9 @@ class _RMSNormFn(torch.autograd.Function):
         dy2 = dy.contiguous().view(-1, H)
         dres = dh.contiguous().view(-1, H) if (ctx.has_res and dh is not None) else None
         dx = torch.empty_like(h)
-        grid = lib.cb_norm_bwd_grid(rows)
+        grid = lib.cb_norm_bwd_grid(rows, H, code(weight.dtype))
         partial = torch.empty(grid, H, dtype=torch.float32, device=h.device)
-        dw = torch.empty_like(weight)
+        dw = torch.empty_like(weight) if rows else torch.zeros_like(weight)
         loader.check(lib.cb_rmsnorm_bwd(loader.ptr(dy2), loader.ptr(h), loader.ptr(weight), loader.ptr(rstd),
                                         loader.ptr(dres), loader.ptr(dx), loader.ptr(partial), loader.ptr(dw), 0,
                                         rows, H, code(h.dtype), loader.stream_ptr()), "rmsnorm_bwd")
@@ -139,7 +139,7 @@ class _LayerNormFn(torch.autograd.Function):
         rows, H = x2.shape
         dy2 = dy.contiguous().view(-1, H)
         dx = torch.empty_like(x2)
-        grid = lib.cb_norm_bwd_grid(rows)
+        grid = lib.cb_norm_bwd_grid(rows, H, code(weight.dtype))
         pw = torch.empty(grid, H, dtype=torch.float32, device=x2.device)
         pb = torch.empty_like(pw)
         dw = torch.empty_like(weight)
