@@ -51,6 +51,8 @@ struct Launchers {
   int (*norm_bwd_grid)(int, int, int);
   int (*glu_fwd)(const void*, void*, int64_t, int, int, int, const int64_t*, cudaStream_t);
   int (*glu_bwd)(const void*, const void*, void*, int64_t, int, int, int, const int64_t*, cudaStream_t);
+  int (*rope)(const void*, void*, const int64_t*, const float*, const float*, int64_t, int64_t, int, int, int, int, float, int, int,
+              cudaStream_t);
   int (*row_stats)(const void*, const int64_t*, float*, int, int, int, int64_t, int64_t, int, cudaStream_t);
   int (*ce_loss)(const float*, const int64_t*, float*, int64_t*, int, int64_t, int, cudaStream_t);
   int (*softmax_grad)(const void*, const int64_t*, const float*, const float*, const float*, const float*, const int64_t*, void*,
@@ -69,10 +71,10 @@ struct Count {
   const char* name;
   std::atomic<long long> n{0};
 };
-Count n_norm_fwd{"rmsnorm_fwd"}, n_norm_bwd{"rmsnorm_bwd"}, n_glu_fwd{"glu_fwd"}, n_glu_bwd{"glu_bwd"},
+Count n_norm_fwd{"rmsnorm_fwd"}, n_norm_bwd{"rmsnorm_bwd"}, n_glu_fwd{"glu_fwd"}, n_glu_bwd{"glu_bwd"}, n_rope{"rope"},
     n_stats{"ce_row_stats"}, n_loss{"ce_loss"}, n_grad{"ce_softmax_grad"}, n_flash_fwd{"flash_attn_varlen_fwd"},
     n_flash_bwd{"flash_attn_bwd"}, n_decode{"paged_decode_attention"};
-Count* const COUNTS[] = {&n_norm_fwd, &n_norm_bwd, &n_glu_fwd, &n_glu_bwd, &n_stats, &n_loss, &n_grad, &n_flash_fwd, &n_flash_bwd,
+Count* const COUNTS[] = {&n_norm_fwd, &n_norm_bwd, &n_glu_fwd, &n_glu_bwd, &n_rope, &n_stats, &n_loss, &n_grad, &n_flash_fwd, &n_flash_bwd,
                          &n_decode};
 
 void launched(int rc, Count& c, int n = 1) {
@@ -141,6 +143,40 @@ struct Glu : torch::autograd::Function<Glu> {
                        stream_of(gu)),
              n_glu_bwd);
     return {dgu, Tensor()};
+  }
+};
+
+// ------------------------------------------------------------------------------------------------ rotary positions
+// a contiguous tensor of x's shape whose rows are x's with the first heads turned; rows that are strided as wholes are read
+// where they lie
+Tensor rotated(const Tensor& x, const Tensor& pos, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t D, int64_t rot,
+               float sign, bool interleaved) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t vec = 16 / x.element_size();
+  const bool as_is = x.dim() == 2 && x.stride(1) == 1 && x.stride(0) % vec == 0 &&
+                     reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 16 == 0;
+  const Tensor rows = as_is ? x : packed(x);
+  const int64_t T = rows.size(0), width = T ? rows.numel() / T : 0;
+  Tensor out = at::empty(x.sizes(), x.options());
+  launched(L.rope(ptr(rows), mut(out), as<int64_t>(pos), as<float>(cos), as<float>(sin), T, T ? rows.stride(0) : 0, (int)width,
+                  (int)heads, (int)D, (int)rot, sign, interleaved, code_of(x), stream_of(x)),
+           n_rope);
+  return out;
+}
+
+struct Rope : torch::autograd::Function<Rope> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& qkv, const Tensor& pos, const Tensor& cos, const Tensor& sin,
+                        int64_t heads, int64_t D, int64_t rot, bool interleaved) {
+    ctx->save_for_backward({pos, cos, sin});
+    ctx->saved_data["args"] = std::vector<int64_t>{heads, D, rot, (int64_t)interleaved};
+    return rotated(qkv, pos, cos, sin, heads, D, rot, 1.f, interleaved);
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const std::vector<int64_t> a = ctx->saved_data["args"].toIntVector();
+    return {rotated(grads[0], s[0], s[1], s[2], a[0], a[1], a[2], -1.f, a[3] != 0), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(),
+            Tensor(), Tensor()};
   }
 };
 
@@ -251,6 +287,7 @@ void bind(const std::map<std::string, uint64_t>& t) {
   take(t, "cb_norm_bwd_grid", L.norm_bwd_grid);
   take(t, "cb_glu_fwd_bounded", L.glu_fwd);
   take(t, "cb_glu_bwd_bounded", L.glu_bwd);
+  take(t, "cb_rope", L.rope);
   take(t, "cb_ce_row_stats", L.row_stats);
   take(t, "cb_ce_loss", L.ce_loss);
   take(t, "cb_ce_softmax_grad", L.softmax_grad);
@@ -283,6 +320,10 @@ PYBIND11_MODULE(cb200_host, m) {
         },
         release());
   m.def("glu", [](const Tensor& gu, int64_t act) { return Glu::apply(gu, act); }, release());
+  m.def("rope",
+        [](const Tensor& x, const Tensor& pos, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t D, int64_t rot,
+           bool interleaved) { return Rope::apply(x, pos, cos, sin, heads, D, rot, interleaved); },
+        release());
   m.def("cross_entropy",
         [](const Tensor& x, const Tensor& t, int64_t ignore, int64_t start, int64_t valid, bool mean) {
           return CrossEntropy::apply(x, t, ignore, start, valid, mean);

@@ -11,7 +11,7 @@ from typing import Optional, Tuple
 import torch
 
 from ..kernel import loader
-from ._dispatch import use_native
+from ._dispatch import plain_call, use_native
 from ._dtypes import code
 
 _lib = None
@@ -63,36 +63,39 @@ def rope_ref(x: torch.Tensor, positions: Optional[torch.Tensor], cos: torch.Tens
     return torch.cat([out, xp], dim=-1).to(x.dtype)
 
 
-def _native_rope_(qkv2d: torch.Tensor, positions, cos, sin, n_rot_heads: int, D: int, rot_dim: int, sign: float,
-                  interleaved: bool) -> None:
-    lib = _get_lib()
-    loader.check(lib.cb_rope(loader.ptr(qkv2d), loader.ptr(positions), loader.ptr(cos), loader.ptr(sin),
-                             ctypes.c_int64(qkv2d.shape[0]), ctypes.c_int64(qkv2d.stride(0)), n_rot_heads, D,
-                             rot_dim, ctypes.c_float(sign), int(interleaved), code(qkv2d.dtype),
-                             loader.stream_ptr()), "rope")
+def _native_rope(x: torch.Tensor, positions, cos, sin, n_rot_heads: int, D: int, rot_dim: int, sign: float,
+                 interleaved: bool) -> torch.Tensor:
+    """A contiguous tensor of x's shape whose rows are x's with the first heads turned.  Rows that are strided as wholes
+    (a slice of a wider projection, a batch-expanded gradient) are read where they lie; anything else is packed first."""
+    vec = 4 if x.dtype == torch.float32 else 8
+    rows = x if x.dim() == 2 and x.stride(1) == 1 and x.stride(0) % vec == 0 else x.contiguous()
+    if rows.data_ptr() % 16 != 0:                          # a view at an odd offset: 16-byte loads want its copy
+        rows = rows.clone(memory_format=torch.contiguous_format)
+    T = rows.shape[0]
+    width = rows.numel() // max(T, 1)
+    out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    loader.check(_get_lib().cb_rope(loader.ptr(rows), loader.ptr(out), loader.ptr(positions), loader.ptr(cos), loader.ptr(sin),
+                                    ctypes.c_int64(T), ctypes.c_int64(rows.stride(0) if T else 0), width, n_rot_heads, D,
+                                    rot_dim, ctypes.c_float(sign), int(interleaved), code(x.dtype), loader.stream_ptr()), "rope")
     loader.launch_counter.add("rope")
+    return out
 
 
 class _RopeQKVFn(torch.autograd.Function):
-    """Rotates heads [0, n_rot_heads) of every token row of a packed [T, n_heads_total*D] buffer.
-    The forward returns a NEW tensor (one extra write) so autograd never sees an in-place op on a saved tensor;
-    the backward rotates the incoming gradient in place (it is a fresh buffer)."""
+    """Rotates heads [0, n_rot_heads) of every token row of a packed [T, n_heads_total*D] buffer into a NEW tensor (so
+    autograd never sees an in-place op on a saved tensor); the backward turns the incoming gradient back the same way."""
 
     @staticmethod
     def forward(ctx, qkv, positions, cos, sin, n_rot_heads, D, rot_dim, interleaved):
-        out = qkv.clone(memory_format=torch.contiguous_format)
-        _native_rope_(out.view(out.shape[0], -1), positions, cos, sin, n_rot_heads, D, rot_dim, 1.0, interleaved)
         ctx.save_for_backward(positions, cos, sin)
         ctx.cfg = (n_rot_heads, D, rot_dim, interleaved)
-        return out
+        return _native_rope(qkv, positions, cos, sin, n_rot_heads, D, rot_dim, 1.0, interleaved)
 
     @staticmethod
     def backward(ctx, dout):
         positions, cos, sin = ctx.saved_tensors
         n_rot_heads, D, rot_dim, interleaved = ctx.cfg
-        d = dout.contiguous().clone() if not dout.is_contiguous() or dout._base is not None else dout.clone()
-        _native_rope_(d.view(d.shape[0], -1), positions, cos, sin, n_rot_heads, D, rot_dim, -1.0, interleaved)
-        return d, None, None, None, None, None, None, None
+        return (_native_rope(dout, positions, cos, sin, n_rot_heads, D, rot_dim, -1.0, interleaved),) + (None,) * 7
 
 
 def rope_qkv(qkv: torch.Tensor, positions: Optional[torch.Tensor], cos: torch.Tensor, sin: torch.Tensor,
@@ -103,10 +106,14 @@ def rope_qkv(qkv: torch.Tensor, positions: Optional[torch.Tensor], cos: torch.Te
     vec = 4 if qkv.dtype == torch.float32 else 8
     if positions is not None and positions.dtype != torch.int64:
         positions = positions.long()
+    width = qkv.numel() // max(qkv.shape[0], 1)
     if (use_native(qkv) and qkv.dtype in (torch.float32, torch.float16, torch.bfloat16)
-            and (rot // 2) % vec == 0 and head_dim % vec == 0):
+            and (rot // 2) % vec == 0 and head_dim % vec == 0
+            and (qkv.shape[0] == 0 or (width % vec == 0 and (n_q_heads + n_kv_heads) * head_dim <= width))):
         if positions is None:
             positions = torch.arange(qkv.shape[0], device=qkv.device)
+        if plain_call(qkv, positions, cos, sin):
+            return loader.host().rope(qkv, positions.contiguous(), cos, sin, n_q_heads + n_kv_heads, head_dim, rot, interleaved)
         return _RopeQKVFn.apply(qkv, positions.contiguous(), cos, sin, n_q_heads + n_kv_heads, head_dim, rot,
                                 interleaved)
     T = qkv.shape[0]

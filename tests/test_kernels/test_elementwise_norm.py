@@ -115,6 +115,33 @@ def test_rope_qkv(dtype, interleaved, rot):
     torch.testing.assert_close(qkv.grad.float(), qr.grad, **_tol(dtype))
 
 
+@pytest.mark.parametrize("layout", ["packed", "strided", "odd_offset", "expanded_grad"])
+@pytest.mark.parametrize("T,hq,hkv,D,rot,interleaved", [(1, 1, 1, 16, 16, False), (3, 5, 1, 24, 16, True),
+                                                        (2, 33, 3, 96, 64, False), (5, 64, 8, 128, 128, False)])
+def test_rope_row_layouts(layout, T, hq, hkv, D, rot, interleaved):
+    """The rows the one-pass kernel reads where they lie and those it packs first, with an odd number of pass-through
+    vectors and more items than a block has threads: both directions equal the reference's rounding of fp32 values."""
+    torch.manual_seed(1)
+    W = (hq + 2 * hkv) * D
+    base = torch.randn(T * (W + 16) + 8, device="cuda").bfloat16()
+    x = {"strided": base[: T * (W + 16)].view(T, W + 16)[:, 8: 8 + W], "odd_offset": base[3: 3 + T * W].view(T, W)}.get(
+        layout, base[: T * W].view(T, W))
+    x = x.detach().requires_grad_(True)
+    pos = torch.randint(0, 64, (T,), device="cuda")
+    cos, sin = ops.build_rope_cache(64, rot, 10000.0, device="cuda")
+    out = ops.rope_qkv(x, pos, cos, sin, hq, hkv, D, rot_dim=rot, interleaved=interleaved)
+    g = torch.randn(1, 1, device="cuda").bfloat16().expand(T, W) if layout == "expanded_grad" else torch.randn(T, W, device="cuda").bfloat16()
+    out.backward(g)
+
+    def turned(z, sign):
+        z = z.detach().reshape(T, -1, D)
+        return torch.cat([ops.rope_ref(z[:, : hq + hkv], pos, cos, sin * sign, rot, interleaved), z[:, hq + hkv:]], 1).reshape(T, -1)
+
+    # two roundings of the same fp32 value (contracted or not) differ by one step of 2^-8 at most
+    torch.testing.assert_close(out, turned(x, 1), rtol=2 ** -7, atol=1e-6)
+    torch.testing.assert_close(x.grad, turned(g, -1), rtol=2 ** -7, atol=1e-6)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("V,valid,start", [(32000, 32000, 0), (16064, 16000, 16064), (4096, 4096, 8192)])
 def test_cross_entropy_blocks(dtype, V, valid, start):

@@ -10,7 +10,7 @@ from colossalai_b200.kernel import loader
 from colossalai_b200.ops import inference
 from colossalai_b200.shardformer.layer import loss as loss_mod
 
-MODULES = [importlib.import_module("colossalai_b200.ops." + m) for m in ("norm", "activation", "attention", "inference")] + [loss_mod]
+MODULES = [importlib.import_module("colossalai_b200.ops." + m) for m in ("norm", "activation", "attention", "inference", "rope")] + [loss_mod]
 
 
 def test_plain_call_sees_what_watches():
@@ -103,6 +103,19 @@ def test_glu_saved_tensor_hooks_and_checkpoint(monkeypatch, act):
         z = checkpoint(lambda t: ops.glu(t, act), gu, use_reentrant=False)
         (g2,) = torch.autograd.grad(z, gu, torch.ones_like(z))
         return y.detach(), g1, z.detach(), g2
+
+    _same(*_both(monkeypatch, fn))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(0, 24 * 16), (3, 24 * 16), (3, 24, 16)])
+def test_rope(monkeypatch, shape):
+    def fn():
+        torch.manual_seed(0)
+        x = torch.randn(shape, device="cuda", requires_grad=True)
+        pos = torch.arange(shape[0], device="cuda")
+        y = ops.rope_qkv(x, pos, *ops.build_rope_cache(8, 16, 1e4, device="cuda"), 16, 4, 16)
+        return y.detach(), torch.autograd.grad(y, x, torch.ones((), device="cuda").expand(shape))[0]
 
     _same(*_both(monkeypatch, fn))
 
