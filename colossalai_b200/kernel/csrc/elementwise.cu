@@ -36,50 +36,71 @@ template <int ACT> CB_DEVICE float act_grad_f(float x) {
   return ACT == 1 ? gelu_tanh_grad_f(x) : gelu_erf_grad_f(x);
 }
 
+// Gated unit, forward and backward.  A block takes GLU_ITEMS x 256 vectors of one row, so that a thread has all its loads in
+// flight before its first store and no index needs a 64-bit division.
+// Bound: HBM.  8192 x 14336 bf16: one vector per thread of a grid-stride loop 118 us forward (6.0 TB/s) and 189 us backward
+// (6.2); now 102 (6.9) and 169 (7.0).
+// row_limit (device scalar, optional): only the first *row_limit rows hold data - expert-parallel receive buffers are sized
+// for the worst case and the number of rows that actually arrived is only known on the device.
+constexpr int GLU_THREADS = 256;
+constexpr int GLU_ITEMS = 2;
+
 template <typename T, int ACT>
-__global__ void __launch_bounds__(256) glu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out, int64_t rows,
-                                                      int I, const int64_t* __restrict__ row_limit) {
+__global__ void __launch_bounds__(GLU_THREADS) glu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out, int blocks_per_row,
+                                                              int I, const int64_t* __restrict__ row_limit) {
   constexpr int VEC = Vec16<T>::N;
-  // row_limit (device scalar, optional): only the first *row_limit rows hold data - expert-parallel receive buffers are
-  // sized for the worst case and the number of rows that actually arrived is only known on the device
-  if (row_limit != nullptr) rows = min(rows, *row_limit);
-  const int64_t vec_per_row = I / VEC, total = rows * vec_per_row;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = idx / vec_per_row;
-    const int c = (int)(idx - r * vec_per_row) * VEC;
-    Vec16<T> g, u, o;
-    g.load_nc(gu + r * 2 * I + c);
-    u.load_nc(gu + r * 2 * I + I + c);
+  const unsigned r = blockIdx.x / (unsigned)blocks_per_row;
+  if (row_limit != nullptr && (int64_t)r >= *row_limit) return;
+  const int c0 = ((blockIdx.x - r * blocks_per_row) * GLU_THREADS * GLU_ITEMS + threadIdx.x) * VEC;
+  const T* gr = gu + (size_t)r * 2 * I;
+  T* o_r = out + (size_t)r * I;
+  Vec16<T> g[GLU_ITEMS], u[GLU_ITEMS], o;
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) o.set(i, act_f<ACT>(g.get(i)) * u.get(i));
-    o.store_na(out + r * I + c);
+  for (int k = 0; k < GLU_ITEMS; ++k) {
+    const int c = c0 + k * GLU_THREADS * VEC;
+    if (c < I) { g[k].load_nc(gr + c); u[k].load_nc(gr + I + c); }
+  }
+#pragma unroll
+  for (int k = 0; k < GLU_ITEMS; ++k) {
+    const int c = c0 + k * GLU_THREADS * VEC;
+    if (c < I) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) o.set(i, act_f<ACT>(g[k].get(i)) * u[k].get(i));
+      o.store_na(o_r + c);
+    }
   }
 }
 
 template <typename T, int ACT>
-__global__ void __launch_bounds__(256) glu_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ gu,
-                                                      T* __restrict__ dgu, int64_t rows, int I,
-                                                      const int64_t* __restrict__ row_limit) {
+__global__ void __launch_bounds__(GLU_THREADS) glu_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ gu,
+                                                              T* __restrict__ dgu, int blocks_per_row, int I,
+                                                              const int64_t* __restrict__ row_limit) {
   constexpr int VEC = Vec16<T>::N;
-  if (row_limit != nullptr) rows = min(rows, *row_limit);
-  const int64_t vec_per_row = I / VEC, total = rows * vec_per_row;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = idx / vec_per_row;
-    const int c = (int)(idx - r * vec_per_row) * VEC;
-    Vec16<T> g, u, d, dg, du;
-    g.load_nc(gu + r * 2 * I + c);
-    u.load_nc(gu + r * 2 * I + I + c);
-    d.load_nc(dout + r * I + c);
+  const unsigned r = blockIdx.x / (unsigned)blocks_per_row;
+  if (row_limit != nullptr && (int64_t)r >= *row_limit) return;
+  const int c0 = ((blockIdx.x - r * blocks_per_row) * GLU_THREADS * GLU_ITEMS + threadIdx.x) * VEC;
+  const T* gr = gu + (size_t)r * 2 * I;
+  const T* dr = dout + (size_t)r * I;
+  T* or_ = dgu + (size_t)r * 2 * I;
+  Vec16<T> g[GLU_ITEMS], u[GLU_ITEMS], d[GLU_ITEMS], dg, du;
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      const float gf = g.get(i), uf = u.get(i), df = d.get(i);
-      dg.set(i, df * uf * act_grad_f<ACT>(gf));
-      du.set(i, df * act_f<ACT>(gf));
+  for (int k = 0; k < GLU_ITEMS; ++k) {
+    const int c = c0 + k * GLU_THREADS * VEC;
+    if (c < I) { g[k].load_nc(gr + c); u[k].load_nc(gr + I + c); d[k].load_nc(dr + c); }
+  }
+#pragma unroll
+  for (int k = 0; k < GLU_ITEMS; ++k) {
+    const int c = c0 + k * GLU_THREADS * VEC;
+    if (c < I) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) {
+        const float gf = g[k].get(i), uf = u[k].get(i), df = d[k].get(i);
+        dg.set(i, df * uf * act_grad_f<ACT>(gf));
+        du.set(i, df * act_f<ACT>(gf));
+      }
+      dg.store_na(or_ + c);
+      du.store_na(or_ + I + c);
     }
-    dg.store_na(dgu + r * 2 * I + c);
-    du.store_na(dgu + r * 2 * I + I + c);
   }
 }
 
@@ -227,30 +248,29 @@ static inline int ew_grid(int64_t items, int block) {
 
 extern "C" {
 
+#define GLU_LAUNCH(KERNEL, ...)                                                                       \
+  CB_DISPATCH_FLOAT(dtype, T, {                                                                       \
+    const int vecs = I / Vec16<T>::N, per = GLU_THREADS * GLU_ITEMS, bpr = (vecs + per - 1) / per;    \
+    if (rows * bpr > 0x7fffffffll) return (int)cudaErrorInvalidValue;                                 \
+    const unsigned grid = (unsigned)(rows * bpr);                                                     \
+    if (act == 0) KERNEL<T, 0><<<grid, GLU_THREADS, 0, s>>>(__VA_ARGS__, bpr, I, row_limit);          \
+    else if (act == 1) KERNEL<T, 1><<<grid, GLU_THREADS, 0, s>>>(__VA_ARGS__, bpr, I, row_limit);           \
+    else KERNEL<T, 2><<<grid, GLU_THREADS, 0, s>>>(__VA_ARGS__, bpr, I, row_limit);                   \
+  })
+
 int cb_glu_fwd_bounded(const void* gu, void* out, int64_t rows, int I, int act, int dtype, const int64_t* row_limit, cudaStream_t s) {
-  if (rows == 0) return 0;
-  CB_DISPATCH_FLOAT(dtype, T, {
-    const int64_t items = rows * (I / Vec16<T>::N);
-    const int g = ew_grid(items, 256);
-    if (act == 0) glu_fwd_kernel<T, 0><<<g, 256, 0, s>>>((const T*)gu, (T*)out, rows, I, row_limit);
-    else if (act == 1) glu_fwd_kernel<T, 1><<<g, 256, 0, s>>>((const T*)gu, (T*)out, rows, I, row_limit);
-    else glu_fwd_kernel<T, 2><<<g, 256, 0, s>>>((const T*)gu, (T*)out, rows, I, row_limit);
-  });
+  if (rows == 0 || I == 0) return 0;
+  GLU_LAUNCH(glu_fwd_kernel, (const T*)gu, (T*)out);
   return CB_LAUNCH_CHECK();
 }
 
 int cb_glu_bwd_bounded(const void* dout, const void* gu, void* dgu, int64_t rows, int I, int act, int dtype,
-               const int64_t* row_limit, cudaStream_t s) {
-  if (rows == 0) return 0;
-  CB_DISPATCH_FLOAT(dtype, T, {
-    const int64_t items = rows * (I / Vec16<T>::N);
-    const int g = ew_grid(items, 256);
-    if (act == 0) glu_bwd_kernel<T, 0><<<g, 256, 0, s>>>((const T*)dout, (const T*)gu, (T*)dgu, rows, I, row_limit);
-    else if (act == 1) glu_bwd_kernel<T, 1><<<g, 256, 0, s>>>((const T*)dout, (const T*)gu, (T*)dgu, rows, I, row_limit);
-    else glu_bwd_kernel<T, 2><<<g, 256, 0, s>>>((const T*)dout, (const T*)gu, (T*)dgu, rows, I, row_limit);
-  });
+                       const int64_t* row_limit, cudaStream_t s) {
+  if (rows == 0 || I == 0) return 0;
+  GLU_LAUNCH(glu_bwd_kernel, (const T*)dout, (const T*)gu, (T*)dgu);
   return CB_LAUNCH_CHECK();
 }
+#undef GLU_LAUNCH
 
 int cb_glu_fwd(const void* gu, void* out, int64_t rows, int I, int act, int dtype, cudaStream_t s) {
   return cb_glu_fwd_bounded(gu, out, rows, I, act, dtype, nullptr, s);
