@@ -375,17 +375,20 @@ __global__ void __launch_bounds__(128) scan_prepare_kernel(ScanParams p, ScanWor
 
 template <typename T, int VEC> CB_DEVICE void load_vec(const void* p, bool f32, int64_t i, float (&v)[VEC]);
 
-// The same for rows mode on widths and addresses that allow four channels per access (the launcher checks): nothing there
-// needs more of a row than the channel itself, so a thread takes quads of q, k, decay and value channels as they come.
-template <typename T>
-__global__ void __launch_bounds__(256) scan_prepare_rows_vec_kernel(ScanParams p, ScanWork w) {
+// The same for rows and decay mode (without rotation) on widths and addresses that allow four channels per access (the launcher
+// checks): nothing there needs more of a row than the channel itself, so a thread takes quads of q, k, decay and value
+// channels as they come.  Bound: HBM.  12000 tokens of 16 heads x 128 (decay mode, bf16 in): one channel per access 189 us,
+// this 112 us.
+template <typename T, bool ROWS>
+__global__ void __launch_bounds__(256) scan_prepare_vec_kernel(ScanParams p, ScanWork w) {
+  constexpr int SECS = ROWS ? 3 : 2;
   const int64_t t = blockIdx.x;
-  const int dim = p.dim, dq = w.DK / 4, nq = p.heads * dq, vq = w.VP / 4, items = 3 * nq + p.heads * vq;
+  const int dim = p.dim, dq = w.DK / 4, nq = p.heads * dq, vq = w.VP / 4, items = SECS * nq + p.heads * vq;
 #pragma unroll 4
   for (int it = threadIdx.x; it < items; it += 256) {
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     float x[4];
-    if (it < 3 * nq) {
+    if (it < SECS * nq) {
       const int sec = it < nq ? 0 : (it < 2 * nq ? 1 : 2), r = it - sec * nq, h = r / dq, i = r % dq * 4;
       if (sec == 2) {
         o = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -399,14 +402,22 @@ __global__ void __launch_bounds__(256) scan_prepare_rows_vec_kernel(ScanParams p
         const float f = sec == 0 ? p.q_scale : p.k_scale;
         const T* src = sec == 0 ? (const T*)p.q + t * p.ldq : (const T*)p.k + t * p.ldk;
         load_vec<T, 4>(src, false, h * dim + i, x);
+        if (!ROWS && p.act_silu) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[e] = silu_f(x[e]);
+        }
         o = make_float4(x[0] * f, x[1] * f, x[2] * f, x[3] * f);
       }
       float* dst = sec == 0 ? w.q : (sec == 1 ? w.k : w.g);
       *reinterpret_cast<float4*>(dst + (t * p.heads + h) * w.DK + i) = o;
     } else {
-      const int r = it - 3 * nq, h = r / vq, c = r % vq * 4;
+      const int r = it - SECS * nq, h = r / vq, c = r % vq * 4;
       if (c < p.vdim) {
         load_vec<T, 4>((const T*)p.v + t * p.ldv, false, h * p.vdim + c, x);
+        if (!ROWS && p.act_silu) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[e] = silu_f(x[e]);
+        }
         o = make_float4(x[0], x[1], x[2], x[3]);
       }
       *reinterpret_cast<float4*>(w.v + (t * p.heads + h) * w.VP + c) = o;
@@ -481,6 +492,28 @@ __global__ void __launch_bounds__(128) exp_gate_kernel(ScanParams p, ScanWork w,
   if (lane == 0) *mg = m;
 }
 
+// two fp32 operations in one instruction, each rounded as the single one
+CB_DEVICE uint64_t pair_of(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+CB_DEVICE float2 halves(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+CB_DEVICE uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+CB_DEVICE uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 template <int DK, int MODE>
 __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanParams p, ScanWork w) {
   constexpr int PARTS = ScanTile<DK>::PARTS, RP = ScanTile<DK>::RP, RPP = ScanTile<DK>::RPP, DKP = ScanTile<DK>::DKP;
@@ -505,18 +538,26 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
   float* Sg = p.state + ((int64_t)p.slots[s] * p.heads + h) * dim * vdim;
   const bool vec = vdim % 4 == 0 && j0 < vdim;                 // whole quads of columns, 16-byte aligned
   const bool carried = p.ctx_len[s] > 0;
-  float S[RP][SCAN_CPL];
+  // Pairs of neighbouring ROWS share an instruction: q, k and the decays arrive from shared memory as such pairs, and only the
+  // token's SCAN_CPL values are duplicated.
+  uint64_t S[RP / 2][SCAN_CPL];
 #pragma unroll
-  for (int i = 0; i < RP; ++i) {
-    const bool row = carried && r0 + i < dim;
-    const float* src = Sg + (int64_t)(r0 + i) * vdim + j0;
-    if (vec) {
-      const float4 x = row ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
-      S[i][0] = x.x; S[i][1] = x.y; S[i][2] = x.z; S[i][3] = x.w;
-    } else {
+  for (int i = 0; i < RP; i += 2) {
+    float x[2][SCAN_CPL];
 #pragma unroll
-      for (int c = 0; c < SCAN_CPL; ++c) S[i][c] = (row && j0 + c < vdim) ? src[c] : 0.f;
+    for (int e = 0; e < 2; ++e) {
+      const bool row = carried && r0 + i + e < dim;
+      const float* src = Sg + (int64_t)(r0 + i + e) * vdim + j0;
+      if (vec) {
+        const float4 y = row ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[e][0] = y.x; x[e][1] = y.y; x[e][2] = y.z; x[e][3] = y.w;
+      } else {
+#pragma unroll
+        for (int c = 0; c < SCAN_CPL; ++c) x[e][c] = (row && j0 + c < vdim) ? src[c] : 0.f;
+      }
     }
+#pragma unroll
+    for (int c = 0; c < SCAN_CPL; ++c) S[i / 2][c] = pair_of(x[0][c], x[1][c]);
   }
   const float hd = MODE == SCAN_DECAY ? p.head_decay[h] : 0.f;
   const float skip = (MODE == SCAN_GATED && p.head_decay != nullptr) ? p.head_decay[h] : 0.f;
@@ -590,20 +631,24 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
         for (int c = 0; c < SCAN_CPL; ++c) u[c] *= wr;
       }
       if (MODE == SCAN_DELTA) {
-        float a[SCAN_CPL] = {0.f, 0.f, 0.f, 0.f};
+        uint64_t a2[SCAN_CPL] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
         for (int i = 0; i < RP; i += 4) {
-          const float4 g4 = *reinterpret_cast<const float4*>(gq + i);
-          const float4 k4 = *reinterpret_cast<const float4*>(kq + i);
-          const float gr[4] = {g4.x, g4.y, g4.z, g4.w}, kr[4] = {k4.x, k4.y, k4.z, k4.w};
+          const ulonglong2 g4 = *reinterpret_cast<const ulonglong2*>(gq + i);
+          const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kq + i);
+          const uint64_t gr[2] = {g4.x, g4.y}, kr[2] = {k4.x, k4.y};
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
+          for (int e = 0; e < 2; ++e)
 #pragma unroll
             for (int c = 0; c < SCAN_CPL; ++c) {
-              S[i + e][c] *= gr[e];
-              a[c] = fmaf(S[i + e][c], kr[e], a[c]);
+              uint64_t& x = S[i / 2 + e][c];
+              x = mul2(x, gr[e]);
+              a2[c] = fma2(x, kr[e], a2[c]);
             }
         }
+        float a[SCAN_CPL];
+#pragma unroll
+        for (int c = 0; c < SCAN_CPL; ++c) { const float2 h = halves(a2[c]); a[c] = h.x + h.y; }
         // every lane of a column group corrects one column, then collects the quad's four
         const float mine = sbeta[tt] * (sv[tt * SCAN_COLS + c0 + (part & 3)] - join_quads(fold(a)));
         const float nb = __shfl_xor_sync(ALL, mine, 1);
@@ -611,21 +656,29 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
         const float xl = __shfl_xor_sync(ALL, lo, 2), xh = __shfl_xor_sync(ALL, hi, 2);
         u[0] = b1 ? xl : lo; u[1] = b1 ? xh : hi; u[2] = b1 ? lo : xl; u[3] = b1 ? hi : xh;
       }
-      float o[SCAN_CPL] = {0.f, 0.f, 0.f, 0.f};
+      uint64_t o2[SCAN_CPL] = {0ull, 0ull, 0ull, 0ull}, u2[SCAN_CPL];
+#pragma unroll
+      for (int c = 0; c < SCAN_CPL; ++c) u2[c] = pair_of(u[c], u[c]);
+      const uint64_t dec2 = pair_of(dec, dec);
 #pragma unroll
       for (int i = 0; i < RP; i += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(kq + i);
-        const float4 q4 = *reinterpret_cast<const float4*>(qq + i);
-        const float4 g4 = MODE == SCAN_ROWS ? *reinterpret_cast<const float4*>(gq + i) : make_float4(dec, dec, dec, dec);
-        const float gr[4] = {g4.x, g4.y, g4.z, g4.w}, kr[4] = {k4.x, k4.y, k4.z, k4.w}, qr[4] = {q4.x, q4.y, q4.z, q4.w};
+        const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kq + i);
+        const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qq + i);
+        ulonglong2 g4 = make_ulonglong2(dec2, dec2);
+        if (MODE == SCAN_ROWS) g4 = *reinterpret_cast<const ulonglong2*>(gq + i);
+        const uint64_t gr[2] = {g4.x, g4.y}, kr[2] = {k4.x, k4.y}, qr[2] = {q4.x, q4.y};
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+        for (int e = 0; e < 2; ++e)
 #pragma unroll
           for (int c = 0; c < SCAN_CPL; ++c) {
-            S[i + e][c] = MODE == SCAN_DELTA ? fmaf(kr[e], u[c], S[i + e][c]) : fmaf(gr[e], S[i + e][c], kr[e] * u[c]);
-            o[c] = fmaf(S[i + e][c], qr[e], o[c]);
+            uint64_t& x = S[i / 2 + e][c];
+            x = MODE == SCAN_DELTA ? fma2(kr[e], u2[c], x) : fma2(gr[e], x, mul2(kr[e], u2[c]));
+            o2[c] = fma2(x, qr[e], o2[c]);
           }
       }
+      float o[SCAN_CPL];
+#pragma unroll
+      for (int c = 0; c < SCAN_CPL; ++c) { const float2 h = halves(o2[c]); o[c] = h.x + h.y; }
       return fold(o);
     };
     auto emit = [&](int tt, float o) {           // column (part & 3) of token tt's read-out
@@ -660,17 +713,23 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
     __syncthreads();                            // this stage may be refilled in the next pass
   }
 #pragma unroll
-  for (int i = 0; i < RP; ++i)
-    if (r0 + i < dim) {
-      float* dst = Sg + (int64_t)(r0 + i) * vdim + j0;
-      if (vec) {
-        *reinterpret_cast<float4*>(dst) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
-      } else {
+  for (int i = 0; i < RP; i += 2) {
+    float2 x[SCAN_CPL];
 #pragma unroll
-        for (int c = 0; c < SCAN_CPL; ++c)
-          if (j0 + c < vdim) dst[c] = S[i][c];
+    for (int c = 0; c < SCAN_CPL; ++c) x[c] = halves(S[i / 2][c]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (r0 + i + e < dim) {
+        float* dst = Sg + (int64_t)(r0 + i + e) * vdim + j0;
+        if (vec) {
+          *reinterpret_cast<float4*>(dst) = e ? make_float4(x[0].y, x[1].y, x[2].y, x[3].y) : make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
+        } else {
+#pragma unroll
+          for (int c = 0; c < SCAN_CPL; ++c)
+            if (j0 + c < vdim) dst[c] = e ? x[c].y : x[c].x;
+        }
       }
-    }
+  }
 }
 
 template <int DK, int MODE> int launch_scan_dk(const ScanParams& p, const ScanWork& w, int nseq, cudaStream_t st) {
@@ -705,10 +764,13 @@ int launch_scan(const ScanParams& p, float* work, int64_t tokens, int nseq, cuda
   w.gw = w.beta;
   w.v = w.beta + (MODE == SCAN_DELTA ? (tokens * p.heads + 3) / 4 * 4 : (MODE == SCAN_GATED ? tokens * p.heads * 4 : 0));
   auto quads = [](const void* q, int64_t ld, size_t es) { return ld % 4 == 0 && ((uintptr_t)q % (4 * es)) == 0; };
-  if (MODE == SCAN_ROWS && !p.act_silu && !p.unit_qk && p.rot_table == nullptr && p.heads == p.qk_heads && p.dim % 4 == 0 &&
-      p.vdim % 4 == 0 && quads(p.q, p.ldq, sizeof(T)) && quads(p.k, p.ldk, sizeof(T)) && quads(p.v, p.ldv, sizeof(T)) &&
-      quads(p.araw, p.lda, 4) && quads(p.dt_bias, 0, 4) && quads(work, 0, 4))
-    scan_prepare_rows_vec_kernel<T><<<(unsigned)tokens, 256, 0, st>>>(p, w);
+  const bool no_row_math = !p.unit_qk && p.rot_table == nullptr && p.heads == p.qk_heads && p.dim % 4 == 0 && p.vdim % 4 == 0 &&
+                           quads(p.q, p.ldq, sizeof(T)) && quads(p.k, p.ldk, sizeof(T)) && quads(p.v, p.ldv, sizeof(T)) &&
+                           quads(work, 0, 4);
+  if (MODE == SCAN_ROWS && !p.act_silu && no_row_math && quads(p.araw, p.lda, 4) && quads(p.dt_bias, 0, 4))
+    scan_prepare_vec_kernel<T, true><<<(unsigned)tokens, 256, 0, st>>>(p, w);
+  else if (MODE == SCAN_DECAY && no_row_math)
+    scan_prepare_vec_kernel<T, false><<<(unsigned)tokens, 256, 0, st>>>(p, w);
   else
     scan_prepare_kernel<MODE, T><<<(unsigned)tokens, 128, 0, st>>>(p, w);
   if (MODE == SCAN_GATED && p.gate_kind == GATE_EXP) {
