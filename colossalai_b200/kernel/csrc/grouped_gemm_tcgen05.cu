@@ -37,9 +37,18 @@ constexpr int MAX_GROUPS = 512;
 constexpr int A_BYTES = 128 * BK * 2;
 constexpr int B_BYTES = 128 * BK * 2;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + (MAX_GROUPS + 1) * 4;
-
 enum { MODE_NT = 0, MODE_NN = 1, MODE_TN = 2 };
+// behind the barriers: the tile list (variable-M modes) or the staging of the epilogue (weight gradients, two 32 x 64 boxes per
+// epilogue warp)
+constexpr int BOX_BYTES = 32 * 128;
+template <int MODE> constexpr int smem_bytes() {
+  return STAGES * STAGE_BYTES + 1024 + (MODE == MODE_TN ? 256 + 4 * 2 * BOX_BYTES : 256 + (MAX_GROUPS + 1) * 4);
+}
+
+SM100_DEVICE void tma_store_3d(const CUtensorMap* map, const void* smem_src, int32_t c0, int32_t c1, int32_t c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+               :: "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
 
 struct GroupedParams {
   const int* offs;          // [E] cumulative row ends
@@ -51,6 +60,7 @@ struct GroupedParams {
   int b_group_rows;         // NT: N rows per expert in the [E * N, K] view of W; NN: K rows per expert in [E * K, N]
   int out_dtype;
   int accumulate;
+  int tma_store;            // TN: 16-bit results that overwrite leave through shared memory and TMA
   uint32_t idesc;
   void* C;
 };
@@ -118,14 +128,15 @@ SM100_DEVICE void store32(float* __restrict__ dst, const uint32_t (&acc)[32], in
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                         const GroupedParams p) {
+                         const __grid_constant__ CUtensorMap tmap_c, const GroupedParams p) {
   constexpr bool A_MN = MODE == MODE_TN;
   constexpr bool B_MN = MODE != MODE_NT;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * A_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint8_t* smem_box = smem + STAGES * STAGE_BYTES;                                      // TN: [4 warps][2] boxes, 1024-byte aligned
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_box + (MODE == MODE_TN ? 4 * 2 * BOX_BYTES : 0));
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + STAGES;
   uint64_t* tmem_full = bars + 2 * STAGES;
@@ -295,6 +306,40 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
 #pragma unroll
           for (int i = 0; i < 32; ++i) { v0[i] = 0u; v1[i] = 0u; }
         }
+        if (MODE == MODE_TN && p.tma_store) {
+          // A weight gradient's reduction is an expert's few hundred rows, so the store of a tile costs as much as its product:
+          // sixteen bytes per lane to 32 rows at a time (4096 clocks a tile) bound this mode (two GEMMs of 64 experts x 2048 x
+          // 2816 / 1408, 384 rows each: 672 us; with the TMA store 510).  The 32 x 64 box of a warp goes
+          // through shared memory in the 128-byte swizzle and leaves as one TMA store, clipped at the expert's edges.
+          uint8_t* box = smem_box + ((quarter * 2 + ((c >> 6) & 1)) * BOX_BYTES);
+          if (lane == 0) tma_store_wait_read<1>();           // the store that last read this box has read it
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t* v = j < 4 ? v0 + 8 * j : v1 + 8 * (j - 4);
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float x = __uint_as_float(v[2 * i]), y = __uint_as_float(v[2 * i + 1]);
+              if (p.out_dtype == CB_BF16) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+                w[i] = *reinterpret_cast<const uint32_t*>(&h);
+              } else {
+                const __half2 h = __floats2half2_rn(x, y);
+                w[i] = *reinterpret_cast<const uint32_t*>(&h);
+              }
+            }
+            *reinterpret_cast<uint4*>(box + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            const int m0 = tl.m_blk * PAIR_M + (int)cta_rank * 128 + quarter * 32;
+            if (m0 < p.M && n0 + c < p.N) tma_store_3d(&tmap_c, box, n0 + c, m0, tl.group);
+            tma_store_commit();
+          }
+          continue;
+        }
 #define CB_G_STORE(V, CC)                                                                              \
         {                                                                                              \
           const int n_valid = p.N - (n0 + (CC));                                                       \
@@ -318,6 +363,7 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
+    if (MODE == MODE_TN && p.tma_store && lane == 0) tma_store_wait<0>();
   }
   tc_fence_before();
   cluster_sync();
@@ -325,16 +371,16 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
 }
 
 template <int MODE>
-int launch_grouped(const CUtensorMap& ta, const CUtensorMap& tb, const GroupedParams& p, cudaStream_t stream) {
+int launch_grouped(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GroupedParams& p, cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(grouped_gemm_2cta_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM_BYTES);
+                                         smem_bytes<MODE>());
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
   const int pairs = cb_num_sms() / 2;      // the number of tiles is only known on the device: full persistent grid
-  grouped_gemm_2cta_kernel<MODE><<<2 * pairs, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
+  grouped_gemm_2cta_kernel<MODE><<<2 * pairs, NUM_THREADS, smem_bytes<MODE>(), stream>>>(ta, tb, tc, p);
   return (int)cudaGetLastError();
 }
 
@@ -363,13 +409,13 @@ int cb_grouped_gemm(const void* x, const void* w, void* y, const int* offs, int 
     if (r) return 2000 + r;
     p.b_group_rows = N;
     p.idesc = make_idesc_f16(PAIR_M, PAIR_N, bf16 ? 1 : 0, 0, 0);
-    return launch_grouped<MODE_NT>(ta, tb, p, stream);
+    return launch_grouped<MODE_NT>(ta, tb, ta, p, stream);
   }
   r = make_tmap_2d_16b(&tb, w, (uint64_t)E * K, N, N, BK, 64, bf16);
   if (r) return 2000 + r;
   p.b_group_rows = K;
   p.idesc = make_idesc_f16(PAIR_M, PAIR_N, bf16 ? 1 : 0, 0, 1);
-  return launch_grouped<MODE_NN>(ta, tb, p, stream);
+  return launch_grouped<MODE_NN>(ta, tb, ta, p, stream);
 }
 
 // Variable-K grouped GEMM (weight gradients): dw[e] [M, N] (+)= dy[rows of e, M]^T x[rows of e, N].  Every group's row
@@ -388,7 +434,13 @@ int cb_grouped_gemm_wgrad(const void* dy, const void* x, void* dw, const int* of
   p.offs = offs; p.E = E; p.total_rows = total_rows; p.M = M; p.N = N; p.K = 0; p.ldc = N;
   p.c_group_stride = (long long)M * N; p.out_dtype = out_dtype; p.accumulate = accumulate; p.C = dw;
   p.idesc = make_idesc_f16(PAIR_M, PAIR_N, bf16 ? 1 : 0, 1, 1);
-  return launch_grouped<MODE_TN>(ta, tb, p, stream);
+  CUtensorMap tc = ta;
+  p.tma_store = out_dtype != CB_F32 && !accumulate && (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
+  if (p.tma_store) {
+    r = make_tmap_3d_16b(&tc, dw, N, M, E, N, (uint64_t)M * N, 64, 32, 1, out_dtype == CB_BF16);
+    if (r) return 3000 + r;
+  }
+  return launch_grouped<MODE_TN>(ta, tb, tc, p, stream);
 }
 
 }  // extern "C"
