@@ -211,6 +211,22 @@ def test_dist_cross_entropy_matches_torch():
     torch.testing.assert_close(logits.grad.float(), lr.grad, atol=1e-5, rtol=5e-2)
 
 
+@pytest.mark.parametrize("I", [8, 24, 1408, 4096, 4104, 14336])
+@pytest.mark.parametrize("act", ["silu", "gelu"])
+def test_glu_row_parts(I, act):
+    """Rows narrower than a block, of one part exactly, of one vector more, of several: forward and both gradients."""
+    torch.manual_seed(I)
+    x = torch.randn(3, 2 * I, device="cuda").bfloat16().requires_grad_(True)
+    xr = x.detach().float().requires_grad_(True)
+    a, b = xr.chunk(2, -1)
+    ref = (torch.nn.functional.silu(a) if act == "silu" else torch.nn.functional.gelu(a)) * b
+    y, g = ops.glu(x, act), torch.randn(3, I, device="cuda").bfloat16()
+    y.backward(g)
+    ref.backward(g.float())
+    torch.testing.assert_close(y.float(), ref, rtol=2 ** -7, atol=1e-5)      # one rounding to bf16, fast exponentials
+    torch.testing.assert_close(x.grad.float(), xr.grad, rtol=2 ** -7, atol=1e-5)
+
+
 def test_glu_row_limit():
     """`valid_rows`: rows past the device-side limit are neither read nor written, forward and backward."""
     import torch
