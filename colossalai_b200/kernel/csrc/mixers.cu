@@ -49,6 +49,8 @@
 //   cb_head_rmsnorm         RMS norm per head with a weight over the head's channels (query heads | key heads); optionally
 //                           the normed key heads go straight into the paged key cache and the un-normed ones into the
 //                           value cache
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -255,16 +257,28 @@ struct ScanParams {
 // value columns of one (sequence, head); a lane holds a tile of S, RP rows x SCAN_CPL columns, in registers, so that a value
 // of q, k or the decay that is read from shared memory serves SCAN_CPL columns; PARTS adjacent lanes share the rows of a
 // column group, and S^T k and S^T q are partial sums per lane joined by shuffles in a fixed order.
-// The workspace rows of SCAN_TOK_TILE tokens arrive by cp.async in a two-stage ring while the previous tile is walked.
+// The workspace rows of SCAN_TOK_TILE tokens arrive by cp.async in a ring of stages while the previous tile is walked (decay
+// mode has three, so that one barrier per tile is enough).
+// Bound: the serial chain of a sequence, shared-memory reads (q and k once per SCAN_CPL columns) and fp32 issue, none of them
+// alone.  12000 tokens in eight sequences, 16 heads, 128 x 128, decay mode: recurrence 741 -> 505 us.
 constexpr int SCAN_CPL = 4;            // value columns per lane
 constexpr int SCAN_COLS = 32;          // value columns per CTA
 
-template <int DK> struct ScanTile {
-  static constexpr int PARTS = DK <= 16 ? 4 : DK <= 128 ? 8 : 16;       // lanes that share the rows of a column group
+template <int DK, int MODE> struct ScanTile {
+  // Lanes that share the rows of a column group.  More lanes are shorter steps for each and more warps to hide them behind, at
+  // more shuffles and reads of the values.  Decay mode, 16 heads, 12000 tokens, with 8 and with 16 lanes: 128 x 128, one
+  // sequence 2.55 and 1.62 ms, eight 740 and 611 us; 64 x 64, eight sequences 378 and 272 us (32 lanes: 1.68 ms, 785 us).
+  static constexpr int PARTS = DK <= 16 ? 4 : DK <= (MODE == SCAN_DECAY ? 32 : 128) ? 8 : 16;
   static constexpr int RP = DK / PARTS;                                 // rows per lane
   static constexpr int RPP = RP == 4 ? 4 : RP + 4;                      // a lane's rows in shared memory start this far apart:
   static constexpr int DKP = PARTS * RPP;                               // the 16-byte reads of 8 lanes hit different banks
   static constexpr int THREADS = PARTS * SCAN_COLS / SCAN_CPL;
+  // Units that an SM is to hold at a time, by their registers: four tokens' reads want more than 128 of a lane (611 us as
+  // above, 692 at 128 and at 255, where an SM holds two of the 128 wide units and eight sequences take two rounds).
+  static constexpr int BLOCKS = MODE != SCAN_DECAY || DK > 128 ? 1 : (DK == 128 ? 384 : 512) / THREADS;
+  static constexpr int STAGES = MODE == SCAN_DECAY ? 3 : 2;
+  static constexpr int NROW = MODE == SCAN_DELTA || MODE == SCAN_ROWS ? 3 : 2;          // q, k, decay rows
+  static constexpr int TOKEN = NROW * DKP + SCAN_COLS + 4;              // floats per token: rows, values, scalars
 };
 
 struct ScanWork {
@@ -383,13 +397,14 @@ template <typename T, bool ROWS>
 __global__ void __launch_bounds__(256) scan_prepare_vec_kernel(ScanParams p, ScanWork w) {
   constexpr int SECS = ROWS ? 3 : 2;
   const int64_t t = blockIdx.x;
-  const int dim = p.dim, dq = w.DK / 4, nq = p.heads * dq, vq = w.VP / 4, items = SECS * nq + p.heads * vq;
+  const int dim = p.dim, dq_log = __popc(w.DK / 4 - 1), nq = p.heads << dq_log, vq = w.VP / 4, items = SECS * nq + p.heads * vq;
+  const bool whole = p.vdim == w.VP;
 #pragma unroll 4
   for (int it = threadIdx.x; it < items; it += 256) {
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     float x[4];
     if (it < SECS * nq) {
-      const int sec = it < nq ? 0 : (it < 2 * nq ? 1 : 2), r = it - sec * nq, h = r / dq, i = r % dq * 4;
+      const int sec = it < nq ? 0 : (it < 2 * nq ? 1 : 2), r = it - sec * nq, h = r >> dq_log, i = (r - (h << dq_log)) * 4;
       if (sec == 2) {
         o = make_float4(1.f, 1.f, 1.f, 1.f);
         if (i < dim) {
@@ -409,10 +424,10 @@ __global__ void __launch_bounds__(256) scan_prepare_vec_kernel(ScanParams p, Sca
         o = make_float4(x[0] * f, x[1] * f, x[2] * f, x[3] * f);
       }
       float* dst = sec == 0 ? w.q : (sec == 1 ? w.k : w.g);
-      *reinterpret_cast<float4*>(dst + (t * p.heads + h) * w.DK + i) = o;
+      *reinterpret_cast<float4*>(dst + t * p.heads * w.DK + r * 4) = o;
     } else {
-      const int r = it - SECS * nq, h = r / vq, c = r % vq * 4;
-      if (c < p.vdim) {
+      const int r = it - SECS * nq, h = whole ? 0 : r / vq, c = (r - h * vq) * 4;      // value rows without padding are one
+      if (whole || c < p.vdim) {
         load_vec<T, 4>((const T*)p.v + t * p.ldv, false, h * p.vdim + c, x);
         if (!ROWS && p.act_silu) {
 #pragma unroll
@@ -420,7 +435,7 @@ __global__ void __launch_bounds__(256) scan_prepare_vec_kernel(ScanParams p, Sca
         }
         o = make_float4(x[0], x[1], x[2], x[3]);
       }
-      *reinterpret_cast<float4*>(w.v + (t * p.heads + h) * w.VP + c) = o;
+      *reinterpret_cast<float4*>(w.v + t * p.heads * w.VP + r * 4) = o;
     }
   }
 }
@@ -514,19 +529,44 @@ CB_DEVICE uint64_t mul2(uint64_t a, uint64_t b) {
   return r;
 }
 
+// The sequence and the unit of it (head and block of columns; `units` per sequence) that a CTA walks.  A unit takes as long as
+// its sequence, and all are resident at once in a usual step, so what a step takes is the SM with the most tokens.  Up to 32
+// sequences are dealt out by length, longest first and every second row of one CTA per SM the other way round; a row that
+// does not fill lands on the SMs that drew short ones before.  More sequences are many more units than fit: they come in order.
+CB_DEVICE void scan_unit(const ScanParams& p, int nseq, int units, int sms, int& s, int& unit) {
+  int rank = blockIdx.x;
+  if (nseq == 1 || nseq > 32) {
+    s = rank / units;
+    unit = rank - s * units;
+    return;
+  }
+  const int row = rank / sms, width = min(sms, (int)gridDim.x - row * sms);
+  if (!(row & 1)) rank = row * sms + width - 1 - (rank - row * sms);
+  const int lane = threadIdx.x & 31, want = rank / units;
+  unit = rank - want * units;
+  const int len = lane < nseq ? p.cu_q[lane + 1] - p.cu_q[lane] : -1;
+  int place = 0;
+  for (int i = 0; i < nseq; ++i) {
+    const int other = __shfl_sync(0xffffffffu, len, i);
+    place += other > len || (other == len && i < lane);
+  }
+  s = __ffs(__ballot_sync(0xffffffffu, lane < nseq && place == want)) - 1;
+}
+
 template <int DK, int MODE>
-__global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanParams p, ScanWork w) {
-  constexpr int PARTS = ScanTile<DK>::PARTS, RP = ScanTile<DK>::RP, RPP = ScanTile<DK>::RPP, DKP = ScanTile<DK>::DKP;
-  constexpr int THREADS = ScanTile<DK>::THREADS;
+__global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE>::BLOCKS) state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
+  constexpr int PARTS = ScanTile<DK, MODE>::PARTS, RP = ScanTile<DK, MODE>::RP, RPP = ScanTile<DK, MODE>::RPP, DKP = ScanTile<DK, MODE>::DKP;
+  constexpr int THREADS = ScanTile<DK, MODE>::THREADS;
   constexpr bool ROWS = MODE == SCAN_DELTA || MODE == SCAN_ROWS;        // decay rows beside q and k
-  constexpr int NROW = ROWS ? 3 : 2;
-  constexpr int STAGE = SCAN_TOK_TILE * (NROW * DKP + SCAN_COLS + 4);   // floats per stage
+  constexpr int NROW = ScanTile<DK, MODE>::NROW, STAGES = ScanTile<DK, MODE>::STAGES;
+  constexpr int STAGE = SCAN_TOK_TILE * ScanTile<DK, MODE>::TOKEN;      // floats per stage
   constexpr int NTOK = PARTS / SCAN_CPL;                                // tokens whose sums are exchanged together
   constexpr unsigned ALL = 0xffffffffu;
   extern __shared__ __align__(16) float scan_smem[];
   const int vblocks = w.VP / SCAN_COLS;
-  const int h = blockIdx.x / vblocks, vb = blockIdx.x % vblocks;
-  const int s = blockIdx.y;
+  int s, unit;
+  scan_unit(p, nseq, p.heads * vblocks, sms, s, unit);
+  const int h = unit / vblocks, vb = unit % vblocks;
   const int t0 = p.cu_q[s], t1 = p.cu_q[s + 1];
   if (t0 >= t1) return;
   const int part = threadIdx.x % PARTS;
@@ -560,24 +600,63 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
     for (int c = 0; c < SCAN_CPL; ++c) S[i / 2][c] = pair_of(x[0][c], x[1][c]);
   }
   const float hd = MODE == SCAN_DECAY ? p.head_decay[h] : 0.f;
+  // Decay mode holds S / hd^i during a full tile: what token i adds is divided by hd^(i + 1), what it reads multiplied by it,
+  // and the next tile's first token scales S back, so that every other one takes two instructions per pair of rows instead of
+  // three.  The powers are held in two parts: a rounded factor would put the same error on everything it scales, tile after
+  // tile.  S is rounded once per token as before.  Decays below a quarter (S would grow by more than 2^16 inside a tile) and
+  // above one keep the plain form, and so does a part of a tile: a decoder's single token would be scaled there and back.  A
+  // lane of the 16 wide kernel has too few rows for it to pay (4096 tokens x 8 heads x 16 x 64: 59 us plain, 73 scaled).
+  __shared__ float4 powers[SCAN_TOK_TILE + 1];                 // hd^i and hd^-i, each as value and remainder
+  const bool scale_tiles = MODE == SCAN_DECAY && DK > 16 && hd >= 0.25f && hd <= 1.f;
+  if (scale_tiles && threadIdx.x <= SCAN_TOK_TILE) {           // read behind a barrier
+    double f = 1.0;
+    for (int i = 0; i < threadIdx.x; ++i) f *= (double)hd;
+    const float a = (float)f, b = (float)(1.0 / f);
+    powers[threadIdx.x] = make_float4(a, (float)(f - a), b, (float)(1.0 / f - b));
+  }
+  float back = 1.f, back_low = 0.f;                            // S is held divided by this
+  auto scale_back = [&]() {
+    const uint64_t f2 = pair_of(back, back), l2 = pair_of(back_low, back_low);
+#pragma unroll
+    for (int i = 0; i < RP / 2; ++i)
+#pragma unroll
+      for (int c = 0; c < SCAN_CPL; ++c) S[i][c] = fma2(S[i][c], f2, mul2(S[i][c], l2));
+    back = 1.f;
+    back_low = 0.f;
+  };
+
   const float skip = (MODE == SCAN_GATED && p.head_decay != nullptr) ? p.head_decay[h] : 0.f;
 
-  auto load_tile = [&](int stage, int tb) {
+  // A thread copies the same 16-byte piece of every (THREADS / pieces)-th token: its addresses only step, which keeps the
+  // copies to three instructions each (with an address computed per copy they were a tenth of what the kernel issued).
+  constexpr int CH = DK / 4, TPI = THREADS / CH, VCH = SCAN_COLS / 4, VPI = THREADS / VCH;
+  static_assert(THREADS % CH == 0 && TPI <= SCAN_TOK_TILE && THREADS % VCH == 0, "");
+  const int qt = threadIdx.x / CH, qc = (threadIdx.x % CH) * 4, vt = threadIdx.x / VCH, vc = (threadIdx.x % VCH) * 4;
+  const int qdst = qt * DKP + qc / RP * RPP + qc % RP, vdst = NROW * SCAN_TOK_TILE * DKP + vt * SCAN_COLS + vc;
+  const int64_t qstep = (int64_t)p.qk_heads * DK, gstep = (int64_t)p.heads * DK, vstep = (int64_t)p.heads * w.VP;
+  const float* qsrc = w.q + (t0 + qt) * qstep + hk * DK + qc;
+  const float* ksrc = w.k + (t0 + qt) * qstep + hk * DK + qc;
+  const float* gsrc = ROWS ? w.g + (t0 + qt) * gstep + h * DK + qc : nullptr;
+  const float* vsrc = w.v + (t0 + vt) * vstep + h * w.VP + vb * SCAN_COLS + vc;
+  auto load_tile = [&](int stage, int tb) {      // tiles are asked for in order
     float* base = scan_smem + stage * STAGE;
-    const int nt = min(SCAN_TOK_TILE, t1 - tb);
-    constexpr int CH = DK / 4;
-    for (int idx = threadIdx.x; idx < nt * CH; idx += THREADS) {
-      const int tt = idx / CH, c = (idx % CH) * 4;
-      const int dst = tt * DKP + c / RP * RPP + c % RP;
-      const int64_t t = tb + tt;
-      cp_async16f(base + dst, w.q + (t * p.qk_heads + hk) * DK + c);
-      cp_async16f(base + SCAN_TOK_TILE * DKP + dst, w.k + (t * p.qk_heads + hk) * DK + c);
-      if (ROWS) cp_async16f(base + 2 * SCAN_TOK_TILE * DKP + dst, w.g + (t * p.heads + h) * DK + c);
+    const int nt = max(min(SCAN_TOK_TILE, t1 - tb), 0);
+#pragma unroll
+    for (int i = 0; i < SCAN_TOK_TILE; i += TPI) {
+      if (qt + i < nt) {
+        cp_async16f(base + qdst + i * DKP, qsrc);
+        cp_async16f(base + SCAN_TOK_TILE * DKP + qdst + i * DKP, ksrc);
+        if (ROWS) cp_async16f(base + 2 * SCAN_TOK_TILE * DKP + qdst + i * DKP, gsrc);
+      }
+      qsrc += TPI * qstep;
+      ksrc += TPI * qstep;
+      if (ROWS) gsrc += TPI * gstep;
     }
     float* sv = base + NROW * SCAN_TOK_TILE * DKP;
-    for (int idx = threadIdx.x; idx < nt * (SCAN_COLS / 4); idx += THREADS) {
-      const int tt = idx / (SCAN_COLS / 4), c = (idx % (SCAN_COLS / 4)) * 4;
-      cp_async16f(sv + tt * SCAN_COLS + c, w.v + ((int64_t)(tb + tt) * p.heads + h) * w.VP + vb * SCAN_COLS + c);
+#pragma unroll
+    for (int i = 0; i < SCAN_TOK_TILE; i += VPI) {
+      if (vt + i < nt) cp_async16f(base + vdst + i * SCAN_COLS, vsrc);
+      vsrc += (VPI < SCAN_TOK_TILE ? VPI : SCAN_TOK_TILE) * vstep;
     }
     if (MODE == SCAN_DELTA && threadIdx.x < nt)
       sv[SCAN_TOK_TILE * SCAN_COLS + threadIdx.x] = w.beta[(int64_t)(tb + threadIdx.x) * p.heads + h];
@@ -597,27 +676,41 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
   auto join_quads = [&](float v) -> float {
     if (PARTS >= 8) v += __shfl_xor_sync(ALL, v, 4);
     if (PARTS >= 16) v += __shfl_xor_sync(ALL, v, 8);
+    if (PARTS >= 32) v += __shfl_xor_sync(ALL, v, 16);
     return v;
   };
 
+  if (MODE == SCAN_DECAY) __syncthreads();      // the powers
   load_tile(0, t0);
+  if (STAGES == 3) load_tile(1, t0 + SCAN_TOK_TILE);
   int stage = 0;
-  for (int tb = t0; tb < t1; tb += SCAN_TOK_TILE, stage ^= 1) {
+  for (int tb = t0; tb < t1; tb += SCAN_TOK_TILE, stage = stage + 1 == STAGES ? 0 : stage + 1) {
     const int nt = min(SCAN_TOK_TILE, t1 - tb);
-    if (tb + SCAN_TOK_TILE < t1) {              // the other stage was released by the barrier that ended the last pass
-      load_tile(stage ^ 1, tb + SCAN_TOK_TILE);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const bool scaled_tile = scale_tiles && nt == SCAN_TOK_TILE;
+    // a tile past the portion's end is an empty group
+    if (STAGES == 2) load_tile(stage ^ 1, tb + SCAN_TOK_TILE);    // released by the barrier that ended the last pass
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (MODE == SCAN_DECAY) {
+#pragma unroll
+      for (int i = 0; i < SCAN_TOK_TILE; i += VPI)          // a thread scales the values that it copied itself
+        if (vt + i < nt && scaled_tile) {
+          float4* values = reinterpret_cast<float4*>(scan_smem + stage * STAGE + vdst + i * SCAN_COLS);
+          const float4 f = powers[vt + i + 1], x = *values;
+          *values = make_float4(fmaf(x.x, f.z, x.x * f.w), fmaf(x.y, f.z, x.y * f.w), fmaf(x.z, f.z, x.z * f.w),
+                                fmaf(x.w, f.z, x.w * f.w));
+        }
     }
     __syncthreads();
+    // three stages: the tile before last was left by everyone who passed this barrier
+    if (STAGES == 3) load_tile(stage == 0 ? 2 : stage - 1, tb + 2 * SCAN_TOK_TILE);
     const float* sq = scan_smem + stage * STAGE;
     const float* sk = sq + SCAN_TOK_TILE * DKP;
     const float* sg = sk + SCAN_TOK_TILE * DKP;
     const float* sv = sq + NROW * SCAN_TOK_TILE * DKP;
     const float* sbeta = sv + SCAN_TOK_TILE * SCAN_COLS;
     // one token: the lane's part of S is advanced; returns column (part & 3) of the read-out joined over the lane's quad
-    auto advance = [&](int tt) -> float {
+    auto advance = [&](int tt, auto scaled, auto first) -> float {
+      constexpr bool SCALED = decltype(scaled)::value, FIRST = decltype(first)::value;
       const float4 v4 = *reinterpret_cast<const float4*>(sv + tt * SCAN_COLS + c0);
       float u[SCAN_CPL] = {v4.x, v4.y, v4.z, v4.w};
       const float* kq = sk + tt * DKP + r0p;
@@ -659,7 +752,8 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
       uint64_t o2[SCAN_CPL] = {0ull, 0ull, 0ull, 0ull}, u2[SCAN_CPL];
 #pragma unroll
       for (int c = 0; c < SCAN_CPL; ++c) u2[c] = pair_of(u[c], u[c]);
-      const uint64_t dec2 = pair_of(dec, dec);
+      if (SCALED) dec = back;
+      const uint64_t dec2 = pair_of(dec, dec), low2 = pair_of(back_low, back_low);
 #pragma unroll
       for (int i = 0; i < RP; i += 4) {
         const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kq + i);
@@ -672,7 +766,8 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
 #pragma unroll
           for (int c = 0; c < SCAN_CPL; ++c) {
             uint64_t& x = S[i / 2 + e][c];
-            x = MODE == SCAN_DELTA ? fma2(kr[e], u2[c], x) : fma2(gr[e], x, mul2(kr[e], u2[c]));
+            if (MODE == SCAN_DELTA || (SCALED && !FIRST)) x = fma2(kr[e], u2[c], x);
+            else x = fma2(gr[e], x, SCALED ? fma2(low2, x, mul2(kr[e], u2[c])) : mul2(kr[e], u2[c]));
             o2[c] = fma2(x, qr[e], o2[c]);
           }
       }
@@ -689,29 +784,39 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
     // NTOK tokens at a time: only S ties them together, so their loads and sums overlap; the quads exchange their sums so
     // that quad n ends up with token n's total (the same pairs in the same order as one token alone takes: the result does
     // not depend on how a portion falls into groups)
-    int tt = 0;
-#pragma unroll 2
-    for (; tt + NTOK <= nt; tt += NTOK) {        // every lane takes part in the shuffles, also for a padded column
+    auto group = [&](int tt, auto scaled, auto first) {      // every lane takes part in the shuffles, also for a padded column
       float v[NTOK];
 #pragma unroll
-      for (int n = 0; n < NTOK; ++n) v[n] = advance(tt + n);
-      if (NTOK == 4) {
-        const bool q0 = part & 4, q1 = part & 8;
-        const float x = (q0 ? v[1 % NTOK] : v[0]) + __shfl_xor_sync(ALL, q0 ? v[0] : v[1 % NTOK], 4);
-        const float y = (q0 ? v[3 % NTOK] : v[2 % NTOK]) + __shfl_xor_sync(ALL, q0 ? v[2 % NTOK] : v[3 % NTOK], 4);
-        v[0] = (q1 ? y : x) + __shfl_xor_sync(ALL, q1 ? x : y, 8);
-      } else if (NTOK == 2) {
-        const bool q0 = part & 4;
-        v[0] = (q0 ? v[1 % NTOK] : v[0]) + __shfl_xor_sync(ALL, q0 ? v[0] : v[1 % NTOK], 4);
+      for (int n = 0; n < NTOK; ++n) v[n] = n == 0 ? advance(tt, scaled, first) : advance(tt + n, scaled, std::false_type());
+#pragma unroll
+      for (int m = NTOK / 2, bit = 4; m >= 1; m /= 2, bit *= 2) {
+        const bool up = part & bit;
+#pragma unroll
+        for (int n = 0; n < m; ++n) v[n] = (up ? v[2 * n + 1] : v[2 * n]) + __shfl_xor_sync(ALL, up ? v[2 * n] : v[2 * n + 1], bit);
       }
-      emit(tt + part / SCAN_CPL, v[0]);
+      tt += part / SCAN_CPL;
+      if (decltype(scaled)::value) v[0] = fmaf(v[0], powers[tt + 1].x, v[0] * powers[tt + 1].y);
+      emit(tt, v[0]);
+    };
+    if (MODE == SCAN_DECAY && scaled_tile) {
+      group(0, std::true_type(), std::true_type());
+#pragma unroll
+      for (int tt = NTOK; tt < SCAN_TOK_TILE; tt += NTOK) group(tt, std::true_type(), std::false_type());
+      back = powers[SCAN_TOK_TILE].x;
+      back_low = powers[SCAN_TOK_TILE].y;
+    } else {
+      if (MODE == SCAN_DECAY && scale_tiles) scale_back();
+      int tt = 0;
+#pragma unroll 2
+      for (; tt + NTOK <= nt; tt += NTOK) group(tt, std::false_type(), std::false_type());
+      for (; tt < nt; ++tt) {
+        const float o = join_quads(advance(tt, std::false_type(), std::false_type()));
+        if (part < SCAN_CPL) emit(tt, o);
+      }
     }
-    for (; tt < nt; ++tt) {
-      const float o = join_quads(advance(tt));
-      if (part < SCAN_CPL) emit(tt, o);
-    }
-    __syncthreads();                            // this stage may be refilled in the next pass
+    if (STAGES == 2) __syncthreads();           // this stage may be refilled in the next pass
   }
+  if (MODE == SCAN_DECAY && scale_tiles) scale_back();
 #pragma unroll
   for (int i = 0; i < RP; i += 2) {
     float2 x[SCAN_CPL];
@@ -733,8 +838,7 @@ __global__ void __launch_bounds__(ScanTile<DK>::THREADS) state_scan_kernel(ScanP
 }
 
 template <int DK, int MODE> int launch_scan_dk(const ScanParams& p, const ScanWork& w, int nseq, cudaStream_t st) {
-  constexpr int NROW = MODE == SCAN_DELTA || MODE == SCAN_ROWS ? 3 : 2;
-  const size_t smem = (size_t)2 * SCAN_TOK_TILE * (NROW * ScanTile<DK>::DKP + SCAN_COLS + 4) * sizeof(float);
+  const size_t smem = (size_t)ScanTile<DK, MODE>::STAGES * SCAN_TOK_TILE * ScanTile<DK, MODE>::TOKEN * sizeof(float);
   auto kern = state_scan_kernel<DK, MODE>;
   static bool configured = false;
   if (!configured) {
@@ -742,8 +846,7 @@ template <int DK, int MODE> int launch_scan_dk(const ScanParams& p, const ScanWo
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     configured = true;
   }
-  dim3 grid(p.heads * (w.VP / SCAN_COLS), nseq);
-  kern<<<grid, ScanTile<DK>::THREADS, smem, st>>>(p, w);
+  kern<<<p.heads * (w.VP / SCAN_COLS) * nseq, ScanTile<DK, MODE>::THREADS, smem, st>>>(p, w, nseq, cb_num_sms());
   return CB_LAUNCH_CHECK();
 }
 

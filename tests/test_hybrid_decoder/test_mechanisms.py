@@ -87,6 +87,45 @@ def test_decay_scan_matches_token_by_token(device, H, d, dv):
     _close(torch.cat(outs), want, 2e-5)
 
 
+@pytest.mark.parametrize("device", DEVICES)
+@pytest.mark.parametrize("d,dv", [(64, 40), (128, 32), (200, 36)])
+@pytest.mark.parametrize("lens", [[8], [7, 24, 0, 9, 1, 16, 33], [1 + i % 9 for i in range(34)]])
+def test_decay_scan_tiles_and_unit_order(device, d, dv, lens):
+    """Whole tiles of eight tokens, parts of one, sequences without tokens, few and more than 32 sequences, fresh and carried;
+    decays on both sides of the range in which a tile is held scaled."""
+    dev, H = _dev(device), 6
+    g = torch.Generator().manual_seed(d + len(lens))
+    decay = torch.tensor([0.0, 0.2, 0.25, 0.6, 1.0, 1.02])
+    T, n = sum(lens), len(lens)
+    q, k, v = (torch.randn(T, H * w, generator=g) for w in (d, d, dv))
+    state = torch.randn(n, H, d, dv, generator=g)
+    ctx = [5 * (i % 2) for i in range(n)]
+    slots = list(reversed(range(n)))
+    out_s, want, want_mag, ends = state.to(dev), [], [], []
+    at = 0
+    for i, m in enumerate(lens):
+        S = state[slots[i]].double() if ctx[i] and m else torch.zeros(H, d, dv, dtype=torch.float64)
+        A = S.abs()
+        for t in range(at, at + m):
+            kk, vv, qq = (x[t].double().view(H, -1) for x in (k, v, q))
+            S = decay.double()[:, None, None] * S + kk[:, :, None] * vv[:, None, :]
+            A = decay.double()[:, None, None] * A + (kk[:, :, None] * vv[:, None, :]).abs()
+            want.append(torch.einsum("hdv,hd->hv", S, qq).flatten())
+            want_mag.append(torch.einsum("hdv,hd->hv", A, qq.abs()).flatten())
+        ends.append((slots[i], S, A, m))
+        at += m
+    meta = M.RaggedMeta.build(lens, ctx, slots, dev)
+    out = M.state_scan_decay(q.to(dev), k.to(dev), v.to(dev), decay.to(dev), out_s, meta, H, d, dv, act_silu=False)
+    # fp32 sums of d products over states that at most 33 tokens rounded twice each
+    eps = (d + 2 * 33) * 2.0 ** -24
+    assert bool(((out.double().cpu() - torch.stack(want)).abs() <= eps * torch.stack(want_mag) + 1e-12).all())
+    for slot, S, A, m in ends:
+        if m:
+            assert bool(((out_s[slot].double().cpu() - S).abs() <= 2 * 33 * 2.0 ** -24 * A + 1e-12).all())
+        else:
+            assert torch.equal(out_s[slot].cpu(), state[slot])
+
+
 def _delta_inputs(L, H, G, d, dv, seed):
     g = torch.Generator().manual_seed(seed)
     q, k = torch.randn(L, G * d, generator=g), torch.randn(L, G * d, generator=g)
