@@ -81,10 +81,13 @@ SM100_DEVICE void raster(int local, int m_blocks, int n_blocks, int& m_blk, int&
 }
 
 // tile_start[e] = number of row tiles of groups < e (variable-M modes).  `cur` caches the last group found: tiles are
-// visited in increasing order by every role, so the search is amortised O(1).
+// visited in increasing order by every role, so the search is amortised O(1).  Every role looks its tiles up one ahead: the
+// bounds of a group come from memory, and a tile is too short to wait for them (both forward GEMMs of the layer below 409 -> 401
+// us, their gradients 421 -> 405).
 template <int MODE>
-SM100_DEVICE Tile find_tile(int t, const GroupedParams& p, const int* tile_start, int n_blocks, int& cur) {
-  Tile r;
+SM100_DEVICE Tile find_tile(int t, int num_tiles, const GroupedParams& p, const int* tile_start, int n_blocks, int& cur) {
+  Tile r{};
+  if (t >= num_tiles) return r;
   if (MODE == MODE_TN) {
     const int per_group = ((p.M + PAIR_M - 1) / PAIR_M) * n_blocks;
     r.group = t / per_group;
@@ -195,8 +198,10 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     // ================================================================ TMA producer (both CTAs)
     int stage = 0, cur = 0;
     uint32_t phase = 0;
+    Tile ahead = find_tile<MODE>(pair_id, num_tiles, p, tile_start, n_blocks, cur);
     for (int t = pair_id; t < num_tiles; t += num_pairs) {
-      const Tile tl = find_tile<MODE>(t, p, tile_start, n_blocks, cur);
+      const Tile tl = ahead;
+      ahead = find_tile<MODE>(t + num_pairs, num_tiles, p, tile_start, n_blocks, cur);
       int k_blocks, kbase;
       if (MODE == MODE_TN) { k_blocks = (tl.row_end - tl.row0 + BK - 1) / BK; kbase = tl.row0; }
       else { k_blocks = (p.K + BK - 1) / BK; kbase = 0; }
@@ -242,8 +247,10 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       uint32_t phase = 0, acc_phase = 0;
       constexpr uint32_t a_kstep = A_MN ? UMMA_K * 128 : UMMA_K * 2;
       constexpr uint32_t b_kstep = B_MN ? UMMA_K * 128 : UMMA_K * 2;
+      Tile ahead = find_tile<MODE>(pair_id, num_tiles, p, tile_start, n_blocks, cur);
       for (int t = pair_id; t < num_tiles; t += num_pairs) {
-        const Tile tl = find_tile<MODE>(t, p, tile_start, n_blocks, cur);
+        const Tile tl = ahead;
+        ahead = find_tile<MODE>(t + num_pairs, num_tiles, p, tile_start, n_blocks, cur);
         const int k_blocks = MODE == MODE_TN ? (tl.row_end - tl.row0 + BK - 1) / BK : (p.K + BK - 1) / BK;
         mbar_wait(&tmem_empty[acc], acc_phase ^ 1);
         tc_fence_after();
@@ -278,8 +285,10 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     const int quarter = warp & 3;
     int acc = 0, cur = 0;
     uint32_t acc_phase = 0;
+    Tile ahead = find_tile<MODE>(pair_id, num_tiles, p, tile_start, n_blocks, cur);
     for (int t = pair_id; t < num_tiles; t += num_pairs) {
-      const Tile tl = find_tile<MODE>(t, p, tile_start, n_blocks, cur);
+      const Tile tl = ahead;
+      ahead = find_tile<MODE>(t + num_pairs, num_tiles, p, tile_start, n_blocks, cur);
       const int in_tile = (int)cta_rank * 128 + quarter * 32 + lane;
       int row, row_lim;
       size_t base;
@@ -296,31 +305,41 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       mbar_wait(&tmem_full[acc], acc_phase);
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * PAIR_N + ((uint32_t)(quarter * 32) << 16);
-#pragma unroll 1
-      for (int c = 0; c < PAIR_N; c += 64) {
-        uint32_t v0[32], v1[32];
-        tmem_ld_32x32b_x32(taddr + c, v0);
-        tmem_ld_32x32b_x32(taddr + c + 32, v1);
-        tmem_ld_wait();
-        if (empty_k) {
+      if (MODE == MODE_TN && p.tma_store) {
+        // A weight gradient's reduction is an expert's few hundred rows, so the store of a tile costs as much as its product:
+        // sixteen bytes per lane to 32 rows at a time (4096 clocks a tile) bound this mode (two GEMMs of 64 experts x 2048 x
+        // 2816 / 1408, 384 rows each: 672 us; with the TMA store 510, with the next box read while one is packed 501).
+        // The 32 x 64 box of a warp goes through shared memory in the 128-byte swizzle and leaves as one TMA store, clipped at
+        // the expert's edges.  The accumulator is free when its last box is in registers.
+        uint32_t v[2][64];
+        tmem_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&v[0][0]));
+        tmem_ld_32x32b_x32(taddr + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[0][32]));
 #pragma unroll
-          for (int i = 0; i < 32; ++i) { v0[i] = 0u; v1[i] = 0u; }
-        }
-        if (MODE == MODE_TN && p.tma_store) {
-          // A weight gradient's reduction is an expert's few hundred rows, so the store of a tile costs as much as its product:
-          // sixteen bytes per lane to 32 rows at a time (4096 clocks a tile) bound this mode (two GEMMs of 64 experts x 2048 x
-          // 2816 / 1408, 384 rows each: 672 us; with the TMA store 510).  The 32 x 64 box of a warp goes
-          // through shared memory in the 128-byte swizzle and leaves as one TMA store, clipped at the expert's edges.
-          uint8_t* box = smem_box + ((quarter * 2 + ((c >> 6) & 1)) * BOX_BYTES);
+        for (int b = 0; b < PAIR_N / 64; ++b) {
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 64; ++i) asm volatile("" : "+r"(v[b & 1][i]));                  // nothing reads them earlier
+          if (b + 1 < PAIR_N / 64) {
+            tmem_ld_32x32b_x32(taddr + (b + 1) * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[(b + 1) & 1][0]));
+            tmem_ld_32x32b_x32(taddr + (b + 1) * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[(b + 1) & 1][32]));
+          } else {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              if (leader) mbar_arrive(&tmem_empty[acc]);
+              else mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
+            }
+          }
+          uint8_t* box = smem_box + ((quarter * 2 + (b & 1)) * BOX_BYTES);
           if (lane == 0) tma_store_wait_read<1>();           // the store that last read this box has read it
           __syncwarp();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const uint32_t* v = j < 4 ? v0 + 8 * j : v1 + 8 * (j - 4);
             uint32_t w[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const float x = __uint_as_float(v[2 * i]), y = __uint_as_float(v[2 * i + 1]);
+              const float x = empty_k ? 0.f : __uint_as_float(v[b & 1][8 * j + 2 * i]);
+              const float y = empty_k ? 0.f : __uint_as_float(v[b & 1][8 * j + 2 * i + 1]);
               if (p.out_dtype == CB_BF16) {
                 const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
                 w[i] = *reinterpret_cast<const uint32_t*>(&h);
@@ -335,10 +354,23 @@ grouped_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           __syncwarp();
           if (lane == 0) {
             const int m0 = tl.m_blk * PAIR_M + (int)cta_rank * 128 + quarter * 32;
-            if (m0 < p.M && n0 + c < p.N) tma_store_3d(&tmap_c, box, n0 + c, m0, tl.group);
+            if (m0 < p.M && n0 + b * 64 < p.N) tma_store_3d(&tmap_c, box, n0 + b * 64, m0, tl.group);
             tma_store_commit();
           }
-          continue;
+        }
+        acc ^= 1;
+        if (acc == 0) acc_phase ^= 1;
+        continue;
+      }
+#pragma unroll 1
+      for (int c = 0; c < PAIR_N; c += 64) {
+        uint32_t v0[32], v1[32];
+        tmem_ld_32x32b_x32(taddr + c, v0);
+        tmem_ld_32x32b_x32(taddr + c + 32, v1);
+        tmem_ld_wait();
+        if (empty_k) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) { v0[i] = 0u; v1[i] = 0u; }
         }
 #define CB_G_STORE(V, CC)                                                                              \
         {                                                                                              \
