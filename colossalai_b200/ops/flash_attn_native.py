@@ -1,6 +1,6 @@
-"""ctypes face of the sm_100a flash-attention kernels (`kernel/csrc/flash_attn_tcgen05.cu`): tcgen05 forward (validated
-on a B200 in round 2: 17/17 numerics cases) and tcgen05 backward (dK / dV accumulated in TMEM per key tile over the whole
-GQA group, dQ through fp32 reductions).
+"""ctypes face of the sm_100a flash-attention kernels (`kernel/csrc/flash_attn_tcgen05.cu`): tcgen05 forward (persistent, two
+query tiles per unit) and tcgen05 backward (dK / dV accumulated in TMEM per key tile over the whole GQA group, dQ through fp32
+reductions).
 
 `CB200_FLASH_NATIVE=1` (or `enable(True)`) routes `ops.attention` and the ring-attention block functions through them
 for equal-length bf16 / fp16 batches (head_dim 64 / 128 forward, 128 backward; sequence length a multiple of 128);
