@@ -227,7 +227,8 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_kernel(
   // sliding-window attention (Mistral): only the last `window` cached tokens are visible - partitions that lie before
   // the window start contribute nothing (m = -inf, l = 0) and are skipped by the merge
   const int window_start = window > 0 ? max(0, len - window) : 0;
-  const int t0 = max(split * part_len, window_start), t1 = min(len, split * part_len + part_len);
+  const int t0 = max(split * part_len, window_start);
+  const int t1 = min(min(len, max_blocks_per_seq * block_size), split * part_len + part_len);   // (no pages beyond the table's row)
   const int g0 = set * GH;
   const int ng = min(GH, G - g0);
   const int grp = lane / LPT, sub = lane - grp * LPT;
@@ -399,6 +400,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_kernel(
 //   * softmax state per head row is replicated over the four lanes of a quad; the probabilities go straight from the
 //     accumulator layout of S to the A-operand layout of P V (no shared-memory round trip); the output accumulator is
 //     rescaled only when a row max moved;
+//   * partial results use the same (o_part, ml_part) format, so the reduce kernel is shared.
 constexpr int DEC_MMA_TOKENS = 16;
 constexpr int DEC_MMA_STAGES = 3;
 
@@ -433,45 +435,12 @@ template <> CB_DEVICE uint32_t pack2<__half>(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// Work split: the visible tokens of all sequences, in tiles of 16, form one list in sequence order; slot c (a CTA per group of
-// kv heads) takes tiles [c W / G, (c + 1) W / G).  All slots have the same share whatever the lengths are, and all are
-// resident at once (two CTAs of four warps per SM): with a grid of equal partitions per sequence, 64 sequences of 1024..2048
-// tokens were 2.2 waves of uneven CTAs (72.7 us, 5.5 TB/s), 16 of 512..1024 1.8 waves (15.9 us).  The tokens of sequence s
-// that slot c takes are one PIECE; (c, s) walks a staircase, so c + s numbers the pieces.  A sequence in one piece is
-// finished where it is computed, the others are merged by a second kernel.
-constexpr int DEC_MMA_WARPS = 4;
-constexpr int DEC_MIN_TILES = 2;      // smallest share of a slot worth a CTA of its own
-
-struct DecTiles {                     // tiles before sequence s / of all sequences; whole warps
-  int before, mine, total;
-};
-CB_DEVICE int dec_tiles_of(const int* seq_lens, int window, int i) {
-  int len = max(__ldg(seq_lens + i), 0);
-  if (window > 0) len = min(len, window);
-  return (len + DEC_MMA_TOKENS - 1) / DEC_MMA_TOKENS;
-}
-CB_DEVICE int dec_total(const int* seq_lens, int window, int n) {
-  int t = 0;
-  for (int i = threadIdx.x & 31; i < n; i += 32) t += dec_tiles_of(seq_lens, window, i);
-  return __reduce_add_sync(0xffffffffu, t);
-}
-// first and one past the last tile of slot c; slots beyond what DEC_MIN_TILES allows stay empty
-CB_DEVICE int dec_slots(int total, int slots) { return max(1, min(slots, (total + DEC_MIN_TILES - 1) / DEC_MIN_TILES)); }
-CB_DEVICE int dec_bound(int c, int total, int used) { return (int)((int64_t)c * total / used); }
-// the slot that tile `t` belongs to
-CB_DEVICE int dec_slot_of(int t, int total, int used) {
-  int c = (int)(((int64_t)t * used) / max(total, 1));
-  while (c + 1 < used && dec_bound(c + 1, total, used) <= t) ++c;
-  while (c > 0 && dec_bound(c, total, used) > t) --c;
-  return c;
-}
-
 template <typename T, int D>
-__global__ void __launch_bounds__(DEC_MMA_WARPS * 32, 2) paged_decode_mma_kernel(
+__global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
     const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
     const int* __restrict__ block_tables, const int* __restrict__ seq_lens, float* __restrict__ o_part,
-    float* __restrict__ ml_part, int2* __restrict__ pieces, T* __restrict__ out, int num_seqs, int Hq, int Hkv, int block_size,
-    int max_blocks_per_seq, float scale, const float* __restrict__ alibi_slopes, int64_t q_stride, int64_t out_stride, int window) {
+    float* __restrict__ ml_part, int Hq, int Hkv, int block_size, int max_blocks_per_seq, int splits, int part_len,
+    float scale, const float* __restrict__ alibi_slopes, int64_t q_stride, int window) {
   constexpr int NT = DEC_MMA_TOKENS, NST = DEC_MMA_STAGES;
   constexpr int KS = D / 16;                    // k-steps of Q K^T
   constexpr int NO = D / 8;                     // 8-wide column tiles of the output
@@ -479,64 +448,20 @@ __global__ void __launch_bounds__(DEC_MMA_WARPS * 32, 2) paged_decode_mma_kernel
   constexpr int ROW_BYTES = D * 2;
   constexpr int TILE_BYTES = NT * ROW_BYTES;    // one operand (K or V) of one stage
   constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+  const int seq = blockIdx.x, split = blockIdx.z;
   const int G = Hq / Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.y * (blockDim.x >> 5) + warp;
-  const int slot = blockIdx.x;
   if (kvh >= Hkv) return;                       // (no block-wide barrier in this kernel)
-  const int total = dec_total(seq_lens, window, num_seqs);
-  const int used = dec_slots(total, gridDim.x);
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");    // the merge may take its place on the SMs and wait there
-  if (slot == 0 && kvh == 0) {                  // first slot and number of pieces of every sequence, for the merge
-    int before = 0;
-    for (int s0 = 0; s0 < num_seqs; s0 += 32) {
-      const int mine = s0 + lane < num_seqs ? dec_tiles_of(seq_lens, window, s0 + lane) : 0;
-      int upto = mine;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += y;
-      }
-      if (s0 + lane < num_seqs) {
-        const int first = before + upto - mine;
-        const int c0 = mine > 0 ? dec_slot_of(first, total, used) : 0;
-        pieces[s0 + lane] = make_int2(c0, mine > 0 ? dec_slot_of(first + mine - 1, total, used) - c0 + 1 : 0);
-      }
-      before += __shfl_sync(0xffffffffu, upto, 31);
-    }
-  }
-  if (slot >= used) return;
-  const int w0 = dec_bound(slot, total, used), w1 = dec_bound(slot + 1, total, used);   // this slot's tiles
+  const int len = seq_lens[seq];
+  const int window_start = window > 0 ? max(0, len - window) : 0;
+  const int t0 = max(split * part_len, window_start);
+  const int t1 = min(min(len, max_blocks_per_seq * block_size), split * part_len + part_len);   // (no pages beyond the table's row)
   const int row = lane >> 2, quad = lane & 3;   // accumulator layout: head row, column pair inside an 8-wide tile
   const bool row_ok = row < G;                  // rows G..15 of the MMA are padding
   const float scale2 = scale * LOG2E;           // scores in the exp2 domain
   const float slope2 = (alibi_slopes != nullptr && row_ok) ? alibi_slopes[kvh * G + row] * LOG2E : 0.f;
   const bool has_alibi = alibi_slopes != nullptr;
-  extern __shared__ __align__(128) unsigned char dec_smem[];
-  unsigned char* ring = dec_smem + (size_t)warp * NST * 2 * TILE_BYTES;
-  const int bs_shift = (block_size & (block_size - 1)) == 0 ? 31 - __clz(block_size) : -1;
-
-  int base_tiles = 0;                           // tiles of the sequences in front of the current 32
-  for (int s0 = 0; s0 < num_seqs && base_tiles < w1; s0 += 32) {
-  const int mine = s0 + lane < num_seqs ? dec_tiles_of(seq_lens, window, s0 + lane) : 0;
-  int upto = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, upto, o);
-    if (lane >= o) upto += y;
-  }
-  const int first_tile = base_tiles + upto - mine;
-  unsigned todo = __ballot_sync(0xffffffffu, mine > 0 && first_tile < w1 && first_tile + mine > w0);
-  base_tiles += __shfl_sync(0xffffffffu, upto, 31);
-  for (; todo != 0; todo &= todo - 1) {
-  const int pick = __ffs(todo) - 1;
-  const int seq = s0 + pick;
-  const int seq_tile0 = __shfl_sync(0xffffffffu, first_tile, pick), seq_tiles = __shfl_sync(0xffffffffu, mine, pick);
-  const int len = __ldg(seq_lens + seq);
-  const int window_start = window > 0 ? max(0, len - window) : 0;
-  const int t0 = window_start + max(w0 - seq_tile0, 0) * NT, t1 = min(len, window_start + (w1 - seq_tile0) * NT);
-  const bool whole = w0 <= seq_tile0 && w1 >= seq_tile0 + seq_tiles;
-  const int* bt = block_tables + (int64_t)seq * max_blocks_per_seq;
 
   // ---- Q fragments: A operand [16 heads x 16 d] per k-step; a1 / a3 are head rows 8..15 = zero (G <= 8)
   uint32_t qa[KS][4];
@@ -554,6 +479,10 @@ __global__ void __launch_bounds__(DEC_MMA_WARPS * 32, 2) paged_decode_mma_kernel
   for (int j = 0; j < NO; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
   float m_run = -INFINITY, l_run = 0.f;         // per head row, replicated over the quad (l: this lane's share)
 
+  extern __shared__ __align__(128) unsigned char dec_smem[];
+  unsigned char* ring = dec_smem + (size_t)warp * NST * 2 * TILE_BYTES;
+  const int* bt = block_tables + seq * max_blocks_per_seq;
+  const int bs_shift = (block_size & (block_size - 1)) == 0 ? 31 - __clz(block_size) : -1;
   auto issue_stage = [&](int base, int stage) {
     unsigned char* kt = ring + (size_t)stage * 2 * TILE_BYTES;
     unsigned char* vt = kt + TILE_BYTES;
@@ -658,93 +587,15 @@ __global__ void __launch_bounds__(DEC_MMA_WARPS * 32, 2) paged_decode_mma_kernel
     }
     cp_async_wait<0>();
   }
-  // ---- this piece's result (row sum over the quad first)
+  // ---- this unit's partial result (row sum over the quad first)
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-  if (row_ok && whole) {
-    const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-    T* dst = out + (int64_t)seq * out_stride + (int64_t)(kvh * G + row) * D + quad * 2;
-#pragma unroll
-    for (int j = 0; j < NO; ++j) *reinterpret_cast<uint32_t*>(dst + j * 8) = pack2<T>(o[j][0] * inv, o[j][1] * inv);
-  } else if (row_ok) {
-    const int64_t oi = (int64_t)(slot + seq) * Hq + kvh * G + row;
+  if (row_ok) {
+    const int64_t oi = (((int64_t)seq * Hq + kvh * G + row) * splits + split);
     float* dst = o_part + oi * D + quad * 2;
 #pragma unroll
     for (int j = 0; j < NO; ++j) *reinterpret_cast<float2*>(dst + j * 8) = make_float2(o[j][0], o[j][1]);
     if (quad == 0) { ml_part[oi * 2] = m_run * LN2; ml_part[oi * 2 + 1] = l_run; }
-  }
-  }  // pieces
-  }  // 32 sequences at a time
-}
-
-// Merges the pieces of the sequences that have more than one; one CTA per (sequence, head).  A warp takes every fourth piece
-// with D / 32 columns per lane and a running maximum, so that all loads of a warp are in flight together (one thread per
-// column and a serial loop over the pieces took 8.6 us for 65 of them).  Launched while the main kernel runs; waits for
-// its results before it reads any.
-constexpr int DEC_MERGE_WARPS = 4;
-template <typename T, int D>
-__global__ void __launch_bounds__(DEC_MERGE_WARPS * 32) decode_merge_kernel(const float* __restrict__ o_part,
-                                                                            const float* __restrict__ ml_part,
-                                                                            const int2* __restrict__ pieces, T* __restrict__ out,
-                                                                            int Hq, int64_t out_stride) {
-  constexpr int CPL = D / 32;
-  struct alignas(CPL * 4) Cols { float v[CPL]; };
-  __shared__ float part_s[DEC_MERGE_WARPS][D];
-  __shared__ float2 ml_s[DEC_MERGE_WARPS];
-  const int seq = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int2 pc = pieces[seq];
-  if (pc.y == 1) return;                        // written by the slot that computed it
-  T* dst = out + (int64_t)seq * out_stride + (int64_t)h * D;
-  float acc[CPL], m = -INFINITY, l = 0.f;
-#pragma unroll
-  for (int e = 0; e < CPL; ++e) acc[e] = 0.f;
-  constexpr int U = 8;
-  for (int i0 = warp; i0 < pc.y; i0 += DEC_MERGE_WARPS * U) {
-    Cols o[U];
-    float2 ml[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = i0 + u * DEC_MERGE_WARPS;
-      const int64_t oi = (int64_t)(pc.x + (i < pc.y ? i : i0) + seq) * Hq + h;
-      ml[u] = *reinterpret_cast<const float2*>(ml_part + oi * 2);
-      o[u] = *reinterpret_cast<const Cols*>(o_part + oi * D + lane * CPL);
-      if (i >= pc.y) ml[u] = make_float2(-INFINITY, 0.f);
-    }
-    float mn = m;
-#pragma unroll
-    for (int u = 0; u < U; ++u) mn = fmaxf(mn, ml[u].x);
-    const float f0 = m == -INFINITY ? 0.f : __expf(m - mn);
-    l *= f0;
-#pragma unroll
-    for (int e = 0; e < CPL; ++e) acc[e] *= f0;
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const float f = ml[u].x == -INFINITY ? 0.f : __expf(ml[u].x - mn);
-      l = fmaf(ml[u].y, f, l);
-#pragma unroll
-      for (int e = 0; e < CPL; ++e) acc[e] = f == 0.f ? acc[e] : fmaf(o[u].v[e], f, acc[e]);
-    }
-    m = mn;
-  }
-#pragma unroll
-  for (int e = 0; e < CPL; ++e) part_s[warp][lane * CPL + e] = acc[e];
-  if (lane == 0) ml_s[warp] = make_float2(m, l);
-  __syncthreads();
-  float gm = -INFINITY, ls = 0.f, f[DEC_MERGE_WARPS];
-#pragma unroll
-  for (int w = 0; w < DEC_MERGE_WARPS; ++w) gm = fmaxf(gm, ml_s[w].x);
-#pragma unroll
-  for (int w = 0; w < DEC_MERGE_WARPS; ++w) {
-    f[w] = ml_s[w].x == -INFINITY ? 0.f : __expf(ml_s[w].x - gm);
-    ls = fmaf(ml_s[w].y, f[w], ls);
-  }
-  const float inv = ls > 0.f ? 1.f / ls : 0.f;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float v = 0.f;
-#pragma unroll
-    for (int w = 0; w < DEC_MERGE_WARPS; ++w) v = fmaf(part_s[w][d], f[w], v);
-    dst[d] = from_f32<T>(v * inv);              // no tokens: zeros
   }
 }
 
@@ -844,30 +695,7 @@ int cb_rope_kv_cache_write(void* q, void* k, const void* v, void* k_cache, void*
   return CB_LAUNCH_CHECK();
 }
 
-// The tensor-core kernel takes head_dim 64 / 128 and groups of <= 8 q heads; CB200_DECODE=simt forces the CUDA-core kernel
-// (also used for head_dim 256)
-static bool decode_use_mma(int Hq, int Hkv, int D) {
-  const char* impl_env = getenv("CB200_DECODE");
-  return !(impl_env != nullptr && impl_env[0] == 's') && Hq / Hkv <= 8 && (D == 128 || D == 64);
-}
-static int decode_slots(int num_seqs, int kv_heads, int max_len) {
-  const int warps = kv_heads < DEC_MMA_WARPS ? kv_heads : DEC_MMA_WARPS, groups = (kv_heads + warps - 1) / warps;
-  // CTAs that are resident together: two of four warps (98 KB of shared memory each at head_dim 128) per SM
-  int slots = 2 * cb_num_sms() / groups;
-  const int64_t tiles = (int64_t)num_seqs * ((max_len + DEC_MMA_TOKENS - 1) / DEC_MMA_TOKENS);
-  const int64_t most = (tiles + DEC_MIN_TILES - 1) / DEC_MIN_TILES;
-  if (slots > most) slots = (int)most;
-  return slots < 1 ? 1 : slots;
-}
-
-// Partial results per sequence that the workspaces are sized for (num_seqs * this many); *part_len_out: tokens per partition
-// of the CUDA-core kernel.
-int cb_decode_num_splits(int num_seqs, int Hq, int kv_heads, int D, int max_len, int* part_len_out) {
-  if (num_seqs <= 0 || kv_heads <= 0) { *part_len_out = 0; return 1; }
-  if (decode_use_mma(Hq, kv_heads, D)) {       // pieces are numbered slot + sequence; their numbers per sequence behind them
-    *part_len_out = 0;
-    return (decode_slots(num_seqs, kv_heads, max_len) + num_seqs - 1) / num_seqs + 2;
-  }
+int cb_decode_num_splits(int num_seqs, int kv_heads, int max_len, int* part_len_out) {
   // one CTA (up to 8 warps, one per kv head) per SM: aim at >= 2 waves of CTAs, partitions of >= 64 tokens
   const int ctas_per_split = num_seqs * ((kv_heads + 7) / 8);
   const int target = 2 * cb_num_sms();
@@ -883,7 +711,7 @@ int cb_decode_num_splits(int num_seqs, int Hq, int kv_heads, int D, int max_len,
   return splits;
 }
 
-// q: [num_seqs, Hq, D]; out same; caches [nb, bs, Hkv, D]; o_part fp32 num_seqs * splits rows of Hq * D; ml_part [.., 2]
+// q: [num_seqs, Hq, D]; out same; caches [nb, bs, Hkv, D]; o_part fp32 [num_seqs, Hq, splits, D]; ml_part [.., 2]
 int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_cache, const int* block_tables,
                               const int* seq_lens, void* out, float* o_part, float* ml_part, int num_seqs, int Hq,
                               int Hkv, int D, int block_size, int max_blocks_per_seq, int splits, int part_len,
@@ -897,36 +725,25 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
   dim3 grid(num_seqs, (units + warps - 1) / warps, splits);
   const int dec_smem = warps * DEC_STAGES * (2 * DEC_U * 2 * 32) * 16;                    // per-warp cp.async rings
   constexpr int dec_smem_max = (DEC_THREADS / 32) * DEC_STAGES * (2 * DEC_U * 2 * 32) * 16;
-  const bool use_mma = decode_use_mma(Hq, Hkv, D);
-  const int slots = decode_slots(num_seqs, Hkv, max_blocks_per_seq * block_size);
-  if (use_mma && (int64_t)num_seqs * splits < slots + 2 * num_seqs) return (int)cudaErrorInvalidValue;   // workspaces too small
-  int2* pieces = reinterpret_cast<int2*>(ml_part + (int64_t)(slots + num_seqs) * Hq * 2);   // (8-byte aligned: pairs before it)
-  const int mma_warps = Hkv < DEC_MMA_WARPS ? Hkv : DEC_MMA_WARPS;
-  const dim3 mma_grid(slots, (Hkv + mma_warps - 1) / mma_warps);
+  // default: the tensor-core formulation (mma.sync over the GQA group) where it applies (head_dim 64 / 128, groups of
+  // <= 8 q heads); CB200_DECODE=simt forces the CUDA-core kernel (also used for head_dim 256)
+  const char* impl_env = getenv("CB200_DECODE");
+  const bool use_mma = !(impl_env != nullptr && impl_env[0] == 's') && G <= 8 && (D == 128 || D == 64);
+  const int mma_warps = Hkv < DEC_THREADS / 32 ? Hkv : DEC_THREADS / 32;
+  dim3 mma_grid(num_seqs, (Hkv + mma_warps - 1) / mma_warps, splits);
 #define LAUNCH_DEC_MMA(T, DD)                                                                                       \
   {                                                                                                                  \
     constexpr int per_warp = DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * DD * 2;                                           \
     static bool attr_done = false;                                                                                   \
     if (!attr_done) {                                                                                                \
       cudaFuncSetAttribute(paged_decode_mma_kernel<T, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize,              \
-                           DEC_MMA_WARPS * per_warp);                                                                \
+                           (DEC_THREADS / 32) * per_warp);                                                           \
       attr_done = true;                                                                                              \
     }                                                                                                                \
     paged_decode_mma_kernel<T, DD><<<mma_grid, mma_warps * 32, mma_warps * per_warp, s>>>(                           \
-        (const T*)q, (const T*)k_cache, (const T*)v_cache, block_tables, seq_lens, o_part, ml_part, pieces, (T*)out, \
-        num_seqs, Hq, Hkv, block_size, max_blocks_per_seq, scale, alibi_slopes, q_stride, out_stride, window);      \
-    cudaLaunchConfig_t cfg = {};                                                                                     \
-    cfg.gridDim = dim3(num_seqs, Hq);                                                                                \
-    cfg.blockDim = dim3(DEC_MERGE_WARPS * 32);                                                                       \
-    cfg.stream = s;                                                                                                  \
-    cudaLaunchAttribute at[1];                                                                                       \
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;                                                   \
-    at[0].val.programmaticStreamSerializationAllowed = 1;                                                            \
-    cfg.attrs = at;                                                                                                  \
-    cfg.numAttrs = 1;                                                                                                \
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, decode_merge_kernel<T, DD>, (const float*)o_part,                \
-                                              (const float*)ml_part, (const int2*)pieces, (T*)out, Hq, out_stride);  \
-    if (le != cudaSuccess) return (int)le;                                                                           \
+        (const T*)q, (const T*)k_cache, (const T*)v_cache, block_tables, seq_lens, o_part, ml_part, Hq, Hkv,        \
+        block_size, max_blocks_per_seq, splits, part_len, scale, alibi_slopes, q_stride, window);                   \
+    decode_reduce_kernel<T, DD><<<dim3(num_seqs, Hq), 128, 0, s>>>(o_part, ml_part, (T*)out, Hq, splits, out_stride); \
   }
 #define LAUNCH_DEC(T, DD)                                                                                           \
   {                                                                                                                  \

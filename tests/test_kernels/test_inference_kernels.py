@@ -189,3 +189,26 @@ def test_paged_decode_pieces(lens, Hq, Hkv, D, window):
     if live:
         ref = iops.paged_decode_attention_ref(q.float()[live], kc.float(), vc.float(), tables[live], seq[live], window=window or None)
         torch.testing.assert_close(out[live].float(), ref, atol=2e-2, rtol=2e-2)      # weights rounded to bf16
+
+
+@pytest.mark.parametrize("window", [0, 20, 300])
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("width", [4, 5])
+def test_paged_decode_stops_at_the_page_table(D, window, width):
+    """A length beyond what a row of the page table has room for: what the row holds is attended, and neither the next row's pages
+    nor what lies behind the table is looked at (the row behind holds pages of NaN)."""
+    dev = torch.device("cuda")
+    torch.manual_seed(D + window)
+    n, bs, Hkv = 3, 16, 2
+    kc, vc = (torch.randn(n * width + 1, bs, Hkv, D, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    kc[-1] = vc[-1] = float("nan")
+    tables = torch.full((n + 1, width), n * width, device=dev, dtype=torch.int32)
+    tables[:n] = torch.randperm(n * width, device=dev).view(n, width).int()
+    q = torch.randn(n, 8, D, device=dev, dtype=torch.bfloat16)
+    lens = torch.tensor([width * bs, 5, width * bs + 11], device=dev, dtype=torch.int32)
+    out = iops.paged_decode_attention(q, kc, vc, tables[:n], lens, window=window or None)
+    for i, m in enumerate(lens.tolist()):
+        first, end = max(0, m - window) if window else 0, min(m, width * bs)
+        k, v = (c[tables[i].long()].flatten(0, 1)[first:end].double().repeat_interleave(4, 1) for c in (kc, vc))
+        ref = torch.einsum("hk,khd->hd", (torch.einsum("hd,khd->hk", q[i].double(), k) / D ** 0.5).softmax(-1), v)
+        torch.testing.assert_close(out[i].double(), ref, atol=2e-2, rtol=2e-2)      # weights rounded to bf16
