@@ -54,7 +54,8 @@ def row_stats(logits: torch.Tensor, target: torch.Tensor, vocab_start: int, igno
     local = target - vocab_start
     own = (local >= 0) & (local < Vv) & (target != ignore_index)
     tl = xf.gather(-1, local.clamp(0, Vv - 1).unsqueeze(-1)).squeeze(-1)
-    return torch.stack([gmax, torch.exp(xf - gmax.unsqueeze(-1)).sum(-1), torch.where(own, tl, torch.zeros_like(tl))], 0)
+    ref = torch.where(torch.isneginf(gmax), torch.zeros_like(gmax), gmax)    # a row of -inf sums to 0, as in the kernel
+    return torch.stack([gmax, torch.exp(xf - ref.unsqueeze(-1)).sum(-1), torch.where(own, tl, torch.zeros_like(tl))], 0)
 
 
 def rescale(stats: torch.Tensor, gmax: torch.Tensor) -> torch.Tensor:
