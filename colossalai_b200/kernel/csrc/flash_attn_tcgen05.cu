@@ -45,19 +45,60 @@ constexpr int NUM_THREADS = (SOFTMAX_WARP0 + 8) * 32;
 constexpr int UNIT_RING = 2;
 
 // Waits give up after a bounded number of polls (each of which the hardware may suspend), far beyond any wait of a kernel
-// that works; the CTA then drains its copies, frees its tensor memory and leaves, and the flag below is raised.
+// that works.  The CTA then waits, bounded again, for its copies and products in flight, writes the status word, frees its
+// tensor memory and leaves; the next launch from the host returns cudaErrorLaunchTimeout instead of launching.
 constexpr int WAIT_LIMIT = 1 << 22;
-__device__ int g_flash_error;
 
-SM100_DEVICE bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+SM100_DEVICE bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int limit = WAIT_LIMIT) {
   if (mbar_try_wait(bar, parity)) return true;
-  for (int i = 0; i < WAIT_LIMIT; ++i) {
+  for (int i = 0; i < limit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 63) == 63 && *abort_flag) return false;
   }
   *abort_flag = 1;
-  g_flash_error = 1;
   return false;
+}
+// one thread: the rows of a CTA that gave up are not valid
+SM100_DEVICE void report_abort(int* status) {
+  *reinterpret_cast<volatile int*>(status) = 1;
+  __threadfence_system();
+}
+
+// The status word: pinned host memory, so that the host reads it without a call (null: there is none to be had).  One per
+// process, whatever the device.
+int* flash_status() {
+  static int* const word = [] {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // a first launch may be under capture
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      (void)cudaGetLastError();
+      p = nullptr;
+    } else {
+      *static_cast<int*>(p) = 0;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return static_cast<int*>(p);
+  }();
+  return word;
+}
+// what an earlier launch reported, once: every launcher asks before it launches
+int flash_earlier() {
+  int* const word = flash_status();
+  if (word == nullptr) return (int)cudaErrorMemoryAllocation;
+  return __atomic_load_n(word, __ATOMIC_RELAXED) && __atomic_exchange_n(word, 0, __ATOMIC_ACQ_REL) ? (int)cudaErrorLaunchTimeout : 0;
+}
+
+// the wait alone, on a barrier at which nothing arrives
+__global__ void flash_wait_probe_kernel(int limit, int* status) {
+  __shared__ uint64_t bar;
+  __shared__ int gave_up;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    gave_up = 0;
+    fence_barrier_init();
+    if (!wait_or_abort(&bar, 0, &gave_up, limit) && gave_up) report_abort(status);
+  }
 }
 
 template <int D> struct FaCfg {
@@ -90,7 +131,7 @@ struct FaParams {
   // the previous partial result with this launch's keys - is written back in fp32.  No separate rescale / merge pass.
   float* o_state;                    // [rows, hq * D] fp32, or null (plain attention: `out` in the input dtype)
   int has_prev;
-  int out_dtype;
+  int* status;                       // raised when a wait ran out
   uint32_t idesc_qk, idesc_pv;
   // EXTRA variant of the kernel only (inference prefill of sliding-window / ALiBi models):
   int window;                        // > 0: query q sees keys (q - window, q]; key tiles left of every window are skipped
@@ -189,8 +230,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint64_t* u_full = o_empty + 2;          // [UNIT_RING]
   uint64_t* u_empty = u_full + UNIT_RING;  // [UNIT_RING]  10 warps have read the unit
   FaUnit* units = reinterpret_cast<FaUnit*>(u_empty + UNIT_RING);
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(units + UNIT_RING);
+  uint64_t* drained = reinterpret_cast<uint64_t*>(units + UNIT_RING);   // [1]  a CTA that gives up: its products have retired
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(drained + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
+  volatile int* copies = abort_flag + 1;   // [2]  key / value tiles and query tiles that the producer asked for
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -219,6 +262,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       mbar_init(&u_full[i], 1);
       mbar_init(&u_empty[i], 10);
     }
+    mbar_init(drained, 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -318,14 +362,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       }
       if (!__all_sync(0xffffffffu, ok)) break;
     }
-    if (lane == 0 && *abort_flag) {                            // leave no copy in flight behind
-      int none = 0;
-      if (nq > 0) wait_or_abort(q_full, (uint32_t)((nq - 1) & 1), &none);
-      for (int i = max(0, issued - SLOTS); i < issued; ++i) {
-        none = 0;
-        wait_or_abort(&full[i % SLOTS], (uint32_t)((i / SLOTS) & 1), &none);
-      }
-    }
+    if (lane == 0) { copies[0] = issued; copies[1] = nq; }
     __syncwarp();
   } else if (warp == 1) {
     // ================================================================ MMA issuer
@@ -616,6 +653,23 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag) {                         // (nothing writes it any more: uniform) leave nothing in flight behind
+    int none = 0;
+    if (warp == 0 && lane == 0) {
+      const int issued = copies[0], nq = copies[1];
+      if (nq > 0) wait_or_abort(q_full, (uint32_t)((nq - 1) & 1), &none);
+      for (int i = max(0, issued - SLOTS); i < issued; ++i) {
+        none = 0;
+        wait_or_abort(&full[i % SLOTS], (uint32_t)((i / SLOTS) & 1), &none);
+      }
+    }
+    if (warp == 1 && lane == 0) {            // the thread that issued the products
+      umma_commit(drained);
+      wait_or_abort(drained, 0, &none);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) report_abort(p.status);
+  }
   if (warp == 2) tmem_dealloc<C::TMEM_COLS>(tmem_base);
 }
 
@@ -655,7 +709,7 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* out, flo
   p.batch = batch; p.seqlen_q = seqlen_q; p.seqlen_k = seqlen_k; p.hq = hq; p.hkv = hkv; p.causal = causal;
   p.pair_heads = (hq / hkv) % 2 == 0;
   p.scale_log2 = scale * 1.4426950408889634f;
-  p.out = out; p.lse = lse; p.out_dtype = dtype;
+  p.out = out; p.lse = lse; p.status = flash_status();
   p.window = window; p.alibi = alibi;
   p.idesc_qk = make_idesc_f16(BLOCK_Q, BLOCK_KV, bf16 ? 1 : 0, 0, 0);      // S[128 x 128] = Q (K-major) x K (K-major)
   p.idesc_pv = make_idesc_f16(BLOCK_Q, D, bf16 ? 1 : 0, 0, 1);              // O[128 x D]  = P (K-major) x V (MN-major)
@@ -739,7 +793,7 @@ struct FaBwdParams {
   // the block owner's memory (peer-mapped symmetric buffer: the reduction crosses NVLink) instead of being stored
   float* dk_acc;                     // [rows, hkv * D] fp32 or null
   float* dv_acc;
-  int out_dtype;
+  int* status;                       // raised when a wait ran out
   uint32_t idesc_st, idesc_dv, idesc_dqt;
 };
 
@@ -772,9 +826,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint64_t* dq_full = pds_empty + 2;       // [1]  dQ^T is in TMEM
   uint64_t* dq_empty = dq_full + 1;        // [1]  4 drain warps have read it
   uint64_t* acc_full = dq_empty + 1;       // [1]  final dK / dV complete
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint64_t* drained = acc_full + 1;        // [1]  a CTA that gives up: its products have retired
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(drained + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
-  int* work = reinterpret_cast<int*>(tmem_ptr_smem + 2);
+  volatile int* copies = abort_flag + 1;   // [1]  query tiles that the producer asked for
+  int* work = reinterpret_cast<int*>(tmem_ptr_smem + 3);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -827,6 +883,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     mbar_init(dq_full, 1);
     mbar_init(dq_empty, 4);
     mbar_init(acc_full, 1);
+    mbar_init(drained, 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -862,14 +919,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           tma_load_2d(&tmap_do, &qdo_full[stage], sdo + h * (BWD_BLOCK_Q * 128), hq * D + h * 64, q_row0);
         }
       }
-      if (*abort_flag || n_iter == 0) {                  // leave no copy in flight behind
-        int none = 0;
-        wait_or_abort(kv_full, 0, &none);
-        for (int i = max(0, it - ST); i < it; ++i) {
-          none = 0;
-          wait_or_abort(&qdo_full[i % ST], ring_parity(i), &none);
-        }
-      }
+      *copies = it;
+      if (n_iter == 0) wait_or_abort(kv_full, 0, abort_flag);   // nothing waits for K and V: leave no copy in flight behind
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -1108,6 +1159,22 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag) {                         // (nothing writes it any more: uniform) leave nothing in flight behind
+    int none = 0;
+    if (warp == 0 && lane == 0) {
+      wait_or_abort(kv_full, 0, &none);
+      for (int i = max(0, *copies - ST); i < *copies; ++i) {
+        none = 0;
+        wait_or_abort(&qdo_full[i % ST], ring_parity(i), &none);
+      }
+    }
+    if (warp == 1 && lane == 0) {            // the thread that issued the products
+      umma_commit(drained);
+      wait_or_abort(drained, 0, &none);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) report_abort(p.status);
+  }
   if (warp == 2) tmem_dealloc<C::TMEM_COLS>(tmem_base);
 }
 
@@ -1188,7 +1255,7 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* do
   p.cu_seqlens = cu_seqlens;
   p.batch = batch; p.seqlen = seqlen; p.hq = hq; p.hkv = hkv; p.causal = causal;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
-  p.lse = lse; p.delta = delta; p.dq_acc = dq_acc; p.dk = dk; p.dv = dv; p.out_dtype = dtype;
+  p.lse = lse; p.delta = delta; p.dq_acc = dq_acc; p.dk = dk; p.dv = dv; p.status = flash_status();
   p.dk_acc = dk_acc; p.dv_acc = dv_acc;
   const int f = bf16 ? 1 : 0;
   p.idesc_st = make_idesc_f16(BWD_BLOCK_KV, BWD_BLOCK_Q, f, 0, 0);     // [128 keys x 64 q]  = K-major x K-major
@@ -1213,6 +1280,16 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* do
 
 extern "C" {
 
+// cudaErrorLaunchTimeout, once, if a wait of a launch that has run since the last call of any function here ran out
+int cb_flash_attn_status() { return flash_earlier(); }
+
+// A wait that runs out after `limit` polls and reports it, with no copy or product in flight.
+int cb_flash_attn_wait_probe(int limit, cudaStream_t stream) {
+  if (flash_status() == nullptr) return (int)cudaErrorMemoryAllocation;
+  flash_wait_probe_kernel<<<1, 32, 0, stream>>>(limit, flash_status());
+  return (int)cudaGetLastError();
+}
+
 // q [batch * seqlen_q, hq, D], k / v [batch * seqlen_k, hkv, D] contiguous token-major; out like q; lse [batch *
 // seqlen_q, hq] fp32 (may be null).  Requirements: D in {64, 128}, seqlen_q and seqlen_k multiples of 128,
 // causal => seqlen_q == seqlen_k, hq % hkv == 0, 16-byte aligned bases.
@@ -1223,6 +1300,7 @@ int cb_flash_attn_fwd(const void* q, const void* k, const void* v, void* out, fl
   if (hq % hkv || (causal && seqlen_q != seqlen_k)) return (int)cudaErrorInvalidValue;
   // sequence lengths need not be multiples of the tile: partial tiles are masked (keys) / not stored (queries)
   if (dtype != CB_BF16 && dtype != CB_F16) return (int)cudaErrorInvalidValue;
+  if (const int e = flash_earlier()) return e;
   if (head_dim == 128)
     return launch_flash_fwd<128>(q, k, v, out, lse, batch, seqlen_q, seqlen_k, hq, hkv, causal, scale, dtype, stream);
   if (head_dim == 64)
@@ -1238,6 +1316,7 @@ int cb_flash_attn_varlen_fwd(const void* q, const void* k, const void* v, void* 
                              int dtype, cudaStream_t stream) {
   if (batch <= 0 || total_tokens <= 0) return 0;
   if (hq % hkv || (dtype != CB_BF16 && dtype != CB_F16) || cu_seqlens == nullptr) return (int)cudaErrorInvalidValue;
+  if (const int e = flash_earlier()) return e;
   if (head_dim == 128)
     return launch_flash_fwd<128>(q, k, v, out, lse, batch, 0, 0, hq, hkv, causal, scale, dtype, stream, cu_seqlens, total_tokens);
   if (head_dim == 64)
@@ -1253,6 +1332,7 @@ int cb_flash_attn_varlen_fwd_ex(const void* q, const void* k, const void* v, voi
   if (batch <= 0 || total_tokens <= 0) return 0;
   if (hq % hkv || (dtype != CB_BF16 && dtype != CB_F16) || cu_seqlens == nullptr || window < 0)
     return (int)cudaErrorInvalidValue;
+  if (const int e = flash_earlier()) return e;
   if (head_dim == 128)
     return launch_flash_fwd<128>(q, k, v, out, lse, batch, 0, 0, hq, hkv, 1, scale, dtype, stream, cu_seqlens,
                                  total_tokens, nullptr, 0, window, alibi_slopes);
@@ -1274,6 +1354,7 @@ int cb_flash_attn_bwd(const void* q, const void* k, const void* v, const void* o
   // head_dim 64 would make dQ^T an M = 64 MMA (different TMEM lane layout): not wired up yet
   if (hq % hkv || head_dim != 128) return (int)cudaErrorInvalidValue;
   if (dtype != CB_BF16 && dtype != CB_F16) return (int)cudaErrorInvalidValue;
+  if (const int e = flash_earlier()) return e;
   const long long rows = (cu_seqlens ? total_tokens : (long long)batch * seqlen) * hq;
   const long long n = rows * head_dim;
   const int re = dtype == CB_BF16 ? launch_flash_bwd_delta<__nv_bfloat16>(out, dout, delta, dq_acc, rows, head_dim, stream)
@@ -1302,6 +1383,7 @@ int cb_flash_attn_block_fwd(const void* q, const void* k, const void* v, float* 
   if (rows <= 0) return 0;
   if (hq % hkv || (dtype != CB_BF16 && dtype != CB_F16) || o_state == nullptr || lse == nullptr)
     return (int)cudaErrorInvalidValue;
+  if (const int e = flash_earlier()) return e;
   if (head_dim == 128)
     return launch_flash_fwd<128>(q, k, v, nullptr, lse, 1, rows, rows, hq, hkv, causal, scale, dtype, stream, nullptr, 0,
                                  o_state, has_prev);
@@ -1317,6 +1399,7 @@ int cb_flash_attn_block_bwd(const void* q, const void* k, const void* v, const v
   if (rows <= 0) return 0;
   if (hq % hkv || head_dim != 128 || (dtype != CB_BF16 && dtype != CB_F16) || !dq_acc || !dk_acc || !dv_acc)
     return (int)cudaErrorInvalidValue;
+  if (const int e = flash_earlier()) return e;
   return launch_flash_bwd<128>(q, k, v, dout, lse, delta, dq_acc, nullptr, nullptr, 1, rows, hq, hkv, causal, scale, dtype,
                                stream, nullptr, 0, dk_acc, dv_acc);
 }

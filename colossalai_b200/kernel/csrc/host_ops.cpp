@@ -78,6 +78,8 @@ Count* const COUNTS[] = {&n_norm_fwd, &n_norm_bwd, &n_glu_fwd, &n_glu_bwd, &n_ro
                          &n_decode};
 
 void launched(int rc, Count& c, int n = 1) {
+  TORCH_CHECK(rc != cudaErrorLaunchTimeout, c.name, ": a wait inside an earlier attention kernel ran out; what it wrote is not valid (CUDA error ",
+              rc, ")");
   TORCH_CHECK(rc == 0, c.name, ": native launcher returned CUDA error ", rc);
   c.n.fetch_add(n, std::memory_order_relaxed);
 }

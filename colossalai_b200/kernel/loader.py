@@ -257,6 +257,11 @@ def stream_ptr() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
+WAIT_RAN_OUT = 702              # cudaErrorLaunchTimeout, as the attention launchers return it
+
+
 def check(err: int, what: str) -> None:
+    if err == WAIT_RAN_OUT:
+        raise RuntimeError(f"{what}: a wait inside an earlier attention kernel ran out; what it wrote is not valid (CUDA error {err})")
     if err != 0:
         raise RuntimeError(f"{what}: native launcher returned CUDA error {err}")

@@ -41,6 +41,13 @@ def _major(device: int) -> int:
     return torch.cuda.get_device_capability(device)[0]
 
 
+def check_status() -> None:
+    """Raise if a wait inside an attention kernel that has run by now ran out (its outputs are not valid then).  Every call of an
+    attention kernel asks the same before it launches; a program that only replays graphs, or wants to know about its last
+    call, asks here after a synchronisation."""
+    loader.check(_get_lib().cb_flash_attn_status(), "flash_attn")
+
+
 def _tensor_ok(t: torch.Tensor) -> bool:
     return t.is_cuda and t.dim() == 3 and t.dtype in (torch.bfloat16, torch.float16) and t.is_contiguous() \
         and t.data_ptr() % 16 == 0

@@ -272,3 +272,28 @@ def test_flash_unit_list_of_packed_batches(lens, Hq, Hkv, D, causal):
             torch.testing.assert_close(out[a:a + n].float(), torch.einsum("hqk,khd->qhd", s.softmax(-1), vv), atol=2e-2, rtol=2e-2)
             torch.testing.assert_close(lse[a:a + n], s.logsumexp(-1).t(), atol=2e-3, rtol=2e-3)
         a += n
+
+
+def test_a_wait_that_runs_out_is_reported():
+    """The wait alone, on a barrier at which nothing arrives: the next call of an attention operator raises instead of launching,
+    once."""
+    import ctypes
+
+    from colossalai_b200 import ops
+    from colossalai_b200.kernel import loader
+    from colossalai_b200.ops import flash_attn_native as fa
+
+    lib = loader.load("cb200_attn")
+    x = torch.randn(8, 1, 128, device="cuda", dtype=torch.bfloat16)
+    cu = torch.tensor([0, 8], device="cuda", dtype=torch.int32)
+    good = ops.attention(x, x, x, cu_seqlens_q=cu)
+    calls = [lambda: ops.attention(x, x, x, cu_seqlens_q=cu), lambda: fa.flash_fwd(x, x, x, 1, True, None), fa.check_status,
+             lambda: fa.flash_bwd(x, x, x, x, x, torch.zeros(8, 1, device="cuda"), 1, True, None),
+             lambda: fa.flash_prefill(x, x, x, cu, None, window=3)]
+    for call in calls:
+        assert lib.cb_flash_attn_wait_probe(ctypes.c_int(64), loader.stream_ptr()) == 0
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="a wait inside an earlier attention kernel ran out"):
+            call()
+        fa.check_status()
+        assert torch.equal(ops.attention(x, x, x, cu_seqlens_q=cu), good)
