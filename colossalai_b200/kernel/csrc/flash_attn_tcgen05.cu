@@ -834,15 +834,16 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int kv_head = blockIdx.x;
+  // key tiles that see the most queries first; heads vary fastest (both in grid.x: a packed batch may have more key tiles than
+  // grid.y holds)
+  const int unit_of_head = blockIdx.x / p.hkv, kv_head = blockIdx.x - unit_of_head * p.hkv;
   const int group = p.hq / p.hkv;
-  // key tiles that see the most queries first; heads vary fastest
   int kv_tile, seq_row0, len;
   if (p.cu_seqlens != nullptr) {
     if (warp == 0) {
       int unit = -1, start = 0, n = 0;
-      if ((int)blockIdx.y < packed_count(p.cu_seqlens, p.batch, BWD_BLOCK_KV, 0))
-        packed_unit(p.cu_seqlens, p.batch, BWD_BLOCK_KV, (int)blockIdx.y, unit, start, n);
+      if (unit_of_head < packed_count(p.cu_seqlens, p.batch, BWD_BLOCK_KV, 0))
+        packed_unit(p.cu_seqlens, p.batch, BWD_BLOCK_KV, unit_of_head, unit, start, n);
       if (lane == 0) { work[0] = unit; work[1] = start; work[2] = n; }
     }
     __syncthreads();
@@ -850,7 +851,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     seq_row0 = work[1]; len = work[2];
     kv_tile = (len + BWD_BLOCK_KV - 1) / BWD_BLOCK_KV - 1 - work[0];
   } else {
-    kv_tile = blockIdx.y; seq_row0 = (int)blockIdx.z * p.seqlen; len = p.seqlen;
+    kv_tile = unit_of_head; seq_row0 = (int)blockIdx.y * p.seqlen; len = p.seqlen;
   }
   const int q_tiles = (len + BWD_BLOCK_Q - 1) / BWD_BLOCK_Q;
   // causal: query tile i (rows 64 i ..) sees key tile j (keys 128 j ..) iff 64 i + 63 >= 128 j  <=>  i >= 2 j
@@ -1268,10 +1269,9 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* do
     if (e != cudaSuccess) return (int)e;
     attr_set[f] = true;
   }
-  const dim3 grid(hkv, cu_seqlens ? (unsigned)(total_tokens / BWD_BLOCK_KV + batch)
-                                  : (unsigned)((seqlen + BWD_BLOCK_KV - 1) / BWD_BLOCK_KV),
-                  cu_seqlens ? 1 : batch);
-  if (grid.y > 65535 || grid.z > 65535) return (int)cudaErrorInvalidValue;
+  const long long units = (cu_seqlens ? total_tokens / BWD_BLOCK_KV + batch : ((long long)seqlen + BWD_BLOCK_KV - 1) / BWD_BLOCK_KV) * hkv;
+  const dim3 grid((unsigned)units, cu_seqlens ? 1 : batch);
+  if (units > 0x7fffffffll || grid.y > 65535) return (int)cudaErrorInvalidValue;
   kern<<<grid, BWD_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
   return (int)cudaGetLastError();
 }

@@ -297,3 +297,25 @@ def test_a_wait_that_runs_out_is_reported():
             call()
         fa.check_status()
         assert torch.equal(ops.attention(x, x, x, cu_seqlens_q=cu), good)
+
+
+def test_packed_backward_of_very_many_sequences():
+    """More key tiles than a grid's second dimension holds (65535): one token per sequence, so that the output is v, the gradient
+    of v is the output's and queries and keys get none - beside a last sequence of two tiles."""
+    from colossalai_b200 import ops
+
+    n, last, H, D = 70000, 200, 2, 128
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k, v = (torch.randn(n + last, H, D, device="cuda", generator=g).bfloat16().requires_grad_() for _ in range(3))
+    do = torch.randn(n + last, H, D, device="cuda", generator=g).bfloat16()
+    cu = torch.cat([torch.arange(n + 1, device="cuda"), torch.tensor([n + last], device="cuda")]).int()
+    o = ops.attention(q, k, v, causal=True, cu_seqlens_q=cu, cu_seqlens_k=cu)
+    dq, dk, dv = torch.autograd.grad(o, (q, k, v), do)
+    assert torch.equal(o[:n], v[:n]) and torch.equal(dv[:n], do[:n])
+    assert dq[:n].abs().max() < 1e-3 and dk[:n].abs().max() < 1e-3          # p (dp - delta) of two fp32 sums of 128 products
+    r = [t[n:].detach().double().requires_grad_() for t in (q, k, v)]
+    s = torch.einsum("qhd,khd->hqk", r[0], r[1]) / D ** 0.5
+    s = s.masked_fill(~torch.ones(last, last, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    ref = torch.einsum("hqk,khd->qhd", s.softmax(-1), r[2])
+    for a, b in zip((o, dq, dk, dv), (ref,) + torch.autograd.grad(ref, r, do[n:].double())):
+        assert (a[n:].double() - b).norm() <= 1e-2 * b.norm()                  # weights and results rounded to bf16
