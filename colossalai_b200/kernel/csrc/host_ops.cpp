@@ -228,7 +228,8 @@ struct PackedAttention : torch::autograd::Function<PackedAttention> {
     launched(L.flash_varlen_fwd(ptr(q), ptr(k), ptr(v), mut(out), mut_as<float>(lse), as<int>(cu), (int)cu.numel() - 1, T, (int)Hq,
                                 (int)k.size(1), (int)D, causal, (float)scale, code_of(q), stream_of(q)),
              n_flash_fwd);
-    ctx->save_for_backward({q, k, v, out, lse, cu});
+    ctx->save_for_backward({q, k, v, out, lse});
+    ctx->saved_data["cu"] = cu;              // a program may refill a buffer of boundaries: kept without a version check
     ctx->saved_data["causal"] = causal;
     ctx->saved_data["scale"] = scale;
     return out;
@@ -236,7 +237,8 @@ struct PackedAttention : torch::autograd::Function<PackedAttention> {
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list s = ctx->get_saved_variables();
-    const Tensor &q = s[0], &k = s[1], &v = s[2], &out = s[3], &lse = s[4], &cu = s[5];
+    const Tensor &q = s[0], &k = s[1], &v = s[2], &out = s[3], &lse = s[4];
+    const Tensor cu = ctx->saved_data["cu"].toTensor();
     const c10::cuda::CUDAGuard guard(q.device());
     const int64_t T = q.size(0), Hq = q.size(1), D = q.size(2);
     const Tensor dout = packed(grads[0]);

@@ -155,6 +155,27 @@ def test_packed_attention(monkeypatch, D, grad):
 
 
 @pytest.mark.gpu
+def test_packed_attention_boundaries_refilled(monkeypatch):
+    """A static buffer of boundaries that is written again between forward and backward (the same contents here), and what
+    saved-tensor hooks get to see."""
+    from torch.autograd.graph import saved_tensors_hooks
+
+    def fn():
+        torch.manual_seed(0)
+        q, k, v = (torch.randn(150, h, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True) for h in (4, 2, 2))
+        cu = torch.tensor([0, 40, 150], device="cuda", dtype=torch.int32)
+        seen = []
+        with saved_tensors_hooks(lambda t: (seen.append(t.dtype), t)[1], lambda t: t):
+            o = ops.attention(q, k, v, causal=True, cu_seqlens_q=cu, cu_seqlens_k=cu)
+        cu.copy_(torch.tensor([0, 40, 150], dtype=torch.int32))
+        grads = torch.autograd.grad(o, (q, k, v), torch.ones_like(o))
+        assert seen == [torch.bfloat16] * 4 + [torch.float32]
+        return (o.detach(),) + grads[1:]                                     # (dQ is summed in the order of its reductions)
+
+    _same(*_both(monkeypatch, fn))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("D", [64, 256])
 def test_paged_decode(monkeypatch, D):
     def fn():
