@@ -260,21 +260,23 @@ struct ScanParams {
 // The workspace rows of SCAN_TOK_TILE tokens arrive by cp.async in a ring of stages while the previous tile is walked (decay
 // mode has three, so that one barrier per tile is enough).
 // Bound: the serial chain of a sequence, shared-memory reads (q and k once per SCAN_CPL columns) and fp32 issue, none of them
-// alone.  12000 tokens in eight sequences, 16 heads, 128 x 128, decay mode: recurrence 741 -> 505 us.
+// alone.  12000 tokens in eight uneven sequences, 16 heads, 128 x 128, decay mode: recurrence 741 -> 594 us.  Holding S divided
+// by its decay's powers inside a tile of eight tokens (505 us) made the bits depend on how a sequence is cut into portions, and
+// turned infinite values into NaN.
 constexpr int SCAN_CPL = 4;            // value columns per lane
 constexpr int SCAN_COLS = 32;          // value columns per CTA
 
 template <int DK, int MODE> struct ScanTile {
   // Lanes that share the rows of a column group.  More lanes are shorter steps for each and more warps to hide them behind, at
   // more shuffles and reads of the values.  Decay mode, 16 heads, 12000 tokens, with 8 and with 16 lanes: 128 x 128, one
-  // sequence 2.55 and 1.62 ms, eight 740 and 611 us; 64 x 64, eight sequences 378 and 272 us (32 lanes: 1.68 ms, 785 us).
+  // sequence 2.69 and 1.70 ms, eight uneven ones 802 and 701 us; 64 x 64, eight sequences 385 and 278 us.
   static constexpr int PARTS = DK <= 16 ? 4 : DK <= (MODE == SCAN_DECAY ? 32 : 128) ? 8 : 16;
   static constexpr int RP = DK / PARTS;                                 // rows per lane
   static constexpr int RPP = RP == 4 ? 4 : RP + 4;                      // a lane's rows in shared memory start this far apart:
   static constexpr int DKP = PARTS * RPP;                               // the 16-byte reads of 8 lanes hit different banks
   static constexpr int THREADS = PARTS * SCAN_COLS / SCAN_CPL;
-  // Units that an SM is to hold at a time, by their registers: four tokens' reads want more than 128 of a lane (611 us as
-  // above, 692 at 128 and at 255, where an SM holds two of the 128 wide units and eight sequences take two rounds).
+  // Units that an SM is to hold at a time, by their registers: four tokens' reads want more than 128 of a lane, and at 255 an SM
+  // holds two of the 128 wide units, so that eight sequences take two rounds (either 13 % slower).
   static constexpr int BLOCKS = MODE != SCAN_DECAY || DK > 128 ? 1 : (DK == 128 ? 384 : 512) / THREADS;
   static constexpr int STAGES = MODE == SCAN_DECAY ? 3 : 2;
   static constexpr int NROW = MODE == SCAN_DELTA || MODE == SCAN_ROWS ? 3 : 2;          // q, k, decay rows
@@ -600,31 +602,6 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
     for (int c = 0; c < SCAN_CPL; ++c) S[i / 2][c] = pair_of(x[0][c], x[1][c]);
   }
   const float hd = MODE == SCAN_DECAY ? p.head_decay[h] : 0.f;
-  // Decay mode holds S / hd^i during a full tile: what token i adds is divided by hd^(i + 1), what it reads multiplied by it,
-  // and the next tile's first token scales S back, so that every other one takes two instructions per pair of rows instead of
-  // three.  The powers are held in two parts: a rounded factor would put the same error on everything it scales, tile after
-  // tile.  S is rounded once per token as before.  Decays below a quarter (S would grow by more than 2^16 inside a tile) and
-  // above one keep the plain form, and so does a part of a tile: a decoder's single token would be scaled there and back.  A
-  // lane of the 16 wide kernel has too few rows for it to pay (4096 tokens x 8 heads x 16 x 64: 59 us plain, 73 scaled).
-  __shared__ float4 powers[SCAN_TOK_TILE + 1];                 // hd^i and hd^-i, each as value and remainder
-  const bool scale_tiles = MODE == SCAN_DECAY && DK > 16 && hd >= 0.25f && hd <= 1.f;
-  if (scale_tiles && threadIdx.x <= SCAN_TOK_TILE) {           // read behind a barrier
-    double f = 1.0;
-    for (int i = 0; i < threadIdx.x; ++i) f *= (double)hd;
-    const float a = (float)f, b = (float)(1.0 / f);
-    powers[threadIdx.x] = make_float4(a, (float)(f - a), b, (float)(1.0 / f - b));
-  }
-  float back = 1.f, back_low = 0.f;                            // S is held divided by this
-  auto scale_back = [&]() {
-    const uint64_t f2 = pair_of(back, back), l2 = pair_of(back_low, back_low);
-#pragma unroll
-    for (int i = 0; i < RP / 2; ++i)
-#pragma unroll
-      for (int c = 0; c < SCAN_CPL; ++c) S[i][c] = fma2(S[i][c], f2, mul2(S[i][c], l2));
-    back = 1.f;
-    back_low = 0.f;
-  };
-
   const float skip = (MODE == SCAN_GATED && p.head_decay != nullptr) ? p.head_decay[h] : 0.f;
 
   // A thread copies the same 16-byte piece of every (THREADS / pieces)-th token: its addresses only step, which keeps the
@@ -680,26 +657,14 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
     return v;
   };
 
-  if (MODE == SCAN_DECAY) __syncthreads();      // the powers
   load_tile(0, t0);
   if (STAGES == 3) load_tile(1, t0 + SCAN_TOK_TILE);
   int stage = 0;
   for (int tb = t0; tb < t1; tb += SCAN_TOK_TILE, stage = stage + 1 == STAGES ? 0 : stage + 1) {
     const int nt = min(SCAN_TOK_TILE, t1 - tb);
-    const bool scaled_tile = scale_tiles && nt == SCAN_TOK_TILE;
     // a tile past the portion's end is an empty group
     if (STAGES == 2) load_tile(stage ^ 1, tb + SCAN_TOK_TILE);    // released by the barrier that ended the last pass
     asm volatile("cp.async.wait_group 1;" ::: "memory");
-    if (MODE == SCAN_DECAY) {
-#pragma unroll
-      for (int i = 0; i < SCAN_TOK_TILE; i += VPI)          // a thread scales the values that it copied itself
-        if (vt + i < nt && scaled_tile) {
-          float4* values = reinterpret_cast<float4*>(scan_smem + stage * STAGE + vdst + i * SCAN_COLS);
-          const float4 f = powers[vt + i + 1], x = *values;
-          *values = make_float4(fmaf(x.x, f.z, x.x * f.w), fmaf(x.y, f.z, x.y * f.w), fmaf(x.z, f.z, x.z * f.w),
-                                fmaf(x.w, f.z, x.w * f.w));
-        }
-    }
     __syncthreads();
     // three stages: the tile before last was left by everyone who passed this barrier
     if (STAGES == 3) load_tile(stage == 0 ? 2 : stage - 1, tb + 2 * SCAN_TOK_TILE);
@@ -709,8 +674,7 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
     const float* sv = sq + NROW * SCAN_TOK_TILE * DKP;
     const float* sbeta = sv + SCAN_TOK_TILE * SCAN_COLS;
     // one token: the lane's part of S is advanced; returns column (part & 3) of the read-out joined over the lane's quad
-    auto advance = [&](int tt, auto scaled, auto first) -> float {
-      constexpr bool SCALED = decltype(scaled)::value, FIRST = decltype(first)::value;
+    auto advance = [&](int tt) -> float {
       const float4 v4 = *reinterpret_cast<const float4*>(sv + tt * SCAN_COLS + c0);
       float u[SCAN_CPL] = {v4.x, v4.y, v4.z, v4.w};
       const float* kq = sk + tt * DKP + r0p;
@@ -752,8 +716,7 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
       uint64_t o2[SCAN_CPL] = {0ull, 0ull, 0ull, 0ull}, u2[SCAN_CPL];
 #pragma unroll
       for (int c = 0; c < SCAN_CPL; ++c) u2[c] = pair_of(u[c], u[c]);
-      if (SCALED) dec = back;
-      const uint64_t dec2 = pair_of(dec, dec), low2 = pair_of(back_low, back_low);
+      const uint64_t dec2 = pair_of(dec, dec);
 #pragma unroll
       for (int i = 0; i < RP; i += 4) {
         const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kq + i);
@@ -766,8 +729,7 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
 #pragma unroll
           for (int c = 0; c < SCAN_CPL; ++c) {
             uint64_t& x = S[i / 2 + e][c];
-            if (MODE == SCAN_DELTA || (SCALED && !FIRST)) x = fma2(kr[e], u2[c], x);
-            else x = fma2(gr[e], x, SCALED ? fma2(low2, x, mul2(kr[e], u2[c])) : mul2(kr[e], u2[c]));
+            x = MODE == SCAN_DELTA ? fma2(kr[e], u2[c], x) : fma2(gr[e], x, mul2(kr[e], u2[c]));
             o2[c] = fma2(x, qr[e], o2[c]);
           }
       }
@@ -784,39 +746,26 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
     // NTOK tokens at a time: only S ties them together, so their loads and sums overlap; the quads exchange their sums so
     // that quad n ends up with token n's total (the same pairs in the same order as one token alone takes: the result does
     // not depend on how a portion falls into groups)
-    auto group = [&](int tt, auto scaled, auto first) {      // every lane takes part in the shuffles, also for a padded column
+    int tt = 0;
+#pragma unroll 2
+    for (; tt + NTOK <= nt; tt += NTOK) {        // every lane takes part in the shuffles, also for a padded column
       float v[NTOK];
 #pragma unroll
-      for (int n = 0; n < NTOK; ++n) v[n] = n == 0 ? advance(tt, scaled, first) : advance(tt + n, scaled, std::false_type());
+      for (int n = 0; n < NTOK; ++n) v[n] = advance(tt + n);
 #pragma unroll
       for (int m = NTOK / 2, bit = 4; m >= 1; m /= 2, bit *= 2) {
         const bool up = part & bit;
 #pragma unroll
         for (int n = 0; n < m; ++n) v[n] = (up ? v[2 * n + 1] : v[2 * n]) + __shfl_xor_sync(ALL, up ? v[2 * n] : v[2 * n + 1], bit);
       }
-      tt += part / SCAN_CPL;
-      if (decltype(scaled)::value) v[0] = fmaf(v[0], powers[tt + 1].x, v[0] * powers[tt + 1].y);
-      emit(tt, v[0]);
-    };
-    if (MODE == SCAN_DECAY && scaled_tile) {
-      group(0, std::true_type(), std::true_type());
-#pragma unroll
-      for (int tt = NTOK; tt < SCAN_TOK_TILE; tt += NTOK) group(tt, std::true_type(), std::false_type());
-      back = powers[SCAN_TOK_TILE].x;
-      back_low = powers[SCAN_TOK_TILE].y;
-    } else {
-      if (MODE == SCAN_DECAY && scale_tiles) scale_back();
-      int tt = 0;
-#pragma unroll 2
-      for (; tt + NTOK <= nt; tt += NTOK) group(tt, std::false_type(), std::false_type());
-      for (; tt < nt; ++tt) {
-        const float o = join_quads(advance(tt, std::false_type(), std::false_type()));
-        if (part < SCAN_CPL) emit(tt, o);
-      }
+      emit(tt + part / SCAN_CPL, v[0]);
+    }
+    for (; tt < nt; ++tt) {
+      const float o = join_quads(advance(tt));
+      if (part < SCAN_CPL) emit(tt, o);
     }
     if (STAGES == 2) __syncthreads();           // this stage may be refilled in the next pass
   }
-  if (MODE == SCAN_DECAY && scale_tiles) scale_back();
 #pragma unroll
   for (int i = 0; i < RP; i += 2) {
     float2 x[SCAN_CPL];

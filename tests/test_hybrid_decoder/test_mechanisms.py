@@ -92,7 +92,7 @@ def test_decay_scan_matches_token_by_token(device, H, d, dv):
 @pytest.mark.parametrize("lens", [[8], [7, 24, 0, 9, 1, 16, 33], [1 + i % 9 for i in range(34)]])
 def test_decay_scan_tiles_and_unit_order(device, d, dv, lens):
     """Whole tiles of eight tokens, parts of one, sequences without tokens, few and more than 32 sequences, fresh and carried;
-    decays on both sides of the range in which a tile is held scaled."""
+    decays of zero, one and more."""
     dev, H = _dev(device), 6
     g = torch.Generator().manual_seed(d + len(lens))
     decay = torch.tensor([0.0, 0.2, 0.25, 0.6, 1.0, 1.02])
@@ -124,6 +124,55 @@ def test_decay_scan_tiles_and_unit_order(device, d, dv, lens):
             assert bool(((out_s[slot].double().cpu() - S).abs() <= 2 * 33 * 2.0 ** -24 * A + 1e-12).all())
         else:
             assert torch.equal(out_s[slot].cpu(), state[slot])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,dv", [(16, 64), (64, 40), (128, 32), (200, 36)])
+@pytest.mark.parametrize("cuts", [[8, 29], [1] * 37, [5, 8, 3, 20, 1], [16, 16, 4, 1]])
+def test_decay_scan_does_not_depend_on_portions(d, dv, cuts):
+    """A position's read-out and the state behind it are the same bits whatever portions the sequence comes in."""
+    dev, H, L = _dev("cuda"), 5, 37
+    g = torch.Generator().manual_seed(d)
+    decay = torch.tensor([0.0, 0.2, 0.25, 0.7, 0.999]).to(dev)
+    q, k, v = (torch.randn(L, H * w, generator=g).to(dev) for w in (d, d, dv))
+    ran = []
+    for parts in ([L], cuts):
+        assert sum(parts) == L
+        state, outs, at = torch.zeros(1, H, d, dv, device=dev), [], 0
+        for n in parts:
+            meta = M.RaggedMeta.build([n], [at], [0], dev)
+            outs.append(M.state_scan_decay(q[at:at + n], k[at:at + n], v[at:at + n], decay, state, meta, H, d, dv).clone())
+            at += n
+        ran.append((torch.cat(outs), state))
+    assert torch.equal(ran[0][0], ran[1][0]) and torch.equal(ran[0][1], ran[1][1])
+
+
+@pytest.mark.parametrize("device", DEVICES)
+@pytest.mark.parametrize("L", [8, 13, 16])
+def test_decay_scan_of_infinite_and_very_large_values(device, L):
+    """An infinite value or state entry stays infinite and a product near the largest fp32 number stays finite, also inside
+    whole tiles of eight tokens."""
+    dev, H, d, dv = _dev(device), 3, 64, 32
+    decay = torch.tensor([0.3, 0.5, 0.9])
+    q, k = torch.full((L, H * d), 2.0 ** -7), torch.zeros(L, H * d)
+    v = torch.ones(L, H * dv)
+    k[0] = 1.0
+    v[0].view(H, dv)[:, 0] = float("inf")
+    v[0].view(H, dv)[:, 1] = -float("inf")
+    v[0].view(H, dv)[:, 2] = 1e38
+    state = torch.zeros(1, H, d, dv)
+    state[0, :, :, 3] = float("inf")
+    state[0, :, :, 4] = 2e38
+    S, want = state[0].double(), []
+    for t in range(L):
+        S = decay.double()[:, None, None] * S + k[t].double().view(H, d, 1) * v[t].double().view(H, 1, dv)
+        want.append(torch.einsum("hdv,hd->hv", S, q[t].double().view(H, d)).flatten())
+    out_s = state.to(dev)
+    meta = M.RaggedMeta.build([L], [3], [0], dev)
+    # k[t] = 0 behind the first token: an infinite value meets no zero (0 x inf is NaN everywhere)
+    out = M.state_scan_decay(q.to(dev), k.to(dev), v.to(dev), decay.to(dev), out_s, meta, H, d, dv, act_silu=False)
+    torch.testing.assert_close(out.double().cpu(), torch.stack(want), rtol=(d + 2 * L) * 2.0 ** -24, atol=0)
+    torch.testing.assert_close(out_s[0].double().cpu(), S, rtol=2 * L * 2.0 ** -24, atol=0)
 
 
 def _delta_inputs(L, H, G, d, dv, seed):
