@@ -608,11 +608,13 @@ __global__ void __launch_bounds__(128) decode_reduce_kernel(const float* __restr
   float gm = -INFINITY;
   for (int s = 0; s < splits; ++s) gm = fmaxf(gm, ml_part[(base + s) * 2]);
   float ls = 0.f;
+  bool nan = false;                             // scores that are all NaN in a partition: its sum is NaN, its maximum -inf
   for (int s = 0; s < splits; ++s) {
     const float mm = ml_part[(base + s) * 2];
     ls += (mm == -INFINITY) ? 0.f : ml_part[(base + s) * 2 + 1] * __expf(mm - gm);
+    nan |= isnan(ml_part[(base + s) * 2 + 1]);
   }
-  const float inv = ls > 0.f ? 1.f / ls : 0.f;
+  const float inv = nan ? NAN : ls > 0.f ? 1.f / ls : 0.f;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     float acc = 0.f;
     for (int s = 0; s < splits; ++s) {

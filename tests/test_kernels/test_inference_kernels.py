@@ -212,3 +212,19 @@ def test_paged_decode_stops_at_the_page_table(D, window, width):
         k, v = (c[tables[i].long()].flatten(0, 1)[first:end].double().repeat_interleave(4, 1) for c in (kc, vc))
         ref = torch.einsum("hk,khd->hd", (torch.einsum("hd,khd->hk", q[i].double(), k) / D ** 0.5).softmax(-1), v)
         torch.testing.assert_close(out[i].double(), ref, atol=2e-2, rtol=2e-2)      # weights rounded to bf16
+
+
+@pytest.mark.parametrize("length", [16, 2000])
+@pytest.mark.parametrize("keys", ["one", "page", "all"])
+def test_paged_decode_shows_nan(length, keys):
+    """NaN keys give NaN, whether the sequence is finished in one piece or merged from many."""
+    dev = torch.device("cuda")
+    torch.manual_seed(length)
+    kc, vc, tables = _mk_cache(2, length, 16, 2, 128, torch.bfloat16, dev)
+    q = torch.randn(2, 8, 128, device=dev, dtype=torch.bfloat16)
+    lens = torch.tensor([length, length], device=dev, dtype=torch.int32)
+    good = iops.paged_decode_attention(q, kc, vc, tables, lens)
+    for p in tables[1].tolist() if keys == "all" else [int(tables[1, -1])]:
+        kc[p, 3 if keys == "one" else slice(None)] = float("nan")
+    out = iops.paged_decode_attention(q, kc, vc, tables, lens)
+    assert out[1].isnan().all() and torch.equal(out[0], good[0])
