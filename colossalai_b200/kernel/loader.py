@@ -19,6 +19,7 @@ import shutil
 import subprocess
 import sysconfig
 import threading
+import warnings
 from pathlib import Path
 from typing import Dict, List, Optional
 
@@ -107,7 +108,7 @@ def _src_hash(name: str) -> str:
         h.update(hdr.read_bytes())
     h.update(" ".join(_flags(spec)).encode())
     if spec["kind"] == "torch":
-        h.update(torch.__version__.encode())
+        h.update(f"{torch.__version__} {sysconfig.get_config_var('EXT_SUFFIX')}".encode())
     return h.hexdigest()[:16]
 
 
@@ -207,30 +208,38 @@ _HOST_CALLS = {
     "cb200_attn": ["cb_flash_attn_varlen_fwd", "cb_flash_attn_bwd"],
     "cb200_infer": ["cb_decode_num_splits", "cb_paged_decode_attention"],
 }
-_host = None
+_host, _host_asked = None, False
 
 
 def host():
-    """The native host module (`csrc/host_ops.cpp`), with the kernels' launchers bound."""
-    global _host
-    if _host is None:
+    """The native host module (`csrc/host_ops.cpp`) with the kernels' launchers bound, or None where there is none for these
+    sources and this torch: the python autograd functions launch the same kernels then."""
+    global _host, _host_asked
+    if not _host_asked:
         libs = {lib: load(lib) for lib in _HOST_CALLS}
         with _lock:
-            if _host is None:
-                p = lib_path("cb200_host")
-                if not p.exists() or (is_stale("cb200_host") and os.environ.get("CB200_NO_REBUILD") != "1"):
-                    try:
-                        build("cb200_host")
-                    except Exception:
-                        if not p.exists():
-                            raise
-                spec = importlib.util.spec_from_file_location("cb200_host", p)
-                mod = importlib.util.module_from_spec(spec)
-                spec.loader.exec_module(mod)
-                mod.bind({f: ctypes.cast(getattr(libs[lib], f), ctypes.c_void_p).value for lib, fs in _HOST_CALLS.items() for f in fs})
-                launch_counter.native = mod.counts
-                _host = mod
+            if not _host_asked:
+                _host = _load_host(libs)
+                _host_asked = True
     return _host
+
+
+def _load_host(libs):
+    try:
+        # bound to one torch and to the launchers' signatures: unlike a C library it is never taken as it was built for others
+        if is_stale("cb200_host"):
+            if os.environ.get("CB200_NO_REBUILD") == "1":
+                raise RuntimeError("it was built for other sources or another torch, and CB200_NO_REBUILD=1")
+            build("cb200_host")
+        spec = importlib.util.spec_from_file_location("cb200_host", lib_path("cb200_host"))
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.bind({f: ctypes.cast(getattr(libs[lib], f), ctypes.c_void_p).value for lib, fs in _HOST_CALLS.items() for f in fs})
+    except Exception as e:
+        warnings.warn(f"the native host module is not used, small operators run from python: {e}")
+        return None
+    launch_counter.native = mod.counts
+    return mod
 
 
 class KernelLoader:

@@ -114,8 +114,8 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, batch: int = 1,
         packed = cu_seqlens_q is not None and (q.shape[-1] == 128 or (q.shape[-1] == 64 and not needs_grad))
         if fa.supported(q, k, v, cu_seqlens_q, cu_seqlens_k, force=packed):
             if packed and plain_call(q, k, v, cu_seqlens_q) and fa.shapes_ok(q, k, batch, causal, cu_seqlens_q) \
-                    and (not needs_grad or fa.bwd_supported(q, k, batch)):
-                return loader.host().packed_attention(q, k, v, fa._cu32(cu_seqlens_q, q.device), bool(causal),
-                                                      scale if scale is not None else 1.0 / math.sqrt(q.shape[-1]))
+                    and (not needs_grad or fa.bwd_supported(q, k, batch)) and (host := loader.host()) is not None:
+                return host.packed_attention(q, k, v, fa._cu32(cu_seqlens_q, q.device), bool(causal),
+                                             scale if scale is not None else 1.0 / math.sqrt(q.shape[-1]))
             return fa.flash_attention(q, k, v, batch=batch, causal=causal, scale=scale, cu_seqlens_q=cu_seqlens_q)
     return attention_ref(q, k, v, batch, causal, scale, cu_seqlens_q, cu_seqlens_k, attn_mask)

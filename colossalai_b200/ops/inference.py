@@ -71,9 +71,9 @@ def paged_decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     if (use_native(q) and q.dtype in (torch.float16, torch.bfloat16) and k_cache.dtype == q.dtype
             and D in (64, 128, 256) and Hq // Hkv <= 8):
-        if plain_call(q, k_cache, v_cache, block_tables, seq_lens, alibi_slopes):
+        if plain_call(q, k_cache, v_cache, block_tables, seq_lens, alibi_slopes) and (host := loader.host()) is not None:
             ws = _workspace_buffers(q)
-            return loader.host().paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale, alibi_slopes, int(window or 0), *ws)
+            return host.paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale, alibi_slopes, int(window or 0), *ws)
         lib = _get_lib()
         max_len = block_tables.shape[1] * bs
         part = ctypes.c_int(0)

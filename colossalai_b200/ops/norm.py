@@ -103,11 +103,11 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
              residual: Optional[torch.Tensor] = None):
     """RMSNorm over the last dim.  With `residual`, returns `(norm(x + residual) * w, x + residual)`."""
     if _native_ok(x, weight):
-        if plain_call(x, weight, residual):
+        if plain_call(x, weight, residual) and (host := loader.host()) is not None:
             if residual is None:
-                return loader.host().rms_norm(x, weight, eps)
+                return host.rms_norm(x, weight, eps)
             if residual.dtype == x.dtype and residual.shape == x.shape and residual.device == x.device:
-                return loader.host().rms_norm_residual(x, weight, eps, residual)
+                return host.rms_norm_residual(x, weight, eps, residual)
         return _RMSNormFn.apply(x, weight, eps, residual)
     return rms_norm_ref(x, weight, eps, residual)
 

@@ -112,8 +112,8 @@ def rope_qkv(qkv: torch.Tensor, positions: Optional[torch.Tensor], cos: torch.Te
             and (qkv.shape[0] == 0 or (width % vec == 0 and (n_q_heads + n_kv_heads) * head_dim <= width))):
         if positions is None:
             positions = torch.arange(qkv.shape[0], device=qkv.device)
-        if plain_call(qkv, positions, cos, sin):
-            return loader.host().rope(qkv, positions.contiguous(), cos, sin, n_q_heads + n_kv_heads, head_dim, rot, interleaved)
+        if plain_call(qkv, positions, cos, sin) and (host := loader.host()) is not None:
+            return host.rope(qkv, positions.contiguous(), cos, sin, n_q_heads + n_kv_heads, head_dim, rot, interleaved)
         return _RopeQKVFn.apply(qkv, positions.contiguous(), cos, sin, n_q_heads + n_kv_heads, head_dim, rot,
                                 interleaved)
     T = qkv.shape[0]

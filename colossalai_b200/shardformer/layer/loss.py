@@ -106,10 +106,11 @@ def cross_entropy_1d(vocab_logits: torch.Tensor, labels: torch.Tensor, ignore_in
                      process_group: ProcessGroup = None, vocab_size: int = None, dtype: torch.dtype = None,
                      mode: str = "mean") -> torch.Tensor:
     if (_ws_rank(process_group)[0] == 1 and mode in ("mean", "sum") and vocab_logits.dim() == 2 and ce_ops._ok(vocab_logits)
-            and labels.shape == vocab_logits.shape[:1] and labels.device == vocab_logits.device and plain_call(vocab_logits, labels)):
+            and labels.shape == vocab_logits.shape[:1] and labels.device == vocab_logits.device and plain_call(vocab_logits, labels)
+            and (host := loader.host()) is not None):
         V = vocab_logits.shape[1]
         valid = V if vocab_size is None else max(min(V, vocab_size), 0)
-        loss = loader.host().cross_entropy(vocab_logits, labels.long().contiguous(), ignore_index, 0, valid, mode == "mean")
+        loss = host.cross_entropy(vocab_logits, labels.long().contiguous(), ignore_index, 0, valid, mode == "mean")
         return loss.to(dtype or torch.float32)
     return DistCrossEntropy.apply(vocab_logits, labels, ignore_index, process_group, vocab_size,
                                   dtype or torch.float32, mode)

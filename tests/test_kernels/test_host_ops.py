@@ -38,6 +38,44 @@ def test_plain_call_sees_what_watches():
     assert seen == [False] * 5 and plain_call(x)
 
 
+@pytest.mark.parametrize("why", ["no rebuild", "build fails", "does not load"])
+def test_a_host_module_of_other_sources_is_not_taken(monkeypatch, tmp_path, why):
+    """One built for another torch or other launchers, whatever lies in the build folder: the python functions remain."""
+    def build(name, **kw):
+        if why == "build fails":
+            raise RuntimeError("no compiler here")
+
+    (tmp_path / "libcb200_host.so").write_bytes(b"of another torch")
+    monkeypatch.setattr(loader, "BUILD", tmp_path)
+    monkeypatch.setattr(loader, "build", build)
+    monkeypatch.setattr(loader, "load", lambda name: None)
+    monkeypatch.setattr(loader, "_host", None)
+    monkeypatch.setattr(loader, "_host_asked", False, raising=False)
+    monkeypatch.setenv("CB200_NO_REBUILD", "1" if why == "no rebuild" else "0")
+    with pytest.warns(UserWarning, match="host module is not used"):
+        assert loader.host() is None
+    assert loader.host() is None
+
+
+@pytest.mark.gpu
+def test_calls_without_a_host_module(monkeypatch):
+    monkeypatch.setattr(loader, "_host", None)
+    monkeypatch.setattr(loader, "_host_asked", True)
+    x = torch.randn(6, 64, device="cuda", dtype=torch.bfloat16)
+    cu = torch.tensor([0, 6], device="cuda", dtype=torch.int32)
+    cache = torch.randn(2, 16, 1, 64, device="cuda", dtype=torch.bfloat16)
+    pages = torch.tensor([[0], [1]], device="cuda", dtype=torch.int32)
+    calls = [lambda: ops.rms_norm(x, x[0]), lambda: ops.rms_norm(x, x[0], 1e-6, x), lambda: ops.glu(x),
+             lambda: ops.rope_qkv(x, None, *ops.build_rope_cache(8, 16, 1e4, device="cuda"), 2, 1, 16),
+             lambda: ops.attention(x.view(6, 1, 64), x.view(6, 1, 64), x.view(6, 1, 64), cu_seqlens_q=cu),
+             lambda: inference.paged_decode_attention(x[:2].view(2, 1, 64), cache, cache, pages, torch.full_like(cu, 6)),
+             lambda: loss_mod.cross_entropy_1d(x, torch.zeros(6, dtype=torch.int64, device="cuda"), process_group="local")]
+    for call in calls:
+        before = loader.launch_counter.count
+        call()
+        assert loader.launch_counter.count > before
+
+
 def _both(monkeypatch, fn):
     """fn() on the host module and on the python functions; how many launches each made."""
     out = []
