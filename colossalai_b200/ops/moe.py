@@ -253,8 +253,15 @@ def _sum_rows(rows: torch.Tensor, slot: torch.Tensor, w: Optional[torch.Tensor],
     return out
 
 
+def _pick_rows(rows: torch.Tensor, slot: torch.Tensor, tokens: int, k: int) -> torch.Tensor:
+    """[T, k, H]: every choice's row (zeros for a choice of no expert), differentiable."""
+    picked = rows.index_select(0, slot.clamp(min=0).long())
+    return torch.where((slot >= 0).unsqueeze(-1), picked, torch.zeros_like(picked)).view(tokens, k, -1)
+
+
 class TakeRows(torch.autograd.Function):
-    """x [T, H] -> rows [bound, H] grouped by expert (padding rows zero); the gradient sums a token's rows in fp32."""
+    """x [T, H] -> rows [bound, H] grouped by expert (padding rows zero); the gradient sums a token's rows in fp32.  With
+    `create_graph` the gradient is made of torch operations, so that it can be differentiated again."""
 
     @staticmethod
     def forward(ctx, x, slot, src, k):
@@ -270,27 +277,36 @@ class TakeRows(torch.autograd.Function):
     @staticmethod
     def backward(ctx, drows):
         slot, = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            return _pick_rows(drows, slot, *ctx.shape).float().sum(1).to(drows.dtype), None, None, None
         return _sum_rows(_aligned(drows), slot, None, *ctx.shape), None, None, None
 
 
 class CombineRows(torch.autograd.Function):
     """rows [bound, H] grouped by expert, weights [T, k] -> out [T, H] = sum_j weights[t, j] rows[slot[t, j]], in fp32 with
-    one rounding."""
+    one rounding.  The gradient under `create_graph` as in `TakeRows`."""
 
     @staticmethod
     def forward(ctx, rows, weights, slot, src):
-        rows, w = _aligned(rows), weights.float().contiguous()
-        ctx.save_for_backward(rows, w, slot, src)
-        ctx.w_dtype = weights.dtype
-        return _sum_rows(rows, slot, w, *weights.shape)
+        ctx.save_for_backward(rows, weights, slot, src)
+        return _sum_rows(_aligned(rows), slot, weights.float().contiguous(), *weights.shape)
 
     @staticmethod
     def backward(ctx, dout):
-        rows, w, slot, src = ctx.saved_tensors
-        g = _aligned(dout)
+        rows, weights, slot, src = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            T, k = weights.shape
+            live = (src >= 0).unsqueeze(-1)
+            choice = src.clamp(min=0).long()
+            g = dout.float().index_select(0, choice // k)
+            w = weights.float().reshape(-1).index_select(0, choice).unsqueeze(-1)
+            drows = torch.where(live, w * g, torch.zeros_like(g)).to(rows.dtype)
+            dw = (_pick_rows(rows, slot, T, k).float() * dout.float().unsqueeze(1)).sum(-1)
+            return drows, dw.to(weights.dtype), None, None
+        g, rows, w = _aligned(dout), _aligned(rows), weights.float().contiguous()
         drows, dw = torch.empty_like(rows), torch.zeros_like(w)
         loader.check(_get_lib().cb_moe_sum_rows_bwd(loader.ptr(g), loader.ptr(rows), loader.ptr(src), loader.ptr(w),
                                                     loader.ptr(drows), loader.ptr(dw), src.numel(), w.shape[1], rows.shape[1],
                                                     code(rows.dtype), loader.stream_ptr()), "moe_sum_rows_bwd")
         loader.launch_counter.add("moe_sum_rows_bwd")
-        return drows, dw.to(ctx.w_dtype), None, None
+        return drows, dw.to(weights.dtype), None, None

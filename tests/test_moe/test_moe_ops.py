@@ -288,3 +288,59 @@ def test_local_expert_rows(T, k, E, H, dtype):
     # w g rounded, times scale rounded, summed and rounded: three half steps of each term's size
     terms = w.detach().double()[..., None] * dout.double()[:, None] * scale.double()[want].view(T, k, 1)
     assert (dx.double() - terms.sum(1)).abs().le(1.6 * eps * terms.abs().sum(1) + 1e-6).all()
+
+
+def _plain_experts(H, E, dtype, device):
+    """Experts as ordinary torch operations over the grouped rows (a gain per expert), which differentiate any number of times."""
+    g = torch.Generator(device=device).manual_seed(3)
+    gain = torch.rand(E, H, device=device, generator=g).to(dtype)
+
+    def experts(rows, counts):
+        e = torch.repeat_interleave(torch.arange(E, device=device), counts)
+        e = torch.cat([e, e.new_zeros(rows.shape[0] - e.numel())])           # (a buffer's rows behind the last expert)
+        return torch.tanh(rows * gain.index_select(0, e))
+
+    return gain, experts
+
+
+def _dense(x, w, idx, gain):
+    return (torch.tanh(x.unsqueeze(1) * gain[idx]) * w.unsqueeze(-1)).sum(1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,k,E,H", [(1, 1, 1, 8), (50, 2, 5, 24), (200, 4, 40, 64)])
+def test_local_experts_second_order(T, k, E, H):
+    """`create_graph` through gather and combine: gradients of a function of the gradients, against float64."""
+    dt = torch.bfloat16
+    gain, experts = _plain_experts(H, E, dt, "cuda")
+    x = torch.randn(T, H, device="cuda").to(dt)
+    w, idx = torch.randn(T, E, device="cuda").softmax(-1).topk(k, -1)
+    dc.set_moe_backend("nccl")
+    try:
+        def both(x, w, f):
+            x, w = x.requires_grad_(), w.requires_grad_()
+            gx, gw = torch.autograd.grad(f(x, w).double().square().sum(), (x, w), create_graph=True)
+            return (gx, gw) + torch.autograd.grad((gx.double() ** 2).sum() + (gw.double() ** 2).sum(), (x, w))
+
+        got = both(x.clone(), w.clone(), lambda x, w: dc.moe_forward(x, w, idx, experts, E, None))
+        want = both(x.double(), w.double(), lambda x, w: _dense(x, w, idx, gain.double()))
+    finally:
+        dc.set_moe_backend("auto")
+    for a, b, what in zip(got, want, ("dx", "dw", "ddx", "ddw")):
+        # a chain of about eight results rounded to bf16
+        assert (a.double() - b).norm() <= 8 * 2.0 ** -8 * b.norm(), what
+
+
+@pytest.mark.gpu
+def test_local_experts_forward_mode():
+    """Forward-mode derivatives take the index operations, as they did before the kernels."""
+    from torch.autograd import forward_ad
+
+    T, k, E, H, dt = 40, 2, 6, 32, torch.bfloat16
+    gain, experts = _plain_experts(H, E, dt, "cuda")
+    x, dx = (torch.randn(T, H, device="cuda").to(dt) for _ in range(2))
+    w, idx = torch.randn(T, E, device="cuda").softmax(-1).topk(k, -1)
+    with forward_ad.dual_level():
+        y, dy = forward_ad.unpack_dual(dc.moe_forward(forward_ad.make_dual(x, dx), w, idx, experts, E, None))
+    want, dwant = torch.func.jvp(lambda t: _dense(t, w.double(), idx, gain.double()), (x.double(),), (dx.double(),))
+    assert (y.double() - want).norm() <= 4 * 2.0 ** -8 * want.norm() and (dy.double() - dwant).norm() <= 6 * 2.0 ** -8 * dwant.norm()
