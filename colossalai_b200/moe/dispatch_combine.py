@@ -14,7 +14,7 @@ import torch
 import torch.distributed as dist
 
 from ..ops._dispatch import plain_call, use_native
-from ..ops.moe import CombineRows, TakeRows, rows_ok, sort_choices
+from ..ops.moe import SORT_EXPERTS, CombineRows, TakeRows, rows_ok, sort_choices
 from ..parallel import comm
 from ._operation import AllToAllUneven
 from .grouped_gemm import ALIGN
@@ -95,10 +95,10 @@ def moe_forward(x: torch.Tensor, topk_w: torch.Tensor, topk_idx: torch.Tensor, e
     T, H = x.shape
     k = topk_idx.shape[1]
     ep = comm.group_size(ep_group) if ep_group is not None else 1     # None = no expert parallelism (NOT the world)
-    if ep == 1 and T > 0 and use_native(x) and _aligned_rows(x) and rows_ok(x) \
+    if ep == 1 and T > 0 and use_native(x) and _aligned_rows(x) and rows_ok(x) and num_experts <= SORT_EXPERTS \
             and plain_call(x, topk_w, topk_idx):
         # all experts here: the rows are sorted, gathered, combined and differentiated by kernels of their own, without a
-        # host synchronisation (`ops/moe.py`); the index operations below remain for CPU tensors, 32-bit rows, and for calls
+        # host synchronisation (`ops/moe.py`); the index operations below remain for CPU tensors, 32-bit rows, more experts than the sort has counters for, and for calls
         # that functorch, forward mode or a mode watches
         slot, src, counts = sort_choices(topk_idx, num_experts, ALIGN)
         counts.cb200_aligned = True

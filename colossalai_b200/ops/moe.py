@@ -217,6 +217,9 @@ def gather_combine(rows: torch.Tensor, row_of: torch.Tensor, weights: torch.Tens
 
 
 # ------------------------------------------------------------------------------------------------ local experts
+SORT_EXPERTS = 8192               # counters that the sort keeps in shared memory
+
+
 def sort_choices(topk_idx: torch.Tensor, num_experts: int, align: int):
     """topk_idx [T, k] on the GPU -> (slot int32 [T * k], src int32 [bound], counts int64 [E]): choice i's row sits at
     slot[i] of a buffer grouped by expert in which every expert's rows, in the order of their choices, are padded to a

@@ -344,3 +344,15 @@ def test_local_experts_forward_mode():
         y, dy = forward_ad.unpack_dual(dc.moe_forward(forward_ad.make_dual(x, dx), w, idx, experts, E, None))
     want, dwant = torch.func.jvp(lambda t: _dense(t, w.double(), idx, gain.double()), (x.double(),), (dx.double(),))
     assert (y.double() - want).norm() <= 4 * 2.0 ** -8 * want.norm() and (dy.double() - dwant).norm() <= 6 * 2.0 ** -8 * dwant.norm()
+
+
+@pytest.mark.gpu
+def test_more_experts_than_the_sort_counts():
+    E, T, H = mops.SORT_EXPERTS + 1, 5, 16
+    gain, experts = _plain_experts(H, E, torch.bfloat16, "cuda")
+    x = torch.randn(T, H, device="cuda").bfloat16()
+    idx = torch.randint(0, E, (T, 2), device="cuda")
+    idx[:, 1] = (idx[:, 0] + 1) % E
+    w = torch.rand(T, 2, device="cuda")
+    y, want = dc.moe_forward(x, w, idx, experts, E, None), _dense(x.double(), w.double(), idx, gain.double())
+    assert (y.double() - want).norm() <= 4 * 2.0 ** -8 * want.norm()
