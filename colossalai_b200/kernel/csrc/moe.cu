@@ -556,7 +556,8 @@ __global__ void __launch_bounds__(256) moe_take_rows_kernel(const uint4* __restr
   for (int c = lane; c < row_vecs; c += 32) d[c] = i < 0 ? make_uint4(0u, 0u, 0u, 0u) : __ldg(s + c);
 }
 
-// out[t] = sum_j w[t, j] rows[slot[t, j]] (w = null: plain sum), fp32, j ascending, one rounding
+// out[t] = sum_j w[t, j] rows[slot[t, j]] (w = null: plain sum), fp32, j ascending, one rounding.  A choice of no expert (slot
+// -1) cannot be refused without a host synchronisation: its weighted sum is NaN, so that it does not pass for a smaller one.
 template <typename T>
 __global__ void __launch_bounds__(256) moe_sum_rows_kernel(const T* __restrict__ rows, const int* __restrict__ slot,
                                                            const float* __restrict__ w, T* __restrict__ out, int k, int H) {
@@ -569,7 +570,13 @@ __global__ void __launch_bounds__(256) moe_sum_rows_kernel(const T* __restrict__
 #pragma unroll 4
     for (int j = 0; j < k; ++j) {
       const int r = __ldg(slot + t * k + j);
-      if (r < 0) continue;
+      if (r < 0) {
+        if (w != nullptr) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) acc[e] = __int_as_float(0x7fffffff);
+        }
+        continue;
+      }
       const float f = w != nullptr ? __ldg(w + t * k + j) : 1.f;
       Vec16<T> v;
       v.load_nc(rows + (int64_t)r * H + c);

@@ -356,3 +356,17 @@ def test_more_experts_than_the_sort_counts():
     w = torch.rand(T, 2, device="cuda")
     y, want = dc.moe_forward(x, w, idx, experts, E, None), _dense(x.double(), w.double(), idx, gain.double())
     assert (y.double() - want).norm() <= 4 * 2.0 ** -8 * want.norm()
+
+
+@pytest.mark.gpu
+def test_choices_of_no_expert_do_not_vanish():
+    T, k, E, H = 9, 2, 4, 64
+    gain, experts = _plain_experts(H, E, torch.bfloat16, "cuda")
+    x = torch.randn(T, H, device="cuda").bfloat16()
+    w, idx = torch.rand(T, k, device="cuda"), torch.randint(0, E, (T, k), device="cuda")
+    good = dc.moe_forward(x, w, idx, experts, E, None)
+    bad = idx.clone()
+    bad[2, 1], bad[5, 0] = -1, E
+    y = dc.moe_forward(x, w, bad, experts, E, None)
+    rows = [t for t in range(T) if t not in (2, 5)]
+    assert y[[2, 5]].isnan().all() and torch.equal(y[rows], good[rows])
