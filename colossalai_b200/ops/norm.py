@@ -142,8 +142,9 @@ class _LayerNormFn(torch.autograd.Function):
         grid = lib.cb_norm_bwd_grid(rows, H, code(weight.dtype))
         pw = torch.empty(grid, H, dtype=torch.float32, device=x2.device)
         pb = torch.empty_like(pw)
-        dw = torch.empty_like(weight)
-        db = torch.empty_like(weight) if ctx.has_bias else None
+        grad_like = torch.empty_like if rows else torch.zeros_like         # (nothing is launched for no rows)
+        dw = grad_like(weight)
+        db = grad_like(weight) if ctx.has_bias else None
         loader.check(lib.cb_layernorm_bwd(loader.ptr(dy2), loader.ptr(x2), loader.ptr(weight), loader.ptr(mean),
                                           loader.ptr(rstd), loader.ptr(dx), loader.ptr(pw), loader.ptr(pb),
                                           loader.ptr(dw), loader.ptr(db), 0, rows, H, code(x2.dtype),

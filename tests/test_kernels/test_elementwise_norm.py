@@ -46,6 +46,18 @@ def test_rmsnorm_fwd_bwd(dtype, shape, with_res):
     torch.testing.assert_close(w.grad.float(), wr.grad, **wt)
 
 
+@pytest.mark.parametrize("norm", ["rms", "layer", "layer_bias"])
+def test_norm_of_no_rows(norm):
+    """The gradients of the parameters are zero, not what the allocator's memory held."""
+    ps = [torch.ones(1024, device="cuda", requires_grad=True) for _ in range(2 if norm == "layer_bias" else 1)]
+    x = torch.zeros(0, 1024, device="cuda", requires_grad=True)
+    y = ops.rms_norm(x, ps[0]) if norm == "rms" else ops.layer_norm(x, *ps)
+    held = [torch.full((1024,), 7.0, device="cuda") for _ in range(8)]
+    del held
+    grads = torch.autograd.grad(y, [x] + ps, torch.zeros_like(y))
+    assert grads[0].shape == (0, 1024) and not any(g.any() for g in grads[1:])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("bias", [True, False])
 def test_layernorm_fwd_bwd(dtype, bias):
