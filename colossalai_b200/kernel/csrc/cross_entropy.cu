@@ -64,17 +64,24 @@ __global__ void __launch_bounds__(CE_THREADS) ce_row_stats_kernel(const T* __res
 __global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__ stats, const int64_t* __restrict__ target,
                                                        float* __restrict__ loss, int64_t* __restrict__ n_valid, int rows,
                                                        int64_t ignore_index, int mean) {
-  __shared__ float red[64];
-  float acc[2] = {0.f, 0.f};           // (up to 2^24 rows per thread are counted exactly)
+  __shared__ double sums[32];
+  __shared__ unsigned counts[32];
+  double acc = 0.0;
+  unsigned count = 0;                  // whole numbers: an fp32 count is exact up to 2^24 rows only
   for (int r = threadIdx.x; r < rows; r += blockDim.x)
     if (target[r] != ignore_index) {
-      acc[0] += (float)log((double)stats[rows + r]) + stats[r] - stats[2 * rows + r];   // (logf is approximate here)
-      acc[1] += 1.f;
+      acc += log((double)stats[rows + r]) + stats[r] - stats[2 * rows + r];               // (logf is approximate here)
+      ++count;
     }
-  block_sum<2>(acc, red);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  count = __reduce_add_sync(0xffffffffu, count);
+  if ((threadIdx.x & 31) == 0) { sums[threadIdx.x >> 5] = acc; counts[threadIdx.x >> 5] = count; }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    *n_valid = (int64_t)acc[1];
-    *loss = mean ? acc[0] / fmaxf(acc[1], 1.f) : acc[0];
+    for (int w = 1; w < (int)blockDim.x / 32; ++w) { acc += sums[w]; count += counts[w]; }
+    *n_valid = count;
+    *loss = (float)(mean ? acc / max(count, 1u) : acc);
   }
 }
 

@@ -1,4 +1,6 @@
 """Numerics of the sm_100a norm / activation / rope / CE kernels against plain PyTorch fp32 references."""
+import math
+
 import pytest
 import torch
 
@@ -205,6 +207,21 @@ def test_cross_entropy_one_pass_stats(dtype, V, valid):
     assert ((s.double() - ref).abs() <= 2e-5 * ref)[rows].all()
     assert torch.isneginf(m[5]) and s[5] == 0 and (valid <= V // 2 or torch.isnan(s[6]))
     assert torch.equal(tl[rows[:5]], x[rows[:5], 0].float()) and tl[7] == 0 and tl[8] == 0
+
+
+@pytest.mark.parametrize("mean", [True, False])
+@pytest.mark.parametrize("rows", [0, 1, 31, 1025, 2 ** 24 + 77])
+def test_cross_entropy_counts_labels(rows, mean):
+    """The number of labels is a whole number, also past 2^24."""
+    stats = torch.zeros(3, rows, device="cuda")
+    stats[1] = 2.0
+    t = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    t[: rows // 1000] = -100
+    n = rows - rows // 1000
+    loss, n_valid = ce.loss_from_stats(stats, t, -100, mean)
+    assert int(n_valid) == n
+    want = (n / max(n, 1) if mean else n) * math.log(2.0)
+    assert abs(float(loss) - want) <= 2.0 ** -23 * want                       # summed in 64 bits, rounded once
 
 
 def test_dist_cross_entropy_matches_torch():
