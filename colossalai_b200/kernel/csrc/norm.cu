@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_fwd_kernel(const T* __restrict__
 // Bound: HBM (three rows in, one out).  A block's rows follow one another through a reduction, so the next row is loaded before
 // the current one's sum is taken; without that 8192 x 4096 bf16 took 64.8 us (4.1 TB/s), with it 54.9.
 template <typename T, bool HAS_DRES, int MAX_ITERS>
-__global__ void __launch_bounds__(1024) rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ h,
+__global__ void __launch_bounds__(1024, 1) rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ h,
                                                            const T* __restrict__ w, const float* __restrict__ rstd,
                                                            const T* __restrict__ dres, T* __restrict__ dx,
                                                            float* __restrict__ dw_partial, int rows, int H) {
