@@ -57,12 +57,14 @@ __global__ void __launch_bounds__(1024) rmsnorm_fwd_kernel(const T* __restrict__
 // Bound: HBM (three rows in, one out).  A block's rows follow one another through a reduction, so the next row is loaded before
 // the current one's sum is taken; without that 8192 x 4096 bf16 took 64.8 us (4.1 TB/s), with it 54.9.
 template <typename T, bool HAS_DRES, int MAX_ITERS>
-__global__ void __launch_bounds__(1024, 1) rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ h,
+__global__ void __launch_bounds__(1024, MAX_ITERS == 1 && !HAS_DRES && sizeof(T) == 4 ? 2 : 1) rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ h,
                                                            const T* __restrict__ w, const float* __restrict__ rstd,
                                                            const T* __restrict__ dres, T* __restrict__ dx,
                                                            float* __restrict__ dw_partial, int rows, int H) {
   constexpr int VEC = Vec16<T>::N;
-  constexpr bool AHEAD = MAX_ITERS == 1;       // (wider rows fill the registers of a 1024-thread block as they are)
+  // Wider rows fill the registers of a 1024-thread block as they are; 32-bit rows without a second gradient need so few that two
+  // blocks of 1024 threads fit an SM, which the next row's registers would make one (16384 x 4096: 135 us without, 204 with).
+  constexpr bool AHEAD = MAX_ITERS == 1 && (HAS_DRES || VEC == 8);
   __shared__ float red[64];
   struct Row { Vec16<T> dy[MAX_ITERS], h[MAX_ITERS], dr[MAX_ITERS]; float rs; };
   auto fetch = [&](Row& v, int row) {
