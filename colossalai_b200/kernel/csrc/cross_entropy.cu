@@ -60,17 +60,30 @@ __global__ void __launch_bounds__(CE_THREADS) ce_row_stats_kernel(const T* __res
   }
 }
 
-// loss = sum over rows with a label of log(sumexp) + max - target logit, divided by their number (at least 1) when `mean`
+// loss = sum over rows with a label of log(sumexp) + max - target logit, divided by their number (at least 1) when `mean`.
+// One block up to CE_LOSS_ROWS rows; more rows are dealt out to up to CE_LOSS_BLOCKS blocks, whose sums a second launch adds up in
+// their order (131072 rows: one block
+// 130 us, now 3.6 and 2.4 to add them up; 16384 rows 17 us, 3.4 and 1.8).
+constexpr int CE_LOSS_ROWS = 2048, CE_LOSS_BLOCKS = 128;
+struct CePart {
+  double sum;
+  unsigned count;
+};
+CB_DEVICE void ce_loss_finish(double sum, unsigned count, int mean, float* loss, int64_t* n_valid) {
+  *n_valid = count;
+  *loss = (float)(mean ? sum / max(count, 1u) : sum);
+}
+
 __global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__ stats, const int64_t* __restrict__ target,
-                                                       float* __restrict__ loss, int64_t* __restrict__ n_valid, int rows,
-                                                       int64_t ignore_index, int mean) {
+                                                       float* __restrict__ loss, int64_t* __restrict__ n_valid,
+                                                       CePart* __restrict__ parts, int rows, int64_t ignore_index, int mean) {
   __shared__ double sums[32];
   __shared__ unsigned counts[32];
   double acc = 0.0;
   unsigned count = 0;                  // whole numbers: an fp32 count is exact up to 2^24 rows only
-  for (int r = threadIdx.x; r < rows; r += blockDim.x)
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x)
     if (target[r] != ignore_index) {
-      acc += log((double)stats[rows + r]) + stats[r] - stats[2 * rows + r];               // (logf is approximate here)
+      acc += log((double)stats[rows + r]) + stats[r] - stats[2 * (int64_t)rows + r];               // (logf is approximate here)
       ++count;
     }
 #pragma unroll
@@ -80,9 +93,20 @@ __global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < (int)blockDim.x / 32; ++w) { acc += sums[w]; count += counts[w]; }
-    *n_valid = count;
-    *loss = (float)(mean ? acc / max(count, 1u) : acc);
+    if (gridDim.x > 1) parts[blockIdx.x] = CePart{acc, count};
+    else ce_loss_finish(acc, count, mean, loss, n_valid);
   }
+}
+
+__global__ void __launch_bounds__(CE_LOSS_BLOCKS) ce_loss_join_kernel(const CePart* __restrict__ parts, int n, float* __restrict__ loss,
+                                                                      int64_t* __restrict__ n_valid, int mean) {
+  __shared__ CePart s[CE_LOSS_BLOCKS];
+  if ((int)threadIdx.x < n) s[threadIdx.x] = parts[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  CePart a = s[0];
+  for (int i = 1; i < n; ++i) { a.sum += s[i].sum; a.count += s[i].count; }
+  ce_loss_finish(a.sum, a.count, mean, loss, n_valid);
 }
 
 template <typename T>
@@ -130,9 +154,20 @@ int cb_ce_row_stats(const void* x, const int64_t* target, float* stats, int rows
   return CB_LAUNCH_CHECK();
 }
 
-int cb_ce_loss(const float* stats, const int64_t* target, float* loss, int64_t* n_valid, int rows, int64_t ignore_index, int mean,
-               cudaStream_t s) {
-  ce_loss_kernel<<<1, 1024, 0, s>>>(stats, target, loss, n_valid, rows, ignore_index, mean);
+// blocks of cb_ce_loss: its scratch `parts` is 16 bytes for each of them (none for one)
+int cb_ce_loss_blocks(int rows) {
+  if (rows <= CE_LOSS_ROWS) return 1;
+  const int blocks = rows / 1024 + (rows % 1024 != 0);
+  return blocks < CE_LOSS_BLOCKS ? blocks : CE_LOSS_BLOCKS;
+}
+
+int cb_ce_loss(const float* stats, const int64_t* target, float* loss, int64_t* n_valid, void* parts, int rows,
+               int64_t ignore_index, int mean, cudaStream_t s) {
+  static_assert(sizeof(CePart) == 16, "");
+  const int blocks = cb_ce_loss_blocks(rows);
+  if (blocks > 1 && parts == nullptr) return (int)cudaErrorInvalidValue;
+  ce_loss_kernel<<<blocks, 1024, 0, s>>>(stats, target, loss, n_valid, (CePart*)parts, rows, ignore_index, mean);
+  if (blocks > 1) ce_loss_join_kernel<<<1, CE_LOSS_BLOCKS, 0, s>>>((const CePart*)parts, blocks, loss, n_valid, mean);
   return CB_LAUNCH_CHECK();
 }
 

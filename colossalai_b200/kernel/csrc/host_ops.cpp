@@ -54,7 +54,8 @@ struct Launchers {
   int (*rope)(const void*, void*, const int64_t*, const float*, const float*, int64_t, int64_t, int, int, int, int, float, int, int,
               cudaStream_t);
   int (*row_stats)(const void*, const int64_t*, float*, int, int, int, int64_t, int64_t, int, cudaStream_t);
-  int (*ce_loss)(const float*, const int64_t*, float*, int64_t*, int, int64_t, int, cudaStream_t);
+  int (*ce_loss_blocks)(int);
+  int (*ce_loss)(const float*, const int64_t*, float*, int64_t*, void*, int, int64_t, int, cudaStream_t);
   int (*softmax_grad)(const void*, const int64_t*, const float*, const float*, const float*, const float*, const int64_t*, void*,
                       int, int, int, int64_t, int64_t, int, cudaStream_t);
   int (*flash_varlen_fwd)(const void*, const void*, const void*, void*, float*, const int*, int, long long, int, int, int, int,
@@ -194,8 +195,11 @@ struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
     const cudaStream_t s = stream_of(logits);
     launched(L.row_stats(ptr(logits), as<int64_t>(target), mut_as<float>(stats), rows, V, (int)valid, start, ignore, code_of(logits), s),
              n_stats);
-    launched(L.ce_loss(as<float>(stats), as<int64_t>(target), mut_as<float>(loss), mut_as<int64_t>(n_valid), rows, ignore, mean, s),
-             n_loss);
+    const int blocks = L.ce_loss_blocks(rows);
+    const Tensor parts = blocks > 1 ? at::empty({2 * blocks}, stats.options().dtype(at::kDouble)) : Tensor();
+    launched(L.ce_loss(as<float>(stats), as<int64_t>(target), mut_as<float>(loss), mut_as<int64_t>(n_valid), mut(parts), rows, ignore,
+                       mean, s),
+             n_loss, 1 + (blocks > 1));
     ctx->save_for_backward({logits, target, stats, n_valid});
     ctx->saved_data["args"] = std::vector<int64_t>{ignore, start, valid, (int64_t)mean};
     return loss;
@@ -293,6 +297,7 @@ void bind(const std::map<std::string, uint64_t>& t) {
   take(t, "cb_glu_bwd_bounded", L.glu_bwd);
   take(t, "cb_rope", L.rope);
   take(t, "cb_ce_row_stats", L.row_stats);
+  take(t, "cb_ce_loss_blocks", L.ce_loss_blocks);
   take(t, "cb_ce_loss", L.ce_loss);
   take(t, "cb_ce_softmax_grad", L.softmax_grad);
   take(t, "cb_flash_attn_varlen_fwd", L.flash_varlen_fwd);

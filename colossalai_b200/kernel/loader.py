@@ -204,7 +204,7 @@ def load(name: str) -> ctypes.CDLL:
 _HOST_CALLS = {
     "cb200_norm": ["cb_rmsnorm_fwd", "cb_rmsnorm_bwd", "cb_norm_bwd_grid"],
     "cb200_elementwise": ["cb_glu_fwd_bounded", "cb_glu_bwd_bounded", "cb_rope"],
-    "cb200_loss": ["cb_ce_row_stats", "cb_ce_loss", "cb_ce_softmax_grad"],
+    "cb200_loss": ["cb_ce_row_stats", "cb_ce_loss_blocks", "cb_ce_loss", "cb_ce_softmax_grad"],
     "cb200_attn": ["cb_flash_attn_varlen_fwd", "cb_flash_attn_bwd"],
     "cb200_infer": ["cb_decode_num_splits", "cb_paged_decode_attention"],
 }

@@ -82,10 +82,12 @@ def loss_from_stats(stats: torch.Tensor, target: torch.Tensor, ignore_index: int
         loss = torch.empty((), dtype=torch.float32, device=stats.device)
         n_valid = torch.empty((), dtype=torch.int64, device=stats.device)
         tgt = target if target.dtype == torch.int64 else target.long()
+        blocks = _get_lib().cb_ce_loss_blocks(stats.shape[1])
+        parts = torch.empty(2 * blocks, dtype=torch.float64, device=stats.device) if blocks > 1 else None
         loader.check(_get_lib().cb_ce_loss(loader.ptr(stats), loader.ptr(tgt.contiguous()), loader.ptr(loss),
-                                           loader.ptr(n_valid), stats.shape[1], ctypes.c_int64(ignore_index), int(mean),
-                                           loader.stream_ptr()), "ce_loss")
-        loader.launch_counter.add("ce_loss")
+                                           loader.ptr(n_valid), loader.ptr(parts), stats.shape[1], ctypes.c_int64(ignore_index),
+                                           int(mean), loader.stream_ptr()), "ce_loss")
+        loader.launch_counter.add("ce_loss", 1 + (blocks > 1))
         return loss, n_valid
     valid = target != ignore_index
     n_valid = valid.sum()

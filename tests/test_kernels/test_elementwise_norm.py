@@ -224,6 +224,24 @@ def test_cross_entropy_counts_labels(rows, mean):
     assert abs(float(loss) - want) <= 2.0 ** -23 * want                       # summed in 64 bits, rounded once
 
 
+@pytest.mark.parametrize("mean", [True, False])
+@pytest.mark.parametrize("rows", [2047, 2048, 2049, 5000, 8 * 1024, 128 * 1024 + 1, 300000])
+def test_cross_entropy_loss_of_many_rows(rows, mean):
+    """One block and several: the sum over the rows in 64 bits, rounded once, the same whenever it is taken."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    stats = torch.rand(3, rows, device="cuda", generator=g) + 0.5
+    t = torch.randint(-1, 3, (rows,), device="cuda", generator=g)
+    loss, n = ce.loss_from_stats(stats, t, -1, mean)
+    ok = t != -1
+    assert int(n) == int(ok.sum())
+    s = stats.double()
+    terms = (s[1].log() + s[0] - s[2])[ok]
+    want = terms.sum() / (int(n) if mean else 1)
+    # one rounding of the result, and 64-bit sums of at most 300000 terms in another order
+    assert abs(float(loss) - float(want)) <= 2.0 ** -24 * abs(float(want)) + 1e-11 * float(terms.abs().sum()) / (int(n) if mean else 1)
+    assert torch.equal(loss, ce.loss_from_stats(stats, t, -1, mean)[0])
+
+
 def test_dist_cross_entropy_matches_torch():
     from colossalai_b200.shardformer.layer.loss import cross_entropy_1d
 
