@@ -209,6 +209,23 @@ def test_cross_entropy_one_pass_stats(dtype, V, valid):
     assert torch.equal(tl[rows[:5]], x[rows[:5], 0].float()) and tl[7] == 0 and tl[8] == 0
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("vecs", [1, 31, 33, 127, 128, 129, 385, 1000, 2047, 2048, 2049])
+@pytest.mark.parametrize("short", [0, 1])
+def test_cross_entropy_stats_by_width(dtype, vecs, short):
+    """Every block size that a row's width asks for, with and without a last column that does not count."""
+    g = torch.Generator(device="cuda").manual_seed(vecs)
+    V = vecs * (4 if dtype == torch.float32 else 8)
+    x = (3 * torch.randn(5, V, device="cuda", generator=g)).to(dtype)
+    x[:, -1] = 30.0
+    t = torch.randint(0, V - short, (5,), device="cuda", generator=g)
+    m, s, tl = ce.row_stats(x, t, 0, -100, V - short)
+    x64 = x[:, : V - short].double()
+    assert torch.equal(m.double(), x64.max(-1).values) and torch.equal(tl, x[torch.arange(5), t].float())
+    ref = (x64 - x64.max(-1, keepdim=True).values).exp().sum(-1)
+    assert ((s.double() - ref).abs() <= 2e-5 * ref).all()        # approximate exponentials of 2^-21 each, fp32 sums
+
+
 @pytest.mark.parametrize("mean", [True, False])
 @pytest.mark.parametrize("rows", [0, 1, 31, 1025, 2 ** 24 + 77])
 def test_cross_entropy_counts_labels(rows, mean):
