@@ -308,3 +308,33 @@ def test_glu_row_limit():
     xr = x.detach()[:300].clone().requires_grad_(True)
     (gr,) = torch.autograd.grad(ops.glu(xr, "silu"), xr, dy[:300])
     torch.testing.assert_close(g[:300], gr, atol=0, rtol=0)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("heads,kv,D,rot,interleaved", [(1, 1, 16, 16, False), (2, 1, 32, 16, True), (1, 0, 16, 16, False), (12, 5, 32, 32, False),
+                                                       (16, 0, 32, 32, False), (32, 0, 32, 32, False), (33, 0, 32, 32, False)])
+@pytest.mark.parametrize("T", [1, 7, 1000])
+def test_rope_of_narrow_rows(dtype, heads, kv, D, rot, interleaved, T):
+    """Rows of which several share a block, up to and past the widest of them, with a last block that is not full."""
+    torch.manual_seed(T)
+    width = (heads + 2 * kv) * D
+    x = torch.randn(T, width, device="cuda").to(dtype).requires_grad_()
+    pos = torch.randint(0, 50, (T,), device="cuda")
+    cos, sin = ops.build_rope_cache(50, rot, 1e4, device="cuda")
+    y = ops.rope_qkv(x, pos, cos, sin, heads, kv, D, rot_dim=rot, interleaved=interleaved)
+    g = torch.randn_like(y)
+    dx, = torch.autograd.grad(y, x, g)
+
+    def turn(z, sign):
+        z = z.double().view(T, -1, D)
+        c, s = cos[pos].double()[:, None], sign * sin[pos].double()[:, None]
+        h = z[:, : heads + kv]
+        a, b = (h[..., 0:rot:2], h[..., 1:rot:2]) if interleaved else (h[..., : rot // 2], h[..., rot // 2: rot])
+        u, w = a * c - b * s, b * c + a * s
+        r = torch.stack([u, w], -1).flatten(-2) if interleaved else torch.cat([u, w], -1)
+        return torch.cat([torch.cat([r, h[..., rot:]], -1), z[:, heads + kv:]], 1).flatten(1)
+
+    eps = torch.finfo(dtype).eps
+    for got, src, sign in ((y, x, 1), (dx, g, -1)):
+        # two products of at most the largest entry each, rounded to fp32, and one rounding to the type
+        assert (got.double() - turn(src.detach(), sign)).abs().max() <= (0.51 * eps + 3 * 2.0 ** -24) * 1.5 * src.detach().abs().max()
