@@ -338,3 +338,26 @@ def test_rope_of_narrow_rows(dtype, heads, kv, D, rot, interleaved, T):
     for got, src, sign in ((y, x, 1), (dx, g, -1)):
         # two products of at most the largest entry each, rounded to fp32, and one rounding to the type
         assert (got.double() - turn(src.detach(), sign)).abs().max() <= (0.51 * eps + 3 * 2.0 ** -24) * 1.5 * src.detach().abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vecs", [1, 2, 3, 33, 64, 127, 128, 129])
+@pytest.mark.parametrize("rows,limit", [(1, None), (300, None), (300, 257)])
+def test_glu_of_narrow_rows(dtype, vecs, rows, limit):
+    """Rows of which several share a block, up to and past the widest of them; a last block that is not full; only the first
+    rows live."""
+    torch.manual_seed(vecs)
+    I = vecs * (4 if dtype == torch.float32 else 8)
+    gu = torch.randn(rows, 2 * I, device="cuda").to(dtype).requires_grad_()
+    g = torch.randn(rows, I, device="cuda").to(dtype)
+    valid = None if limit is None else torch.tensor([limit], device="cuda")
+    y = ops.glu(gu, "silu", valid_rows=valid)
+    dgu, = torch.autograd.grad(y, gu, g)
+    n = limit or rows
+    ref = gu.detach().double()[:n].requires_grad_()
+    a, b = ref.chunk(2, -1)
+    want = torch.nn.functional.silu(a) * b
+    dwant, = torch.autograd.grad(want, ref, g.double()[:n])
+    eps = max(torch.finfo(dtype).eps, 1e-5)                 # 32 bits: an approximate exponential and division
+    assert (y[:n].double() - want).abs().le(eps * want.abs() + 1e-6).all()
+    assert (dgu[:n].double() - dwant).abs().le(eps * dwant.abs() + 2e-5).all()
