@@ -673,6 +673,394 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   if (warp == 2) tmem_dealloc<C::TMEM_COLS>(tmem_base);
 }
 
+// One query tile per CTA, for calls whose tiles all find an SM at once: six warps (producer, issuer, four softmax warps of one
+// thread per row), two score buffers so that Q K^T of the next key tile runs under the softmax of this one, P through shared
+// memory.  With a single tile to walk the two-tile kernel has nothing to put under it - at heads of 128 its next Q K^T even
+// waits for P V - and the walk of a CTA is the call: 32 / 8 heads of 128, 256 / 512 tokens 15.7 / 21.3
+// us in the two-tile kernel, 8.8 / 13.1 here; 12 heads, 1024 tokens 29.5 and 20.5; 32 heads, 1024 tokens (256 tiles) 31 in both.
+constexpr int TILE_THREADS = 192, TILE_KV_STAGES = 2;
+template <int D> struct FaTileCfg {
+  static constexpr int Q_BYTES = BLOCK_Q * D * 2;
+  static constexpr int K_BYTES = BLOCK_KV * D * 2;
+  static constexpr int V_BYTES = BLOCK_KV * D * 2;
+  static constexpr int P_BYTES = BLOCK_Q * BLOCK_KV * 2;
+  static constexpr int KV_STAGE_BYTES = K_BYTES + V_BYTES;
+  static constexpr int SMEM_BYTES = Q_BYTES + TILE_KV_STAGES * KV_STAGE_BYTES + 2 * P_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int TMEM_COLS = 512;
+  static constexpr int O_COL = 256;
+};
+
+template <int D, bool EXTRA, bool BF16>
+__global__ void __launch_bounds__(TILE_THREADS, 1)
+flash_fwd_tile_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                 const __grid_constant__ CUtensorMap tmap_v, const FaParams p) {
+  using C = FaTileCfg<D>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem_q = smem;
+  uint8_t* smem_kv = smem + C::Q_BYTES;
+  uint8_t* smem_p = smem_kv + TILE_KV_STAGES * C::KV_STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_p + 2 * C::P_BYTES);
+  uint64_t* q_full = bars;                 // [1]
+  uint64_t* kv_full = bars + 1;            // [2]
+  uint64_t* kv_empty = bars + 3;           // [2]
+  uint64_t* s_full = bars + 5;             // [2]
+  uint64_t* s_empty = bars + 7;            // [2]  4 softmax warps
+  uint64_t* p_full = bars + 9;             // [1]  4 softmax warps
+  uint64_t* o_full = bars + 10;            // [1]
+  uint64_t* o_empty = bars + 11;           // [1]  4 softmax warps
+  uint64_t* drained = bars + 12;           // [1]  a CTA that gives up: its products have retired
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 13);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
+  volatile int* copies = abort_flag + 1;   // [1]  key / value tiles that the producer asked for
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int head = blockIdx.y;
+  const int kv_head = head / (p.hq / p.hkv);
+  int q_tile, seq_row0, len_q, len_k;
+  if (p.cu_seqlens != nullptr) {
+    // packed batch: blockIdx.x enumerates (sequence, query tile) pairs in order; surplus CTAs (the grid is sized for
+    // the worst case without knowing the lengths on the host) leave at once
+    int t = (int)blockIdx.x, bsel = -1, start = 0, len = 0;
+    for (int bb = 0; bb < p.batch; ++bb) {
+      start = p.cu_seqlens[bb];
+      len = p.cu_seqlens[bb + 1] - start;
+      const int nt = (len + BLOCK_Q - 1) / BLOCK_Q;
+      if (t < nt) { bsel = bb; break; }
+      t -= nt;
+    }
+    if (bsel < 0) return;                      // uniform across the CTA: nothing has been allocated yet
+    q_tile = t; seq_row0 = start; len_q = len; len_k = len;
+  } else {
+    // heaviest (longest causal) query tiles first
+    const int q_tiles = (p.seqlen_q + BLOCK_Q - 1) / BLOCK_Q;
+    q_tile = p.causal ? (q_tiles - 1 - (int)blockIdx.x) : (int)blockIdx.x;
+    seq_row0 = -1; len_q = p.seqlen_q; len_k = p.seqlen_k;
+  }
+  const int b = blockIdx.z;
+  const int q_row0 = (seq_row0 >= 0 ? seq_row0 : b * p.seqlen_q) + q_tile * BLOCK_Q;   // row in the token-major Q / O
+  const int kv_row0 = seq_row0 >= 0 ? seq_row0 : b * p.seqlen_k;
+  const int kv_tiles_all = (len_k + BLOCK_KV - 1) / BLOCK_KV;
+  // causal with seqlen_q == seqlen_k: key tiles 0..q_tile; otherwise all of them
+  const int kv_last = p.causal ? min(q_tile + 1, kv_tiles_all) : kv_tiles_all;   // one past the last visible key tile
+  // sliding window: the lowest key any row of this query tile can see is (q_tile * BLOCK_Q - window + 1)
+  const int kv_first = (EXTRA && p.window > 0) ? max(0, q_tile * BLOCK_Q - p.window + 1) / BLOCK_KV : 0;
+  const int kv_tiles = kv_last - kv_first;         // tiles walked; loop index j <-> key tile kv_first + j
+  const bool ragged_k = (len_k % BLOCK_KV) != 0;   // the last key tile runs past the end of the sequence
+  const bool resume = p.o_state != nullptr && p.has_prev != 0;   // block mode: continue from the stored state
+
+  if (warp == 0 && lane == 0) {
+    prefetch_tensormap(&tmap_q);
+    prefetch_tensormap(&tmap_k);
+    prefetch_tensormap(&tmap_v);
+  }
+  if (warp == 1 && lane == 0) {
+    mbar_init(q_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&kv_full[i], 1);
+      mbar_init(&kv_empty[i], 1);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&s_empty[i], 4);
+    }
+    mbar_init(p_full, 4);
+    mbar_init(o_full, 1);
+    mbar_init(o_empty, 4);
+    mbar_init(drained, 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 2) tmem_alloc<C::TMEM_COLS>(tmem_ptr_smem);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+  auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag)) != 0; };
+
+  if (warp == 0) {
+    // ================================================================ TMA producer
+    if (lane == 0) {
+      mbar_arrive_expect_tx(q_full, C::Q_BYTES);
+#pragma unroll
+      for (int h = 0; h < D / 64; ++h)                     // boxes [128 rows, 64 d] -> K-major swizzled sub-tiles
+        tma_load_2d(&tmap_q, q_full, smem_q + h * (BLOCK_Q * 128), head * D + h * 64, q_row0);
+    }
+    if (lane == 0) {
+      int j = 0;
+      for (; j < kv_tiles; ++j) {
+        const int stage = j % TILE_KV_STAGES;
+        if (!wait_or_abort(&kv_empty[stage], (uint32_t)(((j / TILE_KV_STAGES) & 1) ^ 1), abort_flag)) break;
+        uint8_t* sk = smem_kv + stage * C::KV_STAGE_BYTES;
+        uint8_t* sv = sk + C::K_BYTES;
+        mbar_arrive_expect_tx(&kv_full[stage], C::KV_STAGE_BYTES);
+        const int row = kv_row0 + (kv_first + j) * BLOCK_KV;
+#pragma unroll
+        for (int h = 0; h < D / 64; ++h) {
+          tma_load_2d(&tmap_k, &kv_full[stage], sk + h * (BLOCK_KV * 128), kv_head * D + h * 64, row);   // K-major B
+          tma_load_2d(&tmap_v, &kv_full[stage], sv + h * (BLOCK_KV * 128), kv_head * D + h * 64, row);   // MN-major B
+        }
+      }
+      *copies = j;
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ================================================================ MMA issuer
+    const uint32_t sq = smem_u32(smem_q);
+    const uint32_t sp = smem_u32(smem_p);
+    const uint64_t dq = make_smem_desc_sw128(sq, 16, 1024);                       // K-major, K = D
+    const uint64_t dp = make_smem_desc_sw128(sp, 16, 1024);                       // K-major, K = keys
+    if (lane == 0) {
+      auto issue_qk = [&](int j) -> bool {
+        const int stage = j % TILE_KV_STAGES;
+        const int sb = j & 1;
+        if (!wait_or_abort(&kv_full[stage], (uint32_t)((j / TILE_KV_STAGES) & 1), abort_flag)) return false;
+        if (!wait_or_abort(&s_empty[sb], (uint32_t)(((j >> 1) & 1) ^ 1), abort_flag)) return false;
+        tc_fence_after();
+        const uint64_t dk = make_smem_desc_sw128(smem_u32(smem_kv + stage * C::KV_STAGE_BYTES), 16, 1024);
+#pragma unroll
+        for (int k = 0; k < D / UMMA_K; ++k) {
+          const uint32_t off = (k >> 2) * (128 * 128) + (k & 3) * (UMMA_K * 2);
+          umma_f16_ss(tmem_base + sb * BLOCK_KV, advance_desc(dq, off), advance_desc(dk, off), p.idesc_qk, k > 0 ? 1u : 0u);
+        }
+        umma_commit(&s_full[sb]);
+        return true;
+      };
+      bool ok = wait_or_abort(q_full, 0, abort_flag) && issue_qk(0);
+      for (int j = 0; j < kv_tiles && ok; ++j) {
+        if (j + 1 < kv_tiles) ok = issue_qk(j + 1);         // tensor pipe works on the next scores during softmax(j)
+        const int stage = j % TILE_KV_STAGES;
+        ok = ok && wait_or_abort(p_full, (uint32_t)(j & 1), abort_flag);   // P_j is in shared memory, O rescaled if it had to be
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t sv = smem_u32(smem_kv + stage * C::KV_STAGE_BYTES + C::K_BYTES);
+        const uint64_t dv = make_smem_desc_sw128(sv, BLOCK_KV * 128, 1024);          // MN-major: [keys, D] row-major
+        const uint64_t dpj = advance_desc(dp, (uint32_t)(j & 1) * C::P_BYTES);
+        // O accumulates in TMEM over all key tiles (the first MMA of the first tile overwrites, unless the accumulator was
+        // pre-loaded with the state of earlier launches)
+        const bool fresh = (j == 0) && !resume;
+#pragma unroll
+        for (int k = 0; k < BLOCK_KV / UMMA_K; ++k) {
+          const uint32_t ao = (k >> 2) * (128 * 128) + (k & 3) * (UMMA_K * 2);
+          umma_f16_ss(tmem_base + C::O_COL, advance_desc(dpj, ao), advance_desc(dv, k * (UMMA_K * 128)), p.idesc_pv,
+                      (fresh && k == 0) ? 0u : 1u);
+        }
+        umma_commit(o_full);
+        umma_commit(&kv_empty[stage]);                      // K_j and V_j are consumed once P_j V_j has retired
+      }
+    }
+    __syncwarp();
+  } else {
+    // ================================================================ softmax + output (warps 2..5)
+    // Thread = query row.  The output accumulator lives in TMEM for the whole walk (P_j V_j accumulates onto it in the
+    // tensor core); the exponentials are taken against a LAGGING row max: the accumulator is only rescaled when the
+    // true max has grown by more than 2^TAU since the last rescale (exact: numerator and denominator use the same
+    // reference, which is what the log-sum-exp is reported against).  Per key tile a thread therefore reads its 128
+    // scores ONCE (four tcgen05.ld in flight, one wait), releases the score buffer at once, and touches the
+    // accumulator only on the rare rescale.
+    constexpr float TAU = 8.f;
+    const int quarter = warp & 3;                        // TMEM lane quarter this warp may access
+    const int r = quarter * 32 + lane;                   // query row inside the tile
+    const int q_pos = q_tile * BLOCK_Q + r;              // position inside the sequence
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    const uint32_t o_addr = tmem_base + lane_addr + C::O_COL;
+    float m_run = -INFINITY;                             // reference max of the exponentials (exp2 domain)
+    float l_run = 0.f;
+    if (resume) {
+      // resume from the merged result of the key blocks processed by earlier launches (normalised output + LSE):
+      // every row stores its previous output (or zeros) into the TMEM accumulator, P_0 V_0 accumulates onto it
+      const size_t row_ = (size_t)q_row0 + r;
+      float lse_prev = -INFINITY;
+      if (q_pos < len_q) lse_prev = p.lse[row_ * p.hq + head];
+      const bool live = lse_prev > -INFINITY;
+      if (live) { m_run = lse_prev * 1.4426950408889634f; l_run = 1.f; }
+      const float4* src = reinterpret_cast<const float4*>(p.o_state + row_ * ((size_t)p.hq * D) + (size_t)head * D);
+#pragma unroll
+      for (int c = 0; c < D; c += 16) {
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 t4 = live ? src[(c >> 2) + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+          w[4 * i] = __float_as_uint(t4.x); w[4 * i + 1] = __float_as_uint(t4.y);
+          w[4 * i + 2] = __float_as_uint(t4.z); w[4 * i + 3] = __float_as_uint(t4.w);
+        }
+        tmem_st_32x32b_x16(o_addr + c, w);
+      }
+      tmem_st_wait();
+    }
+    const float slope2 = (EXTRA && p.alibi != nullptr) ? p.alibi[head] * 1.4426950408889634f : 0.f;
+    (void)slope2;
+    bool ok = true;                                      // this thread's waits so far
+    int j = 0;
+    for (; j < kv_tiles; ++j) {
+      const int sb = j & 1;
+      ok = ok && wait_or_abort(&s_full[sb], (uint32_t)((j >> 1) & 1), abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      tc_fence_after();
+      const uint32_t s_addr = tmem_base + lane_addr + sb * BLOCK_KV;
+      const int kt = kv_first + j;                                       // key tile of this step
+      const bool diag = p.causal && (kt == q_tile);
+      const bool tail_k = ragged_k && (kt == kv_tiles_all - 1);
+      const bool masked = diag || tail_k || (EXTRA && p.window > 0);
+      const int k_lim = diag ? min(q_pos, len_k - 1) : (len_k - 1);      // last visible key position of this row
+      const int k_low = (EXTRA && p.window > 0) ? q_pos - p.window + 1 : 0;   // first visible key position
+      const int k_base = kt * BLOCK_KV;
+      // ---- the whole score row into registers
+      uint32_t v[BLOCK_KV];
+#pragma unroll
+      for (int c = 0; c < BLOCK_KV; c += 32) tmem_ld_32x32b_x32(s_addr + c, *reinterpret_cast<uint32_t(*)[32]>(&v[c]));
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_empty[sb]);          // S buffer may be overwritten by Q K_{j+2}^T
+      // plain variant: the softmax scale (> 0) is folded into the exponent's FMA, the max is taken on the raw scores;
+      // EXTRA variant: scale and ALiBi bias are applied here and the exponent uses a unit multiplier
+      // (four independent partial maxima / sums: a single running value would be a 128-long dependent chain)
+      float mt[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int i = 0; i < BLOCK_KV; ++i) {
+        float sc = __uint_as_float(v[i]);
+        if (EXTRA) sc = fmaf(slope2, (float)(k_base + i - q_pos), sc * p.scale_log2);
+        if (masked && ((k_base + i) > k_lim || (EXTRA && (k_base + i) < k_low))) sc = -INFINITY;
+        v[i] = __float_as_uint(sc);
+        mt[i & 3] = fmaxf(mt[i & 3], sc);
+      }
+      float m_tile = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3]));
+      const float ex_mul = EXTRA ? 1.f : p.scale_log2;
+      m_tile *= ex_mul;
+      // ---- lagging max / rare rescale of the TMEM accumulator
+      const float m_new = fmaxf(m_run, m_tile);
+      if (j == 0 && !resume) {
+        m_run = m_new;                                   // nothing accumulated yet
+      } else {
+        const bool need = (m_new - m_run) > TAU;         // (-inf) - (-inf) = NaN -> false
+        if (__any_sync(0xffffffffu, need)) {
+          if (j > 0) {                                   // P_{j-1} V_{j-1} has retired: the accumulator is stable
+            if (!warp_wait(o_full, (uint32_t)((j - 1) & 1))) break;
+            tc_fence_after();
+          }
+          const float alpha = need ? fast_exp2(m_run - m_new) : 1.f;
+#pragma unroll 1
+          for (int c = 0; c < D; c += 32) {
+            uint32_t t[32];
+            tmem_ld_32x32b_x32(o_addr + c, t);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
+            tmem_st_32x32b_x16(o_addr + c, *reinterpret_cast<uint32_t(*)[16]>(&t[0]));
+            tmem_st_32x32b_x16(o_addr + c + 16, *reinterpret_cast<uint32_t(*)[16]>(&t[16]));
+          }
+          tmem_st_wait();
+          l_run *= alpha;
+          if (need) m_run = m_new;
+        }
+      }
+      const float m_use = (m_run == -INFINITY) ? 0.f : m_run;     // keeps the exponent finite on a fully masked row
+      // ---- p = exp2(s - m), row sum, 16-bit P into the swizzled K-major tile of buffer j & 1
+      // (that buffer was last read by P_{j-2} V_{j-2}, which retired before Q K_j^T - issued after it - completed)
+      uint8_t* p_row = smem_p + (j & 1) * C::P_BYTES + r * 128;
+      float lt[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < BLOCK_KV; c += 32) {
+        uint32_t packed[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const float p0 = fast_exp2(fmaf(__uint_as_float(v[c + i]), ex_mul, -m_use));
+          const float p1 = fast_exp2(fmaf(__uint_as_float(v[c + i + 1]), ex_mul, -m_use));
+          lt[(i >> 1) & 3] += p0 + p1;
+          packed[i >> 1] = pack_16<BF16>(p0, p1);
+        }
+        // 32 keys = 64 bytes = four 16-byte chunks of this row inside sub-tile (c / 64)
+        uint8_t* sub = p_row + (c >> 6) * (BLOCK_Q * 128);
+        const int chunk0 = (c & 32) ? 4 : 0;
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4) {
+          const int chunk = (chunk0 + q4) ^ (r & 7);     // SWIZZLE_128B: 16-byte chunk index XOR (row mod 8)
+          *reinterpret_cast<uint4*>(sub + chunk * 16) =
+              make_uint4(packed[q4 * 4], packed[q4 * 4 + 1], packed[q4 * 4 + 2], packed[q4 * 4 + 3]);
+        }
+      }
+      const float l_tile = (lt[0] + lt[1]) + (lt[2] + lt[3]);
+      l_run += l_tile;
+      // keep in step with the accumulator barrier: observe "P_{j-1} V_{j-1} retired" once per tile.  It completed long
+      // ago in the common case (no stall), but a parity wait is only unambiguous while the waiter is at most ONE phase
+      // behind - the epilogue's wait for the last tile would otherwise pass on the phase before the previous one
+      // (seen on hardware with two-tile launches: output read before the last two P V had landed).
+      if (j > 0) ok = wait_or_abort(o_full, (uint32_t)((j - 1) & 1), abort_flag);
+      tc_fence_before();
+      fence_proxy_async();                               // generic-proxy smem writes -> visible to the tensor core
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);                // P_j is in shared memory, the accumulator is consistent
+    }
+    // ---- epilogue: the last P V has retired; normalise and store this thread's row
+    ok = __all_sync(0xffffffffu, ok && j == kv_tiles && wait_or_abort(o_full, (uint32_t)((kv_tiles - 1) & 1), abort_flag));
+    tc_fence_after();
+    const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
+    const size_t row = (size_t)q_row0 + r;
+    const bool row_ok = q_pos < len_q;                   // rows past the end of a (packed) sequence are never stored
+#pragma unroll 1
+    for (int c = 0; c < D && ok; c += 32) {
+      uint32_t t[32];
+      __syncwarp();
+      tmem_ld_32x32b_x32(o_addr + c, t);                 // executed by every lane (warp-collective), stores predicated
+      tmem_ld_wait();
+      if (!row_ok) {
+        // a row past the end of its (packed) sequence: computed on garbage, never stored
+      } else if (p.o_state != nullptr) {
+        float4* dst = reinterpret_cast<float4*>(p.o_state + row * ((size_t)p.hq * D) + (size_t)head * D + c);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          dst[i] = make_float4(__uint_as_float(t[4 * i]) * inv_l, __uint_as_float(t[4 * i + 1]) * inv_l,
+                               __uint_as_float(t[4 * i + 2]) * inv_l, __uint_as_float(t[4 * i + 3]) * inv_l);
+      } else {
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          w[i] = pack_16<BF16>(__uint_as_float(t[2 * i]) * inv_l, __uint_as_float(t[2 * i + 1]) * inv_l);
+        uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) +
+                                              (row * ((size_t)p.hq * D) + (size_t)head * D + c) * 2);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+      }
+    }
+    if (ok && p.lse && row_ok)
+      p.lse[row * p.hq + head] = l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {                         // (nothing writes it any more: uniform) leave nothing in flight behind
+    int none = 0;
+    if (warp == 0 && lane == 0) {
+      wait_or_abort(q_full, 0, &none);
+      for (int i = max(0, *copies - TILE_KV_STAGES); i < *copies; ++i) {
+        none = 0;
+        wait_or_abort(&kv_full[i % TILE_KV_STAGES], (uint32_t)((i / TILE_KV_STAGES) & 1), &none);
+      }
+    }
+    if (warp == 1 && lane == 0) {            // the thread that issued the products
+      umma_commit(drained);
+      wait_or_abort(drained, 0, &none);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) report_abort(p.status);
+  }
+  if (warp == 2) tmem_dealloc<C::TMEM_COLS>(tmem_base);
+}
+
+template <int D, bool EXTRA, bool BF16>
+int launch_flash_fwd_tile_kernel(dim3 grid, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p,
+                                 cudaStream_t stream) {
+  using C = FaTileCfg<D>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(flash_fwd_tile_kernel<D, EXTRA, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         C::SMEM_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
+  flash_fwd_tile_kernel<D, EXTRA, BF16><<<grid, TILE_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  return (int)cudaGetLastError();
+}
+
 template <int D, bool EXTRA, bool BF16>
 int launch_flash_fwd_kernel(dim3 grid, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p,
                             cudaStream_t stream) {
@@ -713,6 +1101,21 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* out, flo
   p.window = window; p.alibi = alibi;
   p.idesc_qk = make_idesc_f16(BLOCK_Q, BLOCK_KV, bf16 ? 1 : 0, 0, 0);      // S[128 x 128] = Q (K-major) x K (K-major)
   p.idesc_pv = make_idesc_f16(BLOCK_Q, D, bf16 ? 1 : 0, 0, 1);              // O[128 x D]  = P (K-major) x V (MN-major)
+  // Few tiles: one each.  Packed batches have between max(total / BLOCK_Q, batch) and total / BLOCK_Q + batch of them per head.  The
+  // walks of causal tiles differ in length, so half as many again still fit beside the longest, unless many short sequences
+  // fill the SMs evenly (12 heads of 128: one causal sequence of 2048 tokens, 192 tiles, 44 us here and 47 by twos; without the
+  // mask 64 and 49; 4 x 512 tokens 20 and 18).
+  const long long blocks = (cu_seqlens ? total_tokens + BLOCK_Q - 1 : (long long)seqlen_q + BLOCK_Q - 1) / BLOCK_Q;
+  const long long tiles = cu_seqlens ? total_tokens / BLOCK_Q + batch : blocks;
+  const long long few = (cu_seqlens ? (blocks > batch ? blocks : batch) : blocks * batch) * hq;
+  if (few <= cb_num_sms() || (causal && (cu_seqlens || batch == 1) && few <= cb_num_sms() * 3 / 2)) {
+    const dim3 grid((unsigned)tiles, hq, cu_seqlens ? 1 : batch);
+    if (window > 0 || alibi != nullptr)
+      return bf16 ? launch_flash_fwd_tile_kernel<D, true, true>(grid, tq, tk, tv, p, stream)
+                  : launch_flash_fwd_tile_kernel<D, true, false>(grid, tq, tk, tv, p, stream);
+    return bf16 ? launch_flash_fwd_tile_kernel<D, false, true>(grid, tq, tk, tv, p, stream)
+                : launch_flash_fwd_tile_kernel<D, false, false>(grid, tq, tk, tv, p, stream);
+  }
   // units of `per` query rows; packed: at most total / per + batch of them exist per head
   const int per = p.pair_heads ? BLOCK_Q : 2 * BLOCK_Q;
   p.head_units = p.pair_heads ? hq / 2 : hq;
