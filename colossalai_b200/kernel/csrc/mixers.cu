@@ -266,22 +266,43 @@ struct ScanParams {
 constexpr int SCAN_CPL = 4;            // value columns per lane
 constexpr int SCAN_COLS = 32;          // value columns per CTA
 
-template <int DK, int MODE> struct ScanTile {
+// Two rows of a column of S: one register pair for the instructions that do two fp32 operations (long portions), or two numbers
+// that a row's load fills as they come - packing them holds up the state's loads, and those are what a short portion is.  The
+// roundings are the same.
+struct alignas(8) ScanTwo {
+  float a, b;
+};
+
+template <int DK, int MODE, bool SHORT> struct ScanTile {
   // Lanes that share the rows of a column group.  More lanes are shorter steps for each and more warps to hide them behind, at
   // more shuffles and reads of the values.  Decay mode, 16 heads, 12000 tokens, with 8 and with 16 lanes: 128 x 128, one
   // sequence 2.69 and 1.70 ms, eight uneven ones 802 and 701 us; 64 x 64, eight sequences 385 and 278 us.
-  static constexpr int PARTS = DK <= 16 ? 4 : DK <= (MODE == SCAN_DECAY ? 32 : 128) ? 8 : 16;
+  static constexpr int LANES = DK <= 16 ? 4 : DK <= (MODE == SCAN_DECAY ? 32 : 128) ? 8 : 16;
+  // A short portion is little more than the read and the write of the state, for which 8 lanes are enough; a lane then keeps its
+  // sums of the rows of two apart, so that they are joined in the same order.
+  static constexpr int PARTS = SHORT && DK <= 128 && LANES == 16 ? 8 : LANES, SPLIT = LANES / PARTS;
   static constexpr int RP = DK / PARTS;                                 // rows per lane
   static constexpr int RPP = RP == 4 ? 4 : RP + 4;                      // a lane's rows in shared memory start this far apart:
   static constexpr int DKP = PARTS * RPP;                               // the 16-byte reads of 8 lanes hit different banks
   static constexpr int THREADS = PARTS * SCAN_COLS / SCAN_CPL;
-  // Units that an SM is to hold at a time, by their registers: four tokens' reads want more than 128 of a lane, and at 255 an SM
-  // holds two of the 128 wide units, so that eight sequences take two rounds (either 13 % slower).
-  static constexpr int BLOCKS = MODE != SCAN_DECAY || DK > 128 ? 1 : (DK == 128 ? 384 : 512) / THREADS;
-  static constexpr int STAGES = MODE == SCAN_DECAY ? 3 : 2;
+  static constexpr int TPI = THREADS / (DK / 4);                        // tokens that one round of copies covers
+  static constexpr int TILE = SHORT && TPI < 4 ? 4 : SCAN_TOK_TILE;     // tokens per stage
+  // Units that an SM is to hold at a time, by their registers.  A long portion: four tokens' reads want more than 128 of a lane,
+  // and at 255 an SM holds two of the 128 wide units, so that eight sequences take two rounds (either 13 % slower).  A short
+  // one: as much of the states on its way as can be.  256 decoded tokens, 16 heads x 128 x 128, decay / rows / delta mode: 241 /
+  // 271 / 266 us in the long form (three or four units per SM, two rows packed as they come), 154 / 157 / 167 in the short one.
+  static constexpr int LONG_BLOCKS = MODE != SCAN_DECAY || DK > 128 ? 1 : (DK == 128 ? 384 : 512) / THREADS;
+  static constexpr int SHORT_BLOCKS = (RP > 8 ? (MODE == SCAN_DELTA ? 384 : 512) : RP == 8 ? (MODE == SCAN_DELTA ? 512 : 768) : 1024) / THREADS;
+  static constexpr int BLOCKS = SHORT ? SHORT_BLOCKS : LONG_BLOCKS;
+  static constexpr int STAGES = MODE == SCAN_DECAY && !SHORT ? 3 : 2;
   static constexpr int NROW = MODE == SCAN_DELTA || MODE == SCAN_ROWS ? 3 : 2;          // q, k, decay rows
   static constexpr int TOKEN = NROW * DKP + SCAN_COLS + 4;              // floats per token: rows, values, scalars
+  using Pair = typename std::conditional<SHORT, ScanTwo, uint64_t>::type;
+  struct alignas(16) Quad { Pair x, y; };                               // four rows as they lie in shared memory
 };
+// Tokens of the longest portion up to which the short form is taken.  64 sequences, decay / rows / delta mode: of 32 tokens 118 /
+// 131 / 163 us in it, 129 / 139 / 180 in the long one; of 64 tokens 200 / 222 / 298, 203 / 216 / 303; eight of 100 58 / 63 / 82, 47 / 46 / 64.
+constexpr int SCAN_SHORT = 32;
 
 struct ScanWork {
   float *q, *k, *g, *beta, *v;         // [T, qk_heads, DK] x2, [T, heads, DK], [T, heads], [T, heads, VP]
@@ -510,7 +531,8 @@ __global__ void __launch_bounds__(128) exp_gate_kernel(ScanParams p, ScanWork w,
 }
 
 // two fp32 operations in one instruction, each rounded as the single one
-CB_DEVICE uint64_t pair_of(float a, float b) {
+template <typename P> CB_DEVICE P pair_of(float a, float b);
+template <> CB_DEVICE uint64_t pair_of<uint64_t>(float a, float b) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
   return r;
@@ -530,6 +552,11 @@ CB_DEVICE uint64_t mul2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+
+template <> CB_DEVICE ScanTwo pair_of<ScanTwo>(float a, float b) { return ScanTwo{a, b}; }
+CB_DEVICE float2 halves(ScanTwo v) { return make_float2(v.a, v.b); }
+CB_DEVICE ScanTwo fma2(ScanTwo a, ScanTwo b, ScanTwo c) { return ScanTwo{__fmaf_rn(a.a, b.a, c.a), __fmaf_rn(a.b, b.b, c.b)}; }
+CB_DEVICE ScanTwo mul2(ScanTwo a, ScanTwo b) { return ScanTwo{__fmul_rn(a.a, b.a), __fmul_rn(a.b, b.b)}; }
 
 // The sequence and the unit of it (head and block of columns; `units` per sequence) that a CTA walks.  A unit takes as long as
 // its sequence, and all are resident at once in a usual step, so what a step takes is the SM with the most tokens.  Up to 32
@@ -555,15 +582,20 @@ CB_DEVICE void scan_unit(const ScanParams& p, int nseq, int units, int sms, int&
   s = __ffs(__ballot_sync(0xffffffffu, lane < nseq && place == want)) - 1;
 }
 
-template <int DK, int MODE>
-__global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE>::BLOCKS) state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
-  constexpr int PARTS = ScanTile<DK, MODE>::PARTS, RP = ScanTile<DK, MODE>::RP, RPP = ScanTile<DK, MODE>::RPP, DKP = ScanTile<DK, MODE>::DKP;
-  constexpr int THREADS = ScanTile<DK, MODE>::THREADS;
+template <int DK, int MODE, bool SHORT>
+__global__ void __launch_bounds__(ScanTile<DK, MODE, SHORT>::THREADS, ScanTile<DK, MODE, SHORT>::BLOCKS)
+state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
+  using Tile = ScanTile<DK, MODE, SHORT>;
+  constexpr int PARTS = Tile::PARTS, RP = Tile::RP, RPP = Tile::RPP, DKP = Tile::DKP, TILE = Tile::TILE;
+  constexpr int THREADS = Tile::THREADS, SPLIT = Tile::SPLIT;
+  static_assert(SPLIT == 1 || MODE == SCAN_DECAY, "the delta rule's first sum is not split");
   constexpr bool ROWS = MODE == SCAN_DELTA || MODE == SCAN_ROWS;        // decay rows beside q and k
-  constexpr int NROW = ScanTile<DK, MODE>::NROW, STAGES = ScanTile<DK, MODE>::STAGES;
-  constexpr int STAGE = SCAN_TOK_TILE * ScanTile<DK, MODE>::TOKEN;      // floats per stage
+  constexpr int NROW = Tile::NROW, STAGES = Tile::STAGES;
+  constexpr int STAGE = TILE * Tile::TOKEN;                             // floats per stage
   constexpr int NTOK = PARTS / SCAN_CPL;                                // tokens whose sums are exchanged together
   constexpr unsigned ALL = 0xffffffffu;
+  using P = typename Tile::Pair;                                        // two rows of a column
+  using Quad = typename Tile::Quad;
   extern __shared__ __align__(16) float scan_smem[];
   const int vblocks = w.VP / SCAN_COLS;
   int s, unit;
@@ -582,7 +614,7 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
   const bool carried = p.ctx_len[s] > 0;
   // Pairs of neighbouring ROWS share an instruction: q, k and the decays arrive from shared memory as such pairs, and only the
   // token's SCAN_CPL values are duplicated.
-  uint64_t S[RP / 2][SCAN_CPL];
+  P S[RP / 2][SCAN_CPL];
 #pragma unroll
   for (int i = 0; i < RP; i += 2) {
     float x[2][SCAN_CPL];
@@ -599,17 +631,17 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
       }
     }
 #pragma unroll
-    for (int c = 0; c < SCAN_CPL; ++c) S[i / 2][c] = pair_of(x[0][c], x[1][c]);
+    for (int c = 0; c < SCAN_CPL; ++c) S[i / 2][c] = pair_of<P>(x[0][c], x[1][c]);
   }
   const float hd = MODE == SCAN_DECAY ? p.head_decay[h] : 0.f;
   const float skip = (MODE == SCAN_GATED && p.head_decay != nullptr) ? p.head_decay[h] : 0.f;
 
   // A thread copies the same 16-byte piece of every (THREADS / pieces)-th token: its addresses only step, which keeps the
   // copies to three instructions each (with an address computed per copy they were a tenth of what the kernel issued).
-  constexpr int CH = DK / 4, TPI = THREADS / CH, VCH = SCAN_COLS / 4, VPI = THREADS / VCH;
-  static_assert(THREADS % CH == 0 && TPI <= SCAN_TOK_TILE && THREADS % VCH == 0, "");
+  constexpr int CH = DK / 4, TPI = Tile::TPI, VCH = SCAN_COLS / 4, VPI = THREADS / VCH;
+  static_assert(THREADS % CH == 0 && TPI <= TILE && THREADS % VCH == 0, "");
   const int qt = threadIdx.x / CH, qc = (threadIdx.x % CH) * 4, vt = threadIdx.x / VCH, vc = (threadIdx.x % VCH) * 4;
-  const int qdst = qt * DKP + qc / RP * RPP + qc % RP, vdst = NROW * SCAN_TOK_TILE * DKP + vt * SCAN_COLS + vc;
+  const int qdst = qt * DKP + qc / RP * RPP + qc % RP, vdst = NROW * TILE * DKP + vt * SCAN_COLS + vc;
   const int64_t qstep = (int64_t)p.qk_heads * DK, gstep = (int64_t)p.heads * DK, vstep = (int64_t)p.heads * w.VP;
   const float* qsrc = w.q + (t0 + qt) * qstep + hk * DK + qc;
   const float* ksrc = w.k + (t0 + qt) * qstep + hk * DK + qc;
@@ -617,28 +649,28 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
   const float* vsrc = w.v + (t0 + vt) * vstep + h * w.VP + vb * SCAN_COLS + vc;
   auto load_tile = [&](int stage, int tb) {      // tiles are asked for in order
     float* base = scan_smem + stage * STAGE;
-    const int nt = max(min(SCAN_TOK_TILE, t1 - tb), 0);
+    const int nt = max(min(TILE, t1 - tb), 0);
 #pragma unroll
-    for (int i = 0; i < SCAN_TOK_TILE; i += TPI) {
+    for (int i = 0; i < TILE; i += TPI) {
       if (qt + i < nt) {
         cp_async16f(base + qdst + i * DKP, qsrc);
-        cp_async16f(base + SCAN_TOK_TILE * DKP + qdst + i * DKP, ksrc);
-        if (ROWS) cp_async16f(base + 2 * SCAN_TOK_TILE * DKP + qdst + i * DKP, gsrc);
+        cp_async16f(base + TILE * DKP + qdst + i * DKP, ksrc);
+        if (ROWS) cp_async16f(base + 2 * TILE * DKP + qdst + i * DKP, gsrc);
       }
       qsrc += TPI * qstep;
       ksrc += TPI * qstep;
       if (ROWS) gsrc += TPI * gstep;
     }
-    float* sv = base + NROW * SCAN_TOK_TILE * DKP;
+    float* sv = base + NROW * TILE * DKP;
 #pragma unroll
-    for (int i = 0; i < SCAN_TOK_TILE; i += VPI) {
+    for (int i = 0; i < TILE; i += VPI) {
       if (vt + i < nt) cp_async16f(base + vdst + i * SCAN_COLS, vsrc);
-      vsrc += (VPI < SCAN_TOK_TILE ? VPI : SCAN_TOK_TILE) * vstep;
+      vsrc += (VPI < TILE ? VPI : TILE) * vstep;
     }
     if (MODE == SCAN_DELTA && threadIdx.x < nt)
-      sv[SCAN_TOK_TILE * SCAN_COLS + threadIdx.x] = w.beta[(int64_t)(tb + threadIdx.x) * p.heads + h];
+      sv[TILE * SCAN_COLS + threadIdx.x] = w.beta[(int64_t)(tb + threadIdx.x) * p.heads + h];
     if (MODE == SCAN_GATED && threadIdx.x < nt)
-      cp_async16f(sv + SCAN_TOK_TILE * SCAN_COLS + threadIdx.x * 4,
+      cp_async16f(sv + TILE * SCAN_COLS + threadIdx.x * 4,
                   w.gw + ((int64_t)(tb + threadIdx.x) * p.heads + h) * 4);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -658,21 +690,21 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
   };
 
   load_tile(0, t0);
-  if (STAGES == 3) load_tile(1, t0 + SCAN_TOK_TILE);
+  if (STAGES == 3) load_tile(1, t0 + TILE);
   int stage = 0;
-  for (int tb = t0; tb < t1; tb += SCAN_TOK_TILE, stage = stage + 1 == STAGES ? 0 : stage + 1) {
-    const int nt = min(SCAN_TOK_TILE, t1 - tb);
+  for (int tb = t0; tb < t1; tb += TILE, stage = stage + 1 == STAGES ? 0 : stage + 1) {
+    const int nt = min(TILE, t1 - tb);
     // a tile past the portion's end is an empty group
-    if (STAGES == 2) load_tile(stage ^ 1, tb + SCAN_TOK_TILE);    // released by the barrier that ended the last pass
+    if (STAGES == 2) load_tile(stage ^ 1, tb + TILE);    // released by the barrier that ended the last pass
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
     // three stages: the tile before last was left by everyone who passed this barrier
-    if (STAGES == 3) load_tile(stage == 0 ? 2 : stage - 1, tb + 2 * SCAN_TOK_TILE);
+    if (STAGES == 3) load_tile(stage == 0 ? 2 : stage - 1, tb + 2 * TILE);
     const float* sq = scan_smem + stage * STAGE;
-    const float* sk = sq + SCAN_TOK_TILE * DKP;
-    const float* sg = sk + SCAN_TOK_TILE * DKP;
-    const float* sv = sq + NROW * SCAN_TOK_TILE * DKP;
-    const float* sbeta = sv + SCAN_TOK_TILE * SCAN_COLS;
+    const float* sk = sq + TILE * DKP;
+    const float* sg = sk + TILE * DKP;
+    const float* sv = sq + NROW * TILE * DKP;
+    const float* sbeta = sv + TILE * SCAN_COLS;
     // one token: the lane's part of S is advanced; returns column (part & 3) of the read-out joined over the lane's quad
     auto advance = [&](int tt) -> float {
       const float4 v4 = *reinterpret_cast<const float4*>(sv + tt * SCAN_COLS + c0);
@@ -688,17 +720,17 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
         for (int c = 0; c < SCAN_CPL; ++c) u[c] *= wr;
       }
       if (MODE == SCAN_DELTA) {
-        uint64_t a2[SCAN_CPL] = {0ull, 0ull, 0ull, 0ull};
+        P a2[SCAN_CPL] = {};
 #pragma unroll
         for (int i = 0; i < RP; i += 4) {
-          const ulonglong2 g4 = *reinterpret_cast<const ulonglong2*>(gq + i);
-          const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kq + i);
-          const uint64_t gr[2] = {g4.x, g4.y}, kr[2] = {k4.x, k4.y};
+          const Quad g4 = *reinterpret_cast<const Quad*>(gq + i);
+          const Quad k4 = *reinterpret_cast<const Quad*>(kq + i);
+          const P gr[2] = {g4.x, g4.y}, kr[2] = {k4.x, k4.y};
 #pragma unroll
           for (int e = 0; e < 2; ++e)
 #pragma unroll
             for (int c = 0; c < SCAN_CPL; ++c) {
-              uint64_t& x = S[i / 2 + e][c];
+              P& x = S[i / 2 + e][c];
               x = mul2(x, gr[e]);
               a2[c] = fma2(x, kr[e], a2[c]);
             }
@@ -713,29 +745,34 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
         const float xl = __shfl_xor_sync(ALL, lo, 2), xh = __shfl_xor_sync(ALL, hi, 2);
         u[0] = b1 ? xl : lo; u[1] = b1 ? xh : hi; u[2] = b1 ? lo : xl; u[3] = b1 ? hi : xh;
       }
-      uint64_t o2[SCAN_CPL] = {0ull, 0ull, 0ull, 0ull}, u2[SCAN_CPL];
+      P o2[SPLIT][SCAN_CPL] = {}, u2[SCAN_CPL];
 #pragma unroll
-      for (int c = 0; c < SCAN_CPL; ++c) u2[c] = pair_of(u[c], u[c]);
-      const uint64_t dec2 = pair_of(dec, dec);
+      for (int c = 0; c < SCAN_CPL; ++c) u2[c] = pair_of<P>(u[c], u[c]);
+      const P dec2 = pair_of<P>(dec, dec);
 #pragma unroll
       for (int i = 0; i < RP; i += 4) {
-        const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kq + i);
-        const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qq + i);
-        ulonglong2 g4 = make_ulonglong2(dec2, dec2);
-        if (MODE == SCAN_ROWS) g4 = *reinterpret_cast<const ulonglong2*>(gq + i);
-        const uint64_t gr[2] = {g4.x, g4.y}, kr[2] = {k4.x, k4.y}, qr[2] = {q4.x, q4.y};
+        const Quad k4 = *reinterpret_cast<const Quad*>(kq + i);
+        const Quad q4 = *reinterpret_cast<const Quad*>(qq + i);
+        Quad g4{dec2, dec2};
+        if (MODE == SCAN_ROWS) g4 = *reinterpret_cast<const Quad*>(gq + i);
+        const P gr[2] = {g4.x, g4.y}, kr[2] = {k4.x, k4.y}, qr[2] = {q4.x, q4.y};
 #pragma unroll
         for (int e = 0; e < 2; ++e)
 #pragma unroll
           for (int c = 0; c < SCAN_CPL; ++c) {
-            uint64_t& x = S[i / 2 + e][c];
+            P& x = S[i / 2 + e][c];
             x = MODE == SCAN_DELTA ? fma2(kr[e], u2[c], x) : fma2(gr[e], x, mul2(kr[e], u2[c]));
-            o2[c] = fma2(x, qr[e], o2[c]);
+            P& y = o2[i / (RP / SPLIT)][c];
+            y = fma2(x, qr[e], y);
           }
       }
       float o[SCAN_CPL];
 #pragma unroll
-      for (int c = 0; c < SCAN_CPL; ++c) { const float2 h = halves(o2[c]); o[c] = h.x + h.y; }
+      for (int c = 0; c < SCAN_CPL; ++c) {
+        const float2 h = halves(o2[0][c]);
+        o[c] = h.x + h.y;
+        if (SPLIT == 2) { const float2 g = halves(o2[SPLIT - 1][c]); o[c] += g.x + g.y; }
+      }
       return fold(o);
     };
     auto emit = [&](int tt, float o) {           // column (part & 3) of token tt's read-out
@@ -748,7 +785,7 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
     // not depend on how a portion falls into groups)
     int tt = 0;
 #pragma unroll 2
-    for (; tt + NTOK <= nt; tt += NTOK) {        // every lane takes part in the shuffles, also for a padded column
+    for (; !SHORT && tt + NTOK <= nt; tt += NTOK) {        // every lane takes part in the shuffles, also for a padded column
       float v[NTOK];
 #pragma unroll
       for (int n = 0; n < NTOK; ++n) v[n] = advance(tt + n);
@@ -760,6 +797,7 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
       }
       emit(tt + part / SCAN_CPL, v[0]);
     }
+#pragma unroll 1
     for (; tt < nt; ++tt) {
       const float o = join_quads(advance(tt));
       if (part < SCAN_CPL) emit(tt, o);
@@ -786,16 +824,17 @@ __global__ void __launch_bounds__(ScanTile<DK, MODE>::THREADS, ScanTile<DK, MODE
   }
 }
 
-template <int DK, int MODE> int launch_scan_dk(const ScanParams& p, const ScanWork& w, int nseq, cudaStream_t st) {
-  const size_t smem = (size_t)ScanTile<DK, MODE>::STAGES * SCAN_TOK_TILE * ScanTile<DK, MODE>::TOKEN * sizeof(float);
-  auto kern = state_scan_kernel<DK, MODE>;
+template <int DK, int MODE, bool SHORT> int launch_scan_dk(const ScanParams& p, const ScanWork& w, int nseq, cudaStream_t st) {
+  using Tile = ScanTile<DK, MODE, SHORT>;
+  const size_t smem = (size_t)Tile::STAGES * Tile::TILE * Tile::TOKEN * sizeof(float);
+  auto kern = state_scan_kernel<DK, MODE, SHORT>;
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     configured = true;
   }
-  kern<<<p.heads * (w.VP / SCAN_COLS) * nseq, ScanTile<DK, MODE>::THREADS, smem, st>>>(p, w, nseq, cb_num_sms());
+  kern<<<p.heads * (w.VP / SCAN_COLS) * nseq, Tile::THREADS, smem, st>>>(p, w, nseq, cb_num_sms());
   return CB_LAUNCH_CHECK();
 }
 
@@ -804,7 +843,7 @@ static inline int scan_dk(int dim) { return dim <= 16 ? 16 : dim <= 32 ? 32 : di
 static inline int scan_vp(int vdim) { return (vdim + SCAN_COLS - 1) / SCAN_COLS * SCAN_COLS; }
 
 template <int MODE, typename T>
-int launch_scan(const ScanParams& p, float* work, int64_t tokens, int nseq, cudaStream_t st) {
+int launch_scan(const ScanParams& p, float* work, int64_t tokens, int nseq, int max_q, cudaStream_t st) {
   if (p.dim > 256) return (int)cudaErrorInvalidValue;
   ScanWork w;
   w.DK = scan_dk(p.dim);
@@ -833,11 +872,13 @@ int launch_scan(const ScanParams& p, float* work, int64_t tokens, int nseq, cuda
     else if (w.DK == 128) exp_gate_kernel<128><<<blocks, 128, 0, st>>>(p, w, nseq);
     else exp_gate_kernel<256><<<blocks, 128, 0, st>>>(p, w, nseq);
   }
-  if (w.DK == 16) return launch_scan_dk<16, MODE>(p, w, nseq, st);
-  if (w.DK == 32) return launch_scan_dk<32, MODE>(p, w, nseq, st);
-  if (w.DK == 64) return launch_scan_dk<64, MODE>(p, w, nseq, st);
-  if (w.DK == 128) return launch_scan_dk<128, MODE>(p, w, nseq, st);
-  return launch_scan_dk<256, MODE>(p, w, nseq, st);
+#define SCAN_DK(D) (max_q <= SCAN_SHORT ? launch_scan_dk<D, MODE, true>(p, w, nseq, st) : launch_scan_dk<D, MODE, false>(p, w, nseq, st))
+  if (w.DK == 16) return SCAN_DK(16);
+  if (w.DK == 32) return SCAN_DK(32);
+  if (w.DK == 64) return SCAN_DK(64);
+  if (w.DK == 128) return SCAN_DK(128);
+  return SCAN_DK(256);
+#undef SCAN_DK
 }
 
 // ------------------------------------------------------------------------------------------------ norms
@@ -2835,7 +2876,7 @@ int64_t cb_state_scan_workspace(int mode, int64_t tokens, int heads, int qk_head
 int cb_state_scan(int mode, const void* q, int64_t ldq, const void* k, int64_t ldk, const void* v, int64_t ldv,
                   const void* araw, int64_t lda, const void* braw, int64_t ldb, const float* head_decay,
                   const float* a_log, const float* dt_bias, float* state, float* out, float* work, int64_t tokens,
-                  const int* cu_q, const int* ctx_len, const int* slots, int nseq, int heads, int qk_heads, int dim,
+                  const int* cu_q, const int* ctx_len, const int* slots, int nseq, int max_q, int heads, int qk_heads, int dim,
                   int vdim, int act_silu, int unit_qk, float unit_eps, float q_scale, float k_scale,
                   const float* rot_table, int rot_dims, const int* token_pos, int gate_kind, float gate_cap,
                   float* state_n, float* state_m, float tau, int dtype, cudaStream_t st) {
@@ -2850,10 +2891,10 @@ int cb_state_scan(int mode, const void* q, int64_t ldq, const void* k, int64_t l
                heads, qk_heads, dim, vdim, act_silu, unit_qk, unit_eps, q_scale, k_scale, rot_table, rot_dims, token_pos,
                gate_kind, gate_cap, state_n, state_m, 1.f / tau};
   CB_DISPATCH_FLOAT(dtype, T, {
-    if (mode == SCAN_GATED) return launch_scan<SCAN_GATED, T>(p, work, tokens, nseq, st);
-    if (mode == SCAN_DELTA) return launch_scan<SCAN_DELTA, T>(p, work, tokens, nseq, st);
-    if (mode == SCAN_ROWS) return launch_scan<SCAN_ROWS, T>(p, work, tokens, nseq, st);
-    return launch_scan<SCAN_DECAY, T>(p, work, tokens, nseq, st);
+    if (mode == SCAN_GATED) return launch_scan<SCAN_GATED, T>(p, work, tokens, nseq, max_q, st);
+    if (mode == SCAN_DELTA) return launch_scan<SCAN_DELTA, T>(p, work, tokens, nseq, max_q, st);
+    if (mode == SCAN_ROWS) return launch_scan<SCAN_ROWS, T>(p, work, tokens, nseq, max_q, st);
+    return launch_scan<SCAN_DECAY, T>(p, work, tokens, nseq, max_q, st);
   });
   return CB_LAUNCH_CHECK();
 }

@@ -147,6 +147,37 @@ def test_decay_scan_does_not_depend_on_portions(d, dv, cuts):
     assert torch.equal(ran[0][0], ran[1][0]) and torch.equal(ran[0][1], ran[1][1])
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["decay", "rows", "delta", "steps"])
+@pytest.mark.parametrize("d,dv", [(16, 64), (30, 36), (64, 40), (128, 32), (200, 36)])
+@pytest.mark.parametrize("cuts", [[32, 38], [33, 37], [1] * 20 + [50], [4, 5, 31, 30]])
+def test_scans_of_short_and_long_portions_agree(mode, d, dv, cuts):
+    """Portions on both sides of the length from which the long form is taken: the same bits, in every mode."""
+    dev, H, L = _dev("cuda"), 3, 70
+    g = torch.Generator().manual_seed(d)
+    q, k, v = (torch.randn(L, H * w, generator=g).to(dev) for w in (d, d, dv))
+    pre, beta = torch.randn(L, H * d, generator=g).to(dev), torch.randn(L, H, generator=g).to(dev)
+    head, chan = torch.rand(H, generator=g).to(dev), torch.randn(H * d, generator=g).to(dev)
+    ran = []
+    for parts in ([L], cuts):
+        assert sum(parts) == L
+        state, outs, at = torch.zeros(1, H, d, dv, device=dev), [], 0
+        for n in parts:
+            meta, r = M.RaggedMeta.build([n], [at], [0], dev), slice(at, at + n)
+            if mode == "decay":
+                o = M.state_scan_decay(q[r], k[r], v[r], head, state, meta, H, d, dv)
+            elif mode == "rows":
+                o = M.state_scan_gla(q[r], k[r], v[r], pre[r], chan, 16.0, state, meta, H, d, dv)
+            elif mode == "delta":
+                o = M.state_scan_delta(q[r], k[r], v[r], pre[r], beta[r], head, chan, state, meta, H, H, d, dv)
+            else:
+                o = M.state_scan_ssd(q[r], k[r], v[r], beta[r], head, head, head, state, meta, H, H, d, dv)
+            outs.append(o.clone())
+            at += n
+        ran.append((torch.cat(outs), state))
+    assert torch.isfinite(ran[0][0]).all() and torch.equal(ran[0][0], ran[1][0]) and torch.equal(ran[0][1], ran[1][1])
+
+
 @pytest.mark.parametrize("device", DEVICES)
 @pytest.mark.parametrize("L", [8, 13, 16])
 def test_decay_scan_of_infinite_and_very_large_values(device, L):
