@@ -58,11 +58,15 @@ SM100_DEVICE bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* ab
   *abort_flag = 1;
   return false;
 }
-// one thread: the rows of a CTA that gave up are not valid
-SM100_DEVICE void report_abort(int* status) {
-  *reinterpret_cast<volatile int*>(status) = 1;
-  __threadfence_system();
-}
+// one thread: the rows of a CTA that gave up are not valid.  (Without a fence: the host looks after the kernel has ended, and a
+// system-wide fence anywhere in the backward kernel made all of its reductions slower, 467 -> 525 us.)
+SM100_DEVICE void report_abort(int* status) { *reinterpret_cast<volatile int*>(status) = 1; }
+
+// Every role of the backward is done: the producer and the issuer wait for the others, which only say so, and see whether one gave
+// up.  Inside the roles, because code behind their last common barrier cost the kernel 2 % (461 and 473 us; the forward
+// kernels lose by the second barrier instead, 169 and 175 us, and have it behind).
+template <int THREADS> SM100_DEVICE void roles_done_wait() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
+template <int THREADS> SM100_DEVICE void roles_done() { asm volatile("bar.arrive 1, %0;" ::"n"(THREADS) : "memory"); }
 
 // The status word: pinned host memory, so that the host reads it without a call (null: there is none to be had).  One per
 // process, whatever the device.
@@ -1232,8 +1236,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint64_t* drained = acc_full + 1;        // [1]  a CTA that gives up: its products have retired
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(drained + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
-  volatile int* copies = abort_flag + 1;   // [1]  query tiles that the producer asked for
-  int* work = reinterpret_cast<int*>(tmem_ptr_smem + 3);
+  int* work = reinterpret_cast<int*>(tmem_ptr_smem + 2);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -1301,6 +1304,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
   if (warp == 0) {
     // ================================================================ TMA producer
+    int it = 0;
     if (lane == 0) {
       mbar_arrive_expect_tx(kv_full, C::K_BYTES + C::V_BYTES);
 #pragma unroll
@@ -1308,7 +1312,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         tma_load_2d(&tmap_k, kv_full, smem_k + h * (BWD_BLOCK_KV * 128), kv_head * D + h * 64, kv_row0);
         tma_load_2d(&tmap_v, kv_full, smem_v + h * (BWD_BLOCK_KV * 128), kv_head * D + h * 64, kv_row0);
       }
-      int it = 0;
       for (; it < n_iter; ++it) {
         const int stage = it % ST;
         const int hq = kv_head * group + it / n_i;
@@ -1323,8 +1326,17 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           tma_load_2d(&tmap_do, &qdo_full[stage], sdo + h * (BWD_BLOCK_Q * 128), hq * D + h * 64, q_row0);
         }
       }
-      *copies = it;
-      if (n_iter == 0) wait_or_abort(kv_full, 0, abort_flag);   // nothing waits for K and V: leave no copy in flight behind
+    }
+    __syncwarp();
+    roles_done_wait<BWD_THREADS>();
+    if (lane == 0 && (*abort_flag || n_iter == 0)) {     // leave no copy in flight behind (without queries nothing waits for K, V)
+      int none = 0;
+      wait_or_abort(kv_full, 0, &none);
+      for (int i = max(0, it - ST); i < it; ++i) {
+        none = 0;
+        wait_or_abort(&qdo_full[i % ST], ring_parity(i), &none);
+      }
+      if (*abort_flag) report_abort(p.status);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -1398,6 +1410,13 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       }
     }
     __syncwarp();
+    roles_done_wait<BWD_THREADS>();
+    if (lane == 0 && *abort_flag) {                          // nor a product
+      int none = 0;
+      umma_commit(drained);
+      wait_or_abort(drained, 0, &none);
+    }
+    __syncwarp();
   } else if (warp < BWD_SOFTMAX_WARP0) {
     // ================================================================ statistics of the query rows (one row per thread)
     const int qr = (warp - BWD_STAT_WARP0) * 32 + lane;
@@ -1414,6 +1433,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(&stat_full[stage]);
     }
+    roles_done<BWD_THREADS>();
   } else if (warp < BWD_DRAIN_WARP0) {
     // ================================================================ softmax warps: two threads per key row
     constexpr int COLS = BWD_BLOCK_Q / 2;
@@ -1529,6 +1549,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           *reinterpret_cast<uint4*>(base + (c + i * 8) * 2) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
       }
     }
+    __syncwarp();
+    roles_done<BWD_THREADS>();
   } else {
     // ================================================================ dQ drain warps: thread = head-dim lane
     const int quarter = warp & 3;
@@ -1560,25 +1582,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           if (i < q_live) atomicAdd(dst + (size_t)i * row_stride, __uint_as_float(v[i]) * p.scale);
       }
     }
+    __syncwarp();
+    roles_done<BWD_THREADS>();
   }
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag) {                         // (nothing writes it any more: uniform) leave nothing in flight behind
-    int none = 0;
-    if (warp == 0 && lane == 0) {
-      wait_or_abort(kv_full, 0, &none);
-      for (int i = max(0, *copies - ST); i < *copies; ++i) {
-        none = 0;
-        wait_or_abort(&qdo_full[i % ST], ring_parity(i), &none);
-      }
-    }
-    if (warp == 1 && lane == 0) {            // the thread that issued the products
-      umma_commit(drained);
-      wait_or_abort(drained, 0, &none);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) report_abort(p.status);
-  }
   if (warp == 2) tmem_dealloc<C::TMEM_COLS>(tmem_base);
 }
 

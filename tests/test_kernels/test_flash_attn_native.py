@@ -319,3 +319,40 @@ def test_packed_backward_of_very_many_sequences():
     ref = torch.einsum("hqk,khd->qhd", s.softmax(-1), r[2])
     for a, b in zip((o, dq, dk, dv), (ref,) + torch.autograd.grad(ref, r, do[n:].double())):
         assert (a[n:].double() - b).norm() <= 1e-2 * b.norm()                  # weights and results rounded to bf16
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Hq,Hkv", [(4, 2), (3, 1), (148, 74), (222, 74), (224, 56)])
+@pytest.mark.parametrize("lens", [[1], [128], [129, 0, 127], [300, 1, 129, 257, 0, 128]])
+@pytest.mark.parametrize("mask", ["causal", "full", "window"])
+def test_packed_forward_by_number_of_tiles(D, Hq, Hkv, lens, mask):
+    """One tile per CTA and two (of a group's two heads, of one head), on both sides of the lines between them, at partial and empty
+    sequences; with a window in the variant for serving."""
+    from colossalai_b200.ops import flash_attn_native as fa
+
+    T = sum(lens)
+    g = torch.Generator(device="cuda").manual_seed(Hq + T)
+    q = torch.randn(T, Hq, D, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(T, Hkv, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    cu = torch.tensor([0] + lens, device="cuda").cumsum(0).int()
+    if mask == "window":
+        out = fa.flash_prefill(q, k, v, cu, None, window=70)
+    else:
+        out, lse = fa.flash_fwd(q, k, v, 1, mask == "causal", None, cu)
+    at = 0
+    for n in lens:
+        r = slice(at, at + n)
+        at += n
+        if n == 0:
+            continue
+        i = torch.arange(n, device="cuda")
+        seen = torch.ones(n, n, dtype=torch.bool, device="cuda") if mask == "full" else i[:, None] >= i
+        if mask == "window":
+            seen &= i[:, None] - i < 70
+        kk, vv = (t[r].float().repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+        s = (torch.einsum("qhd,khd->hqk", q[r].float(), kk) / D ** 0.5).masked_fill(~seen, float("-inf"))
+        ref = torch.einsum("hqk,khd->qhd", s.softmax(-1), vv)
+        # weights and results rounded to bf16, as in the other forward tests
+        torch.testing.assert_close(out[r].float(), ref, atol=2e-2, rtol=2e-2)
+        if mask != "window":
+            torch.testing.assert_close(lse[r], s.logsumexp(-1).T, atol=1e-3, rtol=1e-3)
