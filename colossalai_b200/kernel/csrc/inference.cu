@@ -453,6 +453,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.y * (blockDim.x >> 5) + warp;
   if (kvh >= Hkv) return;                       // (no block-wide barrier in this kernel)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int len = seq_lens[seq];
   const int window_start = window > 0 ? max(0, len - window) : 0;
   const int t0 = max(split * part_len, window_start);
@@ -625,6 +626,93 @@ __global__ void __launch_bounds__(128) decode_reduce_kernel(const float* __restr
   }
 }
 
+// The same for DEC_WIDE partitions and more, which means few long sequences: the weights are worked out side by side and DEC_AHEAD
+// partial results are on their way to a thread at a time, where the kernel above waits for each in turn (65 partitions of one
+// sequence of 4097 tokens: the call on the device 16.2 us, 13.9 so).  With fewer of them it is no faster (16 x 2048 tokens, 64 / 8 heads, 19
+// partitions 30 us, 33 so) and with many sequences slower (1024 of 64 tokens 78 us, 89 so).
+// Sums in the same order with the same roundings.  Launched while the kernel before it runs,
+// it takes its place on the SMs and waits there.
+constexpr int DEC_WIDE = 48, DEC_AHEAD = 16, DEC_WIDE_THREADS = 128;
+template <typename T, int D>
+__global__ void __launch_bounds__(DEC_WIDE_THREADS) decode_reduce_wide_kernel(const float* __restrict__ o_part,
+                                                                              const float* __restrict__ ml_part,
+                                                                              T* __restrict__ out, int Hq, int splits,
+                                                                              int64_t out_stride) {
+  constexpr int COLS = (D + DEC_WIDE_THREADS - 1) / DEC_WIDE_THREADS;
+  __shared__ float max_s[DEC_WIDE_THREADS / 32];
+  __shared__ float w_s[DEC_WIDE_THREADS], l_s[DEC_WIDE_THREADS];      // weight (-1: a partition without tokens), sum
+  const int seq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+  const int64_t base = ((int64_t)seq * Hq + h) * splits;
+  const float2* ml = reinterpret_cast<const float2*>(ml_part) + base;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  float gm = -INFINITY;
+  for (int s = tid; s < splits; s += DEC_WIDE_THREADS) gm = fmaxf(gm, ml[s].x);
+  gm = warp_max(gm);
+  if ((tid & 31) == 0) max_s[tid >> 5] = gm;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < DEC_WIDE_THREADS / 32; ++w) gm = fmaxf(gm, max_s[w]);
+  float ls = 0.f, acc[COLS];
+  bool nan = false;                             // as above
+#pragma unroll
+  for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
+  for (int s0 = 0; s0 < splits; s0 += DEC_WIDE_THREADS) {
+    const int n = min(DEC_WIDE_THREADS, splits - s0);
+    if (s0 > 0) __syncthreads();
+    if (tid < n) {
+      const float2 x = ml[s0 + tid];
+      w_s[tid] = x.x == -INFINITY ? -1.f : __expf(x.x - gm);
+      l_s[tid] = x.y;
+    }
+    __syncthreads();
+    for (int s = 0; s < n; ++s) {
+      if (w_s[s] >= 0.f) ls = __fadd_rn(ls, __fmul_rn(l_s[s], w_s[s]));
+      nan |= isnan(l_s[s]);
+    }
+    for (int s = 0; s < n; s += DEC_AHEAD) {
+      float o[DEC_AHEAD][COLS];
+#pragma unroll
+      for (int u = 0; u < DEC_AHEAD; ++u)
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+          const int d = tid + c * DEC_WIDE_THREADS;
+          if (s + u < n && d < D) o[u][c] = o_part[(base + s0 + s + u) * D + d];
+        }
+#pragma unroll
+      for (int u = 0; u < DEC_AHEAD; ++u)
+        if (s + u < n && w_s[s + u] >= 0.f) {
+#pragma unroll
+          for (int c = 0; c < COLS; ++c) acc[c] = fmaf(o[u][c], w_s[s + u], acc[c]);
+        }
+    }
+  }
+  const float inv = nan ? NAN : ls > 0.f ? 1.f / ls : 0.f;
+#pragma unroll
+  for (int c = 0; c < COLS; ++c) {
+    const int d = tid + c * DEC_WIDE_THREADS;
+    if (d < D) out[(int64_t)seq * out_stride + (int64_t)h * D + d] = from_f32<T>(acc[c] * inv);
+  }
+}
+
+template <typename T, int D>
+int launch_decode_reduce(const float* o_part, const float* ml_part, T* out, int num_seqs, int Hq, int splits, int64_t out_stride,
+                         cudaStream_t s) {
+  if (splits < DEC_WIDE) {
+    decode_reduce_kernel<T, D><<<dim3(num_seqs, Hq), 128, 0, s>>>(o_part, ml_part, out, Hq, splits, out_stride);
+    return CB_LAUNCH_CHECK();
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(num_seqs, Hq);
+  cfg.blockDim = dim3(DEC_WIDE_THREADS);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, decode_reduce_wide_kernel<T, D>, o_part, ml_part, out, Hq, splits, out_stride);
+}
+
 __global__ void gather_cos_sin_kernel(const float* __restrict__ cos_c, const float* __restrict__ sin_c,
                                       const int* __restrict__ pos, float* __restrict__ cos_o,
                                       float* __restrict__ sin_o, int tokens, int half) {
@@ -745,7 +833,7 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
     paged_decode_mma_kernel<T, DD><<<mma_grid, mma_warps * 32, mma_warps * per_warp, s>>>(                           \
         (const T*)q, (const T*)k_cache, (const T*)v_cache, block_tables, seq_lens, o_part, ml_part, Hq, Hkv,        \
         block_size, max_blocks_per_seq, splits, part_len, scale, alibi_slopes, q_stride, window);                   \
-    decode_reduce_kernel<T, DD><<<dim3(num_seqs, Hq), 128, 0, s>>>(o_part, ml_part, (T*)out, Hq, splits, out_stride); \
+    if (const int e = launch_decode_reduce<T, DD>(o_part, ml_part, (T*)out, num_seqs, Hq, splits, out_stride, s)) return e; \
   }
 #define LAUNCH_DEC(T, DD)                                                                                           \
   {                                                                                                                  \
@@ -758,7 +846,7 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
   paged_decode_kernel<T, T, DD><<<grid, warps * 32, dec_smem, s>>>((const T*)q, (const T*)k_cache, (const T*)v_cache, \
       block_tables, seq_lens, o_part, ml_part, Hq, Hkv, block_size, max_blocks_per_seq, splits, part_len, scale,     \
       alibi_slopes, q_stride, window);                                                                               \
-  decode_reduce_kernel<T, DD><<<dim3(num_seqs, Hq), 128, 0, s>>>(o_part, ml_part, (T*)out, Hq, splits, out_stride)
+  if (const int e = launch_decode_reduce<T, DD>(o_part, ml_part, (T*)out, num_seqs, Hq, splits, out_stride, s)) return e
   CB_DISPATCH_HALF(dtype, T, {
     if (use_mma && D == 128) { LAUNCH_DEC_MMA(T, 128); }
     else if (use_mma && D == 64) { LAUNCH_DEC_MMA(T, 64); }

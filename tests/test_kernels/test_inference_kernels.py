@@ -228,3 +228,20 @@ def test_paged_decode_shows_nan(length, keys):
         kc[p, 3 if keys == "one" else slice(None)] = float("nan")
     out = iops.paged_decode_attention(q, kc, vc, tables, lens)
     assert out[1].isnan().all() and torch.equal(out[0], good[0])
+
+
+@pytest.mark.parametrize("n,longest", [(1, 47 * 64), (1, 48 * 64), (1, 129 * 64), (3, 47 * 64 + 1), (6, 5000), (7, 5000)])
+@pytest.mark.parametrize("D", [64, 128, 256])
+def test_paged_decode_by_number_of_partitions(n, longest, D):
+    """Both ways of summing the partitions, on both sides of the line and past one round of the wide one; a sequence that leaves
+    most of its partitions empty."""
+    dev = torch.device("cuda")
+    torch.manual_seed(longest)
+    kc, vc, tables = _mk_cache(n, longest, 16, 2, D, torch.bfloat16, dev)
+    q = torch.randn(n, 6, D, device=dev, dtype=torch.bfloat16)
+    lens = torch.tensor([longest, 70, 0, 1, 999, longest - 1, 64][:n], device=dev, dtype=torch.int32)
+    out = iops.paged_decode_attention(q, kc, vc, tables, lens)
+    live = [i for i, m in enumerate(lens.tolist()) if m]
+    ref = iops.paged_decode_attention_ref(q.float()[live], kc.float(), vc.float(), tables[live], lens[live])
+    torch.testing.assert_close(out[live].float(), ref, atol=2e-2, rtol=2e-2)      # weights rounded to bf16
+    assert not out[[i for i in range(n) if i not in live]].any()
