@@ -53,9 +53,9 @@ struct GluPart {                      // what a thread works on: its row, first 
   int64_t row;
   int c0, lanes;
 };
-template <int VEC> CB_DEVICE bool glu_part(GluPart& p, int64_t rows, int blocks_per_row, int rows_per_block, int I,
-                                           const int64_t* row_limit) {
-  if (rows_per_block > 1) {
+template <int VEC, bool NARROW> CB_DEVICE bool glu_part(GluPart& p, int64_t rows, int blocks_per_row, int rows_per_block, int I,
+                                                        const int64_t* row_limit) {
+  if (NARROW) {
     p.lanes = (I / VEC + GLU_ITEMS - 1) / GLU_ITEMS;
     const int r = threadIdx.x / p.lanes;
     p.row = (int64_t)blockIdx.x * rows_per_block + r;
@@ -70,13 +70,13 @@ template <int VEC> CB_DEVICE bool glu_part(GluPart& p, int64_t rows, int blocks_
   return row_limit == nullptr || p.row < *row_limit;
 }
 
-template <typename T, int ACT>
+template <typename T, int ACT, bool NARROW>
 __global__ void __launch_bounds__(GLU_THREADS) glu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out, int64_t rows,
                                                               int blocks_per_row, int rows_per_block, int I,
                                                               const int64_t* __restrict__ row_limit) {
   constexpr int VEC = Vec16<T>::N;
   GluPart p;
-  if (!glu_part<VEC>(p, rows, blocks_per_row, rows_per_block, I, row_limit)) return;
+  if (!glu_part<VEC, NARROW>(p, rows, blocks_per_row, rows_per_block, I, row_limit)) return;
   const T* gr = gu + p.row * 2 * I;
   T* o_r = out + p.row * I;
   Vec16<T> g[GLU_ITEMS], u[GLU_ITEMS], o;
@@ -96,13 +96,13 @@ __global__ void __launch_bounds__(GLU_THREADS) glu_fwd_kernel(const T* __restric
   }
 }
 
-template <typename T, int ACT>
+template <typename T, int ACT, bool NARROW>
 __global__ void __launch_bounds__(GLU_THREADS) glu_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ gu,
                                                               T* __restrict__ dgu, int64_t rows, int blocks_per_row,
                                                               int rows_per_block, int I, const int64_t* __restrict__ row_limit) {
   constexpr int VEC = Vec16<T>::N;
   GluPart p;
-  if (!glu_part<VEC>(p, rows, blocks_per_row, rows_per_block, I, row_limit)) return;
+  if (!glu_part<VEC, NARROW>(p, rows, blocks_per_row, rows_per_block, I, row_limit)) return;
   const T* gr = gu + p.row * 2 * I;
   const T* dr = dout + p.row * I;
   T* or_ = dgu + p.row * 2 * I;
@@ -287,9 +287,9 @@ extern "C" {
     if (blocks > 0x7fffffffll) return (int)cudaErrorInvalidValue;                                                       \
     const int part = (vecs + bpr - 1) / bpr;                                                                            \
     const int block = rpb > 1 ? GLU_THREADS : ((part + GLU_ITEMS - 1) / GLU_ITEMS + 31) / 32 * 32;                      \
-    if (act == 0) KERNEL<T, 0><<<(unsigned)blocks, block, 0, s>>>(__VA_ARGS__, rows, bpr, rpb, I, row_limit);           \
-    else if (act == 1) KERNEL<T, 1><<<(unsigned)blocks, block, 0, s>>>(__VA_ARGS__, rows, bpr, rpb, I, row_limit);      \
-    else KERNEL<T, 2><<<(unsigned)blocks, block, 0, s>>>(__VA_ARGS__, rows, bpr, rpb, I, row_limit);                    \
+    auto kern = rpb > 1 ? (act == 0 ? KERNEL<T, 0, true> : act == 1 ? KERNEL<T, 1, true> : KERNEL<T, 2, true>)            \
+                        : (act == 0 ? KERNEL<T, 0, false> : act == 1 ? KERNEL<T, 1, false> : KERNEL<T, 2, false>);        \
+    kern<<<(unsigned)blocks, block, 0, s>>>(__VA_ARGS__, rows, bpr, rpb, I, row_limit);                                  \
   })
 
 int cb_glu_fwd_bounded(const void* gu, void* out, int64_t rows, int I, int act, int dtype, const int64_t* row_limit, cudaStream_t s) {
