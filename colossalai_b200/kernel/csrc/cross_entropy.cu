@@ -73,11 +73,26 @@ __global__ void __launch_bounds__(THREADS) ce_row_stats_kernel(const T* __restri
 // One block up to CE_LOSS_ROWS rows; more rows are dealt out to up to CE_LOSS_BLOCKS blocks, whose sums a second launch adds up in
 // their order (131072 rows: one block
 // 130 us, now 3.6 and 2.4 to add them up; 16384 rows 17 us, 3.4 and 1.8).
-constexpr int CE_LOSS_ROWS = 2048, CE_LOSS_BLOCKS = 128;
+constexpr int CE_LOSS_ROWS = 4096, CE_LOSS_BLOCKS = 128;
 struct CePart {
   double sum;
   unsigned count;
 };
+// sums over the block, always in the same order; in thread 0
+CB_DEVICE void ce_block_sum(double& sum, unsigned& count, double* sums, unsigned* counts) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  count = __reduce_add_sync(0xffffffffu, count);
+  if (lane == 0) { sums[warp] = sum; counts[warp] = count; }
+  __syncthreads();
+  if (warp != 0) return;
+  const bool live = lane < (int)blockDim.x / 32;
+  sum = live ? sums[lane] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  count = __reduce_add_sync(0xffffffffu, live ? counts[lane] : 0u);
+}
 CB_DEVICE void ce_loss_finish(double sum, unsigned count, int mean, float* loss, int64_t* n_valid) {
   *n_valid = count;
   *loss = (float)(mean ? sum / max(count, 1u) : sum);
@@ -95,13 +110,8 @@ __global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__
       acc += log((double)stats[rows + r]) + stats[r] - stats[2 * (int64_t)rows + r];               // (logf is approximate here)
       ++count;
     }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  count = __reduce_add_sync(0xffffffffu, count);
-  if ((threadIdx.x & 31) == 0) { sums[threadIdx.x >> 5] = acc; counts[threadIdx.x >> 5] = count; }
-  __syncthreads();
+  ce_block_sum(acc, count, sums, counts);
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)blockDim.x / 32; ++w) { acc += sums[w]; count += counts[w]; }
     if (gridDim.x > 1) parts[blockIdx.x] = CePart{acc, count};
     else ce_loss_finish(acc, count, mean, loss, n_valid);
   }
@@ -109,13 +119,12 @@ __global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__
 
 __global__ void __launch_bounds__(CE_LOSS_BLOCKS) ce_loss_join_kernel(const CePart* __restrict__ parts, int n, float* __restrict__ loss,
                                                                       int64_t* __restrict__ n_valid, int mean) {
-  __shared__ CePart s[CE_LOSS_BLOCKS];
-  if ((int)threadIdx.x < n) s[threadIdx.x] = parts[threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  CePart a = s[0];
-  for (int i = 1; i < n; ++i) { a.sum += s[i].sum; a.count += s[i].count; }
-  ce_loss_finish(a.sum, a.count, mean, loss, n_valid);
+  __shared__ double sums[32];
+  __shared__ unsigned counts[32];
+  CePart a = {0.0, 0u};
+  if ((int)threadIdx.x < n) a = parts[threadIdx.x];
+  ce_block_sum(a.sum, a.count, sums, counts);
+  if (threadIdx.x == 0) ce_loss_finish(a.sum, a.count, mean, loss, n_valid);
 }
 
 template <typename T>

@@ -242,7 +242,7 @@ def test_cross_entropy_counts_labels(rows, mean):
 
 
 @pytest.mark.parametrize("mean", [True, False])
-@pytest.mark.parametrize("rows", [2047, 2048, 2049, 5000, 8 * 1024, 128 * 1024 + 1, 300000])
+@pytest.mark.parametrize("rows", [2049, 4096, 4097, 5000, 8 * 1024, 128 * 1024 + 1, 300000])
 def test_cross_entropy_loss_of_many_rows(rows, mean):
     """One block and several: the sum over the rows in 64 bits, rounded once, the same whenever it is taken."""
     g = torch.Generator(device="cuda").manual_seed(rows)
