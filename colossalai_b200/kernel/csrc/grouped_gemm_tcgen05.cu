@@ -15,8 +15,8 @@
 //     row range of a group must start and end on a multiple of 128 (one k-block) - the dispatch lays groups out that way
 //     (`moe/grouped_gemm.py` pads with zero rows otherwise) - so a k-block never mixes two experts.
 //
-// Replaces the reference's python loop over local experts (`shardformer/modeling/mixtral.py:177-191`) and round 1's
-// library `torch._grouped_mm`.
+// Replaces the reference's python loop over local experts (`shardformer/modeling/mixtral.py:177-191`) and the
+// library's `torch._grouped_mm`.
 #include <stdlib.h>
 
 #include "common.cuh"

@@ -57,9 +57,8 @@ def _use_fused(x: torch.Tensor, group) -> bool:
 
 def _fused_rs_variant(a: torch.Tensor, weight: torch.Tensor, group, transpose_b: bool) -> str:
     """Implementation of GEMM->reduce-scatter for this shape: 'stream' / 'stagger' (one fused sm_100a kernel) or 'lib'
-    (GEMM + NCCL reduce-scatter).  Measured once per shape on the live tensors by `parallel.fused.rs_variant` - round 1
-    used a fixed reduction-depth threshold (K >= 2048) taken from the TP=8 timings, which was wrong at other TP
-    degrees and froze the library fallback in place."""
+    (GEMM + NCCL reduce-scatter).  Measured once per shape on the live tensors by `parallel.fused.rs_variant`: a
+    threshold on the reduction depth (K >= 2048) that fitted TP = 8 was wrong at other degrees."""
     from ...parallel import fused
 
     return fused.rs_variant(a, weight, group, transpose_b)

@@ -1,5 +1,5 @@
 """Device-timed GEMM microbenchmark: our tcgen05 kernel vs cuBLAS (torch.matmul) on Llama-3 shapes.
-Usage (on the GPU box): python tests/bench_gemm.py > gpurun_out/gemm_bench.json"""
+Usage (on the GPU box): python tests/bench_gemm.py > gemm_bench.json"""
 import json
 import os
 import sys

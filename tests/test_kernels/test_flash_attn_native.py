@@ -1,5 +1,4 @@
-"""tcgen05 flash-attention forward against an fp32 PyTorch reference (out and log-sum-exp), plus gradients.
-First hardware run (round 2): 17/17 pass on a B200 (gpurun_out/c1_flash_test.log)."""
+"""tcgen05 flash-attention forward against an fp32 PyTorch reference (out and log-sum-exp), plus gradients."""
 import os
 
 import pytest
