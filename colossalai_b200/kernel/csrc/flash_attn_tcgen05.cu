@@ -4,23 +4,29 @@
 //
 // Persistent CTAs, one per SM, walk a list of work units, the longest first.  A unit = TWO 128-row query tiles over the same
 // key tiles: two query heads of one kv head where the group is even (the same keys are visible to both), else two
-// neighbouring query tiles of one head.  Twelve warps:
+// neighbouring query tiles of one head.  A step is 64 keys: half of a key tile, for each of the two query tiles.  Sixteen warps:
 //   warp 0       TMA producer: both Q tiles of a unit, then K_0, V_0, K_1, V_1, ... (128 keys each) through one ring
-//   warp 1       MMA issuer (one elected thread): S_t = Q_t K_j^T and O_t += P_t V_j with tcgen05.mma, accumulators in TMEM
+//   warp 1       MMA issuer: S_t = Q_t K_j^T and O_t += P_t V_j with tcgen05.mma, accumulators in TMEM
 //   warp 3       finds the units of a packed batch from its device-resident boundaries, two units ahead
 //   warps 4..7   softmax of tile 0, warps 8..11 of tile 1: thread r owns query row r - tcgen05.ld of its S row, running max /
 //                sum in the exp2 domain, P_t written back to TMEM as the 16-bit A operand of the second product
+//   warps 12..15 output: the rows of a finished unit, divided by their sums
 // Bound: the softmax - 128 exponentials per row and key tile at 16 a clock and SM take as long as the products of D = 128.
 // Two tiles, so that one tile's softmax runs under the other's products (one tile per CTA and the mask as predicated code:
-// 4096 tokens, 32 / 8 heads of 128, causal 239 us = 575 TFLOP/s; now 160 us = 859).  P through TMEM, because a product with
-// both operands in shared memory reads 8 KB per 64-clock MMA, all that shared memory delivers.  Persistent, because a unit
-// of a short sequence walks a handful of key tiles and a CTA of its own spent a third of its life on launch, allocation and
-// its first loads (16 x 1024 tokens, heads of 64: one tile per CTA 290 us, two 198 us, persistent 178 us; packed uneven
-// prompts of that size 360 -> 216 us).  Two threads per row (16 softmax warps) were 5 - 10 % slower than one.
-// TMEM map (512 columns), D = 128: [0,128) S_0, [128,256) S_1, then O_0, O_1; P_t overwrites the first half of S_t once its
-// rows are in registers, so S_t of the next key tile is issued behind the P V that reads P_t.  D = 64: O_t are 64 wide
-// and P_t have columns of their own, [384,448) and [448,512): the next S_t is issued as soon as this one has been read.
-// Shared memory at D = 128: 2 x Q 32 KB + 5 ring slots of 32 KB (at D = 64 2 x 16 KB + 8 x 16 KB) + mbarriers.
+// 4096 tokens, 32 / 8 heads of 128, causal 239 us = 575 TFLOP/s).  P through TMEM, because a product with both operands in
+// shared memory reads 8 KB per 64-clock MMA, all that shared memory delivers.  Persistent, because a unit of a short sequence
+// walks a handful of key tiles and a CTA of its own spent a third of its life on launch, allocation and its first loads.
+// Half steps, because S_t, P_t and O_t of D = 128 fill the tensor memory: with one S_t per tile the next Q K^T waited for the
+// softmax and P V of this one, and the softmax for it; with two halves one is multiplied while the other is exponentiated (and
+// 64 scores of a row in registers instead of 128 leave room for the output warps).  The issuing warp converged and its
+// descriptors in uniform registers: one thread in a branch took 80 clocks a product, which was the bound of this kernel once the
+// steps were halved.  2 x 4096 tokens, 32 / 8 heads of 128, causal: whole steps 309 us, half steps 450, with the converged
+// issuer 289, with output warps of their own 256; five documents of 8192 tokens together 177 -> 143; 16 x 1024, heads of 64,
+// 188 -> 156.  Two threads per row (16 softmax warps) were 5 - 10 % slower than one.
+// TMEM map (512 columns): [0,128) S_0, [128,256) S_1, then O_0, O_1, D wide each; P_t of a half overwrites the first 32 columns of
+// that half of S_t once its scores are in registers.
+// Shared memory at D = 128: 2 x Q 32 KB + 4 ring slots of 32 KB (at D = 64 2 x 16 KB + 8 x 16 KB) + 4 x 32 rows of the output +
+// mbarriers.
 //
 // Reference being replaced: flash-attn 2 `flash_attn_func` / `_flash_attn_varlen_forward` (mma.sync kernels) used by
 // `colossalai/shardformer/layer/attn.py:356-372,720-755`.
@@ -39,9 +45,11 @@ using namespace sm100;
 
 constexpr int BLOCK_Q = 128;
 constexpr int BLOCK_KV = 128;
+constexpr int HALF_KV = 64;            // keys of a step: a score tile is taken in two halves
 constexpr int UMMA_K = 16;
 constexpr int SOFTMAX_WARP0 = 4;
-constexpr int NUM_THREADS = (SOFTMAX_WARP0 + 8) * 32;
+constexpr int OUTPUT_WARP0 = SOFTMAX_WARP0 + 8;
+constexpr int NUM_THREADS = (OUTPUT_WARP0 + 4) * 32;
 constexpr int UNIT_RING = 2;
 
 // Waits give up after a bounded number of polls (each of which the hardware may suspend), far beyond any wait of a kernel
@@ -106,15 +114,15 @@ __global__ void flash_wait_probe_kernel(int limit, int* status) {
 }
 
 template <int D> struct FaCfg {
-  static constexpr bool SPLIT_P = D == 64;                 // P has tensor memory of its own
   static constexpr int Q_BYTES = BLOCK_Q * D * 2;
   static constexpr int SLOT_BYTES = BLOCK_KV * D * 2;      // one K or V tile
-  static constexpr int SLOTS = D == 128 ? 5 : 8;
+  static constexpr int SLOTS = D == 128 ? 4 : 8;
+  static constexpr int BOX_BYTES = 32 * D * 2;             // an output warp's 32 rows on their way out
+  static constexpr int ROW_BYTES = 2 * BLOCK_Q * 8;        // a row's reference maximum and sum
   static constexpr int BAR_BYTES = 512;
-  static constexpr int SMEM_BYTES = 2 * Q_BYTES + SLOTS * SLOT_BYTES + 1024 /*align*/ + BAR_BYTES;
+  static constexpr int SMEM_BYTES = 2 * Q_BYTES + SLOTS * SLOT_BYTES + 4 * BOX_BYTES + ROW_BYTES + BAR_BYTES;
   static constexpr int TMEM_COLS = 512;
   static constexpr int O_COL = 256;
-  static constexpr int P_COL = SPLIT_P ? 384 : 0, P_STEP = SPLIT_P ? 64 : 128;
 };
 
 struct FaParams {
@@ -164,6 +172,11 @@ SM100_DEVICE uint64_t add_f32x2(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+SM100_DEVICE uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 template <bool BF16> SM100_DEVICE uint32_t pack_16(float a, float b) {
   if (BF16) {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -174,28 +187,46 @@ template <bool BF16> SM100_DEVICE uint32_t pack_16(float a, float b) {
 }
 
 // Packed batches: units of `per` rows in descending order of their index inside the sequence (the unit with index i walks the
-// key tiles of i + 1 units), over all sequences: count(i) = units with an index >= i.  One warp, every lane gets the result.
-SM100_DEVICE int packed_count(const int* cu, int batch, int per, int i) {
+// key tiles of i + 1 units), over all sequences: count(i) = units with an index >= i.  One warp, every lane gets the result.  The
+// boundaries of the first 32 sequences stay in registers, a lane a sequence: a search is a dozen counts one after the other, and
+// read from memory for each of them it took longer than a short unit (packed_batch).
+struct PackedBatch {
+  const int* cu;
+  int batch, per, start, len;       // of this lane's sequence (0: none)
+  int units, longest;               // units of this lane's sequence, of the longest one
+};
+SM100_DEVICE int packed_units(const PackedBatch& s, int b) { return (__ldg(s.cu + b + 1) - __ldg(s.cu + b) + s.per - 1) / s.per; }
+SM100_DEVICE PackedBatch packed_batch(const int* cu, int batch, int per) {
   const int lane = threadIdx.x & 31;
-  int c = 0;
-  for (int b = lane; b < batch; b += 32) c += max(0, (__ldg(cu + b + 1) - __ldg(cu + b) + per - 1) / per - i);
+  PackedBatch s;
+  s.cu = cu; s.batch = batch; s.per = per;
+  s.start = lane < batch ? __ldg(cu + lane) : 0;
+  s.len = lane < batch ? __ldg(cu + lane + 1) - s.start : 0;
+  s.units = (s.len + per - 1) / per;
+  int longest = s.units;
+  for (int b = lane + 32; b < batch; b += 32) longest = max(longest, packed_units(s, b));
+  s.longest = __reduce_max_sync(0xffffffffu, longest);
+  return s;
+}
+SM100_DEVICE int packed_count(const PackedBatch& s, int i) {
+  int c = max(0, s.units - i);
+  for (int b = (threadIdx.x & 31) + 32; b < s.batch; b += 32) c += max(0, packed_units(s, b) - i);
   return __reduce_add_sync(0xffffffffu, c);
 }
-SM100_DEVICE void packed_unit(const int* cu, int batch, int per, int r, int& unit, int& start, int& len) {
+SM100_DEVICE void packed_unit(const PackedBatch& s, int r, int& unit, int& start, int& len) {
   const int lane = threadIdx.x & 31;
-  int longest = 0;
-  for (int b = lane; b < batch; b += 32) longest = max(longest, (__ldg(cu + b + 1) - __ldg(cu + b) + per - 1) / per);
-  int lo = 0, hi = __reduce_max_sync(0xffffffffu, longest);       // largest index lo with count(lo) > r
+  int lo = 0, hi = s.longest;                                     // largest index lo with count(lo) > r
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (packed_count(cu, batch, per, mid) > r) lo = mid; else hi = mid;
+    if (packed_count(s, mid) > r) lo = mid; else hi = mid;
   }
-  int nth = r - packed_count(cu, batch, per, lo + 1);             // the nth sequence that has a unit `lo`
+  int nth = r - packed_count(s, lo + 1);                          // the nth sequence that has a unit `lo`
   unit = lo; start = 0; len = 0;
-  for (int b0 = 0; b0 < batch; b0 += 32) {
+  for (int b0 = 0; b0 < s.batch; b0 += 32) {
     const int b = b0 + lane;
-    const int s0 = b < batch ? __ldg(cu + b) : 0, n = b < batch ? __ldg(cu + b + 1) - s0 : 0;
-    const unsigned m = __ballot_sync(0xffffffffu, (n + per - 1) / per > lo);
+    const int s0 = b0 == 0 ? s.start : b < s.batch ? __ldg(s.cu + b) : 0;
+    const int n = b0 == 0 ? s.len : b < s.batch ? __ldg(s.cu + b + 1) - s0 : 0;
+    const unsigned m = __ballot_sync(0xffffffffu, (n + s.per - 1) / s.per > lo);
     if (nth < __popc(m)) {
       const int pick = (int)__fns(m, 0, nth + 1);
       start = __shfl_sync(0xffffffffu, s0, pick);
@@ -205,6 +236,9 @@ SM100_DEVICE void packed_unit(const int* cu, int batch, int per, int r, int& uni
     nth -= __popc(m);
   }
 }
+
+// the same value in every lane, in a way that the compiler sees
+template <typename V> SM100_DEVICE V uniform(V v) { return __shfl_sync(0xffffffffu, v, 0); }
 
 struct FaUnit {
   int live, index, q_start, k_start, len_q, len_k, head0;
@@ -216,30 +250,31 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                  const __grid_constant__ CUtensorMap tmap_v, const FaParams p) {
   using C = FaCfg<D>;
   constexpr int SLOTS = C::SLOTS;
-  constexpr bool SPLIT_P = C::SPLIT_P;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];          // (the swizzle's patterns repeat every 1024 bytes)
   uint8_t* smem_q = smem;                                    // two tiles
   uint8_t* smem_kv = smem + 2 * C::Q_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_kv + SLOTS * C::SLOT_BYTES);
+  uint8_t* smem_box = smem_kv + SLOTS * C::SLOT_BYTES;       // [4 warps]
+  float2* smem_row = reinterpret_cast<float2*>(smem_box + 4 * C::BOX_BYTES);   // [2 tiles][BLOCK_Q]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_row + 2 * BLOCK_Q);
   uint64_t* q_full = bars;                 // [1]
   uint64_t* q_empty = bars + 1;            // [1]  the unit's last Q K^T retired
   uint64_t* full = bars + 2;               // [SLOTS]
   uint64_t* empty = full + SLOTS;          // [SLOTS]
-  uint64_t* s_full = empty + SLOTS;        // [2]  S_t is in tensor memory
-  uint64_t* s_empty = s_full + 2;          // [2]  4 softmax warps have read it (SPLIT_P)
-  uint64_t* p_full = s_empty + 2;          // [2]  4 softmax warps have written P_t
-  uint64_t* o_full = p_full + 2;           // [2]  P_t V_j retired: every j (SPLIT_P), else a unit's last one
-  uint64_t* o_empty = o_full + 2;          // [2]  4 softmax warps have read O_t
-  uint64_t* u_full = o_empty + 2;          // [UNIT_RING]
-  uint64_t* u_empty = u_full + UNIT_RING;  // [UNIT_RING]  10 warps have read the unit
+  uint64_t* s_full = empty + SLOTS;        // [2][2]  a half of S_t is in tensor memory
+  uint64_t* p_full = s_full + 4;           // [2][2]  4 softmax warps have written P_t over it
+  uint64_t* o_full = p_full + 4;           // [2][2]  the product that read P_t there has retired
+  uint64_t* o_empty = o_full + 4;          // [2]  4 output warps have read O_t
+  uint64_t* row_full = o_empty + 2;        // [2]  4 softmax warps are through with a unit: maxima and sums of its rows
+  uint64_t* row_empty = row_full + 2;      // [2]  4 output warps have read them
+  uint64_t* u_full = row_empty + 2;        // [UNIT_RING]
+  uint64_t* u_empty = u_full + UNIT_RING;  // [UNIT_RING]  14 warps have read the unit
   FaUnit* units = reinterpret_cast<FaUnit*>(u_empty + UNIT_RING);
   uint64_t* drained = reinterpret_cast<uint64_t*>(units + UNIT_RING);   // [1]  a CTA that gives up: its products have retired
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(drained + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   volatile int* copies = abort_flag + 1;   // [2]  key / value tiles and query tiles that the producer asked for
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const bool resume = p.o_state != nullptr && p.has_prev != 0;   // block mode: continue from the stored state
 
@@ -255,16 +290,19 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < 4; ++i) {
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], 4);
       mbar_init(&p_full[i], 4);
       mbar_init(&o_full[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
       mbar_init(&o_empty[i], 4);
+      mbar_init(&row_full[i], 4);
+      mbar_init(&row_empty[i], 4);
     }
     for (int i = 0; i < UNIT_RING; ++i) {
       mbar_init(&u_full[i], 1);
-      mbar_init(&u_empty[i], 10);
+      mbar_init(&u_empty[i], 14);
     }
     mbar_init(drained, 1);
     *abort_flag = 0;
@@ -293,16 +331,18 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   // causal with seqlen_q == seqlen_k: key tiles 0..q_tile; otherwise all of them.  Sliding window: the lowest key any row of
   // the first tile can see is (tile_of(0) * BLOCK_Q - window + 1)
   auto first_key_tile = [&]() { return (EXTRA && p.window > 0) ? max(0, tile_of(0) * BLOCK_Q - p.window + 1) / BLOCK_KV : 0; };
-  auto steps_of = [&](int t) {              // key tiles that tile t walks (0: the tile lies behind the sequence's end)
+  auto steps_of = [&](int t) {              // steps of 64 keys that tile t walks (0: the tile lies behind the sequence's end)
     if (tile_of(t) * BLOCK_Q >= un.len_q) return 0;
-    const int all = (un.len_k + BLOCK_KV - 1) / BLOCK_KV;
-    return (p.causal ? min(tile_of(t) + 1, all) : all) - first_key_tile();
+    const int all = (un.len_k + HALF_KV - 1) / HALF_KV;
+    return (p.causal ? min(2 * tile_of(t) + 2, all) : all) - 2 * first_key_tile();
   };
 
   if (warp == 3) {
     // ================================================================ unit list
     const int per = p.pair_heads ? BLOCK_Q : 2 * BLOCK_Q;      // query rows of a unit
-    const int ranks = p.cu_seqlens != nullptr ? packed_count(p.cu_seqlens, p.batch, per, 0) : p.seq_units * p.batch;
+    PackedBatch packed{};
+    if (p.cu_seqlens != nullptr) packed = packed_batch(p.cu_seqlens, p.batch, per);
+    const int ranks = p.cu_seqlens != nullptr ? packed_count(packed, 0) : p.seq_units * p.batch;
     const int total = ranks * p.head_units;
     bool ok = true;
     for (int i = 0; ok; ++i) {
@@ -315,7 +355,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const int rank = u / p.head_units;
         x.head0 = (u - rank * p.head_units) * (p.pair_heads ? 2 : 1);
         if (p.cu_seqlens != nullptr) {
-          packed_unit(p.cu_seqlens, p.batch, per, rank, x.index, x.q_start, x.len_q);
+          packed_unit(packed, rank, x.index, x.q_start, x.len_q);
           x.k_start = x.q_start; x.len_k = x.len_q;
         } else {
           const int b = rank % p.batch;
@@ -336,8 +376,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     // ================================================================ TMA producer
     int issued = 0, nq = 0;
     while (next_unit()) {
-      const int n0 = steps_of(0), n1 = steps_of(1), steps = max(n0, n1);
-      if (steps == 0) continue;
+      const int n0 = steps_of(0), n1 = steps_of(1), tiles = (max(n0, n1) + 1) / 2;
+      if (tiles == 0) continue;
       bool ok = true;
       if (lane == 0) {
         ok = wait_or_abort(q_empty, (uint32_t)((nq & 1) ^ 1), abort_flag);
@@ -350,7 +390,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                           un.q_start + tile_of(t) * BLOCK_Q);
           ++nq;
           const int kv_head = un.head0 / (p.hq / p.hkv), k_tile0 = first_key_tile();
-          for (int i = 0; i < 2 * steps && ok; ++i) {          // K_j (K-major B of Q K^T), V_j (MN-major B of P V)
+          for (int i = 0; i < 2 * tiles && ok; ++i) {          // K_j (K-major B of Q K^T), V_j (MN-major B of P V)
             const int slot = issued % SLOTS;
             ok = wait_or_abort(&empty[slot], (uint32_t)(((issued / SLOTS) & 1) ^ 1), abort_flag);
             if (!ok) break;
@@ -373,89 +413,162 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const uint64_t dq = make_smem_desc_sw128(smem_u32(smem_q), 16, 1024);                 // K-major, K = D
     const uint64_t dk0 = make_smem_desc_sw128(smem_u32(smem_kv), 16, 1024);               // K-major
     const uint64_t dv0 = make_smem_desc_sw128(smem_u32(smem_kv), BLOCK_KV * 128, 1024);   // MN-major: [keys, D] row-major
-    int base = 0, nq = 0;                    // ring index of the unit's K_0; units with work so far
-    int done[2] = {0, 0}, uses[2] = {0, 0};  // per tile: key tiles of earlier units, units it had work in
+    const uint32_t leader = elect_one();
+    int nq = 0, slot = 0;                    // units with work so far; next slot of the ring
+    int uses[2] = {0, 0};                    // per tile: units it had work in
+    uint32_t phase = 0, turn = 0;            // bit 2 t + half: parity of the next P_t in that half; parity of the ring's next slot
+    auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag)) != 0; };
     while (next_unit()) {
-      const int n0 = steps_of(0), n1 = steps_of(1), steps = max(n0, n1);
+      const int n0 = uniform(steps_of(0)), n1 = uniform(steps_of(1)), steps = max(n0, n1), tiles = (steps + 1) / 2;
       if (steps == 0) continue;
-      bool ok = true;
-      if (lane == 0) {
-        auto wait_slot = [&](int i) {
-          i += base;
-          return wait_or_abort(&full[i % SLOTS], (uint32_t)((i / SLOTS) & 1), abort_flag);
-        };
-        auto qk = [&](int t, int j) -> bool {
-          if (SPLIT_P && !wait_or_abort(&s_empty[t], (uint32_t)(((done[t] + j) & 1) ^ 1), abort_flag)) return false;
-          tc_fence_after();
-          const uint32_t ko = ((base + 2 * j) % SLOTS) * C::SLOT_BYTES;
+      auto take = [&](int& at) {             // the next tile of the ring: K_0, V_0, K_1, V_1, ...
+        at = slot;
+        const bool here = warp_wait(&full[slot], turn);
+        if (++slot == SLOTS) { slot = 0; turn ^= 1; }
+        return here;
+      };
+      int ks = 0, vs = 0;                    // slots of the key tile and the value tile in use
+      // half h of S_t <- Q_t times the 64 keys of a step.  What was there has been read: P_t came from it, and the product
+      // that reads P_t was issued before (products of one thread run in order).
+      auto qk = [&](int t, int h) {
+        tc_fence_after();
+        const uint32_t a = desc_lo(dq) + t * (C::Q_BYTES >> 4), b = desc_lo(dk0) + ks * (C::SLOT_BYTES >> 4) + h * (HALF_KV * 128 >> 4);
 #pragma unroll
-          for (int k = 0; k < D / UMMA_K; ++k) {
-            const uint32_t off = (k >> 2) * (128 * 128) + (k & 3) * (UMMA_K * 2);
-            umma_f16_ss(tmem_base + t * BLOCK_KV, advance_desc(dq, t * C::Q_BYTES + off), advance_desc(dk0, ko + off),
-                        p.idesc_qk, k > 0 ? 1u : 0u);
-          }
-          umma_commit(&s_full[t]);
-          return true;
-        };
-        auto pv = [&](int t, int j) -> bool {
-          if (!wait_or_abort(&p_full[t], (uint32_t)((done[t] + j) & 1), abort_flag)) return false;   // O_t rescaled if it had to be
-          // O accumulates in TMEM over all key tiles (the first MMA of a unit overwrites, unless the accumulator was
-          // pre-loaded with the state of earlier launches); P: 16 keys = 8 columns
-          const bool fresh = j == 0 && !resume;
-          if (fresh && !wait_or_abort(&o_empty[t], (uint32_t)((uses[t] & 1) ^ 1), abort_flag)) return false;
-          tc_fence_after();
-          const uint32_t vo = ((base + 2 * j + 1) % SLOTS) * C::SLOT_BYTES;
-#pragma unroll
-          for (int k = 0; k < BLOCK_KV / UMMA_K; ++k)
-            umma_f16_ts(tmem_base + C::O_COL + t * D, tmem_base + C::P_COL + t * C::P_STEP + k * 8,
-                        advance_desc(dv0, vo + k * (UMMA_K * 128)), p.idesc_pv, (fresh && k == 0) ? 0u : 1u);
-          if (SPLIT_P || j == (t ? n1 : n0) - 1) umma_commit(&o_full[t]);
-          return true;
-        };
-        auto release = [&](int i) { umma_commit(&empty[(base + i) % SLOTS]); };
-        ok = wait_or_abort(q_full, (uint32_t)(nq & 1), abort_flag) && wait_slot(0);
-        if (n0 > 0) ok = ok && qk(0, 0);
-        if (n1 > 0) ok = ok && qk(1, 0);
-        if (ok) {
-          release(0);
-          if (steps == 1) umma_commit(q_empty);
+        for (int k = 0; k < D / UMMA_K; ++k) {
+          const uint32_t off = ((k >> 2) * (128 * 128) + (k & 3) * (UMMA_K * 2)) >> 4;
+          umma_f16_ss_warp(leader, tmem_base + t * BLOCK_KV + h * HALF_KV, a + off, desc_hi(dq), b + off, desc_hi(dk0), p.idesc_qk,
+                           k > 0 ? 1u : 0u);
         }
-        for (int j = 0; j < steps && ok; ++j) {
-          const bool next = j + 1 < steps;
-          if (SPLIT_P) {
-            if (next) {                                        // both S of the next key tile, as soon as these were read
-              ok = wait_slot(2 * j + 2);
-              if (j + 1 < n0) ok = ok && qk(0, j + 1);
-              if (j + 1 < n1) ok = ok && qk(1, j + 1);
-              if (ok) release(2 * j + 2);
-              if (ok && j + 2 == steps) umma_commit(q_empty);  // the unit's last Q K^T has been issued
-            }
-            ok = ok && wait_slot(2 * j + 1);
-            if (j < n0) ok = ok && pv(0, j);
-            if (j < n1) ok = ok && pv(1, j);
-            if (ok) release(2 * j + 1);
-          } else {
-            // P_t lies in S_t: the next S_t follows the product that reads P_t (MMAs of one thread run in order)
-            ok = wait_slot(2 * j + 1);
-            if (j < n0) ok = ok && pv(0, j);
-            if (j + 1 < n0) ok = ok && wait_slot(2 * j + 2) && qk(0, j + 1);
-            if (j < n1) ok = ok && pv(1, j);
-            if (ok) release(2 * j + 1);
-            if (j + 1 < n1) ok = ok && wait_slot(2 * j + 2) && qk(1, j + 1);
-            if (next && ok) release(2 * j + 2);
-            if (ok && j + 2 == steps) umma_commit(q_empty);
+        umma_commit_warp(leader, &s_full[2 * t + h]);
+      };
+      auto pv = [&](int t, int h, bool first) -> bool {
+        const int i = 2 * t + h;
+        if (!warp_wait(&p_full[i], (phase >> i) & 1)) return false;      // O_t rescaled if it had to be
+        phase ^= 1u << i;
+        // O accumulates in TMEM over all steps (the first MMA of a unit overwrites, unless the accumulator was
+        // pre-loaded with the state of earlier launches); P: 16 keys = 8 columns
+        const bool fresh = first && !resume;
+        if (fresh && !warp_wait(&o_empty[t], (uint32_t)((uses[t] & 1) ^ 1))) return false;
+        tc_fence_after();
+        const uint32_t b = desc_lo(dv0) + vs * (C::SLOT_BYTES >> 4) + h * (HALF_KV * 128 >> 4);
+#pragma unroll
+        for (int k = 0; k < HALF_KV / UMMA_K; ++k)
+          umma_f16_ts_warp(leader, tmem_base + C::O_COL + t * D, tmem_base + t * BLOCK_KV + h * HALF_KV + k * 8,
+                           b + (k * (UMMA_K * 128) >> 4), desc_hi(dv0), p.idesc_pv, (fresh && k == 0) ? 0u : 1u);
+        umma_commit_warp(leader, &o_full[i]);
+        return true;
+      };
+      bool ok = warp_wait(q_full, (uint32_t)(nq & 1)) && take(ks);
+      if (!ok) break;
+      if (n0 > 0) qk(0, 0);
+      if (n1 > 0) qk(1, 0);
+      if (n0 > 1) qk(0, 1);
+      if (n1 > 1) qk(1, 1);
+      umma_commit_warp(leader, &empty[ks]);
+      if (tiles == 1) umma_commit_warp(leader, q_empty);       // the unit's last Q K^T has been issued
+      for (int j = 0; j < tiles && ok; ++j) {
+        ok = take(vs) && (j + 1 == tiles || take(ks));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int s = 2 * j + h;
+          if (ok && s < n0) {
+            ok = pv(0, h, s == 0);
+            if (ok && s + 2 < n0) qk(0, h);
+          }
+          if (ok && s < n1) {
+            ok = pv(1, h, s == 0);
+            if (ok && s + 2 < n1) qk(1, h);
           }
         }
-        base += 2 * steps;
-        ++nq;
-        done[0] += n0; done[1] += n1;
-        uses[0] += n0 > 0; uses[1] += n1 > 0;
+        if (!ok) break;
+        umma_commit_warp(leader, &empty[vs]);
+        if (j + 1 < tiles) umma_commit_warp(leader, &empty[ks]);
+        if (j + 2 == tiles) umma_commit_warp(leader, q_empty);
       }
-      if (!__all_sync(0xffffffffu, ok)) break;
+      if (!ok) break;
+      ++nq;
+      uses[0] += n0 > 0; uses[1] += n1 > 0;
     }
     __syncwarp();
+  } else if (warp >= OUTPUT_WARP0) {
+    // ================================================================ output
+    // What a unit ends with - its last P V, the division, the way out - runs beside the softmax of the next one.  A warp takes 32
+    // rows of either tile, and through shared memory, so that a store writes whole lines: a lane's own row at a time, every 16
+    // bytes in another line, held up the softmax warps for 8700 clocks per unit of D = 128 (70000 for one of 2112 keys).
+    const int quarter = warp & 3;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    uint8_t* box = smem_box + quarter * C::BOX_BYTES;
+    constexpr int CHUNKS = D / 8;                          // 16-byte pieces of a row
+    uint32_t phase = 0, units_of = 0;                      // bit 2 t + h: parity of the next P V of half h;  bit t: of the next unit
+    bool ok = true;
+    auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag)) != 0; };
+    while (ok && next_unit()) {
+#pragma unroll 1
+      for (int t = 0; t < 2 && ok; ++t) {
+        const int n = steps_of(t);
+        if (n == 0) continue;
+        // the softmax warps are through: S of the last step has come, so the P V before the last of either half has retired
+        ok = warp_wait(&row_full[t], (units_of >> t) & 1);
+        if (!ok) break;
+        units_of ^= 1u << t;
+        const int last = 2 * t + ((n - 1) & 1);
+        phase ^= (uint32_t)(((n + 1) / 2) & 1) << (2 * t) | (uint32_t)((n / 2) & 1) << (2 * t + 1);
+        const int r = quarter * 32 + lane;
+        const float2 ml = smem_row[t * BLOCK_Q + r];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&row_empty[t]);
+        ok = warp_wait(&o_full[last], ((phase >> last) & 1) ^ 1);
+        if (!ok) break;
+        tc_fence_after();
+        const int head = head_of(t), row0 = tile_of(t) * BLOCK_Q + quarter * 32, live = un.len_q - row0;   // rows of this warp
+        const size_t token0 = (size_t)un.q_start + row0, ld = (size_t)p.hq * D;
+        const float inv_l = ml.y > 0.f ? 1.f / ml.y : 0.f;
+#pragma unroll
+        for (int c = 0; c < D; c += 32) {
+          uint32_t w[32];
+          tmem_ld_32x32b_x32(tmem_base + lane_addr + C::O_COL + t * D + c, w);
+          tmem_ld_wait();
+          if (c + 32 == D) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&o_empty[t]);       // O_t may be overwritten by the next unit
+          }
+          if (p.o_state != nullptr) {
+            if (lane < live) {
+              float4* dst = reinterpret_cast<float4*>(p.o_state + (token0 + lane) * ld + (size_t)head * D + c);
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                dst[i] = make_float4(__uint_as_float(w[4 * i]) * inv_l, __uint_as_float(w[4 * i + 1]) * inv_l,
+                                     __uint_as_float(w[4 * i + 2]) * inv_l, __uint_as_float(w[4 * i + 3]) * inv_l);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint32_t h[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                h[e] = pack_16<BF16>(__uint_as_float(w[8 * i + 2 * e]) * inv_l, __uint_as_float(w[8 * i + 2 * e + 1]) * inv_l);
+              *reinterpret_cast<uint4*>(box + (lane * CHUNKS + ((c / 8 + i) ^ (lane & 7))) * 16) = make_uint4(h[0], h[1], h[2], h[3]);
+            }
+          }
+        }
+        if (p.o_state == nullptr) {
+          __syncwarp();
+          uint8_t* out = reinterpret_cast<uint8_t*>(p.out) + (token0 * ld + (size_t)head * D) * 2;
+#pragma unroll
+          for (int i = 0; i < CHUNKS; ++i) {
+            const int at = i * 32 + lane, row = at / CHUNKS, chunk = at % CHUNKS;
+            const uint4 x = *reinterpret_cast<const uint4*>(box + (row * CHUNKS + (chunk ^ (row & 7))) * 16);
+            if (row < live) *reinterpret_cast<uint4*>(out + row * (ld * 2) + chunk * 16) = x;
+          }
+          __syncwarp();
+        }
+        if (p.lse && lane < live)
+          p.lse[(token0 + lane) * p.hq + head] = ml.y > 0.f ? (ml.x + log2f(ml.y)) * 0.6931471805599453f : -INFINITY;
+      }
+    }
   } else if (warp >= SOFTMAX_WARP0) {
-    // ================================================================ softmax + output
+    // ================================================================ softmax
     // Thread = query row.  The output accumulator lives in TMEM for the whole walk (P_j V_j accumulates onto it in the
     // tensor core); the exponentials are taken against a LAGGING row max: the accumulator is only rescaled when the
     // true max has grown by more than 2^TAU since the last rescale (exact: numerator and denominator use the same
@@ -467,25 +580,25 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const uint32_t o_addr = tmem_base + lane_addr + C::O_COL + t * D;
     const uint32_t s_addr = tmem_base + lane_addr + t * BLOCK_KV;
-    const uint32_t p_addr = tmem_base + lane_addr + C::P_COL + t * C::P_STEP;
-    int done = 0, uses = 0;                              // key tiles / units of this tile so far
+    uint32_t phase = 0, units_of = 0;                    // bit h: parity of the next S_t in half h; units of this tile so far
     bool ok = true;
     while (ok && next_unit()) {
       const int n_steps = steps_of(t);
       if (n_steps == 0) continue;
-      const int q_tile = tile_of(t), head = head_of(t), len_q = un.len_q, len_k = un.len_k;
+      const int q_tile = tile_of(t), head = head_of(t), len_k = un.len_k;
       const int kv_first = first_key_tile();
       const int q_pos = q_tile * BLOCK_Q + r;              // position inside the sequence
       const size_t row = (size_t)un.q_start + q_pos;       // row in the token-major Q / O
-      const int last_tile = (len_k + BLOCK_KV - 1) / BLOCK_KV - 1;
-      const bool ragged_k = (len_k % BLOCK_KV) != 0;       // the last key tile runs past the end of the sequence
       float m_run = -INFINITY;                             // reference max of the exponentials (exp2 domain)
       float l_run = 0.f;
       if (resume) {
+        ok = __all_sync(0xffffffffu, wait_or_abort(&o_empty[t], (units_of & 1) ^ 1, abort_flag));
+        if (!ok) break;
+        tc_fence_after();
         // resume from the merged result of the key blocks processed by earlier launches (normalised output + LSE):
         // every row stores its previous output (or zeros) into the TMEM accumulator, P_0 V_0 accumulates onto it
         float lse_prev = -INFINITY;
-        if (q_pos < len_q) lse_prev = p.lse[row * p.hq + head];
+        if (q_pos < un.len_q) lse_prev = p.lse[row * p.hq + head];
         const bool live = lse_prev > -INFINITY;
         if (live) { m_run = lse_prev * 1.4426950408889634f; l_run = 1.f; }
         const float4* src = reinterpret_cast<const float4*>(p.o_state + row * ((size_t)p.hq * D) + (size_t)head * D);
@@ -504,39 +617,38 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       }
       const float slope2 = (EXTRA && p.alibi != nullptr) ? p.alibi[head] * 1.4426950408889634f : 0.f;
       (void)slope2;
-      // one key tile; two copies of the code, because a branch around the mask alone is turned into 128 predicated
-      // comparisons and selections that every tile executes
+      // P V of step j, the last one in its half: the one before in that half retired before S of step j came
+      auto product_done = [&](int j) -> bool {
+        const int h = j & 1;
+        return __all_sync(0xffffffffu, wait_or_abort(&o_full[2 * t + h], ((phase >> h) & 1) ^ 1, abort_flag)) != 0;
+      };
+      // one step of 64 keys; two copies of the code, because a branch around the mask alone is turned into predicated
+      // comparisons and selections that every step executes
       auto step = [&](int j, auto masked_tag) -> bool {
         constexpr bool MASKED = decltype(masked_tag)::value;
-        const int kt = kv_first + j;                         // key tile of this step
-        // ---- the whole score row into registers
-        uint32_t v[BLOCK_KV];
+        const int k_base = kv_first * BLOCK_KV + j * HALF_KV;
+        const uint32_t half_addr = s_addr + (j & 1) * HALF_KV;
+        uint32_t v[HALF_KV];
 #pragma unroll
-        for (int c = 0; c < BLOCK_KV; c += 32) tmem_ld_32x32b_x32(s_addr + c, *reinterpret_cast<uint32_t(*)[32]>(&v[c]));
+        for (int c = 0; c < HALF_KV; c += 32) tmem_ld_32x32b_x32(half_addr + c, *reinterpret_cast<uint32_t(*)[32]>(&v[c]));
         tmem_ld_wait();
-        if (SPLIT_P) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&s_empty[t]);           // S_t may be overwritten by Q K_{j+1}^T
-        }
         // plain variant: the softmax scale (> 0) is folded into the exponent's FMA, the max is taken on the raw scores;
         // EXTRA variant: scale and ALiBi bias are applied here and the exponent uses a unit multiplier
         if (EXTRA || MASKED) {
-          const int k_base = kt * BLOCK_KV;
-          const int k_lim = (p.causal && kt == q_tile) ? min(q_pos, len_k - 1) : (len_k - 1);   // last visible key of this row
+          const int k_lim = p.causal ? min(q_pos, len_k - 1) : len_k - 1;                        // last visible key of this row
           const int k_low = (EXTRA && p.window > 0) ? q_pos - p.window + 1 : 0;                  // first visible key
 #pragma unroll
-          for (int i = 0; i < BLOCK_KV; ++i) {
+          for (int i = 0; i < HALF_KV; ++i) {
             float sc = __uint_as_float(v[i]);
             if (EXTRA) sc = fmaf(slope2, (float)(k_base + i - q_pos), sc * p.scale_log2);
             if (MASKED && ((k_base + i) > k_lim || (EXTRA && (k_base + i) < k_low))) sc = -INFINITY;
             v[i] = __float_as_uint(sc);
           }
         }
-        // (four independent partial maxima / sums: a single running value would be a 128-long dependent chain)
+        // (four independent partial maxima / sums: a single running value would be a 64-long dependent chain)
         float mt[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int i = 0; i < BLOCK_KV; i += 8)
+        for (int i = 0; i < HALF_KV; i += 8)
 #pragma unroll
           for (int e = 0; e < 4; ++e)
             mt[e] = fmaxf(fmaxf(mt[e], __uint_as_float(v[i + e])), __uint_as_float(v[i + e + 4]));
@@ -544,15 +656,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const float m_tile = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3])) * ex_mul;
         // ---- lagging max / rare rescale of the TMEM accumulator
         const float m_new = fmaxf(m_run, m_tile);
-        bool waited = !SPLIT_P || j == 0;                      // P V of the last key tile is known to have retired
         if (j == 0 && !resume) {
           m_run = m_new;                                       // nothing accumulated yet
         } else {
           const bool need = (m_new - m_run) > TAU;             // (-inf) - (-inf) = NaN -> false
           if (__any_sync(0xffffffffu, need)) {
-            if (!waited) {
-              if (!__all_sync(0xffffffffu, wait_or_abort(&o_full[t], (uint32_t)((done - 1) & 1), abort_flag))) return false;
-              waited = true;
+            if (j > 0) {
+              if (!product_done(j - 1)) return false;
               tc_fence_after();
             }
             const float alpha = need ? fast_exp2(m_run - m_new) : 1.f;
@@ -570,16 +680,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             if (need) m_run = m_new;
           }
         }
-        if (!waited) {                                          // P_{j-1} has been read: its columns are free
-          if (!__all_sync(0xffffffffu, wait_or_abort(&o_full[t], (uint32_t)((done - 1) & 1), abort_flag))) return false;
-          tc_fence_after();
-        }
         const float m_use = (m_run == -INFINITY) ? 0.f : m_run;     // keeps the exponent finite on a fully masked row
-        // ---- p = exp2(s - m), row sum, 16-bit P to tensor memory
+        // ---- p = exp2(s - m), row sum, 16-bit P over the scores it came from
         const uint64_t mul2 = pack_f32x2(ex_mul, ex_mul), sub2 = pack_f32x2(-m_use, -m_use);
         uint64_t lt[2] = {0ull, 0ull};
 #pragma unroll
-        for (int c = 0; c < BLOCK_KV; c += 32) {
+        for (int c = 0; c < HALF_KV; c += 32) {
           uint32_t packed[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
@@ -590,7 +696,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             lt[(i >> 1) & 1] = add_f32x2(lt[(i >> 1) & 1], pack_f32x2(p0, p1));
             packed[i >> 1] = pack_16<BF16>(p0, p1);
           }
-          tmem_st_32x32b_x16(p_addr + (c >> 1), packed);
+          tmem_st_32x32b_x16(half_addr + (c >> 1), packed);
         }
         float l0, l1, l2, l3;
         unpack_f32x2(lt[0], l0, l1);
@@ -599,60 +705,28 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&p_full[t]);            // P_j is in tensor memory, the accumulator is consistent
+        if (lane == 0) mbar_arrive(&p_full[2 * t + (j & 1)]);  // P is in tensor memory, the accumulator is consistent
         return true;
       };
+      // a step needs the mask if its last key is behind what this warp's first row sees, or behind the end of the sequence
+      const int k_all = p.causal ? min(q_tile * BLOCK_Q + quarter * 32, len_k - 1) : len_k - 1;
       for (int j = 0; j < n_steps && ok; ++j) {
-        ok = __all_sync(0xffffffffu, wait_or_abort(&s_full[t], (uint32_t)(done & 1), abort_flag));
+        const int h = j & 1;
+        ok = __all_sync(0xffffffffu, wait_or_abort(&s_full[2 * t + h], (phase >> h) & 1, abort_flag));
         if (!ok) break;
+        phase ^= 1u << h;
         tc_fence_after();
-        const int kt = kv_first + j;
-        const bool masked = (p.causal && kt == q_tile) || (ragged_k && kt == last_tile) || (EXTRA && p.window > 0);
+        const bool masked = kv_first * BLOCK_KV + j * HALF_KV + HALF_KV - 1 > k_all || (EXTRA && p.window > 0);
         ok = masked ? step(j, std::true_type{}) : step(j, std::false_type{});
-        ++done;
       }
       if (!ok) break;
-      // ---- epilogue: the last P V has retired; normalise and store this thread's row
-      ok = __all_sync(0xffffffffu, wait_or_abort(&o_full[t], (uint32_t)((SPLIT_P ? done - 1 : uses) & 1), abort_flag));
+      // ---- the row's maximum and sum go to the output warps
+      ok = __all_sync(0xffffffffu, wait_or_abort(&row_empty[t], (units_of & 1) ^ 1, abort_flag));
       if (!ok) break;
-      tc_fence_after();
-      const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
-      const bool row_ok = q_pos < len_q;                   // rows past the end of a (packed) sequence are never stored
-#pragma unroll 1
-      for (int c = 0; c < D; c += 32) {
-        uint32_t w[32];
-        __syncwarp();
-        tmem_ld_32x32b_x32(o_addr + c, w);                 // executed by every lane (warp-collective), stores predicated
-        tmem_ld_wait();
-        if (c + 32 == D) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&o_empty[t]);         // O_t may be overwritten by the next unit
-        }
-        if (!row_ok) {
-          // a row past the end of its (packed) sequence: computed on garbage, never stored
-        } else if (p.o_state != nullptr) {
-          float4* dst = reinterpret_cast<float4*>(p.o_state + row * ((size_t)p.hq * D) + (size_t)head * D + c);
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            dst[i] = make_float4(__uint_as_float(w[4 * i]) * inv_l, __uint_as_float(w[4 * i + 1]) * inv_l,
-                                 __uint_as_float(w[4 * i + 2]) * inv_l, __uint_as_float(w[4 * i + 3]) * inv_l);
-        } else {
-          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) +
-                                                (row * ((size_t)p.hq * D) + (size_t)head * D + c) * 2);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t h[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              h[e] = pack_16<BF16>(__uint_as_float(w[8 * i + 2 * e]) * inv_l, __uint_as_float(w[8 * i + 2 * e + 1]) * inv_l);
-            dst[i] = make_uint4(h[0], h[1], h[2], h[3]);
-          }
-        }
-      }
-      if (p.lse && row_ok)
-        p.lse[row * p.hq + head] = l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
-      ++uses;
+      ++units_of;
+      smem_row[t * BLOCK_Q + r] = make_float2(m_run, l_run);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&row_full[t]);
     }
   }
   tc_fence_before();
@@ -667,7 +741,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         wait_or_abort(&full[i % SLOTS], (uint32_t)((i / SLOTS) & 1), &none);
       }
     }
-    if (warp == 1 && lane == 0) {            // the thread that issued the products
+    if (warp == 1 && elect_one()) {          // the thread that issued the products
       umma_commit(drained);
       wait_or_abort(drained, 0, &none);
     }
@@ -1124,6 +1198,7 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* out, flo
   const int per = p.pair_heads ? BLOCK_Q : 2 * BLOCK_Q;
   p.head_units = p.pair_heads ? hq / 2 : hq;
   p.seq_units = cu_seqlens ? 0 : (seqlen_q + per - 1) / per;
+  p.idesc_qk = make_idesc_f16(BLOCK_Q, HALF_KV, bf16 ? 1 : 0, 0, 0);
   const long long most = (cu_seqlens ? total_tokens / per + batch : (long long)p.seq_units * batch) * p.head_units;
   if (most > (1ll << 30)) return (int)cudaErrorInvalidValue;
   const dim3 grid((unsigned)(most < cb_num_sms() ? most : cb_num_sms()));
@@ -1154,22 +1229,23 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* out, flo
 //   dQ^T = K^T  (A, MN-major view of the resident K tile) x dS (B, MN-major view of the dS^T tile)      [128 d x 64 q]
 // i.e. five tensor-core GEMMs per (key tile, query tile) pair out of four smem operands, no transposition pass.
 //
-// Warps (16): 0 TMA producer (K, V once; Q_i / dO_i through a 3-stage ring), 1 MMA issuer, 2..3 row statistics (log-sum-exp and
+// Warps (16): 0 TMA producer (K, V once; Q_i / dO_i through a 3-stage ring), 1 MMA issuer (converged, as in the forward), 2..3 row statistics (log-sum-exp and
 // delta of the query rows, three tiles ahead), 4..11 softmax (two threads per key row, 32 queries each), 12..15 dQ drain
 // (thread = head-dim lane; 128-byte coalesced fp32 reductions per query row).
 // The issuer runs S^T / dP^T of tile i+1 BEFORE the three accumulation GEMMs of tile i, so the tensor pipe works while
 // the softmax warps are busy (same trick as the forward kernel); P^T / dS^T are double-buffered, so the softmax of tile i+1
 // does not wait for those GEMMs either.
-// Bound: 1280 clocks of MMA per (key tile, query tile).  With four softmax warps, single buffers, a two-stage ring and the
-// statistics fetched inside the softmax (a global load in front of every tile) an iteration took about 6000 clocks:
-// 4096 x 32 / 8 heads x 128 causal 1040 us (with the passes around it), now 538 (638 TFLOP/s).
-// TMEM (512 columns): [0,64) S^T, [64,128) dP^T, [128,192) dQ^T, [256,384) dV, [384,512) dK.
+// Bound: 1280 clocks of MMA per (key tile, query tile), of which products with N = 64 take half as long again for reading their
+// operands from shared memory.  4096 x 32 / 8 heads x 128 causal, two sequences, this kernel alone: 936 us; with the converged
+// issuer (32 products a tile at about 80 clocks each were its bound) 780, with two dQ^T accumulators - the drain of one no longer
+// holds up the issue of what the next tile needs - and without the waits that an earlier one implies 759.
+// TMEM (512 columns): [0,64) S^T, [64,128) dP^T, [128,192) and [192,256) dQ^T, [256,384) dV, [384,512) dK.
 // Shared memory: K 32 KB + V 32 KB + 3 x (Q 16 KB + dO 16 KB) + 2 x (P^T 16 KB + dS^T 16 KB) + statistics = 226 KB (D = 128).
 constexpr int BWD_BLOCK_KV = 128;
 constexpr int BWD_BLOCK_Q = 64;
 constexpr int BWD_THREADS = 512;
 constexpr int BWD_QSTAGES = 3;
-constexpr int BWD_STAT_WARP0 = 2, BWD_SOFTMAX_WARP0 = 4, BWD_DRAIN_WARP0 = 12;
+constexpr int BWD_STAT_WARP0 = 2, BWD_SOFTMAX_WARP0 = 4, BWD_SOFTMAX_WARPS = 8, BWD_DRAIN_WARP0 = 12;
 
 template <int D> struct FaBwdCfg {
   static constexpr int K_BYTES = BWD_BLOCK_KV * D * 2;
@@ -1204,6 +1280,15 @@ struct FaBwdParams {
   uint32_t idesc_st, idesc_dv, idesc_dqt;
 };
 
+// the (query head, query tile) pairs that a key tile walks, tiles fastest
+struct QueryWalk {
+  int first, end, tile, head;
+  SM100_DEVICE QueryWalk(int first_tile, int tiles, int first_head) : first(first_tile), end(tiles), tile(first_tile), head(first_head) {}
+  SM100_DEVICE void next() {
+    if (++tile == end) { tile = first; ++head; }
+  }
+};
+
 template <int D, bool BF16>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -1225,20 +1310,19 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint64_t* qdo_full = bars + 1;           // [ST]
   uint64_t* qdo_empty = qdo_full + ST;     // [ST]
   uint64_t* stat_full = qdo_empty + ST;    // [ST]  2 statistics warps
-  uint64_t* stat_empty = stat_full + ST;   // [ST]  8 softmax warps
+  uint64_t* stat_empty = stat_full + ST;   // [ST]  softmax warps
   uint64_t* sp_full = stat_empty + ST;     // [1]  S^T and dP^T are in TMEM
-  uint64_t* sp_empty = sp_full + 1;        // [1]  8 softmax warps have read them
-  uint64_t* pds_full = sp_empty + 1;       // [2]  8 softmax warps wrote P^T / dS^T to smem
-  uint64_t* pds_empty = pds_full + 2;      // [2]  the three accumulation GEMMs that read them retired
-  uint64_t* dq_full = pds_empty + 2;       // [1]  dQ^T is in TMEM
-  uint64_t* dq_empty = dq_full + 1;        // [1]  4 drain warps have read it
-  uint64_t* acc_full = dq_empty + 1;       // [1]  final dK / dV complete
+  uint64_t* sp_empty = sp_full + 1;        // [1]  the softmax warps have read them
+  uint64_t* pds_full = sp_empty + 1;       // [2]  the softmax warps wrote P^T / dS^T to smem
+  uint64_t* dq_full = pds_full + 2;       // [2]  dQ^T is in TMEM
+  uint64_t* dq_empty = dq_full + 2;        // [2]  4 drain warps have read it
+  uint64_t* acc_full = dq_empty + 2;       // [1]  final dK / dV complete
   uint64_t* drained = acc_full + 1;        // [1]  a CTA that gives up: its products have retired
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(drained + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   int* work = reinterpret_cast<int*>(tmem_ptr_smem + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   // key tiles that see the most queries first; heads vary fastest (both in grid.x: a packed batch may have more key tiles than
   // grid.y holds)
@@ -1248,14 +1332,14 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   if (p.cu_seqlens != nullptr) {
     if (warp == 0) {
       int unit = -1, start = 0, n = 0;
-      if (unit_of_head < packed_count(p.cu_seqlens, p.batch, BWD_BLOCK_KV, 0))
-        packed_unit(p.cu_seqlens, p.batch, BWD_BLOCK_KV, unit_of_head, unit, start, n);
+      const PackedBatch packed = packed_batch(p.cu_seqlens, p.batch, BWD_BLOCK_KV);
+      if (unit_of_head < packed_count(packed, 0)) packed_unit(packed, unit_of_head, unit, start, n);
       if (lane == 0) { work[0] = unit; work[1] = start; work[2] = n; }
     }
     __syncthreads();
     if (work[0] < 0) return;                 // uniform across the CTA: nothing has been allocated yet
-    seq_row0 = work[1]; len = work[2];
-    kv_tile = (len + BWD_BLOCK_KV - 1) / BWD_BLOCK_KV - 1 - work[0];
+    seq_row0 = uniform(work[1]); len = uniform(work[2]);
+    kv_tile = (len + BWD_BLOCK_KV - 1) / BWD_BLOCK_KV - 1 - uniform(work[0]);
   } else {
     kv_tile = unit_of_head; seq_row0 = (int)blockIdx.y * p.seqlen; len = p.seqlen;
   }
@@ -1279,16 +1363,15 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       mbar_init(&qdo_full[i], 1);
       mbar_init(&qdo_empty[i], 1);
       mbar_init(&stat_full[i], 2);
-      mbar_init(&stat_empty[i], 8);
+      mbar_init(&stat_empty[i], BWD_SOFTMAX_WARPS);
     }
     mbar_init(sp_full, 1);
-    mbar_init(sp_empty, 8);
+    mbar_init(sp_empty, BWD_SOFTMAX_WARPS);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&pds_full[i], 8);
-      mbar_init(&pds_empty[i], 1);
+      mbar_init(&pds_full[i], BWD_SOFTMAX_WARPS);
+      mbar_init(&dq_full[i], 1);
+      mbar_init(&dq_empty[i], 4);
     }
-    mbar_init(dq_full, 1);
-    mbar_init(dq_empty, 4);
     mbar_init(acc_full, 1);
     mbar_init(drained, 1);
     *abort_flag = 0;
@@ -1312,10 +1395,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         tma_load_2d(&tmap_k, kv_full, smem_k + h * (BWD_BLOCK_KV * 128), kv_head * D + h * 64, kv_row0);
         tma_load_2d(&tmap_v, kv_full, smem_v + h * (BWD_BLOCK_KV * 128), kv_head * D + h * 64, kv_row0);
       }
-      for (; it < n_iter; ++it) {
-        const int stage = it % ST;
-        const int hq = kv_head * group + it / n_i;
-        const int q_row0 = seq_row0 + (i_start + it % n_i) * BWD_BLOCK_Q;
+      QueryWalk at(i_start, q_tiles, kv_head * group);
+      for (; it < n_iter; ++it, at.next()) {
+        const int stage = it % ST, hq = at.head;
+        const int q_row0 = seq_row0 + at.tile * BWD_BLOCK_Q;
         if (!wait_or_abort(&qdo_empty[stage], ring_parity(it) ^ 1, abort_flag)) break;
         uint8_t* sq = smem_qdo + stage * C::QDO_STAGE_BYTES;
         uint8_t* sdo = sq + C::Q_BYTES;
@@ -1341,77 +1424,73 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     __syncwarp();
   } else if (warp == 1) {
     // ================================================================ MMA issuer
-    if (lane == 0 && n_iter > 0) {
+    const uint32_t leader = elect_one();
+    if (n_iter > 0) {
       const uint32_t sk = smem_u32(smem_k), sv = smem_u32(smem_v);
       const uint64_t dk_kmaj = make_smem_desc_sw128(sk, 16, 1024);                        // A of S^T: [keys x d] K-major
       const uint64_t dv_kmaj = make_smem_desc_sw128(sv, 16, 1024);                        // A of dP^T
       const uint64_t dk_mnmaj = make_smem_desc_sw128(sk, BWD_BLOCK_KV * 128, 1024);       // A of dQ^T: K^T, M = d contiguous
+      // of stage / buffer 0; B operands of the accumulations are MN-major views of the Q / dO tiles: rows = q (the reduction
+      // dim), N = d contiguous, 64-element N chunks are BWD_BLOCK_Q * 128 bytes apart
+      const uint32_t sq = smem_u32(smem_qdo), spt = smem_u32(smem_pt), sdst = smem_u32(smem_dst);
+      const uint64_t dq_b = make_smem_desc_sw128(sq, 16, 1024), ddo_b = make_smem_desc_sw128(sq + C::Q_BYTES, 16, 1024);
+      const uint64_t dq_mn = make_smem_desc_sw128(sq, BWD_BLOCK_Q * 128, 1024);
+      const uint64_t ddo_mn = make_smem_desc_sw128(sq + C::Q_BYTES, BWD_BLOCK_Q * 128, 1024);
+      const uint64_t d_pt = make_smem_desc_sw128(spt, 16, 1024);                          // A of dV: [keys x q] K-major
+      const uint64_t d_dst = make_smem_desc_sw128(sdst, 16, 1024);                        // A of dK
+      const uint64_t d_ds_mn = make_smem_desc_sw128(sdst, BWD_BLOCK_KV * 128, 1024);      // B of dQ^T (N = q)
+      // one product: COUNT instructions of 16 along the reduction; a_off / b_off: bytes of the stage or buffer in use
+      auto product = [&](uint32_t col, uint64_t da, uint32_t a_off, auto a_step, uint64_t db, uint32_t b_off, auto b_step, auto count,
+                         uint32_t idesc, uint32_t acc) {
+#pragma unroll
+        for (int k = 0; k < decltype(count)::value; ++k)
+          umma_f16_ss_warp(leader, tmem_base + col, desc_lo(da) + ((a_off + a_step(k)) >> 4), desc_hi(da),
+                           desc_lo(db) + ((b_off + b_step(k)) >> 4), desc_hi(db), idesc, k > 0 ? 1u : acc);
+      };
+      auto kmaj_kv = [](int k) { return (uint32_t)((k >> 2) * (BWD_BLOCK_KV * 128) + (k & 3) * (UMMA_K * 2)); };
+      auto kmaj_q = [](int k) { return (uint32_t)((k >> 2) * (BWD_BLOCK_Q * 128) + (k & 3) * (UMMA_K * 2)); };
+      auto mnmaj = [](int k) { return (uint32_t)(k * (UMMA_K * 128)); };
+      using OverD = std::integral_constant<int, D / UMMA_K>;
+      using OverQ = std::integral_constant<int, BWD_BLOCK_Q / UMMA_K>;
+      using OverKV = std::integral_constant<int, BWD_BLOCK_KV / UMMA_K>;
+      int ahead = 0;                                           // stage of the next S^T / dP^T
       auto issue_sp = [&](int it) -> bool {
-        const int stage = it % ST;
-        if (!wait_or_abort(&qdo_full[stage], ring_parity(it), abort_flag)) return false;
-        if (!wait_or_abort(sp_empty, (uint32_t)((it & 1) ^ 1), abort_flag)) return false;   // softmax of it-1 has read S^T / dP^T
+        if (!warp_wait(&qdo_full[ahead], ring_parity(it))) return false;
+        if (!warp_wait(sp_empty, (uint32_t)((it & 1) ^ 1))) return false;   // softmax of it-1 has read S^T / dP^T
         tc_fence_after();
-        const uint32_t sq = smem_u32(smem_qdo + stage * C::QDO_STAGE_BYTES);
-        const uint64_t dq_b = make_smem_desc_sw128(sq, 16, 1024);                       // B: [q x d] K-major
-        const uint64_t ddo_b = make_smem_desc_sw128(sq + C::Q_BYTES, 16, 1024);
-#pragma unroll
-        for (int k = 0; k < D / UMMA_K; ++k) {
-          const uint32_t ao = (k >> 2) * (BWD_BLOCK_KV * 128) + (k & 3) * (UMMA_K * 2);
-          const uint32_t bo = (k >> 2) * (BWD_BLOCK_Q * 128) + (k & 3) * (UMMA_K * 2);
-          umma_f16_ss(tmem_base + C::COL_ST, advance_desc(dk_kmaj, ao), advance_desc(dq_b, bo), p.idesc_st,
-                      k > 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < D / UMMA_K; ++k) {
-          const uint32_t ao = (k >> 2) * (BWD_BLOCK_KV * 128) + (k & 3) * (UMMA_K * 2);
-          const uint32_t bo = (k >> 2) * (BWD_BLOCK_Q * 128) + (k & 3) * (UMMA_K * 2);
-          umma_f16_ss(tmem_base + C::COL_DPT, advance_desc(dv_kmaj, ao), advance_desc(ddo_b, bo), p.idesc_st,
-                      k > 0 ? 1u : 0u);
-        }
-        umma_commit(sp_full);
+        const uint32_t off = ahead * C::QDO_STAGE_BYTES;
+        product(C::COL_ST, dk_kmaj, 0, kmaj_kv, dq_b, off, kmaj_q, OverD{}, p.idesc_st, 0u);
+        product(C::COL_DPT, dv_kmaj, 0, kmaj_kv, ddo_b, off, kmaj_q, OverD{}, p.idesc_st, 0u);
+        umma_commit_warp(leader, sp_full);
+        if (++ahead == ST) ahead = 0;
         return true;
       };
-      bool ok = wait_or_abort(kv_full, 0, abort_flag) && issue_sp(0);
-      for (int it = 0; it < n_iter && ok; ++it) {
+      bool ok = warp_wait(kv_full, 0) && issue_sp(0);
+      for (int it = 0, stage = 0; it < n_iter && ok; ++it) {
         if (it + 1 < n_iter) ok = issue_sp(it + 1);            // tensor pipe stays busy during softmax(it)
-        const int stage = it % ST, buf = it & 1;
-        ok = ok && wait_or_abort(&pds_full[buf], (uint32_t)((it >> 1) & 1), abort_flag);
+        const int buf = it & 1;
+        ok = ok && warp_wait(&pds_full[buf], (uint32_t)((it >> 1) & 1));
         if (!ok) break;
         tc_fence_after();
-        const uint32_t sq = smem_u32(smem_qdo + stage * C::QDO_STAGE_BYTES);
-        const uint32_t sdst = smem_u32(smem_dst + buf * C::PT_BYTES);
-        const uint64_t d_pt = make_smem_desc_sw128(smem_u32(smem_pt + buf * C::PT_BYTES), 16, 1024);   // A of dV: [keys x q] K-major
-        const uint64_t d_dst = make_smem_desc_sw128(sdst, 16, 1024);                                    // A of dK
-        const uint64_t d_ds_mn = make_smem_desc_sw128(sdst, BWD_BLOCK_KV * 128, 1024);                  // B of dQ^T (N = q)
-        // B operands, MN-major views of the Q / dO tiles: rows = q (the reduction dim), N = d contiguous,
-        // 64-element N chunks are BWD_BLOCK_Q * 128 bytes apart
-        const uint64_t dq_mn = make_smem_desc_sw128(sq, BWD_BLOCK_Q * 128, 1024);
-        const uint64_t ddo_mn = make_smem_desc_sw128(sq + C::Q_BYTES, BWD_BLOCK_Q * 128, 1024);
+        const uint32_t off = stage * C::QDO_STAGE_BYTES, pds = buf * C::PT_BYTES;
         const uint32_t acc = it > 0 ? 1u : 0u;
-#pragma unroll
-        for (int k = 0; k < BWD_BLOCK_Q / UMMA_K; ++k)      // dV += P^T dO      (reduction over the 64 query rows)
-          umma_f16_ss(tmem_base + C::COL_DV, advance_desc(d_pt, k * (UMMA_K * 2)),
-                      advance_desc(ddo_mn, k * (UMMA_K * 128)), p.idesc_dv, (acc | (k > 0)) ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < BWD_BLOCK_Q / UMMA_K; ++k)      // dK += dS^T Q
-          umma_f16_ss(tmem_base + C::COL_DK, advance_desc(d_dst, k * (UMMA_K * 2)),
-                      advance_desc(dq_mn, k * (UMMA_K * 128)), p.idesc_dv, (acc | (k > 0)) ? 1u : 0u);
-        umma_commit(&qdo_empty[stage]);                      // Q_i / dO_i consumed
-        ok = wait_or_abort(dq_empty, (uint32_t)((it & 1) ^ 1), abort_flag);    // dQ^T of iteration it-1 has been read
+        // dV += P^T dO and dK += dS^T Q (reductions over the 64 query rows)
+        product(C::COL_DV, d_pt, pds, kmaj_q, ddo_mn, off, mnmaj, OverQ{}, p.idesc_dv, acc);
+        product(C::COL_DK, d_dst, pds, kmaj_q, dq_mn, off, mnmaj, OverQ{}, p.idesc_dv, acc);
+        umma_commit_warp(leader, &qdo_empty[stage]);           // Q_i / dO_i consumed
+        ok = warp_wait(&dq_empty[buf], (uint32_t)(((it >> 1) & 1) ^ 1));    // dQ^T of iteration it-2 has been read
         if (!ok) break;
         tc_fence_after();
-#pragma unroll
-        for (int k = 0; k < BWD_BLOCK_KV / UMMA_K; ++k)     // dQ^T = K^T dS     (reduction over the 128 keys)
-          umma_f16_ss(tmem_base + C::COL_DQT, advance_desc(dk_mnmaj, k * (UMMA_K * 128)),
-                      advance_desc(d_ds_mn, k * (UMMA_K * 128)), p.idesc_dqt, k > 0 ? 1u : 0u);
-        umma_commit(dq_full);
-        umma_commit(&pds_empty[buf]);                        // P^T / dS^T smem may be overwritten
-        if (it == n_iter - 1) umma_commit(acc_full);
+        // dQ^T = K^T dS (reduction over the 128 keys)
+        product(C::COL_DQT + buf * BWD_BLOCK_Q, dk_mnmaj, 0, mnmaj, d_ds_mn, pds, mnmaj, OverKV{}, p.idesc_dqt, 0u);
+        umma_commit_warp(leader, &dq_full[buf]);
+        if (it == n_iter - 1) umma_commit_warp(leader, acc_full);
+        if (++stage == ST) stage = 0;
       }
     }
     __syncwarp();
     roles_done_wait<BWD_THREADS>();
-    if (lane == 0 && *abort_flag) {                          // nor a product
+    if (leader && *abort_flag) {                             // nor a product
       int none = 0;
       umma_commit(drained);
       wait_or_abort(drained, 0, &none);
@@ -1420,10 +1499,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   } else if (warp < BWD_SOFTMAX_WARP0) {
     // ================================================================ statistics of the query rows (one row per thread)
     const int qr = (warp - BWD_STAT_WARP0) * 32 + lane;
-    for (int it = 0; it < n_iter; ++it) {
-      const int stage = it % ST;
-      const int hq = kv_head * group + it / n_i;
-      const int q_pos = (i_start + it % n_i) * BWD_BLOCK_Q + qr;
+    QueryWalk walk(i_start, q_tiles, kv_head * group);
+    for (int it = 0; it < n_iter; ++it, walk.next()) {
+      const int stage = it % ST, hq = walk.head;
+      const int q_pos = walk.tile * BWD_BLOCK_Q + qr;
       // rows past the end of the sequence read as 0 (their P / dS are forced to 0 by the softmax warps)
       const size_t at = (size_t)(seq_row0 + q_pos) * p.hq + hq;
       const float l = q_pos < len ? __ldg(p.lse + at) : 0.f, d = q_pos < len ? __ldg(p.delta + at) : 0.f;
@@ -1436,9 +1515,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     roles_done<BWD_THREADS>();
   } else if (warp < BWD_DRAIN_WARP0) {
     // ================================================================ softmax warps: two threads per key row
-    constexpr int COLS = BWD_BLOCK_Q / 2;
+    constexpr int PARTS = BWD_SOFTMAX_WARPS / 4, COLS = BWD_BLOCK_Q / PARTS;
     const int quarter = warp & 3;
-    const int half = (warp - BWD_SOFTMAX_WARP0) >> 2;        // this thread's 32 queries of the tile
+    const int part = (warp - BWD_SOFTMAX_WARP0) >> 2;        // this thread's 32 queries of the tile
     const int r = quarter * 32 + lane;                       // key row inside the tile
     const int key_pos = kv_tile * BWD_BLOCK_KV + r;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
@@ -1449,18 +1528,19 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     auto tile = [&](int it, int q_base, auto masked_tag) -> bool {
       constexpr bool MASKED = decltype(masked_tag)::value;
       const int stage = it % ST, buf = it & 1;
-      if (!warp_wait(&stat_full[stage], ring_parity(it))) return false;
       if (!warp_wait(sp_full, (uint32_t)(it & 1))) return false;
       tc_fence_after();
       uint32_t sv[COLS], dpv[COLS];
-      tmem_ld_32x32b_x32(tmem_base + lane_addr + C::COL_ST + half * COLS, sv);
-      tmem_ld_32x32b_x32(tmem_base + lane_addr + C::COL_DPT + half * COLS, dpv);
+      tmem_ld_32x32b_x32(tmem_base + lane_addr + C::COL_ST + part * COLS, sv);
+      tmem_ld_32x32b_x32(tmem_base + lane_addr + C::COL_DPT + part * COLS, dpv);
+      const bool stats = warp_wait(&stat_full[stage], ring_parity(it));
       tmem_ld_wait();
+      if (!stats) return false;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(sp_empty);                  // S^T / dP^T may be overwritten by iteration it+1
-      const ulonglong2* nlse = reinterpret_cast<const ulonglong2*>(smem_stat + stage * 2 * BWD_BLOCK_Q + half * COLS);
-      const ulonglong2* ndel = reinterpret_cast<const ulonglong2*>(smem_stat + stage * 2 * BWD_BLOCK_Q + BWD_BLOCK_Q + half * COLS);
+      const ulonglong2* nlse = reinterpret_cast<const ulonglong2*>(smem_stat + stage * 2 * BWD_BLOCK_Q + part * COLS);
+      const ulonglong2* ndel = reinterpret_cast<const ulonglong2*>(smem_stat + stage * 2 * BWD_BLOCK_Q + BWD_BLOCK_Q + part * COLS);
       const uint64_t mul2 = pack_f32x2(p.scale_log2, p.scale_log2);
       uint32_t p_packed[COLS / 2], ds_packed[COLS / 2];
 #pragma unroll
@@ -1472,13 +1552,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           const uint64_t y = add_f32x2(pack_f32x2(__uint_as_float(dpv[c + e]), __uint_as_float(dpv[c + e + 1])), e ? d4.y : d4.x);
           float p0, p1, d0, d1;
           unpack_f32x2(x, p0, p1);
-          unpack_f32x2(y, d0, d1);
           p0 = fast_exp2(p0);
           p1 = fast_exp2(p1);
-          d0 *= p0;
-          d1 *= p1;
+          unpack_f32x2(mul_f32x2(y, pack_f32x2(p0, p1)), d0, d1);
           if (MASKED) {
-            const int q0 = q_base + half * COLS + c + e;
+            const int q0 = q_base + part * COLS + c + e;
             if (!(key_live && q0 >= q_lo && q0 < len)) p0 = d0 = 0.f;
             if (!(key_live && q0 + 1 >= q_lo && q0 + 1 < len)) p1 = d1 = 0.f;
           }
@@ -1486,15 +1564,12 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           ds_packed[(c + e) >> 1] = pack_16<BF16>(d0, d1);
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&stat_empty[stage]);
-      // the accumulation GEMMs of iteration it-2 must have retired before their smem operands are replaced
-      if (!warp_wait(&pds_empty[buf], (uint32_t)(((it >> 1) & 1) ^ 1))) return false;
+      // the products of iteration it - 2, which read this buffer, have retired: they were issued before S^T of this one
       uint8_t* pt_row = smem_pt + buf * C::PT_BYTES + r * 128;
       uint8_t* dst_row = smem_dst + buf * C::PT_BYTES + r * 128;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {                          // 64 q = 128 bytes = 8 chunks of 16 B, SWIZZLE_128B
-        const int pos = ((half * 4 + i) ^ (r & 7)) * 16;
+      for (int i = 0; i < COLS / 8; ++i) {                   // 64 q = 128 bytes = 8 chunks of 16 B, SWIZZLE_128B
+        const int pos = ((part * (COLS / 8) + i) ^ (r & 7)) * 16;
         *reinterpret_cast<uint4*>(pt_row + pos) =
             make_uint4(p_packed[i * 4], p_packed[i * 4 + 1], p_packed[i * 4 + 2], p_packed[i * 4 + 3]);
         *reinterpret_cast<uint4*>(dst_row + pos) =
@@ -1502,29 +1577,34 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       }
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&pds_full[buf]);
+      if (lane == 0) {
+        mbar_arrive(&pds_full[buf]);
+        mbar_arrive(&stat_empty[stage]);
+      }
       return true;
     };
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const int q_tile = i_start + it % n_i;
+    QueryWalk at(i_start, q_tiles, kv_head * group);
+    for (int it = 0; it < n_iter && ok; ++it, at.next()) {
+      const int q_tile = at.tile;
       const bool masked = (p.causal && (q_tile <= 2 * kv_tile + 1)) ||
                           (ragged && (kv_tile == (len - 1) / BWD_BLOCK_KV || q_tile == q_tiles - 1));
       ok = masked ? tile(it, q_tile * BWD_BLOCK_Q, std::true_type{}) : tile(it, q_tile * BWD_BLOCK_Q, std::false_type{});
     }
-    // ---- epilogue: this key's row of dV (first half of the warps) or scale * dK (second)
+    // ---- epilogue: half of this key's row of dV (first half of the warps) or scale * dK (second)
     if (ok && n_iter > 0) ok = warp_wait(acc_full, 0);
     if (ok) {
       tc_fence_after();
       const size_t row = (size_t)kv_row0 + r;
       const size_t ld = (size_t)p.hkv * D;
-      const uint32_t col0 = half == 0 ? C::COL_DV : C::COL_DK;
-      const float mul = half == 0 ? 1.f : p.scale;
-      float* acc_row = p.dk_acc != nullptr ? (half == 0 ? p.dv_acc : p.dk_acc) + (row * ld + (size_t)kv_head * D) : nullptr;
-      uint8_t* base = reinterpret_cast<uint8_t*>(half == 0 ? p.dv : p.dk) + (row * ld + (size_t)kv_head * D) * 2;
+      const uint32_t col0 = part < PARTS / 2 ? C::COL_DV : C::COL_DK;
+      const int c_begin = part % (PARTS / 2) * (D / (PARTS / 2));
+      const float mul = part < PARTS / 2 ? 1.f : p.scale;
+      float* acc_row = p.dk_acc != nullptr ? (part < PARTS / 2 ? p.dv_acc : p.dk_acc) + (row * ld + (size_t)kv_head * D) : nullptr;
+      uint8_t* base = reinterpret_cast<uint8_t*>(part < PARTS / 2 ? p.dv : p.dk) + (row * ld + (size_t)kv_head * D) * 2;
       // NOTE: tcgen05.ld is warp-collective (.sync.aligned): every lane runs the loads, only the STORES are predicated on
       // the key being inside the sequence (a ragged last tile leaves some lanes of a warp without a row)
 #pragma unroll 1
-      for (int c = 0; c < D; c += 32) {
+      for (int c = c_begin; c < c_begin + D / (PARTS / 2); c += 32) {
         uint32_t v[32];
         __syncwarp();
         tmem_ld_32x32b_x32(tmem_base + lane_addr + col0 + c, v);
@@ -1557,29 +1637,32 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const int dlane = quarter * 32 + lane;                   // d index (row of dQ^T)
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const size_t row_stride = (size_t)p.hq * D;
-    for (int it = 0; it < n_iter; ++it) {
-      const int hq = kv_head * group + it / n_i;
-      const int q_tile = i_start + it % n_i;
-      const int q_row0 = seq_row0 + q_tile * BWD_BLOCK_Q;
-      const int q_live = min(len - q_tile * BWD_BLOCK_Q, BWD_BLOCK_Q);     // rows of this tile that belong to the sequence
-      if (!warp_wait(dq_full, (uint32_t)(it & 1))) break;
+    QueryWalk at(i_start, q_tiles, kv_head * group);
+    for (int it = 0; it < n_iter; ++it, at.next()) {
+      const int q_row0 = seq_row0 + at.tile * BWD_BLOCK_Q, hq = at.head, buf = it & 1;
+      const int q_live = min(len - at.tile * BWD_BLOCK_Q, BWD_BLOCK_Q);    // rows of this tile that belong to the sequence
+      if (!warp_wait(&dq_full[buf], (uint32_t)((it >> 1) & 1))) break;
       tc_fence_after();
-      uint32_t v[BWD_BLOCK_Q];
-      tmem_ld_32x32b_x32(tmem_base + lane_addr + C::COL_DQT, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
-      tmem_ld_32x32b_x32(tmem_base + lane_addr + C::COL_DQT + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dq_empty);                  // dQ^T may be overwritten while the reductions are on their way
       float* dst = p.dq_acc + ((size_t)q_row0 * p.hq + hq) * D + dlane;
-      if (q_live == BWD_BLOCK_Q) {
 #pragma unroll
-        for (int i = 0; i < BWD_BLOCK_Q; ++i)                // one 128-byte coalesced fp32 reduction per warp and row
-          atomicAdd(dst + (size_t)i * row_stride, __uint_as_float(v[i]) * p.scale);
-      } else {
+      for (int c = 0; c < BWD_BLOCK_Q; c += 32) {
+        uint32_t v[32];
+        tmem_ld_32x32b_x32(tmem_base + lane_addr + C::COL_DQT + buf * BWD_BLOCK_Q + c, v);
+        tmem_ld_wait();
+        if (c + 32 == BWD_BLOCK_Q) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&dq_empty[buf]);        // dQ^T may be overwritten while the reductions are on their way
+        }
+        if (q_live == BWD_BLOCK_Q) {
 #pragma unroll
-        for (int i = 0; i < BWD_BLOCK_Q; ++i)
-          if (i < q_live) atomicAdd(dst + (size_t)i * row_stride, __uint_as_float(v[i]) * p.scale);
+          for (int i = 0; i < 32; ++i)                       // one 128-byte coalesced fp32 reduction per warp and row
+            atomicAdd(dst + (size_t)(c + i) * row_stride, __uint_as_float(v[i]) * p.scale);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c + i < q_live) atomicAdd(dst + (size_t)(c + i) * row_stride, __uint_as_float(v[i]) * p.scale);
+        }
       }
     }
     __syncwarp();

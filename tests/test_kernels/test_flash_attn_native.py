@@ -355,3 +355,35 @@ def test_packed_forward_by_number_of_tiles(D, Hq, Hkv, lens, mask):
         torch.testing.assert_close(out[r].float(), ref, atol=2e-2, rtol=2e-2)
         if mask != "window":
             torch.testing.assert_close(lse[r], s.logsumexp(-1).T, atol=1e-3, rtol=1e-3)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Hq,Hkv", [(150, 50), (200, 50)])
+@pytest.mark.parametrize("lens", [[63, 64, 65, 191], [192, 193, 449, 321]])
+@pytest.mark.parametrize("causal", [True, False])
+def test_forward_steps_of_half_a_key_tile(D, Hq, Hkv, lens, causal):
+    """Walks of odd and even numbers of 64-key steps one after the other in a CTA, two tiles of unequal walks, and scores that grow
+    from step to step, so that the accumulator is rescaled in every one of them."""
+    from colossalai_b200.ops import flash_attn_native as fa
+
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    T = sum(lens)
+    q, k, v = (torch.randn(T, h, D, device="cuda", generator=g) for h in (Hq, Hkv, Hkv))
+    pos = torch.cat([torch.arange(n, device="cuda") for n in lens])
+    q[..., 0] = 8.0
+    k[..., 0] = (pos // 32 * 14.0 * D ** 0.5 / 64).unsqueeze(1)                # a score grows by 14 (in base 2: 20) every 256 keys ..
+    k[..., 0] += (pos // 64 * 12.0 * D ** 0.5 / 8).unsqueeze(1)                # .. and by 12 (17) every 64
+    q, k, v = (t.bfloat16() for t in (q, k, v))
+    cu = torch.tensor([0] + lens, device="cuda").cumsum(0).to(torch.int32)
+    out, lse = fa.flash_fwd(q, k, v, 1, causal, None, cu_seqlens=cu)
+    a = 0
+    for n in lens:
+        kk, vv = (x[a:a + n].double().repeat_interleave(Hq // Hkv, 1) for x in (k, v))
+        s = torch.einsum("qhd,khd->hqk", q[a:a + n].double(), kk) * D ** -0.5
+        if causal:
+            s = s.masked_fill(~torch.ones(n, n, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+        ref = torch.einsum("hqk,khd->qhd", s.softmax(-1), vv)
+        # weights rounded to bf16 (2^-9 each), the result once more; scores up to 100 in fp32
+        assert (out[a:a + n].double() - ref).norm() <= 6e-3 * ref.norm()
+        torch.testing.assert_close(lse[a:a + n].double(), s.logsumexp(-1).t(), atol=2e-3, rtol=1e-4)
+        a += n
