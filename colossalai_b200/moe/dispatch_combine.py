@@ -49,7 +49,7 @@ def _use_fused(x: torch.Tensor, num_experts: int, ep_group) -> bool:
 
 
 def _aligned_rows(x: torch.Tensor) -> bool:
-    """Lay the expert-grouped rows out with every expert's range padded to 128 rows (zero rows): the native grouped
+    """Lay the expert-grouped rows out with every expert's range padded to 16 rows (zero rows): the native grouped
     weight-gradient GEMM then needs no re-layout pass (moe/grouped_gemm.py)."""
     return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
             and os.environ.get("CB200_GROUPED_GEMM", "native") == "native"

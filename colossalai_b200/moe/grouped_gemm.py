@@ -2,8 +2,8 @@
 
 CUDA path: our tcgen05 grouped GEMM (`kernel/csrc/grouped_gemm_tcgen05.cu`) - ONE persistent launch per GEMM walks a tile
 list built on the device from the per-expert row counts (no host sync, no per-expert launches, no padding for the
-forward / dgrad; the weight-gradient GEMM reduces over each expert's token rows and wants the row ranges aligned to the
-128-row k-block, which `_pad_groups` arranges on the device when the caller's layout is not aligned already).
+forward / dgrad; the weight-gradient GEMM reduces over each expert's token rows and wants the row ranges aligned to
+16 rows, which `_pad_groups` arranges on the device when the caller's layout is not aligned already).
 `CB200_GROUPED_GEMM=lib` selects `torch._grouped_mm` (library) instead; CPU tensors take a per-expert loop.
 Replaces the reference's python loop over local experts (`shardformer/modeling/mixtral.py:177-191`).
 """
@@ -16,7 +16,8 @@ from typing import Optional, Tuple
 import torch
 
 _lib = None
-ALIGN = 128           # k-block of the wgrad kernel: group row ranges must start / end on multiples of it
+ALIGN = 16            # reduction of one instruction of the wgrad kernel: group row ranges must start / end on multiples of it
+K_BLOCK = 128         # the input-gradient GEMM reads an expert's weight in blocks of rows that it must not share with the next
 
 
 def _get_lib():
@@ -105,7 +106,7 @@ class _GroupedLinearNative(torch.autograd.Function):
         dy = dy.contiguous()
         dx = dw = None
         if ctx.needs_input_grad[0]:
-            if w.shape[1] % ALIGN == 0:
+            if w.shape[1] % K_BLOCK == 0:
                 dx = _native_fwd(dy, w, offs, False)         # dX = dY @ W[e]  (W [E, O, K] read as [E, K_red = O, N = K])
             else:
                 dx = torch._grouped_mm(dy, w, offs=offs) if hasattr(torch, "_grouped_mm") else None
@@ -152,7 +153,7 @@ class _GroupedLinear(torch.autograd.Function):
 
 def grouped_linear(x: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, aligned: bool = False) -> torch.Tensor:
     """y[rows of expert e] = x[rows of expert e] @ w[e]^T.  `aligned`: the caller guarantees that every expert's row
-    range starts and ends on a multiple of 128 (zero rows as padding) - the weight-gradient GEMM then runs without the
+    range starts and ends on a multiple of 16 (zero rows as padding) - the weight-gradient GEMM then runs without the
     re-layout pass."""
     if native_ok(x, w):
         return _GroupedLinearNative.apply(x, w, counts, aligned or getattr(counts, "cb200_aligned", False))

@@ -87,3 +87,30 @@ def test_grouped_gemm_counts_stay_on_device():
             torch.cuda.set_sync_debug_mode("default")
     torch.cuda.synchronize()
     torch.testing.assert_close(y.float(), _ref(x, w, c), atol=0.5, rtol=2e-2)
+
+
+@pytest.mark.parametrize("counts,K,N", [([16, 0, 256, 272, 496, 512, 528, 16], 256, 384), ([48] * 40 + [144], 128, 264), ([4880], 72, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_groups_of_sixteen_rows(counts, K, N, dtype):
+    """Groups on and beside the edges of one, two and many row tiles (up to 256 rows, multiples of 16), of a 32- and a 64-row box and of a
+    k-block; output widths that end inside a tile.  Rows behind the last group belong to nobody."""
+    from colossalai_b200.moe import grouped_gemm as gg
+
+    g = torch.Generator(device="cuda").manual_seed(len(counts))
+    c = torch.tensor(counts, device="cuda")
+    rows, E = int(sum(counts)), len(counts)
+    x, dy = (torch.randn(rows + 40, n, device="cuda", generator=g).to(dtype) for n in (K, N))
+    w = (torch.randn(E, N, K, device="cuda", generator=g) * K ** -0.5).to(dtype)
+    offs = gg._offs(c, x.device)
+    y = gg._native_fwd(x, w, offs, True)
+    dw = gg._native_wgrad(dy, x, offs, E, dtype)
+    dw32 = gg._native_wgrad(dy, x, offs, E, torch.float32)
+    dx = gg._native_fwd(dy, w, offs, False) if N % gg.K_BLOCK == 0 else None
+    eps = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)                # half a unit of the results' rounding, and fp32 sums
+    s = 0
+    for e, n in enumerate(counts):
+        xe, de, we = x[s:s + n].double(), dy[s:s + n].double(), w[e].double()
+        for got, ref in ((y[s:s + n], xe @ we.t()), (dw[e], de.t() @ xe)) + (((dx[s:s + n], de @ we),) if dx is not None else ()):
+            assert ref.numel() == 0 or (got.double() - ref).abs().max() <= eps * ref.abs().max()
+        assert (dw32[e].double() - de.t() @ xe).norm() <= 1e-5 * (de.t() @ xe).norm()
+        s += n
