@@ -28,8 +28,17 @@ class CUDAGraphRunner:
         torch.cuda.synchronize()
 
     def forward(self, **tensors: torch.Tensor) -> torch.Tensor:
+        # the small inputs of a step of one type in one launch (six copies of their own 11 us); others one by one
+        alike = {}
         for k, v in tensors.items():
-            self.static_inputs[k].copy_(v, non_blocking=True)
+            dst = self.static_inputs[k]
+            if v.device == dst.device and v.dtype == dst.dtype and v.shape == dst.shape and v.is_contiguous() and dst.is_contiguous():
+                alike.setdefault(dst.dtype, ([], []))[0].append(dst)
+                alike[dst.dtype][1].append(v)
+            else:
+                dst.copy_(v, non_blocking=True)
+        for dst, src in alike.values():
+            torch._foreach_copy_(dst, src, non_blocking=True)
         self.graph.replay()
         return self.static_output
 

@@ -100,6 +100,29 @@ CB_DEVICE float block_max(float v, float* smem) {
   return warp_max(x);
 }
 
+// A kernel that takes its place while the one before it in the stream still runs, instead of some microseconds after its end: the
+// launch says so, and the kernel begins with `cb_early_start`, which lets the next one do the same and then waits until everything
+// before it is complete and visible.  Nothing global is read or written ahead of it, so the order is that of an ordinary launch.
+// For the kernels of a decode step, eleven a layer one after the other (16 sequences, 4 layers, library GEMMs: 553 -> 527 us).
+CB_DEVICE void cb_early_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+static inline int cb_launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 static inline int cb_num_sms() {
   static int n = 0;
   if (n == 0) {

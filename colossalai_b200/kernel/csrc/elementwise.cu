@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(GLU_THREADS) glu_fwd_kernel(const T* __restric
                                                               int blocks_per_row, int rows_per_block, int I,
                                                               const int64_t* __restrict__ row_limit) {
   constexpr int VEC = Vec16<T>::N;
+  cb_early_start();
   GluPart p;
   if (!glu_part<VEC, NARROW>(p, rows, blocks_per_row, rows_per_block, I, row_limit)) return;
   const T* gr = gu + p.row * 2 * I;
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(NARROW ? ROPE_BLOCK : 512) rope_kernel(const T
                                                    int64_t src_stride, int width, int n_rot_heads, int D, int rot_dim,
                                                    float sign, int interleaved) {
   constexpr int VEC = Vec16<T>::N;
+  cb_early_start();
   const int half = rot_dim / 2;
   const int vec_per_head = half / VEC;                       // rotated items of a head
   const int n_rot = n_rot_heads * vec_per_head;
@@ -279,7 +281,7 @@ static inline int ew_grid(int64_t items, int block) {
 
 extern "C" {
 
-#define GLU_LAUNCH(KERNEL, ...)                                                                                         \
+#define GLU_LAUNCH(LAUNCH, KERNEL, ...)                                                                                 \
   CB_DISPATCH_FLOAT(dtype, T, {                                                                                         \
     const int vecs = I / Vec16<T>::N, per = GLU_THREADS * GLU_ITEMS, bpr = (vecs + per - 1) / per;                      \
     const int rpb = vecs <= GLU_NARROW ? GLU_THREADS / ((vecs + GLU_ITEMS - 1) / GLU_ITEMS) : 1;                        \
@@ -289,21 +291,25 @@ extern "C" {
     const int block = rpb > 1 ? GLU_THREADS : ((part + GLU_ITEMS - 1) / GLU_ITEMS + 31) / 32 * 32;                      \
     auto kern = rpb > 1 ? (act == 0 ? KERNEL<T, 0, true> : act == 1 ? KERNEL<T, 1, true> : KERNEL<T, 2, true>)            \
                         : (act == 0 ? KERNEL<T, 0, false> : act == 1 ? KERNEL<T, 1, false> : KERNEL<T, 2, false>);        \
-    kern<<<(unsigned)blocks, block, 0, s>>>(__VA_ARGS__, rows, bpr, rpb, I, row_limit);                                  \
+    LAUNCH((unsigned)blocks, block, __VA_ARGS__, rows, bpr, rpb, I, row_limit);                                          \
   })
 
 int cb_glu_fwd_bounded(const void* gu, void* out, int64_t rows, int I, int act, int dtype, const int64_t* row_limit, cudaStream_t s) {
   if (rows == 0 || I == 0) return 0;
-  GLU_LAUNCH(glu_fwd_kernel, (const T*)gu, (T*)out);
+#define EARLY(GRID, BLOCK, ...) if (const int e = cb_launch_early(kern, GRID, BLOCK, 0, s, __VA_ARGS__)) return e
+  GLU_LAUNCH(EARLY, glu_fwd_kernel, (const T*)gu, (T*)out);
+#undef EARLY
   return CB_LAUNCH_CHECK();
 }
 
 int cb_glu_bwd_bounded(const void* dout, const void* gu, void* dgu, int64_t rows, int I, int act, int dtype,
                        const int64_t* row_limit, cudaStream_t s) {
   if (rows == 0 || I == 0) return 0;
-  GLU_LAUNCH(glu_bwd_kernel, (const T*)dout, (const T*)gu, (T*)dgu);
+#define PLAIN(GRID, BLOCK, ...) kern<<<GRID, BLOCK, 0, s>>>(__VA_ARGS__)
+  GLU_LAUNCH(PLAIN, glu_bwd_kernel, (const T*)dout, (const T*)gu, (T*)dgu);
   return CB_LAUNCH_CHECK();
 }
+#undef PLAIN
 #undef GLU_LAUNCH
 
 int cb_glu_fwd(const void* gu, void* out, int64_t rows, int I, int act, int dtype, cudaStream_t s) {
@@ -328,8 +334,8 @@ int cb_rope(const void* src, void* dst, const int64_t* pos, const float* cos_c, 
     const unsigned grid = (unsigned)((tokens + per_block - 1) / per_block);
     auto kern = per_block > 1 ? (vec_table ? rope_kernel<T, true, true> : rope_kernel<T, false, true>)
                               : (vec_table ? rope_kernel<T, true, false> : rope_kernel<T, false, false>);
-    kern<<<grid, block, 0, s>>>((const T*)src, (T*)dst, pos, cos_c, sin_c, tokens, per_block, src_stride, width, n_rot_heads, D, rot_dim,
-                                sign, interleaved);
+    return cb_launch_early(kern, grid, block, 0, s, (const T*)src, (T*)dst, pos, cos_c, sin_c, tokens, per_block, src_stride, width,
+                           n_rot_heads, D, rot_dim, sign, interleaved);
   });
   return CB_LAUNCH_CHECK();
 }

@@ -62,6 +62,8 @@ struct Launchers {
                           float, int, cudaStream_t);
   int (*flash_bwd)(const void*, const void*, const void*, const void*, const void*, const float*, void*, void*, void*, float*,
                    float*, int, int, int, int, int, int, float, int, const int*, long long, cudaStream_t);
+  int (*gemm_rows)(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, cudaStream_t);
+  int (*embed_rows)(const int64_t*, const void*, void*, int64_t, int64_t, int64_t, cudaStream_t);
   int (*decode_splits)(int, int, int, int*);
   int (*decode)(const void*, const void*, const void*, const int*, const int*, void*, float*, float*, int, int, int, int, int, int,
                 int, int, float, const float*, int64_t, int64_t, int, int, cudaStream_t);
@@ -74,9 +76,9 @@ struct Count {
 };
 Count n_norm_fwd{"rmsnorm_fwd"}, n_norm_bwd{"rmsnorm_bwd"}, n_glu_fwd{"glu_fwd"}, n_glu_bwd{"glu_bwd"}, n_rope{"rope"},
     n_stats{"ce_row_stats"}, n_loss{"ce_loss"}, n_grad{"ce_softmax_grad"}, n_flash_fwd{"flash_attn_varlen_fwd"},
-    n_flash_bwd{"flash_attn_bwd"}, n_decode{"paged_decode_attention"};
+    n_flash_bwd{"flash_attn_bwd"}, n_decode{"paged_decode_attention"}, n_rows{"gemm_rows"}, n_embed{"embed_rows"};
 Count* const COUNTS[] = {&n_norm_fwd, &n_norm_bwd, &n_glu_fwd, &n_glu_bwd, &n_rope, &n_stats, &n_loss, &n_grad, &n_flash_fwd, &n_flash_bwd,
-                         &n_decode};
+                         &n_decode, &n_rows, &n_embed};
 
 void launched(int rc, Count& c, int n = 1) {
   TORCH_CHECK(rc != cudaErrorLaunchTimeout, c.name, ": a wait inside an earlier attention kernel ran out; what it wrote is not valid (CUDA error ",
@@ -283,6 +285,28 @@ Tensor paged_decode(const Tensor& q, const Tensor& kc, const Tensor& vc, const T
   return out;
 }
 
+// ------------------------------------------------------------------------------------------------ a step's projections and lookup
+// x [M, K], w [N, K], residual [M, N] or none; the caller has checked types, strides and alignment
+Tensor linear_rows(const Tensor& x, const Tensor& w, const OptTensor& residual) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int M = (int)x.size(0), K = (int)x.size(1), N = (int)w.size(0);
+  const bool add = residual.has_value() && residual->defined();
+  Tensor y = at::empty({M, N}, x.options());
+  launched(L.gemm_rows(ptr(x), ptr(w), mut(y), add ? ptr(*residual) : nullptr, M, N, K, x.stride(0), N, add ? residual->stride(0) : 0,
+                       code_of(x), stream_of(x)),
+           n_rows);
+  return y;
+}
+// ids [n] int64, table [entries, H]
+Tensor embed_rows(const Tensor& ids, const Tensor& table) {
+  const c10::cuda::CUDAGuard guard(ids.device());
+  Tensor out = at::empty({ids.size(0), table.size(1)}, table.options());
+  launched(L.embed_rows(as<int64_t>(ids), ptr(table), mut(out), ids.size(0), table.size(0), table.size(1) * table.element_size(),
+                        stream_of(ids)),
+           n_embed);
+  return out;
+}
+
 template <typename F> void take(const std::map<std::string, uint64_t>& table, const char* name, F& slot) {
   const auto it = table.find(name);
   TORCH_CHECK(it != table.end() && it->second != 0, "launcher ", name, " is missing");
@@ -302,6 +326,8 @@ void bind(const std::map<std::string, uint64_t>& t) {
   take(t, "cb_ce_softmax_grad", L.softmax_grad);
   take(t, "cb_flash_attn_varlen_fwd", L.flash_varlen_fwd);
   take(t, "cb_flash_attn_bwd", L.flash_bwd);
+  take(t, "cb_gemm_rows", L.gemm_rows);
+  take(t, "cb_embed_rows", L.embed_rows);
   take(t, "cb_decode_num_splits", L.decode_splits);
   take(t, "cb_paged_decode_attention", L.decode);
 }
@@ -344,4 +370,6 @@ PYBIND11_MODULE(cb200_host, m) {
         },
         release());
   m.def("paged_decode", &paged_decode, release());
+  m.def("linear_rows", &linear_rows, release());
+  m.def("embed_rows", &embed_rows, release());
 }

@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(256) kv_cache_write_vec_kernel(const T* __rest
                                                                  int vec_per_tok, int block_size, int max_blocks_per_seq,
                                                                  int64_t k_stride, int64_t v_stride) {
   // vec_per_tok = kv_heads * D / 8 (16-bit elements); work items = tokens * 2 (K, V) * vec_per_tok
+  cb_early_start();
   const int64_t total = (int64_t)tokens * 2 * vec_per_tok;
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (int64_t)gridDim.x * blockDim.x) {
     const int t = (int)(w / (2 * vec_per_tok));
@@ -453,7 +454,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.y * (blockDim.x >> 5) + warp;
   if (kvh >= Hkv) return;                       // (no block-wide barrier in this kernel)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  cb_early_start();
   const int len = seq_lens[seq];
   const int window_start = window > 0 ? max(0, len - window) : 0;
   const int t0 = max(split * part_len, window_start);
@@ -604,6 +605,7 @@ template <typename T, int D>
 __global__ void __launch_bounds__(128) decode_reduce_kernel(const float* __restrict__ o_part,
                                                             const float* __restrict__ ml_part, T* __restrict__ out,
                                                             int Hq, int splits, int64_t out_stride) {
+  cb_early_start();
   const int seq = blockIdx.x, h = blockIdx.y;
   const int64_t base = ((int64_t)seq * Hq + h) * splits;
   float gm = -INFINITY;
@@ -630,8 +632,7 @@ __global__ void __launch_bounds__(128) decode_reduce_kernel(const float* __restr
 // partial results are on their way to a thread at a time, where the kernel above waits for each in turn (65 partitions of one
 // sequence of 4097 tokens: the call on the device 16.2 us, 13.9 so).  With fewer of them it is no faster (16 x 2048 tokens, 64 / 8 heads, 19
 // partitions 30 us, 33 so) and with many sequences slower (1024 of 64 tokens 78 us, 89 so).
-// Sums in the same order with the same roundings.  Launched while the kernel before it runs,
-// it takes its place on the SMs and waits there.
+// Sums in the same order with the same roundings.
 constexpr int DEC_WIDE = 48, DEC_AHEAD = 16, DEC_WIDE_THREADS = 128;
 template <typename T, int D>
 __global__ void __launch_bounds__(DEC_WIDE_THREADS) decode_reduce_wide_kernel(const float* __restrict__ o_part,
@@ -644,7 +645,7 @@ __global__ void __launch_bounds__(DEC_WIDE_THREADS) decode_reduce_wide_kernel(co
   const int seq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int64_t base = ((int64_t)seq * Hq + h) * splits;
   const float2* ml = reinterpret_cast<const float2*>(ml_part) + base;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  cb_early_start();
   float gm = -INFINITY;
   for (int s = tid; s < splits; s += DEC_WIDE_THREADS) gm = fmaxf(gm, ml[s].x);
   gm = warp_max(gm);
@@ -697,20 +698,9 @@ __global__ void __launch_bounds__(DEC_WIDE_THREADS) decode_reduce_wide_kernel(co
 template <typename T, int D>
 int launch_decode_reduce(const float* o_part, const float* ml_part, T* out, int num_seqs, int Hq, int splits, int64_t out_stride,
                          cudaStream_t s) {
-  if (splits < DEC_WIDE) {
-    decode_reduce_kernel<T, D><<<dim3(num_seqs, Hq), 128, 0, s>>>(o_part, ml_part, out, Hq, splits, out_stride);
-    return CB_LAUNCH_CHECK();
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(num_seqs, Hq);
-  cfg.blockDim = dim3(DEC_WIDE_THREADS);
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, decode_reduce_wide_kernel<T, D>, o_part, ml_part, out, Hq, splits, out_stride);
+  auto kernel = splits < DEC_WIDE ? decode_reduce_kernel<T, D> : decode_reduce_wide_kernel<T, D>;
+  static_assert(DEC_WIDE_THREADS == 128, "the block of both");
+  return cb_launch_early(kernel, dim3(num_seqs, Hq), DEC_WIDE_THREADS, 0, s, o_part, ml_part, out, Hq, splits, out_stride);
 }
 
 __global__ void gather_cos_sin_kernel(const float* __restrict__ cos_c, const float* __restrict__ sin_c,
@@ -744,9 +734,8 @@ int cb_kv_cache_write(const void* k, const void* v, void* k_cache, void* v_cache
     const int64_t total = (int64_t)tokens * 2 * (n / 8);
     const int grid = (int)((total + 255) / 256 < 16 * cb_num_sms() ? (total + 255) / 256 : 16 * cb_num_sms());
     CB_DISPATCH_HALF(dtype, T, {
-      kv_cache_write_vec_kernel<T><<<grid, 256, 0, s>>>((const T*)k, (const T*)v, (T*)k_cache, (T*)v_cache, block_tables,
-                                                       token_seq, token_pos, tokens, n / 8, block_size,
-                                                       max_blocks_per_seq, k_stride, v_stride);
+      return cb_launch_early(kv_cache_write_vec_kernel<T>, grid, 256, 0, s, (const T*)k, (const T*)v, (T*)k_cache, (T*)v_cache,
+                             block_tables, token_seq, token_pos, tokens, n / 8, block_size, max_blocks_per_seq, k_stride, v_stride);
     });
     return CB_LAUNCH_CHECK();
   }
@@ -830,9 +819,9 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
                            (DEC_THREADS / 32) * per_warp);                                                           \
       attr_done = true;                                                                                              \
     }                                                                                                                \
-    paged_decode_mma_kernel<T, DD><<<mma_grid, mma_warps * 32, mma_warps * per_warp, s>>>(                           \
+    if (const int e = cb_launch_early(paged_decode_mma_kernel<T, DD>, mma_grid, mma_warps * 32, mma_warps * per_warp, s, \
         (const T*)q, (const T*)k_cache, (const T*)v_cache, block_tables, seq_lens, o_part, ml_part, Hq, Hkv,        \
-        block_size, max_blocks_per_seq, splits, part_len, scale, alibi_slopes, q_stride, window);                   \
+        block_size, max_blocks_per_seq, splits, part_len, scale, alibi_slopes, q_stride, window)) return e;         \
     if (const int e = launch_decode_reduce<T, DD>(o_part, ml_part, (T*)out, num_seqs, Hq, splits, out_stride, s)) return e; \
   }
 #define LAUNCH_DEC(T, DD)                                                                                           \

@@ -16,6 +16,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_fwd_kernel(const T* __restrict__
                                                            int rows, int H, float eps) {
   constexpr int VEC = Vec16<T>::N;
   __shared__ float red[64];
+  cb_early_start();
   const int row = blockIdx.x;
   if (row >= rows) return;
   const size_t base = (size_t)row * H;
@@ -316,12 +317,9 @@ int cb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, void* y, vo
     const int block = pick_block(H, Vec16<T>::N);
     const int iters = pick_iters(H, Vec16<T>::N, block);
     CB_DISPATCH_ITERS(iters, IT, {
-      if (res_in)
-        rmsnorm_fwd_kernel<T, true, IT><<<rows, block, 0, stream>>>((const T*)x, (const T*)res_in, (const T*)w,
-                                                                   (T*)y, (T*)res_out, rstd, rows, H, eps);
-      else
-        rmsnorm_fwd_kernel<T, false, IT><<<rows, block, 0, stream>>>((const T*)x, nullptr, (const T*)w, (T*)y,
-                                                                    nullptr, rstd, rows, H, eps);
+      auto kernel = res_in ? rmsnorm_fwd_kernel<T, true, IT> : rmsnorm_fwd_kernel<T, false, IT>;
+      return cb_launch_early(kernel, rows, block, 0, stream, (const T*)x, (const T*)res_in, (const T*)w, (T*)y,
+                             res_in ? (T*)res_out : nullptr, rstd, rows, H, eps);
     });
   });
   return CB_LAUNCH_CHECK();

@@ -47,6 +47,7 @@ LIBS: Dict[str, dict] = {
     "cb200_softmax": {"sources": ["softmax.cu"], "kind": "cuda"},
     "cb200_loss": {"sources": ["cross_entropy.cu"], "kind": "cuda"},
     "cb200_gemm": {"sources": ["gemm_tcgen05.cu"], "kind": "cuda"},
+    "cb200_gemm_rows": {"sources": ["gemm_rows_tcgen05.cu"], "kind": "cuda"},
     "cb200_grouped_gemm": {"sources": ["grouped_gemm_tcgen05.cu"], "kind": "cuda"},
     "cb200_attn": {"sources": ["flash_attn_tcgen05.cu"], "kind": "cuda"},
     "cb200_comm": {"sources": ["fused_comm_gemm.cu"], "kind": "cuda"},
@@ -207,6 +208,7 @@ _HOST_CALLS = {
     "cb200_loss": ["cb_ce_row_stats", "cb_ce_loss_blocks", "cb_ce_loss", "cb_ce_softmax_grad"],
     "cb200_attn": ["cb_flash_attn_varlen_fwd", "cb_flash_attn_bwd"],
     "cb200_infer": ["cb_decode_num_splits", "cb_paged_decode_attention"],
+    "cb200_gemm_rows": ["cb_gemm_rows", "cb_embed_rows"],
 }
 _host, _host_asked = None, False
 

@@ -139,7 +139,7 @@ class Attention(nn.Module):
                 kv_cache=None) -> torch.Tensor:
         cfg, sc = self.cfg, self.shard_config
         D = self.head_dim
-        qkv = self.qkv_proj(x)                                  # [T*, (hq + 2 hkv) * D] local heads
+        qkv = ops.linear_rows(self.qkv_proj, x)                 # [T*, (hq + 2 hkv) * D] local heads
         hq = self.num_heads
         hkv = self.num_kv_heads
         sp_mode = sc.sp_mode if sc is not None else None
@@ -210,7 +210,7 @@ class Attention(nn.Module):
             else:
                 o = all_to_all_comm(o.reshape(B, S, hq, D), sp_group, scatter_dim=1, gather_dim=2)
                 o = o.reshape(B * (S // sp), hq * sp * D)
-        return self.o_proj(o)
+        return ops.linear_rows(self.o_proj, o)
 
     def _head_norm(self, norm: nn.Module, t: torch.Tensor) -> torch.Tensor:
         """Per-head q/k RMSNorm.  Its [head_dim] weight is replicated over TP while every rank only sees its own
@@ -364,7 +364,8 @@ class MLP(nn.Module):
             self._coef32 = {}
         return super()._apply(fn, *a, **k)
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """With `residual` it is added to the result."""
         if self.act == "polynorm":
             key = str(x.device)
             if key not in self._coef32:                   # the four numbers in fp32 on the device, built once
@@ -373,7 +374,7 @@ class MLP(nn.Module):
         elif self.act == "clamped":
             h = ops.clamped_glu(self.gate_up_proj(x), self.limit)
         elif self.cfg.glu:
-            h = ops.glu(self.gate_up_proj(x), self.cfg.hidden_act)
+            h = ops.glu(ops.linear_rows(self.gate_up_proj, x), self.cfg.hidden_act)
         else:
             up = self.up_proj
             if x.is_cuda and x.dtype != torch.float32 and not torch.is_grad_enabled() and up.bias is None \
@@ -385,7 +386,7 @@ class MLP(nn.Module):
                 h = ops.bias_act(y, b, self.cfg.hidden_act)
             else:
                 h = ops.get_activation(self.cfg.hidden_act)(up(x))
-        return self.down_proj(h)
+        return ops.linear_rows(self.down_proj, h, residual)
 
 
 class DecoderLayer(nn.Module):
@@ -458,6 +459,8 @@ class DecoderLayer(nn.Module):
         else:
             x = x + a
             h = self.post_attention_layernorm(x)
+        if type(self.mlp) is MLP and not torch.is_grad_enabled() and ops.unwatched(self.mlp):
+            return self.mlp(h, residual=x)
         return x + self.mlp(h)
 
 
@@ -594,7 +597,7 @@ class TransformerModel(nn.Module):
               token_type_ids: Optional[torch.Tensor] = None,
               inputs_embeds: Optional[torch.Tensor] = None) -> torch.Tensor:
         cfg = self.cfg
-        x = inputs_embeds if inputs_embeds is not None else self.embed_tokens(input_ids)
+        x = inputs_embeds if inputs_embeds is not None else ops.embed_rows(self.embed_tokens, input_ids)
         if cfg.fp32_residual:
             x = x.float()
         if cfg.embed_scale != 1.0:
@@ -852,7 +855,7 @@ class TransformerLMHeadModel(nn.Module):
             # the head's fp32 accumulator is kept (no 16-bit rounding in front of the soft cap's tanh / of the logits)
             logits = torch.mm(h, self.lm_head.weight.t(), out_dtype=torch.float32)
         else:
-            logits = self.lm_head(h)
+            logits = ops.linear_rows(self.lm_head, h)
         if cfg.logit_softcap:
             logits = logits.float()
         if cfg.logit_scale != 1.0:

@@ -1,0 +1,72 @@
+"""Projections of a few token rows: what a decode step spends most of its time on.
+
+A plain `torch.nn.Linear` without bias on up to ROWS_MAX 16-bit rows, outside autograd, runs on the framework's own kernel
+(`kernel/csrc/gemm_rows_tcgen05.cu`: weights streamed once, fp32 sums, residual added before the rounding); every other call is
+the module's own.
+"""
+from __future__ import annotations
+
+import functools
+from typing import Optional
+
+import torch
+from torch import nn
+from torch.nn.modules import module as _module
+
+from ..kernel import loader
+from ._dispatch import plain_call, use_native
+
+__all__ = ["linear_rows", "embed_rows", "unwatched", "ROWS_MAX"]
+
+ROWS_MAX = 32         # what the kernel takes; figures there
+
+
+def unwatched(m: nn.Module) -> bool:
+    """No hook sees a call of the module."""
+    return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                or _module._global_forward_hooks or _module._global_forward_pre_hooks
+                or _module._global_backward_hooks or _module._global_backward_pre_hooks)
+
+
+@functools.lru_cache(maxsize=None)
+def _sm100(device: torch.device) -> bool:
+    return torch.cuda.get_device_capability(device)[0] == 10
+
+
+def _native(linear: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor]) -> bool:
+    if type(linear) is not nn.Linear or torch.is_grad_enabled() or not x.is_cuda or x.dim() != 2 or not 0 < x.shape[0] <= ROWS_MAX:
+        return False
+    w = linear.weight
+    if linear.bias is not None or w.dtype != x.dtype or x.dtype not in (torch.bfloat16, torch.float16) or w.device != x.device:
+        return False
+    n, k = w.shape
+    # one contiguous weight, rows that TMA can address
+    if x.shape[1] != k or k % 8 or k == 0 or n == 0 or not w.is_contiguous() or x.stride(1) != 1 or x.stride(0) % 8 or x.stride(0) < k \
+            or (x.data_ptr() | w.data_ptr()) % 16:
+        return False
+    if residual is not None and (residual.shape != (x.shape[0], n) or residual.dtype != x.dtype or residual.device != x.device
+                                 or residual.stride(1) != 1):
+        return False
+    return (use_native(x) and unwatched(linear) and plain_call(x, w, residual) and not torch.is_autocast_enabled("cuda")
+            and _sm100(x.device))
+
+
+def linear_rows(linear: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """linear(x), plus `residual` if there is one."""
+    if _native(linear, x, residual) and (host := loader.host()) is not None:
+        return host.linear_rows(x, linear.weight, residual)
+    y = linear(x)
+    return y if residual is None else residual + y
+
+
+def embed_rows(embedding: nn.Module, ids: torch.Tensor) -> torch.Tensor:
+    """embedding(ids).  Outside autograd the rows of a plain table come through a kernel with a block per id (16 rows of 4096: 2.6 us,
+    torch's index kernel 14); an id outside the table gives NaN."""
+    w = getattr(embedding, "weight", None)
+    if (type(embedding) is nn.Embedding and embedding.max_norm is None and not torch.is_grad_enabled() and ids.is_cuda and ids.dim() == 1
+            and ids.dtype == torch.int64 and ids.is_contiguous() and ids.numel() > 0 and w.device == ids.device
+            and w.dtype in (torch.bfloat16, torch.float16, torch.float32) and w.is_contiguous()
+            and w.shape[1] * w.element_size() % 16 == 0 and w.shape[1] > 0 and w.data_ptr() % 16 == 0 and use_native(ids)
+            and unwatched(embedding) and plain_call(ids, w) and (host := loader.host()) is not None):
+        return host.embed_rows(ids, w)
+    return embedding(ids)

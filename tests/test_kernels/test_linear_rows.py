@@ -1,0 +1,95 @@
+"""Projections of a few rows and the embedding lookup of a decode step, against 64-bit products of the same 16-bit numbers."""
+import pytest
+import torch
+from torch import nn
+
+SIZES = [(8, 8), (128, 64), (136, 200), (264, 1096), (1000, 2048), (6144, 1024), (18944, 256), (512, 14336)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 32])
+@pytest.mark.parametrize("N,K", SIZES)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_rows_match_64_bits(rows, N, K, dtype):
+    """Widths and depths that end inside a tile and a k-block, every number of splits of the reduction, with a residual and from
+    rows that are a part of wider ones.  A row's bits do not depend on how many rows there are."""
+    from colossalai_b200 import ops
+    from colossalai_b200.kernel import launch_counter
+
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    lin = nn.Linear(K, N, bias=False, device="cuda", dtype=dtype)
+    wide = torch.randn(rows, K + 24, device="cuda", generator=g).to(dtype)
+    x = wide[:, 8:8 + K]
+    res = torch.randn(rows, N, device="cuda", generator=g).to(dtype)
+    ref = x.double() @ lin.weight.detach().double().t()
+    # half a unit of the result's rounding, and fp32 sums of K products
+    unit = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    slack = 1e-6 * (x.double().abs() @ lin.weight.detach().double().abs().t()) + 1e-7
+    with torch.no_grad():
+        before = launch_counter.by_name.get("gemm_rows", 0)
+        y, z = ops.linear_rows(lin, x), ops.linear_rows(lin, x, res)
+        alone = ops.linear_rows(lin, x[rows - 1:])
+    assert launch_counter.by_name["gemm_rows"] == before + 3
+    assert ((y.double() - ref).abs() <= unit * 1.01 * ref.abs() + slack).all()
+    assert ((z.double() - (ref + res.double())).abs() <= unit * 1.01 * (ref + res.double()).abs() + slack).all()
+    assert torch.equal(alone[0], y[-1])
+
+
+@pytest.mark.gpu
+def test_calls_that_stay_with_the_module():
+    """Autograd, hooks, a bias, many rows, other types and subclasses, rows that TMA cannot address: the module's own result."""
+    from colossalai_b200.ops import linear as L
+
+    lin = nn.Linear(64, 32, bias=False, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(4, 64, device="cuda").bfloat16()
+    assert not L._native(lin, x, None)                                       # gradients on
+    with torch.no_grad():
+        assert L._native(lin, x, None) and L._native(lin, x, torch.zeros(4, 32, device="cuda", dtype=torch.bfloat16))
+        assert not L._native(lin, x, torch.zeros(4, 32, device="cuda"))
+        assert not L._native(nn.Linear(64, 32, device="cuda", dtype=torch.bfloat16), x, None)
+        assert not L._native(lin, x.float(), None) and not L._native(lin, x[None], None) and not L._native(lin, x[:0], None)
+        assert not L._native(lin, torch.randn(33, 64, device="cuda").bfloat16(), None)
+        assert not L._native(lin, torch.randn(4, 65, device="cuda").bfloat16()[:, 1:], None)
+        assert not L._native(lin, torch.randn(64, 4, device="cuda").bfloat16().t(), None)
+        with torch.autocast("cuda", dtype=torch.float16):
+            assert not L._native(lin, x, None)
+        seen = []
+        hook = lin.register_forward_hook(lambda m, a, o: seen.append(o))
+        y = L.linear_rows(lin, x, torch.ones(4, 32, device="cuda", dtype=torch.bfloat16))
+        hook.remove()
+        assert len(seen) == 1 and torch.equal(y, seen[0] + 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,H", [(torch.bfloat16, 8), (torch.float16, 264), (torch.float32, 4100), (torch.bfloat16, 12)])
+def test_embed_rows(dtype, H):
+    from colossalai_b200 import ops
+
+    emb = nn.Embedding(50, H, device="cuda", dtype=dtype)
+    ids = torch.tensor([0, 49, 7, 7, 3], device="cuda")
+    with torch.no_grad():
+        assert torch.equal(ops.embed_rows(emb, ids), emb.weight[ids])
+    assert ops.embed_rows(emb, ids).requires_grad
+
+
+def test_on_the_cpu_the_module_is_called():
+    from colossalai_b200 import ops
+
+    lin, emb = nn.Linear(8, 4), nn.Embedding(5, 8)
+    ids = torch.tensor([4, 0])
+    with torch.no_grad():
+        x = ops.embed_rows(emb, ids)
+        assert torch.equal(x, emb(ids)) and torch.equal(ops.linear_rows(lin, x, x[:, :4]), x[:, :4] + lin(x))
+
+
+def test_graph_inputs_of_one_type_are_copied_together():
+    """Copies of alike tensors go together, other types and layouts one by one: the static inputs end up equal."""
+    from colossalai_b200.inference.graph_runner import CUDAGraphRunner
+
+    r = CUDAGraphRunner(None)
+    r.static_inputs = {"a": torch.zeros(3), "b": torch.zeros(2, 2), "c": torch.zeros(4, dtype=torch.int64), "d": torch.zeros(2, 3)}
+    r.graph = type("G", (), {"replay": lambda self: None})()
+    new = {"a": torch.randn(3), "b": torch.randn(1, 2).expand(2, 2), "c": torch.arange(4, dtype=torch.int32), "d": torch.randn(3, 2).t()}
+    r(**new)
+    for k, v in new.items():
+        assert torch.equal(r.static_inputs[k], v.to(r.static_inputs[k].dtype))
