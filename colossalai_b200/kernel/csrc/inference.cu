@@ -404,6 +404,11 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_kernel(
 //   * partial results use the same (o_part, ml_part) format, so the reduce kernel is shared.
 constexpr int DEC_MMA_TOKENS = 16;
 constexpr int DEC_MMA_STAGES = 3;
+// Warps of a CTA, one for each kv head: all of them up to eight, four where there are more, which fill the CTAs and leave less of the
+// SMs idle in the last round.  Device time, us, eight / four warps: 128 x 1024 tokens of 12 heads of 64 62.3 / 56.6, 16 x 1024 of 32 heads of
+// 128 45.0 / 43.8, 24 x 900 of 16 heads 34.3 / 33.3; of 32 / 8 heads 64 x 2048 77.4 / 75.8, but a decode step of 16 x 1024 509 / 514 (an SM
+// that is left free takes the next kernels' CTAs meanwhile).
+constexpr int DEC_MMA_WARPS = 4;
 
 CB_DEVICE void ldmatrix_x4(uint32_t (&r)[4], const void* smem_row) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem_row);
@@ -808,7 +813,7 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
   // <= 8 q heads); CB200_DECODE=simt forces the CUDA-core kernel (also used for head_dim 256)
   const char* impl_env = getenv("CB200_DECODE");
   const bool use_mma = !(impl_env != nullptr && impl_env[0] == 's') && G <= 8 && (D == 128 || D == 64);
-  const int mma_warps = Hkv < DEC_THREADS / 32 ? Hkv : DEC_THREADS / 32;
+  const int mma_warps = Hkv <= DEC_THREADS / 32 ? Hkv : DEC_MMA_WARPS;
   dim3 mma_grid(num_seqs, (Hkv + mma_warps - 1) / mma_warps, splits);
 #define LAUNCH_DEC_MMA(T, DD)                                                                                       \
   {                                                                                                                  \
