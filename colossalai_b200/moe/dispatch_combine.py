@@ -17,7 +17,7 @@ from ..ops._dispatch import plain_call, use_native
 from ..ops.moe import SORT_EXPERTS, CombineRows, TakeRows, rows_ok, sort_choices
 from ..parallel import comm
 from ._operation import AllToAllUneven
-from .grouped_gemm import ALIGN
+from .grouped_gemm import ROW_ALIGN
 
 __all__ = ["moe_forward", "set_moe_backend", "get_moe_backend"]
 
@@ -49,7 +49,7 @@ def _use_fused(x: torch.Tensor, num_experts: int, ep_group) -> bool:
 
 
 def _aligned_rows(x: torch.Tensor) -> bool:
-    """Lay the expert-grouped rows out with every expert's range padded to 16 rows (zero rows): the native grouped
+    """Lay the expert-grouped rows out with every expert's range padded with zero rows (to 16, or to 128 by index operations): the native grouped
     weight-gradient GEMM then needs no re-layout pass (moe/grouped_gemm.py)."""
     return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
             and os.environ.get("CB200_GROUPED_GEMM", "native") == "native"
@@ -100,7 +100,7 @@ def moe_forward(x: torch.Tensor, topk_w: torch.Tensor, topk_idx: torch.Tensor, e
         # all experts here: the rows are sorted, gathered, combined and differentiated by kernels of their own, without a
         # host synchronisation (`ops/moe.py`); the index operations below remain for CPU tensors, 32-bit rows, more experts than the sort has counters for, and for calls
         # that functorch, forward mode or a mode watches
-        slot, src, counts = sort_choices(topk_idx, num_experts, ALIGN)
+        slot, src, counts = sort_choices(topk_idx, num_experts, ROW_ALIGN)
         counts.cb200_aligned = True
         ys = experts(TakeRows.apply(x, slot, src, k), counts)
         if rows_ok(ys):

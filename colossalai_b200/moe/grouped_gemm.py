@@ -16,7 +16,8 @@ from typing import Optional, Tuple
 import torch
 
 _lib = None
-ALIGN = 16            # reduction of one instruction of the wgrad kernel: group row ranges must start / end on multiples of it
+ROW_ALIGN = 16        # reduction of one instruction of the wgrad kernel: group row ranges must start / end on multiples of it
+ALIGN = 128           # a coarser layout, of the sorted path with index operations
 K_BLOCK = 128         # the input-gradient GEMM reads an expert's weight in blocks of rows that it must not share with the next
 
 
@@ -59,7 +60,7 @@ def _native_fwd(x: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, transpose_
 
 
 def _native_wgrad(dy: torch.Tensor, x: torch.Tensor, offs: torch.Tensor, E: int, out_dtype: torch.dtype) -> torch.Tensor:
-    """dw[e] = dy[rows e]^T @ x[rows e]; every group's row range is a multiple of ALIGN."""
+    """dw[e] = dy[rows e]^T @ x[rows e]; every group's row range is a multiple of ROW_ALIGN."""
     from ..kernel import loader
     from ..ops._dtypes import code
 
@@ -74,19 +75,19 @@ def _native_wgrad(dy: torch.Tensor, x: torch.Tensor, offs: torch.Tensor, E: int,
     return dw
 
 
-def _pad_groups(counts: torch.Tensor, rows: int, device) -> Tuple[torch.Tensor, torch.Tensor, int]:
-    """Device-side map from the packed row layout to one where every group starts on a multiple of ALIGN.
+def _pad_groups(counts: torch.Tensor, rows: int, device, align: int = ALIGN) -> Tuple[torch.Tensor, torch.Tensor, int]:
+    """Device-side map from the packed row layout to one where every group starts on a multiple of `align`.
     Returns (dest row of every packed row, padded cumulative offsets int32, static upper bound of padded rows)."""
     c = counts.to(device=device, dtype=torch.int64)
     E = c.numel()
     ends = torch.cumsum(c, 0)
     starts = ends - c
-    pc = (c + ALIGN - 1) // ALIGN * ALIGN
+    pc = (c + align - 1) // align * align
     pends = torch.cumsum(pc, 0)
     pstarts = pends - pc
     row = torch.arange(rows, device=device)
     g = torch.searchsorted(ends, row, right=True)
-    bound = (rows + E * (ALIGN - 1) + ALIGN - 1) // ALIGN * ALIGN
+    bound = (rows + E * (align - 1) + align - 1) // align * align
     # rows past the last group (a caller's over-allocated buffer) go to a dump row behind the padded layout
     dest = torch.where(g < E, row + (pstarts - starts)[g.clamp(max=E - 1)], torch.full_like(row, bound))
     return dest, pends.to(torch.int32), bound
@@ -116,7 +117,7 @@ class _GroupedLinearNative(torch.autograd.Function):
             if ctx.aligned:
                 dw = _native_wgrad(dy, x, offs, w.shape[0], w.dtype)
             else:
-                dest, poffs, bound = _pad_groups(counts, x.shape[0], x.device)
+                dest, poffs, bound = _pad_groups(counts, x.shape[0], x.device, ROW_ALIGN)
                 xp = torch.zeros(bound + 1, x.shape[1], dtype=x.dtype, device=x.device).index_copy_(0, dest, x)
                 dyp = torch.zeros(bound + 1, dy.shape[1], dtype=dy.dtype, device=x.device).index_copy_(0, dest, dy)
                 dw = _native_wgrad(dyp[:bound], xp[:bound], poffs, w.shape[0], w.dtype)
