@@ -389,6 +389,9 @@ class MLP(nn.Module):
         return ops.linear_rows(self.down_proj, h, residual)
 
 
+_MLP_FORWARD = MLP.forward             # the one that takes a residual
+
+
 class DecoderLayer(nn.Module):
     def __init__(self, cfg: ModelConfig, layer_idx: int) -> None:
         super().__init__()
@@ -459,7 +462,7 @@ class DecoderLayer(nn.Module):
         else:
             x = x + a
             h = self.post_attention_layernorm(x)
-        if type(self.mlp) is MLP and not torch.is_grad_enabled() and ops.unwatched(self.mlp):
+        if type(self.mlp) is MLP and not torch.is_grad_enabled() and ops.unwatched(self.mlp, _MLP_FORWARD):
             return self.mlp(h, residual=x)
         return x + self.mlp(h)
 

@@ -19,10 +19,14 @@ from ._dispatch import plain_call, use_native
 __all__ = ["linear_rows", "embed_rows", "unwatched", "ROWS_MAX"]
 
 ROWS_MAX = 32         # what the kernel takes; figures there
+_LINEAR, _EMBEDDING = nn.Linear.forward, nn.Embedding.forward
 
 
-def unwatched(m: nn.Module) -> bool:
-    """No hook sees a call of the module."""
+def unwatched(m: nn.Module, forward) -> bool:
+    """A call of the module runs `forward`, what its class came with, and nothing else: it is replaced neither on the instance (as
+    `convert_linear_to_fp8` and adapters do) nor on the class, not compiled, and no hook sees the call."""
+    if type(m).forward is not forward or "forward" in m.__dict__ or m._compiled_call_impl is not None:
+        return False
     return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
                 or _module._global_forward_hooks or _module._global_forward_pre_hooks
                 or _module._global_backward_hooks or _module._global_backward_pre_hooks)
@@ -47,7 +51,7 @@ def _native(linear: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor]
     if residual is not None and (residual.shape != (x.shape[0], n) or residual.dtype != x.dtype or residual.device != x.device
                                  or residual.stride(1) != 1):
         return False
-    return (use_native(x) and unwatched(linear) and plain_call(x, w, residual) and not torch.is_autocast_enabled("cuda")
+    return (use_native(x) and unwatched(linear, _LINEAR) and plain_call(x, w, residual) and not torch.is_autocast_enabled("cuda")
             and _sm100(x.device))
 
 
@@ -67,6 +71,6 @@ def embed_rows(embedding: nn.Module, ids: torch.Tensor) -> torch.Tensor:
             and ids.dtype == torch.int64 and ids.is_contiguous() and ids.numel() > 0 and w.device == ids.device
             and w.dtype in (torch.bfloat16, torch.float16, torch.float32) and w.is_contiguous()
             and w.shape[1] * w.element_size() % 16 == 0 and w.shape[1] > 0 and w.data_ptr() % 16 == 0 and use_native(ids)
-            and unwatched(embedding) and plain_call(ids, w) and (host := loader.host()) is not None):
+            and unwatched(embedding, _EMBEDDING) and plain_call(ids, w) and (host := loader.host()) is not None):
         return host.embed_rows(ids, w)
     return embedding(ids)

@@ -93,3 +93,65 @@ def test_graph_inputs_of_one_type_are_copied_together():
     r(**new)
     for k, v in new.items():
         assert torch.equal(r.static_inputs[k], v.to(r.static_inputs[k].dtype))
+
+
+def _replaced():
+    """Modules whose call is not what their class came with, on the instance and on the class."""
+    from types import MethodType
+
+    from colossalai_b200.quantization.fp8_hook import convert_linear_to_fp8
+
+    lin, emb = nn.Linear(16, 16, bias=False), nn.Embedding(5, 16)
+    lin.forward = MethodType(lambda self, x: x + 1, lin)
+    emb.forward = MethodType(lambda self, ids: ids + 1, emb)
+    fp8 = nn.Linear(16, 16, bias=False)
+    convert_linear_to_fp8(fp8)
+    compiled = nn.Linear(16, 16, bias=False)
+    compiled._compiled_call_impl = lambda x: x + 1
+    return [(lin, nn.Linear), (emb, nn.Embedding), (fp8, nn.Linear), (compiled, nn.Linear)]
+
+
+def test_a_replaced_forward_is_seen(monkeypatch):
+    from colossalai_b200.ops import linear as L
+
+    lin, emb = nn.Linear(16, 16, bias=False), nn.Embedding(5, 16)
+    assert L.unwatched(lin, L._LINEAR) and L.unwatched(emb, L._EMBEDDING)
+    for m, kind in _replaced():
+        assert not L.unwatched(m, L._LINEAR if kind is nn.Linear else L._EMBEDDING)
+    monkeypatch.setattr(nn.Linear, "forward", lambda self, x: x + 1)
+    assert not L.unwatched(lin, L._LINEAR)
+
+
+@pytest.mark.parametrize("where", ["instance", "class"])
+def test_a_replaced_feed_forward_gets_one_argument(where, monkeypatch):
+    from colossalai_b200.models.config import ModelConfig
+    from colossalai_b200.models.transformer import MLP, TransformerLMHeadModel
+
+    cfg = ModelConfig(vocab_size=32, hidden_size=32, intermediate_size=64, num_hidden_layers=1, num_attention_heads=2,
+                      num_key_value_heads=2)
+    model = TransformerLMHeadModel(cfg)
+    mlp = next(m for m in model.modules() if isinstance(m, MLP))
+    if where == "instance":
+        mlp.forward = lambda x: torch.zeros_like(x)
+    else:
+        monkeypatch.setattr(MLP, "forward", lambda self, x: torch.zeros_like(x))
+    ids = torch.arange(6)[None]
+    want = model(ids)["logits"]
+    with torch.no_grad():
+        assert torch.equal(model(ids)["logits"], want)
+
+
+@pytest.mark.gpu
+def test_a_replaced_forward_is_called():
+    from colossalai_b200 import ops
+    from colossalai_b200.kernel import launch_counter
+
+    x, ids = torch.randn(4, 16, device="cuda").bfloat16(), torch.tensor([4, 0], device="cuda")
+    before = {k: launch_counter.by_name.get(k, 0) for k in ("gemm_rows", "embed_rows")}
+    for m, kind in _replaced():
+        m = m.to("cuda", torch.bfloat16)
+        a = x if kind is nn.Linear else ids
+        with torch.no_grad():
+            got = ops.linear_rows(m, a) if kind is nn.Linear else ops.embed_rows(m, a)
+            assert torch.equal(got, m(a))
+    assert before == {k: launch_counter.by_name.get(k, 0) for k in before}
