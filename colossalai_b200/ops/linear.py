@@ -38,10 +38,13 @@ def _sm100(device: torch.device) -> bool:
 
 
 def _native(linear: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor]) -> bool:
-    if type(linear) is not nn.Linear or torch.is_grad_enabled() or not x.is_cuda or x.dim() != 2 or not 0 < x.shape[0] <= ROWS_MAX:
+    if type(linear) is not nn.Linear or torch.is_grad_enabled() or not use_native(x) or x.dim() != 2 or not 0 < x.shape[0] <= ROWS_MAX:
         return False
     w = linear.weight
     if linear.bias is not None or w.dtype != x.dtype or x.dtype not in (torch.bfloat16, torch.float16) or w.device != x.device:
+        return False
+    # (before strides and pointers are looked at: what vmap, tracing or a mode hands in may have neither)
+    if not plain_call(x, w, residual) or not unwatched(linear, _LINEAR) or torch.is_autocast_enabled("cuda"):
         return False
     n, k = w.shape
     # one contiguous weight, rows that TMA can address
@@ -51,8 +54,7 @@ def _native(linear: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor]
     if residual is not None and (residual.shape != (x.shape[0], n) or residual.dtype != x.dtype or residual.device != x.device
                                  or residual.stride(1) != 1):
         return False
-    return (use_native(x) and unwatched(linear, _LINEAR) and plain_call(x, w, residual) and not torch.is_autocast_enabled("cuda")
-            and _sm100(x.device))
+    return _sm100(x.device)
 
 
 def linear_rows(linear: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -63,14 +65,20 @@ def linear_rows(linear: nn.Module, x: torch.Tensor, residual: Optional[torch.Ten
     return y if residual is None else residual + y
 
 
+def _native_lookup(embedding: nn.Module, ids: torch.Tensor) -> bool:
+    if type(embedding) is not nn.Embedding or embedding.max_norm is not None or torch.is_grad_enabled() or not use_native(ids):
+        return False
+    w = embedding.weight
+    if not plain_call(ids, w) or not unwatched(embedding, _EMBEDDING):
+        return False
+    return (ids.dim() == 1 and ids.dtype == torch.int64 and ids.is_contiguous() and ids.numel() > 0 and w.device == ids.device
+            and w.dtype in (torch.bfloat16, torch.float16, torch.float32) and w.is_contiguous()
+            and w.shape[1] * w.element_size() % 16 == 0 and w.shape[1] > 0 and w.data_ptr() % 16 == 0)
+
+
 def embed_rows(embedding: nn.Module, ids: torch.Tensor) -> torch.Tensor:
     """embedding(ids).  Outside autograd the rows of a plain table come through a kernel with a block per id (16 rows of 4096: 2.6 us,
     torch's index kernel 14); an id outside the table gives NaN."""
-    w = getattr(embedding, "weight", None)
-    if (type(embedding) is nn.Embedding and embedding.max_norm is None and not torch.is_grad_enabled() and ids.is_cuda and ids.dim() == 1
-            and ids.dtype == torch.int64 and ids.is_contiguous() and ids.numel() > 0 and w.device == ids.device
-            and w.dtype in (torch.bfloat16, torch.float16, torch.float32) and w.is_contiguous()
-            and w.shape[1] * w.element_size() % 16 == 0 and w.shape[1] > 0 and w.data_ptr() % 16 == 0 and use_native(ids)
-            and unwatched(embedding, _EMBEDDING) and plain_call(ids, w) and (host := loader.host()) is not None):
-        return host.embed_rows(ids, w)
+    if _native_lookup(embedding, ids) and (host := loader.host()) is not None:
+        return host.embed_rows(ids, embedding.weight)
     return embedding(ids)

@@ -155,3 +155,35 @@ def test_a_replaced_forward_is_called():
             got = ops.linear_rows(m, a) if kind is nn.Linear else ops.embed_rows(m, a)
             assert torch.equal(got, m(a))
     assert before == {k: launch_counter.by_name.get(k, 0) for k in before}
+
+
+@pytest.mark.parametrize("what", ["linear", "embedding"])
+def test_watched_calls_are_not_asked_for_pointers(what):
+    """Under vmap and fake tensors there is none to be had: the module is called."""
+    import warnings
+
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from colossalai_b200 import ops
+
+    with FakeTensorMode(), torch.no_grad(), warnings.catch_warnings():
+        warnings.simplefilter("error")
+        if what == "linear":
+            m, f, one = nn.Linear(64, 32, bias=False, device="cuda", dtype=torch.bfloat16), ops.linear_rows, (4, 64)
+            x = torch.empty(3, *one, device="cuda", dtype=torch.bfloat16)
+        else:
+            m, f, one = nn.Embedding(50, 32, device="cuda", dtype=torch.bfloat16), ops.embed_rows, (4,)
+            x = torch.zeros(3, *one, device="cuda", dtype=torch.int64)
+        assert f(m, x[0]).shape == (4, 32)
+        assert torch.func.vmap(lambda a: f(m, a))(x).shape == (3, 4, 32)
+
+
+@pytest.mark.gpu
+def test_vmap_calls_the_module():
+    from colossalai_b200 import ops
+
+    lin, emb = nn.Linear(64, 32, bias=False, device="cuda", dtype=torch.bfloat16), nn.Embedding(50, 32, device="cuda", dtype=torch.bfloat16)
+    x, ids = torch.randn(3, 4, 64, device="cuda").bfloat16(), torch.randint(0, 50, (3, 4), device="cuda")
+    with torch.no_grad():
+        assert torch.equal(torch.func.vmap(lambda a: ops.linear_rows(lin, a))(x), torch.func.vmap(lin)(x))
+        assert torch.equal(torch.func.vmap(lambda a: ops.embed_rows(emb, a))(ids), emb(ids))
