@@ -14,6 +14,7 @@
 // 39.2, 4096 x 14336 22.9 and 20.4, 32000 x 4096 45.5 and 43.0, 2048 x 8192 13.0 and 8.8, 1536 x 1024 3.6 and 3.7; 32 rows 9.9 / 8.9,
 // 12.4 / 12.0, 41.6 / 39.8, 27.3 / 21.3, 45.8 / 44.3, 13.1 / 9.5, 3.7 / 4.0.  Three stages and four CTAs on an SM were slower for deep
 // matrices (4096 x 14336 22.4).  A decode step of four layers of 4096 x 14336, 16 sequences: 530 us with cuBLAS, 509.
+#include "checked_id.h"
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -208,15 +209,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   if (warp == 1) tmem_dealloc<32>(tmem);
 }
 
-// out[i] = table[ids[i]]: a block per id, 16 bytes a thread and step; NaN (all ones) for an id outside the table
+// out[i] = table[ids[i]]: a block per id, 16 bytes a thread and step
 __global__ void __launch_bounds__(256) embed_rows_kernel(const int64_t* __restrict__ ids, const uint4* __restrict__ table, uint4* __restrict__ out,
                                                          int64_t entries, int vecs) {
   cb_early_start();
-  const int64_t id = ids[blockIdx.x];
-  const bool known = id >= 0 && id < entries;
+  const uint4* src = table + cb_checked_id(ids[blockIdx.x], entries) * vecs;
   uint4* dst = out + (int64_t)blockIdx.x * vecs;
-  const uint4* src = table + (known ? id : 0) * vecs;
-  for (int i = threadIdx.x; i < vecs; i += 256) dst[i] = known ? src[i] : make_uint4(~0u, ~0u, ~0u, ~0u);
+  for (int i = threadIdx.x; i < vecs; i += 256) dst[i] = src[i];
 }
 
 template <typename T, int NT>

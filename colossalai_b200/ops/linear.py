@@ -78,7 +78,7 @@ def _native_lookup(embedding: nn.Module, ids: torch.Tensor) -> bool:
 
 def embed_rows(embedding: nn.Module, ids: torch.Tensor) -> torch.Tensor:
     """embedding(ids).  Outside autograd the rows of a plain table come through a kernel with a block per id (16 rows of 4096: 2.6 us,
-    torch's index kernel 14); an id outside the table gives NaN."""
+    torch's index kernel 14); an id outside the table ends in a device assertion there too."""
     if _native_lookup(embedding, ids) and (host := loader.host()) is not None:
         return host.embed_rows(ids, embedding.weight)
     return embedding(ids)

@@ -187,3 +187,20 @@ def test_vmap_calls_the_module():
     with torch.no_grad():
         assert torch.equal(torch.func.vmap(lambda a: ops.linear_rows(lin, a))(x), torch.func.vmap(lin)(x))
         assert torch.equal(torch.func.vmap(lambda a: ops.embed_rows(emb, a))(ids), emb(ids))
+
+
+@pytest.mark.parametrize("id_,entries,refused", [(0, 1, False), (49, 50, False), (2**40, 2**41, False), (-1, 50, True), (50, 50, True),
+                                                 (2**32, 50, True), (0, 0, True)])
+def test_an_id_outside_the_table_is_refused(id_, entries, refused, tmp_path):
+    """The rule that the lookup kernel applies to every id, run on the host: it ends the program, as torch's own lookup does."""
+    import subprocess
+
+    from colossalai_b200.kernel.loader import CSRC
+
+    assert "cb_checked_id(ids[blockIdx.x], entries)" in (CSRC / "gemm_rows_tcgen05.cu").read_text()
+    src, exe = tmp_path / "id.cpp", tmp_path / "id"
+    src.write_text('#include "checked_id.h"\n#include <stdlib.h>\n'
+                   "int main(int, char** a) { return cb_checked_id(atoll(a[1]), atoll(a[2])) == atoll(a[1]) ? 0 : 1; }\n")
+    subprocess.run(["g++", "-O2", "-I", str(CSRC), str(src), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe), str(id_), str(entries)], capture_output=True, text=True)
+    assert r.returncode == (-6 if refused else 0) and ("outside the table" in r.stderr) == refused
