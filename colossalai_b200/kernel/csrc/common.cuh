@@ -8,6 +8,8 @@
 #include <cuda_fp8.h>
 #include <stdint.h>
 
+#include "device_attr.h"
+
 #define CB_DEVICE __device__ __forceinline__
 #define CB_HOST_DEVICE __host__ __device__ __forceinline__
 

@@ -1128,13 +1128,8 @@ template <int D, bool EXTRA, bool BF16>
 int launch_flash_fwd_tile_kernel(dim3 grid, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p,
                                  cudaStream_t stream) {
   using C = FaTileCfg<D>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(flash_fwd_tile_kernel<D, EXTRA, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, flash_fwd_tile_kernel<D, EXTRA, BF16>, C::SMEM_BYTES)) return e;
   flash_fwd_tile_kernel<D, EXTRA, BF16><<<grid, TILE_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
@@ -1143,13 +1138,8 @@ template <int D, bool EXTRA, bool BF16>
 int launch_flash_fwd_kernel(dim3 grid, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p,
                             cudaStream_t stream) {
   using C = FaCfg<D>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(flash_fwd_kernel<D, EXTRA, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, flash_fwd_kernel<D, EXTRA, BF16>, C::SMEM_BYTES)) return e;
   flash_fwd_kernel<D, EXTRA, BF16><<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
@@ -1757,12 +1747,8 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* do
   p.idesc_dv = make_idesc_f16(BWD_BLOCK_KV, D, f, 0, 1);                // [128 keys x D]     = K-major x MN-major
   p.idesc_dqt = make_idesc_f16(D, BWD_BLOCK_Q, f, 1, 1);                // [D x 64 q]         = MN-major x MN-major
   auto kern = bf16 ? flash_bwd_kernel<D, true> : flash_bwd_kernel<D, false>;
-  static bool attr_set[2] = {false, false};
-  if (!attr_set[f]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set[f] = true;
-  }
+  static CbDeviceAttr attr[2];
+  if (const int e = cb_allow_smem(attr[f], kern, C::SMEM_BYTES)) return e;
   const long long units = (cu_seqlens ? total_tokens / BWD_BLOCK_KV + batch : ((long long)seqlen + BWD_BLOCK_KV - 1) / BWD_BLOCK_KV) * hkv;
   const dim3 grid((unsigned)units, cu_seqlens ? 1 : batch);
   if (units > 0x7fffffffll || grid.y > 65535) return (int)cudaErrorInvalidValue;

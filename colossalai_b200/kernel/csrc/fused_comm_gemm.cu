@@ -919,13 +919,8 @@ int launch_fused_2cta(const void* A, const void* B, int M, int N, int K, int lda
   r = b_mn ? make_tmap_2d_16b(&tb, B, K, N, ldb, BK, 64, bf16) : make_tmap_2d_16b(&tb, B, N, K, ldb, 128, 64, bf16);
   if (r) return 2000 + r;
   p.idesc = make_idesc_f16(PAIR_M, PAIR_N, bf16 ? 1 : 0, a_mn, b_mn);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(fused_gemm_2cta_kernel<MODE, BK, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, fused_gemm_2cta_kernel<MODE, BK, STAGES>, C::SMEM_BYTES)) return e;
   const int grid = cb_num_sms() & ~1;     // all CTAs co-resident (flag spinning): one CTA per SM, whole pairs
   fused_gemm_2cta_kernel<MODE, BK, STAGES><<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(ta, tb, p, c);
   return (int)cudaGetLastError();
@@ -1117,13 +1112,8 @@ int launch_fused(const void* A, const void* B, int M, int N, int K, int lda, int
   r = b_mn ? make_tmap_2d_16b(&tb, B, K, N, ldb, BLOCK_K, 64, bf16) : make_tmap_2d_16b(&tb, B, N, K, ldb, BLOCK_N, 64, bf16);
   if (r) return 2000 + r;
   p.idesc = make_idesc_f16(BLOCK_M, BLOCK_N, bf16 ? 1 : 0, a_mn, b_mn);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(fused_gemm_kernel<BLOCK_N, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, fused_gemm_kernel<BLOCK_N, MODE>, C::SMEM_BYTES)) return e;
   // persistent grid: ALL CTAs must be co-resident (flag spinning) -> exactly one CTA per SM
   const int grid = cb_num_sms();
   fused_gemm_kernel<BLOCK_N, MODE><<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(ta, tb, p, c);

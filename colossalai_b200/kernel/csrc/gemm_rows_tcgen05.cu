@@ -220,12 +220,8 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(const int64_t* __restri
 
 template <typename T, int NT>
 int launch_rows(const CUtensorMap& tw, const CUtensorMap& tx, const RowsParams& p, int tiles, int splits, cudaStream_t stream) {
-  static bool done = false;
-  if (!done) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsCfg<NT>::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    done = true;
-  }
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, gemm_rows_kernel<T, NT>, RowsCfg<NT>::SMEM)) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles, splits);
   cfg.blockDim = dim3(ROWS_THREADS);

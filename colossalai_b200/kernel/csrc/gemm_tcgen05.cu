@@ -671,13 +671,8 @@ int launch_2cta(const void* A, const void* B, void* Cp, int M, int N, int K, int
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.a_mn_major = a_mn; p.b_mn_major = b_mn; p.out_dtype = out_dtype;
   p.accumulate = accumulate; p.C = Cp;
   p.idesc = make_idesc_f16(PAIR_M, PAIR_N, bf16 ? 1 : 0, a_mn, b_mn);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_2cta_kernel<BK, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, gemm_tcgen05_2cta_kernel<BK, STAGES>, C::SMEM_BYTES)) return e;
   const int tiles = ((M + PAIR_M - 1) / PAIR_M) * ((N + PAIR_N - 1) / PAIR_N);
   int pairs = cb_num_sms() / 2;
   if (tiles < pairs) pairs = tiles;
@@ -727,13 +722,8 @@ int launch_2cta_f8(const void* A, const void* B, void* Cp, int M, int N, int K, 
   d |= (uint32_t)(a_fmt & 7) << 7;              // 0 = E4M3, 1 = E5M2
   d |= (uint32_t)(b_fmt & 7) << 10;
   p.idesc = d;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_2cta_kernel<BK, STAGES, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, gemm_tcgen05_2cta_kernel<BK, STAGES, true>, C::SMEM_BYTES)) return e;
   const int tiles = ((M + PAIR_M - 1) / PAIR_M) * ((N + PAIR_N - 1) / PAIR_N);
   int pairs = cb_num_sms() / 2;
   if (tiles < pairs) pairs = tiles;
@@ -759,13 +749,8 @@ int launch(const void* A, const void* B, void* Cp, int M, int N, int K, int lda,
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.a_mn_major = a_mn; p.b_mn_major = b_mn; p.out_dtype = out_dtype;
   p.accumulate = accumulate; p.C = Cp;
   p.idesc = make_idesc_f16(BLOCK_M, BLOCK_N, bf16 ? 1 : 0, a_mn, b_mn);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BLOCK_N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, gemm_tcgen05_kernel<BLOCK_N>, C::SMEM_BYTES)) return e;
   const int tiles = ((M + BLOCK_M - 1) / BLOCK_M) * ((N + BLOCK_N - 1) / BLOCK_N);
   int grid = cb_num_sms();
   if (tiles < grid) grid = tiles;

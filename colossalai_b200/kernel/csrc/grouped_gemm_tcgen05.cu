@@ -559,18 +559,11 @@ grouped_wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   if (warp == 2) tmem_dealloc_2cta<512>(tmem_base);
 }
 
-template <typename K> int allow_smem(K* kernel, int bytes, bool& done) {
-  if (done) return 0;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  done = e == cudaSuccess;
-  return (int)e;
-}
-
 // the number of tiles is only known on the device: full persistent grids
 template <int MODE, typename T>
 int launch_rows(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tx32, const GroupedParams& p, cudaStream_t stream) {
-  static bool done = false;
-  if (const int e = allow_smem(grouped_rows_2cta_kernel<MODE, T>, smem_bytes<MODE>(), done)) return e;
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, grouped_rows_2cta_kernel<MODE, T>, smem_bytes<MODE>())) return e;
   grouped_rows_2cta_kernel<MODE, T><<<cb_num_sms() / 2 * 2, ROWS_THREADS, smem_bytes<MODE>(), stream>>>(tw, tx, tx32, p);
   return (int)cudaGetLastError();
 }
@@ -578,8 +571,8 @@ int launch_rows(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap&
 template <typename OUT>
 int launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ta32, const CUtensorMap& tb32, const CUtensorMap& tc,
                  const GroupedParams& p, cudaStream_t stream) {
-  static bool done = false;
-  if (const int e = allow_smem(grouped_wgrad_2cta_kernel<OUT>, smem_bytes<MODE_TN>(), done)) return e;
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, grouped_wgrad_2cta_kernel<OUT>, smem_bytes<MODE_TN>())) return e;
   grouped_wgrad_2cta_kernel<OUT><<<cb_num_sms() / 2 * 2, WGRAD_THREADS, smem_bytes<MODE_TN>(), stream>>>(ta, tb, ta32, tb32, tc, p);
   return (int)cudaGetLastError();
 }

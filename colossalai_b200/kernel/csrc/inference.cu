@@ -818,12 +818,8 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
 #define LAUNCH_DEC_MMA(T, DD)                                                                                       \
   {                                                                                                                  \
     constexpr int per_warp = DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * DD * 2;                                           \
-    static bool attr_done = false;                                                                                   \
-    if (!attr_done) {                                                                                                \
-      cudaFuncSetAttribute(paged_decode_mma_kernel<T, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize,              \
-                           (DEC_THREADS / 32) * per_warp);                                                           \
-      attr_done = true;                                                                                              \
-    }                                                                                                                \
+    static CbDeviceAttr attr;                                                                                        \
+    if (const int e = cb_allow_smem(attr, paged_decode_mma_kernel<T, DD>, (DEC_THREADS / 32) * per_warp)) return e;  \
     if (const int e = cb_launch_early(paged_decode_mma_kernel<T, DD>, mma_grid, mma_warps * 32, mma_warps * per_warp, s, \
         (const T*)q, (const T*)k_cache, (const T*)v_cache, block_tables, seq_lens, o_part, ml_part, Hq, Hkv,        \
         block_size, max_blocks_per_seq, splits, part_len, scale, alibi_slopes, q_stride, window)) return e;         \
@@ -831,11 +827,8 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
   }
 #define LAUNCH_DEC(T, DD)                                                                                           \
   {                                                                                                                  \
-    static bool attr_done = false;                                                                                   \
-    if (!attr_done) {                                                                                                \
-      cudaFuncSetAttribute(paged_decode_kernel<T, T, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_smem_max);\
-      attr_done = true;                                                                                              \
-    }                                                                                                                \
+    static CbDeviceAttr attr;                                                                                        \
+    if (const int e = cb_allow_smem(attr, paged_decode_kernel<T, T, DD>, dec_smem_max)) return e;                    \
   }                                                                                                                  \
   paged_decode_kernel<T, T, DD><<<grid, warps * 32, dec_smem, s>>>((const T*)q, (const T*)k_cache, (const T*)v_cache, \
       block_tables, seq_lens, o_part, ml_part, Hq, Hkv, block_size, max_blocks_per_seq, splits, part_len, scale,     \

@@ -828,12 +828,8 @@ template <int DK, int MODE, bool SHORT> int launch_scan_dk(const ScanParams& p, 
   using Tile = ScanTile<DK, MODE, SHORT>;
   const size_t smem = (size_t)Tile::STAGES * Tile::TILE * Tile::TOKEN * sizeof(float);
   auto kern = state_scan_kernel<DK, MODE, SHORT>;
-  static bool configured = false;
-  if (!configured) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-    configured = true;
-  }
+  static CbDeviceAttr attr;
+  if (const int e = cb_allow_smem(attr, kern, smem, true)) return e;
   kern<<<p.heads * (w.VP / SCAN_COLS) * nseq, Tile::THREADS, smem, st>>>(p, w, nseq, cb_num_sms());
   return CB_LAUNCH_CHECK();
 }
@@ -2175,12 +2171,8 @@ int launch_attention_mma(const void* q, int64_t ldq, const void* k_cache, const 
   const bool kv_same = v_cache == k_cache && ldv == dim;
   const size_t smem = (size_t)((kv_same ? 2 : 4) * MMA_BN + BM) * (D + 8) * sizeof(T) + (size_t)nbuckets * R * sizeof(float);
   auto kern = paged_bias_attention_mma_kernel<T, D, MT, KS>;
-  static bool configured = false;               // per instantiation: opt in to large shared memory, all of it for CTAs
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-    configured = true;
-  }
+  static CbDeviceAttr attr;                     // per instantiation: opt in to large shared memory, all of it for CTAs
+  if (const int e = cb_allow_smem(attr, kern, 200 * 1024, true)) return e;
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   const int rowtiles = (max_q * R + BM - 1) / BM;
   dim3 grid(rowtiles * (chunk > 0 ? max_splits : 1), kv_heads, nseq);
