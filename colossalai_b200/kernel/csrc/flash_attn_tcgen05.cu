@@ -591,6 +591,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       const size_t row = (size_t)un.q_start + q_pos;       // row in the token-major Q / O
       float m_run = -INFINITY;                             // reference max of the exponentials (exp2 domain)
       float l_run = 0.f;
+      float m_ahead = -INFINITY;                           // maximum of scores that a later step takes
       if (resume) {
         ok = __all_sync(0xffffffffu, wait_or_abort(&o_empty[t], (units_of & 1) ^ 1, abort_flag));
         if (!ok) break;
@@ -622,18 +623,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const int h = j & 1;
         return __all_sync(0xffffffffu, wait_or_abort(&o_full[2 * t + h], ((phase >> h) & 1) ^ 1, abort_flag)) != 0;
       };
-      // one step of 64 keys; two copies of the code, because a branch around the mask alone is turned into predicated
-      // comparisons and selections that every step executes
-      auto step = [&](int j, auto masked_tag) -> bool {
+      // plain variant: the softmax scale (> 0) is folded into the exponent's FMA, the max is taken on the raw scores;
+      // EXTRA variant: scale and ALiBi bias are applied here and the exponent uses a unit multiplier
+      const float ex_mul = EXTRA ? 1.f : p.scale_log2;
+      auto visible = [&](uint32_t (&v)[HALF_KV], int k_base, auto masked_tag) {
         constexpr bool MASKED = decltype(masked_tag)::value;
-        const int k_base = kv_first * BLOCK_KV + j * HALF_KV;
-        const uint32_t half_addr = s_addr + (j & 1) * HALF_KV;
-        uint32_t v[HALF_KV];
-#pragma unroll
-        for (int c = 0; c < HALF_KV; c += 32) tmem_ld_32x32b_x32(half_addr + c, *reinterpret_cast<uint32_t(*)[32]>(&v[c]));
-        tmem_ld_wait();
-        // plain variant: the softmax scale (> 0) is folded into the exponent's FMA, the max is taken on the raw scores;
-        // EXTRA variant: scale and ALiBi bias are applied here and the exponent uses a unit multiplier
         if (EXTRA || MASKED) {
           const int k_lim = p.causal ? min(q_pos, len_k - 1) : len_k - 1;                        // last visible key of this row
           const int k_low = (EXTRA && p.window > 0) ? q_pos - p.window + 1 : 0;                  // first visible key
@@ -645,15 +639,39 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             v[i] = __float_as_uint(sc);
           }
         }
-        // (four independent partial maxima / sums: a single running value would be a 64-long dependent chain)
+      };
+      // (four independent partial maxima / sums: a single running value would be a 64-long dependent chain)
+      auto largest = [&](const uint32_t (&v)[HALF_KV]) {
         float mt[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int i = 0; i < HALF_KV; i += 8)
 #pragma unroll
           for (int e = 0; e < 4; ++e)
             mt[e] = fmaxf(fmaxf(mt[e], __uint_as_float(v[i + e])), __uint_as_float(v[i + e + 4]));
-        const float ex_mul = EXTRA ? 1.f : p.scale_log2;
-        const float m_tile = fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3])) * ex_mul;
+        return fmaxf(fmaxf(mt[0], mt[1]), fmaxf(mt[2], mt[3])) * ex_mul;
+      };
+      auto load = [&](uint32_t (&v)[HALF_KV], int j) {
+#pragma unroll
+        for (int c = 0; c < HALF_KV; c += 32)
+          tmem_ld_32x32b_x32(s_addr + (j & 1) * HALF_KV + c, *reinterpret_cast<uint32_t(*)[32]>(&v[c]));
+        tmem_ld_wait();
+      };
+      // the largest score of step j, in the exp2 domain
+      auto row_max = [&](int j, auto masked_tag) {
+        uint32_t v[HALF_KV];
+        load(v, j);
+        visible(v, kv_first * BLOCK_KV + j * HALF_KV, masked_tag);
+        return largest(v);
+      };
+      // one step of 64 keys; two copies of the code, because a branch around the mask alone is turned into predicated
+      // comparisons and selections that every step executes
+      auto step = [&](int j, auto masked_tag) -> bool {
+        const uint32_t half_addr = s_addr + (j & 1) * HALF_KV;
+        uint32_t v[HALF_KV];
+        load(v, j);
+        visible(v, kv_first * BLOCK_KV + j * HALF_KV, masked_tag);
+        const float m_tile = fmaxf(largest(v), m_ahead);
+        m_ahead = -INFINITY;
         // ---- lagging max / rare rescale of the TMEM accumulator
         const float m_new = fmaxf(m_run, m_tile);
         if (j == 0 && !resume) {
@@ -710,14 +728,23 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       };
       // a step needs the mask if its last key is behind what this warp's first row sees, or behind the end of the sequence
       const int k_all = p.causal ? min(q_tile * BLOCK_Q + quarter * 32, len_k - 1) : len_k - 1;
+      auto needs_mask = [&](int j) { return kv_first * BLOCK_KV + j * HALF_KV + HALF_KV - 1 > k_all || (EXTRA && p.window > 0); };
+      // The first reference is the maximum of the whole first key tile: against that of its first half, a row whose largest score is
+      // in the second rounds its largest weight, which is exactly one otherwise (16 x 1024 tokens, heads of 64: error 2.051e-3, 2.035e-3
+      // so, for 189 and 194.5 us; both halves of a tile in one product 193.5, but 2 x 8192 tokens 944 instead of 926).
+      if (n_steps > 1) {
+        ok = __all_sync(0xffffffffu, wait_or_abort(&s_full[2 * t + 1], (phase >> 1) & 1, abort_flag));
+        if (!ok) break;
+        tc_fence_after();
+        m_ahead = needs_mask(1) ? row_max(1, std::true_type{}) : row_max(1, std::false_type{});
+      }
       for (int j = 0; j < n_steps && ok; ++j) {
         const int h = j & 1;
         ok = __all_sync(0xffffffffu, wait_or_abort(&s_full[2 * t + h], (phase >> h) & 1, abort_flag));
         if (!ok) break;
         phase ^= 1u << h;
         tc_fence_after();
-        const bool masked = kv_first * BLOCK_KV + j * HALF_KV + HALF_KV - 1 > k_all || (EXTRA && p.window > 0);
-        ok = masked ? step(j, std::true_type{}) : step(j, std::false_type{});
+        ok = needs_mask(j) ? step(j, std::true_type{}) : step(j, std::false_type{});
       }
       if (!ok) break;
       // ---- the row's maximum and sum go to the output warps

@@ -387,3 +387,26 @@ def test_forward_steps_of_half_a_key_tile(D, Hq, Hkv, lens, causal):
         assert (out[a:a + n].double() - ref).norm() <= 6e-3 * ref.norm()
         torch.testing.assert_close(lse[a:a + n].double(), s.logsumexp(-1).t(), atol=2e-3, rtol=1e-4)
         a += n
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype,unit", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11)])
+@pytest.mark.parametrize("at", [5, 64, 127])
+def test_the_largest_weight_of_the_first_key_tile_is_not_rounded(D, dtype, unit, at):
+    """One key that stands out by up to 7.5 powers of two, in either half of the first key tile, and is the only one with a value:
+    its weight is one against the tile's maximum, so that the result has the rounding of the output and no other."""
+    from colossalai_b200.ops import flash_attn_native as fa
+
+    S, Hq, Hkv = 1024, 32, 8                                                   # more tiles than SMs: two of them per CTA
+    g = torch.Generator(device="cuda").manual_seed(at)
+    q, k, v = (torch.zeros(S, h, D, device="cuda") for h in (Hq, Hkv, Hkv))
+    gap = torch.rand(S, Hq, device="cuda", generator=g) * 7 + 0.5
+    q[..., 0] = gap * D ** 0.5 * 0.6931471805599453
+    k[at, :, 0] = 1.0
+    v[at] = 1.0
+    q, k, v = (t.to(dtype) for t in (q, k, v))
+    out, _ = fa.flash_fwd(q, k, v, 1, False, None)
+    w = torch.exp(q[..., 0].double() * D ** -0.5)
+    ref = (w / (w + S - 1)).unsqueeze(-1).expand(S, Hq, D)
+    # half a unit of the output, and fp32 exponentials (a score's rounding and the function's, 2^-21) and sums
+    assert ((out.double() / ref - 1).abs() <= unit * 1.001 + 4e-6).all()
