@@ -13,6 +13,8 @@
 //     of 128-row multiples around 384 rows did a third more products than their rows, and the tensor pipe was 80 - 87 % busy with
 //     them (two layers of 64 experts, 24576 rows, 2048 x 2816 and 1408 x 2048: forward 403 us, input gradients 412; now 336 and
 //     360, bound by the loads: a tile of 196 rows wants 70 bytes a clock and SM).  The list is built from `offs` at kernel start.
+//     Row tiles are taken in bands (tile_order.h; one expert of 16384 rows, 4096 x 4096, 416 - 448 us without, 356 so; of 65536
+//     1600 - 1850 and 1380 - 1420).
 //     A tile's last rows may be the next group's (or TMA zero fill) and are not stored;
 //   * variable-K mode: every group owns (M / 256) x (N / 256) tiles whose reduction runs over the group's token rows; the
 //     row range of a group must start and end on a multiple of 16, the reduction of one instruction - the dispatch lays groups out
@@ -25,6 +27,7 @@
 
 #include "common.cuh"
 #include "sm100.cuh"
+#include "tile_order.h"
 
 using namespace sm100;
 
@@ -33,7 +36,6 @@ namespace {
 constexpr int UMMA_K = 16;
 constexpr int ROWS_THREADS = 192;      // producer, issuer, four epilogue warps
 constexpr int WGRAD_THREADS = 320;     // .., eight
-constexpr int GROUP_M = 8;
 constexpr int BOX_ROWS = 32;           // token rows of the smaller TMA box: a request takes as long to issue as one of 64 rows
 constexpr int ROWS_BOX = 64;           // of the larger one, variable-M modes (weight gradients: a k-block)
 constexpr int PAIR_M = 256;
@@ -85,16 +87,6 @@ struct Tile {
   int n;                    // variable-M: rows of the tile, a multiple of 16
 };
 
-SM100_DEVICE void raster(int local, int m_blocks, int n_blocks, int& m_blk, int& n_blk) {
-  const int per_band = GROUP_M * n_blocks;
-  const int band = local / per_band;
-  const int first_m = band * GROUP_M;
-  const int gsize = min(m_blocks - first_m, GROUP_M);
-  const int in_band = local - band * per_band;
-  m_blk = first_m + in_band % gsize;
-  n_blk = in_band / gsize;
-}
-
 // bounds[e] .. bounds[e + 1]: the rows of group e; tile_start[e]: number of row tiles of groups < e (variable-M modes).  Both
 // in shared memory, and every role looks its tiles up one ahead: read from memory where a tile begins they were 1300 of the 6300
 // clocks that a tile of a weight gradient took.  `cur` is the last group found: tiles are visited in increasing order by every
@@ -107,7 +99,7 @@ SM100_DEVICE Tile find_tile(int t, int num_tiles, const GroupedParams& p, const 
     const int m_blocks = (p.M + PAIR_M - 1) / PAIR_M, per_group = m_blocks * blocks;
     while (t >= (cur + 1) * per_group) ++cur;
     r.group = cur;
-    raster(t - cur * per_group, m_blocks, blocks, r.m_blk, r.n_blk);
+    cb_tile_order(t - cur * per_group, m_blocks, blocks, r.m_blk, r.n_blk);
     r.row0 = bounds[cur];
     r.row_end = bounds[cur + 1];
     return r;
@@ -116,9 +108,10 @@ SM100_DEVICE Tile find_tile(int t, int num_tiles, const GroupedParams& p, const 
   r.group = cur;
   const int g0 = bounds[cur], end = bounds[cur + 1];
   const int local = t - tile_start[cur] * blocks, row_tiles = tile_start[cur + 1] - tile_start[cur];
-  r.m_blk = local / row_tiles;                                        // a weight block's row tiles are neighbours
+  int row_tile;
+  cb_tile_order(local, row_tiles, blocks, row_tile, r.m_blk);
   const int per = ((end - g0 + row_tiles - 1) / row_tiles + 15) & ~15;    // <= 256, and row_tiles - 1 of them are less than all
-  r.row0 = g0 + (local - r.m_blk * row_tiles) * per;
+  r.row0 = g0 + row_tile * per;
   r.row_end = min(end, r.row0 + per);
   r.n = (r.row_end - r.row0 + 15) & ~15;
   return r;
