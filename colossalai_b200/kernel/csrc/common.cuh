@@ -102,6 +102,12 @@ CB_DEVICE float block_max(float v, float* smem) {
   return warp_max(x);
 }
 
+// a launch's error, taken out of the runtime's state: the next launcher of this library does not hand it on once more
+static inline int cb_launch_error(cudaError_t e) {
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return (int)e;
+}
+
 // A kernel that takes its place while the one before it in the stream still runs, instead of some microseconds after its end: the
 // launch says so, and the kernel begins with `cb_early_start`, which lets the next one do the same and then waits until everything
 // before it is complete and visible.  Nothing global is read or written ahead of it, so the order is that of an ordinary launch.
@@ -122,7 +128,7 @@ static inline int cb_launch_early(void (*kernel)(P...), dim3 grid, dim3 block, s
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return cb_launch_error(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
 static inline int cb_num_sms() {

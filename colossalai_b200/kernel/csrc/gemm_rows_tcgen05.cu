@@ -236,7 +236,7 @@ int launch_rows(const CUtensorMap& tw, const CUtensorMap& tx, const RowsParams& 
   at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return (int)cudaLaunchKernelEx(&cfg, gemm_rows_kernel<T, NT>, tw, tx, p);
+  return cb_launch_error(cudaLaunchKernelEx(&cfg, gemm_rows_kernel<T, NT>, tw, tx, p));
 }
 
 }  // namespace

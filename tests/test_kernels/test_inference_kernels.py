@@ -245,3 +245,25 @@ def test_paged_decode_by_number_of_partitions(n, longest, D):
     ref = iops.paged_decode_attention_ref(q.float()[live], kc.float(), vc.float(), tables[live], lens[live])
     torch.testing.assert_close(out[live].float(), ref, atol=2e-2, rtol=2e-2)      # weights rounded to bf16
     assert not out[[i for i in range(n) if i not in live]].any()
+
+
+def test_a_refused_launch_is_reported_once():
+    """More partitions than a grid has room for: the runtime refuses the launch before anything runs, the launcher says so, and the
+    next launcher of the library does not say it once more."""
+    import ctypes
+
+    from colossalai_b200.kernel import loader
+
+    lib = loader.load("cb200_infer")
+    t = torch.zeros(8, 128, device="cuda", dtype=torch.bfloat16)
+    p, i = loader.ptr(t), torch.zeros(1, device="cuda", dtype=torch.int32)
+    rc = lib.cb_paged_decode_attention(p, p, p, loader.ptr(i), loader.ptr(i), p, p, p, 1, 8, 8, 128, 16, 1, 70000, 32,
+                                       ctypes.c_float(1.0), loader.ptr(None), ctypes.c_int64(1024), ctypes.c_int64(1024), 2, 0,
+                                       loader.stream_ptr())
+    assert rc != 0
+    c = torch.arange(24.0, device="cuda").view(3, 8)
+    o = torch.zeros(2, 1, 8, device="cuda")
+    pos = torch.tensor([2], device="cuda", dtype=torch.int32)
+    assert lib.cb_gather_cos_sin(loader.ptr(c), loader.ptr(c), loader.ptr(pos), loader.ptr(o[0]), loader.ptr(o[1]), 1, 8,
+                                 loader.stream_ptr()) == 0
+    assert torch.equal(o[0, 0], c[2]) and torch.equal(o[1, 0], c[2])
