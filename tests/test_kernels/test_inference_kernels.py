@@ -267,3 +267,21 @@ def test_a_refused_launch_is_reported_once():
     assert lib.cb_gather_cos_sin(loader.ptr(c), loader.ptr(c), loader.ptr(pos), loader.ptr(o[0]), loader.ptr(o[1]), 1, 8,
                                  loader.stream_ptr()) == 0
     assert torch.equal(o[0, 0], c[2]) and torch.equal(o[1, 0], c[2])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Hkv", [9, 12, 16, 31, 32])
+@pytest.mark.parametrize("group", [1, 4])
+@pytest.mark.parametrize("window", [None, 100])
+def test_paged_decode_more_than_eight_kv_heads(dtype, D, Hkv, group, window):
+    """CTAs of four warps, the last of them with one to four heads."""
+    torch.manual_seed(Hkv * 8 + group)
+    n, max_len = 5, 700
+    kc, vc, tables = _mk_cache(n, max_len, 16, Hkv, D, dtype, torch.device("cuda"))
+    lens = torch.tensor([1, 17, 64, 333, 700], device="cuda", dtype=torch.int32)
+    q = torch.randn(n, Hkv * group, D, device="cuda", dtype=dtype)
+    out = iops.paged_decode_attention(q, kc, vc, tables, lens, window=window).double()
+    ref = iops.paged_decode_attention_ref(q.double(), kc, vc, tables, lens, window=window).double()
+    # every head of every sequence: weights rounded to 16 bits (bf16: 2^-9 each), the result once more
+    assert ((out - ref).norm(dim=-1) <= 6e-3 * ref.norm(dim=-1)).all()

@@ -3,7 +3,10 @@ import pytest
 import torch
 from torch import nn
 
-SIZES = [(8, 8), (128, 64), (136, 200), (264, 1096), (1000, 2048), (6144, 1024), (18944, 256), (512, 14336)]
+# CTAs that share a reduction, on 148 SMs: 1, 1, 1, 4 (the last with less), 8, 4, 1, 8; 2, 8 (the last with nothing), the same with a
+# tile that ends inside the width, 4 (17 k-blocks)
+SIZES = [(8, 8), (128, 64), (136, 200), (264, 1096), (1000, 2048), (6144, 1024), (18944, 256), (512, 14336),
+         (8, 512), (1024, 2112), (1000, 2112), (1536, 1088)]
 
 
 @pytest.mark.gpu

@@ -249,7 +249,8 @@ if __name__ == "__main__":
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("T,k,E,H", [(1, 1, 1, 8), (3, 2, 5, 24), (129, 8, 64, 264), (700, 3, 300, 2056), (4097, 2, 3, 64)])
-def test_local_expert_rows(T, k, E, H, dtype):
+@pytest.mark.parametrize("align", [16, 128])
+def test_local_expert_rows(T, k, E, H, dtype, align):
     """Sort, gather, combine and their gradients at the edges: one token, experts without tokens, more choices than one
     round of the sort covers, rows that are no multiple of a warp's or a block's vectors."""
     g = torch.Generator(device="cuda").manual_seed(T)
@@ -257,10 +258,10 @@ def test_local_expert_rows(T, k, E, H, dtype):
     idx = torch.stack([torch.randperm(E, device="cuda", generator=g)[:k] for _ in range(T)])
     idx[idx == 0] = E - 1                                                   # nobody asks for expert 0 (unless E = 1)
     w = torch.rand(T, k, device="cuda", generator=g).requires_grad_()
-    slot, src, counts = mops.sort_choices(idx, E, 128)
+    slot, src, counts = mops.sort_choices(idx, E, align)
     flat = idx.reshape(-1)
     real = torch.bincount(flat, minlength=E)
-    assert torch.equal(counts, (real + 127) // 128 * 128)
+    assert torch.equal(counts, (real + align - 1) // align * align)
     starts = torch.cumsum(counts, 0) - counts
     order = torch.argsort(flat, stable=True)
     want = torch.empty_like(flat)
