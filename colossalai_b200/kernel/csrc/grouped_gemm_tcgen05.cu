@@ -13,8 +13,8 @@
 //     of 128-row multiples around 384 rows did a third more products than their rows, and the tensor pipe was 80 - 87 % busy with
 //     them (two layers of 64 experts, 24576 rows, 2048 x 2816 and 1408 x 2048: forward 403 us, input gradients 412; now 336 and
 //     360, bound by the loads: a tile of 196 rows wants 70 bytes a clock and SM).  The list is built from `offs` at kernel start.
-//     Row tiles are taken in bands (tile_order.h; one expert of 16384 rows, 4096 x 4096, 416 - 448 us without, 356 so; of 65536
-//     1600 - 1850 and 1380 - 1420).
+//     Row tiles are taken in bands (tile_order.h; one expert of 16384 rows, 4096 x 4096, 416 - 448 us without, 351 so; of 65536
+//     1600 - 1850 and 1340 - 1360).
 //     A tile's last rows may be the next group's (or TMA zero fill) and are not stored;
 //   * variable-K mode: every group owns (M / 256) x (N / 256) tiles whose reduction runs over the group's token rows; the
 //     row range of a group must start and end on a multiple of 16, the reduction of one instruction - the dispatch lays groups out

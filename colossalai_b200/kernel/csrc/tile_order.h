@@ -13,9 +13,13 @@
 constexpr int CB_BAND = 8;
 
 CB_TILE_ORDER void cb_tile_order(int local, int row_tiles, int col_blocks, int& row_tile, int& col_block) {
-  const int band = local / (CB_BAND * col_blocks), first = band * CB_BAND;
-  const int rows = row_tiles - first < CB_BAND ? row_tiles - first : CB_BAND;
-  const int in_band = local - band * (CB_BAND * col_blocks);
-  row_tile = first + in_band % rows;
-  col_block = in_band / rows;
+  int first = 0, rows = row_tiles;
+  if (row_tiles > CB_BAND) {                 // (a group of one band, as most are, is spared the division)
+    const int band = local / (CB_BAND * col_blocks);
+    first = band * CB_BAND;
+    local -= first * col_blocks;
+    rows = row_tiles - first < CB_BAND ? row_tiles - first : CB_BAND;
+  }
+  col_block = local / rows;
+  row_tile = first + local - col_block * rows;
 }
