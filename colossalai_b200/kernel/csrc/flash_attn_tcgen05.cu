@@ -21,8 +21,9 @@
 // 64 scores of a row in registers instead of 128 leave room for the output warps).  The issuing warp converged and its
 // descriptors in uniform registers: one thread in a branch took 80 clocks a product, which was the bound of this kernel once the
 // steps were halved.  2 x 4096 tokens, 32 / 8 heads of 128, causal: whole steps 309 us, half steps 450, with the converged
-// issuer 289, with output warps of their own 256; five documents of 8192 tokens together 177 -> 143; 16 x 1024, heads of 64,
-// 188 -> 156.  Two threads per row (16 softmax warps) were 5 - 10 % slower than one.
+// issuer 289, with output warps of their own 256, and 263 with the first reference from both halves of a key tile; five documents of
+// 8192 tokens together 181 -> 156; sixteen of 16384, heads of 64, 223 -> 191.  Two threads per row (16 softmax warps) were 5 - 10 %
+// slower than one.
 // TMEM map (512 columns): [0,128) S_0, [128,256) S_1, then O_0, O_1, D wide each; P_t of a half overwrites the first 32 columns of
 // that half of S_t once its scores are in registers.
 // Shared memory at D = 128: 2 x Q 32 KB + 4 ring slots of 32 KB (at D = 64 2 x 16 KB + 8 x 16 KB) + 4 x 32 rows of the output +
@@ -1246,9 +1247,9 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* out, flo
 //   dQ^T = K^T  (A, MN-major view of the resident K tile) x dS (B, MN-major view of the dS^T tile)      [128 d x 64 q]
 // i.e. five tensor-core GEMMs per (key tile, query tile) pair out of four smem operands, no transposition pass.
 //
-// Warps (16): 0 TMA producer (K, V once; Q_i / dO_i through a 3-stage ring), 1 MMA issuer (converged, as in the forward), 2..3 row statistics (log-sum-exp and
-// delta of the query rows, three tiles ahead), 4..11 softmax (two threads per key row, 32 queries each), 12..15 dQ drain
-// (thread = head-dim lane; 128-byte coalesced fp32 reductions per query row).
+// Warps (16): 0 TMA producer (K, V once; Q_i / dO_i through a 3-stage ring), 1 MMA issuer (converged, as in the forward), 2..3 row
+// statistics (log-sum-exp and delta of the query rows, three tiles ahead), 4..11 softmax (two threads per key row, 32 queries
+// each), 12..15 dQ drain (thread = head-dim lane; 128-byte coalesced fp32 reductions per query row).
 // The issuer runs S^T / dP^T of tile i+1 BEFORE the three accumulation GEMMs of tile i, so the tensor pipe works while
 // the softmax warps are busy (same trick as the forward kernel); P^T / dS^T are double-buffered, so the softmax of tile i+1
 // does not wait for those GEMMs either.
@@ -1532,7 +1533,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     roles_done<BWD_THREADS>();
   } else if (warp < BWD_DRAIN_WARP0) {
     // ================================================================ softmax warps: two threads per key row
-    constexpr int PARTS = BWD_SOFTMAX_WARPS / 4, COLS = BWD_BLOCK_Q / PARTS;
+    constexpr int COLS = BWD_BLOCK_Q / (BWD_SOFTMAX_WARPS / 4);
     const int quarter = warp & 3;
     const int part = (warp - BWD_SOFTMAX_WARP0) >> 2;        // this thread's 32 queries of the tile
     const int r = quarter * 32 + lane;                       // key row inside the tile
@@ -1607,21 +1608,20 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                           (ragged && (kv_tile == (len - 1) / BWD_BLOCK_KV || q_tile == q_tiles - 1));
       ok = masked ? tile(it, q_tile * BWD_BLOCK_Q, std::true_type{}) : tile(it, q_tile * BWD_BLOCK_Q, std::false_type{});
     }
-    // ---- epilogue: half of this key's row of dV (first half of the warps) or scale * dK (second)
+    // ---- epilogue: this key's row of dV (first half of the warps) or of scale * dK (second)
     if (ok && n_iter > 0) ok = warp_wait(acc_full, 0);
     if (ok) {
       tc_fence_after();
       const size_t row = (size_t)kv_row0 + r;
       const size_t ld = (size_t)p.hkv * D;
-      const uint32_t col0 = part < PARTS / 2 ? C::COL_DV : C::COL_DK;
-      const int c_begin = part % (PARTS / 2) * (D / (PARTS / 2));
-      const float mul = part < PARTS / 2 ? 1.f : p.scale;
-      float* acc_row = p.dk_acc != nullptr ? (part < PARTS / 2 ? p.dv_acc : p.dk_acc) + (row * ld + (size_t)kv_head * D) : nullptr;
-      uint8_t* base = reinterpret_cast<uint8_t*>(part < PARTS / 2 ? p.dv : p.dk) + (row * ld + (size_t)kv_head * D) * 2;
+      const uint32_t col0 = part == 0 ? C::COL_DV : C::COL_DK;
+      const float mul = part == 0 ? 1.f : p.scale;
+      float* acc_row = p.dk_acc != nullptr ? (part == 0 ? p.dv_acc : p.dk_acc) + (row * ld + (size_t)kv_head * D) : nullptr;
+      uint8_t* base = reinterpret_cast<uint8_t*>(part == 0 ? p.dv : p.dk) + (row * ld + (size_t)kv_head * D) * 2;
       // NOTE: tcgen05.ld is warp-collective (.sync.aligned): every lane runs the loads, only the STORES are predicated on
       // the key being inside the sequence (a ragged last tile leaves some lanes of a warp without a row)
 #pragma unroll 1
-      for (int c = c_begin; c < c_begin + D / (PARTS / 2); c += 32) {
+      for (int c = 0; c < D; c += 32) {
         uint32_t v[32];
         __syncwarp();
         tmem_ld_32x32b_x32(tmem_base + lane_addr + col0 + c, v);

@@ -14,6 +14,9 @@
 // 39.2, 4096 x 14336 22.9 and 20.4, 32000 x 4096 45.5 and 43.0, 2048 x 8192 13.0 and 8.8, 1536 x 1024 3.6 and 3.7; 32 rows 9.9 / 8.9,
 // 12.4 / 12.0, 41.6 / 39.8, 27.3 / 21.3, 45.8 / 44.3, 13.1 / 9.5, 3.7 / 4.0.  Three stages and four CTAs on an SM were slower for deep
 // matrices (4096 x 14336 22.4).  A decode step of four layers of 4096 x 14336, 16 sequences: 530 us with cuBLAS, 509.
+// There is no lower bound on the matrix: alone cuBLAS is ahead by 0.1 - 0.3 us at 1536 x 1024, but in a step the early launches are
+// worth more.  Two layers of 1024 x 2816, 5 sequences, with cuBLAS for the projections 103 us, with this 87; four of them, one
+// sequence 198 and 141.
 #include "checked_id.h"
 #include "common.cuh"
 #include "sm100.cuh"

@@ -578,7 +578,7 @@ extern "C" {
 // transpose_b != 0: w [E, N, K] and y = x w[e]^T (forward);  transpose_b == 0: w [E, K, N] and y = x w[e] (dgrad with
 // the forward weight [E, K(out), N(in)]).  y [total_rows, N].  Requirements: contiguous w, K % 8 == 0, N % 8 == 0,
 // 16-byte aligned pointers, E <= 512; transpose_b == 0 additionally needs K % 128 == 0 (a k-block must not straddle
-// two experts' weights).
+// two experts' weights: blocks of 64 rows would allow K % 64, which no caller has asked for and no test has run).
 int cb_grouped_gemm(const void* x, const void* w, void* y, const int* offs, int E, int total_rows, int N, int K, int ldx,
                     int ldy, int transpose_b, int dtype, cudaStream_t stream) {
   if (E <= 0 || total_rows <= 0 || N <= 0) return 0;

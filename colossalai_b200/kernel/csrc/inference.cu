@@ -780,7 +780,8 @@ int cb_rope_kv_cache_write(void* q, void* k, const void* v, void* k_cache, void*
 }
 
 int cb_decode_num_splits(int num_seqs, int kv_heads, int max_len, int* part_len_out) {
-  // one CTA (up to 8 warps, one per kv head) per SM: aim at >= 2 waves of CTAs, partitions of >= 64 tokens
+  // aim at >= 2 waves of CTAs, partitions of >= 64 tokens.  Counted in CTAs of eight kv heads, also where four share one
+  // (DEC_MMA_WARPS): the partitions, and with them a sequence's bits, are what they were.
   const int ctas_per_split = num_seqs * ((kv_heads + 7) / 8);
   const int target = 2 * cb_num_sms();
   int splits = (target + ctas_per_split - 1) / ctas_per_split;

@@ -49,8 +49,8 @@ def _use_fused(x: torch.Tensor, num_experts: int, ep_group) -> bool:
 
 
 def _aligned_rows(x: torch.Tensor) -> bool:
-    """Lay the expert-grouped rows out with every expert's range padded with zero rows (to 16, or to 128 by index operations): the native grouped
-    weight-gradient GEMM then needs no re-layout pass (moe/grouped_gemm.py)."""
+    """Lay the expert-grouped rows out with every expert's range padded with zero rows (to 16, or to 128 by index
+    operations): the native grouped weight-gradient GEMM then needs no re-layout pass (moe/grouped_gemm.py)."""
     return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
             and os.environ.get("CB200_GROUPED_GEMM", "native") == "native"
             and torch.cuda.get_device_capability(x.device)[0] == 10)
@@ -98,8 +98,8 @@ def moe_forward(x: torch.Tensor, topk_w: torch.Tensor, topk_idx: torch.Tensor, e
     if ep == 1 and T > 0 and use_native(x) and _aligned_rows(x) and rows_ok(x) and num_experts <= SORT_EXPERTS \
             and plain_call(x, topk_w, topk_idx):
         # all experts here: the rows are sorted, gathered, combined and differentiated by kernels of their own, without a
-        # host synchronisation (`ops/moe.py`); the index operations below remain for CPU tensors, 32-bit rows, more experts than the sort has counters for, and for calls
-        # that functorch, forward mode or a mode watches
+        # host synchronisation (`ops/moe.py`); the index operations below remain for CPU tensors, 32-bit rows, more experts
+        # than the sort has counters for, and for calls that functorch, forward mode or a mode watches
         slot, src, counts = sort_choices(topk_idx, num_experts, ROW_ALIGN)
         counts.cb200_aligned = True
         ys = experts(TakeRows.apply(x, slot, src, k), counts)

@@ -25,7 +25,8 @@ from ..parallel import comm
 __all__ = ["EPWorkspace", "ep_workspace", "available", "dispatch", "combine", "moe_forward_fused"]
 
 _lib = None
-ALIGN = 128     # row alignment of every local expert's segment in the receive layout (a multiple of the 16 rows that the grouped wgrad GEMM wants)
+# row alignment of every local expert's segment in the receive layout (a multiple of the 16 rows that the grouped wgrad GEMM wants)
+ALIGN = 128
 _workspaces: Dict[tuple, "EPWorkspace"] = {}
 
 
@@ -170,7 +171,8 @@ def _push_assign(ws: EPWorkspace, x: torch.Tensor, idx32: torch.Tensor) -> EPCon
     local_counts = torch.empty(n_local, dtype=torch.int64, device=dev)
     local_offs = torch.empty(n_local, dtype=torch.int32, device=dev)
     real_counts = torch.empty(n_local, dtype=torch.int32, device=dev)
-    local_counts.cb200_aligned = True       # grouped_linear: segments start / end on multiples of 128 (16 is asked for), padding is zero
+    # grouped_linear: segments start / end on multiples of 128 (16 is asked for), padding is zero
+    local_counts.cb200_aligned = True
     meta = torch.zeros(2, dtype=torch.int32, device=dev)
     pos = torch.empty(T * K, dtype=torch.int32, device=dev)
     ws.check_overflow()
