@@ -253,18 +253,18 @@ struct ScanParams {
 
 // Two kernels.  `scan_prepare_kernel` is elementwise and fully parallel: activations, unit norms, decays and write
 // strengths of every token in fp32 into a workspace whose rows are padded to the kernel's key width (q, k: zeros;
-// decay: ones) and value rows to a multiple of SCAN_COLS.  `state_scan_kernel` is the recurrence: a CTA owns SCAN_COLS
-// value columns of one (sequence, head); a lane holds a tile of S, RP rows x SCAN_CPL columns, in registers, so that a value
-// of q, k or the decay that is read from shared memory serves SCAN_CPL columns; PARTS adjacent lanes share the rows of a
+// decay: ones) and value rows to a multiple of SCAN_COLS.  `state_scan_kernel` is the recurrence: a CTA owns 8 x CPL
+// value columns of one (sequence, head); a lane holds a tile of S, RP rows x CPL columns, in registers, so that a value
+// of q, k or the decay that is read from shared memory serves CPL columns; PARTS adjacent lanes share the rows of a
 // column group, and S^T k and S^T q are partial sums per lane joined by shuffles in a fixed order.
 // The workspace rows of SCAN_TOK_TILE tokens arrive by cp.async in a ring of stages while the previous tile is walked (decay
 // mode has three, so that one barrier per tile is enough).
-// Bound: the serial chain of a sequence, shared-memory reads (q and k once per SCAN_CPL columns) and fp32 issue, none of them
-// alone.  12000 tokens in eight uneven sequences, 16 heads, 128 x 128, decay mode: recurrence 741 -> 594 us.  Holding S divided
+// Bound: the serial chain of a sequence, shared-memory reads (q and k once per CPL columns) and fp32 issue, none of them
+// alone (three units on an SM: its fp32 pipe 57 % busy, half of the issue slots; a unit's warp waits 64 % of its time when alone).  12000 tokens in eight uneven sequences, 16 heads, 128 x 128, decay mode: recurrence 741 -> 594 us.  Holding S divided
 // by its decay's powers inside a tile of eight tokens (505 us) made the bits depend on how a sequence is cut into portions, and
 // turned infinite values into NaN.
-constexpr int SCAN_CPL = 4;            // value columns per lane
-constexpr int SCAN_COLS = 32;          // value columns per CTA
+constexpr int SCAN_CPL = 4;            // value columns per lane (fewer: scan_columns)
+constexpr int SCAN_COLS = 32;          // value columns per CTA then, and what value rows are padded to
 
 // Two rows of a column of S: one register pair for the instructions that do two fp32 operations (long portions), or two numbers
 // that a row's load fills as they come - packing them holds up the state's loads, and those are what a short portion is.  The
@@ -272,8 +272,12 @@ constexpr int SCAN_COLS = 32;          // value columns per CTA
 struct alignas(8) ScanTwo {
   float a, b;
 };
+template <int N> struct alignas(4 * N) ScanVec {
+  float x[N];
+};
 
-template <int DK, int MODE, bool SHORT> struct ScanTile {
+template <int DK, int MODE, bool SHORT, int CPL = SCAN_CPL> struct ScanTile {
+  static constexpr int COLS = 8 * CPL;                                  // value columns of a CTA
   // Lanes that share the rows of a column group.  More lanes are shorter steps for each and more warps to hide them behind, at
   // more shuffles and reads of the values.  Decay mode, 16 heads, 12000 tokens, with 8 and with 16 lanes: 128 x 128, one
   // sequence 2.69 and 1.70 ms, eight uneven ones 802 and 701 us; 64 x 64, eight sequences 385 and 278 us.
@@ -284,9 +288,10 @@ template <int DK, int MODE, bool SHORT> struct ScanTile {
   static constexpr int RP = DK / PARTS;                                 // rows per lane
   static constexpr int RPP = RP == 4 ? 4 : RP + 4;                      // a lane's rows in shared memory start this far apart:
   static constexpr int DKP = PARTS * RPP;                               // the 16-byte reads of 8 lanes hit different banks
-  static constexpr int THREADS = PARTS * SCAN_COLS / SCAN_CPL;
+  static constexpr int THREADS = PARTS * COLS / CPL;
   static constexpr int TPI = THREADS / (DK / 4);                        // tokens that one round of copies covers
-  static constexpr int TILE = SHORT && TPI < 4 ? 4 : SCAN_TOK_TILE;     // tokens per stage
+  // tokens per stage: no fewer than exchange their sums together (more than eight: 64 x 64 8 % faster, 128 x 128 2 % slower)
+  static constexpr int TILE = SHORT ? (TPI < 4 ? 4 : SCAN_TOK_TILE) : PARTS / CPL > SCAN_TOK_TILE ? PARTS / CPL : SCAN_TOK_TILE;
   // Units that an SM is to hold at a time, by their registers.  A long portion: four tokens' reads want more than 128 of a lane,
   // and at 255 an SM holds two of the 128 wide units, so that eight sequences take two rounds (either 13 % slower).  A short
   // one: as much of the states on its way as can be.  256 decoded tokens, 16 heads x 128 x 128, decay / rows / delta mode: 241 /
@@ -296,7 +301,7 @@ template <int DK, int MODE, bool SHORT> struct ScanTile {
   static constexpr int BLOCKS = SHORT ? SHORT_BLOCKS : LONG_BLOCKS;
   static constexpr int STAGES = MODE == SCAN_DECAY && !SHORT ? 3 : 2;
   static constexpr int NROW = MODE == SCAN_DELTA || MODE == SCAN_ROWS ? 3 : 2;          // q, k, decay rows
-  static constexpr int TOKEN = NROW * DKP + SCAN_COLS + 4;              // floats per token: rows, values, scalars
+  static constexpr int TOKEN = NROW * DKP + COLS + 4;                   // floats per token: rows, values, scalars
   using Pair = typename std::conditional<SHORT, ScanTwo, uint64_t>::type;
   struct alignas(16) Quad { Pair x, y; };                               // four rows as they lie in shared memory
 };
@@ -582,71 +587,74 @@ CB_DEVICE void scan_unit(const ScanParams& p, int nseq, int units, int sms, int&
   s = __ffs(__ballot_sync(0xffffffffu, lane < nseq && place == want)) - 1;
 }
 
-template <int DK, int MODE, bool SHORT>
-__global__ void __launch_bounds__(ScanTile<DK, MODE, SHORT>::THREADS, ScanTile<DK, MODE, SHORT>::BLOCKS)
+template <int DK, int MODE, bool SHORT, int CPL>
+__global__ void __launch_bounds__(ScanTile<DK, MODE, SHORT, CPL>::THREADS, ScanTile<DK, MODE, SHORT, CPL>::BLOCKS)
 state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
-  using Tile = ScanTile<DK, MODE, SHORT>;
+  using Tile = ScanTile<DK, MODE, SHORT, CPL>;
   constexpr int PARTS = Tile::PARTS, RP = Tile::RP, RPP = Tile::RPP, DKP = Tile::DKP, TILE = Tile::TILE;
-  constexpr int THREADS = Tile::THREADS, SPLIT = Tile::SPLIT;
+  constexpr int THREADS = Tile::THREADS, SPLIT = Tile::SPLIT, COLS = Tile::COLS;
   static_assert(SPLIT == 1 || MODE == SCAN_DECAY, "the delta rule's first sum is not split");
+  static_assert((CPL == SCAN_CPL || (CPL < SCAN_CPL && MODE == SCAN_DECAY && !SHORT)) && PARTS % CPL == 0, "");
   constexpr bool ROWS = MODE == SCAN_DELTA || MODE == SCAN_ROWS;        // decay rows beside q and k
   constexpr int NROW = Tile::NROW, STAGES = Tile::STAGES;
   constexpr int STAGE = TILE * Tile::TOKEN;                             // floats per stage
-  constexpr int NTOK = PARTS / SCAN_CPL;                                // tokens whose sums are exchanged together
+  constexpr int NTOK = PARTS / CPL;                                     // tokens whose sums are exchanged together
   constexpr unsigned ALL = 0xffffffffu;
   using P = typename Tile::Pair;                                        // two rows of a column
   using Quad = typename Tile::Quad;
   extern __shared__ __align__(16) float scan_smem[];
-  const int vblocks = w.VP / SCAN_COLS;
+  const int vblocks = w.VP / COLS;
   int s, unit;
   scan_unit(p, nseq, p.heads * vblocks, sms, s, unit);
   const int h = unit / vblocks, vb = unit % vblocks;
   const int t0 = p.cu_q[s], t1 = p.cu_q[s + 1];
   if (t0 >= t1) return;
   const int part = threadIdx.x % PARTS;
-  const int c0 = threadIdx.x / PARTS * SCAN_CPL;               // first of the lane's columns inside the CTA's block
-  const int j0 = vb * SCAN_COLS + c0;
+  const int c0 = threadIdx.x / PARTS * CPL;                    // first of the lane's columns inside the CTA's block
+  const int j0 = vb * COLS + c0;
   const int hk = h / (p.heads / p.qk_heads);
   const int dim = p.dim, vdim = p.vdim;
   const int r0 = part * RP, r0p = part * RPP;
   float* Sg = p.state + ((int64_t)p.slots[s] * p.heads + h) * dim * vdim;
-  const bool vec = vdim % 4 == 0 && j0 < vdim;                 // whole quads of columns, 16-byte aligned
+  const bool vec = vdim % CPL == 0 && j0 < vdim;               // all of the lane's columns, aligned
   const bool carried = p.ctx_len[s] > 0;
   // Pairs of neighbouring ROWS share an instruction: q, k and the decays arrive from shared memory as such pairs, and only the
-  // token's SCAN_CPL values are duplicated.
-  P S[RP / 2][SCAN_CPL];
+  // token's CPL values are duplicated.
+  P S[RP / 2][CPL];
 #pragma unroll
   for (int i = 0; i < RP; i += 2) {
-    float x[2][SCAN_CPL];
+    float x[2][CPL];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const bool row = carried && r0 + i + e < dim;
       const float* src = Sg + (int64_t)(r0 + i + e) * vdim + j0;
       if (vec) {
-        const float4 y = row ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
-        x[e][0] = y.x; x[e][1] = y.y; x[e][2] = y.z; x[e][3] = y.w;
+        ScanVec<CPL> y{};
+        if (row) y = *reinterpret_cast<const ScanVec<CPL>*>(src);
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) x[e][c] = y.x[c];
       } else {
 #pragma unroll
-        for (int c = 0; c < SCAN_CPL; ++c) x[e][c] = (row && j0 + c < vdim) ? src[c] : 0.f;
+        for (int c = 0; c < CPL; ++c) x[e][c] = (row && j0 + c < vdim) ? src[c] : 0.f;
       }
     }
 #pragma unroll
-    for (int c = 0; c < SCAN_CPL; ++c) S[i / 2][c] = pair_of<P>(x[0][c], x[1][c]);
+    for (int c = 0; c < CPL; ++c) S[i / 2][c] = pair_of<P>(x[0][c], x[1][c]);
   }
   const float hd = MODE == SCAN_DECAY ? p.head_decay[h] : 0.f;
   const float skip = (MODE == SCAN_GATED && p.head_decay != nullptr) ? p.head_decay[h] : 0.f;
 
   // A thread copies the same 16-byte piece of every (THREADS / pieces)-th token: its addresses only step, which keeps the
   // copies to three instructions each (with an address computed per copy they were a tenth of what the kernel issued).
-  constexpr int CH = DK / 4, TPI = Tile::TPI, VCH = SCAN_COLS / 4, VPI = THREADS / VCH;
+  constexpr int CH = DK / 4, TPI = Tile::TPI, VCH = COLS / 4, VPI = THREADS / VCH;
   static_assert(THREADS % CH == 0 && TPI <= TILE && THREADS % VCH == 0, "");
   const int qt = threadIdx.x / CH, qc = (threadIdx.x % CH) * 4, vt = threadIdx.x / VCH, vc = (threadIdx.x % VCH) * 4;
-  const int qdst = qt * DKP + qc / RP * RPP + qc % RP, vdst = NROW * TILE * DKP + vt * SCAN_COLS + vc;
+  const int qdst = qt * DKP + qc / RP * RPP + qc % RP, vdst = NROW * TILE * DKP + vt * COLS + vc;
   const int64_t qstep = (int64_t)p.qk_heads * DK, gstep = (int64_t)p.heads * DK, vstep = (int64_t)p.heads * w.VP;
   const float* qsrc = w.q + (t0 + qt) * qstep + hk * DK + qc;
   const float* ksrc = w.k + (t0 + qt) * qstep + hk * DK + qc;
   const float* gsrc = ROWS ? w.g + (t0 + qt) * gstep + h * DK + qc : nullptr;
-  const float* vsrc = w.v + (t0 + vt) * vstep + h * w.VP + vb * SCAN_COLS + vc;
+  const float* vsrc = w.v + (t0 + vt) * vstep + h * w.VP + vb * COLS + vc;
   auto load_tile = [&](int stage, int tb) {      // tiles are asked for in order
     float* base = scan_smem + stage * STAGE;
     const int nt = max(min(TILE, t1 - tb), 0);
@@ -664,28 +672,34 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
     float* sv = base + NROW * TILE * DKP;
 #pragma unroll
     for (int i = 0; i < TILE; i += VPI) {
-      if (vt + i < nt) cp_async16f(base + vdst + i * SCAN_COLS, vsrc);
+      if (vt + i < nt) cp_async16f(base + vdst + i * COLS, vsrc);
       vsrc += (VPI < TILE ? VPI : TILE) * vstep;
     }
     if (MODE == SCAN_DELTA && threadIdx.x < nt)
-      sv[TILE * SCAN_COLS + threadIdx.x] = w.beta[(int64_t)(tb + threadIdx.x) * p.heads + h];
+      sv[TILE * COLS + threadIdx.x] = w.beta[(int64_t)(tb + threadIdx.x) * p.heads + h];
     if (MODE == SCAN_GATED && threadIdx.x < nt)
-      cp_async16f(sv + TILE * SCAN_COLS + threadIdx.x * 4,
+      cp_async16f(sv + TILE * COLS + threadIdx.x * 4,
                   w.gw + ((int64_t)(tb + threadIdx.x) * p.heads + h) * 4);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // Sums over the lanes of a column group.  `fold` leaves column (part & 3) of a lane's four partial sums joined over its
-  // quad of lanes: (part 0 + part 1) + (part 2 + part 3); quads are joined afterwards in ascending order.
+  // Sums over the lanes of a column group: parts 1 apart, then 2, then 4 and so on, whatever the lane's columns are.  `fold` leaves
+  // column (part % CPL) of a lane's partial sums joined over the CPL lanes around it.
   const bool b0 = part & 1, b1 = part & 2;
-  auto fold = [&](const float (&o)[SCAN_CPL]) -> float {
-    const float x = (b0 ? o[1] : o[0]) + __shfl_xor_sync(ALL, b0 ? o[0] : o[1], 1);      // column part & 1
-    const float y = (b0 ? o[3] : o[2]) + __shfl_xor_sync(ALL, b0 ? o[2] : o[3], 1);      // column 2 + (part & 1)
-    return (b1 ? y : x) + __shfl_xor_sync(ALL, b1 ? x : y, 2);
+  auto fold = [&](const float (&o)[CPL]) -> float {
+    float x[CPL];
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) x[c] = o[c];
+#pragma unroll
+    for (int m = CPL / 2, bit = 1; m >= 1; m /= 2, bit *= 2) {
+      const bool up = part & bit;
+#pragma unroll
+      for (int n = 0; n < m; ++n) x[n] = (up ? x[2 * n + 1] : x[2 * n]) + __shfl_xor_sync(ALL, up ? x[2 * n] : x[2 * n + 1], bit);
+    }
+    return x[0];
   };
-  auto join_quads = [&](float v) -> float {
-    if (PARTS >= 8) v += __shfl_xor_sync(ALL, v, 4);
-    if (PARTS >= 16) v += __shfl_xor_sync(ALL, v, 8);
-    if (PARTS >= 32) v += __shfl_xor_sync(ALL, v, 16);
+  auto join_rest = [&](float v) -> float {
+#pragma unroll
+    for (int bit = CPL; bit < PARTS; bit *= 2) v += __shfl_xor_sync(ALL, v, bit);
     return v;
   };
 
@@ -704,11 +718,13 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
     const float* sk = sq + TILE * DKP;
     const float* sg = sk + TILE * DKP;
     const float* sv = sq + NROW * TILE * DKP;
-    const float* sbeta = sv + TILE * SCAN_COLS;
-    // one token: the lane's part of S is advanced; returns column (part & 3) of the read-out joined over the lane's quad
+    const float* sbeta = sv + TILE * COLS;
+    // one token: the lane's part of S is advanced; returns column (part % CPL) of the read-out, folded
     auto advance = [&](int tt) -> float {
-      const float4 v4 = *reinterpret_cast<const float4*>(sv + tt * SCAN_COLS + c0);
-      float u[SCAN_CPL] = {v4.x, v4.y, v4.z, v4.w};
+      const ScanVec<CPL> value = *reinterpret_cast<const ScanVec<CPL>*>(sv + tt * COLS + c0);
+      float u[CPL];
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) u[c] = value.x[c];
       const float* kq = sk + tt * DKP + r0p;
       const float* qq = sq + tt * DKP + r0p;
       const float* gq = sg + tt * DKP + r0p;
@@ -717,10 +733,10 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
         dec = sbeta[tt * 4];
         const float wr = sbeta[tt * 4 + 1];
 #pragma unroll
-        for (int c = 0; c < SCAN_CPL; ++c) u[c] *= wr;
+        for (int c = 0; c < CPL; ++c) u[c] *= wr;
       }
-      if (MODE == SCAN_DELTA) {
-        P a2[SCAN_CPL] = {};
+      if constexpr (MODE == SCAN_DELTA) {          // (CPL is four)
+        P a2[CPL] = {};
 #pragma unroll
         for (int i = 0; i < RP; i += 4) {
           const Quad g4 = *reinterpret_cast<const Quad*>(gq + i);
@@ -729,25 +745,25 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
 #pragma unroll
           for (int e = 0; e < 2; ++e)
 #pragma unroll
-            for (int c = 0; c < SCAN_CPL; ++c) {
+            for (int c = 0; c < CPL; ++c) {
               P& x = S[i / 2 + e][c];
               x = mul2(x, gr[e]);
               a2[c] = fma2(x, kr[e], a2[c]);
             }
         }
-        float a[SCAN_CPL];
+        float a[CPL];
 #pragma unroll
-        for (int c = 0; c < SCAN_CPL; ++c) { const float2 h = halves(a2[c]); a[c] = h.x + h.y; }
+        for (int c = 0; c < CPL; ++c) { const float2 h = halves(a2[c]); a[c] = h.x + h.y; }
         // every lane of a column group corrects one column, then collects the quad's four
-        const float mine = sbeta[tt] * (sv[tt * SCAN_COLS + c0 + (part & 3)] - join_quads(fold(a)));
+        const float mine = sbeta[tt] * (sv[tt * COLS + c0 + (part & 3)] - join_rest(fold(a)));
         const float nb = __shfl_xor_sync(ALL, mine, 1);
         const float lo = b0 ? nb : mine, hi = b0 ? mine : nb;
         const float xl = __shfl_xor_sync(ALL, lo, 2), xh = __shfl_xor_sync(ALL, hi, 2);
         u[0] = b1 ? xl : lo; u[1] = b1 ? xh : hi; u[2] = b1 ? lo : xl; u[3] = b1 ? hi : xh;
       }
-      P o2[SPLIT][SCAN_CPL] = {}, u2[SCAN_CPL];
+      P o2[SPLIT][CPL] = {}, u2[CPL];
 #pragma unroll
-      for (int c = 0; c < SCAN_CPL; ++c) u2[c] = pair_of<P>(u[c], u[c]);
+      for (int c = 0; c < CPL; ++c) u2[c] = pair_of<P>(u[c], u[c]);
       const P dec2 = pair_of<P>(dec, dec);
 #pragma unroll
       for (int i = 0; i < RP; i += 4) {
@@ -759,29 +775,29 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
 #pragma unroll
         for (int e = 0; e < 2; ++e)
 #pragma unroll
-          for (int c = 0; c < SCAN_CPL; ++c) {
+          for (int c = 0; c < CPL; ++c) {
             P& x = S[i / 2 + e][c];
             x = MODE == SCAN_DELTA ? fma2(kr[e], u2[c], x) : fma2(gr[e], x, mul2(kr[e], u2[c]));
             P& y = o2[i / (RP / SPLIT)][c];
             y = fma2(x, qr[e], y);
           }
       }
-      float o[SCAN_CPL];
+      float o[CPL];
 #pragma unroll
-      for (int c = 0; c < SCAN_CPL; ++c) {
+      for (int c = 0; c < CPL; ++c) {
         const float2 h = halves(o2[0][c]);
         o[c] = h.x + h.y;
         if (SPLIT == 2) { const float2 g = halves(o2[SPLIT - 1][c]); o[c] += g.x + g.y; }
       }
       return fold(o);
     };
-    auto emit = [&](int tt, float o) {           // column (part & 3) of token tt's read-out
-      if (MODE == SCAN_GATED) o = fmaf(o, sbeta[tt * 4 + 2], skip * sv[tt * SCAN_COLS + c0 + (part & 3)]);
-      const int j = j0 + (part & 3);
+    auto emit = [&](int tt, float o) {           // column (part % CPL) of token tt's read-out
+      if (MODE == SCAN_GATED) o = fmaf(o, sbeta[tt * 4 + 2], skip * sv[tt * COLS + c0 + part % CPL]);
+      const int j = j0 + part % CPL;
       if (j < vdim) p.out[(int64_t)(tb + tt) * ((int64_t)p.heads * vdim) + h * vdim + j] = o;
     };
-    // NTOK tokens at a time: only S ties them together, so their loads and sums overlap; the quads exchange their sums so
-    // that quad n ends up with token n's total (the same pairs in the same order as one token alone takes: the result does
+    // NTOK tokens at a time: only S ties them together, so their loads and sums overlap; the folds exchange their sums so
+    // that fold n ends up with token n's total (the same pairs in the same order as one token alone takes: the result does
     // not depend on how a portion falls into groups)
     int tt = 0;
 #pragma unroll 2
@@ -790,53 +806,70 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
 #pragma unroll
       for (int n = 0; n < NTOK; ++n) v[n] = advance(tt + n);
 #pragma unroll
-      for (int m = NTOK / 2, bit = 4; m >= 1; m /= 2, bit *= 2) {
+      for (int m = NTOK / 2, bit = CPL; m >= 1; m /= 2, bit *= 2) {
         const bool up = part & bit;
 #pragma unroll
         for (int n = 0; n < m; ++n) v[n] = (up ? v[2 * n + 1] : v[2 * n]) + __shfl_xor_sync(ALL, up ? v[2 * n] : v[2 * n + 1], bit);
       }
-      emit(tt + part / SCAN_CPL, v[0]);
+      emit(tt + part / CPL, v[0]);
     }
 #pragma unroll 1
     for (; tt < nt; ++tt) {
-      const float o = join_quads(advance(tt));
-      if (part < SCAN_CPL) emit(tt, o);
+      const float o = join_rest(advance(tt));
+      if (part < CPL) emit(tt, o);
     }
     if (STAGES == 2) __syncthreads();           // this stage may be refilled in the next pass
   }
 #pragma unroll
   for (int i = 0; i < RP; i += 2) {
-    float2 x[SCAN_CPL];
+    float2 x[CPL];
 #pragma unroll
-    for (int c = 0; c < SCAN_CPL; ++c) x[c] = halves(S[i / 2][c]);
+    for (int c = 0; c < CPL; ++c) x[c] = halves(S[i / 2][c]);
 #pragma unroll
     for (int e = 0; e < 2; ++e)
       if (r0 + i + e < dim) {
         float* dst = Sg + (int64_t)(r0 + i + e) * vdim + j0;
         if (vec) {
-          *reinterpret_cast<float4*>(dst) = e ? make_float4(x[0].y, x[1].y, x[2].y, x[3].y) : make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
+          ScanVec<CPL> y;
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) y.x[c] = e ? x[c].y : x[c].x;
+          *reinterpret_cast<ScanVec<CPL>*>(dst) = y;
         } else {
 #pragma unroll
-          for (int c = 0; c < SCAN_CPL; ++c)
+          for (int c = 0; c < CPL; ++c)
             if (j0 + c < vdim) dst[c] = e ? x[c].y : x[c].x;
         }
       }
   }
 }
 
-template <int DK, int MODE, bool SHORT> int launch_scan_dk(const ScanParams& p, const ScanWork& w, int nseq, cudaStream_t st) {
-  using Tile = ScanTile<DK, MODE, SHORT>;
+template <int DK, int MODE, bool SHORT, int CPL = SCAN_CPL> int launch_scan_dk(const ScanParams& p, const ScanWork& w, int nseq, cudaStream_t st) {
+  using Tile = ScanTile<DK, MODE, SHORT, CPL>;
   const size_t smem = (size_t)Tile::STAGES * Tile::TILE * Tile::TOKEN * sizeof(float);
-  auto kern = state_scan_kernel<DK, MODE, SHORT>;
+  auto kern = state_scan_kernel<DK, MODE, SHORT, CPL>;
   static CbDeviceAttr attr;
   if (const int e = cb_allow_smem(attr, kern, smem, true)) return e;
-  kern<<<p.heads * (w.VP / SCAN_COLS) * nseq, Tile::THREADS, smem, st>>>(p, w, nseq, cb_num_sms());
+  kern<<<p.heads * (w.VP / Tile::COLS) * nseq, Tile::THREADS, smem, st>>>(p, w, nseq, cb_num_sms());
   return CB_LAUNCH_CHECK();
 }
 
 // workspace floats for `tokens` tokens: q, k rows, decay rows (delta rule, rows mode), write strengths (delta rule), value rows
 static inline int scan_dk(int dim) { return dim <= 16 ? 16 : dim <= 32 ? 32 : dim <= 64 ? 64 : dim <= 128 ? 128 : 256; }
 static inline int scan_vp(int vdim) { return (vdim + SCAN_COLS - 1) / SCAN_COLS * SCAN_COLS; }
+
+// Decay mode, long portions of 64 and 128 channels: columns of a lane.  With four, columns share what is read of q and k, which is
+// what many units on an SM run out of; but one unit alone takes a token in 265 clocks, most of them waits, and two columns (170) or
+// one (120 at 64 channels) in as many more CTAs wait less.  So fewer columns where the longest sequence's walk is what the call
+// takes: where it is 5 / 4 of the tokens that an SM walks on average, counted with four; and one column where even then every CTA has an
+// SM to itself.  Four / two / one columns, us, prepare kernel included: 1 x 12000 tokens of 16 heads x 128 x 128 (ratio 2.3) 1674 / 1076 / 1617,
+// 2 x 6000 (1.2 to 1.4) 1056 / 1000 / 1654, 4 x 2000 (0.7) 497 / 544 / 949, 8 x 1500 695 / 814 / 1326; 1 x 4534 of 8 heads (128 CTAs of one column) 622 / 396 /
+// 353; 1 x 12000 of 16 heads x 64 x 64 1166 / 691 / 478; 2 x 3000 of 8 heads x 64 x 64 359 / 216 / 152; 1 x 2602 of 4 heads x 64 x 128 253 / 151 / 106;
+// 16 x 500 of 4 heads x 64 x 96 (1.1) 101 / 87 / 106.  The bits are the same.
+static inline int scan_columns(const ScanWork& w, int heads, int nseq, int64_t tokens, int max_q) {
+  const int64_t sms = cb_num_sms();
+  if ((w.DK != 64 && w.DK != 128) || 4 * (int64_t)max_q * sms < 5 * tokens * heads * (w.VP / SCAN_COLS)) return SCAN_CPL;
+  return (int64_t)nseq * heads * (w.VP / 8) <= sms ? 1 : 2;
+}
 
 template <int MODE, typename T>
 int launch_scan(const ScanParams& p, float* work, int64_t tokens, int nseq, int max_q, cudaStream_t st) {
@@ -867,6 +900,11 @@ int launch_scan(const ScanParams& p, float* work, int64_t tokens, int nseq, int 
     else if (w.DK == 64) exp_gate_kernel<64><<<blocks, 128, 0, st>>>(p, w, nseq);
     else if (w.DK == 128) exp_gate_kernel<128><<<blocks, 128, 0, st>>>(p, w, nseq);
     else exp_gate_kernel<256><<<blocks, 128, 0, st>>>(p, w, nseq);
+  }
+  if constexpr (MODE == SCAN_DECAY) {
+    const int columns = max_q > SCAN_SHORT ? scan_columns(w, p.heads, nseq, tokens, max_q) : SCAN_CPL;
+    if (columns == 1) return w.DK == 64 ? launch_scan_dk<64, MODE, false, 1>(p, w, nseq, st) : launch_scan_dk<128, MODE, false, 1>(p, w, nseq, st);
+    if (columns == 2) return w.DK == 64 ? launch_scan_dk<64, MODE, false, 2>(p, w, nseq, st) : launch_scan_dk<128, MODE, false, 2>(p, w, nseq, st);
   }
 #define SCAN_DK(D) (max_q <= SCAN_SHORT ? launch_scan_dk<D, MODE, true>(p, w, nseq, st) : launch_scan_dk<D, MODE, false>(p, w, nseq, st))
   if (w.DK == 16) return SCAN_DK(16);

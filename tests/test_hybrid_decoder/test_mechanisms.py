@@ -178,6 +178,28 @@ def test_scans_of_short_and_long_portions_agree(mode, d, dv, cuts):
     assert torch.isfinite(ran[0][0]).all() and torch.equal(ran[0][0], ran[1][0]) and torch.equal(ran[0][1], ran[1][1])
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,d,dv,lens", [(16, 128, 128, [70]), (24, 64, 99, [41, 40]), (20, 128, 66, [35, 1, 50, 52]),      # two columns a lane
+                                         (3, 128, 37, [47]), (9, 64, 64, [33, 90]), (18, 128, 64, [49]),                    # one
+                                         (16, 64, 128, [60] * 6), (16, 128, 96, [40] * 9)])                                  # four
+def test_decay_scan_columns_of_a_lane(H, d, dv, lens):
+    """Calls on both sides of the rules for a lane's columns: the same bits as each sequence in short portions, from carried states."""
+    dev, n = _dev("cuda"), len(lens)
+    g = torch.Generator().manual_seed(H)
+    q, k, v = (torch.randn(sum(lens), H * w, generator=g).to(dev) for w in (d, d, dv))
+    head, start = torch.rand(H, generator=g).to(dev), torch.randn(n, H, d, dv, generator=g).to(dev)
+    state, parts = start.clone(), start.clone()
+    out = M.state_scan_decay(q, k, v, head, state, M.RaggedMeta.build(lens, [5] * n, list(range(n)), dev), H, d, dv)
+    at = 0
+    for i, m in enumerate(lens):
+        for a in range(at, at + m, 32):
+            r = slice(a, min(a + 32, at + m))
+            o = M.state_scan_decay(q[r], k[r], v[r], head, parts, M.RaggedMeta.build([r.stop - a], [5], [i], dev), H, d, dv)
+            assert torch.equal(o, out[r])
+        at += m
+    assert torch.equal(state, parts)
+
+
 @pytest.mark.parametrize("device", DEVICES)
 @pytest.mark.parametrize("L", [8, 13, 16])
 def test_decay_scan_of_infinite_and_very_large_values(device, L):
