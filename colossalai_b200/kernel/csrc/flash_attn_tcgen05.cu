@@ -23,7 +23,10 @@
 // steps were halved.  2 x 4096 tokens, 32 / 8 heads of 128, causal: whole steps 309 us, half steps 450, with the converged
 // issuer 289, with output warps of their own 256, and 263 with the first reference from both halves of a key tile; five documents of
 // 8192 tokens together 181 -> 156; sixteen of 16384, heads of 64, 223 -> 191.  Two threads per row (16 softmax warps) were 5 - 10 %
-// slower than one.
+// slower than one.  The two tiles' exponentials in turn (`take_turn`): sixteen prompts of 16384 tokens, heads of 64, 188 -> 171 us, two
+// of 8192 920 -> 765; heads of 128, one call after the other, 2 x 4096 tokens 321 -> 281, five documents of 8192 163 -> 153, 24 of 8192 in 64 heads 164 ->
+// 166.  Taken back since: a quarter or an eighth of the exponentials as polynomials of degree 5 (765 -> 840), the next step's scores
+// fetched under the exponentials (997), turns only in units of 8 steps and more (heads of 128: 281 -> 304).
 // TMEM map (512 columns): [0,128) S_0, [128,256) S_1, then O_0, O_1, D wide each; P_t of a half overwrites the first 32 columns of
 // that half of S_t once its scores are in registers.
 // Shared memory at D = 128: 2 x Q 32 KB + 4 ring slots of 32 KB (at D = 64 2 x 16 KB + 8 x 16 KB) + 4 x 32 rows of the output +
@@ -267,7 +270,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint64_t* o_empty = o_full + 4;          // [2]  4 output warps have read O_t
   uint64_t* row_full = o_empty + 2;        // [2]  4 softmax warps are through with a unit: maxima and sums of its rows
   uint64_t* row_empty = row_full + 2;      // [2]  4 output warps have read them
-  uint64_t* u_full = row_empty + 2;        // [UNIT_RING]
+  uint64_t* turn = row_empty + 2;          // [2][4]  a warp of that tile may exponentiate
+  uint64_t* u_full = turn + 8;             // [UNIT_RING]
   uint64_t* u_empty = u_full + UNIT_RING;  // [UNIT_RING]  14 warps have read the unit
   FaUnit* units = reinterpret_cast<FaUnit*>(u_empty + UNIT_RING);
   uint64_t* drained = reinterpret_cast<uint64_t*>(units + UNIT_RING);   // [1]  a CTA that gives up: its products have retired
@@ -301,6 +305,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       mbar_init(&row_full[i], 4);
       mbar_init(&row_empty[i], 4);
     }
+    for (int i = 0; i < 8; ++i) mbar_init(&turn[i], 1);
     for (int i = 0; i < UNIT_RING; ++i) {
       mbar_init(&u_full[i], 1);
       mbar_init(&u_empty[i], 14);
@@ -582,10 +587,27 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const uint32_t o_addr = tmem_base + lane_addr + C::O_COL + t * D;
     const uint32_t s_addr = tmem_base + lane_addr + t * BLOCK_KV;
     uint32_t phase = 0, units_of = 0;                    // bit h: parity of the next S_t in half h; units of this tile so far
+    // The two tiles' warps of a quarter share a scheduler and exponentiate in turn, tile 0 first: at once each took twice as long, while
+    // nothing ran under the maxima, loads and waits of both.  They have as many turns in a unit as the longer tile has steps.
+    uint32_t turns = t ^ 1;                              // parity of the next turn
+    uint64_t* const mine = &turn[4 * t + quarter];
+    uint64_t* const theirs = &turn[4 * (t ^ 1) + quarter];
+    auto take_turn = [&]() -> bool {
+      const bool here = __all_sync(0xffffffffu, wait_or_abort(mine, turns & 1, abort_flag)) != 0;
+      turns ^= 1;
+      return here;
+    };
+    auto pass_turn = [&]() {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(theirs);
+    };
     bool ok = true;
     while (ok && next_unit()) {
-      const int n_steps = steps_of(t);
-      if (n_steps == 0) continue;
+      const int n_steps = steps_of(t), turns_of_unit = max(n_steps, steps_of(t ^ 1));
+      if (n_steps == 0) {
+        for (int j = 0; j < turns_of_unit && ok; ++j) { ok = take_turn(); pass_turn(); }
+        continue;
+      }
       const int q_tile = tile_of(t), head = head_of(t), len_k = un.len_k;
       const int kv_first = first_key_tile();
       const int q_pos = q_tile * BLOCK_Q + r;              // position inside the sequence
@@ -703,11 +725,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         // ---- p = exp2(s - m), row sum, 16-bit P over the scores it came from
         const uint64_t mul2 = pack_f32x2(ex_mul, ex_mul), sub2 = pack_f32x2(-m_use, -m_use);
         uint64_t lt[2] = {0ull, 0ull};
+        if (!take_turn()) return false;
 #pragma unroll
         for (int c = 0; c < HALF_KV; c += 32) {
           uint32_t packed[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
+            if (c + i == 48) pass_turn();                          // (32 to 56 are the same, 64 is 5 % slower)
             float p0, p1;
             unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c + i]), __uint_as_float(v[c + i + 1])), mul2, sub2), p0, p1);
             p0 = fast_exp2(p0);
@@ -747,6 +771,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         tc_fence_after();
         ok = needs_mask(j) ? step(j, std::true_type{}) : step(j, std::false_type{});
       }
+      for (int j = n_steps; j < turns_of_unit && ok; ++j) { ok = take_turn(); pass_turn(); }
       if (!ok) break;
       // ---- the row's maximum and sum go to the output warps
       ok = __all_sync(0xffffffffu, wait_or_abort(&row_empty[t], (units_of & 1) ^ 1, abort_flag));
