@@ -67,6 +67,12 @@ struct Launchers {
   int (*decode_splits)(int, int, int, int*);
   int (*decode)(const void*, const void*, const void*, const int*, const int*, void*, float*, float*, int, int, int, int, int, int,
                 int, int, float, const float*, int64_t, int64_t, int, int, cudaStream_t);
+  int (*moe_sort)(const int64_t*, int64_t, int, int, int, int*, int*, int*, int64_t*, int*, int64_t*, cudaStream_t);
+  int (*moe_take)(const void*, const int*, void*, int, int, int, cudaStream_t);
+  int (*moe_sum)(const void*, const int*, const float*, void*, int, int, int, int, cudaStream_t);
+  int (*moe_sum_bwd)(const void*, const void*, const int*, const float*, void*, float*, int, int, int, int, cudaStream_t);
+  int (*grouped)(const void*, const void*, void*, const int*, int, int, int, int, int, int, int, int, cudaStream_t);
+  int (*grouped_wgrad)(const void*, const void*, void*, const int*, int, int, int, int, int, int, int, int, int, cudaStream_t);
 } L;
 
 // launches by name since the last `counts`
@@ -76,9 +82,11 @@ struct Count {
 };
 Count n_norm_fwd{"rmsnorm_fwd"}, n_norm_bwd{"rmsnorm_bwd"}, n_glu_fwd{"glu_fwd"}, n_glu_bwd{"glu_bwd"}, n_rope{"rope"},
     n_stats{"ce_row_stats"}, n_loss{"ce_loss"}, n_grad{"ce_softmax_grad"}, n_flash_fwd{"flash_attn_varlen_fwd"},
-    n_flash_bwd{"flash_attn_bwd"}, n_decode{"paged_decode_attention"}, n_rows{"gemm_rows"}, n_embed{"embed_rows"};
+    n_flash_bwd{"flash_attn_bwd"}, n_decode{"paged_decode_attention"}, n_rows{"gemm_rows"}, n_embed{"embed_rows"},
+    n_sort{"moe_sort"}, n_take{"moe_take_rows"}, n_sum{"moe_sum_rows"}, n_sum_bwd{"moe_sum_rows_bwd"}, n_grouped{"grouped_gemm"},
+    n_wgrad{"grouped_gemm_wgrad"};
 Count* const COUNTS[] = {&n_norm_fwd, &n_norm_bwd, &n_glu_fwd, &n_glu_bwd, &n_rope, &n_stats, &n_loss, &n_grad, &n_flash_fwd, &n_flash_bwd,
-                         &n_decode, &n_rows, &n_embed};
+                         &n_decode, &n_rows, &n_embed, &n_sort, &n_take, &n_sum, &n_sum_bwd, &n_grouped, &n_wgrad};
 
 void launched(int rc, Count& c, int n = 1) {
   TORCH_CHECK(rc != cudaErrorLaunchTimeout, c.name, ": a wait inside an earlier attention kernel ran out; what it wrote is not valid (CUDA error ",
@@ -124,30 +132,34 @@ struct RmsNorm : torch::autograd::Function<RmsNorm> {
 };
 
 // ------------------------------------------------------------------------------------------------ gated unit
+// valid: int64 [1] on the device, rows to compute, or none
 struct Glu : torch::autograd::Function<Glu> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& gate_up, int64_t act) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& gate_up, int64_t act, const OptTensor& valid) {
     const c10::cuda::CUDAGuard guard(gate_up.device());
     const Tensor gu = gate_up.contiguous();
     const int64_t I = gu.size(-1) / 2, rows = I ? gu.numel() / (2 * I) : 0;
     std::vector<int64_t> shape = gu.sizes().vec();
     shape.back() = I;
     Tensor out = at::empty(shape, gu.options());
-    launched(L.glu_fwd(ptr(gu), mut(out), rows, (int)I, (int)act, code_of(gu), nullptr, stream_of(gu)), n_glu_fwd);
-    ctx->save_for_backward({gu});
+    launched(L.glu_fwd(ptr(gu), mut(out), rows, (int)I, (int)act, code_of(gu), valid.has_value() ? as<int64_t>(*valid) : nullptr,
+                       stream_of(gu)),
+             n_glu_fwd);
+    ctx->save_for_backward({gu, valid.has_value() ? *valid : Tensor()});
     ctx->saved_data["act"] = act;
     return out;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const Tensor gu = ctx->get_saved_variables()[0];
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &gu = saved[0], &valid = saved[1];
     const c10::cuda::CUDAGuard guard(gu.device());
     const int64_t I = gu.size(-1) / 2, rows = I ? gu.numel() / (2 * I) : 0;
     const Tensor d = grads[0].contiguous();
     Tensor dgu = at::empty_like(gu);
-    launched(L.glu_bwd(ptr(d), ptr(gu), mut(dgu), rows, (int)I, (int)ctx->saved_data["act"].toInt(), code_of(gu), nullptr,
-                       stream_of(gu)),
+    launched(L.glu_bwd(ptr(d), ptr(gu), mut(dgu), rows, (int)I, (int)ctx->saved_data["act"].toInt(), code_of(gu),
+                       as<int64_t>(valid), stream_of(gu)),
              n_glu_bwd);
-    return {dgu, Tensor()};
+    return {dgu, Tensor(), Tensor()};
   }
 };
 
@@ -307,6 +319,123 @@ Tensor embed_rows(const Tensor& ids, const Tensor& table) {
   return out;
 }
 
+// ------------------------------------------------------------------------------------------------ local experts
+// The operators of a mixture-of-experts layer (`ops/moe.py`, `moe/grouped_gemm.py`).  As python functions a forward and backward of 64
+// tokens took 518 us, nearly all of it here on the host, and a layer of 24576 rows still waited 120 us for it at its two ends.
+
+// topk_idx [T, k] -> slot, src, padded counts, ends, total, as `ops/moe.py:sort_choices` describes them
+std::vector<Tensor> sort_choices(const Tensor& topk_idx, int64_t E, int64_t align) {
+  const c10::cuda::CUDAGuard guard(topk_idx.device());
+  const Tensor idx = topk_idx.reshape({-1}).to(at::kLong).contiguous();
+  const int64_t n = idx.numel(), bound = (n + E * (align - 1) + align - 1) / align * align;
+  const Tensor work = at::empty({2 * E + n + bound}, idx.options().dtype(at::kInt)), wide = at::empty({E + 1}, idx.options());
+  const Tensor counts = work.narrow(0, 0, E), ends = work.narrow(0, E, E), slot = work.narrow(0, 2 * E, n),
+               src = work.narrow(0, 2 * E + n, bound), padded = wide.narrow(0, 0, E), total = wide.narrow(0, E, 1);
+  launched(L.moe_sort(as<int64_t>(idx), n, (int)E, (int)align, (int)bound, mut_as<int>(counts), mut_as<int>(slot), mut_as<int>(src),
+                      mut_as<int64_t>(padded), mut_as<int>(ends), mut_as<int64_t>(total), stream_of(idx)),
+           n_sort, 2);
+  return {slot, src, padded, ends, total};
+}
+
+Tensor sum_rows(const Tensor& rows, const Tensor& slot, const Tensor& w, int64_t T, int64_t k) {
+  Tensor out = at::empty({T, rows.size(1)}, rows.options());
+  launched(L.moe_sum(ptr(rows), as<int>(slot), as<float>(w), mut(out), (int)T, (int)k, (int)rows.size(1), code_of(rows), stream_of(rows)),
+           n_sum);
+  return out;
+}
+// [T, k, H]: every choice's row (zeros for a choice of no expert), differentiable
+Tensor pick_rows(const Tensor& rows, const Tensor& slot, int64_t T, int64_t k) {
+  const Tensor picked = rows.index_select(0, slot.clamp_min(0).to(at::kLong));
+  return at::where(slot.ge(0).unsqueeze(-1), picked, at::zeros_like(picked)).view({T, k, -1});
+}
+
+// x [T, H] -> rows [bound, H] grouped by expert; a gradient that is to be differentiated again is made of torch operations
+struct TakeRows : torch::autograd::Function<TakeRows> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& slot, const Tensor& src, int64_t k) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const Tensor xa = packed(x);
+    Tensor rows = at::empty({src.numel(), xa.size(1)}, xa.options());
+    launched(L.moe_take(ptr(xa), as<int>(src), mut(rows), (int)src.numel(), (int)k, (int)(xa.size(1) * xa.element_size()), stream_of(xa)),
+             n_take);
+    ctx->save_for_backward({slot});
+    ctx->saved_data["shape"] = std::vector<int64_t>{xa.size(0), k};
+    return rows;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor slot = ctx->get_saved_variables()[0], &d = grads[0];
+    const std::vector<int64_t> s = ctx->saved_data["shape"].toIntVector();
+    const c10::cuda::CUDAGuard guard(d.device());
+    const Tensor dx = at::GradMode::is_enabled() ? pick_rows(d, slot, s[0], s[1]).to(at::kFloat).sum(1).to(d.scalar_type())
+                                                 : sum_rows(packed(d), slot, Tensor(), s[0], s[1]);
+    return {dx, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// rows [bound, H], weights [T, k] -> out [T, H] = sum_j weights[t, j] rows[slot[t, j]]
+struct CombineRows : torch::autograd::Function<CombineRows> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& rows, const Tensor& weights, const Tensor& slot, const Tensor& src) {
+    const c10::cuda::CUDAGuard guard(rows.device());
+    ctx->save_for_backward({rows, weights, slot, src});
+    return sum_rows(packed(rows), slot, weights.to(at::kFloat).contiguous(), weights.size(0), weights.size(1));
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const Tensor &rows = s[0], &weights = s[1], &slot = s[2], &src = s[3];
+    const c10::cuda::CUDAGuard guard(rows.device());
+    const int64_t T = weights.size(0), k = weights.size(1);
+    if (at::GradMode::is_enabled()) {
+      const Tensor live = src.ge(0).unsqueeze(-1), choice = src.clamp_min(0).to(at::kLong), dout = grads[0].to(at::kFloat);
+      const Tensor g = dout.index_select(0, choice.floor_divide(k));
+      const Tensor w = weights.to(at::kFloat).reshape({-1}).index_select(0, choice).unsqueeze(-1);
+      const Tensor dw = (pick_rows(rows, slot, T, k).to(at::kFloat) * dout.unsqueeze(1)).sum(-1);
+      return {at::where(live, w * g, at::zeros_like(g)).to(rows.scalar_type()), dw.to(weights.scalar_type()), Tensor(), Tensor()};
+    }
+    const Tensor g = packed(grads[0]), r = packed(rows), w = weights.to(at::kFloat).contiguous();
+    Tensor drows = at::empty_like(r), dw = at::zeros_like(w);
+    launched(L.moe_sum_bwd(ptr(g), ptr(r), as<int>(src), as<float>(w), mut(drows), mut_as<float>(dw), (int)src.numel(), (int)k,
+                           (int)r.size(1), code_of(r), stream_of(r)),
+             n_sum_bwd);
+    return {drows, dw.to(weights.scalar_type()), Tensor(), Tensor()};
+  }
+};
+
+// y[rows of e] = x[rows of e] w[e]^T; w [E, N, K] contiguous, N a multiple of 128 (the input gradient's blocks), ends int32 [E]: where
+// each expert's rows end, multiples of 16.  The caller has checked types and sizes.
+struct GroupedLinear : torch::autograd::Function<GroupedLinear> {
+  static Tensor product(const Tensor& x, const Tensor& w, const Tensor& ends, bool transposed) {
+    const int64_t N = w.size(transposed ? 1 : 2);
+    Tensor y = at::empty({x.size(0), N}, x.options());
+    launched(L.grouped(ptr(x), ptr(w), mut(y), as<int>(ends), (int)w.size(0), (int)x.size(0), (int)N, (int)x.size(1), (int)x.stride(0),
+                       (int)N, transposed, code_of(x), stream_of(x)),
+             n_grouped);
+    return y;
+  }
+
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& ends) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    ctx->save_for_backward({x, w, ends});
+    return product(x.contiguous(), w, ends, true);
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const Tensor &w = s[1], &ends = s[2], dy = grads[0].contiguous();
+    const c10::cuda::CUDAGuard guard(w.device());
+    Tensor dx, dw;
+    if (ctx->needs_input_grad(0)) dx = product(dy, w, ends, false);
+    if (ctx->needs_input_grad(1)) {
+      const Tensor x = s[0].contiguous();
+      dw = at::empty({w.size(0), dy.size(1), x.size(1)}, w.options());
+      launched(L.grouped_wgrad(ptr(dy), ptr(x), mut(dw), as<int>(ends), (int)w.size(0), (int)x.size(0), (int)dy.size(1), (int)x.size(1),
+                               (int)dy.stride(0), (int)x.stride(0), code_of(x), code_of(w), 0, stream_of(x)),
+               n_wgrad);
+    }
+    return {dx, dw, Tensor()};
+  }
+};
+
 template <typename F> void take(const std::map<std::string, uint64_t>& table, const char* name, F& slot) {
   const auto it = table.find(name);
   TORCH_CHECK(it != table.end() && it->second != 0, "launcher ", name, " is missing");
@@ -330,6 +459,12 @@ void bind(const std::map<std::string, uint64_t>& t) {
   take(t, "cb_embed_rows", L.embed_rows);
   take(t, "cb_decode_num_splits", L.decode_splits);
   take(t, "cb_paged_decode_attention", L.decode);
+  take(t, "cb_moe_sort", L.moe_sort);
+  take(t, "cb_moe_take_rows", L.moe_take);
+  take(t, "cb_moe_sum_rows", L.moe_sum);
+  take(t, "cb_moe_sum_rows_bwd", L.moe_sum_bwd);
+  take(t, "cb_grouped_gemm", L.grouped);
+  take(t, "cb_grouped_gemm_wgrad", L.grouped_wgrad);
 }
 
 std::map<std::string, long long> counts(bool clear) {
@@ -354,7 +489,8 @@ PYBIND11_MODULE(cb200_host, m) {
           return std::make_tuple(o[0], o[1]);
         },
         release());
-  m.def("glu", [](const Tensor& gu, int64_t act) { return Glu::apply(gu, act); }, release());
+  m.def("glu", [](const Tensor& gu, int64_t act) { return Glu::apply(gu, act, OptTensor()); }, release());
+  m.def("glu_of_rows", [](const Tensor& gu, int64_t act, const Tensor& valid) { return Glu::apply(gu, act, OptTensor(valid)); }, release());
   m.def("rope",
         [](const Tensor& x, const Tensor& pos, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t D, int64_t rot,
            bool interleaved) { return Rope::apply(x, pos, cos, sin, heads, D, rot, interleaved); },
@@ -372,4 +508,13 @@ PYBIND11_MODULE(cb200_host, m) {
   m.def("paged_decode", &paged_decode, release());
   m.def("linear_rows", &linear_rows, release());
   m.def("embed_rows", &embed_rows, release());
+  m.def("sort_choices", &sort_choices, release());
+  m.def("take_rows", [](const Tensor& x, const Tensor& slot, const Tensor& src, int64_t k) { return TakeRows::apply(x, slot, src, k); },
+        release());
+  m.def("combine_rows",
+        [](const Tensor& rows, const Tensor& weights, const Tensor& slot, const Tensor& src) {
+          return CombineRows::apply(rows, weights, slot, src);
+        },
+        release());
+  m.def("grouped_linear", [](const Tensor& x, const Tensor& w, const Tensor& ends) { return GroupedLinear::apply(x, w, ends); }, release());
 }

@@ -480,10 +480,11 @@ __global__ void __launch_bounds__(256) moe_count_kernel(const int64_t* __restric
 }
 
 // block e < E: places expert e's choices in order and marks the padding rows behind them (src = -1); block E marks the rows
-// behind the last expert, choices of no expert (slot = -1) and writes the padded counts.
+// behind the last expert, choices of no expert (slot = -1) and writes the padded counts, where each expert's rows end and their total.
 __global__ void __launch_bounds__(SORT_THREADS) moe_place_kernel(const int64_t* __restrict__ topk_idx, int64_t n, int E, int align,
                                                                  int bound, const int* __restrict__ counts, int* __restrict__ slot,
-                                                                 int* __restrict__ src, int64_t* __restrict__ padded_counts) {
+                                                                 int* __restrict__ src, int64_t* __restrict__ padded_counts,
+                                                                 int* __restrict__ ends, int64_t* __restrict__ total_rows) {
   __shared__ int warp_sum_s[SORT_THREADS / 32];
   __shared__ int start_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, e = blockIdx.x;
@@ -502,7 +503,24 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_place_kernel(const int64_t* 
   int at = start_s;
   if (e == E) {
     for (int r = at + tid; r < bound; r += SORT_THREADS) src[r] = -1;
-    for (int o = tid; o < E; o += SORT_THREADS) padded_counts[o] = (counts[o] + align - 1) / align * align;
+    if (warp == 0) {
+      int before = 0;
+      for (int o0 = 0; o0 < E; o0 += 32) {
+        const int o = o0 + lane, own = o < E ? (counts[o] + align - 1) / align * align : 0;
+        int upto = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, upto, d);
+          if (lane >= d) upto += y;
+        }
+        if (o < E) {
+          padded_counts[o] = own;
+          ends[o] = before + upto;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+      }
+      if (lane == 0) *total_rows = before;
+    }
     for (int64_t i = tid; i < n; i += SORT_THREADS)
       if (topk_idx[i] < 0 || topk_idx[i] >= E) slot[i] = -1;
     return;
@@ -665,14 +683,14 @@ int cb_moe_flag_words() { return FLAG_WORDS; }
 // ---- local experts.  counts int32 [E] (zeroed here), slot int32 [n], src int32 [bound], padded_counts int64 [E];
 // bound >= n + E * (align - 1) rounded up to align
 int cb_moe_sort(const int64_t* topk_idx, int64_t n, int E, int align, int bound, int* counts, int* slot, int* src,
-                int64_t* padded_counts, cudaStream_t st) {
+                int64_t* padded_counts, int* ends, int64_t* total_rows, cudaStream_t st) {
   if (E <= 0 || E > 8192) return (int)cudaErrorInvalidValue;
   cudaError_t err = cudaMemsetAsync(counts, 0, (size_t)E * sizeof(int), st);
   if (err != cudaSuccess) return (int)err;
   const int64_t blocks = (n + 1023) / 1024;
   if (n > 0)
     moe_count_kernel<<<(unsigned)(blocks < cb_num_sms() ? blocks : cb_num_sms()), 256, E * sizeof(int), st>>>(topk_idx, n, E, counts);
-  moe_place_kernel<<<E + 1, SORT_THREADS, 0, st>>>(topk_idx, n, E, align, bound, counts, slot, src, padded_counts);
+  moe_place_kernel<<<E + 1, SORT_THREADS, 0, st>>>(topk_idx, n, E, align, bound, counts, slot, src, padded_counts, ends, total_rows);
   return CB_LAUNCH_CHECK();
 }
 

@@ -13,11 +13,12 @@ from typing import Optional
 import torch
 import torch.distributed as dist
 
+from ..kernel import loader
 from ..ops._dispatch import plain_call, use_native
 from ..ops.moe import SORT_EXPERTS, CombineRows, TakeRows, rows_ok, sort_choices
 from ..parallel import comm
 from ._operation import AllToAllUneven
-from .grouped_gemm import ROW_ALIGN
+from .grouped_gemm import ROW_ALIGN, on_sm100
 
 __all__ = ["moe_forward", "set_moe_backend", "get_moe_backend"]
 
@@ -53,7 +54,7 @@ def _aligned_rows(x: torch.Tensor) -> bool:
     operations): the native grouped weight-gradient GEMM then needs no re-layout pass (moe/grouped_gemm.py)."""
     return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
             and os.environ.get("CB200_GROUPED_GEMM", "native") == "native"
-            and torch.cuda.get_device_capability(x.device)[0] == 10)
+            and on_sm100(x.device))
 
 
 def _padded_counts(counts: torch.Tensor) -> torch.Tensor:
@@ -102,9 +103,12 @@ def moe_forward(x: torch.Tensor, topk_w: torch.Tensor, topk_idx: torch.Tensor, e
         # than the sort has counters for, and for calls that functorch, forward mode or a mode watches
         slot, src, counts = sort_choices(topk_idx, num_experts, ROW_ALIGN)
         counts.cb200_aligned = True
-        ys = experts(TakeRows.apply(x, slot, src, k), counts)
+        host = loader.host()
+        ys = experts(TakeRows.apply(x, slot, src, k) if host is None else host.take_rows(x, slot, src, k), counts)
         if rows_ok(ys):
-            return CombineRows.apply(ys, topk_w, slot, src)
+            if host is None or not plain_call(ys, topk_w):
+                return CombineRows.apply(ys, topk_w, slot, src)
+            return host.combine_rows(ys, topk_w, slot, src)
         picked = ys.index_select(0, slot.long()).view(T, k, -1)        # experts of another width or type
         return (picked * topk_w.unsqueeze(-1).to(ys.dtype)).sum(1)
     n_local = num_experts // ep

@@ -11,9 +11,14 @@ from __future__ import annotations
 
 import ctypes
 import os
+from functools import lru_cache
 from typing import Optional, Tuple
 
 import torch
+
+from ..kernel import loader
+from ..ops._dispatch import plain_call
+from ..ops.moe import expert_ends
 
 _lib = None
 ROW_ALIGN = 16        # reduction of one instruction of the wgrad kernel: group row ranges must start / end on multiples of it
@@ -35,7 +40,18 @@ def native_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
         return False
     return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype and x.dim() == 2
             and w.dim() == 3 and x.shape[0] > 0 and x.shape[1] % 8 == 0 and w.shape[1] % 8 == 0 and w.shape[0] <= 512
-            and w.is_contiguous() and torch.cuda.get_device_capability(x.device)[0] == 10)
+            and w.is_contiguous() and on_sm100(x.device))
+
+
+@lru_cache(maxsize=None)
+def on_sm100(device: torch.device) -> bool:
+    return torch.cuda.get_device_capability(device)[0] == 10
+
+
+def rows_of(counts: torch.Tensor) -> torch.Tensor:
+    """The sum of `counts`, a device scalar."""
+    _, total = expert_ends(counts)
+    return counts.sum() if total is None else total.view(())
 
 
 def _offs(counts: torch.Tensor, device) -> torch.Tensor:
@@ -157,7 +173,11 @@ def grouped_linear(x: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, align
     range starts and ends on a multiple of 16 (zero rows as padding) - the weight-gradient GEMM then runs without the
     re-layout pass."""
     if native_ok(x, w):
-        return _GroupedLinearNative.apply(x, w, counts, aligned or getattr(counts, "cb200_aligned", False))
+        aligned = aligned or getattr(counts, "cb200_aligned", False)
+        if aligned and w.shape[1] % K_BLOCK == 0 and plain_call(x, w, counts) and (host := loader.host()) is not None:
+            ends, _ = expert_ends(counts)
+            return host.grouped_linear(x, w, _offs(counts, x.device) if ends is None else ends)
+        return _GroupedLinearNative.apply(x, w, counts, aligned)
     if x.is_cuda and hasattr(torch, "_grouped_mm") and x.dtype == torch.bfloat16 and x.shape[0] > 0 \
             and x.shape[1] % 8 == 0 and w.shape[1] % 8 == 0:
         offs = _offs(counts, x.device)

@@ -81,6 +81,8 @@ def glu(gate_up: torch.Tensor, act: str = "silu", valid_rows: Optional[torch.Ten
     if use_native(gate_up) and gate_up.dtype in (torch.float32, torch.float16, torch.bfloat16) and I % vec == 0:
         if valid_rows is not None:
             valid_rows = valid_rows.to(device=gate_up.device, dtype=torch.int64).reshape(1).contiguous()
+            if plain_call(gate_up, valid_rows) and (host := loader.host()) is not None:
+                return host.glu_of_rows(gate_up, _ACT[act], valid_rows)
         elif plain_call(gate_up) and (host := loader.host()) is not None:
             return host.glu(gate_up, _ACT[act])
         return _GLUFn.apply(gate_up, _ACT[act], valid_rows)

@@ -12,7 +12,7 @@ from typing import Optional, Tuple
 import torch
 
 from ..kernel import loader
-from ._dispatch import use_native
+from ._dispatch import plain_call, use_native
 from ._dtypes import code
 
 _lib = None
@@ -224,17 +224,30 @@ def sort_choices(topk_idx: torch.Tensor, num_experts: int, align: int):
     """topk_idx [T, k] on the GPU -> (slot int32 [T * k], src int32 [bound], counts int64 [E]): choice i's row sits at
     slot[i] of a buffer grouped by expert in which every expert's rows, in the order of their choices, are padded to a
     multiple of `align`; src[r] is the choice of row r (-1: padding); counts are the padded ones.  A choice outside
-    [0, E) gets slot -1.  No host synchronisation."""
-    idx = topk_idx.reshape(-1).to(torch.int64).contiguous()
-    n, dev = idx.numel(), idx.device
-    bound = (n + num_experts * (align - 1) + align - 1) // align * align
-    work = torch.empty(num_experts + n + bound, dtype=torch.int32, device=dev)
-    counts, slot, src = work[:num_experts], work[num_experts: num_experts + n], work[num_experts + n:]
-    padded = torch.empty(num_experts, dtype=torch.int64, device=dev)
-    loader.check(_get_lib().cb_moe_sort(loader.ptr(idx), ctypes.c_int64(n), num_experts, align, bound, loader.ptr(counts),
-                                        loader.ptr(slot), loader.ptr(src), loader.ptr(padded), loader.stream_ptr()), "moe_sort")
-    loader.launch_counter.add("moe_sort", 2)
+    [0, E) gets slot -1.  No host synchronisation.  `expert_ends(counts)` gives what is known of their sums."""
+    if num_experts > 0 and plain_call(topk_idx) and (host := loader.host()) is not None:
+        slot, src, padded, ends, total = host.sort_choices(topk_idx, num_experts, align)
+    else:
+        idx = topk_idx.reshape(-1).to(torch.int64).contiguous()
+        n, dev = idx.numel(), idx.device
+        bound = (n + num_experts * (align - 1) + align - 1) // align * align
+        work = torch.empty(2 * num_experts + n + bound, dtype=torch.int32, device=dev)
+        counts, ends, slot, src = work.split([num_experts, num_experts, n, bound])
+        padded, total = torch.empty(num_experts + 1, dtype=torch.int64, device=dev).split([num_experts, 1])
+        loader.check(_get_lib().cb_moe_sort(loader.ptr(idx), ctypes.c_int64(n), num_experts, align, bound, loader.ptr(counts),
+                                            loader.ptr(slot), loader.ptr(src), loader.ptr(padded), loader.ptr(ends),
+                                            loader.ptr(total), loader.stream_ptr()), "moe_sort")
+        loader.launch_counter.add("moe_sort", 2)
+    if not padded.is_inference():
+        padded.cb200_ends = (padded._version, ends, total)
     return slot, src, padded
+
+
+def expert_ends(counts: torch.Tensor):
+    """(ends int32 [E]: the running sum of `counts`, total int64 [1]) that the sort wrote beside these counts, or (None, None) where
+    they come from elsewhere or were written to since."""
+    version, ends, total = getattr(counts, "cb200_ends", (None, None, None))
+    return (ends, total) if ends is not None and counts._version == version else (None, None)
 
 
 def rows_ok(x: torch.Tensor) -> bool:

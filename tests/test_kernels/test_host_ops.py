@@ -226,3 +226,62 @@ def test_paged_decode(monkeypatch, D):
         return inference.paged_decode_attention(q, kc, vc, tables, lens, window=50),
 
     _same(*_both(monkeypatch, fn))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,E,k,H,inter", [(1, 8, 2, 64, 64), (37, 16, 4, 256, 192), (700, 64, 6, 128, 64), (300, 5, 1, 512, 40)])
+@pytest.mark.parametrize("mode", ["grad", "no_grad", "inference", "frozen"])
+def test_local_experts(monkeypatch, T, E, k, H, inter, mode):
+    """A layer of local experts (outputs of no multiple of 128 included, whose input gradient is not this module's): the same bits and
+    launches without the module, with weights that need no gradient, and with choices of no expert."""
+    from colossalai_b200.models import get_config
+    from colossalai_b200.models.moe import GroupedExperts
+    from colossalai_b200.moe.dispatch_combine import moe_forward
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    experts = GroupedExperts(get_config("deepseek-moe-16b", hidden_size=H), E, inter).cuda().bfloat16()
+    for p in experts.parameters():
+        p.requires_grad_(mode != "frozen")
+    x0 = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    score = torch.rand(T, E, device="cuda", generator=g)
+    dy = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+
+    def fn():
+        x = x0.clone().requires_grad_(mode in ("grad", "frozen"))
+        w, idx = score.topk(k, dim=-1)
+        idx[T // 2, 0] = E                                        # its token's sum is NaN
+        w = w.detach().requires_grad_(mode == "grad")
+        with torch.inference_mode() if mode == "inference" else torch.set_grad_enabled(mode != "no_grad"):
+            y = moe_forward(x, w, idx, experts, E, None)
+        if not y.requires_grad:
+            return [y]
+        ins = [t for t in (x, w, *experts.parameters()) if t.requires_grad]
+        return [y, *torch.autograd.grad(y, ins, dy)]
+
+    out = []
+    for without in (False, True):
+        with monkeypatch.context() as m:
+            if without:
+                m.setattr(loader, "_host", None)
+                m.setattr(loader, "_host_asked", True)
+            else:
+                loader.host()
+            loader.launch_counter.reset()
+            out.append([t.nan_to_num(nan=7.0) for t in fn()])
+            out.append(dict(loader.launch_counter.by_name))
+    _same(out[0], out[2])
+    assert out[1] == out[3] and out[1]["grouped_gemm"] >= 2
+
+
+@pytest.mark.gpu
+def test_counts_written_to_after_the_sort():
+    """The running sums that the sort wrote beside the counts are not taken for counts that changed since."""
+    from colossalai_b200.moe.grouped_gemm import rows_of
+    from colossalai_b200.ops.moe import expert_ends, sort_choices
+
+    idx = torch.tensor([[0, 2], [2, 5]], device="cuda")
+    _, _, counts = sort_choices(idx, 6, 16)
+    ends, total = expert_ends(counts)
+    assert counts.tolist() == [16, 0, 16, 0, 0, 16] and ends.tolist() == [16, 16, 32, 32, 32, 48] and int(total) == int(rows_of(counts)) == 48
+    counts[1] += 16
+    assert expert_ends(counts) == (None, None) and int(rows_of(counts)) == 64 and expert_ends(counts + 0) == (None, None)
