@@ -165,8 +165,19 @@ class PagedKVRuntime:
         rt.set_ragged_step(tables, [seqlen] * batch, [0] * batch, list(range(batch)), device)
         return rt
 
+    def rotate_and_write(self, layer_idx: int, qkv: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
+                         heads: int, kv_heads: int, dim: int, rot_dim: int, interleaved: bool) -> Optional[torch.Tensor]:
+        """A decode step's rows q | k | v as `ops.rope_qkv` turns them, their keys and values written to the layer's pages in the same
+        launch (`attend` is then told so); None where that kernel does not serve."""
+        if self.is_prompt or self.ragged is not None or torch.is_grad_enabled() or type(self).attend is not PagedKVRuntime.attend:
+            return None
+        i = self.cache_index(layer_idx)
+        return iops.rope_pages(qkv, positions, cos, sin, heads, kv_heads, dim, rot_dim, interleaved, self.k_caches[i], self.v_caches[i],
+                               self.block_tables, self.token_seq, self.token_pos)
+
     def attend(self, layer_idx: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, meta, scale: float,
-               alibi_slopes: Optional[torch.Tensor] = None, sliding_window: Optional[int] = None) -> torch.Tensor:
+               alibi_slopes: Optional[torch.Tensor] = None, sliding_window: Optional[int] = None, written: bool = False) -> torch.Tensor:
+        """`written`: k and v are in the pages already."""
         if self.ragged is not None:
             # a ragged step (portions of prompts beside decoded tokens): rotary / plain attention families take the same
             # paged kernels as the hybrid decoders, without bias table and sink
@@ -176,7 +187,8 @@ class PagedKVRuntime:
             o = self.attend_ragged(layer_idx, q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1), scale)
             return o.view(T, hq, -1)
         kc, vc = self.k_caches[self.cache_index(layer_idx)], self.v_caches[self.cache_index(layer_idx)]
-        iops.kv_cache_write(k, v, kc, vc, self.block_tables, self.token_seq, self.token_pos)
+        if not written:
+            iops.kv_cache_write(k, v, kc, vc, self.block_tables, self.token_seq, self.token_pos)
         if sliding_window is not None and self.max_len_host > sliding_window:
             return self._attend_windowed(q, k, v, kc, vc, scale, alibi_slopes, sliding_window)
         return self._attend_full(q, k, v, kc, vc, scale, alibi_slopes)

@@ -6,35 +6,8 @@
 // rotary_embedding (fused_rotary_emb_and_cache_kernel.cu, N15), Triton LlamaActCombine
 // (kernel/triton/llama_act_combine_kernel.py), TorchScript bias_gelu / bias_dropout_add (kernel/jit/*.py),
 // multi_tensor_scale (N7).  All are pure HBM-bandwidth kernels: 16-byte vector I/O, grid-stride, fp32 math.
+#include "activations.cuh"
 #include "common.cuh"
-
-CB_DEVICE float silu_f(float x) { return x / (1.f + __expf(-x)); }
-CB_DEVICE float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }
-CB_DEVICE float gelu_tanh_f(float x) {
-  const float k = 0.7978845608028654f;
-  return 0.5f * x * (1.f + tanhf(k * (x + 0.044715f * x * x * x)));
-}
-CB_DEVICE float gelu_tanh_grad_f(float x) {
-  const float k = 0.7978845608028654f;
-  const float t = tanhf(k * (x + 0.044715f * x * x * x));
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * k * (1.f + 3.f * 0.044715f * x * x);
-}
-CB_DEVICE float gelu_erf_f(float x) { return 0.5f * x * (1.f + erff(x * 0.7071067811865476f)); }
-CB_DEVICE float gelu_erf_grad_f(float x) {
-  return 0.5f * (1.f + erff(x * 0.7071067811865476f)) + x * 0.3989422804014327f * __expf(-0.5f * x * x);
-}
-
-// act: 0 = silu, 1 = gelu(tanh), 2 = gelu(erf)
-// ACT: 0 silu, 1 gelu (tanh), 2 gelu (erf), 3 squared relu
-template <int ACT> CB_DEVICE float act_f(float x) {
-  if (ACT == 3) { const float r = fmaxf(x, 0.f); return r * r; }
-  return ACT == 0 ? silu_f(x) : (ACT == 1 ? gelu_tanh_f(x) : gelu_erf_f(x));
-}
-template <int ACT> CB_DEVICE float act_grad_f(float x) {
-  if (ACT == 3) return 2.f * fmaxf(x, 0.f);
-  if (ACT == 0) { const float s = sigmoid_f(x); return s * (1.f + x * (1.f - s)); }
-  return ACT == 1 ? gelu_tanh_grad_f(x) : gelu_erf_grad_f(x);
-}
 
 // Gated unit, forward and backward.  A block takes an equal part of one row, GLU_ITEMS vectors per thread, so that a thread has
 // all its loads in flight before its first store and no index needs a 64-bit division; at most 256 threads, and no more than
@@ -141,12 +114,21 @@ __global__ void __launch_bounds__(GLU_THREADS) glu_bwd_kernel(const T* __restric
 // backward: a block each 313 us, together 38.  A form of its own: with the stride and the row worked out at run time 8192 rows of 6144
 // took 40 us a direction instead of 35.
 constexpr int ROPE_NARROW = 64, ROPE_BLOCK = 256;
-template <typename T, bool VEC_TABLE, bool NARROW>
+// Where a step's keys and values go beside dst (PAGES): rows of kv_width elements of pages of `page` tokens, found through the page tables.
+// A decode step then has a launch a layer less; with the gated unit's too (gemm_rows_tcgen05.cu) 16 sequences, 4 layers of 4096 x 14336,
+// take 498 us instead of 513, 5 sequences, 2 layers of 1024 x 2816, 81 instead of 85.
+template <typename T> struct RopePages {
+  T *k, *v;
+  const int *tables, *token_seq, *token_pos;
+  int page, table_width, kv_width;     // tokens of a page, entries of a table, elements of a token's keys
+  int k_at;                            // first element of the keys in a row; the values follow them
+};
+template <typename T, bool VEC_TABLE, bool NARROW, bool PAGES>
 __global__ void __launch_bounds__(NARROW ? ROPE_BLOCK : 512) rope_kernel(const T* __restrict__ src, T* __restrict__ dst,
                                                    const int64_t* __restrict__ pos, const float* __restrict__ cos_c,
                                                    const float* __restrict__ sin_c, int64_t tokens, int per_block,
                                                    int64_t src_stride, int width, int n_rot_heads, int D, int rot_dim,
-                                                   float sign, int interleaved) {
+                                                   float sign, int interleaved, RopePages<T> pages) {
   constexpr int VEC = Vec16<T>::N;
   cb_early_start();
   const int half = rot_dim / 2;
@@ -162,6 +144,16 @@ __global__ void __launch_bounds__(NARROW ? ROPE_BLOCK : 512) rope_kernel(const T
   const T* in = src + t * src_stride;
   T* out = dst + t * width;
   const int64_t p = pos[t];
+  int64_t slot = 0;                                          // first element of the token's rows in the pages
+  if (PAGES) {
+    const int at = pages.token_pos[t], page = pages.tables[pages.token_seq[t] * pages.table_width + at / pages.page];
+    slot = ((int64_t)page * pages.page + at % pages.page) * pages.kv_width;
+  }
+  auto put = [&](const Vec16<T>& x, int o) {
+    x.store_na(out + o);
+    if (PAGES && o >= pages.k_at) x.store(o < pages.k_at + pages.kv_width ? pages.k + slot + (o - pages.k_at)
+                                                                          : pages.v + slot + (o - pages.k_at - pages.kv_width));
+  };
   auto copy_at = [&](int c) {
     return c < n_head_copy ? (c / copy_per_head) * D + rot_dim + (c % copy_per_head) * VEC : n_rot_heads * D + (c - n_head_copy) * VEC;
   };
@@ -173,8 +165,8 @@ __global__ void __launch_bounds__(NARROW ? ROPE_BLOCK : 512) rope_kernel(const T
       const int o1 = two ? copy_at(c0 + 1) : o0;
       a.load_nc(in + o0);
       b.load_nc(in + o1);
-      a.store_na(out + o0);
-      if (two) b.store_na(out + o1);
+      put(a, o0);
+      if (two) put(b, o1);
       continue;
     }
     const int h = j / vec_per_head, v = j - h * vec_per_head;
@@ -203,8 +195,8 @@ __global__ void __launch_bounds__(NARROW ? ROPE_BLOCK : 512) rope_kernel(const T
         u.set(i, x * c[i] - y * sn);
         w.set(i, y * c[i] + x * sn);
       }
-      u.store_na(out + o0);
-      w.store_na(out + o1);
+      put(u, o0);
+      put(w, o1);
     } else {
       // GPT-J / ChatGLM style: pairs are adjacent elements (2i, 2i + 1); the item's 2 VEC elements hold VEC pairs
 #pragma unroll
@@ -216,8 +208,8 @@ __global__ void __launch_bounds__(NARROW ? ROPE_BLOCK : 512) rope_kernel(const T
         b.set(i, z * cb - w * sb);
         b.set(i + 1, w * cb + z * sb);
       }
-      a.store_na(out + o0);
-      b.store_na(out + o1);
+      put(a, o0);
+      put(b, o1);
     }
   }
 }
@@ -269,6 +261,23 @@ __global__ void __launch_bounds__(256) scale_check_kernel(const TI* __restrict__
     out[i] = from_f32<TO>(v * scale);
   }
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) *flag = 1;
+}
+
+template <typename T, bool PAGES>
+static int launch_rope(const T* src, T* dst, const int64_t* pos, const float* cos_c, const float* sin_c, int64_t tokens, int64_t src_stride,
+                       int width, int n_rot_heads, int D, int rot_dim, float sign, int interleaved, const RopePages<T>& pages,
+                       cudaStream_t s) {
+  if (tokens == 0) return 0;
+  const bool vec_table = (((uintptr_t)cos_c | (uintptr_t)sin_c) & 15) == 0;
+  // (the same count as in the kernel: rotated pairs, and vectors that pass through two by two)
+  const int rotated = n_rot_heads * (rot_dim / 2 / Vec16<T>::N), items = rotated + (width / Vec16<T>::N - 2 * rotated + 1) / 2;
+  const int per_block = items > 0 && items <= ROPE_NARROW ? ROPE_BLOCK / items : 1;
+  const int block = per_block > 1 ? ROPE_BLOCK : items >= 512 ? 512 : (items + 31) / 32 * 32;
+  const unsigned grid = (unsigned)((tokens + per_block - 1) / per_block);
+  auto kern = per_block > 1 ? (vec_table ? rope_kernel<T, true, true, PAGES> : rope_kernel<T, false, true, PAGES>)
+                            : (vec_table ? rope_kernel<T, true, false, PAGES> : rope_kernel<T, false, false, PAGES>);
+  return cb_launch_early(kern, grid, block, 0, s, src, dst, pos, cos_c, sin_c, tokens, per_block, src_stride, width, n_rot_heads, D,
+                         rot_dim, sign, interleaved, pages);
 }
 
 static inline int ew_grid(int64_t items, int block) {
@@ -324,18 +333,25 @@ int cb_glu_bwd(const void* dout, const void* gu, void* dgu, int64_t rows, int I,
 int cb_rope(const void* src, void* dst, const int64_t* pos, const float* cos_c, const float* sin_c, int64_t tokens,
             int64_t src_stride, int width, int n_rot_heads, int D, int rot_dim, float sign, int interleaved, int dtype,
             cudaStream_t s) {
-  if (tokens == 0) return 0;
-  const bool vec_table = (((uintptr_t)cos_c | (uintptr_t)sin_c) & 15) == 0;
   CB_DISPATCH_FLOAT(dtype, T, {
-    // (the same count as in the kernel: rotated pairs, and vectors that pass through two by two)
-    const int rotated = n_rot_heads * (rot_dim / 2 / Vec16<T>::N), items = rotated + (width / Vec16<T>::N - 2 * rotated + 1) / 2;
-    const int per_block = items > 0 && items <= ROPE_NARROW ? ROPE_BLOCK / items : 1;
-    const int block = per_block > 1 ? ROPE_BLOCK : items >= 512 ? 512 : (items + 31) / 32 * 32;
-    const unsigned grid = (unsigned)((tokens + per_block - 1) / per_block);
-    auto kern = per_block > 1 ? (vec_table ? rope_kernel<T, true, true> : rope_kernel<T, false, true>)
-                              : (vec_table ? rope_kernel<T, true, false> : rope_kernel<T, false, false>);
-    return cb_launch_early(kern, grid, block, 0, s, (const T*)src, (T*)dst, pos, cos_c, sin_c, tokens, per_block, src_stride, width,
-                           n_rot_heads, D, rot_dim, sign, interleaved);
+    return (launch_rope<T, false>((const T*)src, (T*)dst, pos, cos_c, sin_c, tokens, src_stride, width, n_rot_heads, D, rot_dim, sign,
+                                  interleaved, RopePages<T>{}, s));
+  });
+  return CB_LAUNCH_CHECK();
+}
+
+// The same of rows q | k | v with kv_heads heads of keys and of values each (n_rot_heads: q and k), 16-bit, forward; keys and values
+// also go to their pages: token t to (tables[token_seq[t]][token_pos[t] / page], token_pos[t] % page).  Pages 16-byte aligned.
+int cb_rope_pages(const void* src, void* dst, const int64_t* pos, const float* cos_c, const float* sin_c, int64_t tokens,
+                  int64_t src_stride, int width, int n_rot_heads, int kv_heads, int D, int rot_dim, int interleaved, int dtype,
+                  void* k_pages, void* v_pages, const int* tables, const int* token_seq, const int* token_pos, int page, int table_width,
+                  cudaStream_t s) {
+  if (width != (n_rot_heads + kv_heads) * D || (dtype != CB_BF16 && dtype != CB_F16)) return (int)cudaErrorInvalidValue;
+  CB_DISPATCH_FLOAT(dtype, T, {
+    const RopePages<T> pages{(T*)k_pages, (T*)v_pages, tables, token_seq, token_pos, page, table_width, kv_heads * D,
+                             (n_rot_heads - kv_heads) * D};
+    return (launch_rope<T, true>((const T*)src, (T*)dst, pos, cos_c, sin_c, tokens, src_stride, width, n_rot_heads, D, rot_dim, 1.f,
+                                 interleaved, pages, s));
   });
   return CB_LAUNCH_CHECK();
 }

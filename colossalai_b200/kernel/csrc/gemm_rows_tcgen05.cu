@@ -1,6 +1,8 @@
 // y = x w^T (+ residual) for a few token rows on sm_100a: the projections of a decode step.  And its embedding lookup.
 //
 //   x [M, K] 16-bit, M <= 32; w [N, K] (torch.nn.Linear's layout); y [M, N]; residual [M, N], added before the rounding
+//   gated unit: w [2 N, K], gate rows before up rows; y = act(x gate^T) (x up^T), both rounded to 16 bits first, as a projection and
+//   the unit behind it would leave them
 //
 // Bound: HBM - every weight is read once and meets a handful of rows.  The product is computed transposed, 128 rows of w being the
 // M of tcgen05.mma and the tokens, padded to 16 or 32, its N, so that the tensor pipe needs an eighth of the time the loads
@@ -17,6 +19,7 @@
 // There is no lower bound on the matrix: alone cuBLAS is ahead by 0.1 - 0.3 us at 1536 x 1024, but in a step the early launches are
 // worth more.  Two layers of 1024 x 2816, 5 sequences, with cuBLAS for the projections 103 us, with this 87; four of them, one
 // sequence 198 and 141.
+#include "activations.cuh"
 #include "checked_id.h"
 #include "common.cuh"
 #include "sm100.cuh"
@@ -26,7 +29,8 @@ using namespace sm100;
 namespace {
 
 constexpr int UMMA_K = 16;
-constexpr int TILE = 128;              // rows of w
+constexpr int TILE = 128;              // rows of w; of a gated unit half of them gate, half up
+constexpr int HALF = TILE / 2;
 constexpr int BK = 64;
 constexpr int ROWS_THREADS = 192;      // producer, issuer, four epilogue warps
 constexpr int W_BYTES = TILE * BK * 2;
@@ -40,7 +44,7 @@ template <int NT> struct RowsCfg {
 };
 
 struct RowsParams {
-  int M, N, k_blocks, per_split;       // k-blocks in all / of one CTA of the cluster
+  int M, N, k_blocks, per_split;       // N: columns of y; k-blocks in all / of one CTA of the cluster
   int packed;                          // rows of y are 8-byte aligned
   int64_t ldy, ldr;
   void* y;
@@ -64,11 +68,15 @@ SM100_DEVICE float4 load_cluster_v4(uint32_t addr) {
   return v;
 }
 
-template <typename T, int NT>
+// ACT: of a gated unit, as in activations.cuh, or PLAIN.  Its tile is HALF gate rows and the HALF up rows that belong to them, in two boxes,
+// so that a CTA has both sides of a product of the unit.  (The unit in a launch of its own cost a decode step 2 us a layer; elementwise.cu.)
+constexpr int PLAIN = -1;
+template <typename T, int NT, int ACT>
 __global__ void __launch_bounds__(ROWS_THREADS, 2)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const RowsParams p) {
   using C = RowsCfg<NT>;
   constexpr int STAGES = C::STAGES;
+  constexpr bool GATED = ACT != PLAIN;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* smem_w = smem;
   uint8_t* smem_x = smem + STAGES * W_BYTES;
@@ -82,14 +90,17 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const int splits = gridDim.y, split = blockIdx.y;          // a cluster is one tile's splits
-  const int n0 = blockIdx.x * TILE;
+  const int n0 = blockIdx.x * (GATED ? HALF : TILE);         // first column of y
   const int kb0 = split * p.per_split, kbs = max(0, min(p.k_blocks - kb0, p.per_split));
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (warp == 0 && lane == 0) {
     prefetch_tensormap(&tmap_w);
     prefetch_tensormap(&tmap_x);
-    for (int i = 0; i < min(kbs, STAGES); ++i) prefetch_l2_2d(&tmap_w, (kb0 + i) * BK, n0);
+    for (int i = 0; i < min(kbs, STAGES); ++i) {
+      prefetch_l2_2d(&tmap_w, (kb0 + i) * BK, n0);
+      if (GATED) prefetch_l2_2d(&tmap_w, (kb0 + i) * BK, p.N + n0);
+    }
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
@@ -116,6 +127,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         if (!ok) break;
         mbar_arrive_expect_tx(&full[stage], W_BYTES + C::X_BYTES);
         tma_load_2d(&tmap_w, &full[stage], smem_w + stage * W_BYTES, (kb0 + i) * BK, n0);
+        if (GATED) tma_load_2d(&tmap_w, &full[stage], smem_w + stage * W_BYTES + W_BYTES / 2, (kb0 + i) * BK, p.N + n0);
         tma_load_2d(&tmap_x, &full[stage], smem_x + stage * C::X_BYTES, (kb0 + i) * BK, 0);
         ++issued;
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -159,7 +171,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 #pragma unroll
       for (int t = 0; t < NT; ++t) v[t] = ok ? 0u : 0x7fffffffu;
     }
-    if (splits == 1) {
+    if (!GATED && splits == 1) {
       const int n = n0 + r;
       if (n < p.N) {
         T* y = reinterpret_cast<T*>(p.y) + n;
@@ -172,25 +184,42 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     } else {
 #pragma unroll
       for (int t = 0; t < NT; ++t) part[t * TILE + r] = __uint_as_float(v[t]);
+      if (splits == 1) asm volatile("bar.sync 1, 128;" ::: "memory");        // the epilogue's own warps
     }
   }
-  if (splits > 1) {
-    cluster_sync();
+  if (GATED || splits > 1) {
+    if (splits > 1) cluster_sync();
     if (warp >= 2) {
       // four rows of w at a time, of one token; every CTA has its share of neighbours.  All parts of a sum are asked for before
       // the first is added: one after the other the sums of 32 tokens took 3 us.
-      const int groups = TILE / 4 * p.M, share = (groups + splits - 1) / splits;
+      constexpr int COLS = GATED ? HALF : TILE;
+      const int groups = COLS / 4 * p.M, share = (groups + splits - 1) / splits;
       for (int e = split * share + threadIdx.x - 64; e < min(groups, (split + 1) * share); e += 128) {
-        const int t = e / (TILE / 4), r = e % (TILE / 4) * 4, n = n0 + r;
+        const int t = e / (COLS / 4), r = e % (COLS / 4) * 4, n = n0 + r;
         const uint32_t at = smem_u32(part + t * TILE + r);
         float4 v[MAX_SPLITS];
+        auto ask = [&](uint32_t from) {
 #pragma unroll
-        for (int s = 0; s < MAX_SPLITS; ++s)
-          if (s < splits) v[s] = load_cluster_v4(map_to_cta(at, s));
-        float sum[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+          for (int s = 0; s < MAX_SPLITS; ++s)
+            if (s < splits) v[s] = load_cluster_v4(map_to_cta(from, s));
+        };
+        auto add_up = [&](float (&sum)[4]) {
+          sum[0] = v[0].x; sum[1] = v[0].y; sum[2] = v[0].z; sum[3] = v[0].w;
 #pragma unroll
-        for (int s = 1; s < MAX_SPLITS; ++s)
-          if (s < splits) { sum[0] += v[s].x; sum[1] += v[s].y; sum[2] += v[s].z; sum[3] += v[s].w; }
+          for (int s = 1; s < MAX_SPLITS; ++s)
+            if (s < splits) { sum[0] += v[s].x; sum[1] += v[s].y; sum[2] += v[s].z; sum[3] += v[s].w; }
+        };
+        float sum[4];
+        ask(at);
+        add_up(sum);
+        if (GATED) {
+          float up[4];
+          ask(at + HALF * 4);
+          add_up(up);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            sum[i] = act_f<GATED ? ACT : 0>(to_f32<T>(from_f32<T>(sum[i]))) * to_f32<T>(from_f32<T>(up[i]));
+        }
         T* y = reinterpret_cast<T*>(p.y) + t * p.ldy + n;
         const T* res = reinterpret_cast<const T*>(p.residual) + t * p.ldr + n;
         union { uint2 raw; T v[4]; } o;
@@ -205,7 +234,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
       }
     }
-    cluster_sync();                                                          // nobody leaves while its sums are read
+    if (splits > 1) cluster_sync();                                          // nobody leaves while its sums are read
   }
   tc_fence_before();
   __syncthreads();
@@ -221,10 +250,10 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(const int64_t* __restri
   for (int i = threadIdx.x; i < vecs; i += 256) dst[i] = src[i];
 }
 
-template <typename T, int NT>
+template <typename T, int NT, int ACT>
 int launch_rows(const CUtensorMap& tw, const CUtensorMap& tx, const RowsParams& p, int tiles, int splits, cudaStream_t stream) {
   static CbDeviceAttr attr;
-  if (const int e = cb_allow_smem(attr, gemm_rows_kernel<T, NT>, RowsCfg<NT>::SMEM)) return e;
+  if (const int e = cb_allow_smem(attr, gemm_rows_kernel<T, NT, ACT>, RowsCfg<NT>::SMEM)) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles, splits);
   cfg.blockDim = dim3(ROWS_THREADS);
@@ -239,23 +268,19 @@ int launch_rows(const CUtensorMap& tw, const CUtensorMap& tx, const RowsParams& 
   at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return cb_launch_error(cudaLaunchKernelEx(&cfg, gemm_rows_kernel<T, NT>, tw, tx, p));
+  return cb_launch_error(cudaLaunchKernelEx(&cfg, gemm_rows_kernel<T, NT, ACT>, tw, tx, p));
 }
 
-}  // namespace
-
-extern "C" {
-
-// x [M, K] (row stride ldx), w [N, K] contiguous, y [M, N] (row stride ldy), residual [M, N] (row stride ldr) or null.  M <= 32;
-// K, ldx multiples of 8 and x, w 16-byte aligned (TMA).
-int cb_gemm_rows(const void* x, const void* w, void* y, const void* residual, int M, int N, int K, int64_t ldx, int64_t ldy, int64_t ldr,
-                 int dtype, cudaStream_t stream) {
+// N columns of y, w_rows of w
+template <int ACT>
+int rows_product(const void* x, const void* w, void* y, const void* residual, int M, int N, int w_rows, int K, int64_t ldx, int64_t ldy,
+                 int64_t ldr, int dtype, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (M > 32 || K <= 0 || (K & 7) || (ldx & 7) || (dtype != CB_BF16 && dtype != CB_F16)) return (int)cudaErrorInvalidValue;
   const bool bf16 = dtype == CB_BF16;
-  const int nt = M <= 16 ? 16 : 32;
+  const int nt = M <= 16 ? 16 : 32, columns = ACT == PLAIN ? TILE : HALF;
   CUtensorMap tw, tx;
-  int r = make_tmap_2d_16b(&tw, w, N, K, K, TILE, BK, bf16);
+  int r = make_tmap_2d_16b(&tw, w, w_rows, K, K, columns, BK, bf16);
   if (r) return 1000 + r;
   r = make_tmap_2d_16b(&tx, x, M, K, ldx, nt, BK, bf16);
   if (r) return 2000 + r;
@@ -267,13 +292,34 @@ int cb_gemm_rows(const void* x, const void* w, void* y, const void* residual, in
   // as many CTAs as run at once, two on an SM, none of fewer than four k-blocks.  A second round of a few costs a round, and
   // clusters of other sizes than powers of two find their SMs late: 6144 x 4096 in 384 CTAs of 8 splits 15.5 us, in 288 of 6 14.9,
   // in 192 of 4 11.5.
-  const int tiles = (N + TILE - 1) / TILE;
+  const int tiles = (N + columns - 1) / columns;
   int splits = 1;
   while (splits < MAX_SPLITS && tiles * splits <= cb_num_sms() && p.k_blocks >= splits * 8) splits *= 2;
   p.per_split = (p.k_blocks + splits - 1) / splits;
   if (nt == 16)
-    return bf16 ? launch_rows<__nv_bfloat16, 16>(tw, tx, p, tiles, splits, stream) : launch_rows<__half, 16>(tw, tx, p, tiles, splits, stream);
-  return bf16 ? launch_rows<__nv_bfloat16, 32>(tw, tx, p, tiles, splits, stream) : launch_rows<__half, 32>(tw, tx, p, tiles, splits, stream);
+    return bf16 ? launch_rows<__nv_bfloat16, 16, ACT>(tw, tx, p, tiles, splits, stream) : launch_rows<__half, 16, ACT>(tw, tx, p, tiles, splits, stream);
+  return bf16 ? launch_rows<__nv_bfloat16, 32, ACT>(tw, tx, p, tiles, splits, stream) : launch_rows<__half, 32, ACT>(tw, tx, p, tiles, splits, stream);
+}
+
+}  // namespace
+
+extern "C" {
+
+// x [M, K] (row stride ldx), w [N, K] contiguous, y [M, N] (row stride ldy), residual [M, N] (row stride ldr) or null.  M <= 32;
+// K, ldx multiples of 8 and x, w 16-byte aligned (TMA).
+int cb_gemm_rows(const void* x, const void* w, void* y, const void* residual, int M, int N, int K, int64_t ldx, int64_t ldy, int64_t ldr,
+                 int dtype, cudaStream_t stream) {
+  return rows_product<PLAIN>(x, w, y, residual, M, N, N, K, ldx, ldy, ldr, dtype, stream);
+}
+
+// The gated unit behind a projection: w [2 N, K], y [M, N]; act: 0 silu, 1 gelu (tanh), 2 gelu (erf)
+int cb_gemm_rows_gated(const void* x, const void* w, void* y, int M, int N, int K, int64_t ldx, int64_t ldy, int act, int dtype,
+                       cudaStream_t stream) {
+  if (N > 0x3fffffff) return (int)cudaErrorInvalidValue;
+  if (act == 0) return rows_product<0>(x, w, y, nullptr, M, N, 2 * N, K, ldx, ldy, 0, dtype, stream);
+  if (act == 1) return rows_product<1>(x, w, y, nullptr, M, N, 2 * N, K, ldx, ldy, 0, dtype, stream);
+  if (act == 2) return rows_product<2>(x, w, y, nullptr, M, N, 2 * N, K, ldx, ldy, 0, dtype, stream);
+  return (int)cudaErrorInvalidValue;
 }
 
 // table [entries, row_bytes], out [n, row_bytes]; row_bytes a multiple of 16, both 16-byte aligned

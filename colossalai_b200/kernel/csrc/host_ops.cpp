@@ -53,6 +53,8 @@ struct Launchers {
   int (*glu_bwd)(const void*, const void*, void*, int64_t, int, int, int, const int64_t*, cudaStream_t);
   int (*rope)(const void*, void*, const int64_t*, const float*, const float*, int64_t, int64_t, int, int, int, int, float, int, int,
               cudaStream_t);
+  int (*rope_pages)(const void*, void*, const int64_t*, const float*, const float*, int64_t, int64_t, int, int, int, int, int, int, int, void*,
+                    void*, const int*, const int*, const int*, int, int, cudaStream_t);
   int (*row_stats)(const void*, const int64_t*, float*, int, int, int, int64_t, int64_t, int, cudaStream_t);
   int (*ce_loss_blocks)(int);
   int (*ce_loss)(const float*, const int64_t*, float*, int64_t*, void*, int, int64_t, int, cudaStream_t);
@@ -63,6 +65,7 @@ struct Launchers {
   int (*flash_bwd)(const void*, const void*, const void*, const void*, const void*, const float*, void*, void*, void*, float*,
                    float*, int, int, int, int, int, int, float, int, const int*, long long, cudaStream_t);
   int (*gemm_rows)(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, cudaStream_t);
+  int (*gemm_rows_gated)(const void*, const void*, void*, int, int, int, int64_t, int64_t, int, int, cudaStream_t);
   int (*embed_rows)(const int64_t*, const void*, void*, int64_t, int64_t, int64_t, cudaStream_t);
   int (*decode_splits)(int, int, int, int*);
   int (*decode)(const void*, const void*, const void*, const int*, const int*, void*, float*, float*, int, int, int, int, int, int,
@@ -197,6 +200,21 @@ struct Rope : torch::autograd::Function<Rope> {
   }
 };
 
+// a decode step's rows q | k | v [T, (Hq + 2 Hkv) D], rotated, their keys and values also in the pages [pages, page, Hkv, D] (16-byte
+// aligned) that tables int32 [sequences, width] name; rows that are strided as wholes are read where they lie
+Tensor rope_pages(const Tensor& x, const Tensor& pos, const Tensor& cos, const Tensor& sin, int64_t Hq, int64_t rot, bool interleaved,
+                  const Tensor& k_pages, const Tensor& v_pages, const Tensor& tables, const Tensor& token_seq, const Tensor& token_pos) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t Hkv = k_pages.size(2), D = k_pages.size(3), T = x.size(0), width = x.size(1), vec = 16 / x.element_size();
+  const Tensor rows = x.stride(1) == 1 && x.stride(0) % vec == 0 && reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 16 == 0 ? x : packed(x);
+  Tensor out = at::empty(x.sizes(), x.options());
+  launched(L.rope_pages(ptr(rows), mut(out), as<int64_t>(pos), as<float>(cos), as<float>(sin), T, rows.stride(0), (int)width, (int)(Hq + Hkv),
+                        (int)Hkv, (int)D, (int)rot, interleaved, code_of(x), mut(k_pages), mut(v_pages), as<int>(tables), as<int>(token_seq),
+                        as<int>(token_pos), (int)k_pages.size(1), (int)tables.size(1), stream_of(x)),
+           n_rope);
+  return out;
+}
+
 // ------------------------------------------------------------------------------------------------ cross entropy
 // one vocabulary shard: logits [T, V] contiguous, target int64 [T] contiguous
 struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
@@ -307,6 +325,14 @@ Tensor linear_rows(const Tensor& x, const Tensor& w, const OptTensor& residual) 
   launched(L.gemm_rows(ptr(x), ptr(w), mut(y), add ? ptr(*residual) : nullptr, M, N, K, x.stride(0), N, add ? residual->stride(0) : 0,
                        code_of(x), stream_of(x)),
            n_rows);
+  return y;
+}
+// x [M, K], w [2 N, K] -> act(x gate^T) (x up^T) [M, N]
+Tensor gated_rows(const Tensor& x, const Tensor& w, int64_t act) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int M = (int)x.size(0), K = (int)x.size(1), N = (int)(w.size(0) / 2);
+  Tensor y = at::empty({M, N}, x.options());
+  launched(L.gemm_rows_gated(ptr(x), ptr(w), mut(y), M, N, K, x.stride(0), N, (int)act, code_of(x), stream_of(x)), n_rows);
   return y;
 }
 // ids [n] int64, table [entries, H]
@@ -449,6 +475,7 @@ void bind(const std::map<std::string, uint64_t>& t) {
   take(t, "cb_glu_fwd_bounded", L.glu_fwd);
   take(t, "cb_glu_bwd_bounded", L.glu_bwd);
   take(t, "cb_rope", L.rope);
+  take(t, "cb_rope_pages", L.rope_pages);
   take(t, "cb_ce_row_stats", L.row_stats);
   take(t, "cb_ce_loss_blocks", L.ce_loss_blocks);
   take(t, "cb_ce_loss", L.ce_loss);
@@ -456,6 +483,7 @@ void bind(const std::map<std::string, uint64_t>& t) {
   take(t, "cb_flash_attn_varlen_fwd", L.flash_varlen_fwd);
   take(t, "cb_flash_attn_bwd", L.flash_bwd);
   take(t, "cb_gemm_rows", L.gemm_rows);
+  take(t, "cb_gemm_rows_gated", L.gemm_rows_gated);
   take(t, "cb_embed_rows", L.embed_rows);
   take(t, "cb_decode_num_splits", L.decode_splits);
   take(t, "cb_paged_decode_attention", L.decode);
@@ -495,6 +523,7 @@ PYBIND11_MODULE(cb200_host, m) {
         [](const Tensor& x, const Tensor& pos, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t D, int64_t rot,
            bool interleaved) { return Rope::apply(x, pos, cos, sin, heads, D, rot, interleaved); },
         release());
+  m.def("rope_pages", &rope_pages, release());
   m.def("cross_entropy",
         [](const Tensor& x, const Tensor& t, int64_t ignore, int64_t start, int64_t valid, bool mean) {
           return CrossEntropy::apply(x, t, ignore, start, valid, mean);
@@ -507,6 +536,7 @@ PYBIND11_MODULE(cb200_host, m) {
         release());
   m.def("paged_decode", &paged_decode, release());
   m.def("linear_rows", &linear_rows, release());
+  m.def("gated_rows", &gated_rows, release());
   m.def("embed_rows", &embed_rows, release());
   m.def("sort_choices", &sort_choices, release());
   m.def("take_rows", [](const Tensor& x, const Tensor& slot, const Tensor& src, int64_t k) { return TakeRows::apply(x, slot, src, k); },

@@ -172,9 +172,13 @@ class Attention(nn.Module):
             q = self._head_norm(self.q_norm, q.reshape(T, hq, D)).reshape(T, hq * D)
             k = self._head_norm(self.k_norm, k.reshape(T, hkv, D)).reshape(T, hkv * D)
             qkv = torch.cat([q, k, v], dim=-1)
+        written = None
         if rope is not None:
-            qkv = ops.rope_qkv(qkv, meta.positions, rope[0], rope[1], hq, hkv, D, rot_dim=cfg.rotary_dim,
-                               interleaved=cfg.rope_interleaved)
+            if hasattr(kv_cache, "rotate_and_write"):
+                written = kv_cache.rotate_and_write(self.layer_idx, qkv, meta.positions, rope[0], rope[1], hq, hkv, D, cfg.rotary_dim,
+                                                    cfg.rope_interleaved)
+            qkv = written if written is not None else ops.rope_qkv(qkv, meta.positions, rope[0], rope[1], hq, hkv, D,
+                                                                   rot_dim=cfg.rotary_dim, interleaved=cfg.rope_interleaved)
         q, k, v = qkv.split([hq * D, hkv * D, hkv * D], dim=-1)
         q, k, v = q.reshape(T, hq, D), k.reshape(T, hkv, D), v.reshape(T, hkv, D)
         if kv_cache is not None:
@@ -182,6 +186,8 @@ class Attention(nn.Module):
             extra = {} if slopes is None else {"alibi_slopes": slopes}
             if cfg.sliding_window:
                 extra["sliding_window"] = cfg.sliding_window
+            if written is not None:
+                extra["written"] = True
             o = kv_cache.attend(self.layer_idx, q, k, v, meta, self.scale, **extra)
         elif sp_mode == "ring_attn" and comm.group_size(sp_group) > 1:
             o = RingAttention.attention(q, k, v, sp_group, batch=meta.batch, scale=self.scale)
@@ -374,7 +380,7 @@ class MLP(nn.Module):
         elif self.act == "clamped":
             h = ops.clamped_glu(self.gate_up_proj(x), self.limit)
         elif self.cfg.glu:
-            h = ops.glu(ops.linear_rows(self.gate_up_proj, x), self.cfg.hidden_act)
+            h = ops.gated_rows(self.gate_up_proj, x, self.cfg.hidden_act)
         else:
             up = self.up_proj
             if x.is_cuda and x.dtype != torch.float32 and not torch.is_grad_enabled() and up.bias is None \

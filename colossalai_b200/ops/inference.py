@@ -42,6 +42,29 @@ def kv_cache_write(k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_ca
     v_cache[blk, slot] = v.to(v_cache.dtype)
 
 
+def rope_pages(qkv: torch.Tensor, positions: Optional[torch.Tensor], cos: torch.Tensor, sin: torch.Tensor, heads: int, kv_heads: int,
+               dim: int, rot_dim: Optional[int], interleaved: bool, k_cache: torch.Tensor, v_cache: torch.Tensor,
+               block_tables: torch.Tensor, token_seq: torch.Tensor, token_pos: torch.Tensor) -> Optional[torch.Tensor]:
+    """`ops.rope_qkv` and `kv_cache_write` of its keys and values in one launch, for 16-bit rows q | k | v outside autograd; None, and
+    nothing done, for calls that it does not take."""
+    rot = rot_dim or dim
+    if not (use_native(qkv) and qkv.dtype in (torch.float16, torch.bfloat16) and qkv.dim() == 2 and positions is not None
+            and 0 < qkv.shape[0] == positions.numel() == token_pos.numel() == token_seq.numel()):
+        return None
+    tensors = (qkv, positions, cos, sin, k_cache, v_cache, block_tables, token_seq, token_pos)
+    if not plain_call(*tensors) or any(t.device != qkv.device for t in tensors):
+        return None
+    pages = (k_cache, v_cache)
+    if qkv.shape[1] != (heads + 2 * kv_heads) * dim or dim % 8 or rot % 16 or rot > dim or positions.dtype != torch.int64 \
+            or any(t.dtype != qkv.dtype or not t.is_contiguous() or t.dim() != 4 or t.data_ptr() % 16 for t in pages) \
+            or k_cache.shape != v_cache.shape or tuple(k_cache.shape[2:]) != (kv_heads, dim) \
+            or any(t.dtype != torch.int32 or not t.is_contiguous() for t in (block_tables, token_seq, token_pos)) \
+            or any(t.dtype != torch.float32 or not t.is_contiguous() for t in (cos, sin)) or (host := loader.host()) is None:
+        return None
+    return host.rope_pages(qkv, positions.contiguous(), cos, sin, heads, rot, bool(interleaved), k_cache, v_cache, block_tables,
+                           token_seq, token_pos)
+
+
 def _workspace_buffers(q: torch.Tensor):
     from ..inference.flash_decoding_utils import FDIntermTensors
 

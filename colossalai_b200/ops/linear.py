@@ -15,8 +15,9 @@ from torch.nn.modules import module as _module
 
 from ..kernel import loader
 from ._dispatch import plain_call, use_native
+from .activation import glu
 
-__all__ = ["linear_rows", "embed_rows", "unwatched", "ROWS_MAX"]
+__all__ = ["linear_rows", "gated_rows", "embed_rows", "unwatched", "ROWS_MAX"]
 
 ROWS_MAX = 32         # what the kernel takes; figures there
 _LINEAR, _EMBEDDING = nn.Linear.forward, nn.Embedding.forward
@@ -63,6 +64,17 @@ def linear_rows(linear: nn.Module, x: torch.Tensor, residual: Optional[torch.Ten
         return host.linear_rows(x, linear.weight, residual)
     y = linear(x)
     return y if residual is None else residual + y
+
+
+_GATED = {"silu": 0, "swiglu": 0, "gelu_tanh": 1, "gelu_new": 1, "gelu_pytorch_tanh": 1, "gelu": 2, "geglu": 2}
+
+
+def gated_rows(linear: nn.Module, x: torch.Tensor, act: str) -> torch.Tensor:
+    """glu(linear(x), act), the unit in the projection's epilogue where that is the framework's own kernel: a decode step then has one launch
+    less a layer, with the same roundings."""
+    if act in _GATED and _native(linear, x, None) and linear.weight.shape[0] % 16 == 0 and (host := loader.host()) is not None:
+        return host.gated_rows(x, linear.weight, _GATED[act])
+    return glu(linear_rows(linear, x), act)
 
 
 def _native_lookup(embedding: nn.Module, ids: torch.Tensor) -> bool:

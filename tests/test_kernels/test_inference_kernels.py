@@ -285,3 +285,37 @@ def test_paged_decode_more_than_eight_kv_heads(dtype, D, Hkv, group, window):
     ref = iops.paged_decode_attention_ref(q.double(), kc, vc, tables, lens, window=window).double()
     # every head of every sequence: weights rounded to 16 bits (bf16: 2^-9 each), the result once more
     assert ((out - ref).norm(dim=-1) <= 6e-3 * ref.norm(dim=-1)).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,kv,D,rot,interleaved", [(32, 8, 128, 128, False), (4, 2, 64, 32, False), (3, 1, 128, 64, True), (2, 2, 16, 16, False),
+                                                        (1, 1, 64, 64, True)])
+@pytest.mark.parametrize("tokens,page", [(1, 16), (5, 16), (300, 7)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_rotation_with_page_write(heads, kv, D, rot, interleaved, tokens, page, dtype):
+    """Rotation and page write in one launch: the bits of both, one after the other, and nothing else in the pages, from rows that are a
+    part of wider ones and with several tokens a sequence."""
+    from colossalai_b200 import ops
+    from colossalai_b200.ops import inference
+
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    width = (heads + 2 * kv) * D
+    qkv = torch.randn(tokens, width + 16, device="cuda", generator=g).to(dtype)[:, 8:8 + width]
+    seqs, most = (tokens + 1) // 2, 3 * page
+    tables = torch.randperm(seqs * 3, device="cuda", generator=g).to(torch.int32).view(seqs, 3)
+    seq = (torch.arange(tokens, device="cuda") // 2).to(torch.int32)
+    pos = (torch.randint(0, most // 2, (tokens,), device="cuda", generator=g) * 2 + torch.arange(tokens, device="cuda") % 2).clamp(max=most - 1)
+    cos, sin = ops.build_rope_cache(most, rot, 1e4, device="cuda")
+    pages = [torch.randn(seqs * 3, page, kv, D, device="cuda", generator=g).to(dtype) for _ in "kv"]
+    want = ops.rope_qkv(qkv, pos, cos, sin, heads, kv, D, rot_dim=rot, interleaved=interleaved)
+    kw, vw = pages[0].clone(), pages[1].clone()
+    _, k, v = (t.view(tokens, -1, D) for t in want.split([heads * D, kv * D, kv * D], -1))
+    inference.kv_cache_write(k, v, kw, vw, tables, seq, pos.to(torch.int32))
+    args = (qkv, pos, cos, sin, heads, kv, D, rot, interleaved, *pages, tables, seq, pos.to(torch.int32))
+    with torch.no_grad():
+        got = inference.rope_pages(*args)
+    assert torch.equal(got, want) and torch.equal(pages[0], kw) and torch.equal(pages[1], vw)
+    refused = [(0, qkv.float()), (0, qkv[:, 8:]), (1, None), (1, pos.int()), (9, pages[0].float()), (10, pages[1][:, :, :, : D // 2]), (11, tables.long()),
+               (2, cos.half())]
+    assert all(inference.rope_pages(*(value if i == at else a for i, a in enumerate(args))) is None for at, value in refused)
+    assert torch.equal(pages[0], kw) and torch.equal(pages[1], vw)

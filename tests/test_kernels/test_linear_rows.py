@@ -39,6 +39,35 @@ def test_rows_match_64_bits(rows, N, K, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 16, 17, 32])
+@pytest.mark.parametrize("I,K", [(8, 8), (64, 64), (72, 200), (704, 1096), (1408, 2048), (9472, 256), (256, 14336), (9536, 512), (512, 2112)])
+@pytest.mark.parametrize("dtype,act", [(torch.bfloat16, "silu"), (torch.float16, "gelu_tanh"), (torch.bfloat16, "gelu")])
+def test_gated_rows(rows, I, K, dtype, act):
+    """The unit in the projection's epilogue against projection and unit one after the other: the same bits where both cut the matrix into
+    the same tiles (multiples of 64), otherwise up to the order of fp32 sums, which may turn a rounding of either factor."""
+    from colossalai_b200 import ops
+    from colossalai_b200.kernel import launch_counter
+
+    g = torch.Generator(device="cuda").manual_seed(I + K)
+    lin = nn.Linear(K, 2 * I, bias=False, device="cuda", dtype=dtype)
+    x = torch.randn(rows, K + 24, device="cuda", generator=g).to(dtype)[:, 8:8 + K]
+    with torch.no_grad():
+        want = ops.glu(ops.linear_rows(lin, x), act)
+        launch_counter.reset()
+        y = ops.gated_rows(lin, x, act)
+        assert dict(launch_counter.by_name) == {"gemm_rows": 1}
+        assert torch.equal(ops.gated_rows(lin, x[rows - 1:], act)[0], y[-1])
+    assert y.shape == want.shape and y.dtype == dtype
+    if I % 64 == 0:
+        assert torch.equal(y, want)
+    else:
+        unit = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+        assert ((y - want).abs() <= 6 * unit * want.abs() + 1e-6).all()       # a unit of each factor and of the result, twice over
+    y = ops.gated_rows(lin, x, act)                                           # autograd: the module and the unit
+    assert y.requires_grad
+
+
+@pytest.mark.gpu
 def test_calls_that_stay_with_the_module():
     """Autograd, hooks, a bias, many rows, other types and subclasses, rows that TMA cannot address: the module's own result."""
     from colossalai_b200.ops import linear as L
