@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(512) ce_softmax_grad_kernel(const T* __restric
                                                               int V, int Vv, int64_t vocab_start,
                                                               int64_t ignore_index) {
   constexpr int VEC = Vec16<T>::N;
-  const int r = blockIdx.x;
+  const int r = gridDim.x - 1 - blockIdx.x;                    // from the end: what the forward read last is in L2 yet (533 -> 526 us)
   const T* row = x + (size_t)r * V;
   T* grow = g + (size_t)r * V;
   const int64_t t = target[r];
@@ -148,17 +148,39 @@ __global__ void __launch_bounds__(512) ce_softmax_grad_kernel(const T* __restric
   const float m = gmax[r], inv = ignored ? 0.f : f / sumexp[r];
   const float sc = ignored ? 0.f : f;
   const int64_t local = t - vocab_start;
-  for (int c = threadIdx.x * VEC; c < V; c += blockDim.x * VEC) {
-    Vec16<T> v, o;
-    v.load_nc(row + c);
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      float p = (c + i < Vv) ? __expf(v.get(i) - m) * inv : 0.f;
-      if ((int64_t)(c + i) == local) p -= sc;
-      o.set(i, p);
-    }
-    o.store_na(grow + c);
+  // Without a label every gradient is an exponential times zero: zero, unless one is not finite, which the maximum and the sum show
+  // (a sum that is zero: a row of -inf).  The logits are not read again then; 4096 x 128256 bf16, a third of them: 532 -> 478 us.
+  if (ignored && fabsf(m) < INFINITY && sumexp[r] > 0.f && sumexp[r] < INFINITY) {
+    Vec16<T> o;
+    o.raw = make_uint4(0u, 0u, 0u, 0u);
+    for (int c = threadIdx.x * VEC; c < V; c += blockDim.x * VEC) o.store_na(grow + c);
+    return;
   }
+  constexpr int STEP = 512 * VEC;
+  constexpr int UNROLL = sizeof(T) == 4 ? 1 : CE_UNROLL;       // 4096 x 128256 bf16, all with labels: one vector 560 us (with the forward), four 528; fp32
+                                                               // 1700 x 151936 496 and 498
+  auto part = [&](int c0, auto whole_tag) {      // (a copy of the code for a row's end, as above)
+    constexpr bool WHOLE = decltype(whole_tag)::value;
+    Vec16<T> v[UNROLL], o;
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u)
+      if (WHOLE || c0 + u * STEP < V) v[u].load_nc(row + c0 + u * STEP);
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      const int c = c0 + u * STEP;
+      if (!WHOLE && c >= V) break;
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) {
+        float p = (WHOLE || c + i < Vv) ? __expf(v[u].get(i) - m) * inv : 0.f;
+        if ((int64_t)(c + i) == local) p -= sc;
+        o.set(i, p);
+      }
+      o.store_na(grow + c);
+    }
+  };
+  int c0 = threadIdx.x * VEC;
+  for (; c0 + (UNROLL - 1) * STEP + VEC <= Vv; c0 += UNROLL * STEP) part(c0, std::true_type{});
+  for (; c0 < V; c0 += UNROLL * STEP) part(c0, std::false_type{});
 }
 
 extern "C" {

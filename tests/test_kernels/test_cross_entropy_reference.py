@@ -57,3 +57,27 @@ def _shards(rank, world_size, port):
 @rerun_if_address_is_in_use()
 def test_vocab_shards_without_a_finite_column():
     spawn(_shards, 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V", [8, 1000, 4096, 16384, 16392, 20488])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gradient_of_rows_without_a_label(V, dtype):
+    """Zero where every logit is finite (or minus infinity beside finite ones) and NaN where the exponentials against the row's maximum
+    are not numbers, between rows with labels; sizes on and beside what a block's threads hold at a time."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn(8, V, device="cuda", generator=g).to(dtype)
+    x[1, 3], x[2, 5], x[4, 2], x[6] = float("nan"), float("inf"), -float("inf"), -float("inf")
+    labels = torch.full((8,), -100, device="cuda")
+    labels[0], labels[7], labels[5] = V - 1, 0, 2
+    z = x.clone().requires_grad_(True)
+    (grad,) = torch.autograd.grad(cross_entropy_1d(z, labels, process_group="local"), z)
+    top = torch.where(x.isnan(), -float("inf"), x).amax(-1, keepdim=True).double()
+    want = (x.double() - top).exp() * 0.0
+    keep = labels >= 0
+    want[keep] = (x[keep].double().softmax(-1) - torch.nn.functional.one_hot(labels[keep], V)) / 3
+    assert torch.equal(grad.isnan(), want.isnan()) and int(grad.isnan().sum()) == V + 2
+    # a rounding to the type, and of the exponential and the sum in fp32
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
+    assert ((grad.double() - want).abs()[~want.isnan()] <= unit * want.abs()[~want.isnan()] + 1e-9).all()
+    assert not grad[3].any() and not grad[4].any()
