@@ -37,28 +37,27 @@ constexpr int UMMA_K = 16;
 constexpr int ROWS_THREADS = 192;      // producer, issuer, four epilogue warps
 constexpr int WGRAD_THREADS = 320;     // .., eight
 constexpr int BOX_ROWS = 32;           // token rows of the smaller TMA box: a request takes as long to issue as one of 64 rows
-constexpr int ROWS_BOX = 64;           // of the larger one, variable-M modes (weight gradients: a k-block)
+constexpr int ROWS_BOX = 64;           // of the larger one, variable-M modes (weight gradients: a k-block, as many)
 constexpr int PAIR_M = 256;
 constexpr int PAIR_N = 256;
 constexpr int MAX_GROUPS = 512;
 enum { MODE_NT = 0, MODE_NN = 1, MODE_TN = 2 };
-// K-blocks and stages.  The same bytes are in flight: a tile of few rows is bound by its loads and takes them in smaller pieces
-// (forward 347 and 337 us, input gradients 367 and 361 for the layers above), a weight gradient, three blocks long, in larger ones
-// (468, 496 with the smaller).
+// K-blocks and stages.  A tile of few rows is bound by its loads and takes them in small pieces (two layers of 64 experts, 2048 x 2816 and 1408 x
+// 2048: K-blocks of 128 forward 347 us, input gradients 367; of 64 337 and 361).  A weight gradient gives a stage for second boxes of
+// its epilogue (blocks of 96 and three stages: 498, 482 so).
+constexpr int BK = 64;
 template <int MODE> struct Block {
-  static constexpr int K = MODE == MODE_TN ? 128 : 64;
-  static constexpr int STAGES = MODE == MODE_TN ? 3 : 6;
-  static constexpr int A_BYTES = 128 * K * 2, B_BYTES = 128 * K * 2;
+  static constexpr int STAGES = MODE == MODE_TN ? 5 : 6;
+  static constexpr int A_BYTES = 128 * BK * 2, B_BYTES = 128 * BK * 2;
 };
-constexpr int STAGE_RING = 6 * 32 * 1024;
-static_assert(Block<MODE_NT>::STAGES * (Block<MODE_NT>::A_BYTES + Block<MODE_NT>::B_BYTES) == STAGE_RING, "");
-static_assert(Block<MODE_TN>::STAGES * (Block<MODE_TN>::A_BYTES + Block<MODE_TN>::B_BYTES) == STAGE_RING, "");
-// behind the stages: the staging of the epilogue (weight gradients: a 32 x 64 box per epilogue warp; variable-M modes: 32 rows x
+template <int MODE> constexpr int stage_ring() { return Block<MODE>::STAGES * (Block<MODE>::A_BYTES + Block<MODE>::B_BYTES); }
+constexpr int BOXES = 2;               // of an epilogue warp of weight gradients
+// behind the stages: the staging of the epilogue (weight gradients: BOXES of 32 x 64 per epilogue warp; variable-M modes: 32 rows x
 // 32 columns per warp), the barriers, the groups' boundaries and the tile list of the variable-M modes
 constexpr int BOX_BYTES = 32 * 128;
 constexpr int ROW_BOX_BYTES = 32 * 64;
 template <int MODE> constexpr int smem_bytes() {
-  return STAGE_RING + 256 + (MAX_GROUPS + 1) * 4 + (MODE == MODE_TN ? 8 * BOX_BYTES : 4 * ROW_BOX_BYTES + (MAX_GROUPS + 1) * 4);
+  return stage_ring<MODE>() + 256 + (MAX_GROUPS + 1) * 4 + (MODE == MODE_TN ? 8 * BOXES * BOX_BYTES : 4 * ROW_BOX_BYTES + (MAX_GROUPS + 1) * 4);
 }
 
 SM100_DEVICE void tma_store_3d(const CUtensorMap* map, const void* smem_src, int32_t c0, int32_t c1, int32_t c2) {
@@ -146,11 +145,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROWS_THREADS, 1)
 grouped_rows_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                          const __grid_constant__ CUtensorMap tmap_x32, const GroupedParams p) {
   constexpr bool A_MN = MODE == MODE_NN;
-  constexpr int BK = Block<MODE>::K, STAGES = Block<MODE>::STAGES, A_BYTES = Block<MODE>::A_BYTES, B_BYTES = Block<MODE>::B_BYTES;
+  constexpr int STAGES = Block<MODE>::STAGES, A_BYTES = Block<MODE>::A_BYTES, B_BYTES = Block<MODE>::B_BYTES;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * A_BYTES;
-  uint8_t* smem_box = smem + STAGE_RING;                                                // [4 warps]
+  uint8_t* smem_box = smem + stage_ring<MODE>();                                                // [4 warps]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_box + 4 * ROW_BOX_BYTES);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + STAGES;
@@ -345,12 +344,12 @@ grouped_wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
                           const __grid_constant__ CUtensorMap tmap_a32, const __grid_constant__ CUtensorMap tmap_b32,
                           const __grid_constant__ CUtensorMap tmap_c, const GroupedParams p) {
   using B = Block<MODE_TN>;
-  constexpr int BK = B::K, STAGES = B::STAGES, A_BYTES = B::A_BYTES, B_BYTES = B::B_BYTES;
+  constexpr int STAGES = B::STAGES, A_BYTES = B::A_BYTES, B_BYTES = B::B_BYTES;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * A_BYTES;
-  uint8_t* smem_box = smem + STAGE_RING;                                                // [8 warps], 1024-byte aligned
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_box + 8 * BOX_BYTES);
+  uint8_t* smem_box = smem + stage_ring<MODE_TN>();                                                // [8 warps], 1024-byte aligned
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_box + 8 * BOXES * BOX_BYTES);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + STAGES;
   uint64_t* tmem_full = bars + 2 * STAGES;
@@ -358,7 +357,7 @@ grouped_wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   int* bounds = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + 256);         // [E + 1]
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const uint32_t cta_rank = cluster_ctarank();
   const bool leader = cta_rank == 0;
@@ -432,25 +431,26 @@ grouped_wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   } else if (warp == 1) {
     // ================================================================ MMA issuer (leader CTA)
     if (leader) {
+      const uint32_t one = elect_one();
+      const uint64_t da0 = make_smem_desc_sw128(smem_u32(smem_a), BK * 128, 1024), db0 = make_smem_desc_sw128(smem_u32(smem_b), BK * 128, 1024);
       int stage = 0, cur = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       Tile ahead = find_tile<MODE_TN>(pair_id, num_tiles, p, bounds, nullptr, n_blocks, cur);
       for (int t = pair_id; t < num_tiles; t += num_pairs) {
-        const int k_rows = ahead.row_end - ahead.row0;
+        const int k_rows = __shfl_sync(0xffffffffu, ahead.row_end - ahead.row0, 0);
         mbar_wait(&tmem_empty[acc], acc_phase ^ 1);
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * PAIR_N;
         for (int k0 = 0; k0 < k_rows; k0 += BK) {
           mbar_wait(&full_bar[stage], phase);
           tc_fence_after();
-          if (lane == 0) {
-            const uint64_t da = make_smem_desc_sw128(smem_u32(smem_a + stage * A_BYTES), BK * 128, 1024);
-            const uint64_t db = make_smem_desc_sw128(smem_u32(smem_b + stage * B_BYTES), BK * 128, 1024);
+          const uint32_t a = desc_lo(da0) + stage * (A_BYTES >> 4), b = desc_lo(db0) + stage * (B_BYTES >> 4);
 #pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k)              // as many as the group has rows
-              if (k0 + k * UMMA_K < k_rows)
-                umma_f16_ss_2cta(tmem_d, advance_desc(da, k * (UMMA_K * 128)), advance_desc(db, k * (UMMA_K * 128)), p.idesc,
-                                 (k0 > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < BK / UMMA_K; ++k)                // as many as the group has rows
+            if (k0 + k * UMMA_K < k_rows)
+              umma_f16_ss_2cta_warp(one, tmem_d, a + (k * (UMMA_K * 128) >> 4), desc_hi(da0), b + (k * (UMMA_K * 128) >> 4), desc_hi(db0), p.idesc,
+                                    (k0 > 0 || k > 0) ? 1u : 0u);
+          if (one) {
             umma_commit_2cta(&empty_bar[stage], 3);
             if (k0 + BK >= k_rows) umma_commit_2cta(&tmem_full[acc], 3);
           }
@@ -468,7 +468,7 @@ grouped_wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     // ================================================================ epilogue (warps 2..9, both CTAs)
     const int quarter = warp & 3, half = (warp - 2) >> 2;                    // 32 rows x 128 columns of the CTA's 128 x 256
     constexpr int COLS = PAIR_N / 2;
-    uint8_t* box = smem_box + (warp - 2) * BOX_BYTES;
+    uint8_t* const boxes = smem_box + (warp - 2) * BOXES * BOX_BYTES;
     int acc = 0, cur = 0;
     uint32_t acc_phase = 0;
     Tile ahead = find_tile<MODE_TN>(pair_id, num_tiles, p, bounds, nullptr, n_blocks, cur);
@@ -494,7 +494,10 @@ grouped_wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           // sixteen bytes per lane to 32 rows at a time (4096 clocks a tile) bound this mode (two GEMMs of 64 experts x 2048 x
           // 2816 / 1408, 384 rows each: 672 us).  The 32 x 64 box of a warp goes through shared memory in the 128-byte swizzle
           // and leaves as one TMA store, clipped at the expert's edges, the next box read while one is packed (501).  Four warps
-          // took 5000 clocks for a tile whose product takes 3100: eight of them and fewer rows of padding, 465.
+          // took 5000 clocks for a tile whose product takes 3100: eight of them and fewer rows of padding, 465.  Two boxes a warp,
+          // so that one is packed while the other leaves, and a converged issuer: one call after the other 507 -> 482, 64 experts with 28 rows each 291 ->
+          // 277.  Of that 282 are the 1.1 GB that are written, at the 3.9 TB/s that HBM takes from writes alone.  The tiles of three to sixteen experts in
+          // turn, so that large and small reductions meet, were no faster (3: 493, 16: 543).
           uint32_t v[2][64];
           tmem_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&v[0][0]));
           tmem_ld_32x32b_x32(taddr + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[0][32]));
@@ -509,7 +512,8 @@ grouped_wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             } else {
               release();
             }
-            if (lane == 0) tma_store_wait_read<0>();           // the store that last read this box has read it
+            uint8_t* box = boxes + (b % BOXES) * BOX_BYTES;
+            if (lane == 0) tma_store_wait_read<BOXES - 1>();   // the store that last read this box has read it
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -598,7 +602,7 @@ int cb_grouped_gemm(const void* x, const void* w, void* y, const int* offs, int 
     p.w_group_rows = N;
     return bf16 ? launch_rows<MODE_NT, __nv_bfloat16>(tw, tx, tx32, p, stream) : launch_rows<MODE_NT, __half>(tw, tx, tx32, p, stream);
   }
-  r = make_tmap_2d_16b(&tw, w, (uint64_t)E * K, N, N, Block<MODE_NN>::K, 64, bf16);
+  r = make_tmap_2d_16b(&tw, w, (uint64_t)E * K, N, N, BK, 64, bf16);
   if (r) return 2000 + r;
   p.w_group_rows = K;
   return bf16 ? launch_rows<MODE_NN, __nv_bfloat16>(tw, tx, tx32, p, stream) : launch_rows<MODE_NN, __half>(tw, tx, tx32, p, stream);
@@ -612,10 +616,10 @@ int cb_grouped_gemm_wgrad(const void* dy, const void* x, void* dw, const int* of
   if (E > MAX_GROUPS || (in_dtype != CB_BF16 && in_dtype != CB_F16) || (M & 7) || (N & 7)) return (int)cudaErrorInvalidValue;
   const bool bf16 = in_dtype == CB_BF16;
   CUtensorMap ta, tb, ta32, tb32;
-  int r = make_tmap_2d_16b(&ta, dy, total_rows, M, lddy, Block<MODE_TN>::K, 64, bf16);
+  int r = make_tmap_2d_16b(&ta, dy, total_rows, M, lddy, BK, 64, bf16);
   if (!r) r = make_tmap_2d_16b(&ta32, dy, total_rows, M, lddy, BOX_ROWS, 64, bf16);
   if (r) return 1000 + r;
-  r = make_tmap_2d_16b(&tb, x, total_rows, N, ldx, Block<MODE_TN>::K, 64, bf16);
+  r = make_tmap_2d_16b(&tb, x, total_rows, N, ldx, BK, 64, bf16);
   if (!r) r = make_tmap_2d_16b(&tb32, x, total_rows, N, ldx, BOX_ROWS, 64, bf16);
   if (r) return 2000 + r;
   GroupedParams p{};
