@@ -112,24 +112,26 @@ __global__ void __launch_bounds__(GLU_THREADS) glu_bwd_kernel(const T* __restric
 // through - so that no thread's share differs from another's.  Rows of at most ROPE_NARROW items share a block of ROPE_BLOCK
 // threads, one item each: 300000 rows of 48 bf16 forward and
 // backward: a block each 313 us, together 38.  A form of its own: with the stride and the row worked out at run time 8192 rows of 6144
-// took 40 us a direction instead of 35.
-constexpr int ROPE_NARROW = 64, ROPE_BLOCK = 256;
+// took 40 us a direction instead of 35.  Wide rows: ROPE_ITEMS items a thread, all their loads before the first store (one item, in
+// as many more threads, 34.5 us, two 33.0, three 32.7, four 33.2; both directions 69.3 -> 65.7); where a few tokens leave SMs idle, one.
+constexpr int ROPE_NARROW = 64, ROPE_BLOCK = 256, ROPE_ITEMS = 3;
 // Where a step's keys and values go beside dst (PAGES): rows of kv_width elements of pages of `page` tokens, found through the page tables.
 // A decode step then has a launch a layer less; with the gated unit's too (gemm_rows_tcgen05.cu) 16 sequences, 4 layers of 4096 x 14336,
 // take 498 us instead of 513, 5 sequences, 2 layers of 1024 x 2816, 81 instead of 85.
-template <typename T> struct RopePages {
+template <typename T, bool PAGES> struct RopePages {
   T *k, *v;
   const int *tables, *token_seq, *token_pos;
   int page, table_width, kv_width;     // tokens of a page, entries of a table, elements of a token's keys
   int k_at;                            // first element of the keys in a row; the values follow them
 };
+template <typename T> struct RopePages<T, false> {};
 template <typename T, bool VEC_TABLE, bool NARROW, bool PAGES>
 __global__ void __launch_bounds__(NARROW ? ROPE_BLOCK : 512) rope_kernel(const T* __restrict__ src, T* __restrict__ dst,
                                                    const int64_t* __restrict__ pos, const float* __restrict__ cos_c,
                                                    const float* __restrict__ sin_c, int64_t tokens, int per_block,
                                                    int64_t src_stride, int width, int n_rot_heads, int D, int rot_dim,
-                                                   float sign, int interleaved, RopePages<T> pages) {
-  constexpr int VEC = Vec16<T>::N;
+                                                   float sign, int interleaved, RopePages<T, PAGES> pages) {
+  constexpr int VEC = Vec16<T>::N, UN = NARROW ? 1 : ROPE_ITEMS;
   cb_early_start();
   const int half = rot_dim / 2;
   const int vec_per_head = half / VEC;                       // rotated items of a head
@@ -145,71 +147,88 @@ __global__ void __launch_bounds__(NARROW ? ROPE_BLOCK : 512) rope_kernel(const T
   T* out = dst + t * width;
   const int64_t p = pos[t];
   int64_t slot = 0;                                          // first element of the token's rows in the pages
-  if (PAGES) {
+  if constexpr (PAGES) {
     const int at = pages.token_pos[t], page = pages.tables[pages.token_seq[t] * pages.table_width + at / pages.page];
     slot = ((int64_t)page * pages.page + at % pages.page) * pages.kv_width;
   }
   auto put = [&](const Vec16<T>& x, int o) {
     x.store_na(out + o);
-    if (PAGES && o >= pages.k_at) x.store(o < pages.k_at + pages.kv_width ? pages.k + slot + (o - pages.k_at)
-                                                                          : pages.v + slot + (o - pages.k_at - pages.kv_width));
+    if constexpr (PAGES) {
+      if (o >= pages.k_at)
+        x.store(o < pages.k_at + pages.kv_width ? pages.k + slot + (o - pages.k_at) : pages.v + slot + (o - pages.k_at - pages.kv_width));
+    }
   };
   auto copy_at = [&](int c) {
     return c < n_head_copy ? (c / copy_per_head) * D + rot_dim + (c % copy_per_head) * VEC : n_rot_heads * D + (c - n_head_copy) * VEC;
   };
-  for (int j = threadIdx.x - row * items; j < items; j += NARROW ? items : blockDim.x) {
-    Vec16<T> a, b;
-    if (j >= n_rot) {
-      const int c0 = 2 * (j - n_rot), o0 = copy_at(c0);
-      const bool two = c0 + 1 < n_copy;
-      const int o1 = two ? copy_at(c0 + 1) : o0;
-      a.load_nc(in + o0);
-      b.load_nc(in + o1);
-      put(a, o0);
-      if (two) put(b, o1);
-      continue;
+  const int step = NARROW ? items : blockDim.x;
+  for (int j0 = threadIdx.x - row * items; j0 < items; j0 += UN * step) {
+    Vec16<T> a[UN], b[UN];
+    int o0[UN], o1[UN];
+#pragma unroll
+    for (int k = 0; k < UN; ++k) {
+      const int j = j0 + k * step;
+      if (j >= items) break;
+      if (j >= n_rot) {
+        const int c0 = 2 * (j - n_rot);
+        o0[k] = copy_at(c0);
+        o1[k] = c0 + 1 < n_copy ? copy_at(c0 + 1) : o0[k];
+      } else {
+        const int h = j / vec_per_head, v = j - h * vec_per_head;
+        o0[k] = h * D + (interleaved ? 2 * v * VEC : v * VEC);
+        o1[k] = interleaved ? o0[k] + VEC : o0[k] + half;
+      }
+      a[k].load_nc(in + o0[k]);
+      b[k].load_nc(in + o1[k]);
     }
-    const int h = j / vec_per_head, v = j - h * vec_per_head;
-    const int o0 = h * D + (interleaved ? 2 * v * VEC : v * VEC), o1 = interleaved ? o0 + VEC : o0 + half;
-    a.load_nc(in + o0);
-    b.load_nc(in + o1);
-    float c[VEC], s[VEC];
-    const float* cp = cos_c + p * half + v * VEC;
-    const float* sp = sin_c + p * half + v * VEC;
-    if (VEC_TABLE) {
 #pragma unroll
-      for (int i = 0; i < VEC; i += 4) {
-        const float4 c4 = __ldg(reinterpret_cast<const float4*>(cp + i)), s4 = __ldg(reinterpret_cast<const float4*>(sp + i));
-        c[i] = c4.x; c[i + 1] = c4.y; c[i + 2] = c4.z; c[i + 3] = c4.w;
-        s[i] = s4.x; s[i + 1] = s4.y; s[i + 2] = s4.z; s[i + 3] = s4.w;
+    for (int k = 0; k < UN; ++k) {
+      const int j = j0 + k * step;
+      if (j >= items) break;
+      if (j >= n_rot) {
+        put(a[k], o0[k]);
+        if (o1[k] != o0[k]) put(b[k], o1[k]);
+        continue;
       }
-    } else {
+      const int v = j % vec_per_head;
+      float c[VEC], s[VEC];
+      const float* cp = cos_c + p * half + v * VEC;
+      const float* sp = sin_c + p * half + v * VEC;
+      if (VEC_TABLE) {
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) { c[i] = __ldg(cp + i); s[i] = __ldg(sp + i); }
-    }
-    if (!interleaved) {
-      Vec16<T> u, w;
+        for (int i = 0; i < VEC; i += 4) {
+          const float4 c4 = __ldg(reinterpret_cast<const float4*>(cp + i)), s4 = __ldg(reinterpret_cast<const float4*>(sp + i));
+          c[i] = c4.x; c[i + 1] = c4.y; c[i + 2] = c4.z; c[i + 3] = c4.w;
+          s[i] = s4.x; s[i + 1] = s4.y; s[i + 2] = s4.z; s[i + 3] = s4.w;
+        }
+      } else {
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) {
-        const float x = a.get(i), y = b.get(i), sn = s[i] * sign;
-        u.set(i, x * c[i] - y * sn);
-        w.set(i, y * c[i] + x * sn);
+        for (int i = 0; i < VEC; ++i) { c[i] = __ldg(cp + i); s[i] = __ldg(sp + i); }
       }
-      put(u, o0);
-      put(w, o1);
-    } else {
-      // GPT-J / ChatGLM style: pairs are adjacent elements (2i, 2i + 1); the item's 2 VEC elements hold VEC pairs
+      if (!interleaved) {
+        Vec16<T> u, w;
 #pragma unroll
-      for (int i = 0; i < VEC; i += 2) {
-        const float ca = c[i / 2], sa = s[i / 2] * sign, cb = c[VEC / 2 + i / 2], sb = s[VEC / 2 + i / 2] * sign;
-        const float x = a.get(i), y = a.get(i + 1), z = b.get(i), w = b.get(i + 1);
-        a.set(i, x * ca - y * sa);
-        a.set(i + 1, y * ca + x * sa);
-        b.set(i, z * cb - w * sb);
-        b.set(i + 1, w * cb + z * sb);
+        for (int i = 0; i < VEC; ++i) {
+          const float x = a[k].get(i), y = b[k].get(i), sn = s[i] * sign;
+          u.set(i, x * c[i] - y * sn);
+          w.set(i, y * c[i] + x * sn);
+        }
+        put(u, o0[k]);
+        put(w, o1[k]);
+      } else {
+        // GPT-J / ChatGLM style: pairs are adjacent elements (2i, 2i + 1); the item's 2 VEC elements hold VEC pairs
+#pragma unroll
+        for (int i = 0; i < VEC; i += 2) {
+          const float ca = c[i / 2], sa = s[i / 2] * sign, cb = c[VEC / 2 + i / 2], sb = s[VEC / 2 + i / 2] * sign;
+          const float x = a[k].get(i), y = a[k].get(i + 1), z = b[k].get(i), w = b[k].get(i + 1);
+          a[k].set(i, x * ca - y * sa);
+          a[k].set(i + 1, y * ca + x * sa);
+          b[k].set(i, z * cb - w * sb);
+          b[k].set(i + 1, w * cb + z * sb);
+        }
+        put(a[k], o0[k]);
+        put(b[k], o1[k]);
       }
-      put(a, o0);
-      put(b, o1);
     }
   }
 }
@@ -265,14 +284,15 @@ __global__ void __launch_bounds__(256) scale_check_kernel(const TI* __restrict__
 
 template <typename T, bool PAGES>
 static int launch_rope(const T* src, T* dst, const int64_t* pos, const float* cos_c, const float* sin_c, int64_t tokens, int64_t src_stride,
-                       int width, int n_rot_heads, int D, int rot_dim, float sign, int interleaved, const RopePages<T>& pages,
+                       int width, int n_rot_heads, int D, int rot_dim, float sign, int interleaved, const RopePages<T, PAGES>& pages,
                        cudaStream_t s) {
   if (tokens == 0) return 0;
   const bool vec_table = (((uintptr_t)cos_c | (uintptr_t)sin_c) & 15) == 0;
   // (the same count as in the kernel: rotated pairs, and vectors that pass through two by two)
   const int rotated = n_rot_heads * (rot_dim / 2 / Vec16<T>::N), items = rotated + (width / Vec16<T>::N - 2 * rotated + 1) / 2;
   const int per_block = items > 0 && items <= ROPE_NARROW ? ROPE_BLOCK / items : 1;
-  const int block = per_block > 1 ? ROPE_BLOCK : items >= 512 ? 512 : (items + 31) / 32 * 32;
+  const int share = tokens >= 4 * cb_num_sms() ? (items + ROPE_ITEMS - 1) / ROPE_ITEMS : items;      // of the row's threads
+  const int block = per_block > 1 ? ROPE_BLOCK : share >= 512 ? 512 : (share + 31) / 32 * 32;
   const unsigned grid = (unsigned)((tokens + per_block - 1) / per_block);
   auto kern = per_block > 1 ? (vec_table ? rope_kernel<T, true, true, PAGES> : rope_kernel<T, false, true, PAGES>)
                             : (vec_table ? rope_kernel<T, true, false, PAGES> : rope_kernel<T, false, false, PAGES>);
@@ -335,7 +355,7 @@ int cb_rope(const void* src, void* dst, const int64_t* pos, const float* cos_c, 
             cudaStream_t s) {
   CB_DISPATCH_FLOAT(dtype, T, {
     return (launch_rope<T, false>((const T*)src, (T*)dst, pos, cos_c, sin_c, tokens, src_stride, width, n_rot_heads, D, rot_dim, sign,
-                                  interleaved, RopePages<T>{}, s));
+                                  interleaved, RopePages<T, false>{}, s));
   });
   return CB_LAUNCH_CHECK();
 }
@@ -348,7 +368,7 @@ int cb_rope_pages(const void* src, void* dst, const int64_t* pos, const float* c
                   cudaStream_t s) {
   if (width != (n_rot_heads + kv_heads) * D || (dtype != CB_BF16 && dtype != CB_F16)) return (int)cudaErrorInvalidValue;
   CB_DISPATCH_FLOAT(dtype, T, {
-    const RopePages<T> pages{(T*)k_pages, (T*)v_pages, tables, token_seq, token_pos, page, table_width, kv_heads * D,
+    const RopePages<T, true> pages{(T*)k_pages, (T*)v_pages, tables, token_seq, token_pos, page, table_width, kv_heads * D,
                              (n_rot_heads - kv_heads) * D};
     return (launch_rope<T, true>((const T*)src, (T*)dst, pos, cos_c, sin_c, tokens, src_stride, width, n_rot_heads, D, rot_dim, 1.f,
                                  interleaved, pages, s));

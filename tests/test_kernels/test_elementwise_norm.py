@@ -361,3 +361,17 @@ def test_glu_of_narrow_rows(dtype, vecs, rows, limit):
     eps = max(torch.finfo(dtype).eps, 1e-5)                 # 32 bits: an approximate exponential and division
     assert (y[:n].double() - want).abs().le(eps * want.abs() + 1e-6).all()
     assert (dgu[:n].double() - dwant).abs().le(eps * dwant.abs() + 2e-5).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hq,hkv,D,rot,interleaved", [(32, 8, 128, 128, False), (33, 3, 96, 64, False), (7, 1, 128, 64, True), (64, 8, 256, 64, False)])
+def test_rope_of_many_rows(dtype, hq, hkv, D, rot, interleaved):
+    """A thread's several items in calls of many tokens: the bits of the same rows a few at a time, with items that are no multiple of what
+    a thread or a block takes."""
+    T = 5 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(hq)
+    x = torch.randn(T, (hq + 2 * hkv) * D, device="cuda", generator=g).to(dtype)
+    pos = torch.randint(0, 64, (T,), device="cuda", generator=g)
+    cos, sin = ops.build_rope_cache(64, rot, 10000.0, device="cuda")
+    f = lambda z, p: ops.rope_qkv(z, p, cos, sin, hq, hkv, D, rot_dim=rot, interleaved=interleaved)      # noqa: E731
+    assert torch.equal(f(x, pos), torch.cat([f(a, b) for a, b in zip(x.split(100), pos.split(100))]))
