@@ -375,3 +375,19 @@ def test_rope_of_many_rows(dtype, hq, hkv, D, rot, interleaved):
     cos, sin = ops.build_rope_cache(64, rot, 10000.0, device="cuda")
     f = lambda z, p: ops.rope_qkv(z, p, cos, sin, hq, hkv, D, rot_dim=rot, interleaved=interleaved)      # noqa: E731
     assert torch.equal(f(x, pos), torch.cat([f(a, b) for a, b in zip(x.split(100), pos.split(100))]))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("H", [64, 4096, 8200])
+@pytest.mark.parametrize("odd", [0, 1])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_rmsnorm_of_many_rows(dtype, H, odd, with_res):
+    """Two rows a block in calls of many rows, the last block's second one missing: the bits of the same rows a few at a time."""
+    rows = 8 * torch.cuda.get_device_properties(0).multi_processor_count + 2 + odd
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x, r = (torch.randn(rows, H, device="cuda", generator=g).to(dtype) for _ in "xr")
+    w = torch.randn(H, device="cuda", generator=g).to(dtype)
+    f = lambda a, b: ops.rms_norm(a, w, 1e-5, b) if with_res else (ops.rms_norm(a, w, 1e-5),)      # noqa: E731
+    few = [f(a, b) for a, b in zip(x.split(500), r.split(500))]
+    for i, y in enumerate(f(x, r)):
+        assert torch.equal(y, torch.cat([p[i] for p in few]))
