@@ -40,6 +40,40 @@ CB_DEVICE float ex2_approx(float x) {
 CB_DEVICE void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> CB_DEVICE void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// ---- how a decode step's sequences are cut (cb_decode_num_splits)
+// Warps of a CTA, one for each kv head.  Four heads of 128, so that two CTAs fit an SM and one's beginning and end lie under the other's
+// loads; all heads of 64 up to eight, four where there are more.  Device time, us, eight / four warps: 64 x 2048 tokens of 32 / 8 heads of 128
+// 78.0 / 76.4, 128 x 1024 85.3 / 82.5, 128 x 1024 of 12 heads of 64 62.3 / 56.6, 48 x 2700 of 24 / 8 heads of 64 40.6 / 41.0.
+constexpr int DEC_MMA_WARPS = 4;
+// Few sequences are cut into as many partitions as run at once, equal ones of each sequence's own length: a second round of CTAs, and twice as
+// many partial results to add up, cost more than they balance, and what a table has room for is often several times what is in it.
+// Two rounds of what the table holds / one of the length, tables just wide enough, us: 16 x 1024 tokens of 32 / 8 heads of 128 22.6 / 18.2, 16 x 8000
+// 86 / 79, 2 x 16000 38.0 / 29.6, 10 x 8000 60.0 / 54.9, 28 x 4000 75.0 / 69.8, 6 x 12000 of 16 / 2 heads of 64 29.1 / 22.4, 60 x 2000 of 16 / 2 heads of 128
+// 37.8 / 31.2, 5 x 8000 of 12 heads 50.5 / 43.9; tables of 8192 tokens of which 500 to 1000 are in use, 16 sequences 40.8 / 17, 28 64 / 21.  More
+// than DEC_MOST_SPLITS partitions cost as many results more than they give CTAs (96: 2 x 6000 21.0 instead of 17.8, 1 x 16000 25.2 instead of
+// 26.4).  Where a round is fewer than DEC_ROUND_SPLITS partitions - lengths differ by more than one - two rounds (one / two: 40 x 3000 79.8 / 73.0, 32 x
+// 4000 79.8 / 76.0), and where that is as few, and for more than four heads of 64, of what the table holds (64 x 2048 76.9, own 80.3; 30 x 4000 of 24 / 8
+// heads of 64 38.6, own 43.4).
+constexpr int DEC_PART_MIN = 64, DEC_ROUND_SPLITS = 5, DEC_MOST_SPLITS = 64;
+constexpr int DEC_WIDE = 48;           // partitions from which decode_reduce_wide_kernel adds them up
+static inline int decode_warps(int kv_heads, int head_dim) {
+  const int most = head_dim == 128 || kv_heads > 8 ? DEC_MMA_WARPS : 8;
+  return kv_heads < most ? kv_heads : most;
+}
+struct DecodeCut {
+  const int* seq_lens;
+  int capacity, part_len;              // tokens that a table has room for
+};
+// tokens of a partition: part_len, or, where that is negative, an equal share of the sequence's own, of -part_len at least
+CB_DEVICE int decode_partition(int cached, int splits, int part_len) {
+  return part_len > 0 ? part_len : max(-part_len, ((cached + splits - 1) / splits + 15) & ~15);
+}
+// partitions of a sequence that have tokens
+CB_DEVICE int decode_used(const DecodeCut& c, int seq, int splits) {
+  const int cached = min(c.seq_lens[seq], c.capacity), part = decode_partition(cached, splits, c.part_len);
+  return max(0, min(splits, (cached + part - 1) / part));
+}
+
 template <typename T, typename TC>
 __global__ void __launch_bounds__(256) kv_cache_write_kernel(const T* __restrict__ k, const T* __restrict__ v,
                                                              TC* __restrict__ k_cache, TC* __restrict__ v_cache,
@@ -228,8 +262,10 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_kernel(
   // sliding-window attention (Mistral): only the last `window` cached tokens are visible - partitions that lie before
   // the window start contribute nothing (m = -inf, l = 0) and are skipped by the merge
   const int window_start = window > 0 ? max(0, len - window) : 0;
-  const int t0 = max(split * part_len, window_start);
-  const int t1 = min(min(len, max_blocks_per_seq * block_size), split * part_len + part_len);   // (no pages beyond the table's row)
+  const int cached = min(len, max_blocks_per_seq * block_size);                                 // (no pages beyond the table's row)
+  const int part = decode_partition(cached, splits, part_len);
+  const int t0 = max(split * part, window_start);
+  const int t1 = min(cached, split * part + part);
   const int g0 = set * GH;
   const int ng = min(GH, G - g0);
   const int grp = lane / LPT, sub = lane - grp * LPT;
@@ -404,11 +440,6 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_kernel(
 //   * partial results use the same (o_part, ml_part) format, so the reduce kernel is shared.
 constexpr int DEC_MMA_TOKENS = 16;
 constexpr int DEC_MMA_STAGES = 3;
-// Warps of a CTA, one for each kv head: all of them up to eight, four where there are more, which fill the CTAs and leave less of the
-// SMs idle in the last round.  Device time, us, eight / four warps: 128 x 1024 tokens of 12 heads of 64 62.3 / 56.6, 16 x 1024 of 32 heads of
-// 128 45.0 / 43.8, 24 x 900 of 16 heads 34.3 / 33.3; of 32 / 8 heads 64 x 2048 77.4 / 75.8, but a decode step of 16 x 1024 509 / 514 (an SM
-// that is left free takes the next kernels' CTAs meanwhile).
-constexpr int DEC_MMA_WARPS = 4;
 
 CB_DEVICE void ldmatrix_x4(uint32_t (&r)[4], const void* smem_row) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem_row);
@@ -462,8 +493,10 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
   cb_early_start();
   const int len = seq_lens[seq];
   const int window_start = window > 0 ? max(0, len - window) : 0;
-  const int t0 = max(split * part_len, window_start);
-  const int t1 = min(min(len, max_blocks_per_seq * block_size), split * part_len + part_len);   // (no pages beyond the table's row)
+  const int cached = min(len, max_blocks_per_seq * block_size);                                 // (no pages beyond the table's row)
+  const int part = decode_partition(cached, splits, part_len);
+  const int t0 = max(split * part, window_start);
+  const int t1 = min(cached, split * part + part);
   const int row = lane >> 2, quad = lane & 3;   // accumulator layout: head row, column pair inside an 8-wide tile
   const bool row_ok = row < G;                  // rows G..15 of the MMA are padding
   const float scale2 = scale * LOG2E;           // scores in the exp2 domain
@@ -594,7 +627,9 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
     }
     cp_async_wait<0>();
   }
-  // ---- this unit's partial result (row sum over the quad first)
+  // ---- this unit's partial result (row sum over the quad first).  (Of a partition behind the sequence's end nobody asks for one where there are
+  // many; looked at before the queries are loaded it cost every call .5 us.)
+  if (splits >= DEC_WIDE && split * part >= cached) return;
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
   if (row_ok) {
@@ -638,21 +673,25 @@ __global__ void __launch_bounds__(128) decode_reduce_kernel(const float* __restr
 // sequence of 4097 tokens: the call on the device 16.2 us, 13.9 so).  With fewer of them it is no faster (16 x 2048 tokens, 64 / 8 heads, 19
 // partitions 30 us, 33 so) and with many sequences slower (1024 of 64 tokens 78 us, 89 so).
 // Sums in the same order with the same roundings.
-constexpr int DEC_WIDE = 48, DEC_AHEAD = 16, DEC_WIDE_THREADS = 128;
+constexpr int DEC_AHEAD = 16, DEC_WIDE_THREADS = 128;
 template <typename T, int D>
 __global__ void __launch_bounds__(DEC_WIDE_THREADS) decode_reduce_wide_kernel(const float* __restrict__ o_part,
                                                                               const float* __restrict__ ml_part,
-                                                                              T* __restrict__ out, int Hq, int splits,
-                                                                              int64_t out_stride) {
+                                                                              T* __restrict__ out, int Hq, int all_splits,
+                                                                              int64_t out_stride, DecodeCut cut) {
   constexpr int COLS = (D + DEC_WIDE_THREADS - 1) / DEC_WIDE_THREADS;
   __shared__ float max_s[DEC_WIDE_THREADS / 32];
   __shared__ float w_s[DEC_WIDE_THREADS], l_s[DEC_WIDE_THREADS];      // weight (-1: a partition without tokens), sum
   const int seq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-  const int64_t base = ((int64_t)seq * Hq + h) * splits;
+  const int64_t base = ((int64_t)seq * Hq + h) * all_splits;
   const float2* ml = reinterpret_cast<const float2*>(ml_part) + base;
   cb_early_start();
+  const int splits = decode_used(cut, seq, all_splits);
   float gm = -INFINITY;
-  for (int s = tid; s < splits; s += DEC_WIDE_THREADS) gm = fmaxf(gm, ml[s].x);
+  for (int s = tid; s < all_splits; s += DEC_WIDE_THREADS) {     // (asked for beside the length)
+    const float x = ml[s].x;
+    if (s < splits) gm = fmaxf(gm, x);
+  }
   gm = warp_max(gm);
   if ((tid & 31) == 0) max_s[tid >> 5] = gm;
   __syncthreads();
@@ -702,10 +741,11 @@ __global__ void __launch_bounds__(DEC_WIDE_THREADS) decode_reduce_wide_kernel(co
 
 template <typename T, int D>
 int launch_decode_reduce(const float* o_part, const float* ml_part, T* out, int num_seqs, int Hq, int splits, int64_t out_stride,
-                         cudaStream_t s) {
-  auto kernel = splits < DEC_WIDE ? decode_reduce_kernel<T, D> : decode_reduce_wide_kernel<T, D>;
-  static_assert(DEC_WIDE_THREADS == 128, "the block of both");
-  return cb_launch_early(kernel, dim3(num_seqs, Hq), DEC_WIDE_THREADS, 0, s, o_part, ml_part, out, Hq, splits, out_stride);
+                         const DecodeCut& cut, cudaStream_t s) {
+  const dim3 grid(num_seqs, Hq);
+  return splits < DEC_WIDE ? cb_launch_early(decode_reduce_kernel<T, D>, grid, 128, 0, s, o_part, ml_part, out, Hq, splits, out_stride)
+                           : cb_launch_early(decode_reduce_wide_kernel<T, D>, grid, DEC_WIDE_THREADS, 0, s, o_part, ml_part, out, Hq, splits,
+                                             out_stride, cut);
 }
 
 __global__ void gather_cos_sin_kernel(const float* __restrict__ cos_c, const float* __restrict__ sin_c,
@@ -779,14 +819,24 @@ int cb_rope_kv_cache_write(void* q, void* k, const void* v, void* k_cache, void*
   return CB_LAUNCH_CHECK();
 }
 
-int cb_decode_num_splits(int num_seqs, int kv_heads, int max_len, int* part_len_out) {
-  // aim at >= 2 waves of CTAs, partitions of >= 64 tokens.  Counted in CTAs of eight kv heads, also where four share one
-  // (DEC_MMA_WARPS): the partitions, and with them a sequence's bits, are what they were.
+// partitions of every sequence, and the `part_len` that goes with them (decode_partition).  What a sequence's result is depends on the
+// call's sizes and on its own length, not on the others' lengths.
+int cb_decode_num_splits(int num_seqs, int kv_heads, int head_dim, int max_len, int* part_len_out) {
+  *part_len_out = DEC_PART_MIN;
+  if (num_seqs <= 0 || kv_heads <= 0) return 1;
+  const int sms = cb_num_sms(), most = (max_len + DEC_PART_MIN - 1) / DEC_PART_MIN;
+  const int warps = decode_warps(kv_heads, head_dim);
+  const int fit = 227 * 1024 / (warps * DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * head_dim * 2), per_sm = fit < 8 ? fit : 8;
+  const int ctas = num_seqs * ((kv_heads + warps - 1) / warps), one_round = per_sm * sms / ctas, two_rounds = 2 * per_sm * sms / ctas;
+  if ((head_dim == 128 || kv_heads <= 4) && head_dim <= 128 && (one_round >= DEC_ROUND_SPLITS || two_rounds > DEC_ROUND_SPLITS)) {
+    *part_len_out = -DEC_PART_MIN;
+    const int own = one_round >= DEC_ROUND_SPLITS ? one_round : two_rounds, splits = own < DEC_MOST_SPLITS ? own : DEC_MOST_SPLITS;
+    return splits < most ? splits : most < 1 ? 1 : most;
+  }
+  // two rounds of CTAs of eight kv heads, partitions of at least DEC_PART_MIN of the tokens that a table has room for
   const int ctas_per_split = num_seqs * ((kv_heads + 7) / 8);
-  const int target = 2 * cb_num_sms();
-  int splits = (target + ctas_per_split - 1) / ctas_per_split;
-  const int max_splits = (max_len + 63) / 64;
-  if (splits > max_splits) splits = max_splits;
+  int splits = (2 * sms + ctas_per_split - 1) / ctas_per_split;
+  if (splits > most) splits = most;
   if (splits < 1) splits = 1;
   int part = (max_len + splits - 1) / splits;
   part = ((part + 31) / 32) * 32;
@@ -814,7 +864,8 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
   // <= 8 q heads); CB200_DECODE=simt forces the CUDA-core kernel (also used for head_dim 256)
   const char* impl_env = getenv("CB200_DECODE");
   const bool use_mma = !(impl_env != nullptr && impl_env[0] == 's') && G <= 8 && (D == 128 || D == 64);
-  const int mma_warps = Hkv <= DEC_THREADS / 32 ? Hkv : DEC_MMA_WARPS;
+  const int mma_warps = decode_warps(Hkv, D);
+  const DecodeCut cut{seq_lens, max_blocks_per_seq * block_size, part_len};
   dim3 mma_grid(num_seqs, (Hkv + mma_warps - 1) / mma_warps, splits);
 #define LAUNCH_DEC_MMA(T, DD)                                                                                       \
   {                                                                                                                  \
@@ -824,7 +875,7 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
     if (const int e = cb_launch_early(paged_decode_mma_kernel<T, DD>, mma_grid, mma_warps * 32, mma_warps * per_warp, s, \
         (const T*)q, (const T*)k_cache, (const T*)v_cache, block_tables, seq_lens, o_part, ml_part, Hq, Hkv,        \
         block_size, max_blocks_per_seq, splits, part_len, scale, alibi_slopes, q_stride, window)) return e;         \
-    if (const int e = launch_decode_reduce<T, DD>(o_part, ml_part, (T*)out, num_seqs, Hq, splits, out_stride, s)) return e; \
+    if (const int e = launch_decode_reduce<T, DD>(o_part, ml_part, (T*)out, num_seqs, Hq, splits, out_stride, cut, s)) return e; \
   }
 #define LAUNCH_DEC(T, DD)                                                                                           \
   {                                                                                                                  \
@@ -834,7 +885,7 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
   paged_decode_kernel<T, T, DD><<<grid, warps * 32, dec_smem, s>>>((const T*)q, (const T*)k_cache, (const T*)v_cache, \
       block_tables, seq_lens, o_part, ml_part, Hq, Hkv, block_size, max_blocks_per_seq, splits, part_len, scale,     \
       alibi_slopes, q_stride, window);                                                                               \
-  if (const int e = launch_decode_reduce<T, DD>(o_part, ml_part, (T*)out, num_seqs, Hq, splits, out_stride, s)) return e
+  if (const int e = launch_decode_reduce<T, DD>(o_part, ml_part, (T*)out, num_seqs, Hq, splits, out_stride, cut, s)) return e
   CB_DISPATCH_HALF(dtype, T, {
     if (use_mma && D == 128) { LAUNCH_DEC_MMA(T, 128); }
     else if (use_mma && D == 64) { LAUNCH_DEC_MMA(T, 64); }

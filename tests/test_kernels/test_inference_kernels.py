@@ -319,3 +319,31 @@ def test_rotation_with_page_write(heads, kv, D, rot, interleaved, tokens, page, 
                (2, cos.half())]
     assert all(inference.rope_pages(*(value if i == at else a for i, a in enumerate(args))) is None for at, value in refused)
     assert torch.equal(pages[0], kw) and torch.equal(pages[1], vw)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,Hq,Hkv,D", [(1, 16, 8, 128), (2, 4, 2, 64), (29, 8, 8, 128), (30, 8, 8, 128), (49, 8, 8, 128), (50, 8, 8, 128), (9, 32, 32, 128), (3, 12, 12, 128),
+                                        (118, 4, 2, 128), (119, 4, 2, 128), (150, 4, 4, 64), (7, 8, 8, 64)])
+@pytest.mark.parametrize("room", [80, 1100, 5000])
+def test_paged_decode_partitions_of_a_length(n, Hq, Hkv, D, room):
+    """Sequences cut by their own length and by what a table has room for, on both sides of the rules between them, in tables that are mostly
+    empty: against the reference, and a sequence's bits do not depend on how long the others are."""
+    dev, page = "cuda", 16
+    g = torch.Generator(device=dev).manual_seed(n + room)
+    width = (room + page - 1) // page
+    lens = torch.randint(1, min(room, 700) + 1, (n,), device=dev, generator=g)
+    edges = torch.tensor([1, 16, 63, 64, 65, room], device=dev)[:n]
+    lens[: len(edges)] = edges.clamp(max=room)
+    most = int(lens.max() + page - 1) // page
+    tables = torch.zeros(n, width, dtype=torch.int32, device=dev)
+    tables[:, :most] = torch.randint(0, 200, (n, most), device=dev, generator=g).to(torch.int32)
+    q = torch.randn(n, Hq, D, device=dev, generator=g).bfloat16()
+    kc, vc = (torch.randn(200, page, Hkv, D, device=dev, generator=g).bfloat16() for _ in "kv")
+    lens = lens.to(torch.int32)
+    out = iops.paged_decode_attention(q, kc, vc, tables, lens)
+    ref = iops.paged_decode_attention_ref(q, kc, vc, tables, lens)
+    # probabilities and results rounded to 8 bits: averages of values of about one
+    torch.testing.assert_close(out.float(), ref.float(), atol=2e-2, rtol=2e-2)
+    other = lens.clone()
+    other[1:] = (lens[1:] // 2).clamp(min=1)
+    assert torch.equal(iops.paged_decode_attention(q, kc, vc, tables, other)[0], out[0])
