@@ -564,10 +564,13 @@ CB_DEVICE ScanTwo fma2(ScanTwo a, ScanTwo b, ScanTwo c) { return ScanTwo{__fmaf_
 CB_DEVICE ScanTwo mul2(ScanTwo a, ScanTwo b) { return ScanTwo{__fmul_rn(a.a, b.a), __fmul_rn(a.b, b.b)}; }
 
 // The sequence and the unit of it (head and block of columns; `units` per sequence) that a CTA walks.  A unit takes as long as
-// its sequence, and all are resident at once in a usual step, so what a step takes is the SM with the most tokens.  Up to 32
-// sequences are dealt out by length, longest first and every second row of one CTA per SM the other way round; a row that
-// does not fill lands on the SMs that drew short ones before.  More sequences are many more units than fit: they come in order.
-CB_DEVICE void scan_unit(const ScanParams& p, int nseq, int units, int sms, int& s, int& unit) {
+// its sequence, and what a step takes is the SM with the most tokens.  Up to 32 sequences are dealt out by length, longest first; where all
+// units are resident at once (`at_once`), every second row of one CTA per SM the other way round, and a row that does not fill lands on the
+// SMs that drew short ones before.  Where they are not, the rest goes to the SMs that are done first, and rows all the same way are better: 12000 tokens of 16
+// heads x 128 x 128 in eight sequences, three units an SM, five draws of lengths, 695 722 702 742 679 us turned round, 661 673 704 667 636 so; in five (all
+// at once) 765 and 814 turned round, 808 and 816 so, in 14 of 9000 with 8 heads (448 units for 444 places) 265 and 270.  (Dealing the units to SMs by their tokens beforehand, 750 - 780: a grid's CTAs do not
+// land where their number says.)  More sequences are many more units than fit: they come in order.
+CB_DEVICE void scan_unit(const ScanParams& p, int nseq, int units, int sms, bool at_once, int& s, int& unit) {
   int rank = blockIdx.x;
   if (nseq == 1 || nseq > 32) {
     s = rank / units;
@@ -575,7 +578,7 @@ CB_DEVICE void scan_unit(const ScanParams& p, int nseq, int units, int sms, int&
     return;
   }
   const int row = rank / sms, width = min(sms, (int)gridDim.x - row * sms);
-  if (!(row & 1)) rank = row * sms + width - 1 - (rank - row * sms);
+  if (at_once && !(row & 1)) rank = row * sms + width - 1 - (rank - row * sms);
   const int lane = threadIdx.x & 31, want = rank / units;
   unit = rank - want * units;
   const int len = lane < nseq ? p.cu_q[lane + 1] - p.cu_q[lane] : -1;
@@ -605,7 +608,9 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
   extern __shared__ __align__(16) float scan_smem[];
   const int vblocks = w.VP / COLS;
   int s, unit;
-  scan_unit(p, nseq, p.heads * vblocks, sms, s, unit);
+  // (only the long decay form's BLOCKS are all that an SM holds; a few units more than fit are as if they fitted)
+  const bool at_once = MODE != SCAN_DECAY || SHORT || DK > 128 || 8 * (int)gridDim.x <= 9 * sms * Tile::BLOCKS;
+  scan_unit(p, nseq, p.heads * vblocks, sms, at_once, s, unit);
   const int h = unit / vblocks, vb = unit % vblocks;
   const int t0 = p.cu_q[s], t1 = p.cu_q[s + 1];
   if (t0 >= t1) return;
