@@ -25,6 +25,7 @@
 // library's `torch._grouped_mm`.
 #include <stdlib.h>
 
+#include "activations.cuh"
 #include "common.cuh"
 #include "sm100.cuh"
 #include "tile_order.h"
@@ -34,7 +35,10 @@ using namespace sm100;
 namespace {
 
 constexpr int UMMA_K = 16;
-constexpr int ROWS_THREADS = 192;      // producer, issuer, four epilogue warps
+constexpr int UNGATED = -1;            // of the variable-M modes' ACT: a product alone
+// epilogue warps behind the producer and the issuer: a product's own work hides behind four; a gated unit's does not
+// (64 experts of 25088 rows as below: input gradient 178 us with four, 170 with eight; 8 of 8256, 1024 -> 2 x 512: 22.6 and 20.6, forward 24.7 and 22.6)
+constexpr int rows_warps(int act) { return act == UNGATED ? 4 : 8; }
 constexpr int WGRAD_THREADS = 320;     // .., eight
 constexpr int BOX_ROWS = 32;           // token rows of the smaller TMA box: a request takes as long to issue as one of 64 rows
 constexpr int ROWS_BOX = 64;           // of the larger one, variable-M modes (weight gradients: a k-block, as many)
@@ -56,8 +60,9 @@ constexpr int BOXES = 2;               // of an epilogue warp of weight gradient
 // 32 columns per warp), the barriers, the groups' boundaries and the tile list of the variable-M modes
 constexpr int BOX_BYTES = 32 * 128;
 constexpr int ROW_BOX_BYTES = 32 * 64;
-template <int MODE> constexpr int smem_bytes() {
-  return stage_ring<MODE>() + 256 + (MAX_GROUPS + 1) * 4 + (MODE == MODE_TN ? 8 * BOXES * BOX_BYTES : 4 * ROW_BOX_BYTES + (MAX_GROUPS + 1) * 4);
+template <int MODE> constexpr int smem_bytes(int warps = 8) {
+  return stage_ring<MODE>() + 256 + (MAX_GROUPS + 1) * 4 +
+         (MODE == MODE_TN ? warps * BOXES * BOX_BYTES : warps * ROW_BOX_BYTES + (MAX_GROUPS + 1) * 4);
 }
 
 SM100_DEVICE void tma_store_3d(const CUtensorMap* map, const void* smem_src, int32_t c0, int32_t c1, int32_t c2) {
@@ -78,6 +83,10 @@ struct GroupedParams {
   int tma_store;            // TN: 16-bit results that overwrite leave through shared memory and TMA
   uint32_t idesc;           // variable-M: without N, which is the tile's number of rows
   void* C;
+  // gated forward: N = I columns of the unit's result, w [E, 2 I, K]; C [rows, 2 I] gate | up, unit [rows, I] = act(gate) up.
+  // gated input gradient: N = I, what a row's product is is the unit's gradient; gate_up [rows, 2 I] from the forward, C [rows, 2 I] its gradient
+  void* unit;
+  const void* gate_up;
 };
 
 struct Tile {
@@ -140,17 +149,25 @@ SM100_DEVICE void store_row(float* __restrict__ dst, const uint32_t (&acc)[32], 
 }
 
 // The variable-M modes.  A = the weight (NT: rows of W[e], K-major; NN: columns of W[e], MN-major), B = the token rows (K-major).
-template <int MODE, typename T>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROWS_THREADS, 1)
+// ACT: the gated unit of activations.cuh that lies between two layers of an expert, or UNGATED.  Forward: a CTA's 128 rows of the weight are 64 of the gate and the
+// 64 of up that belong to them, so that both factors meet in its epilogue, which writes the unit's result beside them.  Input gradient: the
+// epilogue has the unit's gradient in its boxes and turns it into that of gate and up.  The roundings are those of launches of their own, which read
+// again what was just written, at the memory's rate.  64 experts of 25088 rows, 2048 -> 2 x 1408 -> 2048: forward 281 -> 255 us (the product alone
+// 239), input gradient 191 -> 170 (137 alone); 16 experts of 16512, 2048 -> 2 x 1024: 120 -> 110 and 83 -> 73.  What is left of the unit are the bytes
+// that it has to move, past products that the SMs' reads bound already.
+template <int MODE, typename T, int ACT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * rows_warps(ACT), 1)
 grouped_rows_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                          const __grid_constant__ CUtensorMap tmap_x32, const GroupedParams p) {
-  constexpr bool A_MN = MODE == MODE_NN;
+  constexpr int WARPS = rows_warps(ACT);
+  constexpr bool A_MN = MODE == MODE_NN, GATED = ACT != UNGATED;
+  constexpr int BLOCK_COLS = GATED && MODE == MODE_NT ? PAIR_M / 2 : PAIR_M;             // columns of N that a pair has
   constexpr int STAGES = Block<MODE>::STAGES, A_BYTES = Block<MODE>::A_BYTES, B_BYTES = Block<MODE>::B_BYTES;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * A_BYTES;
-  uint8_t* smem_box = smem + stage_ring<MODE>();                                                // [4 warps]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_box + 4 * ROW_BOX_BYTES);
+  uint8_t* smem_box = smem + stage_ring<MODE>();                                                // [epilogue warps]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_box + WARPS * ROW_BOX_BYTES);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + STAGES;
   uint64_t* tmem_full = bars + 2 * STAGES;
@@ -165,7 +182,7 @@ grouped_rows_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
   const bool leader_cta = cta_rank == 0;
   const int num_pairs = gridDim.x >> 1;
   const int pair_id = blockIdx.x >> 1;
-  const int blocks = (p.N + PAIR_M - 1) / PAIR_M;
+  const int blocks = (p.N + BLOCK_COLS - 1) / BLOCK_COLS;
 
   // ---- tile list: per-group row-tile counts -> exclusive prefix (every CTA builds its own copy), a warp
   if (warp == 3) {
@@ -203,7 +220,7 @@ grouped_rows_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 8);
+      mbar_init(&tmem_empty[i], 2 * WARPS);
     }
     fence_barrier_init();
   }
@@ -240,6 +257,10 @@ grouped_rows_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
 #pragma unroll
             for (int j = 0; j < 2; ++j)
               tma_load_2d_2sm(&tmap_w, fb, sa + j * (BK * 128), a_m0 + j * 64, tl.group * p.w_group_rows + k0);
+          } else if (GATED) {
+            const int gate = tl.group * p.w_group_rows + tl.m_blk * BLOCK_COLS + (int)cta_rank * 64;
+            tma_load_2d_2sm(&tmap_w, fb, sa, k0, gate);
+            tma_load_2d_2sm(&tmap_w, fb, sa + 64 * 128, k0, gate + p.N);
           } else {
             tma_load_2d_2sm(&tmap_w, fb, sa, k0, tl.group * p.w_group_rows + a_m0);
           }
@@ -290,44 +311,88 @@ grouped_rows_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     }
   } else {
     // ================================================================ epilogue (warps 2..5, both CTAs): lane = output column
-    const int quarter = warp & 3;
-    uint8_t* box = smem_box + quarter * ROW_BOX_BYTES;                     // [32 token rows][32 columns]
+    const int quarter = warp & 3, turn = (warp - 2) >> 2;                  // gated: 32 rows of each 64 a warp
+    uint8_t* box = smem_box + (turn * 4 + quarter) * ROW_BOX_BYTES;        // [32 token rows][32 columns]
+    const auto drained = [&](int a) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (leader_cta) mbar_arrive(&tmem_empty[a]);
+        else mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[a]), 0));
+      }
+    };
     int acc = 0, cur = 0;
     uint32_t acc_phase = 0;
     Tile ahead = find_tile<MODE>(pair_id, num_tiles, p, bounds, tile_start, blocks, cur);
     for (int t = pair_id; t < num_tiles; t += num_pairs) {
       const Tile tl = ahead;
       ahead = find_tile<MODE>(t + num_pairs, num_tiles, p, bounds, tile_start, blocks, cur);
-      const int col = tl.m_blk * PAIR_M + (int)cta_rank * 128 + quarter * 32 + (lane & 3) * 8;
-      T* out = reinterpret_cast<T*>(p.C) + (size_t)(tl.row0 + (lane >> 2)) * p.ldc + col;
+      // gated forward: two warps have the gate and two the up of the CTA's 64 columns
+      const int col = GATED && MODE == MODE_NT ? tl.m_blk * BLOCK_COLS + (int)cta_rank * 64 + (quarter & 1) * 32 + (lane & 3) * 8
+                                               : tl.m_blk * PAIR_M + (int)cta_rank * 128 + quarter * 32 + (lane & 3) * 8;
+      const size_t row = (size_t)(tl.row0 + (lane >> 2));
+      T* out = reinterpret_cast<T*>(p.C) + row * p.ldc + col + (GATED && MODE == MODE_NT && quarter >= 2 ? p.N : 0);
       const int rows = col < p.N ? tl.row_end - tl.row0 - (lane >> 2) : 0;     // N % 8 == 0: a lane's columns exist or do not
       mbar_wait(&tmem_full[acc], acc_phase);
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * PAIR_N + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < tl.n; c += 32) {
+      for (int c = turn * 32; c < tl.n; c += WARPS * 8) {
         uint32_t v[32];
         tmem_ld_32x32b_x32(taddr + c, v);
-        tmem_ld_wait();
-        if (c + 32 >= tl.n) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (leader_cta) mbar_arrive(&tmem_empty[acc]);
-            else mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
-          }
+        Vec16<T> gate[4], up[4];                                           // gated input gradient: asked for ahead, read once
+        if constexpr (GATED && MODE == MODE_NN) {
+          const T* gu = reinterpret_cast<const T*>(p.gate_up) + row * p.ldc + col;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (c + i * 8 < rows) {
+              gate[i].raw = __ldcs(reinterpret_cast<const uint4*>(gu + (size_t)(c + i * 8) * p.ldc));
+              up[i].raw = __ldcs(reinterpret_cast<const uint4*>(gu + (size_t)(c + i * 8) * p.ldc + p.N));
+            }
         }
+        tmem_ld_wait();
+        if (c + WARPS * 8 >= tl.n) drained(acc);
         T* mine = reinterpret_cast<T*>(box) + lane;
 #pragma unroll
         for (int i = 0; i < 32; ++i) mine[i * 32] = from_f32<T>(k_blocks > 0 ? __uint_as_float(v[i]) : 0.f);
-        __syncwarp();
+        if constexpr (GATED && MODE == MODE_NT) asm volatile("bar.sync %0, 128;" ::"r"(1 + turn) : "memory");
+        else __syncwarp();
+        const uint8_t* piece = box + lane * 16;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {                                      // 16 bytes of eight rows at a time
-          const uint4 x = *reinterpret_cast<const uint4*>(box + i * 512 + lane * 16);
-          if (c + i * 8 < rows) *reinterpret_cast<uint4*>(out + (size_t)(c + i * 8) * p.ldc) = x;
+          if (c + i * 8 >= rows) break;
+          T* dst = out + (size_t)(c + i * 8) * p.ldc;
+          Vec16<T> x;
+          x.load(reinterpret_cast<const T*>(piece + i * 512));
+          if constexpr (GATED && MODE == MODE_NN) {
+            Vec16<T> dg, du;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float gf = gate[i].get(e), uf = up[i].get(e), df = x.get(e);
+              dg.set(e, df * uf * act_grad_f<GATED ? ACT : 0>(gf));
+              du.set(e, df * act_f<GATED ? ACT : 0>(gf));
+            }
+            dg.store(dst);
+            du.store(dst + p.N);
+          } else {
+            x.store(dst);
+          }
+          if constexpr (GATED && MODE == MODE_NT) {                        // the unit: half of the rows each
+            if ((i >= 2) == (quarter >= 2)) {
+              const uint8_t* pair = smem_box + (turn * 4 + (quarter & 1)) * ROW_BOX_BYTES + lane * 16 + i * 512;
+              Vec16<T> g, u, o;
+              g.load(reinterpret_cast<const T*>(pair));
+              u.load(reinterpret_cast<const T*>(pair + 2 * ROW_BOX_BYTES));
+#pragma unroll
+              for (int e = 0; e < 8; ++e) o.set(e, act_f<GATED ? ACT : 0>(g.get(e)) * u.get(e));
+              o.store(reinterpret_cast<T*>(p.unit) + (row + c + i * 8) * p.N + col);
+            }
+          }
         }
         __syncwarp();
+        if constexpr (GATED && MODE == MODE_NT) asm volatile("bar.sync %0, 128;" ::"r"(1 + turn) : "memory");
       }
+      if (turn * 32 >= tl.n) drained(acc);
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
@@ -557,12 +622,22 @@ grouped_wgrad_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 }
 
 // the number of tiles is only known on the device: full persistent grids
-template <int MODE, typename T>
+template <int MODE, typename T, int ACT = UNGATED>
 int launch_rows(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tx32, const GroupedParams& p, cudaStream_t stream) {
   static CbDeviceAttr attr;
-  if (const int e = cb_allow_smem(attr, grouped_rows_2cta_kernel<MODE, T>, smem_bytes<MODE>())) return e;
-  grouped_rows_2cta_kernel<MODE, T><<<cb_num_sms() / 2 * 2, ROWS_THREADS, smem_bytes<MODE>(), stream>>>(tw, tx, tx32, p);
+  constexpr int warps = rows_warps(ACT), smem = smem_bytes<MODE>(warps);
+  if (const int e = cb_allow_smem(attr, grouped_rows_2cta_kernel<MODE, T, ACT>, smem)) return e;
+  grouped_rows_2cta_kernel<MODE, T, ACT><<<cb_num_sms() / 2 * 2, 64 + 32 * warps, smem, stream>>>(tw, tx, tx32, p);
   return (int)cudaGetLastError();
+}
+
+template <int MODE>
+int launch_gated(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tx32, const GroupedParams& p, bool bf16, int act, cudaStream_t stream) {
+  if (act < 0 || act > 2) return (int)cudaErrorInvalidValue;
+  if (bf16) return act == 0   ? launch_rows<MODE, __nv_bfloat16, 0>(tw, tx, tx32, p, stream)
+                   : act == 1 ? launch_rows<MODE, __nv_bfloat16, 1>(tw, tx, tx32, p, stream) : launch_rows<MODE, __nv_bfloat16, 2>(tw, tx, tx32, p, stream);
+  return act == 0   ? launch_rows<MODE, __half, 0>(tw, tx, tx32, p, stream)
+         : act == 1 ? launch_rows<MODE, __half, 1>(tw, tx, tx32, p, stream) : launch_rows<MODE, __half, 2>(tw, tx, tx32, p, stream);
 }
 
 template <typename OUT>
@@ -606,6 +681,46 @@ int cb_grouped_gemm(const void* x, const void* w, void* y, const int* offs, int 
   if (r) return 2000 + r;
   p.w_group_rows = K;
   return bf16 ? launch_rows<MODE_NN, __nv_bfloat16>(tw, tx, tx32, p, stream) : launch_rows<MODE_NN, __half>(tw, tx, tx32, p, stream);
+}
+
+// The forward of a gated layer: w [E, 2 I, K] gate | up, gate_up [total_rows, 2 I] = x w[e]^T, unit [total_rows, I] = act(gate) up; act 0 silu,
+// 1 gelu (tanh), 2 gelu (erf).  K, I multiples of 8.
+int cb_grouped_gemm_gated(const void* x, const void* w, void* gate_up, void* unit, const int* offs, int E, int total_rows, int I, int K, int ldx,
+                          int act, int dtype, cudaStream_t stream) {
+  if (E <= 0 || total_rows <= 0 || I <= 0) return 0;
+  if (E > MAX_GROUPS || (dtype != CB_BF16 && dtype != CB_F16) || (K & 7) || (I & 7) || I > 0x3fffffff) return (int)cudaErrorInvalidValue;
+  const bool bf16 = dtype == CB_BF16;
+  CUtensorMap tx, tx32, tw;
+  int r = make_tmap_2d_16b(&tx, x, total_rows, K, ldx, ROWS_BOX, 64, bf16);
+  if (!r) r = make_tmap_2d_16b(&tx32, x, total_rows, K, ldx, BOX_ROWS, 64, bf16);
+  if (r) return 1000 + r;
+  r = make_tmap_2d_16b(&tw, w, (uint64_t)E * 2 * I, K, K, 64, 64, bf16);
+  if (r) return 2000 + r;
+  GroupedParams p{};
+  p.offs = offs; p.E = E; p.total_rows = total_rows; p.N = I; p.K = K; p.ldc = 2 * I; p.out_dtype = dtype; p.C = gate_up; p.unit = unit;
+  p.idesc = make_idesc_f16(PAIR_M, 0, bf16 ? 1 : 0, 0, 0);
+  p.w_group_rows = 2 * I;
+  return launch_gated<MODE_NT>(tw, tx, tx32, p, bf16, act, stream);
+}
+
+// The input gradient of the layer behind it, on through the unit: w [E, K, I], dy [total_rows, K]; d_gate_up [total_rows, 2 I] from dy w[e] and gate_up.
+// K a multiple of 128, I of 8.
+int cb_grouped_gemm_gated_bwd(const void* dy, const void* w, const void* gate_up, void* d_gate_up, const int* offs, int E, int total_rows, int I,
+                              int K, int lddy, int act, int dtype, cudaStream_t stream) {
+  if (E <= 0 || total_rows <= 0 || I <= 0) return 0;
+  if (E > MAX_GROUPS || (dtype != CB_BF16 && dtype != CB_F16) || (K % 128) || (I & 7) || I > 0x3fffffff) return (int)cudaErrorInvalidValue;
+  const bool bf16 = dtype == CB_BF16;
+  CUtensorMap tx, tx32, tw;
+  int r = make_tmap_2d_16b(&tx, dy, total_rows, K, lddy, ROWS_BOX, 64, bf16);
+  if (!r) r = make_tmap_2d_16b(&tx32, dy, total_rows, K, lddy, BOX_ROWS, 64, bf16);
+  if (r) return 1000 + r;
+  r = make_tmap_2d_16b(&tw, w, (uint64_t)E * K, I, I, BK, 64, bf16);
+  if (r) return 2000 + r;
+  GroupedParams p{};
+  p.offs = offs; p.E = E; p.total_rows = total_rows; p.N = I; p.K = K; p.ldc = 2 * I; p.out_dtype = dtype; p.C = d_gate_up; p.gate_up = gate_up;
+  p.idesc = make_idesc_f16(PAIR_M, 0, bf16 ? 1 : 0, 1, 0);
+  p.w_group_rows = K;
+  return launch_gated<MODE_NN>(tw, tx, tx32, p, bf16, act, stream);
 }
 
 // Variable-K grouped GEMM (weight gradients): dw[e] [M, N] (+)= dy[rows of e, M]^T x[rows of e, N].  Every group's row

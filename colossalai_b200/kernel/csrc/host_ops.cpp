@@ -75,6 +75,8 @@ struct Launchers {
   int (*moe_sum)(const void*, const int*, const float*, void*, int, int, int, int, cudaStream_t);
   int (*moe_sum_bwd)(const void*, const void*, const int*, const float*, void*, float*, int, int, int, int, cudaStream_t);
   int (*grouped)(const void*, const void*, void*, const int*, int, int, int, int, int, int, int, int, cudaStream_t);
+  int (*gated)(const void*, const void*, void*, void*, const int*, int, int, int, int, int, int, int, cudaStream_t);
+  int (*gated_bwd)(const void*, const void*, const void*, void*, const int*, int, int, int, int, int, int, int, cudaStream_t);
   int (*grouped_wgrad)(const void*, const void*, void*, const int*, int, int, int, int, int, int, int, int, int, cudaStream_t);
 } L;
 
@@ -451,14 +453,49 @@ struct GroupedLinear : torch::autograd::Function<GroupedLinear> {
     const c10::cuda::CUDAGuard guard(w.device());
     Tensor dx, dw;
     if (ctx->needs_input_grad(0)) dx = product(dy, w, ends, false);
-    if (ctx->needs_input_grad(1)) {
-      const Tensor x = s[0].contiguous();
-      dw = at::empty({w.size(0), dy.size(1), x.size(1)}, w.options());
-      launched(L.grouped_wgrad(ptr(dy), ptr(x), mut(dw), as<int>(ends), (int)w.size(0), (int)x.size(0), (int)dy.size(1), (int)x.size(1),
-                               (int)dy.stride(0), (int)x.stride(0), code_of(x), code_of(w), 0, stream_of(x)),
-               n_wgrad);
-    }
+    if (ctx->needs_input_grad(1)) dw = weight_grad(dy, s[0].contiguous(), w, ends);
     return {dx, dw, Tensor()};
+  }
+
+  static Tensor weight_grad(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& ends) {
+    Tensor dw = at::empty({w.size(0), dy.size(1), x.size(1)}, w.options());
+    launched(L.grouped_wgrad(ptr(dy), ptr(x), mut(dw), as<int>(ends), (int)w.size(0), (int)x.size(0), (int)dy.size(1), (int)x.size(1),
+                             (int)dy.stride(0), (int)x.stride(0), code_of(x), code_of(w), 0, stream_of(x)),
+             n_wgrad);
+    return dw;
+  }
+};
+
+// Both layers of gated experts: x w_up[e]^T, the unit, its result times w_down[e]^T; w_up [E, 2 I, H], w_down [E, H', I], H' a multiple of 128, I of 64
+struct GatedExperts : torch::autograd::Function<GatedExperts> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w_up, const Tensor& w_down, const Tensor& ends, int64_t act) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const Tensor xc = x.contiguous();
+    const int64_t R = xc.size(0), I = w_up.size(1) / 2;
+    Tensor gu = at::empty({R, 2 * I}, x.options()), unit = at::empty({R, I}, x.options());
+    launched(L.gated(ptr(xc), ptr(w_up), mut(gu), mut(unit), as<int>(ends), (int)w_up.size(0), (int)R, (int)I, (int)xc.size(1), (int)xc.stride(0),
+                     (int)act, code_of(x), stream_of(x)),
+             n_grouped);
+    ctx->save_for_backward({x, w_up, w_down, ends, gu, unit});
+    ctx->saved_data["act"] = act;
+    return GroupedLinear::product(unit, w_down, ends, true);
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const Tensor &w_up = s[1], &w_down = s[2], &ends = s[3], &gu = s[4], &unit = s[5], dy = grads[0].contiguous();
+    const c10::cuda::CUDAGuard guard(gu.device());
+    Tensor dx, d_up, d_down, dgu;
+    if (ctx->needs_input_grad(0) || ctx->needs_input_grad(1)) {
+      dgu = at::empty_like(gu);
+      launched(L.gated_bwd(ptr(dy), ptr(w_down), ptr(gu), mut(dgu), as<int>(ends), (int)w_down.size(0), (int)gu.size(0), (int)unit.size(1),
+                           (int)dy.size(1), (int)dy.stride(0), (int)ctx->saved_data["act"].toInt(), code_of(gu), stream_of(gu)),
+               n_grouped);
+    }
+    if (ctx->needs_input_grad(2)) d_down = GroupedLinear::weight_grad(dy, unit, w_down, ends);
+    if (ctx->needs_input_grad(0)) dx = GroupedLinear::product(dgu, w_up, ends, false);
+    if (ctx->needs_input_grad(1)) d_up = GroupedLinear::weight_grad(dgu, s[0].contiguous(), w_up, ends);
+    return {dx, d_up, d_down, Tensor(), Tensor()};
   }
 };
 
@@ -493,6 +530,8 @@ void bind(const std::map<std::string, uint64_t>& t) {
   take(t, "cb_moe_sum_rows_bwd", L.moe_sum_bwd);
   take(t, "cb_grouped_gemm", L.grouped);
   take(t, "cb_grouped_gemm_wgrad", L.grouped_wgrad);
+  take(t, "cb_grouped_gemm_gated", L.gated);
+  take(t, "cb_grouped_gemm_gated_bwd", L.gated_bwd);
 }
 
 std::map<std::string, long long> counts(bool clear) {
@@ -544,6 +583,11 @@ PYBIND11_MODULE(cb200_host, m) {
   m.def("combine_rows",
         [](const Tensor& rows, const Tensor& weights, const Tensor& slot, const Tensor& src) {
           return CombineRows::apply(rows, weights, slot, src);
+        },
+        release());
+  m.def("gated_experts",
+        [](const Tensor& x, const Tensor& w_up, const Tensor& w_down, const Tensor& ends, int64_t act) {
+          return GatedExperts::apply(x, w_up, w_down, ends, act);
         },
         release());
   m.def("grouped_linear", [](const Tensor& x, const Tensor& w, const Tensor& ends) { return GroupedLinear::apply(x, w, ends); }, release());

@@ -205,7 +205,7 @@ def load(name: str) -> ctypes.CDLL:
 _HOST_CALLS = {
     "cb200_norm": ["cb_rmsnorm_fwd", "cb_rmsnorm_bwd", "cb_norm_bwd_grid"],
     "cb200_moe": ["cb_moe_sort", "cb_moe_take_rows", "cb_moe_sum_rows", "cb_moe_sum_rows_bwd"],
-    "cb200_grouped_gemm": ["cb_grouped_gemm", "cb_grouped_gemm_wgrad"],
+    "cb200_grouped_gemm": ["cb_grouped_gemm", "cb_grouped_gemm_wgrad", "cb_grouped_gemm_gated", "cb_grouped_gemm_gated_bwd"],
     "cb200_elementwise": ["cb_glu_fwd_bounded", "cb_glu_bwd_bounded", "cb_rope", "cb_rope_pages"],
     "cb200_loss": ["cb_ce_row_stats", "cb_ce_loss_blocks", "cb_ce_loss", "cb_ce_softmax_grad"],
     "cb200_attn": ["cb_flash_attn_varlen_fwd", "cb_flash_attn_bwd"],

@@ -83,14 +83,12 @@ class GroupedExperts(nn.Module):
 
     def forward(self, x_sorted: torch.Tensor, counts: torch.Tensor) -> torch.Tensor:
         """x_sorted [N, H] rows grouped by local expert; counts [E_local] rows per expert."""
-        from ..moe.grouped_gemm import grouped_linear, rows_of
+        from ..moe.grouped_gemm import gated_experts, grouped_linear, rows_of
 
+        if self.gated_act is None and self.glu:
+            return gated_experts(x_sorted, self.w_up, self.w_down, counts, self.act)
         h = grouped_linear(x_sorted, self.w_up, counts)
-        if self.gated_act is not None:
-            return grouped_linear(self.gated_act(h, rows_of(counts)), self.w_down, counts)
-        # rows past sum(counts) are padding of an over-allocated receive buffer: the activation skips them (the count
-        # stays on the device)
-        h = ops.glu(h, self.act, valid_rows=rows_of(counts)) if self.glu else ops.get_activation(self.act)(h)
+        h = self.gated_act(h, rows_of(counts)) if self.gated_act is not None else ops.get_activation(self.act)(h)
         return grouped_linear(h, self.w_down, counts)
 
 

@@ -18,6 +18,7 @@ import torch
 
 from ..kernel import loader
 from ..ops._dispatch import plain_call
+from ..ops.activation import _ACT, glu
 from ..ops.moe import expert_ends
 
 _lib = None
@@ -186,3 +187,20 @@ def grouped_linear(x: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, align
         except Exception:
             pass
     return _GroupedLinear.apply(x, w, counts.cpu() if counts.is_cuda else counts)
+
+
+def gated_experts(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, counts: torch.Tensor, act: str) -> torch.Tensor:
+    """act(gate) * up of x @ w_up[e]^T, times w_down[e]^T, for rows grouped by expert.  Aligned groups (see `grouped_linear`) run with the unit in
+    the products' epilogues (squared relu, 3, aside), in both directions; other calls one operator after the other."""
+    aligned = getattr(counts, "cb200_aligned", False)
+    unit = _ACT.get(act, 3)
+    if aligned and unit < 3 and native_ok(x, w_up) and w_down.dtype == x.dtype and w_down.dim() == 3 and w_down.is_contiguous() \
+            and w_down.device == x.device and w_up.shape[2] == x.shape[1] and w_down.shape[0] == w_up.shape[0] \
+            and 2 * w_down.shape[2] == w_up.shape[1] and w_up.shape[1] % K_BLOCK == 0 and w_down.shape[1] % K_BLOCK == 0 \
+            and plain_call(x, w_up, w_down, counts) and (host := loader.host()) is not None:
+        ends, _ = expert_ends(counts)
+        return host.gated_experts(x, w_up, w_down, _offs(counts, x.device) if ends is None else ends, unit)
+    # rows past sum(counts) are padding of an over-allocated receive buffer: the activation skips them (the count
+    # stays on the device)
+    h = glu(grouped_linear(x, w_up, counts), act, valid_rows=rows_of(counts))
+    return grouped_linear(h, w_down, counts)

@@ -29,16 +29,13 @@ __all__ = ["HFMoEPolicy", "HFMixtralPolicy", "HFQwen3MoePolicy", "HFQwen2MoePoli
 
 
 def _ep_experts_forward(self, hidden_states: torch.Tensor, top_k_index: torch.Tensor, top_k_weights: torch.Tensor):
-    from ... import ops
     from ...moe.dispatch_combine import moe_forward
-    from ...moe.grouped_gemm import grouped_linear, rows_of
+    from ...moe.grouped_gemm import gated_experts
 
     act = getattr(self, "_cb200_act", "silu")
 
     def experts(rows: torch.Tensor, counts: torch.Tensor) -> torch.Tensor:
-        h = grouped_linear(rows, self.gate_up_proj, counts)
-        h = ops.glu(h, act, valid_rows=rows_of(counts))
-        return grouped_linear(h, self.down_proj, counts)
+        return gated_experts(rows, self.gate_up_proj, self.down_proj, counts, act)
 
     shape = hidden_states.shape
     x = hidden_states.reshape(-1, shape[-1])

@@ -114,3 +114,39 @@ def test_groups_of_sixteen_rows(counts, K, N, dtype):
             assert ref.numel() == 0 or (got.double() - ref).abs().max() <= eps * ref.abs().max()
         assert (dw32[e].double() - de.t() @ xe).norm() <= 1e-5 * (de.t() @ xe).norm()
         s += n
+
+
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "gelu"])
+@pytest.mark.parametrize("counts,H,inter,dtype", [
+    ([16, 0, 48, 272, 256], 128, 64, torch.bfloat16),         # half a block of columns, an empty group, a tile and a little more
+    ([240, 16, 528], 256, 192, torch.float16),                # a block and a half
+    ([0] * 30 + [16] * 34, 512, 1408, torch.bfloat16),        # the smallest groups
+    ([4096, 16, 1024, 2000], 1024, 704, torch.bfloat16),
+])
+def test_gated_experts(counts, H, inter, dtype, act):
+    """The unit in the epilogues of the products before and behind it: the bits of one operator after the other, rows behind the last group left
+    alone."""
+    from colossalai_b200.kernel import loader
+    from colossalai_b200.moe import grouped_gemm as gg
+    from colossalai_b200.ops import glu
+
+    g = torch.Generator(device="cuda").manual_seed(inter)
+    rows, E = sum(counts), len(counts)
+    c = torch.tensor(counts, device="cuda")
+    c.cb200_aligned = True
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g)
+    ins = [rand(rows + 80, H), rand(E, 2 * inter, H) * H ** -0.5, rand(E, H, inter) * inter ** -0.5]
+    ins = [t.to(dtype).requires_grad_(True) for t in ins]
+    dy = rand(rows + 80, H).to(dtype)
+    out = []
+    for fused in (True, False):
+        loader.launch_counter.reset()
+        if fused:
+            y = gg.gated_experts(*ins, c, act)
+        else:
+            y = gg.grouped_linear(glu(gg.grouped_linear(ins[0], ins[1], c), act, valid_rows=gg.rows_of(c)), ins[2], c)
+        dx, d_up, d_down = torch.autograd.grad(y, ins, dy)
+        out.append([y[:rows], dx[:rows], d_up, d_down])
+        assert any("glu" in name for name in loader.launch_counter.by_name) != fused
+    for a, b in zip(*out):
+        assert torch.equal(a, b)

@@ -233,7 +233,7 @@ def test_paged_decode(monkeypatch, D):
 @pytest.mark.parametrize("mode", ["grad", "no_grad", "inference", "frozen"])
 def test_local_experts(monkeypatch, T, E, k, H, inter, mode):
     """A layer of local experts (outputs of no multiple of 128 included, whose input gradient is not this module's): the same bits and
-    launches without the module, with weights that need no gradient, and with choices of no expert."""
+    products without the module, with weights that need no gradient, and with choices of no expert."""
     from colossalai_b200.models import get_config
     from colossalai_b200.models.moe import GroupedExperts
     from colossalai_b200.moe.dispatch_combine import moe_forward
@@ -270,7 +270,8 @@ def test_local_experts(monkeypatch, T, E, k, H, inter, mode):
             out.append([t.nan_to_num(nan=7.0) for t in fn()])
             out.append(dict(loader.launch_counter.by_name))
     _same(out[0], out[2])
-    assert out[1] == out[3] and out[1]["grouped_gemm"] >= 2
+    without_unit = [{name: n for name, n in o.items() if "glu" not in name} for o in (out[1], out[3])]      # (in the products, with the module)
+    assert without_unit[0] == without_unit[1] and out[1]["grouped_gemm"] >= 2
 
 
 @pytest.mark.gpu
