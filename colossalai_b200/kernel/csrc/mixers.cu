@@ -418,53 +418,82 @@ __global__ void __launch_bounds__(128) scan_prepare_kernel(ScanParams p, ScanWor
 template <typename T, int VEC> CB_DEVICE void load_vec(const void* p, bool f32, int64_t i, float (&v)[VEC]);
 
 // The same for rows and decay mode (without rotation) on widths and addresses that allow four channels per access (the launcher
-// checks): nothing there needs more of a row than the channel itself, so a thread takes quads of q, k, decay and value
-// channels as they come.  Bound: HBM.  12000 tokens of 16 heads x 128 (decay mode, bf16 in): one channel per access 189 us,
-// this 112 us.
-template <typename T, bool ROWS>
-__global__ void __launch_bounds__(256) scan_prepare_vec_kernel(ScanParams p, ScanWork w) {
+// checks): nothing there needs more of a row than the channel itself, so a thread takes a quad of channels of q, k, the decay or the
+// values, of TOK tokens, whose loads are on their way together.  Blocks go along a token's channels first, and the warps of one are spread over them:
+// a decay takes longer than a value.  Bound: HBM, and the activation's exponential and division.  12000 tokens of 16 heads x 128, bf16 in,
+// decay / rows mode: one channel per access 189 us, a block for the quads of one token 107 / 114, this 86 / 102 (65 without the activation); two tokens a thread
+// 93 / 109, eight 127; blocks along the tokens first 92; a block's warps side by side 86 / 106.
+template <typename T, bool ROWS, int TOK>
+__global__ void __launch_bounds__(128) scan_prepare_vec_kernel(ScanParams p, ScanWork w, int tokens) {
   constexpr int SECS = ROWS ? 3 : 2;
-  const int64_t t = blockIdx.x;
   const int dim = p.dim, dq_log = __popc(w.DK / 4 - 1), nq = p.heads << dq_log, vq = w.VP / 4, items = SECS * nq + p.heads * vq;
+  const int it = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+  if (it >= items) return;
+  const int64_t t0 = (int64_t)blockIdx.y * TOK;
+  const int nt = min(TOK, tokens - (int)t0);
   const bool whole = p.vdim == w.VP;
-#pragma unroll 4
-  for (int it = threadIdx.x; it < items; it += 256) {
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    float x[4];
-    if (it < SECS * nq) {
-      const int sec = it < nq ? 0 : (it < 2 * nq ? 1 : 2), r = it - sec * nq, h = r >> dq_log, i = (r - (h << dq_log)) * 4;
-      if (sec == 2) {
-        o = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (i < dim) {
-          const float4 z = *reinterpret_cast<const float4*>((const float*)p.araw + t * p.lda + h * dim + i);
-          const float4 b = *reinterpret_cast<const float4*>(p.dt_bias + h * dim + i);
-          o.x = expf(logsigmoid_f(z.x + b.x) * p.inv_tau); o.y = expf(logsigmoid_f(z.y + b.y) * p.inv_tau);
-          o.z = expf(logsigmoid_f(z.z + b.z) * p.inv_tau); o.w = expf(logsigmoid_f(z.w + b.w) * p.inv_tau);
-        }
-      } else if (i < dim) {
-        const float f = sec == 0 ? p.q_scale : p.k_scale;
-        const T* src = sec == 0 ? (const T*)p.q + t * p.ldq : (const T*)p.k + t * p.ldk;
-        load_vec<T, 4>(src, false, h * dim + i, x);
-        if (!ROWS && p.act_silu) {
+  const int sec = it < nq ? 0 : it < 2 * nq ? 1 : it < SECS * nq ? 2 : 3;
+  const int r = it - min(sec, SECS) * nq;
+  const int h = sec < 3 ? r >> dq_log : (whole ? 0 : r / vq), i = (sec < 3 ? r - (h << dq_log) : r - h * vq) * 4;
+  if (ROWS && sec == 2) {
+    const float* src = (const float*)p.araw + t0 * p.lda + h * dim + i;
+    float* dst = w.g + t0 * p.heads * w.DK + r * 4;
+    float4 z[TOK], b;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) x[e] = silu_f(x[e]);
-        }
-        o = make_float4(x[0] * f, x[1] * f, x[2] * f, x[3] * f);
-      }
-      float* dst = sec == 0 ? w.q : (sec == 1 ? w.k : w.g);
-      *reinterpret_cast<float4*>(dst + t * p.heads * w.DK + r * 4) = o;
-    } else {
-      const int r = it - SECS * nq, h = whole ? 0 : r / vq, c = (r - h * vq) * 4;      // value rows without padding are one
-      if (whole || c < p.vdim) {
-        load_vec<T, 4>((const T*)p.v + t * p.ldv, false, h * p.vdim + c, x);
-        if (!ROWS && p.act_silu) {
+    for (int n = 0; n < TOK; ++n)
+      if (i < dim && n < nt) z[n] = *reinterpret_cast<const float4*>(src + n * p.lda);
+    if (i < dim) b = *reinterpret_cast<const float4*>(p.dt_bias + h * dim + i);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) x[e] = silu_f(x[e]);
-        }
-        o = make_float4(x[0], x[1], x[2], x[3]);
+    for (int n = 0; n < TOK; ++n) {
+      if (n >= nt) break;
+      float4 o = make_float4(1.f, 1.f, 1.f, 1.f);
+      if (i < dim) {
+        o.x = expf(logsigmoid_f(z[n].x + b.x) * p.inv_tau); o.y = expf(logsigmoid_f(z[n].y + b.y) * p.inv_tau);
+        o.z = expf(logsigmoid_f(z[n].z + b.z) * p.inv_tau); o.w = expf(logsigmoid_f(z[n].w + b.w) * p.inv_tau);
       }
-      *reinterpret_cast<float4*>(w.v + t * p.heads * w.VP + r * 4) = o;
+      *reinterpret_cast<float4*>(dst + (int64_t)n * p.heads * w.DK) = o;
     }
+    return;
+  }
+  const T* src = sec == 0 ? (const T*)p.q : sec == 1 ? (const T*)p.k : (const T*)p.v;
+  const int64_t ld = sec == 0 ? p.ldq : sec == 1 ? p.ldk : p.ldv;
+  const int width = sec == 3 ? p.vdim : dim, step = p.heads * (sec == 3 ? w.VP : w.DK);
+  float* dst = (sec == 0 ? w.q : sec == 1 ? w.k : w.v) + t0 * step + r * 4;
+  const bool there = (sec == 3 && whole) || i < width;
+  src += t0 * ld + h * width + i;
+  float x[TOK][4];
+#pragma unroll
+  for (int n = 0; n < TOK; ++n)
+    if (there && n < nt) load_vec<T, 4>(src, false, n * ld, x[n]);
+  const float f = sec == 0 ? p.q_scale : p.k_scale;
+#pragma unroll
+  for (int n = 0; n < TOK; ++n) {
+    if (n >= nt) break;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (there) {
+      if (!ROWS && p.act_silu) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[n][e] = silu_f(x[n][e]);
+      }
+      o = sec == 3 ? make_float4(x[n][0], x[n][1], x[n][2], x[n][3]) : make_float4(x[n][0] * f, x[n][1] * f, x[n][2] * f, x[n][3] * f);
+    }
+    *reinterpret_cast<float4*>(dst + (int64_t)n * step) = o;
+  }
+}
+
+// One token a thread where that many blocks are on the chip at a time, or else four: us with one and with four, decay mode, 64 tokens of 16 heads x 128 2.6
+// and 3.4, 16 of 8 x 64 2.0 and 2.9, 256 of 16 x 128 (3072 blocks of one) 4.6 and 4.2, 1024 11.5 and 9.4.
+template <typename T, bool ROWS> void launch_scan_prepare_vec(ScanParams p, ScanWork w, int64_t tokens, cudaStream_t st) {
+  const unsigned chunks = (unsigned)((p.heads * ((ROWS ? 3 : 2) * w.DK + w.VP) / 4 + 127) / 128);
+  const bool several = tokens * chunks > 16 * cb_num_sms();
+  const int64_t most = several ? 4 * 65535 : 65535;                     // a grid has 65535 rows of blocks
+  for (; tokens > 0; tokens -= most) {
+    const int n = (int)(tokens < most ? tokens : most);
+    if (several) scan_prepare_vec_kernel<T, ROWS, 4><<<dim3(chunks, (n + 3) / 4), 128, 0, st>>>(p, w, n);
+    else scan_prepare_vec_kernel<T, ROWS, 1><<<dim3(chunks, n), 128, 0, st>>>(p, w, n);
+    p.q = (const T*)p.q + n * p.ldq; p.k = (const T*)p.k + n * p.ldk; p.v = (const T*)p.v + n * p.ldv;
+    w.q += (int64_t)n * p.heads * w.DK; w.k += (int64_t)n * p.heads * w.DK; w.v += (int64_t)n * p.heads * w.VP;
+    if (ROWS) p.araw = (const float*)p.araw + n * p.lda, w.g += (int64_t)n * p.heads * w.DK;
   }
 }
 
@@ -893,9 +922,9 @@ int launch_scan(const ScanParams& p, float* work, int64_t tokens, int nseq, int 
                            quads(p.q, p.ldq, sizeof(T)) && quads(p.k, p.ldk, sizeof(T)) && quads(p.v, p.ldv, sizeof(T)) &&
                            quads(work, 0, 4);
   if (MODE == SCAN_ROWS && !p.act_silu && no_row_math && quads(p.araw, p.lda, 4) && quads(p.dt_bias, 0, 4))
-    scan_prepare_vec_kernel<T, true><<<(unsigned)tokens, 256, 0, st>>>(p, w);
+    launch_scan_prepare_vec<T, true>(p, w, tokens, st);
   else if (MODE == SCAN_DECAY && no_row_math)
-    scan_prepare_vec_kernel<T, false><<<(unsigned)tokens, 256, 0, st>>>(p, w);
+    launch_scan_prepare_vec<T, false>(p, w, tokens, st);
   else
     scan_prepare_kernel<MODE, T><<<(unsigned)tokens, 128, 0, st>>>(p, w);
   if (MODE == SCAN_GATED && p.gate_kind == GATE_EXP) {

@@ -200,6 +200,32 @@ def test_decay_scan_columns_of_a_lane(H, d, dv, lens):
     assert torch.equal(state, parts)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("mode", ["decay", "rows"])
+@pytest.mark.parametrize("H,d,dv,lens", [(16, 128, 128, [1]), (3, 128, 128, [3, 2]), (5, 80, 40, [4, 9]), (7, 96, 128, [31, 16]),
+                                         (2, 12, 4, [2]), (16, 128, 128, [600, 7]), (5, 80, 40, [1201, 4]), (7, 96, 128, [801, 4]),
+                                         (1, 16, 32, [2048] * 128 + [7])])         # more groups of four tokens than a grid has rows
+def test_scan_preparation_in_quads(H, d, dv, lens, mode, dtype):
+    """Rows that are read four channels of one token or of four at a time: the bits of rows whose strides allow one channel at a time only."""
+    dev, T, n = _dev("cuda"), sum(lens), len(lens)
+    g = torch.Generator(device=dev).manual_seed(T)
+    rand = lambda *shape: torch.randn(*shape, generator=g, device=dev)
+    q, k, v = (rand(T, H * w).to(dtype) for w in (d, d, dv))
+    pre, chan, head = rand(T, H * d), rand(H * d), torch.rand(H, generator=g, device=dev)
+    meta = M.RaggedMeta.build(lens, [5] * n, list(range(n)), dev)
+    start = rand(n, H, d, dv)
+    out = []
+    for odd in (0, 1):
+        state = start.clone()
+        rows = [torch.cat([t, t[:, :odd]], 1)[:, :t.shape[1]] for t in (q, k, v)]
+        assert all(t.stride(0) % 4 == odd for t in rows)
+        o = M.state_scan_decay(*rows, head, state, meta, H, d, dv, q_scale=0.7) if mode == "decay" else \
+            M.state_scan_gla(*rows, pre, chan, 16.0, state, meta, H, d, dv)
+        out.append((o, state))
+    assert torch.isfinite(out[0][0]).all() and torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
 @pytest.mark.parametrize("device", DEVICES)
 @pytest.mark.parametrize("L", [8, 13, 16])
 def test_decay_scan_of_infinite_and_very_large_values(device, L):
