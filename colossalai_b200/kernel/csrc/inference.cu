@@ -472,7 +472,17 @@ template <> CB_DEVICE uint32_t pack2<__half>(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-template <typename T, int D>
+template <typename T> CB_DEVICE float2 unpack2(uint32_t v);
+template <> CB_DEVICE float2 unpack2<__nv_bfloat16>(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&v)); }
+template <> CB_DEVICE float2 unpack2<__half>(uint32_t v) { return __half22float2(*reinterpret_cast<__half2*>(&v)); }
+
+// REST: the rows of P V that have no heads take what the rounding of the weights to 16 bits left.  The largest weight of a partition is exact, and
+// sequences that are cut into fewer partitions than of DEC_PART_MIN tokens have fewer exact ones: error against 64 bits, 16 sequences of up to 1024 tokens
+// in bf16, 2.03e-3 in short partitions, 2.06e-3 in long ones, 1.66e-3 with the rest; one of 16000 in fp16 2.55e-4, 2.70e-4 and 2.10e-4.  For calls
+// that are cut by their own lengths where the table has room for more than DEC_REST tokens a partition: everywhere it would cost 64 sequences of
+// 2048 tokens 2 us of 77, and one of 4097, whose partitions are short, .5 of 14.
+constexpr int DEC_REST = 96;
+template <typename T, int D, bool REST>
 __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
     const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
     const int* __restrict__ block_tables, const int* __restrict__ seq_lens, float* __restrict__ o_part,
@@ -583,7 +593,10 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
       const float corr = (m_new == -INFINITY) ? 1.f : ex2_approx(m_run - m_new);
       l_run *= corr;
 #pragma unroll
-      for (int j = 0; j < NO; ++j) { o[j][0] *= corr; o[j][1] *= corr; }
+      for (int j = 0; j < NO; ++j) {
+        o[j][0] *= corr; o[j][1] *= corr;
+        if (REST) { o[j][2] *= corr; o[j][3] *= corr; }
+      }
     }
     m_run = m_new;
     float pv[4];
@@ -592,10 +605,15 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
       pv[i] = (sv[i] == -INFINITY) ? 0.f : ex2_approx(sv[i] - m_new);
       l_run += pv[i];
     }
-    // P as A operand [16 heads x 16 tokens]: a0 = tokens 0..7 of this row, a2 = tokens 8..15; rows 8..15 are zero
+    // P as A operand [16 heads x 16 tokens]: a0 = tokens 0..7 of this row, a2 = tokens 8..15; rows 8..15 are zero or REST
     uint32_t pa[4];
     pa[0] = row_ok ? pack2<T>(pv[0], pv[1]) : 0u; pa[1] = 0u;
     pa[2] = row_ok ? pack2<T>(pv[2], pv[3]) : 0u; pa[3] = 0u;
+    if (REST) {
+      const float2 a = unpack2<T>(pa[0]), b = unpack2<T>(pa[2]);
+      pa[1] = row_ok ? pack2<T>(pv[0] - a.x, pv[1] - a.y) : 0u;
+      pa[3] = row_ok ? pack2<T>(pv[2] - b.x, pv[3] - b.y) : 0u;
+    }
     // ---- O += P V: V^T fragments through ldmatrix.trans
     {
       const int tr = (lane & 7) + ((lane >> 3) & 1) * 8;     // matrices: (tok 0..7, j), (tok 8..15, j), (0..7, j+1), (8..15, j+1)
@@ -636,7 +654,13 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
     const int64_t oi = (((int64_t)seq * Hq + kvh * G + row) * splits + split);
     float* dst = o_part + oi * D + quad * 2;
 #pragma unroll
-    for (int j = 0; j < NO; ++j) *reinterpret_cast<float2*>(dst + j * 8) = make_float2(o[j][0], o[j][1]);
+    for (int j = 0; j < NO; ++j) {
+      if (REST) {                               // (an infinite value stays what it is: its remainder's sign would make a NaN of it)
+        if (isfinite(o[j][0])) o[j][0] += o[j][2];
+        if (isfinite(o[j][1])) o[j][1] += o[j][3];
+      }
+      *reinterpret_cast<float2*>(dst + j * 8) = make_float2(o[j][0], o[j][1]);
+    }
     if (quad == 0) { ml_part[oi * 2] = m_run * LN2; ml_part[oi * 2 + 1] = l_run; }
   }
 }
@@ -871,8 +895,11 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
   {                                                                                                                  \
     constexpr int per_warp = DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * DD * 2;                                           \
     static CbDeviceAttr attr;                                                                                        \
-    if (const int e = cb_allow_smem(attr, paged_decode_mma_kernel<T, DD>, (DEC_THREADS / 32) * per_warp)) return e;  \
-    if (const int e = cb_launch_early(paged_decode_mma_kernel<T, DD>, mma_grid, mma_warps * 32, mma_warps * per_warp, s, \
+    static CbDeviceAttr attr_rest;                                                                                   \
+    const bool rest = part_len < 0 && cut.capacity > (int64_t)DEC_REST * splits;                                     \
+    auto kern = rest ? paged_decode_mma_kernel<T, DD, true> : paged_decode_mma_kernel<T, DD, false>;                 \
+    if (const int e = cb_allow_smem(rest ? attr_rest : attr, kern, (DEC_THREADS / 32) * per_warp)) return e;         \
+    if (const int e = cb_launch_early(kern, mma_grid, mma_warps * 32, mma_warps * per_warp, s, \
         (const T*)q, (const T*)k_cache, (const T*)v_cache, block_tables, seq_lens, o_part, ml_part, Hq, Hkv,        \
         block_size, max_blocks_per_seq, splits, part_len, scale, alibi_slopes, q_stride, window)) return e;         \
     if (const int e = launch_decode_reduce<T, DD>(o_part, ml_part, (T*)out, num_seqs, Hq, splits, out_stride, cut, s)) return e; \

@@ -347,3 +347,34 @@ def test_paged_decode_partitions_of_a_length(n, Hq, Hkv, D, room):
     other = lens.clone()
     other[1:] = (lens[1:] // 2).clamp(min=1)
     assert torch.equal(iops.paged_decode_attention(q, kc, vc, tables, other)[0], out[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,Hq,Hkv,D,length", [(1, 8, 8, 128, 8000), (4, 16, 4, 64, 7200), (12, 8, 1, 128, 6400)])
+def test_paged_decode_weights_with_their_remainders(n, Hq, Hkv, D, length, dtype):
+    """Sequences in few long partitions: the weights are not rounded to 16 bits, so what differs from 64 bits is the result's own rounding, and an
+    infinite value is infinite in the result."""
+    dev, page = "cuda", 16
+    g = torch.Generator(device=dev).manual_seed(length)
+    width = length // page
+    lens = torch.tensor([length - 37 * i for i in range(n)], dtype=torch.int32, device=dev)
+    tables = torch.randperm(n * width, device=dev, generator=g).view(n, width).to(torch.int32)
+    q = torch.randn(n, Hq, D, device=dev, generator=g).to(dtype)
+    kc, vc = (torch.randn(n * width, page, Hkv, D, device=dev, generator=g).to(dtype) for _ in "kv")
+    out = iops.paged_decode_attention(q, kc, vc, tables, lens)
+    ref = []
+    for i in range(n):
+        k, v = (c[tables[i].long()].flatten(0, 1)[: lens[i]].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+        w = (torch.einsum("hd,khd->hk", q[i].double(), k) * D ** -0.5).softmax(-1)
+        ref.append(torch.einsum("hk,khd->hd", w, v))
+    ref = torch.stack(ref)
+    # half a unit of the last place; weights, one in all, of values of about one: with twice eight bits and two signs 2^-18 (4e-6), and from scores whose
+    # fp32 sums are off by some 2^-17 (8e-6)
+    bits = 8 if dtype == torch.bfloat16 else 11
+    assert ((out.double() - ref).abs() <= 2.0 ** -bits * ref.abs() + 2e-5).all()
+    vc[tables[0, 3].long(), 5, 0, 7] = float("inf")
+    got = iops.paged_decode_attention(q, kc, vc, tables, lens)
+    same = torch.ones(n, Hq, D, dtype=torch.bool, device=dev)
+    same[0, : Hq // Hkv, 7] = False
+    assert (got[~same] == float("inf")).all() and torch.equal(got[same], out[same])
