@@ -50,8 +50,9 @@ constexpr int DEC_MMA_WARPS = 4;
 // Two rounds of what the table holds / one of the length, tables just wide enough, us: 16 x 1024 tokens of 32 / 8 heads of 128 22.6 / 18.2, 16 x 8000
 // 86 / 79, 2 x 16000 38.0 / 29.6, 10 x 8000 60.0 / 54.9, 28 x 4000 75.0 / 69.8, 6 x 12000 of 16 / 2 heads of 64 29.1 / 22.4, 60 x 2000 of 16 / 2 heads of 128
 // 37.8 / 31.2, 5 x 8000 of 12 heads 50.5 / 43.9; tables of 8192 tokens of which 500 to 1000 are in use, 16 sequences 40.8 / 17, 28 64 / 21.  More
-// than DEC_MOST_SPLITS partitions cost as many results more than they give CTAs (96: 2 x 6000 21.0 instead of 17.8, 1 x 16000 25.2 instead of
-// 26.4).  Where a round is fewer than DEC_ROUND_SPLITS partitions - lengths differ by more than one - two rounds (one / two: 40 x 3000 79.8 / 73.0, 32 x
+// than DEC_MOST_SPLITS partitions cost as many results more than they give CTAs (96: 2 x 6000 21.0 instead of 17.8), but for a sequence alone, which
+// takes half as many as there are SMs (74 and 64: 1 x 4700 14.2 and 14.8, 1 x 8000 18.4 and 19.1, 1 x 30000 41.9 and 41.0; 2 x 4600 18.0 and 16.4, 2 x
+// 9000 25.5 and 22.4).  Where a round is fewer than DEC_ROUND_SPLITS partitions - lengths differ by more than one - two rounds (one / two: 40 x 3000 79.8 / 73.0, 32 x
 // 4000 79.8 / 76.0), and where that is as few, and for more than four heads of 64, of what the table holds (64 x 2048 76.9, own 80.3; 30 x 4000 of 24 / 8
 // heads of 64 38.6, own 43.4).
 constexpr int DEC_PART_MIN = 64, DEC_ROUND_SPLITS = 5, DEC_MOST_SPLITS = 64;
@@ -854,7 +855,8 @@ int cb_decode_num_splits(int num_seqs, int kv_heads, int head_dim, int max_len, 
   const int ctas = num_seqs * ((kv_heads + warps - 1) / warps), one_round = per_sm * sms / ctas, two_rounds = 2 * per_sm * sms / ctas;
   if ((head_dim == 128 || kv_heads <= 4) && head_dim <= 128 && (one_round >= DEC_ROUND_SPLITS || two_rounds > DEC_ROUND_SPLITS)) {
     *part_len_out = -DEC_PART_MIN;
-    const int own = one_round >= DEC_ROUND_SPLITS ? one_round : two_rounds, splits = own < DEC_MOST_SPLITS ? own : DEC_MOST_SPLITS;
+    const int own = one_round >= DEC_ROUND_SPLITS ? one_round : two_rounds, cap = num_seqs == 1 ? sms / 2 : DEC_MOST_SPLITS;
+    const int splits = own < cap ? own : cap;
     return splits < most ? splits : most < 1 ? 1 : most;
   }
   // two rounds of CTAs of eight kv heads, partitions of at least DEC_PART_MIN of the tokens that a table has room for
