@@ -650,7 +650,7 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
   const int dim = p.dim, vdim = p.vdim;
   const int r0 = part * RP, r0p = part * RPP;
   float* Sg = p.state + ((int64_t)p.slots[s] * p.heads + h) * dim * vdim;
-  const bool vec = vdim % CPL == 0 && j0 < vdim;               // all of the lane's columns, aligned
+  const bool vec = vdim % CPL == 0 && j0 < vdim && (uintptr_t)Sg % (4 * CPL) == 0;       // all of the lane's columns, aligned
   const bool carried = p.ctx_len[s] > 0;
   // Pairs of neighbouring ROWS share an instruction: q, k and the decays arrive from shared memory as such pairs, and only the
   // token's CPL values are duplicated.

@@ -201,6 +201,27 @@ def test_decay_scan_columns_of_a_lane(H, d, dv, lens):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("offset", [1, 2, 4])
+@pytest.mark.parametrize("H,d,dv,lens", [(20, 128, 66, [50, 35]), (20, 128, 66, [20, 3]), (9, 64, 64, [90]), (16, 128, 128, [70]), (16, 128, 128, [5]),
+                                         (16, 64, 128, [60] * 6), (3, 128, 37, [47])])
+def test_decay_scan_of_a_state_at_any_address(H, d, dv, lens, offset):
+    """A contiguous state that starts between the boundaries of the vectors its rows are otherwise read in, whatever a lane's columns are:
+    the bits of one that starts on them, and nothing written beside it."""
+    dev, n = _dev("cuda"), len(lens)
+    g = torch.Generator().manual_seed(H)
+    q, k, v = (torch.randn(sum(lens), H * w, generator=g).to(dev) for w in (d, d, dv))
+    head, state = torch.rand(H, generator=g).to(dev), torch.randn(n, H, d, dv, generator=g).to(dev)
+    buffer = torch.full((state.numel() + 8,), 7.0, device=dev)
+    moved = buffer[offset: offset + state.numel()].view_as(state)
+    moved.copy_(state)
+    assert moved.data_ptr() % 16 == 4 * offset % 16
+    meta = M.RaggedMeta.build(lens, [5] * n, list(range(n)), dev)
+    out = [M.state_scan_decay(q, k, v, head, s, meta, H, d, dv) for s in (state, moved)]
+    assert torch.equal(*out) and torch.equal(state, moved)
+    assert (buffer[:offset] == 7).all() and (buffer[offset + state.numel():] == 7).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("mode", ["decay", "rows"])
 @pytest.mark.parametrize("H,d,dv,lens", [(16, 128, 128, [1]), (3, 128, 128, [3, 2]), (5, 80, 40, [4, 9]), (7, 96, 128, [31, 16]),
