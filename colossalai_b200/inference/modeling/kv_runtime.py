@@ -169,8 +169,8 @@ class PagedKVRuntime:
                          heads: int, kv_heads: int, dim: int, rot_dim: int, interleaved: bool) -> Optional[torch.Tensor]:
         """A decode step's rows q | k | v as `ops.rope_qkv` turns them, their keys and values written to the layer's pages in the same
         launch (`attend` is then told so); None where that kernel does not serve."""
-        if self.is_prompt or self.ragged is not None or torch.is_grad_enabled() or type(self).attend is not PagedKVRuntime.attend:
-            return None
+        if self.is_prompt or self.ragged is not None or torch.is_grad_enabled() or type(self).attend is not _ATTEND or "attend" in vars(self):
+            return None                                       # (a replaced `attend` knows nothing of `written`)
         i = self.cache_index(layer_idx)
         return iops.rope_pages(qkv, positions, cos, sin, heads, kv_heads, dim, rot_dim, interleaved, self.k_caches[i], self.v_caches[i],
                                self.block_tables, self.token_seq, self.token_pos)
@@ -270,3 +270,6 @@ class PagedKVRuntime:
             outs.append(iops.paged_decode_attention(qj.contiguous(), kc, vc, self.block_tables,
                                                     self.seq_lens - (n - 1 - j), scale))
         return torch.stack(outs, 1).reshape(q.shape)
+
+
+_ATTEND = PagedKVRuntime.attend

@@ -174,7 +174,7 @@ class Attention(nn.Module):
             qkv = torch.cat([q, k, v], dim=-1)
         written = None
         if rope is not None:
-            if hasattr(kv_cache, "rotate_and_write"):
+            if hasattr(type(kv_cache), "rotate_and_write"):    # (its own, not that of a cache that it wraps)
                 written = kv_cache.rotate_and_write(self.layer_idx, qkv, meta.positions, rope[0], rope[1], hq, hkv, D, cfg.rotary_dim,
                                                     cfg.rope_interleaved)
             qkv = written if written is not None else ops.rope_qkv(qkv, meta.positions, rope[0], rope[1], hq, hkv, D,

@@ -64,6 +64,66 @@ def test_engine_matches_naive_greedy_with_continuous_batching():
         assert len(got) == len(ref) or got[-1] == 2
 
 
+@pytest.mark.parametrize("replaced", ["nothing", "instance", "class", "subclass", "wrapper"])
+def test_a_replaced_attend_of_the_cache_is_called_as_it_always_was(monkeypatch, replaced):
+    """A step may leave the page write to the rotation's kernel only where the cache's own `attend` is what runs: a replacement gets the
+    arguments that it always got, with keys and values not written yet.  (A stand-in for the kernel takes every call.)"""
+    from colossalai_b200 import ops
+    from colossalai_b200.inference.modeling import PagedKVRuntime
+    from colossalai_b200.ops import inference as iops
+
+    fused, calls = [], []
+
+    def rope_pages(qkv, positions, cos, sin, heads, kv_heads, dim, rot, interleaved, kc, vc, tables, seq, pos):
+        y = ops.rope_qkv(qkv, positions, cos, sin, heads, kv_heads, dim, rot_dim=rot, interleaved=interleaved)
+        _, k, v = (t.reshape(len(y), -1, dim) for t in y.split([heads * dim, kv_heads * dim, kv_heads * dim], -1))
+        iops.kv_cache_write(k, v, kc, vc, tables, seq, pos)
+        fused.append(1)
+        return y
+
+    def attend(self, layer_idx, q, k, v, meta, scale):                    # a user's own, of before
+        calls.append(1)
+        return original(self, layer_idx, q, k, v, meta, scale)
+
+    class Sub(PagedKVRuntime):
+        def attend(self, layer_idx, q, k, v, meta, scale):
+            calls.append(1)
+            return super().attend(layer_idx, q, k, v, meta, scale)
+
+    class Wrapper:
+        def __init__(self, inner):
+            self.inner = inner
+
+        def attend(self, layer_idx, q, k, v, meta, scale):
+            calls.append(1)
+            return self.inner.attend(layer_idx, q, k, v, meta, scale)
+
+        def __getattr__(self, name):
+            return getattr(self.inner, name)
+
+    original = PagedKVRuntime.attend
+    monkeypatch.setattr(iops, "rope_pages", rope_pages)
+    torch.manual_seed(0)
+    model = build_model("llama-tiny").float().eval()
+    cfg = InferenceConfig(max_batch_size=2, max_input_len=24, max_output_len=6, block_size=8, dtype="fp32", use_cuda_graph=False)
+    engine = InferenceEngine(model, None, cfg)
+    owner = engine.engine
+    rt = owner.kv_runtime
+    if replaced == "instance":
+        rt.attend = attend.__get__(rt)
+    elif replaced == "class":
+        monkeypatch.setattr(PagedKVRuntime, "attend", attend)
+    elif replaced == "subclass":
+        rt.__class__ = Sub
+    elif replaced == "wrapper":
+        owner.kv_runtime = Wrapper(rt)
+    prompt = [5, 9, 13, 200, 7]
+    _, ids = engine.generate(prompts_token_ids=[prompt], return_token_ids=True, generation_config=GenerationConfig(max_new_tokens=6))
+    want = _naive_greedy(model, prompt, 6)
+    assert len(ids[0]) > 1 and ids[0] == want[: len(ids[0])]
+    assert bool(fused) == (replaced == "nothing") and bool(calls) == (replaced != "nothing")
+
+
 def test_speculative_decoding_matches_plain_greedy():
     torch.manual_seed(0)
     model = build_model("llama-tiny").float().eval()
