@@ -480,9 +480,8 @@ template <> CB_DEVICE float2 unpack2<__half>(uint32_t v) { return __half22float2
 // REST: the rows of P V that have no heads take what the rounding of the weights to 16 bits left.  The largest weight of a partition is exact, and
 // sequences that are cut into fewer partitions than of DEC_PART_MIN tokens have fewer exact ones: error against 64 bits, 16 sequences of up to 1024 tokens
 // in bf16, 2.03e-3 in short partitions, 2.06e-3 in long ones, 1.66e-3 with the rest; one of 16000 in fp16 2.55e-4, 2.70e-4 and 2.10e-4.  For calls
-// that are cut by their own lengths where the table has room for more than DEC_REST tokens a partition: everywhere it would cost 64 sequences of
-// 2048 tokens 2 us of 77, and one of 4097, whose partitions are short, .5 of 14.
-constexpr int DEC_REST = 96;
+// that are cut by their own lengths where the table has room for more than DEC_PART_MIN tokens a partition; the others' are no longer than they ever were,
+// and 64 sequences of 2048 tokens, cut by their table, would take 79 us with it instead of 77.
 template <typename T, int D, bool REST>
 __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
     const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
@@ -898,7 +897,7 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
     constexpr int per_warp = DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * DD * 2;                                           \
     static CbDeviceAttr attr;                                                                                        \
     static CbDeviceAttr attr_rest;                                                                                   \
-    const bool rest = part_len < 0 && cut.capacity > (int64_t)DEC_REST * splits;                                     \
+    const bool rest = part_len < 0 && cut.capacity > (int64_t)DEC_PART_MIN * splits;                                     \
     auto kern = rest ? paged_decode_mma_kernel<T, DD, true> : paged_decode_mma_kernel<T, DD, false>;                 \
     if (const int e = cb_allow_smem(rest ? attr_rest : attr, kern, (DEC_THREADS / 32) * per_warp)) return e;         \
     if (const int e = cb_launch_early(kern, mma_grid, mma_warps * 32, mma_warps * per_warp, s, \

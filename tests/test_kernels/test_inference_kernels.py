@@ -351,9 +351,10 @@ def test_paged_decode_partitions_of_a_length(n, Hq, Hkv, D, room):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("n,Hq,Hkv,D,length", [(1, 8, 8, 128, 8000), (4, 16, 4, 64, 7200), (12, 8, 1, 128, 6400)])
+@pytest.mark.parametrize("n,Hq,Hkv,D,length", [(1, 8, 8, 128, 8000), (4, 16, 4, 64, 7200), (12, 8, 1, 128, 6400), (16, 16, 8, 128, 800),
+                                                   (4, 8, 8, 128, 2880), (8, 12, 12, 128, 960), (1, 8, 8, 128, 5600)])
 def test_paged_decode_weights_with_their_remainders(n, Hq, Hkv, D, length, dtype):
-    """Sequences in few long partitions: the weights are not rounded to 16 bits, so what differs from 64 bits is the result's own rounding, and an
+    """Sequences in partitions of more than 64 tokens (80 and 96 among them): the weights are not rounded to 16 bits, so what differs from 64 bits is the result's own rounding, and an
     infinite value is infinite in the result."""
     dev, page = "cuda", 16
     g = torch.Generator(device=dev).manual_seed(length)
