@@ -429,6 +429,30 @@ struct CombineRows : torch::autograd::Function<CombineRows> {
   }
 };
 
+// The same product in torch operations, zeros behind the last expert's rows: what gradients that are to be differentiated again are made of
+Tensor product_by_expert(const Tensor& x, const Tensor& w, const Tensor& ends) {
+  const Tensor host = ends.cpu();
+  variable_list parts;
+  int64_t from = 0;
+  for (int64_t e = 0; e < w.size(0); ++e) {
+    const int64_t to = host.const_data_ptr<int>()[e];
+    parts.push_back(at::matmul(x.slice(0, from, to), w.select(0, e).t()));
+    from = to;
+  }
+  parts.push_back(at::zeros({x.size(0) - from, w.size(1)}, x.options()));
+  return at::cat(parts, 0);
+}
+// gradients, with a graph of their own, of y for the inputs that want one; `tensors`: as many inputs as forward has tensors
+variable_list grads_with_graph(AutogradContext* ctx, const Tensor& y, const Tensor& dy, const variable_list& tensors) {
+  variable_list wanted, out(tensors.size());
+  for (size_t i = 0; i < tensors.size(); ++i)
+    if (ctx->needs_input_grad(i)) wanted.push_back(tensors[i]);
+  const variable_list got = torch::autograd::grad({y}, wanted, {dy}, c10::nullopt, true);
+  for (size_t i = 0, n = 0; i < tensors.size(); ++i)
+    if (ctx->needs_input_grad(i)) out[i] = got[n++];
+  return out;
+}
+
 // y[rows of e] = x[rows of e] w[e]^T; w [E, N, K] contiguous, N a multiple of 128 (the input gradient's blocks), ends int32 [E]: where
 // each expert's rows end, multiples of 16.  The caller has checked types and sizes.
 struct GroupedLinear : torch::autograd::Function<GroupedLinear> {
@@ -451,6 +475,10 @@ struct GroupedLinear : torch::autograd::Function<GroupedLinear> {
     const variable_list s = ctx->get_saved_variables();
     const Tensor &w = s[1], &ends = s[2], dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(w.device());
+    if (at::GradMode::is_enabled()) {
+      const variable_list d = grads_with_graph(ctx, product_by_expert(s[0], w, ends), grads[0], {s[0], w});
+      return {d[0], d[1], Tensor()};
+    }
     Tensor dx, dw;
     if (ctx->needs_input_grad(0)) dx = product(dy, w, ends, false);
     if (ctx->needs_input_grad(1)) dw = weight_grad(dy, s[0].contiguous(), w, ends);
@@ -485,6 +513,13 @@ struct GatedExperts : torch::autograd::Function<GatedExperts> {
     const variable_list s = ctx->get_saved_variables();
     const Tensor &w_up = s[1], &w_down = s[2], &ends = s[3], &gu = s[4], &unit = s[5], dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(gu.device());
+    if (at::GradMode::is_enabled()) {
+      const int64_t act = ctx->saved_data["act"].toInt();
+      const variable_list h = product_by_expert(s[0], w_up, ends).to(at::kFloat).chunk(2, 1);
+      const Tensor a = (act == 0 ? at::silu(h[0]) : at::gelu(h[0], act == 1 ? "tanh" : "none")) * h[1];
+      const variable_list d = grads_with_graph(ctx, product_by_expert(a.to(unit.scalar_type()), w_down, ends), grads[0], {s[0], w_up, w_down});
+      return {d[0], d[1], d[2], Tensor(), Tensor()};
+    }
     Tensor dx, d_up, d_down, dgu;
     if (ctx->needs_input_grad(0) || ctx->needs_input_grad(1)) {
       dgu = at::empty_like(gu);

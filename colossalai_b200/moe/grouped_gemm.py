@@ -121,6 +121,12 @@ class _GroupedLinearNative(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, counts, offs = ctx.saved_tensors
+        if torch.is_grad_enabled():                          # to be differentiated again: torch operations
+            sizes = counts.tolist()
+            n = sum(sizes)
+            dys, xs = dy[:n].split(sizes), x[:n].split(sizes)
+            dx = torch.cat([d @ m for d, m in zip(dys, w)] + [torch.zeros_like(x[n:])]) if ctx.needs_input_grad[0] else None
+            return dx, torch.stack([d.t() @ r for d, r in zip(dys, xs)]) if ctx.needs_input_grad[1] else None, None, None
         dy = dy.contiguous()
         dx = dw = None
         if ctx.needs_input_grad[0]:

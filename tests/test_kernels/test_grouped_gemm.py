@@ -150,3 +150,48 @@ def test_gated_experts(counts, H, inter, dtype, act):
         assert any("glu" in name for name in loader.launch_counter.by_name) != fused
     for a, b in zip(*out):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("form", ["gated", "linear", "python"])
+@pytest.mark.parametrize("frozen", [False, True])
+def test_expert_gradients_that_are_differentiated_again(form, frozen, monkeypatch):
+    """Gradients under `create_graph` carry a graph: their own gradients against 64 bits, for all inputs or for the rows alone."""
+    from colossalai_b200.kernel import loader
+    from colossalai_b200.moe import grouped_gemm as gg
+
+    if form == "python":
+        loader.host()
+        monkeypatch.setattr(loader, "_host", None)
+    counts, H, inter = [16, 0, 48, 32], 128, 64
+    rows = sum(counts)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    c = torch.tensor(counts, device="cuda")
+    c.cb200_aligned = True
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g)
+    ins = [rand(rows + 16, H), rand(4, 2 * inter, H) * H ** -0.5] + ([rand(4, H, inter) * inter ** -0.5] if form == "gated" else [])
+    ins = [t.bfloat16().requires_grad_(i == 0 or not frozen) for i, t in enumerate(ins)]
+    dy = rand(rows + 16, H if form == "gated" else 2 * inter).bfloat16().requires_grad_()
+
+    def second(fn, tensors, dy):
+        live = [t for t in tensors if t.requires_grad]
+        first = torch.autograd.grad(fn(*tensors), live, dy, create_graph=True)
+        total = sum((t[:rows] if t.dim() == 2 else t).double().square().sum() for t in first)
+        return [t.double() for t in torch.autograd.grad(total, live + [dy], allow_unused=True) if t is not None]
+
+    def exact(x, w_up, w_down=None):
+        parts, out = x[:rows].split(counts), []
+        for e, part in enumerate(parts):
+            h = part @ w_up[e].t()
+            if w_down is not None:
+                gate, up = h.chunk(2, -1)
+                h = (torch.nn.functional.silu(gate) * up) @ w_down[e].t()
+            out.append(h)
+        return torch.cat(out + [torch.zeros(16, out[0].shape[1], dtype=x.dtype, device=x.device)])
+
+    fn = (lambda *t: gg.gated_experts(*t, c, "silu")) if form == "gated" else (lambda *t: gg.grouped_linear(*t, c))
+    got = second(fn, ins, dy)
+    wide = [t.detach().double().requires_grad_(t.requires_grad) for t in ins]
+    want = second(exact, wide, dy.detach().double().requires_grad_())
+    assert len(got) == len(want) >= 1
+    for a, b in zip(got, want):                     # 16-bit operands and results throughout: some roundings of 2^-9
+        assert (a - b).norm() <= 2e-2 * b.norm()
