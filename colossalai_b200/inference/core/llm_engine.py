@@ -162,7 +162,8 @@ class LLMEngine(BaseEngine):
         try:
             lib = infer_ops._get_lib()
             part = ctypes.c_int(0)
-            worst = max(n * lib.cb_decode_num_splits(n, hkv, d, max_len, ctypes.byref(part))
+            # (a window's partitions are never more)
+            worst = max(n * lib.cb_decode_num_splits(n, hkv, d, max_len, 0, ctypes.byref(part))
                         for n in range(1, cfg.max_batch_size + 1))
             FDIntermTensors().ensure(worst, hq, d, device=k_caches[0].device)
         except Exception as e:                # extension not built / odd config: the op allocates per call instead

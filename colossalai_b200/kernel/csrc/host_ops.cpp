@@ -67,7 +67,7 @@ struct Launchers {
   int (*gemm_rows)(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int, cudaStream_t);
   int (*gemm_rows_gated)(const void*, const void*, void*, int, int, int, int64_t, int64_t, int, int, cudaStream_t);
   int (*embed_rows)(const int64_t*, const void*, void*, int64_t, int64_t, int64_t, cudaStream_t);
-  int (*decode_splits)(int, int, int, int, int*);
+  int (*decode_splits)(int, int, int, int, int, int*);
   int (*decode)(const void*, const void*, const void*, const int*, const int*, void*, float*, float*, int, int, int, int, int, int,
                 int, int, float, const float*, int64_t, int64_t, int, int, cudaStream_t);
   int (*moe_sort)(const int64_t*, int64_t, int, int, int, int*, int*, int*, int64_t*, int*, int64_t*, cudaStream_t);
@@ -299,7 +299,7 @@ Tensor paged_decode(const Tensor& q, const Tensor& kc, const Tensor& vc, const T
   const c10::cuda::CUDAGuard guard(q.device());
   const int64_t n = q.size(0), Hq = q.size(1), D = q.size(2), page = kc.size(1), Hkv = kc.size(2), width = tables.size(1);
   int part = 0;
-  const int64_t splits = L.decode_splits((int)n, (int)Hkv, (int)D, (int)(width * page), &part);
+  const int64_t splits = L.decode_splits((int)n, (int)Hkv, (int)D, (int)(width * page), (int)window, &part);
   const int64_t rows = n * splits * Hq;
   Tensor o = ws_out.has_value() && ws_out->numel() >= rows * D ? *ws_out : Tensor();
   Tensor ml = ws_ml.has_value() && ws_ml->numel() >= rows * 2 ? *ws_ml : Tensor();

@@ -63,17 +63,23 @@ static inline int decode_warps(int kv_heads, int head_dim) {
 }
 struct DecodeCut {
   const int* seq_lens;
-  int capacity, part_len;              // tokens that a table has room for
+  int capacity, part_len, window;      // tokens that a table has room for
 };
 // tokens of a partition: part_len, or, where that is negative, an equal share of the sequence's own, of -part_len at least
 CB_DEVICE int decode_partition(int cached, int splits, int part_len) {
   return part_len > 0 ? part_len : max(-part_len, ((cached + splits - 1) / splits + 15) & ~15);
 }
-// partitions of a sequence that have tokens
+// Of a window (`window_start`: its first token, or 0) the tokens in sight are shared out, from here on; they are all that is read then.  By whole
+// lengths 16 sequences of 32768 tokens with a window of 4096 had work for two of nine partitions: 254 us, cut by what the table holds 140, so 48.
+CB_DEVICE int decode_first(int window_start, int part_len) { return part_len < 0 ? window_start & ~15 : 0; }
+// partitions of a sequence up to the last that has tokens
 CB_DEVICE int decode_used(const DecodeCut& c, int seq, int splits) {
-  const int cached = min(c.seq_lens[seq], c.capacity), part = decode_partition(cached, splits, c.part_len);
+  const int len = c.seq_lens[seq], first = c.window > 0 ? decode_first(max(0, len - c.window), c.part_len) : 0;
+  const int cached = min(len, c.capacity) - first, part = decode_partition(cached, splits, c.part_len);
   return max(0, min(splits, (cached + part - 1) / part));
 }
+// tokens that partitions of a sequence's own length can have to share out, with what is before a window on its first 16
+static inline int decode_in_sight(int capacity, int window) { return window > 0 && window < capacity - 15 ? window + 15 : capacity; }
 
 template <typename T, typename TC>
 __global__ void __launch_bounds__(256) kv_cache_write_kernel(const T* __restrict__ k, const T* __restrict__ v,
@@ -264,9 +270,10 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_kernel(
   // the window start contribute nothing (m = -inf, l = 0) and are skipped by the merge
   const int window_start = window > 0 ? max(0, len - window) : 0;
   const int cached = min(len, max_blocks_per_seq * block_size);                                 // (no pages beyond the table's row)
-  const int part = decode_partition(cached, splits, part_len);
-  const int t0 = max(split * part, window_start);
-  const int t1 = min(cached, split * part + part);
+  const int first = decode_first(window_start, part_len);
+  const int part = decode_partition(cached - first, splits, part_len);
+  const int t0 = max(first + split * part, window_start);
+  const int t1 = min(cached, first + split * part + part);
   const int g0 = set * GH;
   const int ng = min(GH, G - g0);
   const int grp = lane / LPT, sub = lane - grp * LPT;
@@ -480,8 +487,8 @@ template <> CB_DEVICE float2 unpack2<__half>(uint32_t v) { return __half22float2
 // REST: the rows of P V that have no heads take what the rounding of the weights to 16 bits left.  The largest weight of a partition is exact, and
 // sequences that are cut into fewer partitions than of DEC_PART_MIN tokens have fewer exact ones: error against 64 bits, 16 sequences of up to 1024 tokens
 // in bf16, 2.03e-3 in short partitions, 2.06e-3 in long ones, 1.66e-3 with the rest; one of 16000 in fp16 2.55e-4, 2.70e-4 and 2.10e-4.  For calls
-// that are cut by their own lengths where the table has room for more than DEC_PART_MIN tokens a partition; the others' are no longer than they ever were,
-// and 64 sequences of 2048 tokens, cut by their table, would take 79 us with it instead of 77.
+// that are cut by their own lengths where the table has room for more than DEC_PART_MIN tokens a partition, or in a window; the others' are no longer
+// than they ever were, and 64 sequences of 2048 tokens, cut by their table, would take 79 us with it instead of 77.
 template <typename T, int D, bool REST>
 __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
     const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
@@ -504,9 +511,11 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
   const int len = seq_lens[seq];
   const int window_start = window > 0 ? max(0, len - window) : 0;
   const int cached = min(len, max_blocks_per_seq * block_size);                                 // (no pages beyond the table's row)
-  const int part = decode_partition(cached, splits, part_len);
-  const int t0 = max(split * part, window_start);
-  const int t1 = min(cached, split * part + part);
+  // (asked in every call, one sequence of 4097 tokens took 14.4 us instead of 14.0)
+  const int first = REST ? decode_first(window_start, part_len) : 0;
+  const int part = decode_partition(cached - first, splits, part_len);
+  const int t0 = max(first + split * part, window_start);
+  const int t1 = min(cached, first + split * part + part);
   const int row = lane >> 2, quad = lane & 3;   // accumulator layout: head row, column pair inside an 8-wide tile
   const bool row_ok = row < G;                  // rows G..15 of the MMA are padding
   const float scale2 = scale * LOG2E;           // scores in the exp2 domain
@@ -647,7 +656,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
   }
   // ---- this unit's partial result (row sum over the quad first).  (Of a partition behind the sequence's end nobody asks for one where there are
   // many; looked at before the queries are loaded it cost every call .5 us.)
-  if (splits >= DEC_WIDE && split * part >= cached) return;
+  if (splits >= DEC_WIDE && first + split * part >= cached) return;
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
   if (row_ok) {
@@ -843,22 +852,24 @@ int cb_rope_kv_cache_write(void* q, void* k, const void* v, void* k_cache, void*
   return CB_LAUNCH_CHECK();
 }
 
-// partitions of every sequence, and the `part_len` that goes with them (decode_partition).  What a sequence's result is depends on the
-// call's sizes and on its own length, not on the others' lengths.
-int cb_decode_num_splits(int num_seqs, int kv_heads, int head_dim, int max_len, int* part_len_out) {
+// partitions of every sequence, and the `part_len` that goes with them (decode_partition).  window: of the attention, 0 for none.  What a
+// sequence's result is depends on the call's sizes and on its own length, not on the others' lengths.
+int cb_decode_num_splits(int num_seqs, int kv_heads, int head_dim, int max_len, int window, int* part_len_out) {
   *part_len_out = DEC_PART_MIN;
   if (num_seqs <= 0 || kv_heads <= 0) return 1;
-  const int sms = cb_num_sms(), most = (max_len + DEC_PART_MIN - 1) / DEC_PART_MIN;
+  const int sms = cb_num_sms();
   const int warps = decode_warps(kv_heads, head_dim);
   const int fit = 227 * 1024 / (warps * DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * head_dim * 2), per_sm = fit < 8 ? fit : 8;
   const int ctas = num_seqs * ((kv_heads + warps - 1) / warps), one_round = per_sm * sms / ctas, two_rounds = 2 * per_sm * sms / ctas;
   if ((head_dim == 128 || kv_heads <= 4) && head_dim <= 128 && (one_round >= DEC_ROUND_SPLITS || two_rounds > DEC_ROUND_SPLITS)) {
     *part_len_out = -DEC_PART_MIN;
+    const int most = (decode_in_sight(max_len, window) + DEC_PART_MIN - 1) / DEC_PART_MIN;
     const int own = one_round >= DEC_ROUND_SPLITS ? one_round : two_rounds, cap = num_seqs == 1 ? sms / 2 : DEC_MOST_SPLITS;
     const int splits = own < cap ? own : cap;
     return splits < most ? splits : most < 1 ? 1 : most;
   }
   // two rounds of CTAs of eight kv heads, partitions of at least DEC_PART_MIN of the tokens that a table has room for
+  const int most = (max_len + DEC_PART_MIN - 1) / DEC_PART_MIN;
   const int ctas_per_split = num_seqs * ((kv_heads + 7) / 8);
   int splits = (2 * sms + ctas_per_split - 1) / ctas_per_split;
   if (splits > most) splits = most;
@@ -890,14 +901,14 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
   const char* impl_env = getenv("CB200_DECODE");
   const bool use_mma = !(impl_env != nullptr && impl_env[0] == 's') && G <= 8 && (D == 128 || D == 64);
   const int mma_warps = decode_warps(Hkv, D);
-  const DecodeCut cut{seq_lens, max_blocks_per_seq * block_size, part_len};
+  const DecodeCut cut{seq_lens, max_blocks_per_seq * block_size, part_len, window};
   dim3 mma_grid(num_seqs, (Hkv + mma_warps - 1) / mma_warps, splits);
 #define LAUNCH_DEC_MMA(T, DD)                                                                                       \
   {                                                                                                                  \
     constexpr int per_warp = DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * DD * 2;                                           \
     static CbDeviceAttr attr;                                                                                        \
     static CbDeviceAttr attr_rest;                                                                                   \
-    const bool rest = part_len < 0 && cut.capacity > (int64_t)DEC_PART_MIN * splits;                                     \
+    const bool rest = part_len < 0 && (window > 0 || cut.capacity > (int64_t)DEC_PART_MIN * splits);                   \
     auto kern = rest ? paged_decode_mma_kernel<T, DD, true> : paged_decode_mma_kernel<T, DD, false>;                 \
     if (const int e = cb_allow_smem(rest ? attr_rest : attr, kern, (DEC_THREADS / 32) * per_warp)) return e;         \
     if (const int e = cb_launch_early(kern, mma_grid, mma_warps * 32, mma_warps * per_warp, s, \

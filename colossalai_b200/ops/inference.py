@@ -100,7 +100,7 @@ def paged_decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
         lib = _get_lib()
         max_len = block_tables.shape[1] * bs
         part = ctypes.c_int(0)
-        splits = lib.cb_decode_num_splits(n, Hkv, D, max_len, ctypes.byref(part))
+        splits = lib.cb_decode_num_splits(n, Hkv, D, max_len, int(window or 0), ctypes.byref(part))
         out = torch.empty_like(q)
         ws = _decode_workspace(q, n, Hq, splits, D)
         if ws is not None:

@@ -349,6 +349,44 @@ def test_paged_decode_partitions_of_a_length(n, Hq, Hkv, D, room):
     assert torch.equal(iops.paged_decode_attention(q, kc, vc, tables, other)[0], out[0])
 
 
+def _attention_in_64_bits(q, kc, vc, tables, lens, window=0):
+    out = []
+    for i, m in enumerate(lens.tolist()):
+        first = max(0, m - window) if window else 0
+        k, v = (c[tables[i].long()].flatten(0, 1)[first:m].double().repeat_interleave(q.shape[1] // c.shape[2], 1) for c in (kc, vc))
+        w = (torch.einsum("hd,khd->hk", q[i].double(), k) * q.shape[2] ** -0.5).softmax(-1)
+        out.append(torch.einsum("hk,khd->hd", w, v))
+    return torch.stack(out)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,Hq,Hkv,D", [(1, 8, 8, 128), (3, 4, 2, 64), (9, 32, 32, 128), (16, 16, 8, 128), (40, 8, 8, 128), (60, 8, 8, 128)])
+@pytest.mark.parametrize("window", [1, 40, 64, 1000, 4096])
+@pytest.mark.parametrize("capacity", [500, 6000])
+def test_paged_decode_partitions_of_a_window(n, Hq, Hkv, D, window, capacity):
+    """What partitions of a sequence's own length share out are the tokens that a window shows, however many are cached, and no more partitions than
+    without it: the result against 64 bits, with lengths on and beside the window's edges."""
+    import ctypes
+
+    lib, cut = iops._get_lib(), []
+    for room, w in ((capacity, window), (min(capacity, window + 15), 0), (capacity, 0)):
+        part = ctypes.c_int(0)
+        cut.append((lib.cb_decode_num_splits(n, Hkv, D, room, w, ctypes.byref(part)), part.value))
+    assert cut[0][0] <= cut[2][0] and (cut[0] == cut[1] if cut[0][1] < 0 else cut[0] == cut[2])
+    dev, page = "cuda", 16
+    g = torch.Generator(device=dev).manual_seed(n + window)
+    width = (capacity + page - 1) // page
+    kc, vc = (torch.randn(300, page, Hkv, D, device=dev, generator=g).bfloat16() for _ in "kv")
+    tables = torch.randint(0, 300, (n, width), device=dev, generator=g).to(torch.int32)
+    edges = [capacity, capacity - 1, window, window + 1, window + 15, window + 16, window + 17, window // 2 + 1, 1, 17]
+    lens = torch.tensor([min(max(1, edges[i % len(edges)]), capacity) for i in range(n)], device=dev, dtype=torch.int32)
+    q = torch.randn(n, Hq, D, device=dev, generator=g).bfloat16()
+    out = iops.paged_decode_attention(q, kc, vc, tables, lens, window=window)
+    ref = _attention_in_64_bits(q, kc, vc, tables, lens, window)
+    # weights rounded to 16 bits (2^-9 each), the result once more
+    assert ((out.double() - ref).norm(dim=-1) <= 6e-3 * ref.norm(dim=-1)).all()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("n,Hq,Hkv,D,length", [(1, 8, 8, 128, 8000), (4, 16, 4, 64, 7200), (12, 8, 1, 128, 6400), (16, 16, 8, 128, 800),
@@ -364,12 +402,7 @@ def test_paged_decode_weights_with_their_remainders(n, Hq, Hkv, D, length, dtype
     q = torch.randn(n, Hq, D, device=dev, generator=g).to(dtype)
     kc, vc = (torch.randn(n * width, page, Hkv, D, device=dev, generator=g).to(dtype) for _ in "kv")
     out = iops.paged_decode_attention(q, kc, vc, tables, lens)
-    ref = []
-    for i in range(n):
-        k, v = (c[tables[i].long()].flatten(0, 1)[: lens[i]].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
-        w = (torch.einsum("hd,khd->hk", q[i].double(), k) * D ** -0.5).softmax(-1)
-        ref.append(torch.einsum("hk,khd->hd", w, v))
-    ref = torch.stack(ref)
+    ref = _attention_in_64_bits(q, kc, vc, tables, lens)
     # half a unit of the last place; weights, one in all, of values of about one: with twice eight bits and two signs 2^-18 (4e-6), and from scores whose
     # fp32 sums are off by some 2^-17 (8e-6)
     bits = 8 if dtype == torch.bfloat16 else 11
