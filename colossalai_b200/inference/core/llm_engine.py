@@ -162,9 +162,8 @@ class LLMEngine(BaseEngine):
         try:
             lib = infer_ops._get_lib()
             part = ctypes.c_int(0)
-            # (a window's partitions are never more)
-            worst = max(n * lib.cb_decode_num_splits(n, hkv, d, max_len, 0, ctypes.byref(part))
-                        for n in range(1, cfg.max_batch_size + 1))
+            worst = max(n * lib.cb_decode_num_splits(n, hkv, d, max_len, w, ctypes.byref(part))
+                        for n in range(1, cfg.max_batch_size + 1) for w in {0, self.model_config.sliding_window or 0})
             FDIntermTensors().ensure(worst, hq, d, device=k_caches[0].device)
         except Exception as e:                # extension not built / odd config: the op allocates per call instead
             self.logger.warning(f"persistent decode workspace disabled: {e}", ranks=[0])

@@ -49,10 +49,8 @@ constexpr int DEC_MMA_WARPS = 4;
 // many partial results to add up, cost more than they balance, and what a table has room for is often several times what is in it.
 // Two rounds of what the table holds / one of the length, tables just wide enough, us: 16 x 1024 tokens of 32 / 8 heads of 128 22.6 / 18.2, 16 x 8000
 // 86 / 79, 2 x 16000 38.0 / 29.6, 10 x 8000 60.0 / 54.9, 28 x 4000 75.0 / 69.8, 6 x 12000 of 16 / 2 heads of 64 29.1 / 22.4, 60 x 2000 of 16 / 2 heads of 128
-// 37.8 / 31.2, 5 x 8000 of 12 heads 50.5 / 43.9; tables of 8192 tokens of which 500 to 1000 are in use, 16 sequences 40.8 / 17, 28 64 / 21.  More
-// than DEC_MOST_SPLITS partitions cost as many results more than they give CTAs (96: 2 x 6000 21.0 instead of 17.8), but for a sequence alone, which
-// takes half as many as there are SMs (74 and 64: 1 x 4700 14.2 and 14.8, 1 x 8000 18.4 and 19.1, 1 x 30000 41.9 and 41.0; 2 x 4600 18.0 and 16.4, 2 x
-// 9000 25.5 and 22.4).  Where a round is fewer than DEC_ROUND_SPLITS partitions - lengths differ by more than one - two rounds (one / two: 40 x 3000 79.8 / 73.0, 32 x
+// 37.8 / 31.2, 5 x 8000 of 12 heads 50.5 / 43.9; tables of 8192 tokens of which 500 to 1000 are in use, 16 sequences 40.8 / 17, 28 64 / 21.  How
+// many that is at most: decode_most_splits.  Where a round is fewer than DEC_ROUND_SPLITS partitions - lengths differ by more than one - two rounds (one / two: 40 x 3000 79.8 / 73.0, 32 x
 // 4000 79.8 / 76.0), and where that is as few, and for more than four heads of 64, of what the table holds (64 x 2048 76.9, own 80.3; 30 x 4000 of 24 / 8
 // heads of 64 38.6, own 43.4).
 constexpr int DEC_PART_MIN = 64, DEC_ROUND_SPLITS = 5, DEC_MOST_SPLITS = 64;
@@ -80,6 +78,26 @@ CB_DEVICE int decode_used(const DecodeCut& c, int seq, int splits) {
 }
 // tokens that partitions of a sequence's own length can have to share out, with what is before a window on its first 16
 static inline int decode_in_sight(int capacity, int window) { return window > 0 && window < capacity - 15 ? window + 15 : capacity; }
+
+// At most: DEC_MOST_SPLITS, or half as many as there are SMs for a sequence alone, unless few heads walk long.  A warp takes 16 tokens of 128 in
+// 1.0 us, the sum a partition in .07, so one sequence of T tokens is balanced at sqrt(.88 T) partitions (heads of 64: .5 T); no more than two
+// rounds of CTAs of eight heads, nor than most of one round of these - with every place taken they are slower (2 x 16000 tokens of four heads, 100 / 148
+// partitions, 24.5 / 30.2; of eight heads, 64 / 74, 29.7 / 33.5).  us with the usual number / so: 1 x 16000 of one head 24.3 / 21.2, 1 x 128000
+// 118.7 / 52.8, 2 x 16000 of two heads 25.6 / 22.7, 3 x 16000 of four 28.8 / 26.4, 1 x 16000 of eight 27.0 / 24.3, 1 x 128000 137 / 101.
+// Partitions of DEC_PART_MIN tokens where half again as many are enough for that: their weights need no rest (1 x 6000 of one head 14.5 / 14.0).
+// Parts are of whole pairs of tiles, of 64 by fours (4 x 16000 of two heads, parts of 192 / 224 / 256 19.9 / 21.8 / 19.7).
+static inline int decode_most_splits(int num_seqs, int kv_heads, int head_dim, int one_round, int tokens) {
+  const int sms = cb_num_sms(), usual = num_seqs == 1 ? sms / 2 : DEC_MOST_SPLITS, least = (tokens + DEC_PART_MIN - 1) / DEC_PART_MIN;
+  const int rounds = 2 * sms / (num_seqs * ((kv_heads + 7) / 8)), room = one_round * (num_seqs == 1 ? 15 : 18) / 20, most = rounds < room ? rounds : room;
+  const bool wide = head_dim == 128;
+  if (wide && least <= most && 2 * least <= 3 * usual) return least;
+  int many = (int)sqrtf((wide ? .875f : .5f) * tokens);
+  if (many > most) many = most;
+  if (many <= usual) return usual;
+  const int part = wide ? (tokens / many + 16) / 32 * 32 : (tokens / many + 63) / 64 * 64;
+  many = (tokens + part - 1) / part;
+  return many < usual ? usual : many < most ? many : most;
+}
 
 template <typename T, typename TC>
 __global__ void __launch_bounds__(256) kv_cache_write_kernel(const T* __restrict__ k, const T* __restrict__ v,
@@ -864,7 +882,8 @@ int cb_decode_num_splits(int num_seqs, int kv_heads, int head_dim, int max_len, 
   if ((head_dim == 128 || kv_heads <= 4) && head_dim <= 128 && (one_round >= DEC_ROUND_SPLITS || two_rounds > DEC_ROUND_SPLITS)) {
     *part_len_out = -DEC_PART_MIN;
     const int most = (decode_in_sight(max_len, window) + DEC_PART_MIN - 1) / DEC_PART_MIN;
-    const int own = one_round >= DEC_ROUND_SPLITS ? one_round : two_rounds, cap = num_seqs == 1 ? sms / 2 : DEC_MOST_SPLITS;
+    const int own = one_round >= DEC_ROUND_SPLITS ? one_round : two_rounds;
+    const int cap = decode_most_splits(num_seqs, kv_heads, head_dim, one_round, decode_in_sight(max_len, window));
     const int splits = own < cap ? own : cap;
     return splits < most ? splits : most < 1 ? 1 : most;
   }

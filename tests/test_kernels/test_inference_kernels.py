@@ -321,34 +321,6 @@ def test_rotation_with_page_write(heads, kv, D, rot, interleaved, tokens, page, 
     assert torch.equal(pages[0], kw) and torch.equal(pages[1], vw)
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("n,Hq,Hkv,D", [(1, 16, 8, 128), (2, 4, 2, 64), (29, 8, 8, 128), (30, 8, 8, 128), (49, 8, 8, 128), (50, 8, 8, 128), (9, 32, 32, 128), (3, 12, 12, 128),
-                                        (118, 4, 2, 128), (119, 4, 2, 128), (150, 4, 4, 64), (7, 8, 8, 64)])
-@pytest.mark.parametrize("room", [80, 1100, 5000])
-def test_paged_decode_partitions_of_a_length(n, Hq, Hkv, D, room):
-    """Sequences cut by their own length and by what a table has room for, on both sides of the rules between them, in tables that are mostly
-    empty: against the reference, and a sequence's bits do not depend on how long the others are."""
-    dev, page = "cuda", 16
-    g = torch.Generator(device=dev).manual_seed(n + room)
-    width = (room + page - 1) // page
-    lens = torch.randint(1, min(room, 700) + 1, (n,), device=dev, generator=g)
-    edges = torch.tensor([1, 16, 63, 64, 65, room], device=dev)[:n]
-    lens[: len(edges)] = edges.clamp(max=room)
-    most = int(lens.max() + page - 1) // page
-    tables = torch.zeros(n, width, dtype=torch.int32, device=dev)
-    tables[:, :most] = torch.randint(0, 200, (n, most), device=dev, generator=g).to(torch.int32)
-    q = torch.randn(n, Hq, D, device=dev, generator=g).bfloat16()
-    kc, vc = (torch.randn(200, page, Hkv, D, device=dev, generator=g).bfloat16() for _ in "kv")
-    lens = lens.to(torch.int32)
-    out = iops.paged_decode_attention(q, kc, vc, tables, lens)
-    ref = iops.paged_decode_attention_ref(q, kc, vc, tables, lens)
-    # probabilities and results rounded to 8 bits: averages of values of about one
-    torch.testing.assert_close(out.float(), ref.float(), atol=2e-2, rtol=2e-2)
-    other = lens.clone()
-    other[1:] = (lens[1:] // 2).clamp(min=1)
-    assert torch.equal(iops.paged_decode_attention(q, kc, vc, tables, other)[0], out[0])
-
-
 def _attention_in_64_bits(q, kc, vc, tables, lens, window=0):
     out = []
     for i, m in enumerate(lens.tolist()):
@@ -360,19 +332,46 @@ def _attention_in_64_bits(q, kc, vc, tables, lens, window=0):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,Hq,Hkv,D", [(1, 16, 8, 128), (2, 4, 2, 64), (29, 8, 8, 128), (30, 8, 8, 128), (49, 8, 8, 128), (50, 8, 8, 128), (9, 32, 32, 128), (3, 12, 12, 128),
+                                        (118, 4, 2, 128), (119, 4, 2, 128), (150, 4, 4, 64), (7, 8, 8, 64), (1, 4, 1, 128), (3, 4, 4, 128)])
+@pytest.mark.parametrize("room", [80, 1100, 5000, 20000])
+def test_paged_decode_partitions_of_a_length(n, Hq, Hkv, D, room):
+    """Sequences cut by their own length and by what a table has room for, on both sides of the rules between them, in tables as wide as the
+    longest of uneven lengths: against 64 bits, and a sequence's bits do not depend on how long the others are."""
+    dev, page = "cuda", 16
+    g = torch.Generator(device=dev).manual_seed(n + room)
+    width = (room + page - 1) // page
+    lens = torch.randint(1, min(room, 700) + 1, (n,), device=dev, generator=g)
+    edges = torch.tensor([room, room // 2, 65, 64, 63, 16, 1, room - 1], device=dev)[:n]
+    lens[: len(edges)] = edges.clamp(max=room)
+    tables = torch.randint(0, 200, (n, width), device=dev, generator=g).to(torch.int32)
+    q = torch.randn(n, Hq, D, device=dev, generator=g).bfloat16()
+    kc, vc = (torch.randn(200, page, Hkv, D, device=dev, generator=g).bfloat16() for _ in "kv")
+    lens = lens.to(torch.int32)
+    out = iops.paged_decode_attention(q, kc, vc, tables, lens)
+    ref = _attention_in_64_bits(q, kc, vc, tables, lens)
+    # every head of every sequence: weights rounded to 16 bits (2^-9 each), the result once more
+    assert ((out.double() - ref).norm(dim=-1) <= 6e-3 * ref.norm(dim=-1)).all()
+    other = lens.clone()
+    other[1::4] = (lens[1::4] // 2).clamp(min=1)
+    other[3::4] = (lens[3::4] * 2 + 5).clamp(max=room)
+    assert torch.equal(iops.paged_decode_attention(q, kc, vc, tables, other)[0::2], out[0::2])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n,Hq,Hkv,D", [(1, 8, 8, 128), (3, 4, 2, 64), (9, 32, 32, 128), (16, 16, 8, 128), (40, 8, 8, 128), (60, 8, 8, 128)])
 @pytest.mark.parametrize("window", [1, 40, 64, 1000, 4096])
 @pytest.mark.parametrize("capacity", [500, 6000])
 def test_paged_decode_partitions_of_a_window(n, Hq, Hkv, D, window, capacity):
-    """What partitions of a sequence's own length share out are the tokens that a window shows, however many are cached, and no more partitions than
-    without it: the result against 64 bits, with lengths on and beside the window's edges."""
+    """What partitions of a sequence's own length share out are the tokens that a window shows, however many are cached, in as many as a table of
+    that size has: the result against 64 bits, with lengths on and beside the window's edges."""
     import ctypes
 
     lib, cut = iops._get_lib(), []
     for room, w in ((capacity, window), (min(capacity, window + 15), 0), (capacity, 0)):
         part = ctypes.c_int(0)
         cut.append((lib.cb_decode_num_splits(n, Hkv, D, room, w, ctypes.byref(part)), part.value))
-    assert cut[0][0] <= cut[2][0] and (cut[0] == cut[1] if cut[0][1] < 0 else cut[0] == cut[2])
+    assert cut[0] == (cut[1] if cut[0][1] < 0 else cut[2])
     dev, page = "cuda", 16
     g = torch.Generator(device=dev).manual_seed(n + window)
     width = (capacity + page - 1) // page
@@ -390,7 +389,7 @@ def test_paged_decode_partitions_of_a_window(n, Hq, Hkv, D, window, capacity):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("n,Hq,Hkv,D,length", [(1, 8, 8, 128, 8000), (4, 16, 4, 64, 7200), (12, 8, 1, 128, 6400), (16, 16, 8, 128, 800),
-                                                   (4, 8, 8, 128, 2880), (8, 12, 12, 128, 960), (1, 8, 8, 128, 5600)])
+                                                   (4, 8, 8, 128, 2880), (8, 12, 12, 128, 960), (1, 8, 8, 128, 7680)])
 def test_paged_decode_weights_with_their_remainders(n, Hq, Hkv, D, length, dtype):
     """Sequences in partitions of more than 64 tokens (80 and 96 among them): the weights are not rounded to 16 bits, so what differs from 64 bits is the result's own rounding, and an
     infinite value is infinite in the result."""
