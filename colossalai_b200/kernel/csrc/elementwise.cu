@@ -366,8 +366,8 @@ int cb_rope_pages(const void* src, void* dst, const int64_t* pos, const float* c
                   int64_t src_stride, int width, int n_rot_heads, int kv_heads, int D, int rot_dim, int interleaved, int dtype,
                   void* k_pages, void* v_pages, const int* tables, const int* token_seq, const int* token_pos, int page, int table_width,
                   cudaStream_t s) {
-  if (width != (n_rot_heads + kv_heads) * D || (dtype != CB_BF16 && dtype != CB_F16)) return (int)cudaErrorInvalidValue;
-  CB_DISPATCH_FLOAT(dtype, T, {
+  if (width != (n_rot_heads + kv_heads) * D) return (int)cudaErrorInvalidValue;
+  CB_DISPATCH_HALF(dtype, T, {
     const RopePages<T, true> pages{(T*)k_pages, (T*)v_pages, tables, token_seq, token_pos, page, table_width, kv_heads * D,
                              (n_rot_heads - kv_heads) * D};
     return (launch_rope<T, true>((const T*)src, (T*)dst, pos, cos_c, sin_c, tokens, src_stride, width, n_rot_heads, D, rot_dim, 1.f,
