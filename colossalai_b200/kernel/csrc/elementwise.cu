@@ -112,8 +112,13 @@ __global__ void __launch_bounds__(GLU_THREADS) glu_bwd_kernel(const T* __restric
 // through - so that no thread's share differs from another's.  Rows of at most ROPE_NARROW items share a block of ROPE_BLOCK
 // threads, one item each: 300000 rows of 48 bf16 forward and
 // backward: a block each 313 us, together 38.  A form of its own: with the stride and the row worked out at run time 8192 rows of 6144
-// took 40 us a direction instead of 35.  Wide rows: ROPE_ITEMS items a thread, all their loads before the first store (one item, in
-// as many more threads, 34.5 us, two 33.0, three 32.7, four 33.2; both directions 69.3 -> 65.7); where a few tokens leave SMs idle, one.
+// took 40 us a direction instead of 35.  Wide rows of 16 bits in calls of
+// several rounds of blocks: ROPE_ITEMS items a thread, all their loads before the first store (8192 rows of 6144: one item, in as many more
+// threads, 34.5 us, two 33.0, three 32.7, four 33.2).  In one round of blocks a block more is worth more than what one has on its way, and the narrower
+// the row the longer: three / one, us, 384 items 1000 tokens 5.84 / 5.18, 2500 1.5 % slower, 4000 16.9 / 17.6, 12000 44.7 / 49.0; 288 items 3000
+// tokens 3 % slower, 4000 3 % faster; 144 items 4000 8.06 / 7.06, 8000 13.8 / 13.7, 30000 4 % faster; 160 items of which 144 are rotated, so that a warp
+// has both kinds, 8000 6 % slower, 20000 3 %; 640 items, which a block of one item each does not hold, 600 4 % faster, 4000 28.3 / 30.7.  32 bits: 2 %
+// slower up to 384 items at any number of tokens, at 768 1 % faster.
 constexpr int ROPE_NARROW = 64, ROPE_BLOCK = 256, ROPE_ITEMS = 3;
 // Where a step's keys and values go beside dst (PAGES): rows of kv_width elements of pages of `page` tokens, found through the page tables.
 // A decode step then has a launch a layer less; with the gated unit's too (gemm_rows_tcgen05.cu) 16 sequences, 4 layers of 4096 x 14336,
@@ -125,13 +130,15 @@ template <typename T, bool PAGES> struct RopePages {
   int k_at;                            // first element of the keys in a row; the values follow them
 };
 template <typename T> struct RopePages<T, false> {};
-template <typename T, bool VEC_TABLE, bool NARROW, bool PAGES>
-__global__ void __launch_bounds__(NARROW ? ROPE_BLOCK : 512) rope_kernel(const T* __restrict__ src, T* __restrict__ dst,
+enum { ROPE_SHARED, ROPE_ONE, ROPE_SEVERAL };             // narrow rows that share a block; of a row with its own, items of a thread
+template <typename T, bool VEC_TABLE, int FORM, bool PAGES>
+__global__ void __launch_bounds__(FORM == ROPE_SHARED ? ROPE_BLOCK : 512) rope_kernel(const T* __restrict__ src, T* __restrict__ dst,
                                                    const int64_t* __restrict__ pos, const float* __restrict__ cos_c,
                                                    const float* __restrict__ sin_c, int64_t tokens, int per_block,
                                                    int64_t src_stride, int width, int n_rot_heads, int D, int rot_dim,
                                                    float sign, int interleaved, RopePages<T, PAGES> pages) {
-  constexpr int VEC = Vec16<T>::N, UN = NARROW ? 1 : ROPE_ITEMS;
+  constexpr bool NARROW = FORM == ROPE_SHARED;
+  constexpr int VEC = Vec16<T>::N, UN = FORM == ROPE_SEVERAL ? ROPE_ITEMS : 1;
   cb_early_start();
   const int half = rot_dim / 2;
   const int vec_per_head = half / VEC;                       // rotated items of a head
@@ -291,11 +298,15 @@ static int launch_rope(const T* src, T* dst, const int64_t* pos, const float* co
   // (the same count as in the kernel: rotated pairs, and vectors that pass through two by two)
   const int rotated = n_rot_heads * (rot_dim / 2 / Vec16<T>::N), items = rotated + (width / Vec16<T>::N - 2 * rotated + 1) / 2;
   const int per_block = items > 0 && items <= ROPE_NARROW ? ROPE_BLOCK / items : 1;
-  const int share = tokens >= 4 * cb_num_sms() ? (items + ROPE_ITEMS - 1) / ROPE_ITEMS : items;      // of the row's threads
-  const int block = per_block > 1 ? ROPE_BLOCK : share >= 512 ? 512 : (share + 31) / 32 * 32;
+  const int third = ((items + ROPE_ITEMS - 1) / ROPE_ITEMS + 31) / 32 * 32;
+  const int rounds = items > 512 ? 0 : third >= 96 ? 2560 : rotated % 32 == 0 ? 4096 : 8192;
+  const bool several = (sizeof(T) == 2 || items > 512) && tokens >= 4 * cb_num_sms() && tokens * third >= (int64_t)rounds * cb_num_sms();
+  const int share = several ? third : (items + 31) / 32 * 32;
+  const int block = per_block > 1 ? ROPE_BLOCK : share >= 512 ? 512 : share;
   const unsigned grid = (unsigned)((tokens + per_block - 1) / per_block);
-  auto kern = per_block > 1 ? (vec_table ? rope_kernel<T, true, true, PAGES> : rope_kernel<T, false, true, PAGES>)
-                            : (vec_table ? rope_kernel<T, true, false, PAGES> : rope_kernel<T, false, false, PAGES>);
+  auto kern = per_block > 1 ? (vec_table ? rope_kernel<T, true, ROPE_SHARED, PAGES> : rope_kernel<T, false, ROPE_SHARED, PAGES>)
+              : several     ? (vec_table ? rope_kernel<T, true, ROPE_SEVERAL, PAGES> : rope_kernel<T, false, ROPE_SEVERAL, PAGES>)
+                            : (vec_table ? rope_kernel<T, true, ROPE_ONE, PAGES> : rope_kernel<T, false, ROPE_ONE, PAGES>);
   return cb_launch_early(kern, grid, block, 0, s, src, dst, pos, cos_c, sin_c, tokens, per_block, src_stride, width, n_rot_heads, D,
                          rot_dim, sign, interleaved, pages);
 }

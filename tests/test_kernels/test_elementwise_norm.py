@@ -365,10 +365,11 @@ def test_glu_of_narrow_rows(dtype, vecs, rows, limit):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("hq,hkv,D,rot,interleaved", [(32, 8, 128, 128, False), (33, 3, 96, 64, False), (7, 1, 128, 64, True), (64, 8, 256, 64, False)])
-def test_rope_of_many_rows(dtype, hq, hkv, D, rot, interleaved):
+@pytest.mark.parametrize("per_sm", [5, 30])
+def test_rope_of_many_rows(dtype, hq, hkv, D, rot, interleaved, per_sm):
     """A thread's several items in calls of many tokens: the bits of the same rows a few at a time, with items that are no multiple of what
     a thread or a block takes."""
-    T = 5 * torch.cuda.get_device_properties(0).multi_processor_count
+    T = per_sm * torch.cuda.get_device_properties(0).multi_processor_count
     g = torch.Generator(device="cuda").manual_seed(hq)
     x = torch.randn(T, (hq + 2 * hkv) * D, device="cuda", generator=g).to(dtype)
     pos = torch.randint(0, 64, (T,), device="cuda", generator=g)
