@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(GLU_THREADS) glu_bwd_kernel(const T* __restric
 // threads, 34.5 us, two 33.0, three 32.7, four 33.2).  In one round of blocks a block more is worth more than what one has on its way, and the narrower
 // the row the longer: three / one, us, 384 items 1000 tokens 5.84 / 5.18, 2500 1.5 % slower, 4000 16.9 / 17.6, 12000 44.7 / 49.0; 288 items 3000
 // tokens 3 % slower, 4000 3 % faster; 144 items 4000 8.06 / 7.06, 8000 13.8 / 13.7, 30000 4 % faster; 160 items of which 144 are rotated, so that a warp
-// has both kinds, 8000 6 % slower, 20000 3 %; 640 items, which a block of one item each does not hold, 600 4 % faster, 4000 28.3 / 30.7.  32 bits: 2 %
+// has both kinds, 8000 6 % slower, 20000 3 %; 640 items, which a block does not hold one each, 600 4 % faster, 4000 28.3 / 30.7 (fewer: 512 threads).  32 bits: 2 %
 // slower up to 384 items at any number of tokens, at 768 1 % faster.
 constexpr int ROPE_NARROW = 64, ROPE_BLOCK = 256, ROPE_ITEMS = 3;
 // Where a step's keys and values go beside dst (PAGES): rows of kv_width elements of pages of `page` tokens, found through the page tables.
@@ -305,8 +305,8 @@ static int launch_rope(const T* src, T* dst, const int64_t* pos, const float* co
   const int block = per_block > 1 ? ROPE_BLOCK : share >= 512 ? 512 : share;
   const unsigned grid = (unsigned)((tokens + per_block - 1) / per_block);
   auto kern = per_block > 1 ? (vec_table ? rope_kernel<T, true, ROPE_SHARED, PAGES> : rope_kernel<T, false, ROPE_SHARED, PAGES>)
-              : several     ? (vec_table ? rope_kernel<T, true, ROPE_SEVERAL, PAGES> : rope_kernel<T, false, ROPE_SEVERAL, PAGES>)
-                            : (vec_table ? rope_kernel<T, true, ROPE_ONE, PAGES> : rope_kernel<T, false, ROPE_ONE, PAGES>);
+              : block < items ? (vec_table ? rope_kernel<T, true, ROPE_SEVERAL, PAGES> : rope_kernel<T, false, ROPE_SEVERAL, PAGES>)
+                              : (vec_table ? rope_kernel<T, true, ROPE_ONE, PAGES> : rope_kernel<T, false, ROPE_ONE, PAGES>);
   return cb_launch_early(kern, grid, block, 0, s, src, dst, pos, cos_c, sin_c, tokens, per_block, src_stride, width, n_rot_heads, D,
                          rot_dim, sign, interleaved, pages);
 }
