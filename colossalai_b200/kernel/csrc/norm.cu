@@ -10,8 +10,10 @@
 constexpr int MAX_ITERS_LIMIT = 4;
 
 // A block takes ROWS neighbouring rows, loaded and summed together: two wide ones in calls that fill the SMs several times over (8192 x 4096
-// bf16 with a residual 43.7 -> 42.9 us, 3001 x 5120 21.7 -> 20.8, 5000 x 4096 fp32 54.5 -> 52.3; 8192 x 2048 22.3 and 22.4), else one.
-// Bound: HBM, two rows in and two out.
+// bf16 with a residual 43.7 -> 42.9 us, 3001 x 5120 21.7 -> 20.8, 5000 x 4096 fp32 54.5 -> 52.3; 8192 x 2048 22.3 and 22.4), else one.  With a
+// residual, blocks of 512 threads and 32-bit rows fill the SMs later (two / one: 1200 x 4096 bf16 7.3 / 6.8 us, 1300 7 % slower, 1800 2 % faster; 1200 x
+// 4096 fp32 6 % slower, 2100 1.5 %, 3200 1 % faster, 8192 82.6 / 86.8), and 32-bit rows of less than 768 threads gain nothing (2048 wide 2 to 11 %
+// slower).  Bound: HBM, two rows in and two out.
 constexpr int NORM_ROWS = 2;
 template <typename T, bool HAS_RES, int MAX_ITERS, int ROWS>
 __global__ void __launch_bounds__(1024) rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ res_in,
@@ -339,7 +341,9 @@ int cb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, void* y, vo
     const int iters = pick_iters(H, Vec16<T>::N, block);
     CB_DISPATCH_ITERS(iters, IT, {
       constexpr int R = IT == 1 ? NORM_ROWS : 1;
-      const bool several = block >= 512 && rows >= 8 * cb_num_sms();
+      const bool wide_sums = res_in && sizeof(T) == 4;
+      const int least = wide_sums ? 16 : res_in && block == 512 ? 12 : 8;
+      const bool several = block >= (wide_sums ? 768 : 512) && rows >= least * cb_num_sms();
       auto kernel = several ? (res_in ? rmsnorm_fwd_kernel<T, true, IT, R> : rmsnorm_fwd_kernel<T, false, IT, R>)
                             : (res_in ? rmsnorm_fwd_kernel<T, true, IT, 1> : rmsnorm_fwd_kernel<T, false, IT, 1>);
       return cb_launch_early(kernel, several ? (rows + R - 1) / R : rows, block, 0, stream, (const T*)x, (const T*)res_in, (const T*)w, (T*)y,

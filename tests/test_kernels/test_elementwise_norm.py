@@ -382,9 +382,10 @@ def test_rope_of_many_rows(dtype, hq, hkv, D, rot, interleaved, per_sm):
 @pytest.mark.parametrize("H", [64, 4096, 8200])
 @pytest.mark.parametrize("odd", [0, 1])
 @pytest.mark.parametrize("with_res", [False, True])
-def test_rmsnorm_of_many_rows(dtype, H, odd, with_res):
+@pytest.mark.parametrize("per_sm", [8, 17])
+def test_rmsnorm_of_many_rows(dtype, H, odd, with_res, per_sm):
     """Two rows a block in calls of many rows, the last block's second one missing: the bits of the same rows a few at a time."""
-    rows = 8 * torch.cuda.get_device_properties(0).multi_processor_count + 2 + odd
+    rows = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + 2 + odd
     g = torch.Generator(device="cuda").manual_seed(H)
     x, r = (torch.randn(rows, H, device="cuda", generator=g).to(dtype) for _ in "xr")
     w = torch.randn(H, device="cuda", generator=g).to(dtype)
