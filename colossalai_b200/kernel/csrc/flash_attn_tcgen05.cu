@@ -24,8 +24,8 @@
 // issuer 289, with output warps of their own 256, and 263 with the first reference from both halves of a key tile; five documents of
 // 8192 tokens together 181 -> 156; sixteen of 16384, heads of 64, 223 -> 191.  Two threads per row (16 softmax warps) were 5 - 10 %
 // slower than one.  The two tiles' exponentials in turn (`take_turn`): sixteen prompts of 16384 tokens, heads of 64, 188 -> 171 us, two
-// of 8192 920 -> 765; heads of 128, one call after the other, 2 x 4096 tokens 321 -> 281, five documents of 8192 163 -> 153, 24 of 8192 in 64 heads 164 ->
-// 166.  Taken back since: a quarter or an eighth of the exponentials as polynomials of degree 5 (765 -> 840), the next step's scores
+// of 8192 920 -> 765; heads of 128, one call after the other, 2 x 4096 tokens 321 -> 281, five documents of 8192 163 -> 153; short walks take them
+// together (launch_flash_fwd).  Taken back since: a quarter or an eighth of the exponentials as polynomials of degree 5 (765 -> 840), the next step's scores
 // fetched under the exponentials (997), turns only in units of 8 steps and more (heads of 128: 281 -> 304).
 // TMEM map (512 columns): [0,128) S_0, [128,256) S_1, then O_0, O_1, D wide each; P_t of a half overwrites the first 32 columns of
 // that half of S_t once its scores are in registers.
@@ -248,7 +248,8 @@ struct FaUnit {
   int live, index, q_start, k_start, len_q, len_k, head0;
 };
 
-template <int D, bool EXTRA, bool BF16>
+// TURNS: the exponentials of a unit's two tiles in turn (`take_turn`)
+template <int D, bool EXTRA, bool BF16, bool TURNS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const FaParams p) {
@@ -593,17 +594,19 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     uint64_t* const mine = &turn[4 * t + quarter];
     uint64_t* const theirs = &turn[4 * (t ^ 1) + quarter];
     auto take_turn = [&]() -> bool {
+      if (!TURNS) return true;
       const bool here = __all_sync(0xffffffffu, wait_or_abort(mine, turns & 1, abort_flag)) != 0;
       turns ^= 1;
       return here;
     };
     auto pass_turn = [&]() {
+      if (!TURNS) return;
       __syncwarp();
       if (lane == 0) mbar_arrive(theirs);
     };
     bool ok = true;
     while (ok && next_unit()) {
-      const int n_steps = steps_of(t), turns_of_unit = max(n_steps, steps_of(t ^ 1));
+      const int n_steps = steps_of(t), turns_of_unit = TURNS ? max(n_steps, steps_of(t ^ 1)) : n_steps;
       if (n_steps == 0) {
         for (int j = 0; j < turns_of_unit && ok; ++j) { ok = take_turn(); pass_turn(); }
         continue;
@@ -1189,11 +1192,12 @@ int launch_flash_fwd_tile_kernel(dim3 grid, const CUtensorMap& tq, const CUtenso
 
 template <int D, bool EXTRA, bool BF16>
 int launch_flash_fwd_kernel(dim3 grid, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaParams& p,
-                            cudaStream_t stream) {
+                            bool turns, cudaStream_t stream) {
   using C = FaCfg<D>;
-  static CbDeviceAttr attr;
-  if (const int e = cb_allow_smem(attr, flash_fwd_kernel<D, EXTRA, BF16>, C::SMEM_BYTES)) return e;
-  flash_fwd_kernel<D, EXTRA, BF16><<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  static CbDeviceAttr attr[2];
+  auto kern = turns ? flash_fwd_kernel<D, EXTRA, BF16, true> : flash_fwd_kernel<D, EXTRA, BF16, false>;
+  if (const int e = cb_allow_smem(attr[turns], kern, C::SMEM_BYTES)) return e;
+  kern<<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
 
@@ -1244,12 +1248,19 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* out, flo
   p.idesc_qk = make_idesc_f16(BLOCK_Q, HALF_KV, bf16 ? 1 : 0, 0, 0);
   const long long most = (cu_seqlens ? total_tokens / per + batch : (long long)p.seq_units * batch) * p.head_units;
   if (most > (1ll << 30)) return (int)cudaErrorInvalidValue;
+  // In turn the tile that is ahead waits for the other: in short walks, and where the two tiles of a causal unit walk differently, for nothing.  Together / in
+  // turn, us: heads of 64, units of two tiles of a head, 32 x 256 tokens of 40 / 8 heads 67 / 73, 16 x 384 65 / 70, 20 x 492 98 / 102, 10 x 768 the same,
+  // 8 x 1000 7 % faster in turn; units of two heads 40 x 200 of 64 / 8 heads 118 / 121, 8 x 200 3 % faster in turn, 20 x 492 2 %, 8 x 1000 8 %.  Heads of
+  // 128: 64 x 128 of 40 / 8 112 / 117, 16 x 384 77 / 78, 3 x 768 1 % faster in turn, 4 x 2000 of 32 / 8 5 %.  A template: as a branch between the
+  // exponentials either form took what the slower one does, and long walks up to 12 % more.
+  const long long walk = cu_seqlens ? total_tokens / (batch > 0 ? batch : 1) : seqlen_k;
+  const bool turns = walk >= 704 || ((p.pair_heads || !causal) && (walk >= 320 || most <= 5 * cb_num_sms()));
   const dim3 grid((unsigned)(most < cb_num_sms() ? most : cb_num_sms()));
   if (window > 0 || alibi != nullptr)
-    return bf16 ? launch_flash_fwd_kernel<D, true, true>(grid, tq, tk, tv, p, stream)
-                : launch_flash_fwd_kernel<D, true, false>(grid, tq, tk, tv, p, stream);
-  return bf16 ? launch_flash_fwd_kernel<D, false, true>(grid, tq, tk, tv, p, stream)
-              : launch_flash_fwd_kernel<D, false, false>(grid, tq, tk, tv, p, stream);
+    return bf16 ? launch_flash_fwd_kernel<D, true, true>(grid, tq, tk, tv, p, turns, stream)
+                : launch_flash_fwd_kernel<D, true, false>(grid, tq, tk, tv, p, turns, stream);
+  return bf16 ? launch_flash_fwd_kernel<D, false, true>(grid, tq, tk, tv, p, turns, stream)
+              : launch_flash_fwd_kernel<D, false, false>(grid, tq, tk, tv, p, turns, stream);
 }
 
 

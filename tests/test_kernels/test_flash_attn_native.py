@@ -358,6 +358,27 @@ def test_packed_forward_by_number_of_tiles(D, Hq, Hkv, lens, mask):
 
 
 @pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Hq,Hkv", [(40, 8), (32, 8)])
+@pytest.mark.parametrize("lens", [[600] * 6, [250] * 30, [130, 1, 300, 257, 128] * 6])
+@pytest.mark.parametrize("window", [0, 100])
+def test_forward_tiles_in_turn_and_together(D, Hq, Hkv, lens, window):
+    """The two tiles' exponentials in turn (long walks on average) and together: a sequence's bits are the same, whatever the batch has beside it."""
+    from colossalai_b200.ops import flash_attn_native as fa
+
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    T, n = sum(lens) + 40000, sum(lens)
+    q, k, v = (torch.randn(T, h, D, device="cuda", generator=g).bfloat16() for h in (Hq, Hkv, Hkv))
+    few, many = (torch.tensor([0] + x, device="cuda").cumsum(0).to(torch.int32) for x in (lens, lens + [40000]))
+    assert n // len(lens) < 704 <= T // (len(lens) + 1)                     # (600 tokens of paired heads are in turn both times)
+    if window:
+        a, b = fa.flash_prefill(q[:n], k[:n], v[:n], few, None, window=window), fa.flash_prefill(q, k, v, many, None, window=window)
+    else:
+        (a, lse_a), (b, lse_b) = fa.flash_fwd(q[:n], k[:n], v[:n], 1, True, None, cu_seqlens=few), fa.flash_fwd(q, k, v, 1, True, None, cu_seqlens=many)
+        assert torch.equal(lse_a, lse_b[:n])
+    assert torch.equal(a, b[:n])
+
+
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("Hq,Hkv", [(150, 50), (200, 50)])
 @pytest.mark.parametrize("lens", [[63, 64, 65, 191], [192, 193, 449, 321]])
 @pytest.mark.parametrize("causal", [True, False])
