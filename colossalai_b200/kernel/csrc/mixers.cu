@@ -313,7 +313,6 @@ struct ScanWork {
   float *q, *k, *g, *beta, *v;         // [T, qk_heads, DK] x2, [T, heads, DK], [T, heads], [T, heads, VP]
   float* gw;                           // gated mode: [T, heads, 4] = decay, write strength, read-out factor, unused
   int DK, VP;
-  int vectors;                         // a lane's columns of the state may be read and written as one vector
 };
 
 CB_DEVICE void cp_async16f(void* smem_dst, const void* gmem_src) {
@@ -651,7 +650,7 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
   const int dim = p.dim, vdim = p.vdim;
   const int r0 = part * RP, r0p = part * RPP;
   float* Sg = p.state + ((int64_t)p.slots[s] * p.heads + h) * dim * vdim;
-  const bool vec = w.vectors && j0 < vdim;                     // all of the lane's columns, aligned
+  const bool vec = vdim % CPL == 0 && j0 < vdim;               // all of the lane's columns, aligned
   const bool carried = p.ctx_len[s] > 0;
   // Pairs of neighbouring ROWS share an instruction: q, k and the decays arrive from shared memory as such pairs, and only the
   // token's CPL values are duplicated.
@@ -884,9 +883,7 @@ template <int DK, int MODE, bool SHORT, int CPL = SCAN_CPL> int launch_scan_dk(c
   auto kern = state_scan_kernel<DK, MODE, SHORT, CPL>;
   static CbDeviceAttr attr;
   if (const int e = cb_allow_smem(attr, kern, smem, true)) return e;
-  ScanWork v = w;                      // (asked of the address in the kernel, eight sequences of 12000 tokens took 1.4 % more)
-  v.vectors = p.vdim % CPL == 0 && (uintptr_t)p.state % (CPL * sizeof(float)) == 0;
-  kern<<<p.heads * (w.VP / Tile::COLS) * nseq, Tile::THREADS, smem, st>>>(p, v, nseq, cb_num_sms());
+  kern<<<p.heads * (w.VP / Tile::COLS) * nseq, Tile::THREADS, smem, st>>>(p, w, nseq, cb_num_sms());
   return CB_LAUNCH_CHECK();
 }
 

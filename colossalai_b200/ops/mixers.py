@@ -294,6 +294,11 @@ def _scan_native(mode, q, k, v, araw, braw, head_decay, a_log, dt_bias, state, m
     for t in (q, k, v):
         assert t.stride(1) == 1
     assert state.dtype == torch.float32 and state.is_contiguous()
+    slots, home = meta.slots, None
+    if state.data_ptr() % 16 and vdim % 2 == 0:            # its rows are read and written in vectors: the step's slots, elsewhere
+        home = state, state_n, state_m
+        state, state_n, state_m = (None if t is None else t.index_select(0, slots) for t in home)
+        slots = torch.arange(meta.nseq, dtype=torch.int32, device=q.device)
     ld = lambda t: _i64(0 if t is None else t.stride(0))
     lib = _get_lib()
     # fp32 rows the elementwise prepare kernel writes and the recurrence streams through shared memory
@@ -302,11 +307,15 @@ def _scan_native(mode, q, k, v, araw, braw, head_decay, a_log, dt_bias, state, m
         mode, loader.ptr(q), ld(q), loader.ptr(k), ld(k), loader.ptr(v), ld(v), loader.ptr(araw), ld(araw),
         loader.ptr(braw), ld(braw), loader.ptr(head_decay), loader.ptr(a_log), loader.ptr(dt_bias), loader.ptr(state),
         loader.ptr(out), loader.ptr(work), _i64(T), loader.ptr(meta.cu_q), loader.ptr(meta.ctx_len),
-        loader.ptr(meta.slots), meta.nseq, meta.max_q, heads, qk_heads, dim, vdim, int(act_silu), int(unit_qk), _f(unit_eps),
+        loader.ptr(slots), meta.nseq, meta.max_q, heads, qk_heads, dim, vdim, int(act_silu), int(unit_qk), _f(unit_eps),
         _f(q_scale), _f(k_scale), loader.ptr(rot_table), int(rot_dims if rot_table is not None else 0),
         loader.ptr(meta.token_pos), int(gate_kind), _f(gate_cap), loader.ptr(state_n), loader.ptr(state_m), _f(tau),
         code(q.dtype), loader.stream_ptr()), "state_scan")
     loader.launch_counter.add("state_scan", 3 if gate_kind == 2 else 2)
+    if home is not None:
+        for t, done in zip(home, (state, state_n, state_m)):
+            if t is not None:
+                t.index_copy_(0, meta.slots.long(), done)
     return out
 
 

@@ -215,9 +215,16 @@ def test_decay_scan_of_a_state_at_any_address(H, d, dv, lens, offset):
     moved = buffer[offset: offset + state.numel()].view_as(state)
     moved.copy_(state)
     assert moved.data_ptr() % 16 == 4 * offset % 16
-    meta = M.RaggedMeta.build(lens, [5] * n, list(range(n)), dev)
+    meta = M.RaggedMeta.build(lens, [5] * n, list(range(n))[::-1], dev)
     out = [M.state_scan_decay(q, k, v, head, s, meta, H, d, dv) for s in (state, moved)]
     assert torch.equal(*out) and torch.equal(state, moved)
+    gates, bias = torch.randn(sum(lens), 2 * H, generator=g).to(dev), torch.randn(2 * H, generator=g).to(dev)
+    norm, top = torch.rand(n, H, d, generator=g).to(dev), torch.rand(n, H, generator=g).to(dev)
+    out = []
+    for s in (state, moved):                    # (a memory with a normaliser of its own)
+        beside = norm.clone(), top.clone()
+        out.append((M.state_scan_mlstm(q, k, v, gates, bias, 15.0, s, *beside, meta, H, d, dv, 0.5), *beside))
+    assert all(torch.equal(a, b) for a, b in zip(*out)) and torch.equal(state, moved)
     assert (buffer[:offset] == 7).all() and (buffer[offset + state.numel():] == 7).all()
 
 
