@@ -313,6 +313,7 @@ struct ScanWork {
   float *q, *k, *g, *beta, *v;         // [T, qk_heads, DK] x2, [T, heads, DK], [T, heads], [T, heads, VP]
   float* gw;                           // gated mode: [T, heads, 4] = decay, write strength, read-out factor, unused
   int DK, VP;
+  int turned;                          // decay mode, long portions: every second row of CTAs the other way round (scan_turned)
 };
 
 CB_DEVICE void cp_async16f(void* smem_dst, const void* gmem_src) {
@@ -594,12 +595,14 @@ CB_DEVICE ScanTwo mul2(ScanTwo a, ScanTwo b) { return ScanTwo{__fmul_rn(a.a, b.a
 
 // The sequence and the unit of it (head and block of columns; `units` per sequence) that a CTA walks.  A unit takes as long as
 // its sequence, and what a step takes is the SM with the most tokens.  Up to 32 sequences are dealt out by length, longest first; where all
-// units are resident at once (`at_once`), every second row of one CTA per SM the other way round, and a row that does not fill lands on the
-// SMs that drew short ones before.  Where they are not, the rest goes to the SMs that are done first, and rows all the same way are better: 12000 tokens of 16
-// heads x 128 x 128 in eight sequences, three units an SM, five draws of lengths, 695 722 702 742 679 us turned round, 661 673 704 667 636 so; in five (all
-// at once) 765 and 814 turned round, 808 and 816 so, in 14 of 9000 with 8 heads (448 units for 444 places) 265 and 270.  (Dealing the units to SMs by their tokens beforehand, 750 - 780: a grid's CTAs do not
-// land where their number says.)  More sequences are many more units than fit: they come in order.
-CB_DEVICE void scan_unit(const ScanParams& p, int nseq, int units, int sms, bool at_once, int& s, int& unit) {
+// units are resident at once, or one sequence is twice as long as they are on average (`turned`), every second row of one CTA per SM the other way
+// round, and a row that does not fill lands on the SMs that drew short ones before.  Else the rest goes to the SMs that are done first, and rows all the same way
+// are better: 12000 tokens of 16 heads x 128 x 128 in eight sequences, three units an SM, five draws of lengths, 695 722 702 742 679 us turned round, 661
+// 673 704 667 636 so; in five (all at once) 765 and 814 turned round, 808 and 816 so, in 14 of 9000 with 8 heads (448 units for 444 places) 265 and 270; one of
+// 3000 and seven of 500, 32 heads, 644 and 764, two of 4000 and ten of 300, 16 heads, 676 and 941, eight of at most 1.7 times their average 632 - 640 and
+// 629 - 635.  (Dealing the units to SMs by their tokens beforehand, 750 - 780: a grid's CTAs do not land where their number says.)  More sequences are many
+// more units than fit: they come in order.
+CB_DEVICE void scan_unit(const ScanParams& p, int nseq, int units, int sms, bool turned, int& s, int& unit) {
   int rank = blockIdx.x;
   if (nseq == 1 || nseq > 32) {
     s = rank / units;
@@ -607,7 +610,7 @@ CB_DEVICE void scan_unit(const ScanParams& p, int nseq, int units, int sms, bool
     return;
   }
   const int row = rank / sms, width = min(sms, (int)gridDim.x - row * sms);
-  if (at_once && !(row & 1)) rank = row * sms + width - 1 - (rank - row * sms);
+  if (turned && !(row & 1)) rank = row * sms + width - 1 - (rank - row * sms);
   const int lane = threadIdx.x & 31, want = rank / units;
   unit = rank - want * units;
   const int len = lane < nseq ? p.cu_q[lane + 1] - p.cu_q[lane] : -1;
@@ -637,9 +640,7 @@ state_scan_kernel(ScanParams p, ScanWork w, int nseq, int sms) {
   extern __shared__ __align__(16) float scan_smem[];
   const int vblocks = w.VP / COLS;
   int s, unit;
-  // (only the long decay form's BLOCKS are all that an SM holds; a few units more than fit are as if they fitted)
-  const bool at_once = MODE != SCAN_DECAY || SHORT || DK > 128 || 8 * (int)gridDim.x <= 9 * sms * Tile::BLOCKS;
-  scan_unit(p, nseq, p.heads * vblocks, sms, at_once, s, unit);
+  scan_unit(p, nseq, p.heads * vblocks, sms, MODE != SCAN_DECAY || SHORT || DK > 128 || w.turned, s, unit);
   const int h = unit / vblocks, vb = unit % vblocks;
   const int t0 = p.cu_q[s], t1 = p.cu_q[s + 1];
   if (t0 >= t1) return;
@@ -883,7 +884,10 @@ template <int DK, int MODE, bool SHORT, int CPL = SCAN_CPL> int launch_scan_dk(c
   auto kern = state_scan_kernel<DK, MODE, SHORT, CPL>;
   static CbDeviceAttr attr;
   if (const int e = cb_allow_smem(attr, kern, smem, true)) return e;
-  kern<<<p.heads * (w.VP / Tile::COLS) * nseq, Tile::THREADS, smem, st>>>(p, w, nseq, cb_num_sms());
+  const int grid = p.heads * (w.VP / Tile::COLS) * nseq;
+  ScanWork v = w;
+  v.turned = 8 * grid <= 9 * cb_num_sms() * Tile::BLOCKS || w.turned;
+  kern<<<grid, Tile::THREADS, smem, st>>>(p, v, nseq, cb_num_sms());
   return CB_LAUNCH_CHECK();
 }
 
@@ -894,14 +898,18 @@ static inline int scan_vp(int vdim) { return (vdim + SCAN_COLS - 1) / SCAN_COLS 
 // Decay mode, long portions of 64 and 128 channels: columns of a lane.  With four, columns share what is read of q and k, which is
 // what many units on an SM run out of; but one unit alone takes a token in 265 clocks, most of them waits, and two columns (170) or
 // one (120 at 64 channels) in as many more CTAs wait less.  So fewer columns where the longest sequence's walk is what the call
-// takes: where it is 5 / 4 of the tokens that an SM walks on average, counted with four; and one column where even then every CTA has an
+// takes: where it is 5 / 4 of the tokens that an SM walks on average, counted with four - twice them for 128 channels in sequences of one
+// length or more than 32 of them, where two columns are two units for some SMs and the same time (3 x 1000 of 8 heads 163, four 150; 2000 and 40 of 20, 16 heads 332,
+// four 311); and one column where even then every CTA has an
 // SM to itself.  Four / two / one columns, us, prepare kernel included: 1 x 12000 tokens of 16 heads x 128 x 128 (ratio 2.3) 1674 / 1076 / 1617,
 // 2 x 6000 (1.2 to 1.4) 1056 / 1000 / 1654, 4 x 2000 (0.7) 497 / 544 / 949, 8 x 1500 695 / 814 / 1326; 1 x 4534 of 8 heads (128 CTAs of one column) 622 / 396 /
 // 353; 1 x 12000 of 16 heads x 64 x 64 1166 / 691 / 478; 2 x 3000 of 8 heads x 64 x 64 359 / 216 / 152; 1 x 2602 of 4 heads x 64 x 128 253 / 151 / 106;
 // 16 x 500 of 4 heads x 64 x 96 (1.1) 101 / 87 / 106.  The bits are the same.
 static inline int scan_columns(const ScanWork& w, int heads, int nseq, int64_t tokens, int max_q) {
   const int64_t sms = cb_num_sms();
-  if ((w.DK != 64 && w.DK != 128) || 4 * (int64_t)max_q * sms < 5 * tokens * heads * (w.VP / SCAN_COLS)) return SCAN_CPL;
+  const bool even = 10 * tokens >= 9 * (int64_t)nseq * max_q;
+  const int over = w.DK == 128 && (even || nseq > 32) ? 8 : 5;
+  if ((w.DK != 64 && w.DK != 128) || 4 * (int64_t)max_q * sms < over * tokens * heads * (w.VP / SCAN_COLS)) return SCAN_CPL;
   return (int64_t)nseq * heads * (w.VP / 8) <= sms ? 1 : 2;
 }
 
@@ -935,6 +943,7 @@ int launch_scan(const ScanParams& p, float* work, int64_t tokens, int nseq, int 
     else if (w.DK == 128) exp_gate_kernel<128><<<blocks, 128, 0, st>>>(p, w, nseq);
     else exp_gate_kernel<256><<<blocks, 128, 0, st>>>(p, w, nseq);
   }
+  w.turned = (int64_t)nseq * max_q >= 2 * tokens;
   if constexpr (MODE == SCAN_DECAY) {
     const int columns = max_q > SCAN_SHORT ? scan_columns(w, p.heads, nseq, tokens, max_q) : SCAN_CPL;
     if (columns == 1) return w.DK == 64 ? launch_scan_dk<64, MODE, false, 1>(p, w, nseq, st) : launch_scan_dk<128, MODE, false, 1>(p, w, nseq, st);
