@@ -157,8 +157,9 @@ __global__ void __launch_bounds__(512) ce_softmax_grad_kernel(const T* __restric
     return;
   }
   constexpr int STEP = 512 * VEC;
-  constexpr int UNROLL = sizeof(T) == 4 ? 1 : CE_UNROLL;       // 4096 x 128256 bf16, all with labels: one vector 560 us (with the forward), four 528; fp32
-                                                               // 1700 x 151936 496 and 498
+  // 4096 x 128256 bf16, all with labels: one vector at a time 560 us (with the forward), four 528; fp32, one and two: 64 x 32000 19.1 and 17.8, 300 x 128256
+  // 98 and 87, 2000 x 102400 397 and 390 (one, as the compiler unrolled it in a plain loop, 18.1, 97.7 and 399)
+  constexpr int UNROLL = sizeof(T) == 4 ? 2 : CE_UNROLL;
   auto part = [&](int c0, auto whole_tag) {      // (a copy of the code for a row's end, as above)
     constexpr bool WHOLE = decltype(whole_tag)::value;
     Vec16<T> v[UNROLL], o;
