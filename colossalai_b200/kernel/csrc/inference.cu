@@ -42,17 +42,21 @@ template <int N> CB_DEVICE void cp_async_wait() { asm volatile("cp.async.wait_gr
 // ---- how a decode step's sequences are cut (cb_decode_num_splits)
 // Warps of a CTA, one for each kv head.  Four heads of 128, so that two CTAs fit an SM and one's beginning and end lie under the other's
 // loads; all heads of 64 up to eight, four where there are more.  Device time, us, eight / four warps: 64 x 2048 tokens of 32 / 8 heads of 128
-// 78.0 / 76.4, 128 x 1024 85.3 / 82.5, 128 x 1024 of 12 heads of 64 62.3 / 56.6, 48 x 2700 of 24 / 8 heads of 64 40.6 / 41.0.
+// 78.0 / 76.4, 128 x 1024 85.3 / 82.5, 128 x 1024 of 12 heads of 64 62.3 / 56.6, 48 x 2700 of 24 / 8 heads of 64 40.6 / 41.0.  Six heads of 128 in one CTA: 8 x
+// 500 9.9 instead of 10.8, but 8 x 2000 18.0 instead of 16.9.
 constexpr int DEC_MMA_WARPS = 4;
 // Few sequences are cut into as many partitions as run at once, equal ones of each sequence's own length: a second round of CTAs, and twice as
 // many partial results to add up, cost more than they balance, and what a table has room for is often several times what is in it.
 // Two rounds of what the table holds / one of the length, tables just wide enough, us: 16 x 1024 tokens of 32 / 8 heads of 128 22.6 / 18.2, 16 x 8000
 // 86 / 79, 2 x 16000 38.0 / 29.6, 10 x 8000 60.0 / 54.9, 28 x 4000 75.0 / 69.8, 6 x 12000 of 16 / 2 heads of 64 29.1 / 22.4, 60 x 2000 of 16 / 2 heads of 128
-// 37.8 / 31.2, 5 x 8000 of 12 heads 50.5 / 43.9; tables of 8192 tokens of which 500 to 1000 are in use, 16 sequences 40.8 / 17, 28 64 / 21.  How
-// many that is at most: decode_most_splits.  Where a round is fewer than DEC_ROUND_SPLITS partitions - lengths differ by more than one - two rounds (one / two: 40 x 3000 79.8 / 73.0, 32 x
-// 4000 79.8 / 76.0), and where that is as few, and for more than four heads of 64, of what the table holds (64 x 2048 76.9, own 80.3; 30 x 4000 of 24 / 8
-// heads of 64 38.6, own 43.4).
-constexpr int DEC_PART_MIN = 64, DEC_ROUND_SPLITS = 5, DEC_MOST_SPLITS = 64;
+// 37.8 / 31.2, 5 x 8000 of 12 heads 50.5 / 43.9; tables of 8192 tokens of which 500 to 1000 are in use, 16 sequences 40.8 / 17, 28 64 / 21.  Four heads gain
+// where tables are wide or lengths equal (6 x 8000 34 / 27); 32 to 64 sequences of uneven lengths in tables just wide enough lose 7 to 11 %.
+// How many that is at most: decode_most_splits.  Where a round is fewer than DEC_ROUND_SPLITS partitions - lengths differ by more than one - two rounds
+// (one / two: 40 x 3000 79.8 / 73.0, 32 x 4000 79.8 / 76.0), unless three or four are of DEC_SHORT / 4 to DEC_SHORT tokens, whose beginnings count for more
+// (32 x 1000 26.4 / 28.7, 24 x 1000 of 12 heads 24.7 / 28.1, 64 x 500 of four 16.5 / 19.2, 128 x 1000 of two 25.8 / 29.0; 64 x 2000 of four, parts of 500, 44.6 /
+// 45.1).  Where two rounds are as few, and for more than four heads of 64, by what the table holds (64 x 2048 76.9, own 80.3; 30 x 4000 of 24 / 8 heads of 64
+// 38.6, own 43.4).
+constexpr int DEC_PART_MIN = 64, DEC_ROUND_SPLITS = 5, DEC_MOST_SPLITS = 64, DEC_SHORT_SPLITS = 3, DEC_SHORT = 384;
 constexpr int DEC_WIDE = 48;           // partitions from which decode_reduce_wide_kernel adds them up
 static inline int decode_warps(int kv_heads, int head_dim) {
   const int most = head_dim == 128 || kv_heads > 8 ? DEC_MMA_WARPS : 8;
@@ -61,6 +65,7 @@ static inline int decode_warps(int kv_heads, int head_dim) {
 struct DecodeCut {
   const int* seq_lens;
   int capacity, part_len, window;      // tokens that a table has room for
+  unsigned per;                        // 2^32 / part_len, rounded up, where that divides what a table has room for; or 0
 };
 // tokens of a partition: part_len, or, where that is negative, an equal share of the sequence's own, of -part_len at least
 CB_DEVICE int decode_partition(int cached, int splits, int part_len) {
@@ -71,6 +76,7 @@ CB_DEVICE int decode_partition(int cached, int splits, int part_len) {
 CB_DEVICE int decode_first(int window_start, int part_len) { return part_len < 0 ? window_start & ~15 : 0; }
 // partitions of a sequence up to the last that has tokens
 CB_DEVICE int decode_used(const DecodeCut& c, int seq, int splits) {
+  if (c.per) return min(splits, (int)__umulhi(max(0, min(c.seq_lens[seq], c.capacity)) + c.part_len - 1, c.per));   // (a division: + .2 us)
   const int len = c.seq_lens[seq], first = c.window > 0 ? decode_first(max(0, len - c.window), c.part_len) : 0;
   const int cached = min(len, c.capacity) - first, part = decode_partition(cached, splits, c.part_len);
   return max(0, min(splits, (cached + part - 1) / part));
@@ -437,8 +443,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 1) paged_decode_mma_kernel(
   const int len = seq_lens[seq];
   const int window_start = window > 0 ? max(0, len - window) : 0;
   const int cached = min(len, max_blocks_per_seq * block_size);                                 // (no pages beyond the table's row)
-  // (asked in every call, one sequence of 4097 tokens took 14.4 us instead of 14.0)
-  const int first = REST ? decode_first(window_start, part_len) : 0;
+  const int first = REST ? decode_first(window_start, part_len) : 0;           // (in every call: one sequence of 4097 tokens 14.4 us, 14.0 so)
   const int part = decode_partition(cached - first, splits, part_len);
   const int t0 = max(first + split * part, window_start);
   const int t1 = min(cached, first + split * part + part);
@@ -758,15 +763,21 @@ int cb_decode_num_splits(int num_seqs, int kv_heads, int head_dim, int max_len, 
   if (num_seqs <= 0 || kv_heads <= 0) return 1;
   const int sms = cb_num_sms();
   const int warps = decode_warps(kv_heads, head_dim);
-  const int fit = 227 * 1024 / (warps * DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * head_dim * 2), per_sm = fit < 8 ? fit : 8;
+  // CTAs of an SM: as many as fit, of eight warps in all for heads of 128 (three heads, two or three CTAs: 32 x 2000 23 and 29, 64 x 500 15 and 19)
+  const int fit = 227 * 1024 / (warps * DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * head_dim * 2), some = (head_dim == 128 ? 8 : 16) / warps;
+  const int per_sm = fit < some ? fit : some < 8 ? some : 8;
   const int ctas = num_seqs * ((kv_heads + warps - 1) / warps), one_round = per_sm * sms / ctas, two_rounds = 2 * per_sm * sms / ctas;
   if ((head_dim == 128 || kv_heads <= 4) && head_dim <= 128 && (one_round >= DEC_ROUND_SPLITS || two_rounds > DEC_ROUND_SPLITS)) {
     *part_len_out = -DEC_PART_MIN;
-    const int most = (decode_in_sight(max_len, window) + DEC_PART_MIN - 1) / DEC_PART_MIN;
-    const int own = one_round >= DEC_ROUND_SPLITS ? one_round : two_rounds;
-    const int cap = decode_most_splits(num_seqs, kv_heads, head_dim, one_round, decode_in_sight(max_len, window));
-    const int splits = own < cap ? own : cap;
-    return splits < most ? splits : most < 1 ? 1 : most;
+    const int tokens = decode_in_sight(max_len, window), most = (tokens + DEC_PART_MIN - 1) / DEC_PART_MIN;
+    const bool short_parts = one_round >= DEC_SHORT_SPLITS && tokens <= DEC_SHORT * one_round && tokens > DEC_SHORT / 4 * one_round;
+    const int own = one_round >= DEC_ROUND_SPLITS || short_parts ? one_round : two_rounds;
+    const int cap = decode_most_splits(num_seqs, kv_heads, head_dim, one_round, tokens);
+    int splits = own < cap ? own : cap;
+    if (most <= cap && most <= own + own / 4) splits = most;          // (a few more than fit, whose weights need no rest)
+    if (splits < most) return splits;
+    if (window <= 0) *part_len_out = DEC_PART_MIN;                    // what every length's own share comes to then
+    return most < 1 ? 1 : most;
   }
   // two rounds of CTAs of eight kv heads, partitions of at least DEC_PART_MIN of the tokens that a table has room for
   const int most = (max_len + DEC_PART_MIN - 1) / DEC_PART_MIN;
@@ -801,14 +812,16 @@ int cb_paged_decode_attention(const void* q, const void* k_cache, const void* v_
   const char* impl_env = getenv("CB200_DECODE");
   const bool use_mma = !(impl_env != nullptr && impl_env[0] == 's') && G <= 8 && (D == 128 || D == 64);
   const int mma_warps = decode_warps(Hkv, D);
-  const DecodeCut cut{seq_lens, max_blocks_per_seq * block_size, part_len, window};
+  const int capacity = max_blocks_per_seq * block_size;
+  const bool divides = part_len > 0 && (int64_t)(capacity + part_len) * part_len < (1ll << 32);
+  const DecodeCut cut{seq_lens, capacity, part_len, window, divides ? (unsigned)(((1ull << 32) + part_len - 1) / part_len) : 0u};
   dim3 mma_grid(num_seqs, (Hkv + mma_warps - 1) / mma_warps, splits);
 #define LAUNCH_DEC_MMA(T, DD)                                                                                       \
   {                                                                                                                  \
     constexpr int per_warp = DEC_MMA_STAGES * 2 * DEC_MMA_TOKENS * DD * 2;                                           \
     static CbDeviceAttr attr;                                                                                        \
     static CbDeviceAttr attr_rest;                                                                                   \
-    const bool rest = part_len < 0 && (window > 0 || cut.capacity > (int64_t)DEC_PART_MIN * splits);                   \
+    const bool rest = part_len < 0;                                                                                  \
     auto kern = rest ? paged_decode_mma_kernel<T, DD, true> : paged_decode_mma_kernel<T, DD, false>;                 \
     if (const int e = cb_allow_smem(rest ? attr_rest : attr, kern, (DEC_THREADS / 32) * per_warp)) return e;         \
     if (const int e = cb_launch_early(kern, mma_grid, mma_warps * 32, mma_warps * per_warp, s, \
