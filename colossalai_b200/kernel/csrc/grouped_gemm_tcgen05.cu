@@ -310,7 +310,7 @@ grouped_rows_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
       }
     }
   } else {
-    // ================================================================ epilogue (warps 2..5, both CTAs): lane = output column
+    // ================================================================ epilogue (warps 2..5, gated 2..9, both CTAs): lane = output column
     const int quarter = warp & 3, turn = (warp - 2) >> 2;                  // gated: 32 rows of each 64 a warp
     uint8_t* box = smem_box + (turn * 4 + quarter) * ROW_BOX_BYTES;        // [32 token rows][32 columns]
     const auto drained = [&](int a) {

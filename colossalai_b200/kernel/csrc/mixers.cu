@@ -260,7 +260,7 @@ struct ScanParams {
 // The workspace rows of SCAN_TOK_TILE tokens arrive by cp.async in a ring of stages while the previous tile is walked (decay
 // mode has three, so that one barrier per tile is enough).
 // Bound: the serial chain of a sequence, shared-memory reads (q and k once per CPL columns) and fp32 issue, none of them
-// alone (three units on an SM: its fp32 pipe 57 % busy, half of the issue slots; a unit's warp waits 64 % of its time when alone).  12000 tokens in eight uneven sequences, 16 heads, 128 x 128, decay mode: recurrence 741 -> 594 us.  Holding S divided
+// alone (three units on an SM: its fp32 pipe 57 % busy, half of the issue slots; a unit's warp waits 64 % of its time when alone).  12000 tokens in eight uneven sequences, 16 heads, 128 x 128, decay mode: recurrence 741 -> 543 us.  Holding S divided
 // by its decay's powers inside a tile of eight tokens (505 us) made the bits depend on how a sequence is cut into portions, and
 // turned infinite values into NaN.
 constexpr int SCAN_CPL = 4;            // value columns per lane (fewer: scan_columns)
